@@ -122,6 +122,20 @@ const size_t* resolve_metadata(const size_t* meta, size_t count);
 // used in stream order on the thread's current stream.
 void* scratch(size_t bytes);
 
+// Workspace of one call, in the order of the stream the calling thread launches on: allocated there, freed there when it
+// goes out of scope, so calls on different streams or threads never share it and a stream switch needs no wait.  take()
+// fails, with no error recorded, while that stream is being captured or when memory is short; the caller then takes the
+// route it has without a workspace.
+struct StreamWorkspace {
+    void* ptr = nullptr;
+    cudaStream_t stream = 0;
+    bool take(size_t bytes);
+    StreamWorkspace() {}
+    StreamWorkspace(const StreamWorkspace&) = delete;
+    StreamWorkspace& operator=(const StreamWorkspace&) = delete;
+    ~StreamWorkspace();
+};
+
 int sm_count();
 // Blocks of `kernel` that stay resident on one SM at this block size and dynamic shared memory (at least 1).
 int resident_blocks(const void* kernel, int threads, size_t dynamic_smem = 0);

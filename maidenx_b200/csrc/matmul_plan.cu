@@ -36,6 +36,9 @@ bool mm_parse(const size_t* hm, MmDesc& d) {
     d.k_bwd = d.b_nd >= 2 ? b_shape[d.b_nd - 2] : a_shape[d.a_nd - 1];  // matmul.rs:170-176
     d.g_size = 1;
     for (size_t i = 0; i < d.out_nd; i++) d.g_size *= out_shape[i];
+    d.a_elems = d.b_elems = 1;
+    for (size_t i = 0; i < d.a_nd; i++) d.a_elems *= a_shape[i];
+    for (size_t i = 0; i < d.b_nd; i++) d.b_elems *= b_shape[i];
     d.a_cont = contiguous(d.a_nd, a_shape, a_st);
     d.b_cont = contiguous(d.b_nd, b_shape, b_st);
     if (d.a_nd >= 2) {

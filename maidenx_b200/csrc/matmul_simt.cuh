@@ -209,6 +209,7 @@ struct MmDesc {
     int64_t a_strides[3];          // batch (a_strides[0]), row (a_strides[nd-2]), col (a_strides[nd-1]); rank 1: col only
     int64_t b_strides[3];
     uint64_t a_off, b_off;
+    uint64_t a_elems, b_elems;     // products of the operands' shapes
 };
 bool mm_parse(const size_t* hm, MmDesc& d);
 size_t mm_meta_words(const size_t* head3);

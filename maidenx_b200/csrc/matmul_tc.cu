@@ -26,6 +26,7 @@
 // error word, stops issuing work and falls through to the common exit, where TMEM is freed.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <unordered_map>
@@ -47,7 +48,8 @@ std::atomic<int> g_group_m{16};  // row-tiles per column sweep of the one-CTA ke
 
 constexpr int BM = 128, BN = 256, BK = 64;    // CTA tile; BK * 2 bytes = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-constexpr int STAGES = 4;
+constexpr int STAGES = 4;                     // ring stages of full-width tiles; narrower ones get as many as fit the same bytes
+constexpr int MAX_STAGES = 8;
 constexpr int A_STAGE_BYTES = BM * BK * 2;    // 16 KB
 constexpr int B_STAGE_BYTES = BN * BK * 2;    // 32 KB
 constexpr int EPI_WARPS = 4;
@@ -59,25 +61,27 @@ constexpr int GROUP_M = 16;                   // row-tiles per column sweep (L2 
 
 struct SmemLayout {
     // offsets inside the dynamic shared memory block (base aligned to 1024 bytes)
-    static constexpr int a = 0;
-    static constexpr int b = a + STAGES * A_STAGE_BYTES;
-    static constexpr int epi = b + STAGES * B_STAGE_BYTES;
+    static constexpr int ring = 0;  // stage s: A block, then B block (bn rows of 128 bytes), s * stage_bytes further
+    static constexpr int epi = ring + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES);
     static constexpr int bars = epi + EPI_WARPS * 2 * EPI_STAGE_BYTES;
     static constexpr int total = bars + 256;
 };
 constexpr int TC_SMEM_BYTES = SmemLayout::total + 1024;  // slack for the 1024-byte alignment
 
+// Split-K of a short reduction: what its second launch and the wider partial results cost, in k-blocks (0.27 us each on one CTA)
+constexpr double kSplitFixed16 = 10.0;
+
 constexpr int MN_CHUNK_BYTES = 64 * BK * 2;  // one [64 K-rows x 64 MN] box
 
 // Instruction descriptor of tcgen05.mma kind::f16 with f32 accumulation.
-__host__ __device__ constexpr uint32_t make_idesc(bool is_bf16, bool a_mn_major, bool b_mn_major) {
+__host__ __device__ constexpr uint32_t make_idesc(bool is_bf16, bool a_mn_major, bool b_mn_major, int bn) {
     uint32_t d = 0;
     d |= 1u << 4;                               // D format: f32
     d |= (is_bf16 ? 1u : 0u) << 7;              // A format: 0 = f16, 1 = bf16
     d |= (is_bf16 ? 1u : 0u) << 10;             // B format
     d |= (a_mn_major ? 1u : 0u) << 15;          // A major: 0 = K, 1 = MN
     d |= (b_mn_major ? 1u : 0u) << 16;          // B major
-    d |= (uint32_t)(BN >> 3) << 17;             // N / 8
+    d |= (uint32_t)(bn >> 3) << 17;             // N / 8
     d |= (uint32_t)(BM >> 4) << 24;             // M / 16
     return d;
 }
@@ -94,6 +98,13 @@ struct TcParams {
     const void* bias;  // fuse != 0: one element of the operand type in device memory
     int a_mn, b_mn;  // operand is MN-major in global memory ([K, MN] row-major) instead of K-major ([MN, K])
     int group_m;     // row-tiles per column sweep (L2 re-use of the A panels)
+    int bn;          // columns of an output tile: 64, 128, 192 or 256 (tile_columns)
+    int stages, stage_bytes;  // of the operand ring
+    int split_kb;    // > 0: split-K; batch s of the launch reduces the k-blocks [s * split_kb, (s + 1) * split_kb) of one product
+    // The output's rows are not 16-byte multiples (or its base is not aligned), which no tensor map can describe: the epilogue
+    // warps copy their staged rows to `d` themselves, in steps of 2 bytes (1) or, for even N, 4 bytes (2).  0: tensor stores.
+    int d_plain;
+    void* d;
     // Short reductions (num_kb <= STAGES, one batch): `b_keep` CTAs share each column tile, CTA j of them takes the row
     // tiles j, j + b_keep, ...; the B panel of the column tile is loaded once into the B slots of the ring (slot = k-block,
     // the ring is num_kb slots long) and only A streams.  0: the general schedule.
@@ -141,6 +152,18 @@ __device__ __forceinline__ float round16(float v, int is_bf16) {
     return is_bf16 ? to_f32(from_f32<bf16>(v)) : to_f32(from_f32<f16>(v));
 }
 
+// What the epilogue does is compiled in: each form keeps its registers and its code to itself, and the plain product's loop is
+// not laid out around the others.
+enum TcMode {
+    TC_STORE = 0,  // tensor stores of the rounded product or of f32 split-K partials
+    TC_BIAS,       // fuse 1..3, tensor stores
+    TC_PLAIN,      // d_plain: rows written by the warps; fuse 0 or 3
+};
+
+// BN_T: the tile's columns where they are 256, else 0 (from the parameters).  The ring of full-width tiles is four stages deep and waits
+// out a round trip to L2 in them, so the single producer thread's own instructions between a freed stage and its refill count:
+// with the geometry from the parameters the products of a 16384 x 8192 layer took 12 % longer at full clock.
+template <int MODE, int BN_T>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                const __grid_constant__ CUtensorMap map_d2, TcParams p, int* err, int tag) {
@@ -149,17 +172,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t smem_base = smem_u32(smem);
     const uint32_t bar_base = smem_base + SmemLayout::bars;
-    // barrier slots (8 bytes each): full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2]; then the TMEM base word
+    // barrier slots (8 bytes each): full[MAX_STAGES], empty[MAX_STAGES], tmem_full[2], tmem_empty[2]; then the TMEM base word
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
-    auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
-    auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
-    auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
-    volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(smem + SmemLayout::bars + 8 * (2 * STAGES + 4));
+    auto empty_bar = [&](int s) { return bar_base + 8u * (MAX_STAGES + s); };
+    auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * MAX_STAGES + a); };
+    auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * MAX_STAGES + 2 + a); };
+    volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(smem + SmemLayout::bars + 8 * (2 * MAX_STAGES + 4));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? STAGES : p.stages, stage_bytes = BN_T ? A_STAGE_BYTES + BN_T * BK * 2 : p.stage_bytes;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) {
+        for (int s = 0; s < MAX_STAGES; s++) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
@@ -184,31 +208,31 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            const int ring = p.b_keep ? p.num_kb : STAGES;
+            const int ring = p.b_keep ? p.num_kb : stages;
             int tm, tn, tb;
             for (int it = 0; ok && next_tile(it, p, tm, tn, tb); it++) {
                 const int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
+                int k = tb * p.split_kb * BK;              // a k-block past the end of K is all fill: zeros
                 const bool load_b = !p.b_keep || it == 0;  // the kept B panel arrives with the first tile's A blocks
-                for (int kb = 0; kb < p.num_kb; kb++) {
+                for (int kb = 0; kb < p.num_kb; kb++, k += BK) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, err, tag, 1)) {
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(full_bar(stage), A_STAGE_BYTES + (load_b ? B_STAGE_BYTES : 0));
-                    const uint32_t sa = smem_base + SmemLayout::a + stage * A_STAGE_BYTES;
-                    const uint32_t sb = smem_base + SmemLayout::b + stage * B_STAGE_BYTES;
+                    mbar_expect_tx(full_bar(stage), A_STAGE_BYTES + (load_b ? bn * BK * 2 : 0));
+                    const uint32_t sa = smem_base + SmemLayout::ring + stage * stage_bytes, sb = sa + A_STAGE_BYTES;
                     if (!p.a_mn) {
-                        tma_load_3d(sa, &map_a, kb * BK, tm * BM, za, full_bar(stage));
+                        tma_load_3d(sa, &map_a, k, tm * BM, za, full_bar(stage));
                     } else {
 #pragma unroll
-                        for (int h = 0; h < BM / 64; h++) tma_load_3d(sa + h * MN_CHUNK_BYTES, &map_a, tm * BM + h * 64, kb * BK, za, full_bar(stage));
+                        for (int h = 0; h < BM / 64; h++) tma_load_3d(sa + h * MN_CHUNK_BYTES, &map_a, tm * BM + h * 64, k, za, full_bar(stage));
                     }
                     if (!load_b) {
                     } else if (!p.b_mn) {
-                        tma_load_3d(sb, &map_b, kb * BK, tn * BN, zb, full_bar(stage));
+                        tma_load_3d(sb, &map_b, k, tn * bn, zb, full_bar(stage));
                     } else {
 #pragma unroll
-                        for (int h = 0; h < BN / 64; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * BN + h * 64, kb * BK, zb, full_bar(stage));
+                        for (int h = 0; h < bn / 64; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * bn + h * 64, k, zb, full_bar(stage));
                     }
                     if (++stage == ring) {
                         stage = 0;
@@ -220,14 +244,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (lane == 0) {
-            const uint32_t idesc = make_idesc(p.is_bf16 != 0, p.a_mn != 0, p.b_mn != 0);
+            const uint32_t idesc = make_idesc(p.is_bf16 != 0, p.a_mn != 0, p.b_mn != 0, bn);
             // per-operand descriptor geometry: (leading, stride) byte offsets and the K step in 16-byte units
             const uint32_t a_lbo = p.a_mn ? MN_CHUNK_BYTES : 16, b_lbo = p.b_mn ? MN_CHUNK_BYTES : 16;
             const uint64_t a_kstep = p.a_mn ? (2048 >> 4) : (32 >> 4), b_kstep = p.b_mn ? (2048 >> 4) : (32 >> 4);
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
-            const int ring = p.b_keep ? p.num_kb : STAGES;
+            const int ring = p.b_keep ? p.num_kb : stages;
             int tm, tn, tb;
             for (int it = 0; ok && next_tile(it, p, tm, tn, tb); it++) {
                 if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1, err, tag, 2)) break;
@@ -239,8 +263,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t da = smem_desc_sw128(smem_base + SmemLayout::a + stage * A_STAGE_BYTES, a_lbo, 1024);
-                    const uint64_t db = smem_desc_sw128(smem_base + SmemLayout::b + stage * B_STAGE_BYTES, b_lbo, 1024);
+                    const uint32_t sa = smem_base + SmemLayout::ring + stage * stage_bytes;
+                    const uint64_t da = smem_desc_sw128(sa, a_lbo, 1024), db = smem_desc_sw128(sa + A_STAGE_BYTES, b_lbo, 1024);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; k++) umma_f16(d_tmem, da + a_kstep * k, db + b_kstep * k, idesc, (kb | k) != 0);
                     umma_commit(empty_bar(stage));  // the stage may be refilled once these MMAs have read it
@@ -265,13 +289,13 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         int acc = 0, buf = 0;
         uint32_t acc_phase = 0;
         float fused_bias = 0.0f;
-        if (p.fuse == 1 || p.fuse == 2) fused_bias = p.is_bf16 ? to_f32(*static_cast<const bf16*>(p.bias)) : to_f32(*static_cast<const f16*>(p.bias));
+        if (MODE == TC_BIAS && p.fuse != 3) fused_bias = p.is_bf16 ? to_f32(*static_cast<const bf16*>(p.bias)) : to_f32(*static_cast<const f16*>(p.bias));
         int tm, tn, tb;
         for (int it = 0; next_tile(it, p, tm, tn, tb); it++) {
             // the TMEM loads below are warp-collective: leave the loop only as a whole warp
             // four warps wait here for most of a tile's reduction: they sleep between polls, so that their polling does not
             // take shared-memory cycles from the TMA writes and the tensor core's operand reads
-            if (p.fuse == 3) {  // this thread's output row inside the batch's matrix
+            if (MODE != TC_STORE && p.fuse == 3) {  // this thread's output row inside the batch's matrix
                 const int row = tm * BM + quarter * 32 + lane;
                 fused_bias = row < p.M ? (p.is_bf16 ? to_f32(static_cast<const bf16*>(p.bias)[row]) : to_f32(static_cast<const f16*>(p.bias)[row])) : 0.0f;
             }
@@ -279,9 +303,51 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             if (!__all_sync(0xFFFFFFFFu, ready)) break;
             tc_fence_after();
             const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
+            const int rows_here = min(32, p.M - (tm * BM + quarter * 32));  // may be <= 0: this warp's rows lie below the matrix
+            // Hands the staged 32 rows of 128 bytes (first output column `col`) to the copy engine, or writes them itself.
+            auto flush = [&](const CUtensorMap* map, int col) {
+                unsigned char* src = stage_buf + buf * EPI_STAGE_BYTES;
+                buf ^= 1;
+                if constexpr (MODE != TC_PLAIN) {
+                    if (lane == 0) {
+                        tma_store_3d(map, smem_u32(src), col, tm * BM + quarter * 32, tb);
+                        tma_store_commit();
+                    }
+                    return;
+                }
+                uint16_t* dst = static_cast<uint16_t*>(p.d) + ((size_t)tb * p.M + tm * BM + quarter * 32) * p.N + col;
+                const int cols = min(64, p.N - col);
+                // Eight rows at a time, all loads before the first store: the compiler cannot tell the staging tile from `d`, and a
+                // load behind a store waits for it.
+                if (p.d_plain == 2) {
+                    for (int r0 = 0; r0 < 32; r0 += 8) {
+                        uint32_t v[8];
+#pragma unroll
+                        for (int r = 0; r < 8; r++) v[r] = *reinterpret_cast<const uint32_t*>(src + (r0 + r) * 128 + (((lane >> 2) ^ r) << 4) + (lane & 3) * 4);
+#pragma unroll
+                        for (int r = 0; r < 8; r++)
+                            if (r0 + r < rows_here && 2 * lane < cols) *reinterpret_cast<uint32_t*>(dst + (size_t)(r0 + r) * p.N + 2 * lane) = v[r];
+                    }
+                    return;
+                }
+                const int c0 = lane, c1 = lane + 32;
+                for (int r0 = 0; r0 < 32; r0 += 8) {
+                    uint16_t v0[8], v1[8];
+#pragma unroll
+                    for (int r = 0; r < 8; r++) {
+                        v0[r] = *reinterpret_cast<const uint16_t*>(src + (r0 + r) * 128 + (((c0 >> 3) ^ r) << 4) + (c0 & 7) * 2);
+                        v1[r] = *reinterpret_cast<const uint16_t*>(src + (r0 + r) * 128 + (((c1 >> 3) ^ r) << 4) + (c1 & 7) * 2);
+                    }
+#pragma unroll
+                    for (int r = 0; r < 8; r++) {
+                        if (r0 + r < rows_here && c0 < cols) dst[(size_t)(r0 + r) * p.N + c0] = v0[r];
+                        if (r0 + r < rows_here && c1 < cols) dst[(size_t)(r0 + r) * p.N + c1] = v1[r];
+                    }
+                }
+            };
             // One 64-column chunk: round, stage in shared memory (XOR-swizzled rows), hand to the copy engine.
             auto store_chunk = [&](int c, uint32_t (&v0)[32], uint32_t (&v1)[32]) {
-                if (p.fuse) {
+                if (MODE == TC_BIAS || (MODE == TC_PLAIN && p.fuse)) {
                     // Linear + bias (+ GELU) in one pass, with the roundings of the separate ops: the product is rounded to
                     // the operand type, the bias is added in f32 and rounded (u), the activation is evaluated on u in f32
                     // and rounded (act) - bit for bit what cuda_matmul, cuda_add and cuda_gelu give one after the other.
@@ -292,7 +358,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        if (h == 1 && p.fuse != 2) break;
+                        if (h == 1 && (MODE == TC_PLAIN || p.fuse != 2)) break;
                         if (lane == 0) tma_store_wait_read<1>();
                         __syncwarp();
                         unsigned char* dst = stage_buf + buf * EPI_STAGE_BYTES + lane * 128;
@@ -311,15 +377,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         }
                         fence_proxy_async_smem();
                         __syncwarp();
-                        if (lane == 0) {
-                            tma_store_3d(h ? &map_d2 : &map_d, smem_u32(stage_buf + buf * EPI_STAGE_BYTES), tn * BN + c * EPI_CHUNK_COLS, tm * BM + quarter * 32, tb);
-                            tma_store_commit();
-                        }
-                        buf ^= 1;
+                        flush(h ? &map_d2 : &map_d, tn * bn + c * EPI_CHUNK_COLS);
                     }
                     return;
                 }
-                if (p.out_f32) {
+                if (MODE == TC_STORE && p.out_f32) {
                     // two 32-column f32 chunks (128 bytes per row each), one per staging buffer
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
@@ -333,7 +395,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) {
-                            tma_store_3d(&map_d, smem_u32(stage_buf + buf * EPI_STAGE_BYTES), tn * BN + c * EPI_CHUNK_COLS + h * 32, tm * BM + quarter * 32, tb);
+                            tma_store_3d(&map_d, smem_u32(stage_buf + buf * EPI_STAGE_BYTES), tn * bn + c * EPI_CHUNK_COLS + h * 32, tm * BM + quarter * 32, tb);
                             tma_store_commit();
                         }
                         buf ^= 1;
@@ -356,33 +418,38 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) {
-                    tma_store_3d(&map_d, smem_u32(stage_buf + buf * EPI_STAGE_BYTES), tn * BN + c * EPI_CHUNK_COLS, tm * BM + quarter * 32, tb);
-                    tma_store_commit();
-                }
-                buf ^= 1;
+                flush(&map_d, tn * bn + c * EPI_CHUNK_COLS);
             };
             // The TMEM loads of chunk c + 1 are in flight while chunk c is converted and stored.
+            const int chunks = bn / EPI_CHUNK_COLS;
+            auto hand_back = [&] {  // every TMEM read of this accumulator is done: hand it back to the MMA warp
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(tempty_bar(acc));
+            };
             uint32_t a0[32], a1[32], b0[32], b1[32];
             tmem_ld_32x32b_x32(t_row, a0);
             tmem_ld_32x32b_x32(t_row + 32, a1);
 #pragma unroll
             for (int c = 0; c < BN / EPI_CHUNK_COLS; c += 2) {
+                if (c >= chunks) break;
                 tmem_ld_wait_for(a0);
                 reg_fence(a1);
-                tmem_ld_32x32b_x32(t_row + (c + 1) * EPI_CHUNK_COLS, b0);
-                tmem_ld_32x32b_x32(t_row + (c + 1) * EPI_CHUNK_COLS + 32, b1);
+                if (c + 1 < chunks) {
+                    tmem_ld_32x32b_x32(t_row + (c + 1) * EPI_CHUNK_COLS, b0);
+                    tmem_ld_32x32b_x32(t_row + (c + 1) * EPI_CHUNK_COLS + 32, b1);
+                } else {
+                    hand_back();
+                }
                 store_chunk(c, a0, a1);
+                if (c + 1 >= chunks) break;
                 tmem_ld_wait_for(b0);
                 reg_fence(b1);
-                if (c + 2 < BN / EPI_CHUNK_COLS) {
+                if (c + 2 < chunks) {
                     tmem_ld_32x32b_x32(t_row + (c + 2) * EPI_CHUNK_COLS, a0);
                     tmem_ld_32x32b_x32(t_row + (c + 2) * EPI_CHUNK_COLS + 32, a1);
                 } else {
-                    // every TMEM read of this accumulator is done: hand it back to the MMA warp
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(tempty_bar(acc));
+                    hand_back();
                 }
                 store_chunk(c + 1, b0, b1);
             }
@@ -426,10 +493,11 @@ bool opt_in_shared_memory() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
-        if (cudaFuncSetAttribute(tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
+        for (auto kernel : {tc_gemm_kernel<TC_STORE, BN>, tc_gemm_kernel<TC_BIAS, BN>, tc_gemm_kernel<TC_STORE, 0>, tc_gemm_kernel<TC_BIAS, 0>, tc_gemm_kernel<TC_PLAIN, 0>})
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
         done[dev] = true;
     }
     return true;
@@ -450,32 +518,22 @@ int keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, int ctas) {
     return tiles_m >= 4 * per_col ? per_col : 0;
 }
 
-bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, int fuse = 0, const void* bias = nullptr, void* D2 = nullptr) {
-    const void *A = c.A, *B = c.B;
-    const bool a_mn = c.a_mn, b_mn = c.b_mn;
+// The two-CTA kernel: B is staged in halves of 128 columns, a pair of CTAs owns a 256 x 256 tile.  Its split-K slices are
+// sub-matrices behind the third coordinate of the tensor maps.  false: nothing was launched.
+bool launch_two_cta(bool is_bf16, const TcProduct& c, void* D, const char* where, int grid) {
     const uint64_t M = c.m, N = c.n;
-    uint64_t K = c.k, batch = c.batch;
-    if (!opt_in_shared_memory()) return false;
-    TcParams p;
-    p.M = (int)M;
-    p.N = (int)N;
-    p.tiles_m = (int)((M + BM - 1) / BM);
-    p.tiles_n = (int)((N + BN - 1) / BN);
-    p.tiles_per_batch = p.tiles_m * p.tiles_n;
-    int grid = sm_count();
-    if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
-    // few output tiles, long reduction: cut K into slices that run as the batches of this launch
-    const int slices = (batch == 1 && !fuse) ? splitk_slices((uint64_t)p.tiles_per_batch, K, BK, grid) : 1;
+    uint64_t K = c.k, batch = c.batch, a_bs = (uint64_t)c.a_bs, b_bs = (uint64_t)c.b_bs, a_pitch = 0, b_pitch = 0;
+    const int tiles_m = (int)((M + BM - 1) / BM), tiles_n = (int)((N + BN - 1) / BN);
+    const int slices = batch == 1 ? splitk_slices((uint64_t)tiles_m * tiles_n, K, BK, grid) : 1;
     float* partial = nullptr;
-    uint64_t a_bs = (uint64_t)c.a_bs, b_bs = (uint64_t)c.b_bs, a_pitch = 0, b_pitch = 0;
     if (slices > 1) {
         partial = static_cast<float*>(scratch((size_t)slices * M * N * sizeof(float)));
         if (!partial) return false;
         const uint64_t Ks = K / slices;
-        a_pitch = a_mn ? M : K;  // rows keep the pitch of the whole matrix
-        b_pitch = b_mn ? N : K;
-        a_bs = a_mn ? Ks * M : Ks;  // MN-major: Ks rows further; K-major: Ks columns further
-        b_bs = b_mn ? Ks * N : Ks;
+        a_pitch = c.a_mn ? M : K;  // rows keep the pitch of the whole matrix
+        b_pitch = c.b_mn ? N : K;
+        a_bs = c.a_mn ? Ks * M : Ks;  // MN-major: Ks rows further; K-major: Ks columns further
+        b_bs = c.b_mn ? Ks * N : Ks;
         K = Ks;
         batch = (uint64_t)slices;
     }
@@ -485,55 +543,133 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     const CUtensorMapDataType t16 = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const CUtensorMapSwizzle sw = CU_TENSOR_MAP_SWIZZLE_128B;
     CUtensorMap ma, mb, md;
-    if (g_two_cta.load(std::memory_order_relaxed) && grid >= 2 && !fuse) {
-        // the two-CTA kernel: B is staged in halves of 128 columns, a pair of CTAs owns a 256 x 256 tile
-        const bool oka2 = a_mn ? make_map_3d(&ma, t16, 2, A, K, M, batch, a_bs, 64, sw, a_pitch) : make_map_3d(&ma, t16, 2, A, M, K, batch, a_bs, tc2::BM, sw, a_pitch);
-        const bool okb2 = b_mn ? make_map_3d(&mb, t16, 2, B, K, N, batch, b_bs, 64, sw, b_pitch) : make_map_3d(&mb, t16, 2, B, N, K, batch, b_bs, tc2::BN_HALF, sw, b_pitch);
-        const bool okd2 = partial ? make_map_3d(&md, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, partial, M, N, batch, M * N, 32) : make_map(&md, is_bf16, D, M, N, batch, M * N, 32);
-        if (oka2 && okb2 && okd2) {
-            tc2::Params q;
-            q.tile_pairs_m = (p.tiles_m + 1) / 2;
-            q.tiles_n = p.tiles_n;
-            q.tiles_per_batch = q.tile_pairs_m * q.tiles_n;
-            q.num_tiles = (int)batch * q.tiles_per_batch;
-            q.num_kb = (int)((K + BK - 1) / BK);
-            q.a_batched = (batch > 1 && a_bs != 0) ? 1 : 0;
-            q.b_batched = (batch > 1 && b_bs != 0) ? 1 : 0;
-            q.is_bf16 = is_bf16 ? 1 : 0;
-            q.out_f32 = partial ? 1 : 0;
-            q.a_mn = a_mn ? 1 : 0;
-            q.b_mn = b_mn ? 1 : 0;
-            if (tc2::launch(ma, mb, md, q, grid, err, tag, ctx().stream)) {
-                check_launch(where);
-                if (partial) splitk_reduce(is_bf16 ? 0 : 1, partial, slices, (size_t)(M * N), D, where);
-                return true;
-            }
-        }
-    }
-    const bool oka = a_mn ? make_map_3d(&ma, t16, 2, A, K, M, batch, a_bs, 64, sw, a_pitch) : make_map_3d(&ma, t16, 2, A, M, K, batch, a_bs, BM, sw, a_pitch);
-    const bool okb = b_mn ? make_map_3d(&mb, t16, 2, B, K, N, batch, b_bs, 64, sw, b_pitch) : make_map_3d(&mb, t16, 2, B, N, K, batch, b_bs, BN, sw, b_pitch);
+    const bool oka = c.a_mn ? make_map_3d(&ma, t16, 2, c.A, K, M, batch, a_bs, 64, sw, a_pitch) : make_map_3d(&ma, t16, 2, c.A, M, K, batch, a_bs, tc2::BM, sw, a_pitch);
+    const bool okb = c.b_mn ? make_map_3d(&mb, t16, 2, c.B, K, N, batch, b_bs, 64, sw, b_pitch) : make_map_3d(&mb, t16, 2, c.B, N, K, batch, b_bs, tc2::BN_HALF, sw, b_pitch);
     const bool okd = partial ? make_map_3d(&md, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, partial, M, N, batch, M * N, 32) : make_map(&md, is_bf16, D, M, N, batch, M * N, 32);
     if (!oka || !okb || !okd) return false;
+    tc2::Params q;
+    q.tile_pairs_m = (tiles_m + 1) / 2;
+    q.tiles_n = tiles_n;
+    q.tiles_per_batch = q.tile_pairs_m * q.tiles_n;
+    q.num_tiles = (int)batch * q.tiles_per_batch;
+    q.num_kb = (int)((K + BK - 1) / BK);
+    q.a_batched = (batch > 1 && a_bs != 0) ? 1 : 0;
+    q.b_batched = (batch > 1 && b_bs != 0) ? 1 : 0;
+    q.is_bf16 = is_bf16 ? 1 : 0;
+    q.out_f32 = partial ? 1 : 0;
+    q.a_mn = c.a_mn ? 1 : 0;
+    q.b_mn = c.b_mn ? 1 : 0;
+    if (!tc2::launch(ma, mb, md, q, grid, err, tag, ctx().stream)) return false;
+    check_launch(where);
+    if (partial) splitk_reduce(is_bf16 ? 0 : 1, partial, slices, M, N, N, D, where);
+    return true;
+}
+
+int ring_stages(int bn) { return std::min(MAX_STAGES, STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) / (A_STAGE_BYTES + bn * BK * 2)); }
+// k-blocks of tensor-core time (M128 N256 K64: 512 cycles) that one k-block of a bn-wide tile takes: the columns' share; the
+// operand reads from shared memory (a k-step of N64 needs 48 cycles for its 6 KB, 32 for its multiplications); or the ring, whose
+// stages all wait out one round trip to L2 of about 1.2 us.
+double kb_cost(int bn) { return std::max(std::max(bn / 256.0, (128 + bn) / 512.0), 4.4 / ring_stages(bn)); }
+// Columns of an output tile.  256 feeds the tensor core best, so narrower tiles are for products that 256-wide tiles serve
+// badly: an N that fills its last tile poorly (N = 64 would compute 256 columns, N = 384 512) or too few tiles to reach every
+// SM.  The estimate is in k-blocks of a 256-wide tile: a wave's reduction, and its epilogue in proportion to the columns.
+// From two waves of 256-wide tiles on only the columns count: at the power cap a part-filled last wave costs nothing.
+// bf16 512 x 1024 x 1024 (64 tiles of 64 columns instead of 16): 8.7 us, 10.0 on full-width tiles.
+double tile_cost(int bn, uint64_t tiles_m, uint64_t N, uint64_t batch, uint64_t num_kb, int grid) {
+    const uint64_t tiles = tiles_m * ((N + bn - 1) / bn) * batch, tiles_256 = tiles_m * ((N + 255) / 256) * batch;
+    const double waves = tiles_256 > 2 * (uint64_t)grid ? (double)tiles / grid : (double)((tiles + grid - 1) / grid);
+    return waves * ((double)num_kb * kb_cost(bn) + 3.0 * bn / 256.0);
+}
+int tile_columns(uint64_t tiles_m, uint64_t N, uint64_t batch, uint64_t num_kb, int grid) {
+    int best = 256;
+    for (int bn : {192, 128, 64})
+        if (tile_cost(bn, tiles_m, N, batch, num_kb, grid) < 0.93 * tile_cost(best, tiles_m, N, batch, num_kb, grid)) best = bn;
+    return best;
+}
+
+bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, int fuse = 0, const void* bias = nullptr, void* D2 = nullptr) {
+    const void *A = c.A, *B = c.B;
+    const bool a_mn = c.a_mn, b_mn = c.b_mn;
+    const uint64_t M = c.m, N = c.n;
+    const uint64_t K = c.k;
+    uint64_t batch = c.batch;
+    if (!opt_in_shared_memory()) return false;
+    int grid = sm_count();
+    if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
+    const CUtensorMapDataType t16 = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    const CUtensorMapSwizzle sw = CU_TENSOR_MAP_SWIZZLE_128B;
+    CUtensorMap ma, mb, md;
+    if (g_two_cta.load(std::memory_order_relaxed) && grid >= 2 && !fuse && !c.a_pitch && !c.b_pitch && !c.d_plain)
+        if (launch_two_cta(is_bf16, c, D, where, grid)) return true;
+    TcParams p;
+    p.M = (int)M;
+    p.N = (int)N;
+    p.K = (int)K;
+    p.tiles_m = (int)((M + BM - 1) / BM);
+    p.num_kb = (int)((K + BK - 1) / BK);
+    p.split_kb = 0;
+    p.bn = N < 192 ? (int)((N + 63) / 64 * 64) : BN;
+    p.tiles_n = (int)((N + p.bn - 1) / p.bn);
+    p.b_keep = keep_b_ctas(p.tiles_m, p.tiles_n, p.num_kb, (int)batch, std::min(grid, (int)std::min<uint64_t>(batch * p.tiles_m * p.tiles_n, 1u << 30)));
+    // few output tiles: cut K into slices that run as the batches of this launch
+    int slices = 1;
+    const int bn_whole = p.b_keep ? p.bn : tile_columns((uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid);
+    if (batch == 1 && !fuse && !p.b_keep) {
+        slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
+        if (slices == 1)
+            slices = splitk_short((uint64_t)p.tiles_m * p.tiles_n, (uint64_t)p.num_kb, grid, kb_cost(p.bn),
+                                  tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid) - kSplitFixed16);
+    }
+    StreamWorkspace partial;
+    const uint64_t n_pitch = (N + 3) / 4 * 4;
+    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float))) slices = 1;
+    if (slices > 1) {
+        p.split_kb = (p.num_kb + slices - 1) / slices;
+        p.num_kb = p.split_kb;
+        batch = (uint64_t)slices;
+    } else if (!p.b_keep) {
+        p.bn = bn_whole;
+        p.tiles_n = (int)((N + p.bn - 1) / p.bn);
+    }
+    p.tiles_per_batch = p.tiles_m * p.tiles_n;
+    p.stages = ring_stages(p.bn);
+    p.stage_bytes = A_STAGE_BYTES + p.bn * BK * 2;
+    int tag = 0;
+    int* err = next_launch_error_word(&tag);
+    if (!err) return false;
+    const uint64_t a_bs = (uint64_t)c.a_bs, b_bs = (uint64_t)c.b_bs;
+    const bool oka = a_mn ? make_map_3d(&ma, t16, 2, A, K, M, c.batch, a_bs, 64, sw, c.a_pitch) : make_map_3d(&ma, t16, 2, A, M, K, c.batch, a_bs, BM, sw, c.a_pitch);
+    const bool okb = b_mn ? make_map_3d(&mb, t16, 2, B, K, N, c.batch, b_bs, 64, sw, c.b_pitch) : make_map_3d(&mb, t16, 2, B, N, K, c.batch, b_bs, (uint32_t)p.bn, sw, c.b_pitch);
+    if (!oka || !okb) return false;
+    p.d_plain = slices > 1 ? 0 : c.d_plain;
+    p.d = D;
+    if (slices > 1) {
+        if (!make_map_3d(&md, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, partial.ptr, M, N, batch, M * n_pitch, 32, sw, n_pitch)) return false;
+    } else if (p.d_plain) {
+        md = ma;  // not used
+    } else if (!make_map(&md, is_bf16, D, M, N, batch, M * N, 32)) {
+        return false;
+    }
     CUtensorMap md2 = md;
     if (fuse == 2 && !make_map(&md2, is_bf16, D2, M, N, batch, M * N, 32)) return false;
     p.fuse = fuse;
     p.bias = bias;
     p.group_m = g_group_m.load(std::memory_order_relaxed);
-    p.K = (int)K;
     p.num_tiles = (int)batch * p.tiles_per_batch;
-    p.a_batched = (batch > 1 && a_bs != 0) ? 1 : 0;
-    p.b_batched = (batch > 1 && b_bs != 0) ? 1 : 0;
-    p.num_kb = (int)((K + BK - 1) / BK);
+    p.a_batched = (c.batch > 1 && a_bs != 0) ? 1 : 0;
+    p.b_batched = (c.batch > 1 && b_bs != 0) ? 1 : 0;
     p.is_bf16 = is_bf16 ? 1 : 0;
-    p.out_f32 = partial ? 1 : 0;
+    p.out_f32 = slices > 1 ? 1 : 0;
     p.a_mn = a_mn ? 1 : 0;
     p.b_mn = b_mn ? 1 : 0;
     if (grid > p.num_tiles) grid = p.num_tiles;
-    p.b_keep = keep_b_ctas(p.tiles_m, p.tiles_n, p.num_kb, (int)batch, grid);
     if (p.b_keep) grid = p.b_keep * p.tiles_n;
-    tc_gemm_kernel<<<grid, TC_THREADS, TC_SMEM_BYTES, ctx().stream>>>(ma, mb, md, md2, p, err, tag);
+    const bool full = p.bn == BN;
+    const auto kernel = p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0>
+                                  : (fuse ? (full ? tc_gemm_kernel<TC_BIAS, BN> : tc_gemm_kernel<TC_BIAS, 0>) : (full ? tc_gemm_kernel<TC_STORE, BN> : tc_gemm_kernel<TC_STORE, 0>));
+    kernel<<<grid, TC_THREADS, TC_SMEM_BYTES, ctx().stream>>>(ma, mb, md, md2, p, err, tag);
     check_launch(where);
-    if (partial) splitk_reduce(is_bf16 ? 0 : 1, partial, slices, (size_t)(M * N), D, where);
+    if (slices > 1) splitk_reduce(is_bf16 ? 0 : 1, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
     return true;
 }
 
@@ -605,41 +741,142 @@ int splitk_slices(uint64_t tiles, uint64_t K, int block_k, int sms) {
     return best;
 }
 
-template <class T>
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, int slices, size_t n, T* __restrict__ out) {
-    const size_t nvec = n / 4, stride = (size_t)gridDim.x * 256;
+int splitk_short(uint64_t tiles, uint64_t num_kb, int sms, double kb_cost, double below) {
+    if (tiles == 0 || tiles * 2 > (uint64_t)sms) return 1;
+    int best = 1;
+    for (uint64_t s = 2; s * tiles <= (uint64_t)sms && s * 2 <= num_kb && s <= 32; s++) {
+        const uint64_t per = (num_kb + s - 1) / s;
+        if ((num_kb + per - 1) / per != s) continue;  // the last slices would be empty
+        const double cost = (double)per * kb_cost + 0.1 * (double)s;
+        if (cost < below) {
+            below = cost;
+            best = (int)s;
+        }
+    }
+    return best;
+}
+
+// `vec` elements per step: 4 when the output's rows are whole vectors (then rows and padded rows coincide), else 1.
+template <class T, int VEC>
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, int slices, size_t rows, uint32_t cols, uint32_t pitch, FastDiv div,
+                                                            T* __restrict__ out) {
+    const size_t nvec = rows * cols / VEC, stride = (size_t)gridDim.x * 256, slice = rows * pitch;
     for (size_t v = (size_t)blockIdx.x * 256 + threadIdx.x; v < nvec; v += stride) {
-        float4 acc = *reinterpret_cast<const float4*>(partial + 4 * v);
+        size_t src = VEC * v;
+        if constexpr (VEC == 1) {
+            const uint32_t r = div.div((uint32_t)v);
+            src = (size_t)r * pitch + ((uint32_t)v - r * cols);
+        }
+        float acc[VEC];
+        *reinterpret_cast<Vec<float, VEC>*>(acc) = *reinterpret_cast<const Vec<float, VEC>*>(partial + src);
         for (int s = 1; s < slices; s++) {
-            const float4 q = *reinterpret_cast<const float4*>(partial + (size_t)s * n + 4 * v);
-            acc.x += q.x;
-            acc.y += q.y;
-            acc.z += q.z;
-            acc.w += q.w;
+            const Vec<float, VEC> q = *reinterpret_cast<const Vec<float, VEC>*>(partial + (size_t)s * slice + src);
+#pragma unroll
+            for (int j = 0; j < VEC; j++) acc[j] += q.v[j];
         }
-        if constexpr (std::is_same<T, float>::value) {
-            *reinterpret_cast<float4*>(out + 4 * v) = acc;
-        } else {
-            Vec<T, 4> o;
-            o.v[0] = from_f32<T>(acc.x);
-            o.v[1] = from_f32<T>(acc.y);
-            o.v[2] = from_f32<T>(acc.z);
-            o.v[3] = from_f32<T>(acc.w);
-            *reinterpret_cast<Vec<T, 4>*>(out + 4 * v) = o;
+        Vec<T, VEC> o;
+#pragma unroll
+        for (int j = 0; j < VEC; j++) {
+            if constexpr (std::is_same<T, float>::value) o.v[j] = acc[j];
+            else o.v[j] = from_f32<T>(acc[j]);
         }
+        *reinterpret_cast<Vec<T, VEC>*>(out + VEC * v) = o;
     }
 }
 
-void splitk_reduce(int dtype, const float* partial, int slices, size_t n, void* out, const char* where) {
-    // n is a multiple of 4 here: the tensor-core path requires N to be a multiple of 16 bytes' worth of elements
-    size_t blocks = (n / 4 + 255) / 256;
+template <class T>
+static void splitk_reduce_t(const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out) {
+    const bool vec = cols == pitch && reinterpret_cast<uintptr_t>(out) % (4 * sizeof(T)) == 0;
+    size_t blocks = (rows * cols / (vec ? 4 : 1) + 255) / 256;
     const size_t cap = (size_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    if (dtype == 0) splitk_reduce_kernel<bf16><<<(unsigned)blocks, 256, 0, ctx().stream>>>(partial, slices, n, static_cast<bf16*>(out));
-    else if (dtype == 1) splitk_reduce_kernel<f16><<<(unsigned)blocks, 256, 0, ctx().stream>>>(partial, slices, n, static_cast<f16*>(out));
-    else splitk_reduce_kernel<float><<<(unsigned)blocks, 256, 0, ctx().stream>>>(partial, slices, n, static_cast<float*>(out));
+    const FastDiv div((uint32_t)cols);
+    if (vec) splitk_reduce_kernel<T, 4><<<(unsigned)blocks, 256, 0, ctx().stream>>>(partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out));
+    else splitk_reduce_kernel<T, 1><<<(unsigned)blocks, 256, 0, ctx().stream>>>(partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out));
+}
+
+void splitk_reduce(int dtype, const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out, const char* where) {
+    if (dtype == 0) splitk_reduce_t<bf16>(partial, slices, rows, cols, pitch, out);
+    else if (dtype == 1) splitk_reduce_t<f16>(partial, slices, rows, cols, pitch, out);
+    else splitk_reduce_t<float>(partial, slices, rows, cols, pitch, out);
     check_launch(where);
+}
+
+// Rows of `cols` elements, dense and starting anywhere, copied to rows of `pitch` elements (a multiple of 128 bytes): one
+// 16-byte vector of a destination row per thread and step, assembled from the one or two aligned 16-byte words of the
+// source it straddles.  The words read all hold at least one element of the vector, so nothing outside the aligned words
+// of the source's own elements is touched.  Bound by HBM (or L2): reads and writes the operand once.
+template <class W>
+__global__ void __launch_bounds__(256) repack_rows_kernel(const W* __restrict__ in, W* __restrict__ out, uint32_t vecs, FastDiv per_row, uint32_t cols, uint32_t pitch) {
+    constexpr uint32_t VEC = 16 / sizeof(W);
+    const uint32_t stride = gridDim.x * 256;
+    for (uint32_t v = blockIdx.x * 256 + threadIdx.x; v < vecs; v += stride) {
+        uint32_t row, c;
+        per_row.divmod(v, row, c);
+        c *= VEC;
+        const uint32_t need = min(VEC, cols - c) * (uint32_t)sizeof(W);
+        const uintptr_t src = reinterpret_cast<uintptr_t>(in + (size_t)row * cols + c);
+        const uint32_t sh = (uint32_t)(src & 15);
+        const uint4* words = reinterpret_cast<const uint4*>(src - sh);
+        const uint4 lo = words[0];
+        uint4 hi = make_uint4(0, 0, 0, 0);
+        if (sh + need > 16) hi = words[1];
+        uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        uint4 r;
+        const uint32_t bits = (sh & 3) * 8;
+#pragma unroll
+        for (int k = 0; k < 2; k++)  // word-wise shift by sh / 4 in two steps with compile-time indices
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if ((sh >> 2) & (2 >> k)) w[i] = i + (2 >> k) < 8 ? w[i + (2 >> k)] : 0;
+        r.x = __funnelshift_r(w[0], w[1], bits);
+        r.y = __funnelshift_r(w[1], w[2], bits);
+        r.z = __funnelshift_r(w[2], w[3], bits);
+        r.w = __funnelshift_r(w[3], w[4], bits);
+        *reinterpret_cast<uint4*>(out + (size_t)row * pitch + c) = r;
+    }
+}
+
+static bool repack_rows(size_t es, const void* in, void* out, uint64_t rows, uint64_t cols, uint64_t pitch) {
+    const uint64_t per_row = (cols * es + 15) / 16, vecs = rows * per_row;  // the padding itself is never read
+    uint64_t blocks = (vecs + 255) / 256;
+    const uint64_t cap = (uint64_t)sm_count() * 32;
+    if (blocks > cap) blocks = cap;
+    const FastDiv div((uint32_t)per_row);
+    if (es == 2)
+        repack_rows_kernel<uint16_t><<<(unsigned)blocks, 256, 0, ctx().stream>>>(static_cast<const uint16_t*>(in), static_cast<uint16_t*>(out), (uint32_t)vecs, div, (uint32_t)cols,
+                                                                                 (uint32_t)pitch);
+    else
+        repack_rows_kernel<uint32_t><<<(unsigned)blocks, 256, 0, ctx().stream>>>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), (uint32_t)vecs, div, (uint32_t)cols,
+                                                                                 (uint32_t)pitch);
+    return true;
+}
+
+bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* where) {
+    if (!c.a_repack && !c.b_repack) return true;
+    // rows of whole 128-byte lines: a tensor copy's 128-byte box rows then read one line each, not parts of two
+    const uint64_t q = 128 / es;
+    const uint64_t a_rows = (c.a_mn ? c.k : c.m) * (c.a_bs ? c.batch : 1), a_cols = c.a_mn ? c.m : c.k, a_pitch = (a_cols + q - 1) / q * q;
+    const uint64_t b_rows = (c.b_mn ? c.k : c.n) * (c.b_bs ? c.batch : 1), b_cols = c.b_mn ? c.n : c.k, b_pitch = (b_cols + q - 1) / q * q;
+    const uint64_t a_bytes = c.a_repack ? (a_rows * a_pitch * es + 255) / 256 * 256 : 0, b_bytes = c.b_repack ? b_rows * b_pitch * es : 0;
+    if (a_bytes / 16 > 0x7FFFFFFFull || b_bytes / 16 > 0x7FFFFFFFull) return false;  // the copy counts vectors in 32 bits
+    if (!ws.take(a_bytes + b_bytes)) return false;
+    if (c.a_repack) {
+        repack_rows(es, c.A, ws.ptr, a_rows, a_cols, a_pitch);
+        c.A = static_cast<const char*>(ws.ptr);
+        c.a_pitch = a_pitch;
+        if (c.a_bs) c.a_bs = (int64_t)((c.a_mn ? c.k : c.m) * a_pitch);
+    }
+    if (c.b_repack) {
+        char* dst = static_cast<char*>(ws.ptr) + a_bytes;
+        repack_rows(es, c.B, dst, b_rows, b_cols, b_pitch);
+        c.B = dst;
+        c.b_pitch = b_pitch;
+        if (c.b_bs) c.b_bs = (int64_t)((c.b_mn ? c.k : c.n) * b_pitch);
+    }
+    check_launch(where);
+    return true;
 }
 
 namespace {
@@ -723,30 +960,54 @@ extern "C" int mx_debug_tc_gemm_poke_status(int value) {
 
 namespace mx {
 
+// Sizes the tensor-core kernels can index and are worth a persistent launch for.
+static bool in_range(uint64_t M, uint64_t N, uint64_t K, uint64_t batch) {
+    if (M == 0 || N == 0 || K == 0) return false;
+    if (M > 0x7FFFFFFFull || N > 0x7FFFFFFFull || K > 0x7FFFFFFFull) return false;
+    if (batch > 0x7FFFull) return false;
+    if (batch * M * N * K < (1ull << 24)) return false;  // small problems are not worth a persistent launch
+    return batch * ((M + 127) / 128) * ((N + 63) / 64) <= 0x3FFFFFFFull;
+}
 // TMA wants 16-byte aligned bases and row pitches: the contiguous extent of every matrix (K for K-major
 // operands, MN for MN-major ones, N for D) must be a multiple of 16 / elem_size elements.
 static bool eligible(size_t es, uint64_t M, uint64_t N, uint64_t K, uint64_t batch, bool a_mn, bool b_mn, const void* a, const void* b, const void* d) {
     const uint64_t q = 16 / es;
-    if (M == 0 || N == 0 || K == 0) return false;
+    if (!in_range(M, N, K, batch)) return false;
     if (N % q != 0) return false;
     if ((a_mn ? M : K) % q != 0 || (b_mn ? N : K) % q != 0) return false;
     if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)d) % 16 != 0) return false;
-    if (M > 0x7FFFFFFFull || N > 0x7FFFFFFFull || K > 0x7FFFFFFFull) return false;
     if (batch > 1 && (M * N) % q != 0) return false;  // every batch's output starts on a 16-byte boundary
-    if (batch * M * N * K < (1ull << 24)) return false;  // small problems are not worth a persistent launch
-    if (batch * ((M + 127) / 128) * ((N + 127) / 128) > 0x3FFFFFFFull) return false;
+    return true;
+}
+// What a product of dense operands needs before the kernels can take it: an operand whose rows (or base) are not
+// 16-byte multiples is copied to padded rows first (repack_operands), an output like that is written by the epilogue warps
+// without tensor stores.  One pass over the operand against 8 TFLOP/s on the CUDA cores: bf16 4099 x 1543 x 1000, whose
+// 1543-wide matrices all need it, takes 20-40 us a product (1804 us on the CUDA cores).
+static bool plan_ragged(size_t es, TcProduct& c, const void* d) {
+    const uint64_t q = 16 / es;
+    if (!in_range(c.m, c.n, c.k, c.batch)) return false;
+    if (((uintptr_t)c.A | (uintptr_t)c.B | (uintptr_t)d) % es != 0) return false;
+    const uint64_t a_cols = c.a_mn ? c.m : c.k, b_cols = c.b_mn ? c.n : c.k;
+    c.a_repack = a_cols % q != 0 || (uintptr_t)c.A % 16 != 0;
+    c.b_repack = b_cols % q != 0 || (uintptr_t)c.B % 16 != 0;
+    if (c.batch > 1) {
+        // the batches of a copied operand must lie one after the other; an uncopied one's batch stride is a tensor-map stride
+        if (c.a_bs != 0 && c.a_bs != (int64_t)(c.m * c.k)) return false;
+        if (c.b_bs != 0 && c.b_bs != (int64_t)(c.k * c.n)) return false;
+    }
+    c.ragged = true;
+    const bool plain = c.n % q != 0 || (uintptr_t)d % 16 != 0;
+    c.d_plain = !plain ? 0 : (c.n % 2 == 0 && (uintptr_t)d % 4 == 0 ? 2 : 1);
     return true;
 }
 
 // Forward product C[m, n] = sum_k A[m, k] * B[k, n]: can it run on a tensor-core kernel, and with which operand
 // majors?  Unbatched, every operand either dense row-major or the transposed view of a dense matrix.
-static bool classify_forward(const MmDesc& d, size_t es, size_t num_els, const void* x, const void* y, const void* out, TcProduct& c) {
+static bool forward_operands(const MmDesc& d, size_t es, size_t num_els, const void* x, const void* y, TcProduct& c) {
     if (d.out_nd < 2 || d.a_nd < 2 || d.b_nd < 2) return false;
     const uint64_t m = d.m, n = d.n, k = d.k_fwd;
-    if (m == 0 || n == 0 || num_els % (m * n) != 0) return false;
+    if (m == 0 || n == 0 || k == 0 || num_els % (m * n) != 0) return false;
     const uint64_t batch = num_els / (m * n);
-    // batched: rank-3 operands only (for higher ranks the reference indexes the batch through strides[0] alone)
-    if (batch > 1 && !(d.out_nd == 3 && d.a_nd == 3 && d.b_nd == 3)) return false;
     if (batch > 0x7FFFull) return false;
     c.A = static_cast<const char*>(x) + d.a_off * es;
     c.B = static_cast<const char*>(y) + d.b_off * es;
@@ -759,7 +1020,11 @@ static bool classify_forward(const MmDesc& d, size_t es, size_t num_els, const v
         b_mnmajor = true;
         c.a_bs = (int64_t)(m * k);
         c.b_bs = (int64_t)(k * n);
+        // ranks other than three: every leading dim folds into the batch, as long as both operands have all of it
+        if (batch > 1 && !(d.out_nd == 3 && d.a_nd == 3 && d.b_nd == 3) && (d.a_elems != batch * m * k || d.b_elems != batch * k * n)) return false;
     } else {
+        // batched: rank-3 operands only (for higher ranks the reference indexes the batch through strides[0] alone)
+        if (batch > 1 && !(d.out_nd == 3 && d.a_nd == 3 && d.b_nd == 3)) return false;
         // strided branch: A[b * as0 + m * as1 + k * as2], B[b * bs0 + k * bs1 + n * bs2]
         a_kmajor = d.a_strides[2] == 1 && d.a_strides[1] == (int64_t)k;
         a_mnmajor = d.a_strides[1] == 1 && d.a_strides[2] == (int64_t)m;  // transposed view of a dense [k, m] matrix
@@ -769,19 +1034,51 @@ static bool classify_forward(const MmDesc& d, size_t es, size_t num_els, const v
         c.b_bs = batch > 1 ? d.b_strides[0] : 0;
     }
     if (!(a_kmajor || a_mnmajor) || !(b_kmajor || b_mnmajor)) return false;
-    if (batch > 1) {
-        // a batch stride is a TMA stride: a multiple of 16 bytes, and whole matrices apart (no overlap tricks)
-        const int64_t q = (int64_t)(16 / es);
-        if (c.a_bs < 0 || c.b_bs < 0 || c.a_bs % q != 0 || c.b_bs % q != 0) return false;
-        if ((c.a_bs != 0 && c.a_bs < (int64_t)(m * k)) || (c.b_bs != 0 && c.b_bs < (int64_t)(k * n))) return false;
-    }
+    // batches are whole matrices apart (no overlap tricks)
+    if (batch > 1 && (c.a_bs < 0 || c.b_bs < 0 || (c.a_bs != 0 && c.a_bs < (int64_t)(m * k)) || (c.b_bs != 0 && c.b_bs < (int64_t)(k * n)))) return false;
     c.a_mn = !a_kmajor;
     c.b_mn = !b_kmajor;
     c.m = m;
     c.n = n;
     c.k = k;
     c.batch = batch;
-    return eligible(es, m, n, k, batch, c.a_mn, c.b_mn, c.A, c.B, out);
+    return true;
+}
+
+static bool backward_operands(const MmDesc& d, int which, size_t nea, size_t neb, const void* x, const void* y, TcProduct& c) {
+    const uint64_t m = d.m, n = d.n, k = d.k_bwd;
+    if (d.out_nd < 2 || m == 0 || n == 0 || k == 0 || d.g_size % (m * n) != 0) return false;
+    // both gradients have every batch of g (an operand broadcast over the batch has fewer elements): dense batched products
+    const uint64_t batch = d.g_size / (m * n);
+    if (batch > 0x7FFFull || nea != batch * m * k || neb != batch * k * n) return false;
+    c.batch = batch;
+    const int64_t g_bs = batch > 1 ? (int64_t)(m * n) : 0, a_bs = batch > 1 ? (int64_t)(m * k) : 0, b_bs = batch > 1 ? (int64_t)(k * n) : 0;
+    if (which == 1) {
+        c.A = static_cast<const char*>(x);
+        c.B = static_cast<const char*>(y);
+        c.a_bs = g_bs;
+        c.b_bs = b_bs;
+        c.a_mn = c.b_mn = false;
+        c.m = m;
+        c.n = k;
+        c.k = n;
+    } else {
+        c.A = static_cast<const char*>(y);
+        c.B = static_cast<const char*>(x);
+        c.a_bs = a_bs;
+        c.b_bs = g_bs;
+        c.a_mn = c.b_mn = true;
+        c.m = k;
+        c.n = n;
+        c.k = m;
+    }
+    return true;
+}
+
+// The batch strides of operands that tensor maps reach in place are multiples of 16 bytes.
+static bool aligned_batches(size_t es, const TcProduct& c) {
+    const int64_t q = (int64_t)(16 / es);
+    return c.batch <= 1 || (c.a_bs % q == 0 && c.b_bs % q == 0);
 }
 
 // which = 0: forward (x = A base, y = B base).  1: grad_a[m, k] = sum_n g[m, n] * B[k, n] (x = g, y = B + offset),
@@ -790,28 +1087,23 @@ static bool classify_forward(const MmDesc& d, size_t es, size_t num_els, const v
 // (strides ignored, crates/maidenx_cpu/src/ops/matmul.rs:196-261).
 bool tc_classify(const MmDesc& d, int which, size_t es, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, const void* out,
                  TcProduct& c) {
-    if (which == 0) return classify_forward(d, es, num_els, x, y, out, c);
-    if (d.out_nd != 2) return false;
-    const uint64_t m = d.m, n = d.n, k = d.k_bwd;
-    if (d.g_size != m * n || nea != m * k || neb != k * n) return false;
-    c.batch = 1;
-    c.a_bs = c.b_bs = 0;
-    if (which == 1) {
-        c.A = static_cast<const char*>(x);
-        c.B = static_cast<const char*>(y);
-        c.a_mn = c.b_mn = false;
-        c.m = m;
-        c.n = k;
-        c.k = n;
-    } else {
-        c.A = static_cast<const char*>(y);
-        c.B = static_cast<const char*>(x);
-        c.a_mn = c.b_mn = true;
-        c.m = k;
-        c.n = n;
-        c.k = m;
+    if (which == 0) {
+        if (d.out_nd > 3 && num_els > d.m * d.n) return false;
+        if (!forward_operands(d, es, num_els, x, y, c)) return false;
+    } else if (d.out_nd != 2 || !backward_operands(d, which, nea, neb, x, y, c)) {
+        return false;
     }
-    return eligible(es, c.m, c.n, c.k, 1, c.a_mn, c.b_mn, c.A, c.B, out);
+    return aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out);
+}
+
+bool tc_classify_any(const MmDesc& d, int which, size_t es, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, const void* out,
+                     TcProduct& c) {
+    if (which == 0 ? !forward_operands(d, es, num_els, x, y, c) : !backward_operands(d, which, nea, neb, x, y, c)) return false;
+    c.ragged = d.out_nd > (which == 0 ? 3 : 2);  // aligned, but new to these kernels: batches beyond rank 3, batched backward
+    if (aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out)) return true;
+    // the copy reads whole operands: every batch must be there (a size-1 batch dim passes the contiguity test)
+    if (which == 0 && c.batch > 1 && d.a_cont && d.b_cont && (d.a_elems != c.batch * c.m * c.k || d.b_elems != c.batch * c.k * c.n)) return false;
+    return plan_ragged(es, c, out);
 }
 
 // x [rows, in] . w[out, in]^T with the bias add (and GELU) in the epilogue; false = shape not taken (the caller runs the ops one by one)
@@ -845,15 +1137,18 @@ bool tc_batched_row_bias(bool is_bf16, uint64_t batch, uint64_t rows, uint64_t k
     c.batch = batch;
     c.a_bs = 0;
     c.b_bs = (int64_t)(k * n);
-    if (!bias || !out || batch == 0 || batch > 0x7FFFull || !eligible(2, c.m, c.n, c.k, batch, false, true, w, cols, out)) return false;
-    return launch_gemm(is_bf16, c, out, where, 3, bias, nullptr);
+    if (!bias || !out || batch == 0 || batch > 0x7FFFull) return false;
+    if (!eligible(2, c.m, c.n, c.k, batch, false, true, w, cols, out) && !plan_ragged(2, c, out)) return false;
+    StreamWorkspace ws;
+    return repack_operands(2, c, ws, where) && launch_gemm(is_bf16, c, out, where, 3, bias, nullptr);
 }
 
 bool tc_gemm_bf16_f16(bool is_bf16, const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out,
                       const char* where) {
     TcProduct c;
-    if (!tc_classify(d, which, 2, num_els, nea, neb, x, y, out, c)) return false;
-    return launch_gemm(is_bf16, c, out, where);
+    if (!tc_classify_any(d, which, 2, num_els, nea, neb, x, y, out, c)) return false;
+    StreamWorkspace ws;
+    return repack_operands(2, c, ws, where) && launch_gemm(is_bf16, c, out, where);
 }
 
 }  // namespace mx

@@ -13,18 +13,20 @@
 // Two-level accumulation.  The tensor core adds each instruction's products into the f32 accumulator with
 // truncation, which pulls a long running sum towards zero by about half an ulp per instruction (measured:
 // -6e-6 relative after 147 instructions); over K = 8192 that would eat the whole 1e-4 budget.  So the TMEM
-// accumulator only ever holds the sum of CHUNK_KB k-blocks (128 values of K, 48 instructions): the epilogue warps
-// drain it after every chunk and keep the running total in registers, added with round-to-nearest, while the tensor
-// core fills the other accumulator.  The pull towards zero is then bounded by the chunk length (about -2e-6 of the
-// result) whatever K is.
+// accumulator only ever holds the sum of a few k-blocks: the epilogue warps drain it after every chunk and keep the
+// running total in registers, added with round-to-nearest, while the tensor core fills the other accumulator.  The pull
+// towards zero is then bounded by the chunk length whatever K is.  Two lengths: CHUNK_FAST k-blocks (128 values of K, error
+// 1e-6 of the result), and one k-block (2.2e-7) for the ragged products, which the CUDA cores computed before
+// with 2e-7 to 6e-7; a drain per k-block no longer hides behind the tensor work (conv products [256 x 1152] . [1152 x 196]: 40 us
+// with the long chunk, 58 with the short one).  In a chunk of one the eight products with a small factor come first, so that they are summed while the accumulator is still 2^-11 of the result; longer chunks interleave them.
 //
 // One persistent CTA per SM, 320 threads in four roles:
 //   warp 0      TMA producer: raw f32 A [128 x 32] and B [BN x 32] k-blocks (128-byte swizzle rows of 32 floats)
-//               into a ring of STAGES stages;
+//               into a ring of stages;
 //   warps 6-9   splitter: when a stage has landed, read the raw tiles and write the `small` tiles beside them
 //               (element-wise, so the swizzled placement carries over unchanged), then hand the stage to
-//   warp 1      the MMA issuer: 4 k-steps x 3 tcgen05.mma (M128, N = BN, K8) per k-block into one of two TMEM
-//               accumulators, switching accumulator every CHUNK_KB k-blocks; commits the stage back to the
+//   warp 1      the MMA issuer: 4 k-steps x 3 tcgen05.mma (M128, N up to BN, K8) per k-block into one of two TMEM
+//               accumulators, switching accumulator every chunk_kb k-blocks; commits the stage back to the
 //               producer and each finished chunk to
 //   warps 2-5   the epilogue: per chunk tcgen05.ld of the warp's 32 rows x BN columns, added into BN registers per
 //               thread; after the tile's last chunk the totals go through a swizzled 4 KB staging tile to TMA stores.
@@ -46,22 +48,21 @@ namespace {
 
 constexpr int BM = 128, BN = 128, BK = 32;     // CTA tile; BK * 4 bytes = one 128-byte swizzle row
 constexpr int UMMA_K = 8;                      // tf32: 32 bytes of K per instruction
-constexpr int STAGES = 3;
+constexpr int STAGES = 3, MAX_STAGES = 4;      // of 128- and of 64-column tiles
 constexpr int A_TILE = BM * BK * 4;            // 16 KB
 constexpr int B_TILE = BN * BK * 4;
-constexpr int RAW_BYTES = A_TILE + B_TILE;     // what TMA delivers per stage
-constexpr int STAGE_BYTES = 2 * RAW_BYTES;     // [A raw | B raw | A small | B small]
+constexpr int STAGE_BYTES = 2 * (A_TILE + B_TILE);  // [A raw | B raw | A small | B small] of a 128-column tile
 constexpr int EPI_WARPS = 4, SPLIT_WARPS = 4;
 constexpr int EPI_CHUNK_COLS = 32;             // 32 f32 = 128 bytes per staged row
 constexpr int EPI_STAGE_BYTES = 32 * EPI_CHUNK_COLS * 4;  // 4 KB per warp per buffer
 constexpr int THREADS = 32 * (2 + EPI_WARPS + SPLIT_WARPS);
 constexpr int TMEM_COLS = 2 * BN;              // two f32 accumulators
 constexpr int GROUP_M = 16;
-constexpr int CHUNK_KB = 4;                    // k-blocks summed inside TMEM before the registers take over
+constexpr int CHUNK_FAST = 4;
 constexpr int MN_CHUNK_BYTES = BK * 128;       // one [32 K-rows x 32 MN-elements] box
 
 static_assert(TMEM_COLS == 256 || TMEM_COLS == 512, "TMEM allocations are powers of two");
-static_assert(RAW_BYTES % (16 * 32 * SPLIT_WARPS) == 0, "the splitter moves 16 bytes per thread and step");
+static_assert(A_TILE % (16 * 32 * SPLIT_WARPS) == 0 && B_TILE / 2 % (16 * 32 * SPLIT_WARPS) == 0, "the splitter moves 16 bytes per thread and step");
 
 struct Smem {
     static constexpr int stages = 0;
@@ -72,14 +73,14 @@ struct Smem {
 constexpr int SMEM_BYTES = Smem::total + 1024;  // slack for the 1024-byte alignment
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 
-__host__ __device__ constexpr uint32_t make_idesc_tf32(bool a_mn_major, bool b_mn_major) {
+__host__ __device__ constexpr uint32_t make_idesc_tf32(bool a_mn_major, bool b_mn_major, int bn) {
     uint32_t d = 0;
     d |= 1u << 4;                               // D format: f32
     d |= 2u << 7;                               // A format: tf32
     d |= 2u << 10;                              // B format: tf32
     d |= (a_mn_major ? 1u : 0u) << 15;
     d |= (b_mn_major ? 1u : 0u) << 16;
-    d |= (uint32_t)(BN >> 3) << 17;
+    d |= (uint32_t)(bn >> 3) << 17;
     d |= (uint32_t)(BM >> 4) << 24;
     return d;
 }
@@ -89,6 +90,14 @@ struct Params {
     int tiles_per_batch;       // tiles_m * tiles_n; num_tiles = batch * tiles_per_batch
     int a_batched, b_batched;  // 0: the operand is one matrix shared by every batch (third TMA coordinate stays 0)
     int a_mn, b_mn;
+    int M, N;
+    int chunk_kb;   // k-blocks summed inside TMEM before the registers take over
+    int bn;         // columns of an output tile: 64 or 128
+    int stages;     // of the ring
+    int raw_bytes;  // what TMA delivers per stage: A and bn rows of B
+    int split_kb;   // > 0: split-K; batch s of the launch reduces the k-blocks [s * split_kb, (s + 1) * split_kb) of one product
+    int d_plain;    // != 0: the output's rows (or base) are not 16-byte multiples: the epilogue warps write them to `d` themselves
+    float* d;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, const Params& p, int& tm, int& tn, int& tb) {
@@ -120,18 +129,18 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)tcf_smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t smem_base = smem_u32(smem);
     const uint32_t bar_base = smem_base + Smem::bars;
-    // barrier slots (8 bytes each): full[STAGES], split[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2]; then the TMEM base word
+    // barrier slots (8 bytes each): full[MAX_STAGES], split[MAX_STAGES], empty[MAX_STAGES], tmem_full[2], tmem_empty[2]; then the TMEM base word
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
-    auto split_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
-    auto empty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + s); };
-    auto tfull_bar = [&](int a) { return bar_base + 8u * (3 * STAGES + a); };
-    auto tempty_bar = [&](int a) { return bar_base + 8u * (3 * STAGES + 2 + a); };
-    volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(smem + Smem::bars + 8 * (3 * STAGES + 4));
+    auto split_bar = [&](int s) { return bar_base + 8u * (MAX_STAGES + s); };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (2 * MAX_STAGES + s); };
+    auto tfull_bar = [&](int a) { return bar_base + 8u * (3 * MAX_STAGES + a); };
+    auto tempty_bar = [&](int a) { return bar_base + 8u * (3 * MAX_STAGES + 2 + a); };
+    volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(smem + Smem::bars + 8 * (3 * MAX_STAGES + 4));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) {
+        for (int s = 0; s < MAX_STAGES; s++) {
             mbar_init(full_bar(s), 1);
             mbar_init(split_bar(s), SPLIT_WARPS);
             mbar_init(empty_bar(s), 1);
@@ -161,27 +170,27 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 int tm, tn, tb;
                 tile_coords(tile, p, tm, tn, tb);
                 const int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
+                const int k_base = tb * p.split_kb * BK;  // a k-block past the end of K is all fill: zeros
                 for (int kb = 0; kb < p.num_kb; kb++) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, err, tag, 1)) {
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(full_bar(stage), RAW_BYTES);
-                    const uint32_t sa = smem_base + Smem::stages + stage * STAGE_BYTES;
+                    mbar_expect_tx(full_bar(stage), p.raw_bytes);
+                    const uint32_t sa = smem_base + Smem::stages + stage * 2 * p.raw_bytes;
                     const uint32_t sb = sa + A_TILE;
                     if (!p.a_mn) {
-                        tma_load_3d(sa, &map_a, kb * BK, tm * BM, za, full_bar(stage));
+                        tma_load_3d(sa, &map_a, k_base + kb * BK, tm * BM, za, full_bar(stage));
                     } else {
 #pragma unroll
-                        for (int h = 0; h < BM / 32; h++) tma_load_3d(sa + h * MN_CHUNK_BYTES, &map_a, tm * BM + h * 32, kb * BK, za, full_bar(stage));
+                        for (int h = 0; h < BM / 32; h++) tma_load_3d(sa + h * MN_CHUNK_BYTES, &map_a, tm * BM + h * 32, k_base + kb * BK, za, full_bar(stage));
                     }
                     if (!p.b_mn) {
-                        tma_load_3d(sb, &map_b, kb * BK, tn * BN, zb, full_bar(stage));
+                        tma_load_3d(sb, &map_b, k_base + kb * BK, tn * p.bn, zb, full_bar(stage));
                     } else {
-#pragma unroll
-                        for (int h = 0; h < BN / 32; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * BN + h * 32, kb * BK, zb, full_bar(stage));
+                        for (int h = 0; h < p.bn / 32; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * p.bn + h * 32, k_base + kb * BK, zb, full_bar(stage));
                     }
-                    if (++stage == STAGES) {
+                    if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1;
                     }
@@ -191,21 +200,21 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (lane == 0) {
-            const uint32_t idesc = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0);
+            const uint32_t idesc = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, p.bn);
             // K-major: 8 floats further along the 128-byte row; MN-major: the next group of eight K-rows
             const uint64_t a_kstep = p.a_mn ? (1024 >> 4) : (32 >> 4), b_kstep = p.b_mn ? (1024 >> 4) : (32 >> 4);
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
-                for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += CHUNK_KB) {
+                for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += p.chunk_kb) {
                     if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1, err, tag, 2)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
-                    const int kb1 = min(kb0 + CHUNK_KB, p.num_kb);
+                    const int kb1 = min(kb0 + p.chunk_kb, p.num_kb);
                     for (int kb = kb0; kb < kb1; kb++) {
                         // the raw tiles (TMA) and the small tiles (splitter) are both operands
                         if (!mbar_wait(full_bar(stage), phase, err, tag, 3) || !mbar_wait(split_bar(stage), phase, err, tag, 6)) {
@@ -213,23 +222,33 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             break;
                         }
                         tc_fence_after();
-                        const uint32_t s0 = smem_base + Smem::stages + stage * STAGE_BYTES;
+                        const uint32_t s0 = smem_base + Smem::stages + stage * 2 * p.raw_bytes;
                         // K-major: rows of 32 floats, groups of eight rows 1024 bytes apart.  MN-major: 32-byte-atom swizzle,
                         // groups of four K-rows 512 bytes apart, 128-byte-wide MN chunks one box (4 KB) apart.
                         const uint64_t a_big = p.a_mn ? smem_desc_sw128_atom32(s0, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0, 16, 1024);
                         const uint64_t b_big = p.b_mn ? smem_desc_sw128_atom32(s0 + A_TILE, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + A_TILE, 16, 1024);
                         const uint64_t a_small =
-                            p.a_mn ? smem_desc_sw128_atom32(s0 + RAW_BYTES, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + RAW_BYTES, 16, 1024);
-                        const uint64_t b_small = p.b_mn ? smem_desc_sw128_atom32(s0 + RAW_BYTES + A_TILE, MN_CHUNK_BYTES, 512)
-                                                        : smem_desc_sw128(s0 + RAW_BYTES + A_TILE, 16, 1024);
+                            p.a_mn ? smem_desc_sw128_atom32(s0 + p.raw_bytes, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + p.raw_bytes, 16, 1024);
+                        const uint64_t b_small = p.b_mn ? smem_desc_sw128_atom32(s0 + p.raw_bytes + A_TILE, MN_CHUNK_BYTES, 512)
+                                                        : smem_desc_sw128(s0 + p.raw_bytes + A_TILE, 16, 1024);
+                        if (p.chunk_kb == 1) {
 #pragma unroll
-                        for (int k = 0; k < BK / UMMA_K; k++) {
-                            umma_tf32(d_tmem, a_small + a_kstep * k, b_big + b_kstep * k, idesc, (kb != kb0) || (k != 0));
-                            umma_tf32(d_tmem, a_big + a_kstep * k, b_small + b_kstep * k, idesc, 1);
-                            umma_tf32(d_tmem, a_big + a_kstep * k, b_big + b_kstep * k, idesc, 1);
+                            for (int k = 0; k < BK / UMMA_K; k++) {
+                                umma_tf32(d_tmem, a_small + a_kstep * k, b_big + b_kstep * k, idesc, k != 0);
+                                umma_tf32(d_tmem, a_big + a_kstep * k, b_small + b_kstep * k, idesc, 1);
+                            }
+#pragma unroll
+                            for (int k = 0; k < BK / UMMA_K; k++) umma_tf32(d_tmem, a_big + a_kstep * k, b_big + b_kstep * k, idesc, 1);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < BK / UMMA_K; k++) {
+                                umma_tf32(d_tmem, a_small + a_kstep * k, b_big + b_kstep * k, idesc, (kb != kb0) || (k != 0));
+                                umma_tf32(d_tmem, a_big + a_kstep * k, b_small + b_kstep * k, idesc, 1);
+                                umma_tf32(d_tmem, a_big + a_kstep * k, b_big + b_kstep * k, idesc, 1);
+                            }
                         }
                         umma_commit(empty_bar(stage));
-                        if (++stage == STAGES) {
+                        if (++stage == p.stages) {
                             stage = 0;
                             phase ^= 1;
                         }
@@ -257,9 +276,9 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             float total[BN];  // this thread's row of the tile (registers: every index below is a compile-time constant)
 #pragma unroll
             for (int j = 0; j < BN; j++) total[j] = 0.0f;
-            for (int kb0 = 0; kb0 < p.num_kb; kb0 += CHUNK_KB) {
+            for (int kb0 = 0; kb0 < p.num_kb; kb0 += p.chunk_kb) {
                 // the TMEM loads below are warp-collective: leave the loops only as a whole warp
-                const bool ready = mbar_wait_relaxed(tfull_bar(acc), acc_phase, err, tag, 4, 200);
+                const bool ready = mbar_wait_relaxed(tfull_bar(acc), acc_phase, err, tag, 4, p.chunk_kb == 1 ? 20 : 200);
                 if (!__all_sync(0xFFFFFFFFu, ready)) {
                     ok = false;
                     break;
@@ -268,6 +287,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
 #pragma unroll
                 for (int c = 0; c < BN / 32; c++) {
+                    if (c * 32 >= p.bn) break;
                     uint32_t v[32];
                     tmem_ld_32x32b_x32(t_row + c * 32, v);
                     tmem_ld_wait();
@@ -286,6 +306,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if (!ok) break;
 #pragma unroll
             for (int c = 0; c < BN / EPI_CHUNK_COLS; c++) {
+                if (c * EPI_CHUNK_COLS >= p.bn) break;
                 // the staging buffer must have been read by its previous TMA store
                 if (lane == 0) tma_store_wait_read<1>();
                 __syncwarp();
@@ -296,8 +317,20 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         make_float4(total[c * 32 + 4 * j], total[c * 32 + 4 * j + 1], total[c * 32 + 4 * j + 2], total[c * 32 + 4 * j + 3]);
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) {
-                    tma_store_3d(&map_d, smem_u32(stage_buf + buf * EPI_STAGE_BYTES), tn * BN + c * EPI_CHUNK_COLS, tm * BM + quarter * 32, tb);
+                const int row0 = tm * BM + quarter * 32, col0 = tn * p.bn + c * EPI_CHUNK_COLS;
+                unsigned char* src = stage_buf + buf * EPI_STAGE_BYTES;
+                if (p.d_plain) {
+                    float* out = p.d + ((size_t)tb * p.M + row0) * p.N + col0 + lane;
+                    for (int r0 = 0; r0 < 32; r0 += 8) {
+                        float v[8];
+#pragma unroll
+                        for (int r = 0; r < 8; r++) v[r] = *reinterpret_cast<const float*>(src + (r0 + r) * 128 + (((lane >> 2) ^ r) << 4) + (lane & 3) * 4);
+#pragma unroll
+                        for (int r = 0; r < 8; r++)
+                            if (row0 + r0 + r < p.M && col0 + lane < p.N) out[(size_t)(r0 + r) * p.N] = v[r];
+                    }
+                } else if (lane == 0) {
+                    tma_store_3d(&map_d, smem_u32(src), col0, row0, tb);
                     tma_store_commit();
                 }
                 buf ^= 1;
@@ -317,18 +350,21 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     ok = false;
                     break;
                 }
-                const uint4* raw = reinterpret_cast<const uint4*>(smem + Smem::stages + stage * STAGE_BYTES);
-                uint4* small = reinterpret_cast<uint4*>(smem + Smem::stages + stage * STAGE_BYTES + RAW_BYTES);
-                constexpr int STEPS = RAW_BYTES / 16 / (32 * SPLIT_WARPS);
-#pragma unroll 8
-                for (int i = 0; i < STEPS; i++) {
-                    const uint4 q = raw[t + i * 32 * SPLIT_WARPS];
-                    small[t + i * 32 * SPLIT_WARPS] = make_uint4(small_part(q.x), small_part(q.y), small_part(q.z), small_part(q.w));
+                const uint4* raw = reinterpret_cast<const uint4*>(smem + Smem::stages + stage * 2 * p.raw_bytes);
+                uint4* small = reinterpret_cast<uint4*>(smem + Smem::stages + stage * 2 * p.raw_bytes + p.raw_bytes);
+                const int steps = p.raw_bytes / 16 / (32 * SPLIT_WARPS);
+                for (int i0 = 0; i0 < steps; i0 += 4) {  // 12 or 16 steps; loads first: the compiler cannot tell the two tiles apart
+                    uint4 q[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) q[i] = raw[t + (i0 + i) * 32 * SPLIT_WARPS];
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        small[t + (i0 + i) * 32 * SPLIT_WARPS] = make_uint4(small_part(q[i].x), small_part(q[i].y), small_part(q[i].z), small_part(q[i].w));
                 }
                 fence_proxy_async_smem();  // the tensor core reads these through the async proxy
                 __syncwarp();
                 if (lane == 0) mbar_arrive(split_bar(stage));
-                if (++stage == STAGES) {
+                if (++stage == p.stages) {
                     stage = 0;
                     phase ^= 1;
                 }
@@ -375,51 +411,79 @@ bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, 
                        mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, pitch);
 }
 
-// D[M,N] = sum_k Aop[m,k] * Bop[n,k]; K-major operand = dense row-major [MN, K], MN-major = dense row-major [K, MN].
+// Columns of an output tile: 64 where 128-wide tiles would be half empty (N <= 64) or leave SMs without a tile; a 64-wide
+// tile costs three quarters of a 128-wide one (shared-memory traffic of A and B together bounds both).
+double tile_cost(int bn, uint64_t tiles_m, uint64_t N, uint64_t batch, int grid) {
+    const uint64_t tiles = tiles_m * ((N + bn - 1) / bn) * batch, waves = (tiles + grid - 1) / grid;
+    return (double)waves * (128 + bn) / 256.0;
+}
+int tile_columns(uint64_t tiles_m, uint64_t N, uint64_t batch, int grid) {
+    return tile_cost(64, tiles_m, N, batch, grid) < 0.93 * tile_cost(128, tiles_m, N, batch, grid) ? 64 : 128;
+}
+// what the second launch of a split-K product costs, in k-blocks (about 0.9 us each on one CTA)
+constexpr double kSplitFixed32 = 3.0;
+
+// D[M,N] = sum_k Aop[m,k] * Bop[n,k]; K-major operand = row-major [MN, K], MN-major = row-major [K, MN].
 bool launch(const TcProduct& c, void* D, const char* where) {
-    const void *A = c.A, *B = c.B;
     const bool a_mn = c.a_mn, b_mn = c.b_mn;
-    const uint64_t M = c.m, N = c.n;
-    uint64_t K = c.k, batch = c.batch;
+    const uint64_t M = c.m, N = c.n, K = c.k;
+    uint64_t batch = c.batch;
     if (!opt_in_shared_memory()) return false;
     Params p;
+    p.M = (int)M;
+    p.N = (int)N;
+    p.chunk_kb = c.ragged ? 1 : CHUNK_FAST;
+    p.bn = N <= 64 ? 64 : BN;
     p.tiles_m = (int)((M + BM - 1) / BM);
-    p.tiles_n = (int)((N + BN - 1) / BN);
-    p.tiles_per_batch = p.tiles_m * p.tiles_n;
+    p.tiles_n = (int)((N + p.bn - 1) / p.bn);
+    p.num_kb = (int)((K + BK - 1) / BK);
+    p.split_kb = 0;
     int grid = sm_count();
     if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
-    // few output tiles, long reduction: cut K into slices that run as the batches of this launch (see tc_ptx.cuh)
-    const int slices = batch == 1 ? splitk_slices((uint64_t)p.tiles_per_batch, K, BK, grid) : 1;
-    float* partial = nullptr;
-    uint64_t a_bs = (uint64_t)c.a_bs, b_bs = (uint64_t)c.b_bs, a_pitch = 0, b_pitch = 0;
-    if (slices > 1) {
-        partial = static_cast<float*>(scratch((size_t)slices * M * N * sizeof(float)));
-        if (!partial) return false;
-        const uint64_t Ks = K / slices;
-        a_pitch = a_mn ? M : K;
-        b_pitch = b_mn ? N : K;
-        a_bs = a_mn ? Ks * M : Ks;
-        b_bs = b_mn ? Ks * N : Ks;
-        K = Ks;
-        batch = (uint64_t)slices;
+    // few output tiles: cut K into slices that run as the batches of this launch (see tc_ptx.cuh)
+    int slices = 1;
+    const int bn_whole = tile_columns((uint64_t)p.tiles_m, N, batch, grid);
+    if (batch == 1) {
+        slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
+        if (slices == 1)
+            slices = splitk_short((uint64_t)p.tiles_m * p.tiles_n, (uint64_t)p.num_kb, grid, (128 + p.bn) / 256.0,
+                                  tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, grid) * p.num_kb - kSplitFixed32);
     }
+    StreamWorkspace partial;
+    const uint64_t n_pitch = (N + 3) / 4 * 4;
+    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float))) slices = 1;
+    if (slices > 1) {
+        p.split_kb = (p.num_kb + slices - 1) / slices;
+        p.num_kb = p.split_kb;
+        batch = (uint64_t)slices;
+    } else {
+        p.bn = bn_whole;
+        p.tiles_n = (int)((N + p.bn - 1) / p.bn);
+    }
+    p.tiles_per_batch = p.tiles_m * p.tiles_n;
+    p.raw_bytes = A_TILE + p.bn * BK * 4;
+    p.stages = STAGES * STAGE_BYTES / (2 * p.raw_bytes);
     int tag = 0;
     int* err = next_launch_error_word(&tag);
     if (!err) return false;
     CUtensorMap ma, mb, md;
-    const bool oka = a_mn ? make_map(&ma, A, K, M, batch, a_bs, BK, true, a_pitch) : make_map(&ma, A, M, K, batch, a_bs, BM, false, a_pitch);
-    const bool okb = b_mn ? make_map(&mb, B, K, N, batch, b_bs, BK, true, b_pitch) : make_map(&mb, B, N, K, batch, b_bs, BN, false, b_pitch);
-    if (!oka || !okb || !make_map(&md, partial ? static_cast<void*>(partial) : D, M, N, batch, M * N, 32)) return false;
+    const uint64_t a_bs = (uint64_t)c.a_bs, b_bs = (uint64_t)c.b_bs;
+    const bool oka = a_mn ? make_map(&ma, c.A, K, M, c.batch, a_bs, BK, true, c.a_pitch) : make_map(&ma, c.A, M, K, c.batch, a_bs, BM, false, c.a_pitch);
+    const bool okb = b_mn ? make_map(&mb, c.B, K, N, c.batch, b_bs, BK, true, c.b_pitch) : make_map(&mb, c.B, N, K, c.batch, b_bs, (uint32_t)p.bn, false, c.b_pitch);
+    if (!oka || !okb) return false;
+    p.d_plain = slices > 1 ? 0 : c.d_plain;
+    p.d = static_cast<float*>(D);
+    if (p.d_plain) md = ma;  // not used
+    else if (slices > 1 ? !make_map(&md, partial.ptr, M, N, batch, M * n_pitch, 32, false, n_pitch) : !make_map(&md, D, M, N, batch, M * N, 32)) return false;
     p.num_tiles = (int)batch * p.tiles_per_batch;
-    p.a_batched = (batch > 1 && a_bs != 0) ? 1 : 0;
-    p.b_batched = (batch > 1 && b_bs != 0) ? 1 : 0;
-    p.num_kb = (int)((K + BK - 1) / BK);
+    p.a_batched = (c.batch > 1 && a_bs != 0) ? 1 : 0;
+    p.b_batched = (c.batch > 1 && b_bs != 0) ? 1 : 0;
     p.a_mn = a_mn ? 1 : 0;
     p.b_mn = b_mn ? 1 : 0;
     if (grid > p.num_tiles) grid = p.num_tiles;
     tc_gemm_f32_kernel<<<grid, THREADS, SMEM_BYTES, ctx().stream>>>(ma, mb, md, p, err, tag);
     check_launch(where);
-    if (partial) splitk_reduce(2, partial, slices, (size_t)(M * N), D, where);
+    if (slices > 1) splitk_reduce(2, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
     return true;
 }
 
@@ -427,8 +491,9 @@ bool launch(const TcProduct& c, void* D, const char* where) {
 
 bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out, const char* where) {
     TcProduct c;
-    if (!tc_classify(d, which, 4, num_els, nea, neb, x, y, out, c)) return false;
-    return launch(c, out, where);
+    if (!tc_classify_any(d, which, 4, num_els, nea, neb, x, y, out, c)) return false;
+    StreamWorkspace ws;
+    return repack_operands(4, c, ws, where) && launch(c, out, where);
 }
 
 }  // namespace mx

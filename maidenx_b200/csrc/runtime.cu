@@ -173,6 +173,57 @@ void* scratch(size_t bytes) {
     return s.ptr;
 }
 
+// One pool per device.  Up to kWorkspaceKeep bytes that no call holds stay with the pool across synchronisations (a freed
+// block is otherwise unmapped at the next one and mapped again by the next call); what a large call took beyond that goes back,
+// and all of it when cuda_malloc runs out of memory.
+constexpr uint64_t kWorkspaceKeep = 512ull << 20;
+static std::mutex g_workspace_mutex;
+static cudaMemPool_t g_workspace_pools[64] = {nullptr};
+static cudaMemPool_t workspace_pool(int dev) {
+    cudaMemPool_t* const pools = g_workspace_pools;
+    std::lock_guard<std::mutex> lk(g_workspace_mutex);
+    if (!pools[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        uint64_t keep = kWorkspaceKeep;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools[dev] = pool;
+    }
+    return pools[dev];
+}
+
+// Hands back what the current device's pool holds and no call uses; false: it has no pool.
+static bool workspace_trim() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    std::lock_guard<std::mutex> lk(g_workspace_mutex);
+    return g_workspace_pools[dev] && cudaDeviceSynchronize() == cudaSuccess && cudaMemPoolTrimTo(g_workspace_pools[dev], 0) == cudaSuccess;
+}
+
+bool StreamWorkspace::take(size_t bytes) {
+    stream = ctx().stream;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    if (ptr || cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone || cudaGetDevice(&dev) != cudaSuccess ||
+        dev < 0 || dev >= 64 || !(pool = workspace_pool(dev)) || cudaMallocFromPoolAsync(&ptr, bytes ? bytes : 1, pool, stream) != cudaSuccess) {
+        cudaGetLastError();
+        ptr = nullptr;
+        return false;
+    }
+    return true;
+}
+StreamWorkspace::~StreamWorkspace() {
+    if (ptr && cudaFreeAsync(ptr, stream) != cudaSuccess) cudaGetLastError();
+}
+
 static void side_table_forget(const void* p, size_t bytes) {
     std::lock_guard<std::mutex> lk(g_meta_mutex);
     forget_range_locked(p, bytes);
@@ -356,7 +407,12 @@ int cuda_malloc(void** ptr, size_t size) {
             return (int)cudaSuccess;
         }
     }
-    return (int)cudaMalloc(ptr, size);
+    cudaError_t e = cudaMalloc(ptr, size);
+    if (e == cudaErrorMemoryAllocation && workspace_trim()) {
+        cudaGetLastError();
+        e = cudaMalloc(ptr, size);
+    }
+    return (int)e;
 }
 
 int cuda_free(void* ptr) {

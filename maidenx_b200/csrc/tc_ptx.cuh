@@ -227,8 +227,11 @@ bool make_map_3d(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes, con
 // range of a K-major operand, a row range of an MN-major one), the f32 partial results [slices, M, N] go to scratch and
 // splitk_reduce adds them up and rounds once.  Returns 1 when splitting does not pay.
 int splitk_slices(uint64_t tiles, uint64_t K, int block_k, int sms);
-// out[i] = round(sum_s partial[s * n + i]); dtype: 0 bf16, 1 f16, 2 f32.
-void splitk_reduce(int dtype, const float* partial, int slices, size_t n, void* out, const char* where);
+// The same for reductions of a few k-blocks (any K): s equal runs of k-blocks, the last one shorter, when one run
+// (k-blocks * kb_cost) comes out below `below`, the cost of the unsplit product less that of the second launch.
+int splitk_short(uint64_t tiles, uint64_t num_kb, int sms, double kb_cost, double below);
+// out[r * cols + c] = round(sum_s partial[(s * rows + r) * pitch + c]); dtype: 0 bf16, 1 f16, 2 f32.  pitch: cols rounded up to 4.
+void splitk_reduce(int dtype, const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out, const char* where);
 
 // The error word of the calling thread's current device (allocated on first use) and the tag of the launch about
 // to be made.  Returns nullptr when there is no usable device.
@@ -236,5 +239,12 @@ int* next_launch_error_word(int* tag);
 // The same word and a fresh tag as a WaitReport, for the staged elementwise / conv kernels (codes 21..23).
 WaitReport next_wait_report();
 
+}  // namespace tc
+
+struct TcProduct;
+namespace tc {
+// Copies the operands a product marks for it into `ws` and points the product at the copies.  false: no workspace to be had
+// (nothing launched); the caller falls back to the CUDA-core kernel.
+bool repack_operands(size_t elem_size, TcProduct& c, StreamWorkspace& ws, const char* where);
 }  // namespace tc
 }  // namespace mx

@@ -350,3 +350,78 @@ def test_short_reductions_with_the_b_panel_resident(oracle, cuda, dt, case):
     finally:
         lib.mx_debug_set_gemm_keep_b(1)
     assert np.array_equal(kept, general)
+
+
+# ---------------------------------------------------------------------------------------
+# Products whose matrices are not 16-byte multiples: operands copied to padded rows, output rows
+# written without tensor stores; and the plain tensor-core products that have more than one batch
+# dim or are a batched backward.  Bounds: 16-bit results carry one rounding (2^-9 bf16, 2^-11 f16) of an f32 sum;
+# f32 the split-tf32 bound of the aligned cases above.
+# ---------------------------------------------------------------------------------------
+RAGGED = [
+    # name, batch dims, M, N, K, a_major, b_major, a_off, b_off
+    ("nt-odd", [], 257, 515, 129, "k", "k", 0, 0),
+    ("nn-odd", [], 259, 517, 131, "k", "mn", 0, 0),
+    ("tn-odd", [], 261, 519, 127, "mn", "mn", 0, 0),
+    ("tt-odd", [], 263, 521, 133, "mn", "k", 0, 0),
+    ("n-odd", [], 200, 301, 392, "k", "k", 0, 0),             # aligned operands, only the output's rows are ragged
+    ("n-even", [], 136, 518, 320, "k", "mn", 0, 0),           # 16-bit rows start on 4 bytes: stores in pairs
+    ("k-odd", [], 264, 256, 393, "k", "mn", 0, 0),            # only one operand is copied
+    ("offsets", [], 264, 256, 384, "k", "mn", 1, 3),          # regular sizes behind unaligned bases
+    ("one-row", [], 1, 4099, 4099, "k", "mn", 0, 0),
+    ("narrow", [], 4099, 5, 1001, "k", "k", 0, 0),            # N below one 64-column tile
+    ("long-k", [], 33, 65, 9001, "mn", "mn", 0, 0),           # split along K into runs of k-blocks, the last one short
+    ("short-split", [], 130, 264, 1032, "k", "k", 0, 0),      # the same on aligned operands, K below the long-reduction plan
+    ("batched-odd", [5], 150, 197, 121, "k", "mn", 0, 0),
+    ("rank-4", [2, 3], 200, 264, 72, "k", "mn", 0, 0),        # every leading dim is a batch
+    ("rank-4-odd", [2, 3], 200, 197, 75, "k", "mn", 0, 0),
+    ("wide-batch", [3], 128, 192, 256, "k", "mn", 0, 0),      # 192-column tiles
+]
+
+
+@pytest.mark.parametrize("dt", [D.BF16, D.F16, D.F32], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", RAGGED, ids=lambda c: c[0])
+def test_products_with_ragged_rows(oracle, cuda, dt, case):
+    from oracle import binding
+    name, bd, m, n, k, amaj, bmaj, aoff, boff = case
+    rng = np.random.default_rng(zlib_seed(name + dt.name))
+    cs = H.contiguous_strides
+    nb = H.numel(bd) if bd else 1
+    a_sh, b_sh, o = [*bd, m, k], [*bd, k, n], [*bd, m, n]
+    ast = cs(a_sh) if amaj == "k" else [1, m]
+    bst = cs(b_sh) if bmaj == "mn" else [1, k]
+    a = H.random_store(rng, dt, nb * m * k + aoff, dist="normal")
+    b = H.random_store(rng, dt, nb * k * n + boff, dist="normal")
+    meta = H.matmul_metadata(o, a_sh, b_sh, ast, bst, aoff, boff)
+    got = H.run_matmul(cuda, dt, meta, nb * m * n, a, b)
+    binding.set_wide(True)
+    try:
+        ref = H.run_matmul(oracle, dt, meta, nb * m * n, a, b)
+    finally:
+        binding.set_wide(False)
+    H.assert_same("matmul", dt, got, ref, float_rel=1e-5 if dt.name == "f32" else 1e-2, what=name, scale=np.sqrt(k))
+
+
+@pytest.mark.parametrize("dt", [D.BF16, D.F16, D.F32], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [("batched", [4], 152, 136, 216), ("batched-odd", [4], 151, 133, 219), ("rank-4", [2, 2], 152, 136, 216), ("odd", [], 301, 259, 227),
+                                  ("broadcast-b", None, 150, 136, 216)], ids=lambda c: c[0])
+def test_batched_and_ragged_backward(oracle, cuda, dt, case):
+    from oracle import binding
+    name, bd, m, n, k = case
+    rng = np.random.default_rng(zlib_seed("bwd" + name + dt.name))
+    cs = H.contiguous_strides
+    shared = bd is None     # B is one matrix for a batch of four: not a batched product, the reference's index rules apply
+    bd = [4] if shared else bd
+    nb = H.numel(bd) if bd else 1
+    a_sh, b_sh, o = [*bd, m, k], [k, n] if shared else [*bd, k, n], [*bd, m, n]
+    nea, neb = H.numel(a_sh), H.numel(b_sh)
+    a, b, g = (H.random_store(rng, dt, x, dist="normal") for x in (nea, neb, nb * m * n))
+    meta = H.matmul_metadata(o, a_sh, b_sh, cs(a_sh), cs(b_sh), 0, 0)
+    got = H.run_matmul_backward(cuda, dt, meta, nea, neb, g, a, b)
+    binding.set_wide(True)
+    try:
+        ref = H.run_matmul_backward(oracle, dt, meta, nea, neb, g, a, b)
+    finally:
+        binding.set_wide(False)
+    for key in ref:
+        H.assert_same("matmul_backward", dt, got[key], ref[key], float_rel=1e-5 if dt.name == "f32" else 1e-2, what=f"{name}/{key}", scale=np.sqrt(n if key == "ga" else m))
