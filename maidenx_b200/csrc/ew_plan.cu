@@ -305,6 +305,39 @@ void ew_fill_tile_params(const EwPlan& pl, int tile, EwTileParams& P, uint32_t& 
     blocks = (uint32_t)(nb * P.tiles_p * P.tiles_q);
 }
 
+bool ew_fill_dense_params(const EwPlan& pl, size_t in_size, size_t out_size, const void* out, const void* a, const void* b, EwDenseParams& P) {
+    const int vec = (int)(16 / in_size);
+    if (pl.n == 0 || pl.n > 0x7FFFFFFFull - vec || pl.nd < 1 || !aligned_to(out, 0, out_size, vec * out_size)) return false;
+    int64_t acc = 1, span[3] = {0, 0, 0};
+    bool flat[3] = {true, true, true};
+    for (int d = pl.nd - 1; d >= 0; d--) {
+        if (pl.st[0][d] != acc) return false;
+        for (int k = 1; k < 3; k++) {
+            if (pl.st[k][d] != acc) flat[k] = false;
+            const int64_t s = pl.st[k][d] < 0 ? -pl.st[k][d] : pl.st[k][d];
+            if (s > 0x3FFFFFFF || (span[k] += s * (int64_t)pl.dim[d]) > 0x3FFFFFFF) {
+                if (k <= pl.nin && !flat[k]) return false;
+                span[k] = 0;  // a flat operand's offsets are below n
+            }
+        }
+        acc *= pl.dim[d];
+    }
+    const void* ptr[3] = {out, a, b};
+    for (int k = 1; k < 3; k++) {
+        if (flat[k]) P.kind[k] = aligned_to(ptr[k], 0, in_size, 16) ? EWD_VECTOR : EWD_ELEMENT;
+        else P.kind[k] = pl.st[k][pl.nd - 1] == 0 ? EWD_CONST : EWD_STEP;
+    }
+    P.nd = pl.nd;
+    P.n = (uint32_t)pl.n;
+    P.q = pl.dim[pl.nd - 1];
+    P.q_div.init(P.q);
+    for (int d = 0; d < pl.nd; d++) {
+        P.div[d].init(pl.dim[d]);
+        for (int k = 0; k < 3; k++) P.st[k][d] = (int)pl.st[k][d];
+    }
+    return true;
+}
+
 void ew_fill_gen_params(const EwPlan& pl, EwGenParams& P) {
     P.nd = pl.nd;
     P.n = pl.n;

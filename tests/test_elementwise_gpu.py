@@ -431,3 +431,41 @@ def test_wait_report_of_a_staged_kernel_is_surfaced_by_the_next_copy(oracle, cud
         lib.mx_clear_error()
         for x in bufs:
             x.free()
+
+
+def gathered_layouts():
+    """Dense outputs whose rows are no whole vectors: (name, dims, lhs_strides, rhs_strides, lhs_off, rhs_off, lhs_len, rhs_len)"""
+    cs = H.contiguous_strides
+    out = []
+    for name, dims in (("row-odd", [37, 45]), ("row-long-odd", [9, 1027]), ("row-short", [301, 3]), ("row-7", [90, 7])):
+        n = H.numel(dims)
+        out.append((name + "/rhs-row", dims, cs(dims), [0, 1], 0, 0, n, dims[1]))
+        out.append((name + "/rhs-col", dims, cs(dims), [1, 0], 0, 0, n, dims[0]))
+        out.append((name + "/lhs-col", dims, [1, 0], cs(dims), 0, 0, dims[0], n))
+        out.append((name + "/both-bcast", dims, [1, 0], [0, 1], 0, 0, dims[0], dims[1]))
+        out.append((name + "/unaligned-flat", dims, cs(dims), [0, 1], 1, 2, n + 1, dims[1] + 2))
+    for hw in (3, 7):  # per-channel operands of feature maps
+        dims = [5, 11, hw, hw]
+        out.append((f"channel-{hw}", dims, cs(dims), [0, 1, 0, 0], 0, 0, H.numel(dims), 11))
+    out.append(("permuted", [5, 6, 7], [1, 35, 5], [42, 7, 1], 0, 0, 210, 210))
+    out.append(("every-second", [41, 13], [26, 2], [13, 1], 0, 0, 41 * 26, 41 * 13))
+    out.append(("one-dim-strided", [1001], [3], [1], 0, 0, 3003, 1001))
+    return out
+
+
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16, D.F64, D.I32, D.U8], ids=lambda d: d.name)
+def test_dense_outputs_with_gathered_operands(oracle, cuda, dt):
+    rng = np.random.default_rng(zlib.crc32(b"gathered" + dt.name.encode()))
+    for name, dims, ls, rs, lo, ro, ll, rl in gathered_layouts():
+        lhs, rhs = H.full_range_store(rng, dt, ll), H.full_range_store(rng, dt, rl)
+        for op in ("add", "div", "lt"):  # packed, checked-quotient and one-byte-output forms
+            ref = H.run_binary(oracle, op, dt, dims, ls, rs, lo, ro, lhs, rhs)
+            got = H.run_binary(cuda, op, dt, dims, ls, rs, lo, ro, lhs, rhs)
+            H.assert_same(op, dt, got, ref, what=name)
+        if ls == H.contiguous_strides(dims):
+            ref = H.run_binary_inplace(oracle, "mul_inplace", dt, dims, ls, rs, lo, ro, lhs, rhs)
+            got = H.run_binary_inplace(cuda, "mul_inplace", dt, dims, ls, rs, lo, ro, lhs, rhs)
+            H.assert_same("mul_inplace", dt, got, ref, what=name)
+        ref = H.run_unary(oracle, "square", dt, dims, rs, ro, rhs)
+        got = H.run_unary(cuda, "square", dt, dims, rs, ro, rhs)
+        H.assert_same("square", dt, got, ref, what=name)
