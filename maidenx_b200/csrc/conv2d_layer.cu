@@ -68,6 +68,7 @@ struct Ops {
     void (*add)(size_t, size_t, const size_t*, const void*, const void*, void*);
     void (*add_inplace)(size_t, size_t, const size_t*, void*, const void*);
     void (*sum)(size_t, size_t, size_t, const size_t*, const void*, void*);
+    void (*sum_to_shape)(size_t, size_t, const size_t*, const void*, void*);
     void (*contiguous)(size_t, size_t, const size_t*, const void*, void*);
     int half_kind;  // 1 bf16, 2 f16, 0 anything else
 };
@@ -76,6 +77,7 @@ struct Ops {
         reinterpret_cast<decltype(mx::Ops::im2col)>(cuda_conv2d_im2col_##T), reinterpret_cast<decltype(mx::Ops::col2im)>(cuda_conv2d_col2im_##T), \
             reinterpret_cast<decltype(mx::Ops::matmul)>(cuda_matmul_##T), reinterpret_cast<decltype(mx::Ops::add)>(cuda_add_##T),                 \
             reinterpret_cast<decltype(mx::Ops::add_inplace)>(cuda_add_inplace_##T), reinterpret_cast<decltype(mx::Ops::sum)>(cuda_sum_##T),        \
+            reinterpret_cast<decltype(mx::Ops::sum_to_shape)>(cuda_sum_to_shape_##T),                                                     \
             reinterpret_cast<decltype(mx::Ops::contiguous)>(mx_contiguous_##T), mx::half_kind_of<mx_##T>()                                       \
     }
 
@@ -219,7 +221,13 @@ void backward(const Ops& ops, size_t es, const MxConv2d* c, int mode, const void
         const size_t d3[3] = {g.B, g.Co, g.K};
         sum_dim(ops, d3, 3, 0, gw_batch, grad_w);
     }
-    if (grad_bias) bias_gradient(ops, g, es, grad_out, sums, grad_bias);
+    if (grad_bias && es >= 4) {
+        // the bias is broadcast over [B, Co, P]: one fold to [1, Co, 1] (16-bit types keep the roundings of the three sums)
+        const size_t fm[10] = {g.B, g.Co, g.P, g.Co * g.P, g.P, 1, 1, g.Co, 1, 0};
+        ops.sum_to_shape(g.B * g.Co * g.P, 3, fm, grad_out, grad_bias);
+    } else if (grad_bias) {
+        bias_gradient(ops, g, es, grad_out, sums, grad_bias);
+    }
 }
 
 }  // namespace

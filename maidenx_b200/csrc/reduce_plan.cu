@@ -120,6 +120,7 @@ void red_plan_shape(RedPlan& pl, size_t n, size_t nd, const size_t* hm) {
             return;
         }
     const bool cont = contiguous(nd, idims, ist);
+    bool outer = false;
     if (n != 0 && cont && in == n) {
         // classify dims: keep (out == in) / reduce (out == 1); size-1 dims are neutral
         bool simple = true;
@@ -178,13 +179,19 @@ void red_plan_shape(RedPlan& pl, size_t n, size_t nd, const size_t* hm) {
                 pl.I = sizes[2];
                 return;
             }
+            if (m == 3) {  // [R, K, R]
+                outer = true;
+                pl.R = sizes[0];
+                pl.O = sizes[1];
+                pl.I = sizes[2];
+            }
         }
     }
     if (nd > (size_t)kRedMaxDims) {
         pl.kind = RP_ERROR;
         return;
     }
-    RedGenParams& g = pl.gen;
+    RedGenParams& g = pl.gen;  // filled for the outer form too: extents beyond its 32-bit counts take the scatter
     g.mode = 1;
     g.n = n;
     g.nd = (int)nd;
@@ -195,13 +202,13 @@ void red_plan_shape(RedPlan& pl, size_t n, size_t nd, const size_t* hm) {
         g.out_dims[d] = odims[d];
     }
     g.off = pl.off;
-    pl.kind = RP_GENERIC;
+    pl.kind = outer ? RP_OUTER : RP_GENERIC;
 }
 
 }  // namespace mx
 
 // Host-only view of the reduction planner (see mx_debug_elementwise_plan): returns the RedPlanKind
-// (0 empty, 1 rows, 2 cols, 3 generic scatter, 4 error) and the recognised [O, R, I] structure.
+// (0 empty, 1 rows, 2 cols, 3 generic scatter, 4 error, 5 outer) and the recognised [O, R, I] structure.
 // sum_to_shape != 0 reads metadata as [in_dims | in_strides | out_dims | offset] and ignores num_red_dims.
 extern "C" int mx_debug_reduce_plan(size_t num_els, size_t num_dims, size_t num_red_dims, const size_t* host_metadata, int sum_to_shape,
                                     size_t* outer, size_t* reduced, size_t* inner) {

@@ -13,6 +13,8 @@
 // split reductions write per-block partials to scratch and a second launch folds them:
 // the classic two-pass grid reduce.  Every path is atomic-free, so results are
 // deterministic, and the output is overwritten (no pre-zero contract).
+//   outer   (sum_to_shape of [Q, O, I] to [1, O, 1]: the gradient of a per-channel operand) one of the two above down to
+//           wide partials, [O, I] sums over Q or [Q, O] sums over I, and a second launch that folds those.
 // Accumulation: bf16/f16 in f32 with one final rounding, f32 in f32, f64 in f64, integers
 // wrapping in 32/64 bits (truncation to the element width commutes with wrapping adds).
 // Anything else (several reduced dims, non-contiguous input, partial sum_to_shape
@@ -347,6 +349,27 @@ __global__ void __launch_bounds__(kColLanes* kColRows) reduce_cols_kernel(const 
     }
 }
 
+// Second pass of an "outer" reduction: out[o] = fold of partial[o * so + i * si + j], i < ni, j < nj.  G = 32: a warp per
+// output; G = kRedThreads: a block per output.
+template <class T, int KIND, int G>
+__global__ void __launch_bounds__(kRedThreads) reduce_outer_fold_kernel(const typename RedTraits<T, KIND>::Acc* __restrict__ partial, T* out, u64 count, u64 so, u32 ni,
+                                                                      u64 si, u32 nj, FastDiv nj_div, u64 factor) {
+    typedef RedTraits<T, KIND> TR;
+    const u64 o = (u64)blockIdx.x * (kRedThreads / G) + threadIdx.x / G;
+    if (G == 32 && o >= count) return;
+    const u32 t = threadIdx.x % G, total = ni * nj;
+    typename TR::Acc acc = TR::init();
+#pragma unroll 4
+    for (u32 e = t; e < total; e += G) {
+        u32 i, j;
+        nj_div.divmod(e, i, j);
+        acc = TR::combine(acc, partial[o * so + i * si + j]);
+    }
+    if constexpr (G == 32) acc = warp_reduce<TR>(acc);
+    else acc = block_reduce<TR, kRedThreads>(acc);
+    if (t == 0) out[o] = TR::finalize(acc, factor);
+}
+
 // ---------------------------------------------------------------------------------
 // generic scatter path (literal index formulas, wide atomics into scratch)
 // ---------------------------------------------------------------------------------
@@ -459,11 +482,11 @@ __global__ void __launch_bounds__(kRedThreads) reduce_scatter_kernel(const T* in
 // ---------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------
-enum RedPlanKind { RP_EMPTY = 0, RP_ROWS, RP_COLS, RP_GENERIC, RP_ERROR };
+enum RedPlanKind { RP_EMPTY = 0, RP_ROWS, RP_COLS, RP_GENERIC, RP_ERROR, RP_OUTER };
 
 struct RedPlan {
     int kind;
-    u64 O, R, I;      // rows: O rows of R; cols: [O, R, I]
+    u64 O, R, I;      // rows: O rows of R; cols: [O, R, I]; outer: [R, O, I] -> [O]
     u64 out_count;
     u64 factor;       // elements folded into each output (mean divisor)
     u64 off;
@@ -576,6 +599,53 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
         }
         check_launch(where);
         return;
+    }
+    if (pl.kind == RP_OUTER) {
+        const u64 O = pl.O, R = pl.R, I = pl.I;
+        const int occ = 8;
+        // Long inner runs fold first (one row per (r, o), coalesced, a single value left of each); short ones fold last, so
+        // that the first pass walks down R over whole rows of O * I neighbouring elements.  The line: below 1024 elements a
+        // block has less than one trip per row; above it the O * I wide partials would be written and read for nothing.
+        if (I >= 1024 && R * O <= 65535 && R * 512 <= 0x7FFFFFFFull) {
+            const u64 rows = R * O, unit = (u64)kRedThreads * VEC * 4;
+            u64 splits = split_count(rows, (u64)sms * occ), max_splits = (I + unit - 1) / unit;
+            if (splits > max_splits) splits = max_splits;
+            u64 seg = (I + splits - 1) / splits;
+            seg = (seg + VEC - 1) / VEC * VEC;
+            splits = (I + seg - 1) / seg;
+            const u32 pitch = splits < 2 ? 2 : (u32)splits;  // two or more "splits" make the kernel leave its partials
+            Acc* part = static_cast<Acc*>(scratch(sizeof(Acc) * rows * pitch));
+            if (!part) return;
+            dim3 grid((u32)splits, (u32)rows);
+            if (base_aligned && I % VEC == 0) reduce_rows_block_kernel<T, KIND, VEC><<<grid, kRedThreads, 0, s>>>(in, out, part, I, seg, pitch, pl.factor, nullptr, 0);
+            else reduce_rows_block_kernel<T, KIND, 1><<<grid, kRedThreads, 0, s>>>(in, out, part, I, seg, pitch, pl.factor, nullptr, 0);
+            check_launch(where);
+            reduce_outer_fold_kernel<T, KIND, 32><<<(u32)((O + 7) / 8), kRedThreads, 0, s>>>(part, out, O, pitch, (u32)R, O * pitch, (u32)splits, FastDiv((u32)splits), pl.factor);
+            check_launch(where);
+            return;
+        }
+        const u64 cols = O * I;
+        const bool vec = base_aligned && cols % VEC == 0;
+        const int v = vec ? VEC : 1;
+        const u64 gx = (cols + (u64)kColLanes * v - 1) / ((u64)kColLanes * v);
+        u64 splits = split_count(gx, (u64)sms * occ), max_splits = (R + 63) / 64;
+        if (splits > max_splits) splits = max_splits;
+        u64 seg = (R + splits - 1) / splits;
+        splits = (R + seg - 1) / seg;
+        if (splits * I <= 0x7FFFFFFFull && gx <= 0x7FFFFFFFull && splits <= 65535) {
+            Acc* part = static_cast<Acc*>(scratch(sizeof(Acc) * splits * cols));
+            if (!part) return;
+            dim3 grid((u32)gx, (u32)splits, 1);
+            const u32 leave = splits < 2 ? 2 : (u32)splits;
+            if (vec) reduce_cols_kernel<T, KIND, VEC><<<grid, kColLanes * kColRows, 0, s>>>(in, out, part, 1, R, cols, seg, leave, pl.factor, nullptr);
+            else reduce_cols_kernel<T, KIND, 1><<<grid, kColLanes * kColRows, 0, s>>>(in, out, part, 1, R, cols, seg, leave, pl.factor, nullptr);
+            check_launch(where);
+            const FastDiv div((u32)I);
+            if (splits * I <= 2048) reduce_outer_fold_kernel<T, KIND, 32><<<(u32)((O + 7) / 8), kRedThreads, 0, s>>>(part, out, O, I, (u32)splits, cols, (u32)I, div, pl.factor);
+            else reduce_outer_fold_kernel<T, KIND, kRedThreads><<<(u32)O, kRedThreads, 0, s>>>(part, out, O, I, (u32)splits, cols, (u32)I, div, pl.factor);
+            check_launch(where);
+            return;
+        }
     }
     // generic scatter
     Acc* ws = static_cast<Acc*>(scratch(sizeof(Acc) * (pl.out_count ? pl.out_count : 1)));

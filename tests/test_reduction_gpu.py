@@ -133,3 +133,25 @@ def test_f32_max_of_only_negative_infinity_is_type_min(oracle, cuda):
     ref = H.run_reduce(oracle, "max", D.F32, [2, 3], [3, 1], [3], [1], 0, x)
     got = H.run_reduce(cuda, "max", D.F32, [2, 3], [3, 1], [3], [1], 0, x)
     assert np.array_equal(ref, got) and got[0] == np.finfo(np.float32).min
+
+
+@pytest.mark.parametrize("shape", [(2, 3, 5), (3, 300, 49), (256, 64, 49), (64, 7, 9), (130, 33, 1), (4, 8, 4096), (5, 3, 1027), (2, 2, 70001), (700, 2, 3)], ids=str)
+def test_outer_and_inner_dims_folded_around_a_kept_one(oracle, cuda, shape):
+    """sum_to_shape [Q, O, I] -> [1, O, 1], the gradient of a per-channel operand: both orders of the two passes, split and
+    unsplit, vector and scalar strips.  Bound: the sums' tolerance of this file (f32 and wider accumulation, one rounding)."""
+    from oracle import binding
+    q, o, i = shape
+    rng = np.random.default_rng(q * 1000 + o)
+    for dt in (D.F32, D.BF16, D.F16, D.F64, D.I32, D.U8):
+        dims, out_dims = [q, o, i], [1, o, 1]
+        x = H.random_store(rng, dt, H.numel(dims) + 1, dist="normal") if dt.kind == "float" else H.full_range_store(rng, dt, H.numel(dims) + 1)
+        for off in (0, 1):
+            binding.set_wide(True)
+            try:
+                ref = H.run_sum_to_shape(oracle, dt, dims, H.contiguous_strides(dims), out_dims, off, x)
+            finally:
+                binding.set_wide(False)
+            got = H.run_sum_to_shape(cuda, dt, dims, H.contiguous_strides(dims), out_dims, off, x)
+            again = H.run_sum_to_shape(cuda, dt, dims, H.contiguous_strides(dims), out_dims, off, x)
+            assert np.array_equal(got, again)
+            H.assert_same("sum_to_shape", dt, got, ref, float_rel=SUM_TOL.get(dt.name, 0.0), what=str((shape, off)), scale=np.sqrt(q * i))
