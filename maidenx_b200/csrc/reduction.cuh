@@ -212,25 +212,36 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_block_kernel(const T*
     }
 }
 
-// One warp per row (32 <= R < ~2048).
-template <class T, int KIND, int VEC>
-__global__ void __launch_bounds__(kRedThreads) reduce_rows_warp_kernel(const T* in, T* out, u64 rows, u64 R, u64 factor) {
+// G lanes of a warp per row (8 <= R < ~2048), G the smallest of 4, 8, 16, 32 that gives every vector of the row a lane: a
+// row of 56 bf16 is seven vectors, and a whole warp for it left 25 lanes idle (sum over the last dim of [64, 256, 56, 56] bf16
+// and the one after it: 124 us, now 55).  Four loads per lane in flight.
+template <class T, int KIND, int VEC, int G>
+__global__ void __launch_bounds__(kRedThreads) reduce_rows_group_kernel(const T* in, T* out, u64 rows, u64 R, u64 factor) {
     typedef RedTraits<T, KIND> TR;
-    const u64 row = (u64)blockIdx.x * (kRedThreads / 32) + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    const int lane = threadIdx.x & 31;
-    const T* p = in + row * R;
+    const u64 row = (u64)blockIdx.x * (kRedThreads / G) + threadIdx.x / G;
+    const bool live = row < rows;  // the shuffles below take the whole warp
+    const T* p = in + (live ? row : 0) * R;
     typename TR::Acc acc = TR::init();
-    for (u64 i = (u64)lane * VEC; i < R; i += 32 * VEC) {
-        Vec<T, VEC> a = *reinterpret_cast<const Vec<T, VEC>*>(p + i);
+    if (live) {
+        constexpr int STEP = G * VEC;
+        for (u64 i = (threadIdx.x % G) * VEC; i < R; i += 4 * STEP) {
+            Vec<T, VEC> v[4];
 #pragma unroll
-        for (int j = 0; j < VEC; j++) acc = TR::combine(acc, TR::load(a.v[j]));
+            for (int q = 0; q < 4; q++)
+                if (i + q * STEP < R) v[q] = *reinterpret_cast<const Vec<T, VEC>*>(p + i + q * STEP);
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (i + q * STEP < R)
+#pragma unroll
+                    for (int j = 0; j < VEC; j++) acc = TR::combine(acc, TR::load(v[q].v[j]));
+        }
     }
-    acc = warp_reduce<TR>(acc);
-    if (lane == 0) out[row] = TR::finalize(acc, factor);
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) acc = TR::combine(acc, __shfl_xor_sync(0xFFFFFFFFu, acc, o));
+    if (live && threadIdx.x % G == 0) out[row] = TR::finalize(acc, factor);
 }
 
-// One thread per row (R < 32).
+// One thread per row (R < 8).
 template <class T, int KIND>
 __global__ void __launch_bounds__(kRedThreads) reduce_rows_thread_kernel(const T* in, T* out, u64 rows, u64 R, u64 factor) {
     typedef RedTraits<T, KIND> TR;
@@ -506,6 +517,16 @@ u32* arrival_counters(u64 count);                      // zeroed counters for la
 void red_plan_dims(RedPlan& pl, size_t num_els, size_t num_dims, size_t num_red, const size_t* hm);
 void red_plan_shape(RedPlan& pl, size_t num_els, size_t num_dims, const size_t* hm);
 
+template <class T, int KIND, int VEC>
+void red_rows_group_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaStream_t s) {
+    const u64 lanes = (R + VEC - 1) / VEC;
+    auto blocks = [&](int g) { return (u32)((O + kRedThreads / g - 1) / (kRedThreads / g)); };
+    if (lanes <= 4) reduce_rows_group_kernel<T, KIND, VEC, 4><<<blocks(4), kRedThreads, 0, s>>>(in, out, O, R, factor);
+    else if (lanes <= 8) reduce_rows_group_kernel<T, KIND, VEC, 8><<<blocks(8), kRedThreads, 0, s>>>(in, out, O, R, factor);
+    else if (lanes <= 16) reduce_rows_group_kernel<T, KIND, VEC, 16><<<blocks(16), kRedThreads, 0, s>>>(in, out, O, R, factor);
+    else reduce_rows_group_kernel<T, KIND, VEC, 32><<<blocks(32), kRedThreads, 0, s>>>(in, out, O, R, factor);
+}
+
 template <class T, int KIND>
 void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
     typedef RedTraits<T, KIND> TR;
@@ -522,13 +543,12 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
     const bool base_aligned = ((uintptr_t)in) % 16 == 0;
     if (pl.kind == RP_ROWS) {
         const u64 O = pl.O, R = pl.R;
-        if (R < 32) {
+        if (R < 8) {
             u64 blocks = (O + kRedThreads - 1) / kRedThreads;
             reduce_rows_thread_kernel<T, KIND><<<(u32)blocks, kRedThreads, 0, s>>>(in, out, O, R, pl.factor);
-        } else if (R < 2048 && O >= (u64)sms * 4) {
-            u64 blocks = (O + 7) / 8;
-            if (base_aligned && R % VEC == 0) reduce_rows_warp_kernel<T, KIND, VEC><<<(u32)blocks, kRedThreads, 0, s>>>(in, out, O, R, pl.factor);
-            else reduce_rows_warp_kernel<T, KIND, 1><<<(u32)blocks, kRedThreads, 0, s>>>(in, out, O, R, pl.factor);
+        } else if (R < 32 || (R < 2048 && O >= (u64)sms * 4)) {
+            if (base_aligned && R % VEC == 0) red_rows_group_launch<T, KIND, VEC>(in, out, O, R, pl.factor, s);
+            else red_rows_group_launch<T, KIND, 1>(in, out, O, R, pl.factor, s);
         } else {
             // block per (row, split); split long rows when there are too few rows to fill the GPU
             const bool vec = base_aligned && R % VEC == 0;
@@ -543,8 +563,7 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
             seg = (seg + VEC - 1) / VEC * VEC;
             splits = (R + seg - 1) / seg;
             if (O > 65535) {  // grid.y limit: fall back to one warp per row
-                u64 blocks = (O + 7) / 8;
-                reduce_rows_warp_kernel<T, KIND, 1><<<(u32)blocks, kRedThreads, 0, s>>>(in, out, O, R, pl.factor);
+                red_rows_group_launch<T, KIND, 1>(in, out, O, R, pl.factor, s);
             } else {
                 Acc* part = nullptr;
                 u32* counters = nullptr;
