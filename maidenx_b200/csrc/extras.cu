@@ -861,6 +861,167 @@ __global__ void __launch_bounds__(kExThreads) softmax_cols_kernel(const T* __res
     }
 }
 
+// Rows of any length and alignment: the same one-read form with single elements, lane t holding elements t, t + G, ... of
+// the row in registers.  f32 and f64 keep expf / exp and the quotient of the general kernel, whose rows these were;
+// 16-bit types, whose rounding step is 2^-9, take the hardware exp2 and one reciprocal.  Bound by HBM / L2 with a
+// 64-byte (16-bit) or 128-byte request per warp and load: [192 x 197, 197] bf16 9.9 us, 109 in the general kernel.
+template <class T, int G, int K>
+__global__ void __launch_bounds__(kExThreads) softmax_rows_any_kernel(const T* __restrict__ in, T* __restrict__ out, u64 rows, u32 n) {
+    typedef typename std::conditional<std::is_same<T, f64>::value, f64, f32>::type A;
+    __shared__ A part_max[kExThreads / 32], part_sum[kExThreads / 32];
+    const u32 t = threadIdx.x % G;
+    const u64 row = (u64)blockIdx.x * (kExThreads / G) + threadIdx.x / G;
+    if (G == 32 && row >= rows) return;  // whole warps; the warp form uses no block barrier
+    const T* src = in + row * n;
+    T raw[K];
+    A x[K];
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        if (k * G + t < n) raw[k] = src[k * G + t];
+    A mx = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (k * G + t < n) {
+            if constexpr (is_half_v<T>) x[k] = to_f32(raw[k]);
+            else x[k] = (A)raw[k];
+            mx = x[k] > mx ? x[k] : mx;  // a NaN never becomes the maximum
+        }
+    }
+    mx = softmax_group_all<A, G, true>(mx, part_max);
+    A sum = (A)0;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (k * G + t < n) {
+            if constexpr (std::is_same<A, f64>::value) x[k] = exp(x[k] - mx);
+            else if constexpr (is_half_v<T>) x[k] = exp2_approx((x[k] - mx) * 1.4426950408889634f);
+            else x[k] = expf(x[k] - mx);
+            sum += x[k];
+        }
+    }
+    sum = softmax_group_all<A, G, false>(sum, part_sum);
+    const A inv = (A)1 / sum;
+    T* dst = out + row * n;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (k * G + t < n) {
+            if constexpr (is_half_v<T>) dst[k * G + t] = from_f32<T>(x[k] * inv);
+            else dst[k * G + t] = (T)(x[k] / sum);
+        }
+    }
+}
+
+// Column softmax whose elements fit the registers: thread (lane, ry) of a block holds elements ry, ry + ROWS, ... of its
+// VEC neighbouring columns, so each element is read once instead of three times, with the formulas of softmax_cols_kernel.
+// The widest strip whose columns fit: 128, 64 or 32 bytes of each row.
+template <class T, int VEC, int LANES, int K>
+__global__ void __launch_bounds__(kExThreads) softmax_cols_reg_kernel(const T* __restrict__ in, T* __restrict__ out, u64 pre, u32 n, u64 post) {
+    typedef typename std::conditional<std::is_same<T, f64>::value, f64, f32>::type A;
+    constexpr int ROWS = kExThreads / LANES;
+    __shared__ A part[kExThreads / 32][LANES][VEC];
+    const int lane = threadIdx.x % LANES, ry = threadIdx.x / LANES;
+    const u64 col = ((u64)blockIdx.x * LANES + lane) * VEC;
+    const bool live = col < pre * post;
+    const u64 pre_idx = live ? col / post : 0, post_idx = live ? col - pre_idx * post : 0;
+    const u64 base = pre_idx * n * post + post_idx;
+    auto has = [&](int k) { return live && (u32)(k * ROWS + ry) < n; };
+    // over the threads of a column: by shuffles inside a warp, then over the eight warps through shared memory
+    auto column_all = [&](A (&v)[VEC], bool is_max) {
+#pragma unroll
+        for (int j = 0; j < VEC; j++)
+#pragma unroll
+            for (int o = LANES; o < 32; o <<= 1) {
+                const A w = __shfl_xor_sync(0xFFFFFFFFu, v[j], o);
+                v[j] = is_max ? (w > v[j] ? w : v[j]) : v[j] + w;
+            }
+        __syncthreads();  // the previous use of `part` has been read
+        if (threadIdx.x % 32 < LANES) {
+#pragma unroll
+            for (int j = 0; j < VEC; j++) part[threadIdx.x / 32][lane][j] = v[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < VEC; j++) {
+            A r = part[0][lane][j];
+#pragma unroll
+            for (int k = 1; k < kExThreads / 32; k++) r = is_max ? (part[k][lane][j] > r ? part[k][lane][j] : r) : r + part[k][lane][j];
+            v[j] = r;
+        }
+    };
+    Vec<T, VEC> raw[K];
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        if (has(k)) raw[k] = *reinterpret_cast<const Vec<T, VEC>*>(in + base + (u64)(k * ROWS + ry) * post);
+    A x[K][VEC], mx[VEC], sum[VEC];
+#pragma unroll
+    for (int j = 0; j < VEC; j++) {
+        mx[j] = -INFINITY;
+        sum[j] = (A)0;
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (has(k)) {
+#pragma unroll
+            for (int j = 0; j < VEC; j++) {
+                if constexpr (is_half_v<T>) x[k][j] = to_f32(raw[k].v[j]);
+                else x[k][j] = (A)raw[k].v[j];
+                mx[j] = x[k][j] > mx[j] ? x[k][j] : mx[j];
+            }
+        }
+    }
+    column_all(mx, true);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (has(k)) {
+#pragma unroll
+            for (int j = 0; j < VEC; j++) {
+                if constexpr (std::is_same<A, f64>::value) x[k][j] = exp(x[k][j] - mx[j]);
+                else x[k][j] = expf(x[k][j] - mx[j]);
+                sum[j] += x[k][j];
+            }
+        }
+    }
+    column_all(sum, false);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (has(k)) {
+            Vec<T, VEC> r;
+#pragma unroll
+            for (int j = 0; j < VEC; j++) {
+                const A q = x[k][j] / sum[j];
+                if constexpr (is_half_v<T>) r.v[j] = from_f32<T>(q);
+                else r.v[j] = (T)q;
+            }
+            *reinterpret_cast<Vec<T, VEC>*>(out + base + (u64)(k * ROWS + ry) * post) = r;
+        }
+    }
+}
+// false: the columns do not fit (more than 64 32-bit values per thread)
+template <class T, int VEC, int LANES>
+bool softmax_cols_reg_launch(const T* in, T* out, u64 pre, u64 n, u64 post, cudaStream_t s) {
+    constexpr int ROWS = kExThreads / LANES, KMAX = (sizeof(T) == 8 ? 32 : 64) / VEC;
+    const u64 per = (n + ROWS - 1) / ROWS;
+    const unsigned blocks = (unsigned)((pre * post / VEC + LANES - 1) / LANES);
+    if (per <= KMAX / 4) softmax_cols_reg_kernel<T, VEC, LANES, KMAX / 4><<<blocks, kExThreads, 0, s>>>(in, out, pre, (u32)n, post);
+    else if (per <= KMAX / 2) softmax_cols_reg_kernel<T, VEC, LANES, KMAX / 2><<<blocks, kExThreads, 0, s>>>(in, out, pre, (u32)n, post);
+    else if (per <= KMAX) softmax_cols_reg_kernel<T, VEC, LANES, KMAX><<<blocks, kExThreads, 0, s>>>(in, out, pre, (u32)n, post);
+    else return false;
+    return true;
+}
+
+template <class T, int G>
+bool softmax_rows_any_launch(const T* in, T* out, u64 rows, u32 n, cudaStream_t s) {
+    const u32 per = (n + G - 1) / G;  // elements per thread
+    const unsigned blocks = (unsigned)((rows + kExThreads / G - 1) / (kExThreads / G));
+    if (per <= 2) softmax_rows_any_kernel<T, G, 2><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
+    else if (per <= 4) softmax_rows_any_kernel<T, G, 4><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
+    else if (per <= 8) softmax_rows_any_kernel<T, G, 8><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
+    else if (per <= 16) softmax_rows_any_kernel<T, G, 16><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
+    else if (per <= 32) softmax_rows_any_kernel<T, G, 32><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
+    else if (sizeof(T) <= 4 && per <= 64) softmax_rows_any_kernel<T, G, sizeof(T) <= 4 ? 64 : 32><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
+    else return false;
+    return true;
+}
+
 template <class T, int G>
 bool softmax_rows_launch(const T* in, T* out, u64 rows, u32 n, cudaStream_t s) {
     constexpr int VEC = 16 / (int)sizeof(T);
@@ -920,8 +1081,23 @@ void softmax_entry(size_t num_els, size_t nd, size_t dim, const size_t* meta, co
                 return;
             }
         }
+        // rows that are not whole aligned vectors: a warp up to 1024 elements (32 per lane), a block beyond
+        if (P.post == 1 && P.pre < (1ull << 31) && P.n <= 64ull * kExThreads) {
+            const bool done = P.n <= 1024 ? softmax_rows_any_launch<T, 32>(src, out, P.pre, (u32)P.n, st)
+                                          : softmax_rows_any_launch<T, kExThreads>(src, out, P.pre, (u32)P.n, st);
+            if (done) {
+                check_launch(where);
+                return;
+            }
+        }
         if (P.post >= 16) {
             const bool wide = P.post % VEC == 0 && (reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+            if (wide ? softmax_cols_reg_launch<T, VEC, 8>(src, out, P.pre, P.n, P.post, st) || softmax_cols_reg_launch<T, VEC, 4>(src, out, P.pre, P.n, P.post, st) ||
+                           softmax_cols_reg_launch<T, VEC, 2>(src, out, P.pre, P.n, P.post, st)
+                     : softmax_cols_reg_launch<T, 1, 32>(src, out, P.pre, P.n, P.post, st)) {
+                check_launch(where);
+                return;
+            }
             if (wide) softmax_cols_kernel<T, VEC, 8><<<(unsigned)((slices / VEC + 7) / 8), kExThreads, 0, st>>>(src, out, P.pre, P.n, P.post);
             else softmax_cols_kernel<T, 1, 32><<<(unsigned)((slices + 31) / 32), kExThreads, 0, st>>>(src, out, P.pre, P.n, P.post);
             check_launch(where);

@@ -293,3 +293,25 @@ def test_softmax_special_values(oracle, cuda):
                 assert np.all(np.abs(got[ok] - ref[ok]) <= tol * np.maximum(np.abs(ref[ok]), 1e-30 if dt.name == "f32" else 1e-4)), (dt.name, dims, dim)
     finally:
         oracle.b.set_wide(False)
+
+
+@pytest.mark.parametrize("dt", [D.F32, D.F64, D.BF16, D.F16], ids=lambda d: d.name)
+def test_softmax_of_ragged_rows_and_of_columns_in_registers(oracle, cuda, dt):
+    """Row lengths around the steps of the single-element row form (a warp up to 1024, a block up to its registers, the
+    general kernel beyond) and column lengths around those of the one-read column form, vector and scalar strips.  f32
+    and f64 keep the general kernel's functions: a few ulp of each quotient; 16-bit results carry one rounding."""
+    rng = np.random.default_rng(31)
+    tol = {"f32": 2e-6, "f64": 1e-14, "bf16": 2.0 ** -7, "f16": 2.0 ** -10}[dt.name]
+    cases = [([9, n], 1, off) for n, off in ((1, 0), (2, 1), (31, 0), (33, 0), (64, 1), (65, 0), (197, 0), (255, 1), (513, 0), (1023, 0), (1025, 0), (2049, 0), (4097, 1), (8193, 0), (16383, 0), (16391, 0))]
+    cases += [([2, n, post], 1, off) for n in (3, 8, 33, 65, 127, 257, 513, 1031) for post, off in ((16, 0), (40, 0), (37, 0), (40, 1))]
+    oracle.b.set_wide(True)
+    try:
+        for dims, dim, off in cases:
+            x = D.encode(rng.standard_normal(H.numel(dims) + off) * 3.0, dt)
+            st = H.contiguous_strides(dims)
+            ref = D.decode(H.run_softmax(oracle, dt, dims, st, off, dim, x), dt).astype(np.float64)
+            got = D.decode(H.run_softmax(cuda, dt, dims, st, off, dim, x), dt).astype(np.float64)
+            floor = 6.2e-5 if dt.name == "f16" else 1e-300  # below the smallest normal f16 the rounding step no longer shrinks
+            assert np.all(np.abs(got - ref) <= tol * np.maximum(np.abs(ref), floor)), (dims, off, np.abs(got / np.maximum(ref, 1e-30) - 1).max())
+    finally:
+        oracle.b.set_wide(False)
