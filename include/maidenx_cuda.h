@@ -265,6 +265,12 @@ MX_DTYPES_ALL(MX_DECL_CAST_FROM, _)
  * 0 turns both off: every request goes to cudaMalloc / cudaFree / cudaMemcpy, as in the reference. */
 void mx_set_small_pool(int enabled);
 
+/* What a dispatch layer does around an op, in two calls: select `device`, cuda_malloc a metadata block and cuda_memcpy_h2d
+ * `count` words into it (returns the first failing call's code, 0 = ok); after the op, cuda_free the block (returns the
+ * sticky status of mx_last_error). */
+int mx_dispatch_begin(int device, const size_t* host_metadata, size_t count, void** block);
+int mx_dispatch_end(void* block);
+
 /* Stream used by this thread's subsequent op launches (NULL = legacy default stream). */
 void mx_set_stream(void* stream);
 void* mx_get_stream(void);

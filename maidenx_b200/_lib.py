@@ -25,6 +25,8 @@ RUNTIME_SIGNATURES = {
     "cuda_stream_synchronize": ([ctypes.c_void_p], ctypes.c_int),
     "cuda_pointer_get_attributes": ([ctypes.c_void_p, ctypes.c_void_p], ctypes.c_int),
     "cuda_error_string": ([ctypes.c_int], ctypes.c_char_p),
+    "mx_dispatch_begin": ([ctypes.c_int, ctypes.c_char_p, ctypes.c_size_t, ctypes.POINTER(ctypes.c_void_p)], ctypes.c_int),
+    "mx_dispatch_end": ([ctypes.c_void_p], ctypes.c_int),
     "mx_set_stream": ([ctypes.c_void_p], None),
     "mx_get_stream": ([], ctypes.c_void_p),
     "mx_last_error": ([], ctypes.c_int),

@@ -524,6 +524,22 @@ int cuda_memcpy_d2d(void* dst, const void* src, size_t size) {
     return (int)cudaMemcpy(dst, src, size, cudaMemcpyDeviceToDevice);
 }
 
+// The calls around an op in the dispatch pattern, folded into two (fewer crossings for callers behind a foreign-function layer).
+int mx_dispatch_begin(int device, const size_t* host_metadata, size_t count, void** block) {
+    *block = nullptr;
+    int e = (int)cudaSetDevice(device);
+    if (e == 0) e = cuda_malloc(block, count ? count * sizeof(size_t) : 1);
+    if (e == 0 && count && (e = cuda_memcpy_h2d(*block, host_metadata, count * sizeof(size_t))) != 0) {
+        cuda_free(*block);
+        *block = nullptr;
+    }
+    return e;
+}
+int mx_dispatch_end(void* block) {
+    cuda_free(block);
+    return ctx().status;
+}
+
 int cuda_set_device(int device_id) { return (int)cudaSetDevice(device_id); }
 int cuda_get_device(int* device_id) { return (int)cudaGetDevice(device_id); }
 int cuda_stream_create(void** stream) { return (int)cudaStreamCreate(reinterpret_cast<cudaStream_t*>(stream)); }
