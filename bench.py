@@ -816,10 +816,10 @@ def config1_row(torch, lib, steps=200, with_cpu=True):
 MLP_LAYERS, MLP_DIM, MLP_GLOBAL_BATCH, MLP_LR = 4, 8192, 16384, 1e-3
 MLP_GEMMS_PER_STEP = 3 * MLP_LAYERS - 1       # dX of the first layer is not needed and not computed
 # kernels launched per step: 11 GEMMs (the 4 forward ones carry the bias add and GELU in their epilogue) + 2 (mse,
-# mse finish) + 3 gelu backward + 4 bias-gradient sums (partials folded inside the same launch) + 8 SGD updates (weights
-# and bias per layer; on a side stream at N = 1); with the NVLink exchange the 8 SGD launches become
-# 4 x (barrier, fused reduce + update, barrier)
-MLP_KERNELS_PER_STEP = MLP_GEMMS_PER_STEP + 2 + (MLP_LAYERS - 1) + MLP_LAYERS + 2 * MLP_LAYERS
+# mse finish; the last layer's bias gradient rides along) + 3 x 2 (gelu backward with the bias gradient's partial sums, their
+# fold) + 4 SGD updates (weights and bias of a layer in one launch; on a side stream at N = 1); with the NVLink exchange the
+# 4 SGD launches become 4 x (barrier, fused reduce + update, barrier)
+MLP_KERNELS_PER_STEP = MLP_GEMMS_PER_STEP + 2 + 2 * (MLP_LAYERS - 1) + MLP_LAYERS
 
 
 EXCHANGE_TEXT = {
@@ -1239,7 +1239,7 @@ def main():
                            "per_gpu_batch": local_batch, "parallelism": f"dp{world}", "allreduce": EXCHANGE_TEXT[mlp_exchange],
                            "l2": "per-step working set (weights 0.5 GB + activations 2 GB per GPU at N=1) far exceeds the 126 MB L2; sweep inputs are 0.5-2 GB",
                            "verified": verified if verify else "skipped (--no-verify)"},
-                "loss": loss, "clocks": clocks, "gpu_launches": (MLP_KERNELS_PER_STEP + (3 * MLP_LAYERS - 2 * MLP_LAYERS if exch else 0)) * args.steps,
+                "loss": loss, "clocks": clocks, "gpu_launches": (MLP_KERNELS_PER_STEP + (3 * MLP_LAYERS - MLP_LAYERS if exch else 0)) * args.steps,
                 "roofline": roofline, "e2e": e2e, "cpu_baseline": cpu, "sweeps": sweeps_out}
         print(json.dumps(line))
 

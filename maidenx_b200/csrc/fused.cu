@@ -10,6 +10,7 @@
 //                                                        f32 master copy of the 16-bit weights
 // All are HBM-bound: 16-byte vector accesses, four vectors in flight per thread, math in f32,
 // one rounding per stored value.
+#include "fused.cuh"
 #include "abi_common.cuh"
 #include "ops.cuh"
 #include "matmul_tc.cuh"
@@ -76,30 +77,62 @@ __device__ __forceinline__ float gelu_grad_f32(float x) {
     return 0.5f * (1.0f + th) + 0.5f * x * sech2 * s * (1.0f + 3.0f * c * x2);
 }
 
-template <class T>
+// The block's sum of v; valid in thread 0.
+__device__ __forceinline__ float fused_block_sum(float v) {
+    __shared__ float warp_part[kFusedThreads / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < kFusedThreads / 32; w++) v += warp_part[w];
+    return v;
+}
+
+// SUM: per-block partial sums of du into `partial` (the bias gradient), which the pass over du that used to follow read it back for.
+template <class T, bool SUM>
 __global__ void __launch_bounds__(kFusedThreads) gelu_backward_kernel(const T* __restrict__ dy, const T* __restrict__ u, T* __restrict__ du,
-                                                                     uint64_t n) {
+                                                                     uint64_t n, float* __restrict__ partial) {
+    float acc = 0.0f;
     constexpr int VEC = 16 / sizeof(T);
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
     for (uint64_t v = (uint64_t)blockIdx.x * kFusedThreads + threadIdx.x; v < nvec; v += stride) {
         Vec<T, VEC> g = *reinterpret_cast<const Vec<T, VEC>*>(dy + v * VEC), x = *reinterpret_cast<const Vec<T, VEC>*>(u + v * VEC), o;
 #pragma unroll
-        for (int j = 0; j < VEC; j++) o.v[j] = st_from_f32<T>(up(g.v[j]) * gelu_grad_f32(up(x.v[j])));
+        for (int j = 0; j < VEC; j++) {
+            o.v[j] = st_from_f32<T>(up(g.v[j]) * gelu_grad_f32(up(x.v[j])));
+            if (SUM) acc += up(o.v[j]);
+        }
         *reinterpret_cast<Vec<T, VEC>*>(du + v * VEC) = o;
     }
     if (blockIdx.x == 0)
-        for (uint64_t i = nvec * VEC + threadIdx.x; i < n; i += kFusedThreads) du[i] = st_from_f32<T>(up(dy[i]) * gelu_grad_f32(up(u[i])));
+        for (uint64_t i = nvec * VEC + threadIdx.x; i < n; i += kFusedThreads) {
+            du[i] = st_from_f32<T>(up(dy[i]) * gelu_grad_f32(up(u[i])));
+            if (SUM) acc += up(du[i]);
+        }
+    if constexpr (SUM) {
+        acc = fused_block_sum(acc);
+        if (threadIdx.x == 0) partial[blockIdx.x] = acc;
+    }
+}
+// One block: the rounded sum of the partial sums, in a fixed order.
+template <class T>
+__global__ void __launch_bounds__(kFusedThreads) sum_finish_kernel(const float* __restrict__ partial, int count, T* __restrict__ out) {
+    float acc = 0.0f;
+    for (int i = threadIdx.x; i < count; i += kFusedThreads) acc += partial[i];
+    acc = fused_block_sum(acc);
+    if (threadIdx.x == 0) *out = st_from_f32<T>(acc);
 }
 
-// Pass 1: grad = 2 (p - t) / n, per-block partial sums of (p - t)^2 into `partial`.
-template <class T>
+// Pass 1: grad = 2 (p - t) / n, per-block partial sums of (p - t)^2 into `partial` and, with SUM, of grad behind them.
+template <class T, bool SUM>
 __global__ void __launch_bounds__(kFusedThreads) mse_kernel(const T* __restrict__ p, const T* __restrict__ t, T* __restrict__ grad,
                                                            float* __restrict__ partial, uint64_t n, float two_over_n) {
     constexpr int VEC = 16 / sizeof(T);
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
-    float acc = 0.0f;
+    float acc = 0.0f, acc_g = 0.0f;
     for (uint64_t v = (uint64_t)blockIdx.x * kFusedThreads + threadIdx.x; v < nvec; v += stride) {
         Vec<T, VEC> a = *reinterpret_cast<const Vec<T, VEC>*>(p + v * VEC), b = *reinterpret_cast<const Vec<T, VEC>*>(t + v * VEC), o;
 #pragma unroll
@@ -108,6 +141,7 @@ __global__ void __launch_bounds__(kFusedThreads) mse_kernel(const T* __restrict_
             float d = up(st_from_f32<T>(up(a.v[j]) - up(b.v[j])));
             acc += d * d;
             o.v[j] = st_from_f32<T>(d * two_over_n);
+            if (SUM) acc_g += up(o.v[j]);
         }
         *reinterpret_cast<Vec<T, VEC>*>(grad + v * VEC) = o;
     }
@@ -116,39 +150,55 @@ __global__ void __launch_bounds__(kFusedThreads) mse_kernel(const T* __restrict_
             float d = up(st_from_f32<T>(up(p[i]) - up(t[i])));
             acc += d * d;
             grad[i] = st_from_f32<T>(d * two_over_n);
+            if (SUM) acc_g += up(grad[i]);
         }
-    __shared__ float warp_part[kFusedThreads / 32];
+    __shared__ float warp_part[SUM ? 2 : 1][kFusedThreads / 32];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = acc;
+    for (int o = 16; o > 0; o >>= 1) {
+        acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+        if (SUM) acc_g += __shfl_xor_sync(0xFFFFFFFFu, acc_g, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        warp_part[0][threadIdx.x >> 5] = acc;
+        if (SUM) warp_part[SUM ? 1 : 0][threadIdx.x >> 5] = acc_g;
+    }
     __syncthreads();
-    if (threadIdx.x < 32) {
-        float v = threadIdx.x < kFusedThreads / 32 ? warp_part[threadIdx.x] : 0.0f;
+    if (threadIdx.x < (SUM ? 64 : 32)) {  // the first warp folds the losses, the second the gradients
+        const int which = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        float v = lane < kFusedThreads / 32 ? warp_part[which][lane] : 0.0f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        if (threadIdx.x == 0) partial[blockIdx.x] = v;
+        if (lane == 0) partial[which * gridDim.x + blockIdx.x] = v;
     }
 }
-// Pass 2: one block folds the partials in a fixed order.
-__global__ void __launch_bounds__(kFusedThreads) mse_finish_kernel(const float* __restrict__ partial, int count, float inv_n, float* __restrict__ loss) {
+// Pass 2: one block per output folds its partials in a fixed order: block 0 the loss, block 1 the gradient's sum.
+template <class T>
+__global__ void __launch_bounds__(kFusedThreads) mse_finish_kernel(const float* __restrict__ partial, int count, float inv_n, float* __restrict__ loss, T* __restrict__ grad_sum) {
     __shared__ float sm[kFusedThreads];
     float acc = 0.0f;
-    for (int i = threadIdx.x; i < count; i += kFusedThreads) acc += partial[i];
+    for (int i = threadIdx.x; i < count; i += kFusedThreads) acc += partial[(int)blockIdx.x * count + i];
     sm[threadIdx.x] = acc;
     __syncthreads();
     for (int o = kFusedThreads / 2; o > 0; o >>= 1) {
         if (threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *loss = sm[0] * inv_n;
+    if (threadIdx.x) return;
+    if (blockIdx.x == 0) *loss = sm[0] * inv_n;
+    else *grad_sum = st_from_f32<T>(sm[0]);
 }
 
 template <class T>
 __global__ void __launch_bounds__(kFusedThreads) sgd_kernel(float* __restrict__ w32, const T* __restrict__ g, T* __restrict__ w16, uint64_t n,
-                                                           float step) {
+                                                           float step, float* __restrict__ b32, const T* __restrict__ gb, T* __restrict__ b16) {
     constexpr int VEC = 16 / sizeof(T);  // elements per 16-byte vector of the gradient; w32 moves as VEC floats
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
+    if (b32 && blockIdx.x == 0 && threadIdx.x == 0) {  // the layer's one-element bias
+        const float w = *b32 - step * up(*gb);
+        *b32 = w;
+        *b16 = st_from_f32<T>(w);
+    }
     for (uint64_t v = (uint64_t)blockIdx.x * kFusedThreads + threadIdx.x; v < nvec; v += stride) {
         Vec<T, VEC> gi = *reinterpret_cast<const Vec<T, VEC>*>(g + v * VEC), wo;
         // the master weights are promised 16-byte aligned only: move them as float4 quads, never as one 32-byte access
@@ -197,39 +247,67 @@ void bias_gelu_launch(size_t n, const T* z, const T* bias, T* u, T* a, const cha
     check_launch(where);
 }
 template <class T>
-void gelu_backward_launch(size_t n, const T* dy, const T* u, T* du, const char* where) {
+void gelu_backward_launch(size_t n, const T* dy, const T* u, T* du, T* grad_sum, const char* where) {
     if (!n) return;
     if (!aligned16(dy) || !aligned16(u) || !aligned16(du)) {
         set_error(kErrUnsupported, 0, where);
         return;
     }
-    gelu_backward_kernel<T><<<fused_grid(n, 16 / sizeof(T)), kFusedThreads, 0, ctx().stream>>>(dy, u, du, n);
+    const unsigned blocks = fused_grid(n, 16 / sizeof(T));
+    if (!grad_sum) {
+        gelu_backward_kernel<T, false><<<blocks, kFusedThreads, 0, ctx().stream>>>(dy, u, du, n, nullptr);
+    } else {
+        float* partial = static_cast<float*>(scratch(sizeof(float) * blocks));
+        if (!partial) return;
+        gelu_backward_kernel<T, true><<<blocks, kFusedThreads, 0, ctx().stream>>>(dy, u, du, n, partial);
+        sum_finish_kernel<T><<<1, kFusedThreads, 0, ctx().stream>>>(partial, (int)blocks, grad_sum);
+    }
     check_launch(where);
 }
 template <class T>
-void mse_launch(size_t n, const T* p, const T* t, T* grad, float* loss, const char* where) {
+void mse_launch(size_t n, const T* p, const T* t, T* grad, float* loss, T* grad_sum, const char* where) {
     if (!n) return;
     if (!aligned16(p) || !aligned16(t) || !aligned16(grad)) {
         set_error(kErrUnsupported, 0, where);
         return;
     }
     unsigned blocks = fused_grid(n, 16 / sizeof(T));
-    float* partial = static_cast<float*>(scratch(sizeof(float) * blocks));
+    float* partial = static_cast<float*>(scratch(sizeof(float) * blocks * (grad_sum ? 2 : 1)));
     if (!partial) return;
-    mse_kernel<T><<<blocks, kFusedThreads, 0, ctx().stream>>>(p, t, grad, partial, n, 2.0f / (float)n);
-    mse_finish_kernel<<<1, kFusedThreads, 0, ctx().stream>>>(partial, (int)blocks, 1.0f / (float)n, loss);
+    if (grad_sum) mse_kernel<T, true><<<blocks, kFusedThreads, 0, ctx().stream>>>(p, t, grad, partial, n, 2.0f / (float)n);
+    else mse_kernel<T, false><<<blocks, kFusedThreads, 0, ctx().stream>>>(p, t, grad, partial, n, 2.0f / (float)n);
+    mse_finish_kernel<T><<<grad_sum ? 2 : 1, kFusedThreads, 0, ctx().stream>>>(partial, (int)blocks, 1.0f / (float)n, loss, grad_sum);
     check_launch(where);
 }
 template <class T>
-void sgd_launch(size_t n, float* w32, const T* g, T* w16, float lr, float grad_scale, const char* where) {
+void sgd_launch(size_t n, float* w32, const T* g, T* w16, float lr, float grad_scale, const char* where, float* b32 = nullptr, const T* gb = nullptr, T* b16 = nullptr) {
     if (!n) return;
     if (!aligned16(w32) || !aligned16(g) || !aligned16(w16)) {
         set_error(kErrUnsupported, 0, where);
         return;
     }
-    sgd_kernel<T><<<fused_grid(n, 16 / sizeof(T)), kFusedThreads, 0, ctx().stream>>>(w32, g, w16, n, lr * grad_scale);
+    sgd_kernel<T><<<fused_grid(n, 16 / sizeof(T)), kFusedThreads, 0, ctx().stream>>>(w32, g, w16, n, lr * grad_scale, b32, gb, b16);
     check_launch(where);
 }
+
+template <class T>
+void mse_loss_grad_sum(size_t n, const T* pred, const T* target, T* grad, float* loss, T* grad_sum, const char* where) {
+    mse_launch<T>(n, pred, target, grad, loss, grad_sum, where);
+}
+template <class T>
+void gelu_backward_sum(size_t n, const T* dy, const T* u, T* du, T* grad_sum, const char* where) {
+    gelu_backward_launch<T>(n, dy, u, du, grad_sum, where);
+}
+template <class T>
+void sgd_update_layer(size_t n, float* w32, const T* grad, T* w16, float* b32, const T* grad_b, T* b16, float lr, float grad_scale, const char* where) {
+    sgd_launch<T>(n, w32, grad, w16, lr, grad_scale, where, b32, grad_b, b16);
+}
+template void mse_loss_grad_sum<bf16>(size_t, const bf16*, const bf16*, bf16*, float*, bf16*, const char*);
+template void mse_loss_grad_sum<f16>(size_t, const f16*, const f16*, f16*, float*, f16*, const char*);
+template void gelu_backward_sum<bf16>(size_t, const bf16*, const bf16*, bf16*, bf16*, const char*);
+template void gelu_backward_sum<f16>(size_t, const f16*, const f16*, f16*, f16*, const char*);
+template void sgd_update_layer<bf16>(size_t, float*, const bf16*, bf16*, float*, const bf16*, bf16*, float, float, const char*);
+template void sgd_update_layer<f16>(size_t, float*, const f16*, f16*, float*, const f16*, f16*, float, float, const char*);
 
 }  // namespace mx
 
@@ -238,10 +316,10 @@ void sgd_launch(size_t n, float* w32, const T* g, T* w16, float lr, float grad_s
         mx::bias_gelu_launch<mx_##T>(n, z, bias, u, a, "mx_bias_gelu_" #T);                                                             \
     }                                                                                                                                   \
     void mx_gelu_backward_##T(size_t n, const mx_##T* dy, const mx_##T* u, mx_##T* du) {                                                \
-        mx::gelu_backward_launch<mx_##T>(n, dy, u, du, "mx_gelu_backward_" #T);                                                         \
+        mx::gelu_backward_launch<mx_##T>(n, dy, u, du, nullptr, "mx_gelu_backward_" #T);                                                \
     }                                                                                                                                   \
     void mx_mse_loss_grad_##T(size_t n, const mx_##T* pred, const mx_##T* target, mx_##T* grad, float* loss) {                          \
-        mx::mse_launch<mx_##T>(n, pred, target, grad, loss, "mx_mse_loss_grad_" #T);                                                    \
+        mx::mse_launch<mx_##T>(n, pred, target, grad, loss, nullptr, "mx_mse_loss_grad_" #T);                                           \
     }                                                                                                                                   \
     void mx_sgd_update_##T(size_t n, float* w32, const mx_##T* grad, mx_##T* w16, float lr, float grad_scale) {                         \
         mx::sgd_launch<mx_##T>(n, w32, grad, w16, lr, grad_scale, "mx_sgd_update_" #T);                                                 \

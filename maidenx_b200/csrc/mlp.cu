@@ -12,8 +12,8 @@
 //                                     (crates/maidenx_tensor_v2/src/ops/_try_matmul.rs:98-140)
 // (dX and dW are the mathematically correct products; the reference's eager matmul_backward,
 // which ignores the strides of the transposed weight view, is exercised separately by the
-// parity tests.)  Elementwise passes use the fused mx_* kernels; the bias gradient is a
-// cuda_sum_<T> over du.
+// parity tests.)  Elementwise passes use the fused mx_* kernels; the bias gradient is the
+// sum of du, taken where du is produced.
 //
 // The step is split so that a data-parallel driver can overlap the gradient all-reduce of layer
 // l with the backward of layer l-1: forward, loss_backward, backward_layer(l), sgd_layer(l).
@@ -24,18 +24,13 @@
 #include <vector>
 
 #include "abi_common.cuh"
+#include "fused.cuh"
 
 extern "C" {
 void mx_bias_gelu_bf16(size_t, const mx_bf16*, const mx_bf16*, mx_bf16*, mx_bf16*);
 void mx_bias_gelu_f16(size_t, const mx_f16*, const mx_f16*, mx_f16*, mx_f16*);
-void mx_gelu_backward_bf16(size_t, const mx_bf16*, const mx_bf16*, mx_bf16*);
-void mx_gelu_backward_f16(size_t, const mx_f16*, const mx_f16*, mx_f16*);
-void mx_mse_loss_grad_bf16(size_t, const mx_bf16*, const mx_bf16*, mx_bf16*, float*);
-void mx_mse_loss_grad_f16(size_t, const mx_f16*, const mx_f16*, mx_f16*, float*);
 void mx_linear_bias_gelu_bf16(size_t, size_t, size_t, const mx_bf16*, const mx_bf16*, const mx_bf16*, mx_bf16*, mx_bf16*);
 void mx_linear_bias_gelu_f16(size_t, size_t, size_t, const mx_f16*, const mx_f16*, const mx_f16*, mx_f16*, mx_f16*);
-void mx_sgd_update_bf16(size_t, float*, const mx_bf16*, mx_bf16*, float, float);
-void mx_sgd_update_f16(size_t, float*, const mx_f16*, mx_f16*, float, float);
 void mx_dp_barrier(void* const*, size_t, int, int, uint32_t, uint32_t*, void*);
 void mx_dp_reduce_sgd(int, void* const*, void*, const void* const*, int, int, size_t, size_t, size_t, float*, size_t, size_t, float*, void*, float, int, void*);
 void mx_mlp_destroy(void*);
@@ -147,8 +142,8 @@ template <class T>
 static void loss_backward_t(Mlp* m, const T* y) {
     const size_t n = m->batch * m->dim;
     const T* pred = reinterpret_cast<const T*>(m->u[m->layers - 1]);
-    if constexpr (std::is_same<T, bf16>::value) mx_mse_loss_grad_bf16(n, pred, y, reinterpret_cast<T*>(m->du[(m->layers - 1) & 1]), m->loss);
-    else mx_mse_loss_grad_f16(n, pred, y, reinterpret_cast<T*>(m->du[(m->layers - 1) & 1]), m->loss);
+    // the same pass leaves the last layer's bias gradient, the sum of the gradient it writes
+    mse_loss_grad_sum<T>(n, pred, y, reinterpret_cast<T*>(m->du[(m->layers - 1) & 1]), m->loss, reinterpret_cast<T*>(m->gb[m->layers - 1]), "mx_mlp_loss_backward");
 }
 
 // Backward of layer l, first part: the gradient w.r.t. the pre-activation, the bias gradient, and the gradient
@@ -157,19 +152,11 @@ template <class T>
 static void backward_input_t(Mlp* m, int l) {
     const size_t B = m->batch, D = m->dim, n = B * D;
     T* du = reinterpret_cast<T*>(m->du[l & 1]);
-    if (l != m->layers - 1) {
-        // d_act holds the gradient w.r.t. a[l]; turn it into the gradient w.r.t. u[l]
-        if constexpr (std::is_same<T, bf16>::value)
-            mx_gelu_backward_bf16(n, reinterpret_cast<const T*>(m->d_act), reinterpret_cast<const T*>(m->u[l]), du);
-        else
-            mx_gelu_backward_f16(n, reinterpret_cast<const T*>(m->d_act), reinterpret_cast<const T*>(m->u[l]), du);
-    }
-    // bias gradient: sum of du over all elements (the scalar bias broadcasts over the whole output)
-    {
-        const size_t meta[] = {n, 1, n, 1, 0};  // dims | strides | red_len | red_stride | offset
-        if constexpr (std::is_same<T, bf16>::value) cuda_sum_bf16(n, 1, 1, meta, du, reinterpret_cast<T*>(m->gb[l]));
-        else cuda_sum_f16(n, 1, 1, meta, du, reinterpret_cast<T*>(m->gb[l]));
-    }
+    // d_act holds the gradient w.r.t. a[l]; turn it into the gradient w.r.t. u[l].  The same pass leaves the bias gradient, the sum
+    // of du over all elements (the scalar bias broadcasts over the whole output); the last layer's came with its du.
+    // At 16384 x 8192 the sums' own passes took 51 us a layer.
+    if (l != m->layers - 1)
+        gelu_backward_sum<T>(n, reinterpret_cast<const T*>(m->d_act), reinterpret_cast<const T*>(m->u[l]), du, reinterpret_cast<T*>(m->gb[l]), "mx_mlp_backward_layer");
     // gradient for the layer below: da_prev [B, D_in] = du [B, D_out] . W [D_out, D_in]
     if (l > 0) {
         const size_t meta[] = {2, 2, 2, B, D, B, D, D, D, D, 1, D, 1, 0, 0};
@@ -198,13 +185,8 @@ static void backward_layer_t(Mlp* m, int l) {
 template <class T>
 static void sgd_layer_t(Mlp* m, int l, float lr, float grad_scale) {
     const size_t D = m->dim;
-    if constexpr (std::is_same<T, bf16>::value) {
-        mx_sgd_update_bf16(D * D, m->w32[l], reinterpret_cast<const T*>(m->gw[l]), reinterpret_cast<T*>(m->w16[l]), lr, grad_scale);
-        mx_sgd_update_bf16(1, m->b32[l], reinterpret_cast<const T*>(m->gb[l]), reinterpret_cast<T*>(m->b16[l]), lr, grad_scale);
-    } else {
-        mx_sgd_update_f16(D * D, m->w32[l], reinterpret_cast<const T*>(m->gw[l]), reinterpret_cast<T*>(m->w16[l]), lr, grad_scale);
-        mx_sgd_update_f16(1, m->b32[l], reinterpret_cast<const T*>(m->gb[l]), reinterpret_cast<T*>(m->b16[l]), lr, grad_scale);
-    }
+    sgd_update_layer<T>(D * D, m->w32[l], reinterpret_cast<const T*>(m->gw[l]), reinterpret_cast<T*>(m->w16[l]), m->b32[l], reinterpret_cast<const T*>(m->gb[l]),
+                        reinterpret_cast<T*>(m->b16[l]), lr, grad_scale, "mx_mlp_sgd_layer");
 }
 
 }  // namespace mx
