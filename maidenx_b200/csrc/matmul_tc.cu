@@ -1143,6 +1143,21 @@ bool tc_batched_row_bias(bool is_bf16, uint64_t batch, uint64_t rows, uint64_t k
     return repack_operands(2, c, ws, where) && launch_gemm(is_bf16, c, out, where, 3, bias, nullptr);
 }
 
+bool tc_batch_sum_f32(uint64_t batch, uint64_t m, uint64_t n, uint64_t k, const float* a, const float* b, float* out, const char* where) {
+    TcProduct c;
+    c.A = reinterpret_cast<const char*>(a);
+    c.B = reinterpret_cast<const char*>(b);
+    c.a_mn = c.b_mn = false;
+    c.m = m;
+    c.n = n;
+    c.k = k;
+    c.batch = batch;
+    c.a_bs = (int64_t)(m * k);
+    c.b_bs = (int64_t)(n * k);
+    c.sum_batches = true;
+    return batch * k <= 0x7FFFFFFFull && eligible(4, m, n, k, batch, false, false, a, b, out) && tc_launch_f32(c, out, where);
+}
+
 bool tc_gemm_bf16_f16(bool is_bf16, const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out,
                       const char* where) {
     TcProduct c;

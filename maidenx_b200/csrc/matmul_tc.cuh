@@ -19,6 +19,7 @@ struct TcProduct {
     uint64_t a_pitch = 0, b_pitch = 0;        // elements between rows of a copied operand (0: dense)
     bool a_repack = false, b_repack = false;  // the operand has to be copied to 16-byte-multiple rows first
     bool ragged = false;                      // a product tc_classify leaves to the CUDA cores
+    bool sum_batches = false;                 // D is one [m, n] matrix, the sum of the batches' products
     int d_plain = 0;                          // the output is written without tensor stores: 1 element-wise, 2 in pairs
 };
 // which: 0 forward, 1 grad_a, 2 grad_b (see matmul_tc.cu); elem_size in bytes.
@@ -41,6 +42,10 @@ bool tc_linear_bias_act(bool is_bf16, uint64_t rows, uint64_t in_features, uint6
 // form of a convolution's forward pass over its column buffer.  false = not taken by the tensor-core kernel, nothing launched.
 bool tc_batched_row_bias(bool is_bf16, uint64_t batch, uint64_t rows, uint64_t k, uint64_t n, const void* w, const void* cols, const void* bias, void* out,
                          const char* where);
+// out[m, n] = sum_b a[b][m, k] . b[b][n, k]^T over the whole batch in one reduction: the weight gradient of a convolution.
+// false = not taken (rows of k or n that are not 16-byte multiples, a small product).
+bool tc_batch_sum_f32(uint64_t batch, uint64_t m, uint64_t n, uint64_t k, const float* a, const float* b, float* out, const char* where);
+bool tc_launch_f32(const TcProduct& c, void* out, const char* where);
 bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out, const char* where);
 
 template <class T>

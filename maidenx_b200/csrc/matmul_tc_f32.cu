@@ -96,6 +96,7 @@ struct Params {
     int stages;     // of the ring
     int raw_bytes;  // what TMA delivers per stage: A and bn rows of B
     int split_kb;   // > 0: split-K; batch s of the launch reduces the k-blocks [s * split_kb, (s + 1) * split_kb) of one product
+    int kb_per_z;   // > 0: the reduction runs over the operands' batches too: k-block i is block i % kb_per_z of batch i / kb_per_z
     int d_plain;    // != 0: the output's rows (or base) are not 16-byte multiples: the epilogue warps write them to `d` themselves
     float* d;
 };
@@ -169,8 +170,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
                 int tm, tn, tb;
                 tile_coords(tile, p, tm, tn, tb);
-                const int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
-                const int k_base = tb * p.split_kb * BK;  // a k-block past the end of K is all fill: zeros
+                int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
                 for (int kb = 0; kb < p.num_kb; kb++) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, err, tag, 1)) {
                         ok = false;
@@ -179,16 +179,22 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     mbar_expect_tx(full_bar(stage), p.raw_bytes);
                     const uint32_t sa = smem_base + Smem::stages + stage * 2 * p.raw_bytes;
                     const uint32_t sb = sa + A_TILE;
+                    int block = tb * p.split_kb + kb;  // a block past the end of K (or of the batches) is all fill: zeros
+                    if (p.kb_per_z) {
+                        za = zb = block / p.kb_per_z;
+                        block -= za * p.kb_per_z;
+                    }
+                    const int k = block * BK;
                     if (!p.a_mn) {
-                        tma_load_3d(sa, &map_a, k_base + kb * BK, tm * BM, za, full_bar(stage));
+                        tma_load_3d(sa, &map_a, k, tm * BM, za, full_bar(stage));
                     } else {
 #pragma unroll
-                        for (int h = 0; h < BM / 32; h++) tma_load_3d(sa + h * MN_CHUNK_BYTES, &map_a, tm * BM + h * 32, k_base + kb * BK, za, full_bar(stage));
+                        for (int h = 0; h < BM / 32; h++) tma_load_3d(sa + h * MN_CHUNK_BYTES, &map_a, tm * BM + h * 32, k, za, full_bar(stage));
                     }
                     if (!p.b_mn) {
-                        tma_load_3d(sb, &map_b, k_base + kb * BK, tn * p.bn, zb, full_bar(stage));
+                        tma_load_3d(sb, &map_b, k, tn * p.bn, zb, full_bar(stage));
                     } else {
-                        for (int h = 0; h < p.bn / 32; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * p.bn + h * 32, k_base + kb * BK, zb, full_bar(stage));
+                        for (int h = 0; h < p.bn / 32; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * p.bn + h * 32, k, zb, full_bar(stage));
                     }
                     if (++stage == p.stages) {
                         stage = 0;
@@ -438,13 +444,19 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.tiles_n = (int)((N + p.bn - 1) / p.bn);
     p.num_kb = (int)((K + BK - 1) / BK);
     p.split_kb = 0;
+    p.kb_per_z = 0;
+    if (c.sum_batches) {
+        p.kb_per_z = p.num_kb;
+        p.num_kb *= (int)batch;
+        batch = 1;
+    }
     int grid = sm_count();
     if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
     // few output tiles: cut K into slices that run as the batches of this launch (see tc_ptx.cuh)
     int slices = 1;
     const int bn_whole = tile_columns((uint64_t)p.tiles_m, N, batch, grid);
     if (batch == 1) {
-        slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
+        if (!c.sum_batches) slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
         if (slices == 1)
             slices = splitk_short((uint64_t)p.tiles_m * p.tiles_n, (uint64_t)p.num_kb, grid, (128 + p.bn) / 256.0,
                                   tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, grid) * p.num_kb - kSplitFixed32);
@@ -488,6 +500,8 @@ bool launch(const TcProduct& c, void* D, const char* where) {
 }
 
 }  // namespace
+
+bool tc_launch_f32(const TcProduct& c, void* out, const char* where) { return launch(c, out, where); }
 
 bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out, const char* where) {
     TcProduct c;

@@ -152,3 +152,27 @@ def test_bias_in_the_product_epilogue_equals_the_separate_add(cuda, dt, shape):
     assert np.array_equal(got["out"], ref["out"])
     for key in ("grad_x", "grad_w", "grad_bias"):
         assert np.array_equal(got[key], ref[key]), key
+
+
+# large enough for the tensor cores, with maps whose rows are no 16-byte multiples (14 x 14, 7 x 7) and regular ones
+RAGGED_TC = [
+    (5, 24, 14, 14, 136, 3, 3, 1, 1, 1, 1),
+    (6, 24, 12, 12, 136, 3, 3, 1, 1, 1, 1),   # P = 144: the weight gradient is one product over batch and positions
+    (40, 24, 7, 7, 72, 3, 3, 1, 1, 1, 1),
+    (10, 16, 15, 15, 72, 5, 5, 2, 2, 2, 2),
+    (33, 64, 8, 8, 40, 1, 1, 1, 1, 0, 0),     # many batches of one k-block each, split over CTAs
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("shape", RAGGED_TC, ids=lambda s: "x".join(map(str, s)))
+def test_direct_layer_on_ragged_maps(cuda, dt, shape):
+    """Bounds: f32 1e-5 of the sums' scale (split-tf32 products, f32 sums); 16-bit out and gradients carry at most the
+    roundings of the product and of the sum of kh * kw terms."""
+    x, w, b, g = _data(15, dt, shape)
+    got = CC.run_layer(dt, 1, shape, x, w, b, g)
+    ref = CC.direct_conv_f64(shape, D.decode(x, dt), D.decode(w, dt), D.decode(b, dt), D.decode(g, dt))
+    sc = _scales(shape)
+    for key in ("out", "grad_x", "grad_w", "grad_bias"):
+        H.assert_same("conv2d", dt, got[key], D.encode(ref[key], dt), float_rel={"f32": 1e-5}.get(dt.name, 2e-2), what=key, scale=sc[key])
