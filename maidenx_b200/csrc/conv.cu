@@ -4,13 +4,13 @@
 //   metadata = [B, C, H, W, kh, kw, out_h, out_w, pad_h, pad_w, stride_h, stride_w]
 //   col layout [B][C, kh, kw][out_h, out_w]
 //
-// im2col: one block per (b, c) image plane.  The plane is read once into shared memory
-// with coalesced loads; each of the kh*kw shifted copies is then written as one contiguous
-// run of out_h*out_w elements with 16-byte stores.  DRAM traffic is the algorithmic
+// im2col: a block takes a few neighbouring (b, c) image planes.  They are read once into shared memory
+// with coalesced loads; the kh*kw shifted copies of all of them are one contiguous run of the column buffer, written
+// with 16-byte stores.  DRAM traffic is the algorithmic
 // minimum (input once + col once) where the reference re-reads the input kh*kw times.
 //
-// col2im: gather formulation, one thread per output pixel summing the (at most kh*kw) col
-// entries that map to it in the reference's (h_out, w_out) order and in the element type,
+// col2im: gather formulation, the column planes of a few image planes staged in shared memory and one thread per
+// output pixel summing the (at most kh*kw) col entries that map to it in the reference's (h_out, w_out) order and in the element type,
 // so the result is bit-identical to the CPU backend, deterministic, needs no atomics and
 // overwrites the output (the reference's CUDA kernel scatters with atomicAdd into a
 // pre-zeroed buffer).  `num_els` bounds the readable part of col: entries at or beyond it
@@ -28,23 +28,80 @@ namespace mx {
 struct ConvParams {
     uint32_t B, C, H, W, KH, KW, OH, OW, PH, PW, SH, SW;
     uint64_t num_els;
-    FastDiv ow_div, w_div;
+    uint32_t planes, per_block;  // planes written, planes of one block (staged kernels)
+    FastDiv ow_div, w_div, ohw_div, hw_div, kk_div, kw_div, sh_div, sw_div;
 };
 
 constexpr int kConvThreads = 256;
 
-template <class T, int VEC, bool STAGED>
-__global__ void __launch_bounds__(kConvThreads) im2col_kernel(const T* __restrict__ x, T* __restrict__ col, ConvParams P) {
+// `count` consecutive elements into shared memory, as 16-byte vectors where the source allows.
+template <class T>
+__device__ __forceinline__ void stage_run(T* dst, const T* __restrict__ src, uint32_t count) {
+    constexpr uint32_t VEC = 16 / sizeof(T);
+    uint32_t done = 0;
+    if ((uintptr_t)src % 16 == 0) {
+        done = count / VEC * VEC;
+        for (uint32_t i = threadIdx.x * VEC; i < done; i += kConvThreads * VEC) *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
+    }
+    for (uint32_t i = done + threadIdx.x; i < count; i += kConvThreads) dst[i] = src[i];
+}
+
+// The block's planes share one flat index over [plane, kh, kw, out_h, out_w], a thread takes VEC consecutive columns of it from
+// one index computation and walks on from there, so that small maps (14 x 14: 49 vectors of a plane's 441) keep every thread
+// busy and ragged ones (7 x 7) are written as vectors too.  Bound by HBM / L2 writes: [32, 128, 14, 14] f32, 3 x 3: 12 us, 23 with one
+// plane and one kernel offset at a time.
+template <class T, int VEC>
+__global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* __restrict__ x, T* __restrict__ col, ConvParams P) {
     extern __shared__ __align__(16) unsigned char conv_smem[];
-    T* plane = reinterpret_cast<T*>(conv_smem);
+    T* img = reinterpret_cast<T*>(conv_smem);
+    const uint32_t bc0 = blockIdx.x * P.per_block, np = min(P.per_block, P.planes - bc0);
+    const uint32_t HW = P.H * P.W, OHW = P.OH * P.OW, KK = P.KH * P.KW;
+    stage_run(img, x + (uint64_t)bc0 * HW, np * HW);
+    __syncthreads();
+    const T zero = zero_of<T>();
+    const uint64_t base = (uint64_t)bc0 * KK * OHW;
+    const uint32_t total = (uint32_t)min((uint64_t)np * KK * OHW, P.num_els - base);
+    for (uint32_t e = threadIdx.x * VEC; e < total; e += kConvThreads * VEC) {
+        uint32_t row, o, plane, kk, kh, kw, ho, wo;
+        P.ohw_div.divmod(e, row, o);
+        P.kk_div.divmod(row, plane, kk);
+        P.kw_div.divmod(kk, kh, kw);
+        P.ow_div.divmod(o, ho, wo);
+        Vec<T, VEC> r;
+#pragma unroll
+        for (int j = 0; j < VEC; j++) {
+            const int hi = (int)(ho * P.SH + kh) - (int)P.PH, wi = (int)(wo * P.SW + kw) - (int)P.PW;
+            r.v[j] = (uint32_t)hi < P.H && (uint32_t)wi < P.W && plane < np ? img[plane * HW + hi * P.W + wi] : zero;
+            if (VEC > 1 && ++wo == P.OW) {
+                wo = 0;
+                if (++ho == P.OH) {
+                    ho = 0;
+                    if (++kw == P.KW) {
+                        kw = 0;
+                        if (++kh == P.KH) {
+                            kh = 0;
+                            plane++;
+                        }
+                    }
+                }
+            }
+        }
+        if (e + VEC <= total) {
+            *reinterpret_cast<Vec<T, VEC>*>(col + base + e) = r;
+        } else {
+#pragma unroll
+            for (int j = 0; j < VEC; j++)
+                if (e + j < total) col[base + e + j] = r.v[j];
+        }
+    }
+}
+
+// Planes too large for shared memory: one block per plane, the input read in place.
+template <class T, int VEC>
+__global__ void __launch_bounds__(kConvThreads) im2col_kernel(const T* __restrict__ x, T* __restrict__ col, ConvParams P) {
     const uint64_t bc = blockIdx.x;  // b * C + c
     const uint32_t HW = P.H * P.W, OHW = P.OH * P.OW, KK = P.KH * P.KW;
-    const T* src = x + bc * HW;
-    if constexpr (STAGED) {
-        for (uint32_t i = threadIdx.x; i < HW; i += kConvThreads) plane[i] = src[i];
-        __syncthreads();
-    }
-    const T* img = STAGED ? plane : src;
+    const T* img = x + bc * HW;
     const T zero = zero_of<T>();
     const uint64_t out_base = bc * KK * OHW;
     const uint32_t nvec = (OHW + VEC - 1) / VEC;
@@ -82,6 +139,44 @@ template <class T>
 __device__ __forceinline__ T conv_add(T a, T b) {
     if constexpr (is_half_v<T>) return from_f32<T>(to_f32(a) + to_f32(b));
     else return a + b;
+}
+
+// The same sums from shared memory: the KH * KW column planes of the block's image planes arrive in one contiguous run; a
+// column entry crosses from L2 once instead of once per term.  UNIT: strides of 1.  [32, 128, 14, 14] f32, 3 x 3: 15 us, 18 from L2.
+template <class T, bool UNIT>
+__global__ void __launch_bounds__(kConvThreads) col2im_planes_kernel(const T* __restrict__ col, T* __restrict__ out, ConvParams P) {
+    extern __shared__ __align__(16) unsigned char conv_smem[];
+    T* cols = reinterpret_cast<T*>(conv_smem);
+    const uint32_t bc0 = blockIdx.x * P.per_block, np = min(P.per_block, P.planes - bc0);
+    const uint32_t HW = P.H * P.W, OHW = P.OH * P.OW, KK = P.KH * P.KW;
+    const uint64_t base = (uint64_t)bc0 * KK * OHW;
+    const uint32_t want = np * KK * OHW, have = base >= P.num_els ? 0 : (uint32_t)min((uint64_t)want, P.num_els - base);
+    stage_run(cols, col + base, have);
+    for (uint32_t i = have + threadIdx.x; i < want; i += kConvThreads) cols[i] = zero_of<T>();  // adding +0 is skipping: the sum is never -0
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < np * HW; i += kConvThreads) {
+        uint32_t plane, pix, h, w;
+        P.hw_div.divmod(i, plane, pix);
+        P.w_div.divmod(pix, h, w);
+        const uint32_t hp = h + P.PH, wp = w + P.PW;
+        // conv.rs:121-125
+        const uint32_t hs0 = hp >= P.KH - 1 ? hp - (P.KH - 1) : 0, ws0 = wp >= P.KW - 1 ? wp - (P.KW - 1) : 0;
+        const uint32_t hs = UNIT ? hs0 : P.sh_div.div(hs0 + P.SH - 1), ws = UNIT ? ws0 : P.sw_div.div(ws0 + P.SW - 1);
+        const uint32_t he = min((UNIT ? hp : P.sh_div.div(hp)) + 1, P.OH), we = min((UNIT ? wp : P.sw_div.div(wp)) + 1, P.OW);
+        const uint32_t SH = UNIT ? 1 : P.SH, SW = UNIT ? 1 : P.SW;
+        const T* mine = cols + plane * KK * OHW;
+        T sum = zero_of<T>();
+        for (uint32_t ho = hs; ho < he; ho++) {
+            const uint32_t kh = hp - ho * SH;
+            if (kh >= P.KH) continue;
+            const T* row = mine + kh * P.KW * OHW + ho * P.OW;
+            for (uint32_t wo = ws; wo < we; wo++) {
+                const uint32_t kw = wp - wo * SW;
+                if (kw < P.KW) sum = conv_add(sum, row[kw * OHW + wo]);
+            }
+        }
+        out[(uint64_t)bc0 * HW + i] = sum;
+    }
 }
 
 template <class T>
@@ -139,7 +234,25 @@ static bool conv_params(const size_t* meta, size_t num_els, ConvParams& P, const
     }
     P.ow_div.init(P.OW);
     P.w_div.init(P.W);
+    P.ohw_div.init(P.OH * P.OW);
+    P.hw_div.init(P.H * P.W);
+    P.kk_div.init(P.KH * P.KW);
+    P.kw_div.init(P.KW);
+    P.sh_div.init(P.SH);
+    P.sw_div.init(P.SW);
     return true;
+}
+
+// Planes of one block of the staged kernels: up to 16 KB of them in shared memory (at least one), so that a block has a few
+// vectors or pixels per thread, but not so many that fewer than eight blocks per SM (all its threads) are left;
+// a multiple of `step`.  0: not even `step` planes fit `most` bytes.
+static uint32_t planes_per_block(uint64_t planes, uint64_t plane_bytes, uint64_t step, uint64_t most) {
+    if (step * plane_bytes > most) return 0;
+    uint64_t n = 16 * 1024 / plane_bytes;
+    const uint64_t spread = planes / (8 * (uint64_t)sm_count());
+    if (n > spread) n = spread;
+    n = n / step * step;
+    return (uint32_t)(n < step ? step : n);
 }
 
 template <class T>
@@ -187,16 +300,25 @@ void im2col_entry(size_t num_els, const size_t* meta, const T* x, T* col, const 
             }
         }
     }
-    if (plane_bytes <= 200 * 1024) {
+    // a block's columns start on a vector boundary when its planes' chunks add up to whole vectors
+    uint64_t step = 1;
+    while (step < VEC && (chunk * step) % VEC != 0) step *= 2;
+    const bool col_aligned = (uintptr_t)col % 16 == 0;
+    const uint32_t pb_vec = col_aligned ? planes_per_block(planes_touched, plane_bytes, step, step == 1 ? 200 * 1024 : 48 * 1024) : 0;
+    const uint32_t pb = pb_vec ? pb_vec : planes_per_block(planes_touched, plane_bytes, 1, 200 * 1024);
+    if (pb && pb * chunk < 0x7FFFFFFFull) {
+        P.planes = (uint32_t)planes_touched;
+        P.per_block = pb;
+        const size_t smem = pb * plane_bytes;
         auto launch = [&](auto kernel) {
-            if (plane_bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_bytes);
-            kernel<<<grid, kConvThreads, plane_bytes, s>>>(x, col, P);
+            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            kernel<<<(unsigned)((planes_touched + pb - 1) / pb), kConvThreads, smem, s>>>(x, col, P);
         };
-        if (vec) launch(im2col_kernel<T, VEC, true>);
-        else launch(im2col_kernel<T, 1, true>);
+        if (pb_vec) launch(im2col_planes_kernel<T, VEC>);
+        else launch(im2col_planes_kernel<T, 1>);
     } else {
-        if (vec) im2col_kernel<T, VEC, false><<<grid, kConvThreads, 0, s>>>(x, col, P);
-        else im2col_kernel<T, 1, false><<<grid, kConvThreads, 0, s>>>(x, col, P);
+        if (vec) im2col_kernel<T, VEC><<<grid, kConvThreads, 0, s>>>(x, col, P);
+        else im2col_kernel<T, 1><<<grid, kConvThreads, 0, s>>>(x, col, P);
     }
     check_launch(where);
 }
@@ -255,6 +377,21 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
                 return;
             }
         }
+    }
+    const uint64_t col_plane = (uint64_t)P.KH * P.KW * P.OH * P.OW;
+    const uint32_t pb = planes <= 0x7FFFFFFFull && col_plane && HW < 0x7FFFFFFFull ? planes_per_block(planes, col_plane * sizeof(T), 1, 100 * 1024) : 0;
+    if (pb && pb * HW < 0x7FFFFFFFull) {
+        P.planes = (uint32_t)planes;
+        P.per_block = pb;
+        const size_t smem = pb * col_plane * sizeof(T);
+        auto launch = [&](auto kernel) {
+            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            kernel<<<(unsigned)((planes + pb - 1) / pb), kConvThreads, smem, s>>>(col, out, P);
+        };
+        if (P.SH == 1 && P.SW == 1) launch(col2im_planes_kernel<T, true>);
+        else launch(col2im_planes_kernel<T, false>);
+        check_launch(where);
+        return;
     }
     // grid.y carries the plane index; fold very large plane counts into several launches
     const unsigned gx = (unsigned)((HW + kConvThreads - 1) / kConvThreads);

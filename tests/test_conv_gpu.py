@@ -85,3 +85,29 @@ def test_im2col_col2im_adjoint(cuda):
     cx = H.run_im2col(cuda, dt, meta, ncol, x)
     ty = H.run_col2im(cuda, dt, meta, ncol, y, x.size)
     assert np.isclose(np.dot(cx, y), np.dot(x, ty), rtol=1e-12)
+
+
+MANY_PLANES = [
+    # name, B, C, H, W, kh, kw, ph, pw, sh, sw: enough planes for several per block, maps that are whole vectors and maps that are not
+    ("14x14", 7, 131, 14, 14, 3, 3, 1, 1, 1, 1),
+    ("7x7-s2", 5, 211, 7, 7, 3, 3, 1, 1, 2, 2),
+    ("9x11-5x5", 3, 300, 9, 11, 5, 5, 2, 2, 1, 1),
+    ("1x1-odd", 4, 401, 5, 5, 1, 1, 0, 0, 1, 1),
+    ("even-kernel", 3, 257, 6, 10, 2, 4, 1, 0, 1, 3),
+    ("plane-beyond-shared-memory", 1, 2, 170, 331, 3, 3, 1, 1, 2, 2),
+]
+
+
+@pytest.mark.parametrize("dt", D.FLOATS, ids=lambda d: d.name)
+@pytest.mark.parametrize("case", MANY_PLANES, ids=lambda c: c[0])
+def test_planes_sharing_a_block(oracle, cuda, dt, case):
+    """Bit-exact like every case of this file; also column buffers that end inside a plane (num_els)."""
+    rng = np.random.default_rng(34)
+    B, C, Hh, W, kh, kw, oh, ow, ph, pw, sh, sw = _geom(case)
+    meta = H.conv_metadata(B, C, Hh, W, kh, kw, oh, ow, ph, pw, sh, sw)
+    ncol, out_len = B * C * kh * kw * oh * ow, B * C * Hh * W
+    x, col = H.random_store(rng, dt, out_len, dist="normal"), H.random_store(rng, dt, ncol, dist="normal")
+    for n in (ncol, ncol - kh * kw * oh * ow // 2 - 1):
+        H.assert_same("conv2d_im2col", dt, H.run_im2col(cuda, dt, meta, n, x), H.run_im2col(oracle, dt, meta, n, x), what=f"{case[0]} {n}")
+    for n in (ncol, ncol // 2 + 1):
+        H.assert_same("conv2d_col2im", dt, H.run_col2im(cuda, dt, meta, n, col, out_len), H.run_col2im(oracle, dt, meta, n, col, out_len), what=f"{case[0]} {n}")
