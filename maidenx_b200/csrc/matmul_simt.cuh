@@ -48,117 +48,93 @@ __device__ __forceinline__ T mm_store(typename MmAcc<T>::type a) {
     else return (T)a;
 }
 
-constexpr int kMmTile = 64;   // output tile edge
-constexpr int kMmK = 16;      // reduction step
 constexpr int kMmThreads = 256;
 
-template <class T>
-__global__ void __launch_bounds__(kMmThreads) matmul_simt_kernel(const T* __restrict__ X, const T* __restrict__ Y, T* __restrict__ out, MmParams P) {
+// TILE x TILE outputs of one batch per block: 64 (4 x 4 per thread), or 32 (2 x 2) for products whose 64-wide tiles would leave
+// most SMs without a block.  Row and batch are resolved once per loaded element, not once per k-step (a 64-bit division each), and
+// the next k-step's operands are on their way from memory while the current one is multiplied.  Bound by that latency
+// for small products, by the separate multiply and add for large ones.  f32: 64 x 64 x 512 17 us (163 before), 256 x 256 x 128 5.8 (42).
+template <class T, int TILE>
+__global__ void __launch_bounds__(kMmThreads) matmul_simt_kernel(const T* __restrict__ X, const T* __restrict__ Y, T* __restrict__ out, MmParams P, uint32_t tiles_m, uint64_t first) {
     typedef typename MmAcc<T>::type Acc;
-    __shared__ Acc xs[kMmK][kMmTile + 1];  // [r][row]
-    __shared__ Acc ys[kMmK][kMmTile + 1];  // [r][col]
-    const uint64_t row0 = (uint64_t)blockIdx.x * kMmTile, col0 = (uint64_t)blockIdx.y * kMmTile;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
-    Acc acc[4][4];
+    constexpr int kMmK = TILE == 32 ? (sizeof(Acc) == 8 ? 32 : 64) : 16;  // reduction step: the narrow tile is for products with few blocks, which wait for memory once per step
+    constexpr int PER = TILE / 16, LOADS = TILE * kMmK / kMmThreads;
+    __shared__ Acc xs[2][kMmK][TILE + 1];  // [buffer][r][row]
+    __shared__ Acc ys[2][kMmK][TILE + 1];  // [buffer][r][col]
+    const uint64_t batch = (first + blockIdx.x) / tiles_m;
+    const uint64_t m0 = (first + blockIdx.x) % tiles_m * TILE, col0 = (uint64_t)blockIdx.y * TILE;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads; rows ty + 16 i, columns tx + 16 j
+    Acc acc[PER][PER];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < PER; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = (Acc)0;
+        for (int j = 0; j < PER; j++) acc[i][j] = (Acc)0;
 
     // loader mapping: pick the fast index along the operand's smaller stride
     const bool x_r_fast = (P.xs_r <= P.xs_m) || P.xs_m == 0;
     const bool y_c_fast = (P.ys_c <= P.ys_r) || P.ys_r == 0;
-
-    for (uint64_t k0 = 0; k0 < P.K; k0 += kMmK) {
+    uint64_t ix[LOADS], iy[LOADS];       // element index at the k-step to be loaded next
+    int xr[LOADS], yr[LOADS];            // its r inside the step; -1: a row or column outside the matrix
+    int xo[LOADS], yo[LOADS];            // its row or column inside the tile
 #pragma unroll
-        for (int it = 0; it < (kMmTile * kMmK) / kMmThreads; it++) {
-            int e = threadIdx.x + it * kMmThreads;
-            int lr, lrow;
-            if (x_r_fast) {
-                lr = e % kMmK;
-                lrow = e / kMmK;
-            } else {
-                lrow = e % kMmTile;
-                lr = e / kMmTile;
-            }
-            uint64_t row = row0 + lrow, r = k0 + lr;
-            Acc v = (Acc)0;
-            if (row < P.rows && r < P.K) {
-                uint64_t batch = row / P.M, mi = row % P.M;
-                uint64_t ix = (uint64_t)((int64_t)batch * P.xs_b + (int64_t)mi * P.xs_m + (int64_t)r * P.xs_r);
-                if (ix < P.x_limit) v = mm_load<T>(X[ix]);
-            }
-            xs[lr][lrow] = v;
+    for (int it = 0; it < LOADS; it++) {
+        const int e = threadIdx.x + it * kMmThreads;
+        const int r = x_r_fast ? e % kMmK : e / TILE, row = x_r_fast ? e / kMmK : e % TILE;
+        const uint64_t mi = m0 + row;
+        xo[it] = r * (TILE + 1) + row;
+        xr[it] = mi < P.M && batch * P.M + mi < P.rows ? r : -1;
+        ix[it] = (uint64_t)((int64_t)batch * P.xs_b + (int64_t)mi * P.xs_m + (int64_t)r * P.xs_r);
+        const int yrr = y_c_fast ? e / TILE : e % kMmK, col = y_c_fast ? e % TILE : e / kMmK;
+        yo[it] = yrr * (TILE + 1) + col;
+        yr[it] = col0 + col < P.N ? yrr : -1;
+        iy[it] = (uint64_t)((int64_t)batch * P.ys_b + (int64_t)yrr * P.ys_r + (int64_t)(col0 + col) * P.ys_c);
+    }
+    Acc xv[LOADS], yv[LOADS];
+    auto load = [&](uint64_t k0) {
+#pragma unroll
+        for (int it = 0; it < LOADS; it++) {
+            xv[it] = xr[it] >= 0 && k0 + xr[it] < P.K && ix[it] < P.x_limit ? mm_load<T>(X[ix[it]]) : (Acc)0;
+            yv[it] = yr[it] >= 0 && k0 + yr[it] < P.K && iy[it] < P.y_limit ? mm_load<T>(Y[iy[it]]) : (Acc)0;
+            ix[it] += (uint64_t)(kMmK * P.xs_r);
+            iy[it] += (uint64_t)(kMmK * P.ys_r);
         }
+    };
+    load(0);
+    int buf = 0;
+    for (uint64_t k0 = 0; k0 < P.K; k0 += kMmK, buf ^= 1) {
+        Acc* xt = &xs[buf][0][0];
+        Acc* yt = &ys[buf][0][0];
 #pragma unroll
-        for (int it = 0; it < (kMmTile * kMmK) / kMmThreads; it++) {
-            int e = threadIdx.x + it * kMmThreads;
-            int lr, lcol;
-            if (y_c_fast) {
-                lcol = e % kMmTile;
-                lr = e / kMmTile;
-            } else {
-                lr = e % kMmK;
-                lcol = e / kMmK;
-            }
-            // the batch of a tile row is needed for Y too; rows of one tile may span batches,
-            // so Y is staged per (r, col) for the batch of the tile's FIRST row and re-read
-            // directly for rows of other batches (rare: only when M is not a multiple of 64)
-            uint64_t col = col0 + lcol, r = k0 + lr;
-            Acc v = (Acc)0;
-            if (col < P.N && r < P.K) {
-                uint64_t batch = row0 / P.M;
-                uint64_t iy = (uint64_t)((int64_t)batch * P.ys_b + (int64_t)r * P.ys_r + (int64_t)col * P.ys_c);
-                if (iy < P.y_limit) v = mm_load<T>(Y[iy]);
-            }
-            ys[lr][lcol] = v;
+        for (int it = 0; it < LOADS; it++) {
+            xt[xo[it]] = xv[it];
+            yt[yo[it]] = yv[it];
         }
-        __syncthreads();
-        const uint64_t batch0 = row0 / P.M;
+        __syncthreads();  // one per step: the buffer written next was last read before the previous step's barrier
+        if (k0 + kMmK < P.K) load(k0 + kMmK);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            uint64_t row = row0 + ty * 4 + i;
-            if (row >= P.rows) continue;
-            uint64_t batch = row / P.M;
-            if (batch == batch0) {
+        for (int kk = 0; kk < kMmK; kk++) {
+            Acc xk[PER], yk[PER];
 #pragma unroll
-                for (int kk = 0; kk < kMmK; kk++) {
-                    Acc xv = xs[kk][ty * 4 + i];
+            for (int i = 0; i < PER; i++) {
+                xk[i] = xs[buf][kk][ty + 16 * i];
+                yk[i] = ys[buf][kk][tx + 16 * i];
+            }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        if constexpr (is_half_v<T>) acc[i][j] = fmaf(xv, ys[kk][tx * 4 + j], acc[i][j]);  // product exact in f32
-                        else acc[i][j] = acc[i][j] + xv * ys[kk][tx * 4 + j];
-                    }
+            for (int i = 0; i < PER; i++)
+#pragma unroll
+                for (int j = 0; j < PER; j++) {
+                    if constexpr (is_half_v<T>) acc[i][j] = fmaf(xk[i], yk[j], acc[i][j]);  // product exact in f32
+                    else acc[i][j] = acc[i][j] + xk[i] * yk[j];
                 }
-            } else {
-                // this row belongs to a later batch than the staged Y tile: read Y directly
-                for (int kk = 0; kk < kMmK; kk++) {
-                    uint64_t r = k0 + kk;
-                    if (r >= P.K) break;
-                    Acc xv = xs[kk][ty * 4 + i];
-                    for (int j = 0; j < 4; j++) {
-                        uint64_t col = col0 + tx * 4 + j;
-                        Acc yv = (Acc)0;
-                        if (col < P.N) {
-                            uint64_t iy = (uint64_t)((int64_t)batch * P.ys_b + (int64_t)r * P.ys_r + (int64_t)col * P.ys_c);
-                            if (iy < P.y_limit) yv = mm_load<T>(Y[iy]);
-                        }
-                        if constexpr (is_half_v<T>) acc[i][j] = fmaf(xv, yv, acc[i][j]);
-                        else acc[i][j] = acc[i][j] + xv * yv;
-                    }
-                }
-            }
         }
-        __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        uint64_t row = row0 + ty * 4 + i;
-        if (row >= P.rows) continue;
+    for (int i = 0; i < PER; i++) {
+        const uint64_t mi = m0 + ty + 16 * i, row = batch * P.M + mi;
+        if (mi >= P.M || row >= P.rows) continue;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            uint64_t col = col0 + tx * 4 + j;
-            uint64_t o = row * P.N + col;
+        for (int j = 0; j < PER; j++) {
+            const uint64_t col = col0 + tx + 16 * j, o = row * P.N + col;
             if (col < P.N && o < P.out_elems) out[o] = mm_store<T>(acc[i][j]);
         }
     }
@@ -222,14 +198,22 @@ void mm_launch(const MmParams& P, const T* X, const T* Y, T* out, const char* wh
         check_launch(where);
         return;
     }
-    uint64_t gx = (P.rows + kMmTile - 1) / kMmTile, gy = (P.N + kMmTile - 1) / kMmTile;
-    if (gy > 65535 || gx > 0x7FFFFFFFull) {  // more than 4M output columns
-        set_error(kErrUnsupported, 0, where);
-        return;
-    }
-    dim3 grid((unsigned)gx, (unsigned)gy);
-    matmul_simt_kernel<T><<<grid, kMmThreads, 0, ctx().stream>>>(X, Y, out, P);
-    check_launch(where);
+    const uint64_t batches = (P.rows + P.M - 1) / P.M;
+    auto go = [&](auto kernel, uint64_t tile) {
+        const uint64_t tiles_m = ((P.M < P.rows ? P.M : P.rows) + tile - 1) / tile, gx = batches * tiles_m, gy = (P.N + tile - 1) / tile;
+        if (gy > 65535) {  // more than 4M output columns
+            set_error(kErrUnsupported, 0, where);
+            return;
+        }
+        for (uint64_t first = 0; first < gx; first += 0x7FFFFFFFull) {
+            const uint64_t count = gx - first < 0x7FFFFFFFull ? gx - first : 0x7FFFFFFFull;
+            kernel<<<dim3((unsigned)count, (unsigned)gy), kMmThreads, 0, ctx().stream>>>(X, Y, out, P, (uint32_t)tiles_m, first);
+        }
+        check_launch(where);
+    };
+    const uint64_t m = P.M < P.rows ? P.M : P.rows;
+    if (batches * ((m + 63) / 64) * ((P.N + 63) / 64) < (uint64_t)sm_count()) go(matmul_simt_kernel<T, 32>, 32);
+    else go(matmul_simt_kernel<T, 64>, 64);
 }
 
 }  // namespace mx

@@ -961,18 +961,21 @@ extern "C" int mx_debug_tc_gemm_poke_status(int value) {
 namespace mx {
 
 // Sizes the tensor-core kernels can index and are worth a persistent launch for.
-static bool in_range(uint64_t M, uint64_t N, uint64_t K, uint64_t batch) {
+// `least`: multiply-adds from which on.
+constexpr uint64_t kTcLeast = 1ull << 24;
+static bool in_range(uint64_t M, uint64_t N, uint64_t K, uint64_t batch, uint64_t least = kTcLeast) {
     if (M == 0 || N == 0 || K == 0) return false;
     if (M > 0x7FFFFFFFull || N > 0x7FFFFFFFull || K > 0x7FFFFFFFull) return false;
     if (batch > 0x7FFFull) return false;
-    if (batch * M * N * K < (1ull << 24)) return false;  // small problems are not worth a persistent launch
+    if (batch * M * N * K < least) return false;  // small problems are not worth a persistent launch
     return batch * ((M + 127) / 128) * ((N + 63) / 64) <= 0x3FFFFFFFull;
 }
 // TMA wants 16-byte aligned bases and row pitches: the contiguous extent of every matrix (K for K-major
 // operands, MN for MN-major ones, N for D) must be a multiple of 16 / elem_size elements.
-static bool eligible(size_t es, uint64_t M, uint64_t N, uint64_t K, uint64_t batch, bool a_mn, bool b_mn, const void* a, const void* b, const void* d) {
+static bool eligible(size_t es, uint64_t M, uint64_t N, uint64_t K, uint64_t batch, bool a_mn, bool b_mn, const void* a, const void* b, const void* d,
+                     uint64_t least = kTcLeast) {
     const uint64_t q = 16 / es;
-    if (!in_range(M, N, K, batch)) return false;
+    if (!in_range(M, N, K, batch, least)) return false;
     if (N % q != 0) return false;
     if ((a_mn ? M : K) % q != 0 || (b_mn ? N : K) % q != 0) return false;
     if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)d) % 16 != 0) return false;
@@ -983,9 +986,9 @@ static bool eligible(size_t es, uint64_t M, uint64_t N, uint64_t K, uint64_t bat
 // 16-byte multiples is copied to padded rows first (repack_operands), an output like that is written by the epilogue warps
 // without tensor stores.  One pass over the operand against 8 TFLOP/s on the CUDA cores: bf16 4099 x 1543 x 1000, whose
 // 1543-wide matrices all need it, takes 20-40 us a product (1804 us on the CUDA cores).
-static bool plan_ragged(size_t es, TcProduct& c, const void* d) {
+static bool plan_ragged(size_t es, TcProduct& c, const void* d, uint64_t least = kTcLeast) {
     const uint64_t q = 16 / es;
-    if (!in_range(c.m, c.n, c.k, c.batch)) return false;
+    if (!in_range(c.m, c.n, c.k, c.batch, least)) return false;
     if (((uintptr_t)c.A | (uintptr_t)c.B | (uintptr_t)d) % es != 0) return false;
     const uint64_t a_cols = c.a_mn ? c.m : c.k, b_cols = c.b_mn ? c.n : c.k;
     c.a_repack = a_cols % q != 0 || (uintptr_t)c.A % 16 != 0;
@@ -1100,10 +1103,14 @@ bool tc_classify_any(const MmDesc& d, int which, size_t es, size_t num_els, size
                      TcProduct& c) {
     if (which == 0 ? !forward_operands(d, es, num_els, x, y, c) : !backward_operands(d, which, nea, neb, x, y, c)) return false;
     c.ragged = d.out_nd > (which == 0 ? 3 : 2);  // aligned, but new to these kernels: batches beyond rank 3, batched backward
-    if (aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out)) return true;
+    // 16-bit products far below kTcLeast still gain when their reduction is long: the CUDA-core kernel's time is its chain of
+    // k-steps (64 x 64 x 512: 22 us, 128 x 10 x 784: 33), the tensor-core kernel's about 4.5 us, 1.6 us more per copied operand.
+    // f32 keeps the line: below it results are bit for bit those of the element-type loop.
+    const uint64_t least = es == 2 && c.k >= 256 ? 1ull << 18 : kTcLeast;
+    if (aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out, least)) return true;
     // the copy reads whole operands: every batch must be there (a size-1 batch dim passes the contiguity test)
     if (which == 0 && c.batch > 1 && d.a_cont && d.b_cont && (d.a_elems != c.batch * c.m * c.k || d.b_elems != c.batch * c.k * c.n)) return false;
-    return plan_ragged(es, c, out);
+    return plan_ragged(es, c, out, least);
 }
 
 // x [rows, in] . w[out, in]^T with the bias add (and GELU) in the epilogue; false = shape not taken (the caller runs the ops one by one)
