@@ -126,7 +126,7 @@ extern "C" void mx_sum_f32_noalloc(size_t num_els, size_t num_dims, size_t num_r
         seg = (seg + VEC - 1) / VEC * VEC;
         splits = (R + seg - 1) / seg;
         if (O > 65535) {  // beyond the grid's row limit: one warp per row, no workspace
-            reduce_rows_group_kernel<f32, RED_SUM, 1, 32><<<(u32)((O + 7) / 8), kRedThreads, 0, s>>>(inp, out, O, R, pl.factor);
+            reduce_rows_warp_kernel<f32, RED_SUM, 1><<<(u32)((O + 7) / 8), kRedThreads, 0, s>>>(inp, out, O, R, pl.factor);
             check_launch(where);
             return;
         }

@@ -212,33 +212,59 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_block_kernel(const T*
     }
 }
 
-// G lanes of a warp per row (8 <= R < ~2048), G the smallest of 4, 8, 16, 32 that gives every vector of the row a lane: a
-// row of 56 bf16 is seven vectors, and a whole warp for it left 25 lanes idle (sum over the last dim of [64, 256, 56, 56] bf16
-// and the one after it: 124 us, now 55).  Four loads per lane in flight.
-template <class T, int KIND, int VEC, int G>
-__global__ void __launch_bounds__(kRedThreads) reduce_rows_group_kernel(const T* in, T* out, u64 rows, u64 R, u64 factor) {
+// G lanes of a warp per row (8 <= R <= 32 vectors), G the smallest of 4, 8, 16, 32 that gives every vector of the row a lane: a
+// row of 56 bf16 is seven vectors, and a whole warp for it left 25 lanes idle.  Q rows per group with their loads in flight
+// together: with one row a block of 256 threads lived for a single load (sums over the last two dims of [64, 256, 56, 56] bf16:
+// 124 us with a warp per row, 55 with eight lanes and one row, 32 with eight lanes and four).
+template <class T, int KIND, int VEC, int G, int Q>
+__global__ void __launch_bounds__(kRedThreads) reduce_rows_short_kernel(const T* in, T* out, u64 rows, u32 R, u64 factor) {
     typedef RedTraits<T, KIND> TR;
-    const u64 row = (u64)blockIdx.x * (kRedThreads / G) + threadIdx.x / G;
-    const bool live = row < rows;  // the shuffles below take the whole warp
-    const T* p = in + (live ? row : 0) * R;
-    typename TR::Acc acc = TR::init();
-    if (live) {
-        constexpr int STEP = G * VEC;
-        for (u64 i = (threadIdx.x % G) * VEC; i < R; i += 4 * STEP) {
-            Vec<T, VEC> v[4];
+    constexpr u32 ROWS = kRedThreads / G;  // rows a block has in one step
+    const u64 row0 = (u64)blockIdx.x * ROWS * Q + threadIdx.x / G;
+    const u32 i = threadIdx.x % G * VEC;
+    Vec<T, VEC> v[Q];
+    typename TR::Acc acc[Q];
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (i + q * STEP < R) v[q] = *reinterpret_cast<const Vec<T, VEC>*>(p + i + q * STEP);
+    for (int q = 0; q < Q; q++)
+        if (i < R && row0 + q * ROWS < rows) v[q] = *reinterpret_cast<const Vec<T, VEC>*>(in + (row0 + q * ROWS) * R + i);
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (i + q * STEP < R)
+    for (int q = 0; q < Q; q++) {
+        acc[q] = TR::init();
+        if (i < R && row0 + q * ROWS < rows)
 #pragma unroll
-                    for (int j = 0; j < VEC; j++) acc = TR::combine(acc, TR::load(v[q].v[j]));
-        }
+            for (int j = 0; j < VEC; j++) acc[q] = TR::combine(acc[q], TR::load(v[q].v[j]));
     }
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) acc = TR::combine(acc, __shfl_xor_sync(0xFFFFFFFFu, acc, o));
-    if (live && threadIdx.x % G == 0) out[row] = TR::finalize(acc, factor);
+    for (int o = G / 2; o > 0; o >>= 1)  // the shuffles take the whole warp
+#pragma unroll
+        for (int q = 0; q < Q; q++) acc[q] = TR::combine(acc[q], __shfl_xor_sync(0xFFFFFFFFu, acc[q], o));
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+        if (threadIdx.x % G == 0 && row0 + q * ROWS < rows) out[row0 + q * ROWS] = TR::finalize(acc[q], factor);
+}
+
+// One warp per longer row (R < ~2048), four loads per lane in flight.
+template <class T, int KIND, int VEC>
+__global__ void __launch_bounds__(kRedThreads) reduce_rows_warp_kernel(const T* in, T* out, u64 rows, u64 R, u64 factor) {
+    typedef RedTraits<T, KIND> TR;
+    const u64 row = (u64)blockIdx.x * (kRedThreads / 32) + threadIdx.x / 32;
+    if (row >= rows) return;
+    constexpr int STEP = 32 * VEC;
+    const T* p = in + row * R;
+    typename TR::Acc acc = TR::init();
+    for (u64 i = (threadIdx.x % 32) * VEC; i < R; i += 4 * STEP) {
+        Vec<T, VEC> v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (i + q * STEP < R) v[q] = *reinterpret_cast<const Vec<T, VEC>*>(p + i + q * STEP);
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (i + q * STEP < R)
+#pragma unroll
+                for (int j = 0; j < VEC; j++) acc = TR::combine(acc, TR::load(v[q].v[j]));
+    }
+    acc = warp_reduce<TR>(acc);
+    if (threadIdx.x % 32 == 0) out[row] = TR::finalize(acc, factor);
 }
 
 // One thread per row (R < 8).
@@ -517,14 +543,21 @@ u32* arrival_counters(u64 count);                      // zeroed counters for la
 void red_plan_dims(RedPlan& pl, size_t num_els, size_t num_dims, size_t num_red, const size_t* hm);
 void red_plan_shape(RedPlan& pl, size_t num_els, size_t num_dims, const size_t* hm);
 
+template <class T, int KIND, int VEC, int G>
+void red_rows_short_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaStream_t s) {
+    constexpr u64 ROWS = kRedThreads / G;
+    // four rows per group while that leaves every SM its eight blocks
+    if (O >= 4 * ROWS * 8 * (u64)sm_count()) reduce_rows_short_kernel<T, KIND, VEC, G, 4><<<(u32)((O + 4 * ROWS - 1) / (4 * ROWS)), kRedThreads, 0, s>>>(in, out, O, (u32)R, factor);
+    else reduce_rows_short_kernel<T, KIND, VEC, G, 1><<<(u32)((O + ROWS - 1) / ROWS), kRedThreads, 0, s>>>(in, out, O, (u32)R, factor);
+}
 template <class T, int KIND, int VEC>
 void red_rows_group_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaStream_t s) {
     const u64 lanes = (R + VEC - 1) / VEC;
-    auto blocks = [&](int g) { return (u32)((O + kRedThreads / g - 1) / (kRedThreads / g)); };
-    if (lanes <= 4) reduce_rows_group_kernel<T, KIND, VEC, 4><<<blocks(4), kRedThreads, 0, s>>>(in, out, O, R, factor);
-    else if (lanes <= 8) reduce_rows_group_kernel<T, KIND, VEC, 8><<<blocks(8), kRedThreads, 0, s>>>(in, out, O, R, factor);
-    else if (lanes <= 16) reduce_rows_group_kernel<T, KIND, VEC, 16><<<blocks(16), kRedThreads, 0, s>>>(in, out, O, R, factor);
-    else reduce_rows_group_kernel<T, KIND, VEC, 32><<<blocks(32), kRedThreads, 0, s>>>(in, out, O, R, factor);
+    if (lanes <= 4) red_rows_short_launch<T, KIND, VEC, 4>(in, out, O, R, factor, s);
+    else if (lanes <= 8) red_rows_short_launch<T, KIND, VEC, 8>(in, out, O, R, factor, s);
+    else if (lanes <= 16) red_rows_short_launch<T, KIND, VEC, 16>(in, out, O, R, factor, s);
+    else if (lanes <= 32) red_rows_short_launch<T, KIND, VEC, 32>(in, out, O, R, factor, s);
+    else reduce_rows_warp_kernel<T, KIND, VEC><<<(u32)((O + kRedThreads / 32 - 1) / (kRedThreads / 32)), kRedThreads, 0, s>>>(in, out, O, R, factor);
 }
 
 template <class T, int KIND>

@@ -155,3 +155,22 @@ def test_outer_and_inner_dims_folded_around_a_kept_one(oracle, cuda, shape):
             again = H.run_sum_to_shape(cuda, dt, dims, H.contiguous_strides(dims), out_dims, off, x)
             assert np.array_equal(got, again)
             H.assert_same("sum_to_shape", dt, got, ref, float_rel=SUM_TOL.get(dt.name, 0.0), what=str((shape, off)), scale=np.sqrt(q * i))
+
+
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.I32], ids=lambda d: d.name)
+@pytest.mark.parametrize("shape", [(303200, 8), (151600, 56), (76000, 13), (38000, 100), (37900, 30), (700, 31), (700, 33), (700, 1023), (700, 1032)], ids=str)
+def test_rows_shared_by_part_of_a_warp(oracle, cuda, shape, dt):
+    """Row lengths around the lanes a row gets (4 to 32, then a warp that walks the row), and row counts on both sides of the
+    form with four rows per group; the sum within this file's tolerance, the maximum exact."""
+    from oracle import binding
+    rows, r = shape
+    rng = np.random.default_rng(rows + r)
+    x = H.random_store(rng, dt, rows * r, dist="normal") if dt.kind == "float" else H.full_range_store(rng, dt, rows * r)
+    for op in ("sum", "max"):
+        binding.set_wide(True)
+        try:
+            ref = _run_dim(oracle, op, dt, [rows, r], None, [1], 0, x)
+        finally:
+            binding.set_wide(False)
+        got = _run_dim(cuda, op, dt, [rows, r], None, [1], 0, x)
+        H.assert_same(op, dt, got, ref, float_rel=SUM_TOL.get(dt.name, 0.0) if op == "sum" else 0.0, what=str((op, shape)), scale=np.sqrt(r))
