@@ -123,6 +123,10 @@ __device__ __forceinline__ uint32_t small_part(uint32_t bits) {
     return (bits & 0x7F800000u) == 0x7F800000u ? 0u : s;
 }
 
+// BN_T = 128: the form of 128-column tiles, long chunks and tensor stores, all known to the compiler; 0: everything from the
+// parameters.  The difference is the splitter's: with the distance between a raw and its small tile a constant, its loads run
+// ahead of its stores (8192 x 4096 x 4096: 164 TFLOP/s, 148 in batches of four).
+template <int BN_T>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                    Params p, int* err, int tag) {
@@ -139,6 +143,8 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(smem + Smem::bars + 8 * (3 * MAX_STAGES + 4));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int chunk_kb = BN_T ? CHUNK_FAST : p.chunk_kb;
+    const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? STAGES : p.stages, raw_bytes = BN_T ? A_TILE + BN_T * BK * 4 : p.raw_bytes;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; s++) {
@@ -176,8 +182,8 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(full_bar(stage), p.raw_bytes);
-                    const uint32_t sa = smem_base + Smem::stages + stage * 2 * p.raw_bytes;
+                    mbar_expect_tx(full_bar(stage), raw_bytes);
+                    const uint32_t sa = smem_base + Smem::stages + stage * 2 * raw_bytes;
                     const uint32_t sb = sa + A_TILE;
                     int block = tb * p.split_kb + kb;  // a block past the end of K (or of the batches) is all fill: zeros
                     if (p.kb_per_z) {
@@ -192,11 +198,11 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         for (int h = 0; h < BM / 32; h++) tma_load_3d(sa + h * MN_CHUNK_BYTES, &map_a, tm * BM + h * 32, k, za, full_bar(stage));
                     }
                     if (!p.b_mn) {
-                        tma_load_3d(sb, &map_b, k, tn * p.bn, zb, full_bar(stage));
+                        tma_load_3d(sb, &map_b, k, tn * bn, zb, full_bar(stage));
                     } else {
-                        for (int h = 0; h < p.bn / 32; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * p.bn + h * 32, k, zb, full_bar(stage));
+                        for (int h = 0; h < bn / 32; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * bn + h * 32, k, zb, full_bar(stage));
                     }
-                    if (++stage == p.stages) {
+                    if (++stage == stages) {
                         stage = 0;
                         phase ^= 1;
                     }
@@ -206,21 +212,21 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (lane == 0) {
-            const uint32_t idesc = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, p.bn);
+            const uint32_t idesc = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, bn);
             // K-major: 8 floats further along the 128-byte row; MN-major: the next group of eight K-rows
             const uint64_t a_kstep = p.a_mn ? (1024 >> 4) : (32 >> 4), b_kstep = p.b_mn ? (1024 >> 4) : (32 >> 4);
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
-                for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += p.chunk_kb) {
+                for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += chunk_kb) {
                     if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1, err, tag, 2)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
-                    const int kb1 = min(kb0 + p.chunk_kb, p.num_kb);
+                    const int kb1 = min(kb0 + chunk_kb, p.num_kb);
                     for (int kb = kb0; kb < kb1; kb++) {
                         // the raw tiles (TMA) and the small tiles (splitter) are both operands
                         if (!mbar_wait(full_bar(stage), phase, err, tag, 3) || !mbar_wait(split_bar(stage), phase, err, tag, 6)) {
@@ -228,16 +234,16 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             break;
                         }
                         tc_fence_after();
-                        const uint32_t s0 = smem_base + Smem::stages + stage * 2 * p.raw_bytes;
+                        const uint32_t s0 = smem_base + Smem::stages + stage * 2 * raw_bytes;
                         // K-major: rows of 32 floats, groups of eight rows 1024 bytes apart.  MN-major: 32-byte-atom swizzle,
                         // groups of four K-rows 512 bytes apart, 128-byte-wide MN chunks one box (4 KB) apart.
                         const uint64_t a_big = p.a_mn ? smem_desc_sw128_atom32(s0, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0, 16, 1024);
                         const uint64_t b_big = p.b_mn ? smem_desc_sw128_atom32(s0 + A_TILE, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + A_TILE, 16, 1024);
                         const uint64_t a_small =
-                            p.a_mn ? smem_desc_sw128_atom32(s0 + p.raw_bytes, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + p.raw_bytes, 16, 1024);
-                        const uint64_t b_small = p.b_mn ? smem_desc_sw128_atom32(s0 + p.raw_bytes + A_TILE, MN_CHUNK_BYTES, 512)
-                                                        : smem_desc_sw128(s0 + p.raw_bytes + A_TILE, 16, 1024);
-                        if (p.chunk_kb == 1) {
+                            p.a_mn ? smem_desc_sw128_atom32(s0 + raw_bytes, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + raw_bytes, 16, 1024);
+                        const uint64_t b_small = p.b_mn ? smem_desc_sw128_atom32(s0 + raw_bytes + A_TILE, MN_CHUNK_BYTES, 512)
+                                                        : smem_desc_sw128(s0 + raw_bytes + A_TILE, 16, 1024);
+                        if (chunk_kb == 1) {
 #pragma unroll
                             for (int k = 0; k < BK / UMMA_K; k++) {
                                 umma_tf32(d_tmem, a_small + a_kstep * k, b_big + b_kstep * k, idesc, k != 0);
@@ -254,7 +260,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                             }
                         }
                         umma_commit(empty_bar(stage));
-                        if (++stage == p.stages) {
+                        if (++stage == stages) {
                             stage = 0;
                             phase ^= 1;
                         }
@@ -282,9 +288,9 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             float total[BN];  // this thread's row of the tile (registers: every index below is a compile-time constant)
 #pragma unroll
             for (int j = 0; j < BN; j++) total[j] = 0.0f;
-            for (int kb0 = 0; kb0 < p.num_kb; kb0 += p.chunk_kb) {
+            for (int kb0 = 0; kb0 < p.num_kb; kb0 += chunk_kb) {
                 // the TMEM loads below are warp-collective: leave the loops only as a whole warp
-                const bool ready = mbar_wait_relaxed(tfull_bar(acc), acc_phase, err, tag, 4, p.chunk_kb == 1 ? 20 : 200);
+                const bool ready = mbar_wait_relaxed(tfull_bar(acc), acc_phase, err, tag, 4, chunk_kb == 1 ? 20 : 200);
                 if (!__all_sync(0xFFFFFFFFu, ready)) {
                     ok = false;
                     break;
@@ -293,7 +299,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
 #pragma unroll
                 for (int c = 0; c < BN / 32; c++) {
-                    if (c * 32 >= p.bn) break;
+                    if (c * 32 >= bn) break;
                     uint32_t v[32];
                     tmem_ld_32x32b_x32(t_row + c * 32, v);
                     tmem_ld_wait();
@@ -312,7 +318,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if (!ok) break;
 #pragma unroll
             for (int c = 0; c < BN / EPI_CHUNK_COLS; c++) {
-                if (c * EPI_CHUNK_COLS >= p.bn) break;
+                if (c * EPI_CHUNK_COLS >= bn) break;
                 // the staging buffer must have been read by its previous TMA store
                 if (lane == 0) tma_store_wait_read<1>();
                 __syncwarp();
@@ -323,9 +329,9 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         make_float4(total[c * 32 + 4 * j], total[c * 32 + 4 * j + 1], total[c * 32 + 4 * j + 2], total[c * 32 + 4 * j + 3]);
                 fence_proxy_async_smem();
                 __syncwarp();
-                const int row0 = tm * BM + quarter * 32, col0 = tn * p.bn + c * EPI_CHUNK_COLS;
+                const int row0 = tm * BM + quarter * 32, col0 = tn * bn + c * EPI_CHUNK_COLS;
                 unsigned char* src = stage_buf + buf * EPI_STAGE_BYTES;
-                if (p.d_plain) {
+                if (!BN_T && p.d_plain) {
                     float* out = p.d + ((size_t)tb * p.M + row0) * p.N + col0 + lane;
                     for (int r0 = 0; r0 < 32; r0 += 8) {
                         float v[8];
@@ -356,21 +362,30 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     ok = false;
                     break;
                 }
-                const uint4* raw = reinterpret_cast<const uint4*>(smem + Smem::stages + stage * 2 * p.raw_bytes);
-                uint4* small = reinterpret_cast<uint4*>(smem + Smem::stages + stage * 2 * p.raw_bytes + p.raw_bytes);
-                const int steps = p.raw_bytes / 16 / (32 * SPLIT_WARPS);
-                for (int i0 = 0; i0 < steps; i0 += 4) {  // 12 or 16 steps; loads first: the compiler cannot tell the two tiles apart
-                    uint4 q[4];
+                const uint4* raw = reinterpret_cast<const uint4*>(smem + Smem::stages + stage * 2 * raw_bytes);
+                uint4* small = reinterpret_cast<uint4*>(smem + Smem::stages + stage * 2 * raw_bytes + raw_bytes);
+                if constexpr (BN_T != 0) {
+                    constexpr int STEPS = (A_TILE + BN_T * BK * 4) / 16 / (32 * SPLIT_WARPS);
+#pragma unroll 8
+                    for (int i = 0; i < STEPS; i++) {
+                        const uint4 q = raw[t + i * 32 * SPLIT_WARPS];
+                        small[t + i * 32 * SPLIT_WARPS] = make_uint4(small_part(q.x), small_part(q.y), small_part(q.z), small_part(q.w));
+                    }
+                } else {
+                    const int steps = raw_bytes / 16 / (32 * SPLIT_WARPS);
+                    for (int i0 = 0; i0 < steps; i0 += 4) {  // 12 or 16 steps; loads first: the compiler cannot tell the two tiles apart
+                        uint4 q[4];
 #pragma unroll
-                    for (int i = 0; i < 4; i++) q[i] = raw[t + (i0 + i) * 32 * SPLIT_WARPS];
+                        for (int i = 0; i < 4; i++) q[i] = raw[t + (i0 + i) * 32 * SPLIT_WARPS];
 #pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        small[t + (i0 + i) * 32 * SPLIT_WARPS] = make_uint4(small_part(q[i].x), small_part(q[i].y), small_part(q[i].z), small_part(q[i].w));
+                        for (int i = 0; i < 4; i++)
+                            small[t + (i0 + i) * 32 * SPLIT_WARPS] = make_uint4(small_part(q[i].x), small_part(q[i].y), small_part(q[i].z), small_part(q[i].w));
+                    }
                 }
                 fence_proxy_async_smem();  // the tensor core reads these through the async proxy
                 __syncwarp();
                 if (lane == 0) mbar_arrive(split_bar(stage));
-                if (++stage == p.stages) {
+                if (++stage == stages) {
                     stage = 0;
                     phase ^= 1;
                 }
@@ -401,10 +416,11 @@ bool opt_in_shared_memory() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
-        if (cudaFuncSetAttribute(tc_gemm_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
+        for (auto kernel : {tc_gemm_f32_kernel<BN>, tc_gemm_f32_kernel<0>})
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
         done[dev] = true;
     }
     return true;
@@ -493,7 +509,8 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.a_mn = a_mn ? 1 : 0;
     p.b_mn = b_mn ? 1 : 0;
     if (grid > p.num_tiles) grid = p.num_tiles;
-    tc_gemm_f32_kernel<<<grid, THREADS, SMEM_BYTES, ctx().stream>>>(ma, mb, md, p, err, tag);
+    const auto kernel = p.bn == BN && !p.d_plain && p.chunk_kb == CHUNK_FAST ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>;
+    kernel<<<grid, THREADS, SMEM_BYTES, ctx().stream>>>(ma, mb, md, p, err, tag);
     check_launch(where);
     if (slices > 1) splitk_reduce(2, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
     return true;
