@@ -60,6 +60,7 @@ constexpr int TMEM_COLS = 2 * BN;              // two f32 accumulators
 constexpr int GROUP_M = 16;
 constexpr int CHUNK_FAST = 4;
 constexpr int MN_CHUNK_BYTES = BK * 128;       // one [32 K-rows x 32 MN-elements] box
+constexpr int REDO_BITS = 2048;
 
 static_assert(TMEM_COLS == 256 || TMEM_COLS == 512, "TMEM allocations are powers of two");
 static_assert(A_TILE % (16 * 32 * SPLIT_WARPS) == 0 && B_TILE / 2 % (16 * 32 * SPLIT_WARPS) == 0, "the splitter moves 16 bytes per thread and step");
@@ -68,7 +69,8 @@ struct Smem {
     static constexpr int stages = 0;
     static constexpr int epi = stages + STAGES * STAGE_BYTES;
     static constexpr int bars = epi + EPI_WARPS * 2 * EPI_STAGE_BYTES;
-    static constexpr int total = bars + 256;
+    static constexpr int redo = bars + 256;  // one bit per tile of this CTA (number modulo REDO_BITS), then whether any is set: see redo_tile
+    static constexpr int total = redo + REDO_BITS / 8 + 16;
 };
 constexpr int SMEM_BYTES = Smem::total + 1024;  // slack for the 1024-byte alignment
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
@@ -97,8 +99,13 @@ struct Params {
     int raw_bytes;  // what TMA delivers per stage: A and bn rows of B
     int split_kb;   // > 0: split-K; batch s of the launch reduces the k-blocks [s * split_kb, (s + 1) * split_kb) of one product
     int kb_per_z;   // > 0: the reduction runs over the operands' batches too: k-block i is block i % kb_per_z of batch i / kb_per_z
-    int d_plain;    // != 0: the output's rows (or base) are not 16-byte multiples: the epilogue warps write them to `d` themselves
-    float* d;
+    int d_plain;    // != 0: the output's rows (or base) are not 16-byte multiples: the epilogue warps write them to `out` themselves
+    // The operands and the output as plain memory, for redo_tile: element (row, k) of batch z at z * bs + row * rs + k * ks.
+    const float *a, *b;
+    int64_t a_bs, a_rs, a_ks, b_bs, b_rs, b_ks;
+    int K, zs;      // zs: batches of the operands (kb_per_z > 0)
+    float* out;     // D or the split-K partial results, rows `out_ld` elements apart
+    int64_t out_ld;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, const Params& p, int& tm, int& tn, int& tb) {
@@ -121,6 +128,65 @@ __device__ __forceinline__ uint32_t small_part(uint32_t bits) {
     const float big = __uint_as_float(bits & 0xFFFFE000u);
     const uint32_t s = (__float_as_uint(x - big) + 0x1000u) & 0xFFFFE000u;
     return (bits & 0x7F800000u) == 0x7F800000u ? 0u : s;
+}
+
+// A tile whose result is not finite, again and in f32 arithmetic: the split has no form for infinities (inf times the zero `small` of
+// an operand that tf32 holds exactly is NaN) and the tensor core reads a NaN whose payload sits in the low bits as one.  An
+// infinity or NaN among the operands always leaves a non-finite sum here, whatever becomes of it, so the epilogue's look at its totals
+// finds every such tile at the cost of one FMA per output, and finite operands cost nothing else (products of K = 64: 4 to 7 %; of
+// K = 1024 and more: none).  k ascending with separate multiply and add, as on the CUDA cores.  All threads of the block; `stage` is the operand ring, which nothing uses any more.
+__device__ __forceinline__ void redo_tile(const Params& p, int bn, int tm, int tn, int tb, float* stage) {
+    constexpr int LD = BM + 4, T = 16;  // 16 x 16 threads, rows ty + 16 i, columns tx + 16 j
+    float *xs = stage, *ys = stage + BK * LD;  // [k][row], [k][column]
+    const int tx = threadIdx.x % T, ty = threadIdx.x / T;
+    float acc[BM / T][BN / T];
+#pragma unroll
+    for (int i = 0; i < BM / T; i++)
+#pragma unroll
+        for (int j = 0; j < BN / T; j++) acc[i][j] = 0.0f;
+    for (int kb = 0; kb < p.num_kb; kb++) {
+        int block = tb * p.split_kb + kb, za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
+        if (p.kb_per_z) {
+            za = zb = block / p.kb_per_z;
+            block -= za * p.kb_per_z;
+            if (za >= p.zs) break;  // the last slice runs past the last batch
+        }
+        const int k0 = block * BK;
+        if (k0 >= p.K) break;
+        for (int e = threadIdx.x; e < BM * BK; e += THREADS) {
+            const int k = p.a_mn ? e / BM : e % BK, r = p.a_mn ? e % BM : e / BK;
+            xs[k * LD + r] = k0 + k < p.K && tm * BM + r < p.M ? p.a[za * p.a_bs + (tm * BM + r) * p.a_rs + (k0 + k) * p.a_ks] : 0.0f;
+        }
+        for (int e = threadIdx.x; e < BN * BK; e += THREADS) {
+            const int k = p.b_mn ? e / BN : e % BK, c = p.b_mn ? e % BN : e / BK;
+            ys[k * LD + c] = c < bn && k0 + k < p.K && tn * bn + c < p.N ? p.b[zb * p.b_bs + (tn * bn + c) * p.b_rs + (k0 + k) * p.b_ks] : 0.0f;
+        }
+        __syncthreads();
+        if (ty < T) {
+            for (int k = 0; k < BK; k++) {
+                float x[BM / T], y[BN / T];
+#pragma unroll
+                for (int i = 0; i < BM / T; i++) x[i] = xs[k * LD + ty + T * i];
+#pragma unroll
+                for (int j = 0; j < BN / T; j++) y[j] = ys[k * LD + tx + T * j];
+#pragma unroll
+                for (int i = 0; i < BM / T; i++)
+#pragma unroll
+                    for (int j = 0; j < BN / T; j++) acc[i][j] = acc[i][j] + x[i] * y[j];
+            }
+        }
+        __syncthreads();
+    }
+    if (ty >= T) return;
+#pragma unroll
+    for (int i = 0; i < BM / T; i++) {
+        const int row = tm * BM + ty + T * i;
+#pragma unroll
+        for (int j = 0; j < BN / T; j++) {
+            const int c = tx + T * j;
+            if (row < p.M && c < bn && tn * bn + c < p.N) p.out[((int64_t)tb * p.M + row) * p.out_ld + tn * bn + c] = acc[i][j];
+        }
+    }
 }
 
 // BN_T = 128: the form of 128-column tiles, long chunks and tensor stores, all known to the compiler; 0: everything from the
@@ -146,6 +212,8 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const int chunk_kb = BN_T ? CHUNK_FAST : p.chunk_kb;
     const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? STAGES : p.stages, raw_bytes = BN_T ? A_TILE + BN_T * BK * 4 : p.raw_bytes;
 
+    auto redo = [&] { return reinterpret_cast<uint32_t*>(smem + Smem::redo); };
+    if (threadIdx.x <= REDO_BITS / 32) redo()[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; s++) {
             mbar_init(full_bar(s), 1);
@@ -316,6 +384,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 }
             }
             if (!ok) break;
+            float zero = 0.0f;  // NaN from the first total on that is not finite
 #pragma unroll
             for (int c = 0; c < BN / EPI_CHUNK_COLS; c++) {
                 if (c * EPI_CHUNK_COLS >= bn) break;
@@ -327,12 +396,19 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 for (int j = 0; j < 8; j++)  // eight 16-byte chunks per row, XOR-swizzled by the row index
                     *reinterpret_cast<float4*>(dst + ((j ^ (lane & 7)) << 4)) =
                         make_float4(total[c * 32 + 4 * j], total[c * 32 + 4 * j + 1], total[c * 32 + 4 * j + 2], total[c * 32 + 4 * j + 3]);
+                float even = 0.0f, odd = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                    even = fmaf(total[c * 32 + j], 0.0f, even);
+                    odd = fmaf(total[c * 32 + j + 1], 0.0f, odd);
+                }
+                zero += even + odd;
                 fence_proxy_async_smem();
                 __syncwarp();
                 const int row0 = tm * BM + quarter * 32, col0 = tn * bn + c * EPI_CHUNK_COLS;
                 unsigned char* src = stage_buf + buf * EPI_STAGE_BYTES;
                 if (!BN_T && p.d_plain) {
-                    float* out = p.d + ((size_t)tb * p.M + row0) * p.N + col0 + lane;
+                    float* out = p.out + ((size_t)tb * p.M + row0) * p.N + col0 + lane;
                     for (int r0 = 0; r0 < 32; r0 += 8) {
                         float v[8];
 #pragma unroll
@@ -346,6 +422,11 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     tma_store_commit();
                 }
                 buf ^= 1;
+            }
+            if (__any_sync(0xFFFFFFFFu, zero != 0.0f) && lane == 0) {
+                const int it = (tile - (int)blockIdx.x) / (int)gridDim.x;
+                atomicOr(&redo()[it % REDO_BITS / 32], 1u << it % 32);
+                redo()[REDO_BITS / 32] = 1;
             }
         }
         if (lane == 0) tma_store_wait_all();
@@ -406,6 +487,16 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+
+    // the tile stores have completed (tma_store_wait_all before the barrier above): their places may be written again
+    if (!redo()[REDO_BITS / 32]) return;
+    fence_proxy_async();
+    for (int tile = blockIdx.x, it = 0; tile < p.num_tiles; tile += gridDim.x, it++) {
+        if (!(redo()[it % REDO_BITS / 32] >> it % 32 & 1)) continue;
+        int tm, tn, tb;
+        tile_coords(tile, p, tm, tn, tb);
+        redo_tile(p, bn, tm, tn, tb, reinterpret_cast<float*>(smem + Smem::stages));
     }
 }
 
@@ -500,7 +591,6 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     const bool okb = b_mn ? make_map(&mb, c.B, K, N, c.batch, b_bs, BK, true, c.b_pitch) : make_map(&mb, c.B, N, K, c.batch, b_bs, (uint32_t)p.bn, false, c.b_pitch);
     if (!oka || !okb) return false;
     p.d_plain = slices > 1 ? 0 : c.d_plain;
-    p.d = static_cast<float*>(D);
     if (p.d_plain) md = ma;  // not used
     else if (slices > 1 ? !make_map(&md, partial.ptr, M, N, batch, M * n_pitch, 32, false, n_pitch) : !make_map(&md, D, M, N, batch, M * N, 32)) return false;
     p.num_tiles = (int)batch * p.tiles_per_batch;
@@ -508,6 +598,19 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.b_batched = (c.batch > 1 && b_bs != 0) ? 1 : 0;
     p.a_mn = a_mn ? 1 : 0;
     p.b_mn = b_mn ? 1 : 0;
+    p.a = reinterpret_cast<const float*>(c.A);
+    p.b = reinterpret_cast<const float*>(c.B);
+    p.a_bs = c.batch > 1 ? c.a_bs : 0;
+    p.b_bs = c.batch > 1 ? c.b_bs : 0;
+    const int64_t a_ld = (int64_t)(c.a_pitch ? c.a_pitch : a_mn ? M : K), b_ld = (int64_t)(c.b_pitch ? c.b_pitch : b_mn ? N : K);
+    p.a_rs = a_mn ? 1 : a_ld;
+    p.a_ks = a_mn ? a_ld : 1;
+    p.b_rs = b_mn ? 1 : b_ld;
+    p.b_ks = b_mn ? b_ld : 1;
+    p.K = (int)K;
+    p.zs = (int)c.batch;
+    p.out = static_cast<float*>(slices > 1 ? partial.ptr : D);
+    p.out_ld = (int64_t)(slices > 1 ? n_pitch : N);
     if (grid > p.num_tiles) grid = p.num_tiles;
     const auto kernel = p.bn == BN && !p.d_plain && p.chunk_kb == CHUNK_FAST ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>;
     kernel<<<grid, THREADS, SMEM_BYTES, ctx().stream>>>(ma, mb, md, p, err, tag);

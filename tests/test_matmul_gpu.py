@@ -425,3 +425,84 @@ def test_batched_and_ragged_backward(oracle, cuda, dt, case):
         binding.set_wide(False)
     for key in ref:
         H.assert_same("matmul_backward", dt, got[key], ref[key], float_rel=1e-5 if dt.name == "f32" else 1e-2, what=f"{name}/{key}", scale=np.sqrt(n if key == "ga" else m))
+
+
+# ---------------------------------------------------------------------------------------
+# Infinities and NaNs in f32 products.  The split into two tf32 parts has no form for them (inf times the zero second part of
+# 1.0 would be NaN); the product must give what f32 arithmetic gives.  Every form of the split kernel: aligned, copied and plain-store
+# operands, batches, runs along K, 64- and 128-column tiles.
+# ---------------------------------------------------------------------------------------
+NONFINITE = [
+    # name, batch dims, M, N, K, a_major, b_major
+    ("aligned", [], 264, 256, 384, "k", "mn"),
+    ("aligned-nt", [], 520, 516, 1024, "k", "k"),
+    ("aligned-tn", [], 384, 512, 512, "mn", "mn"),
+    ("ragged", [], 257, 515, 1031, "k", "k"),
+    ("ragged-tt", [], 263, 521, 1033, "mn", "k"),
+    ("n-even", [], 200, 514, 1000, "k", "mn"),
+    ("narrow", [], 4099, 12, 1001, "k", "k"),
+    ("split", [], 130, 264, 4000, "k", "k"),
+    ("long-split", [], 132, 264, 8192, "mn", "mn"),
+    ("batched", [3], 136, 264, 520, "k", "mn"),
+    ("rank-4", [2, 3], 200, 264, 516, "k", "mn"),
+]
+
+
+def special_operands(rng, m, n, k, nb):
+    """Mostly values that tf32 holds exactly (small integers, zeros among them), with rows of A and columns of B that hold
+    infinities, NaNs of several payloads and both, and one large finite value whose products stay exact."""
+    a = rng.integers(-3, 4, (nb, m, k)).astype(np.float32)
+    b = rng.integers(-3, 4, (nb, k, n)).astype(np.float32)
+    bits = lambda u: np.uint32(u).view(np.float32)  # noqa: E731
+    rows, cols = np.arange(0, m, 7), np.arange(3, n, 11)
+    for i, v in enumerate((np.inf, -np.inf, bits(0x7F800001), bits(0x7FC00000), bits(0xFF800400), 2.0 ** 20)):
+        for z in range(nb):
+            if i < len(rows):
+                a[z, rows[i], (5 * i + 31 * z) % k] = v
+            if i < len(cols):
+                b[z, (17 * i + z + k // 2) % k, cols[i]] = v
+    a[:, -1, k - 1] = np.inf      # the last row, the last value of K
+    b[:, k - 1, -1] = 0.5         # times an exact value
+    if m > 20:
+        a[:, 20, 0], a[:, 20, k // 2] = np.inf, -np.inf   # inf - inf
+        b[:, 0, :] = np.abs(b[:, 0, :]) + 1
+    return a, b
+
+
+@pytest.mark.parametrize("case", NONFINITE, ids=lambda c: c[0])
+def test_f32_products_of_infinities_and_nans(oracle, cuda, case):
+    """NaN and infinity patterns are those of the f64 product; the finite sums are of integers that f32 holds
+    (the bound leaves room for the one product of 2^40 that takes small terms with it)."""
+    name, bd, m, n, k, amaj, bmaj = case
+    rng = np.random.default_rng(zlib_seed("nonfinite" + name))
+    cs = H.contiguous_strides
+    nb = H.numel(bd) if bd else 1
+    a, b = special_operands(rng, m, n, k, nb)
+    with np.errstate(all="ignore"):
+        ref = np.matmul(a.astype(np.float64), b.astype(np.float64)).astype(np.float32).reshape(-1)
+    a_sh, b_sh, o = [*bd, m, k], [*bd, k, n], [*bd, m, n]
+    ast = cs(a_sh) if amaj == "k" else [1, m]
+    bst = cs(b_sh) if bmaj == "mn" else [1, k]
+    astore = a.reshape(-1) if amaj == "k" else np.ascontiguousarray(a[0].T).reshape(-1)
+    bstore = b.reshape(-1) if bmaj == "mn" else np.ascontiguousarray(b[0].T).reshape(-1)
+    meta = H.matmul_metadata(o, a_sh, b_sh, ast, bst, 0, 0)
+    got = H.run_matmul(cuda, D.F32, meta, nb * m * n, astore, bstore)
+    H.assert_same("matmul", D.F32, got, ref, float_rel=1e-5, what=name, scale=np.sqrt(k))
+
+
+def test_f32_backward_products_of_infinities_and_nans(oracle, cuda):
+    for bd, m, n, k in (([4], 264, 272, 280), ([], 301, 519, 227), ([], 264, 512, 256)):
+        rng = np.random.default_rng(m)
+        cs = H.contiguous_strides
+        nb = H.numel(bd) if bd else 1
+        g, bt = special_operands(rng, m, k, n, nb)        # grad_a = g . B^T
+        bw = np.ascontiguousarray(bt.transpose(0, 2, 1))  # B [k, n]
+        a = rng.integers(-2, 3, (nb, m, k)).astype(np.float32)
+        a[:, 5, 3] = np.inf
+        meta = H.matmul_metadata([*bd, m, n], [*bd, m, k], [*bd, k, n], cs([*bd, m, k]), cs([*bd, k, n]), 0, 0)
+        got = H.run_matmul_backward(cuda, D.F32, meta, nb * m * k, nb * k * n, g.reshape(-1), a.reshape(-1), bw.reshape(-1))
+        with np.errstate(all="ignore"):
+            ra = np.matmul(g.astype(np.float64), bt.astype(np.float64)).astype(np.float32).reshape(-1)
+            rb = np.matmul(a.astype(np.float64).transpose(0, 2, 1), g.astype(np.float64)).astype(np.float32).reshape(-1)
+        H.assert_same("matmul_backward", D.F32, got["ga"], ra, float_rel=1e-5, what="ga", scale=np.sqrt(n))
+        H.assert_same("matmul_backward", D.F32, got["gb"], rb, float_rel=1e-5, what="gb", scale=np.sqrt(m))
