@@ -12,18 +12,24 @@ extern "C" {
 /* Host-only views of the launch planners, for tests that run without a GPU: which kernel class a call with this
  * HOST metadata and these base addresses would take.  Elementwise: 0 empty, 1 flat, 2 row, 3 tile, 4 generic,
  * 5 serial (an in-place lhs that overlaps itself), 6 error, 7 flat with shifted loads (operands not 16-byte aligned).  Reduction: 0 empty, 1 rows, 2 columns, 3 generic
- * scatter, 4 error, with the recognised [outer, reduced, inner] extents. */
+ * scatter, 4 error, 5 first and last dim folded around a kept one, with the recognised [outer, reduced, inner] extents. */
 int mx_debug_elementwise_plan(size_t num_els, size_t num_dims, const size_t* host_metadata, int num_inputs, int inplace, size_t elem_size,
                               size_t out_elem_size, const void* out, const void* a, const void* b, int* merged_rank, int* vector_ok,
                               int* transposed_mask);
-/* Would cuda_matmul_<bf16|f16> with this HOST metadata run on the tcgen05 kernel (1) or on the SIMT kernel (0)?
+/* Would cuda_matmul_<bf16|f16> with this HOST metadata run on the tcgen05 kernel (its batches) or on the CUDA-core kernels (0)?
  * Also returns the operand layouts (0 = K-major, 1 = MN-major) and the extents of the launch. */
 int mx_debug_matmul_forward_path(size_t num_els, const size_t* host_metadata, const void* a, const void* b, const void* out, int* a_mn_major,
                                  int* b_mn_major, size_t* m, size_t* n, size_t* k);
+/* The decision of every cuda_matmul / cuda_matmul_backward call (elem_size 2: bf16 / f16, 4: f32; which: 0 forward with x = a, y = b,
+ * 1 grad_a with x = g, y = b, 2 grad_b with x = g, y = a): 0 = CUDA-core kernels, else the number of batches of the tensor-core launch.
+ * *prepared: 1 the first operand of the product is copied to padded rows, 2 the second, 4 or 8 the output is written without tensor
+ * stores, element-wise or in pairs.  The two calls above and below are this one for the forward product. */
+int mx_debug_matmul_plan(size_t elem_size, int which, size_t num_els, size_t nea, size_t neb, const size_t* host_metadata, const void* x, const void* y,
+                         const void* out, int* a_mn_major, int* b_mn_major, size_t* m, size_t* n, size_t* k, int* prepared);
 int mx_debug_reduce_plan(size_t num_els, size_t num_dims, size_t num_red_dims, const size_t* host_metadata, int sum_to_shape, size_t* outer,
                          size_t* reduced, size_t* inner);
 
-/* Would cuda_matmul_f32 with this HOST metadata run on the tcgen05 split-tf32 kernel (1) or on the SIMT kernel (0)? */
+/* Would cuda_matmul_f32 with this HOST metadata run on the tcgen05 split-tf32 kernel (its batches) or on the CUDA-core kernels (0)? */
 int mx_debug_matmul_forward_path_f32(size_t num_els, const size_t* host_metadata, const void* a, const void* b, const void* out, int* a_mn_major,
                                      int* b_mn_major, size_t* m, size_t* n, size_t* k);
 /* Tuning aid: row-tiles per column sweep in the one-CTA tensor-core kernel's tile order (default 16). */

@@ -74,6 +74,9 @@ RUNTIME_SIGNATURES = {
     "mx_debug_matmul_forward_path_f32": ([ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(ctypes.c_int),
                                           ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_size_t),
                                           ctypes.POINTER(ctypes.c_size_t)], ctypes.c_int),
+    "mx_debug_matmul_plan": ([ctypes.c_size_t, ctypes.c_int, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+                              ctypes.c_void_p, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_size_t),
+                              ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_int)], ctypes.c_int),
     "mx_debug_tc_gemm_poke_status": ([ctypes.c_int], ctypes.c_int),
     "mx_debug_set_gemm_group_m": ([ctypes.c_int], None),
     "mx_debug_gemm_max_resident_pairs": ([], ctypes.c_int),

@@ -1089,17 +1089,6 @@ static bool aligned_batches(size_t es, const TcProduct& c) {
 // reduction over m, both operands MN-major.  The backward products read g, A and B as dense row-major matrices
 // (strides ignored, crates/maidenx_cpu/src/ops/matmul.rs:196-261).
 bool tc_classify(const MmDesc& d, int which, size_t es, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, const void* out,
-                 TcProduct& c) {
-    if (which == 0) {
-        if (d.out_nd > 3 && num_els > d.m * d.n) return false;
-        if (!forward_operands(d, es, num_els, x, y, c)) return false;
-    } else if (d.out_nd != 2 || !backward_operands(d, which, nea, neb, x, y, c)) {
-        return false;
-    }
-    return aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out);
-}
-
-bool tc_classify_any(const MmDesc& d, int which, size_t es, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, const void* out,
                      TcProduct& c) {
     if (which == 0 ? !forward_operands(d, es, num_els, x, y, c) : !backward_operands(d, which, nea, neb, x, y, c)) return false;
     c.ragged = d.out_nd > (which == 0 ? 3 : 2);  // aligned, but new to these kernels: batches beyond rank 3, batched backward
@@ -1168,27 +1157,28 @@ bool tc_batch_sum_f32(uint64_t batch, uint64_t m, uint64_t n, uint64_t k, const 
 bool tc_gemm_bf16_f16(bool is_bf16, const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out,
                       const char* where) {
     TcProduct c;
-    if (!tc_classify_any(d, which, 2, num_els, nea, neb, x, y, out, c)) return false;
+    if (!tc_classify(d, which, 2, num_els, nea, neb, x, y, out, c)) return false;
     StreamWorkspace ws;
     return repack_operands(2, c, ws, where) && launch_gemm(is_bf16, c, out, where);
 }
 
 }  // namespace mx
 
-// Host-only view for tests without a GPU: would cuda_matmul_<bf16|f16> with this HOST metadata and these base
-// addresses run on the tensor-core kernel?  Returns 0 (SIMT kernel) or 1, and the operand majors (0 = K-major,
-// 1 = MN-major) and extents it would be launched with.
-static int debug_forward_path(size_t es, size_t num_els, const size_t* host_metadata, const void* a, const void* b, const void* out, int* a_mn_major,
-                              int* b_mn_major, size_t* m, size_t* n, size_t* k) {
+// Host-only view for tests without a GPU: would cuda_matmul[_backward]_<bf16|f16|f32> with this HOST metadata and these base
+// addresses run on a tensor-core kernel?  Returns 0 (CUDA-core kernels) or the number of batches, and how the product would be
+// launched: operand majors (0 = K-major, 1 = MN-major), extents, and what is prepared for it (include/maidenx_cuda_testing.h).
+extern "C" int mx_debug_matmul_plan(size_t elem_size, int which, size_t num_els, size_t nea, size_t neb, const size_t* host_metadata, const void* x, const void* y,
+                                    const void* out, int* a_mn_major, int* b_mn_major, size_t* m, size_t* n, size_t* k, int* prepared) {
     mx::MmDesc d;
     if (!host_metadata || !mx::mm_parse(host_metadata, d)) return 0;
     mx::TcProduct c;
-    if (!mx::tc_classify(d, 0, es, num_els, 0, 0, a, b, out, c)) return 0;
+    if (!mx::tc_classify(d, which, elem_size, num_els, nea, neb, x, y, out, c)) return 0;
     if (a_mn_major) *a_mn_major = c.a_mn ? 1 : 0;
     if (b_mn_major) *b_mn_major = c.b_mn ? 1 : 0;
     if (m) *m = c.m;
     if (n) *n = c.n;
     if (k) *k = c.k;
+    if (prepared) *prepared = (c.a_repack ? 1 : 0) | (c.b_repack ? 2 : 0) | (c.d_plain << 2);
     return (int)c.batch;
 }
 // 2: bf16 / f16 products run on the two-CTA kernel (pairs of SMs share the B tile); 1: on the one-CTA kernel.
@@ -1201,9 +1191,9 @@ extern "C" int mx_debug_gemm_keep_b_ctas(int tiles_m, int tiles_n, int num_kb, i
 extern "C" int mx_debug_splitk_slices(size_t tiles, size_t k, int block_k, int sms) { return mx::tc::splitk_slices(tiles, k, block_k, sms); }
 extern "C" int mx_debug_matmul_forward_path(size_t num_els, const size_t* host_metadata, const void* a, const void* b, const void* out, int* a_mn_major,
                                             int* b_mn_major, size_t* m, size_t* n, size_t* k) {
-    return debug_forward_path(2, num_els, host_metadata, a, b, out, a_mn_major, b_mn_major, m, n, k);
+    return mx_debug_matmul_plan(2, 0, num_els, 0, 0, host_metadata, a, b, out, a_mn_major, b_mn_major, m, n, k, nullptr);
 }
 extern "C" int mx_debug_matmul_forward_path_f32(size_t num_els, const size_t* host_metadata, const void* a, const void* b, const void* out,
                                                 int* a_mn_major, int* b_mn_major, size_t* m, size_t* n, size_t* k) {
-    return debug_forward_path(4, num_els, host_metadata, a, b, out, a_mn_major, b_mn_major, m, n, k);
+    return mx_debug_matmul_plan(4, 0, num_els, 0, 0, host_metadata, a, b, out, a_mn_major, b_mn_major, m, n, k, nullptr);
 }

@@ -18,18 +18,15 @@ struct TcProduct {
     int64_t a_bs, b_bs;  // elements between consecutive batches of each operand; 0 = one matrix shared by all
     uint64_t a_pitch = 0, b_pitch = 0;        // elements between rows of a copied operand (0: dense)
     bool a_repack = false, b_repack = false;  // the operand has to be copied to 16-byte-multiple rows first
-    bool ragged = false;                      // a product tc_classify leaves to the CUDA cores
+    bool ragged = false;                      // not the plain form: rows or bases off 16 bytes, batches beyond rank 3, batched backward
     bool sum_batches = false;                 // D is one [m, n] matrix, the sum of the batches' products
     int d_plain = 0;                          // the output is written without tensor stores: 1 element-wise, 2 in pairs
 };
+// Every product the kernels compute, with the fields that say what has to be prepared for it: dense and transposed operands, ragged
+// rows and unaligned bases (copied operands, plain stores), batches of any rank, batched backward products.
 // which: 0 forward, 1 grad_a, 2 grad_b (see matmul_tc.cu); elem_size in bytes.
 bool tc_classify(const MmDesc& d, int which, size_t elem_size, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, const void* out,
                  TcProduct& c);
-
-// The same for every product the kernels can compute, with the fields that say what has to be prepared for it: also ragged
-// rows and unaligned bases (copied operands, plain stores), batched backward products and contiguous operands of any rank.
-bool tc_classify_any(const MmDesc& d, int which, size_t elem_size, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, const void* out,
-                     TcProduct& c);
 
 bool tc_gemm_bf16_f16(bool is_bf16, const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out,
                       const char* where);

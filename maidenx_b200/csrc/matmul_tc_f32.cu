@@ -625,7 +625,7 @@ bool tc_launch_f32(const TcProduct& c, void* out, const char* where) { return la
 
 bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out, const char* where) {
     TcProduct c;
-    if (!tc_classify_any(d, which, 4, num_els, nea, neb, x, y, out, c)) return false;
+    if (!tc_classify(d, which, 4, num_els, nea, neb, x, y, out, c)) return false;
     StreamWorkspace ws;
     return repack_operands(4, c, ws, where) && launch(c, out, where);
 }

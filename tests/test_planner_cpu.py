@@ -5,6 +5,7 @@ import ctypes
 
 import numpy as np
 
+import harness as H
 from maidenx_b200 import _lib
 
 FLAT, ROW, TILE, GENERIC, SERIAL, FLAT_SHIFT = 1, 2, 3, 4, 5, 7
@@ -98,13 +99,56 @@ def test_the_three_products_of_a_linear_layer_run_on_the_tensor_core_kernel():
         assert mm_path([2, 2, 2, B, D, B, D, D, D, D, 1, D, 1, 0, 0], B * D) == (1, 0, 1, B, D, D)       # NN
 
 
+def mm_plan(dt, out_shape, a_shape, b_shape, ast=None, bst=None, aoff=0, boff=0, which=0, out=BASE + (2 << 32)):
+    """(batches, operand majors, M, N, K, prepared) of a product; dt "f32" or a 16-bit type.  prepared: 1 / 2 = first / second operand
+    copied, 4 / 8 = output without tensor stores, element-wise / in pairs."""
+    lib = _lib.load()
+    esz = 4 if dt == "f32" else 2
+    meta = np.asarray(H.matmul_metadata(out_shape, a_shape, b_shape, ast or H.contiguous_strides(a_shape), bst or H.contiguous_strides(b_shape), aoff, boff),
+                      dtype=np.uint64)
+    amn, bmn, prep = ctypes.c_int(-1), ctypes.c_int(-1), ctypes.c_int(-1)
+    M, N, K = ctypes.c_size_t(), ctypes.c_size_t(), ctypes.c_size_t()
+    a, b = BASE, BASE + (1 << 32)
+    x, y = {0: (a, b), 1: (a, b + boff * esz), 2: (a, b + aoff * esz)}[which]   # backward calls pass g and the other operand's first element
+    tc = lib.mx_debug_matmul_plan(esz, which, H.numel(out_shape), H.numel(a_shape), H.numel(b_shape), meta.ctypes.data, x, y, out, ctypes.byref(amn),
+                                  ctypes.byref(bmn), ctypes.byref(M), ctypes.byref(N), ctypes.byref(K), ctypes.byref(prep))
+    return (tc, amn.value, bmn.value, M.value, N.value, K.value, prep.value) if tc else 0
+
+
 def test_products_the_tensor_core_kernel_does_not_take():
     assert mm_path([2, 2, 2, 64, 64, 64, 64, 64, 64, 64, 1, 64, 1, 0, 0], 64 * 64)[0] == 0               # too small for a persistent launch
-    assert mm_path([2, 2, 2, 512, 516, 512, 512, 512, 516, 512, 1, 516, 1, 0, 0], 512 * 516)[0] == 0     # N not a multiple of 8 elements
-    assert mm_path([2, 2, 2, 512, 512, 512, 512, 512, 512, 512, 1, 512, 1, 1, 0], 512 * 512)[0] == 0     # offset 1: base not 16-byte aligned
     assert mm_path([2, 2, 2, 512, 512, 512, 512, 512, 512, 1024, 2, 512, 1, 0, 0], 512 * 512)[0] == 0    # A with a stride of 2 along k
     assert mm_path([3, 3, 3, 4, 512, 512, 4, 512, 512, 4, 512, 512, 262144, 512, 1, 262144, 512, 1, 0, 0], 4 * 512 * 512)[0] == 4  # batched rank-3: one launch, four batches
-    assert mm_path([4, 4, 4, 2, 2, 512, 512, 2, 2, 512, 512, 2, 2, 512, 512, 524288, 262144, 512, 1, 524288, 262144, 512, 1, 0, 0], 4 * 512 * 512)[0] == 0  # rank 4
+    # batches of one operand that are not whole matrices apart cannot be copied; in place they only need 16-byte strides
+    cs = [512 * 512 + 8, 512, 1]
+    assert mm_plan("bf16", [3, 512, 512], [3, 512, 512], [3, 512, 512], ast=cs)[0] == 3
+    assert mm_plan("bf16", [3, 512, 511], [3, 512, 512], [3, 512, 511], ast=cs) == 0
+    assert mm_plan("bf16", [4, 512, 512], [1, 512, 512], [4, 512, 511 + 1], aoff=1) == 0   # a size-1 batch dim: the copy would read four batches
+    assert mm_plan("bf16", [4, 512, 512], [4, 512, 512], [512, 512], which=2) == 0        # b shared by the batch: not a batched product
+
+
+def test_products_that_are_prepared_for_the_tensor_core_kernel():
+    """Operands whose rows or bases are not 16-byte multiples are copied (1, 2), output rows like that written without tensor stores
+    (4 element-wise, 8 in pairs); batches of any rank and batched backward products need nothing."""
+    assert mm_plan("bf16", [512, 516], [512, 512], [512, 516]) == (1, 0, 1, 512, 516, 512, 2 | 8)
+    assert mm_plan("bf16", [512, 515], [512, 512], [512, 515]) == (1, 0, 1, 512, 515, 512, 2 | 4)
+    assert mm_plan("bf16", [512, 516], [512, 512], [512, 516], bst=[1, 512]) == (1, 0, 0, 512, 516, 512, 8)
+    assert mm_plan("f16", [512, 512], [512, 512], [512, 512], aoff=1) == (1, 0, 1, 512, 512, 512, 1)
+    assert mm_plan("f16", [512, 512], [512, 512], [512, 512], out=BASE + 2) == (1, 0, 1, 512, 512, 512, 4)
+    assert mm_plan("f32", [512, 514], [512, 512], [512, 514]) == (1, 0, 1, 512, 514, 512, 2 | 8)
+    assert mm_plan("f32", [512, 512], [512, 511], [511, 512], ast=[1, 512]) == (1, 1, 1, 512, 512, 511, 0)
+    assert mm_plan("bf16", [2, 2, 512, 512], [2, 2, 512, 512], [2, 2, 512, 512]) == (4, 0, 1, 512, 512, 512, 0)
+    assert mm_plan("bf16", [4, 256, 512], [4, 256, 384], [4, 384, 512], which=1) == (4, 0, 0, 256, 384, 512, 0)
+    assert mm_plan("bf16", [4, 256, 512], [4, 256, 384], [4, 384, 512], which=2) == (4, 1, 1, 384, 512, 256, 0)
+    assert mm_plan("bf16", [256, 512], [256, 383], [383, 512], which=2) == (1, 1, 1, 383, 512, 256, 1)
+
+
+def test_small_16_bit_products_with_long_reductions_take_the_tensor_core_kernel():
+    assert mm_plan("bf16", [64, 64], [64, 256], [256, 64])[0] == 1
+    assert mm_plan("bf16", [64, 64], [64, 255], [255, 64]) == 0        # fewer than 256 terms
+    assert mm_plan("f16", [32, 32], [32, 256], [256, 32])[0] == 1      # 2^18 multiply-adds
+    assert mm_plan("f16", [31, 32], [31, 256], [256, 32]) == 0
+    assert mm_plan("f32", [64, 64], [64, 256], [256, 64]) == 0         # f32 keeps the element-type loop's order below 2^24
 
 
 def test_f32_products_take_the_split_tf32_kernel_when_rows_are_16_byte_multiples():
@@ -114,7 +158,6 @@ def test_f32_products_take_the_split_tf32_kernel_when_rows_are_16_byte_multiples
     # conv forward at the benchmark shape: cols [200704, 2304] . weight^T view of [256, 2304]
     assert mm_path([2, 2, 2, 200704, 256, 200704, 2304, 2304, 256, 2304, 1, 1, 2304, 0, 0], 200704 * 256, f32=True) == (1, 0, 0, 200704, 256, 2304)
     assert mm_path([2, 2, 2, 512, 516, 512, 512, 512, 516, 512, 1, 516, 1, 0, 0], 512 * 516, f32=True)[0] == 1   # 516 = 4 * 129
-    assert mm_path([2, 2, 2, 512, 514, 512, 512, 512, 514, 512, 1, 514, 1, 0, 0], 512 * 514, f32=True)[0] == 0
     assert mm_path([2, 2, 2, 64, 64, 64, 64, 64, 64, 64, 1, 64, 1, 0, 0], 64 * 64, f32=True)[0] == 0             # small: SIMT, bit-exact order
 
 
