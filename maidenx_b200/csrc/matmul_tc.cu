@@ -982,13 +982,17 @@ static bool eligible(size_t es, uint64_t M, uint64_t N, uint64_t K, uint64_t bat
     if (batch > 1 && (M * N) % q != 0) return false;  // every batch's output starts on a 16-byte boundary
     return true;
 }
+// f32 products that are not of the plain form (ragged, rank > 3, batched backward) were the CUDA cores' before; they go to the split kernel
+// only where that is no less exact.  Error against 64 bits, CUDA cores / split kernel: K = 64 1.5e-7 / 2.2e-7, 128 2.1e-7 / 2.2e-7, 192 2.5e-7
+// / 2.2e-7, 1024 5.7e-7 / 2.4e-7 for normal values; K = 128 1.6e-7 / 1.7e-7, 192 2.1e-7 / 1.7e-7 for positive ones.
+constexpr uint64_t kSplitLeastK = 192;
 // What a product of dense operands needs before the kernels can take it: an operand whose rows (or base) are not
 // 16-byte multiples is copied to padded rows first (repack_operands), an output like that is written by the epilogue warps
 // without tensor stores.  One pass over the operand against 8 TFLOP/s on the CUDA cores: bf16 4099 x 1543 x 1000, whose
 // 1543-wide matrices all need it, takes 20-40 us a product (1804 us on the CUDA cores).
 static bool plan_ragged(size_t es, TcProduct& c, const void* d, uint64_t least = kTcLeast) {
     const uint64_t q = 16 / es;
-    if (!in_range(c.m, c.n, c.k, c.batch, least)) return false;
+    if (!in_range(c.m, c.n, c.k, c.batch, least) || (es == 4 && c.k < kSplitLeastK)) return false;
     if (((uintptr_t)c.A | (uintptr_t)c.B | (uintptr_t)d) % es != 0) return false;
     const uint64_t a_cols = c.a_mn ? c.m : c.k, b_cols = c.b_mn ? c.n : c.k;
     c.a_repack = a_cols % q != 0 || (uintptr_t)c.A % 16 != 0;
@@ -1096,6 +1100,7 @@ bool tc_classify(const MmDesc& d, int which, size_t es, size_t num_els, size_t n
     // k-steps (64 x 64 x 512: 22 us, 128 x 10 x 784: 33), the tensor-core kernel's about 4.5 us, 1.6 us more per copied operand.
     // f32 keeps the line: below it results are bit for bit those of the element-type loop.
     const uint64_t least = es == 2 && c.k >= 256 ? 1ull << 18 : kTcLeast;
+    if (es == 4 && c.ragged && c.k < kSplitLeastK) return false;
     if (aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out, least)) return true;
     // the copy reads whole operands: every batch must be there (a size-1 batch dim passes the contiguity test)
     if (which == 0 && c.batch > 1 && d.a_cont && d.b_cont && (d.a_elems != c.batch * c.m * c.k || d.b_elems != c.batch * c.k * c.n)) return false;

@@ -16,8 +16,8 @@
 // accumulator only ever holds the sum of a few k-blocks: the epilogue warps drain it after every chunk and keep the
 // running total in registers, added with round-to-nearest, while the tensor core fills the other accumulator.  The pull
 // towards zero is then bounded by the chunk length whatever K is.  Two lengths: CHUNK_FAST k-blocks (128 values of K, error
-// 1e-6 of the result), and one k-block (2.2e-7) for the ragged products, which the CUDA cores computed before
-// with 2e-7 to 6e-7; a drain per k-block no longer hides behind the tensor work (conv products [256 x 1152] . [1152 x 196]: 40 us
+// 1e-6 of the result), and one k-block for the ragged products, which the CUDA cores would compute: 2.2e-7 at K = 192, where these
+// begin (CUDA cores 2.5e-7; below that K they are the more exact), 3e-7 at K = 4096 (1.1e-6); a drain per k-block no longer hides behind the tensor work (conv products [256 x 1152] . [1152 x 196]: 40 us
 // with the long chunk, 58 with the short one).  In a chunk of one the eight products with a small factor come first, so that they are summed while the accumulator is still 2^-11 of the result; longer chunks interleave them.
 //
 // One persistent CTA per SM, 320 threads in four roles:

@@ -506,3 +506,24 @@ def test_f32_backward_products_of_infinities_and_nans(oracle, cuda):
             rb = np.matmul(a.astype(np.float64).transpose(0, 2, 1), g.astype(np.float64)).astype(np.float32).reshape(-1)
         H.assert_same("matmul_backward", D.F32, got["ga"], ra, float_rel=1e-5, what="ga", scale=np.sqrt(n))
         H.assert_same("matmul_backward", D.F32, got["gb"], rb, float_rel=1e-5, what="gb", scale=np.sqrt(m))
+
+
+@pytest.mark.parametrize("k", [16, 63, 191, 192, 600])
+def test_ragged_f32_products_are_no_less_exact_than_f32_sums(cuda, k):
+    """Against 64 bits, next to a serial f32 sum with separate multiplies and adds (what the CUDA cores compute).  Below K = 192 the
+    two are the same bits; above it the split kernel's error is the smaller one (its parts lose 2^-22 a product, the serial sum half an ulp
+    of a growing total a term), 10 % are left for the sample."""
+    m, n = 1031, 1031
+    for positive in (False, True):
+        rng = np.random.default_rng(k)
+        a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+        if positive:
+            a, b = np.abs(a), np.abs(b)
+        meta = H.matmul_metadata([m, n], [m, k], [k, n], [k, 1], [n, 1], 0, 0)
+        got = H.run_matmul(cuda, D.F32, meta, m * n, a.reshape(-1), b.reshape(-1)).reshape(m, n)
+        serial = np.zeros((m, n), np.float32)
+        for i in range(k):
+            serial += a[:, i:i + 1] * b[i]
+        ref = a.astype(np.float64) @ b.astype(np.float64)
+        err = lambda x: np.linalg.norm(x - ref) / np.linalg.norm(ref)  # noqa: E731
+        assert err(got) <= 1.1 * err(serial), (k, positive, err(got), err(serial))

@@ -143,6 +143,18 @@ def test_products_that_are_prepared_for_the_tensor_core_kernel():
     assert mm_plan("bf16", [256, 512], [256, 383], [383, 512], which=2) == (1, 1, 1, 383, 512, 256, 1)
 
 
+def test_f32_products_of_short_reductions_stay_where_they_are_more_exact():
+    """Below K = 192 the sums of the CUDA cores are closer to 64 bits than the split into two tf32 parts: ragged rows, rank 4 and
+    batched backward products; the plain form keeps the split kernel at any K."""
+    for k, taken in ((191, 0), (192, 1)):
+        assert (mm_plan("f32", [1030, 515], [1030, k], [k, 515]) != 0) == taken
+        assert (mm_plan("f32", [1030, 512], [1030, k], [k, 512], aoff=1) != 0) == taken
+        assert (mm_plan("f32", [2, 4, 512, 512], [2, 4, 512, k // 4 * 4], [2, 4, k // 4 * 4, 512]) != 0) == taken
+        assert (mm_plan("f32", [8, 512, k], [8, 512, 512], [8, 512, k], which=1) != 0) == taken
+        assert (mm_plan("f32", [8, k, 512], [8, k, 512], [8, 512, 512], which=2) != 0) == taken
+    assert mm_plan("f32", [1024, 512], [1024, 64], [64, 512])[0] == 1
+
+
 def test_small_16_bit_products_with_long_reductions_take_the_tensor_core_kernel():
     assert mm_plan("bf16", [64, 64], [64, 256], [256, 64])[0] == 1
     assert mm_plan("bf16", [64, 64], [64, 255], [255, 64]) == 0        # fewer than 256 terms
