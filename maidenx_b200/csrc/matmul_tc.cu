@@ -838,6 +838,14 @@ __global__ void __launch_bounds__(256) repack_rows_kernel(const W* __restrict__ 
     }
 }
 
+// Elements between the rows of a copy.  Whole 128-byte lines, so that a tensor copy's 128-byte box rows read one line each and
+// not parts of two (bf16 100000 x 3 x 257: 19 us, 40 with the 257 rows of three elements 16 bytes apart); where rows shorter than a line would
+// make that much memory, the 16-byte multiple that a tensor map asks for.
+uint64_t copy_pitch(size_t es, uint64_t rows, uint64_t cols) {
+    const uint64_t q = (cols * es >= 128 || rows <= kCopyFree / 128 ? 128 : 16) / es;
+    return (cols + q - 1) / q * q;
+}
+
 static bool repack_rows(size_t es, const void* in, void* out, uint64_t rows, uint64_t cols, uint64_t pitch) {
     const uint64_t per_row = (cols * es + 15) / 16, vecs = rows * per_row;  // the padding itself is never read
     uint64_t blocks = (vecs + 255) / 256;
@@ -855,10 +863,8 @@ static bool repack_rows(size_t es, const void* in, void* out, uint64_t rows, uin
 
 bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* where) {
     if (!c.a_repack && !c.b_repack) return true;
-    // rows of whole 128-byte lines: a tensor copy's 128-byte box rows then read one line each, not parts of two
-    const uint64_t q = 128 / es;
-    const uint64_t a_rows = (c.a_mn ? c.k : c.m) * (c.a_bs ? c.batch : 1), a_cols = c.a_mn ? c.m : c.k, a_pitch = (a_cols + q - 1) / q * q;
-    const uint64_t b_rows = (c.b_mn ? c.k : c.n) * (c.b_bs ? c.batch : 1), b_cols = c.b_mn ? c.n : c.k, b_pitch = (b_cols + q - 1) / q * q;
+    const uint64_t a_rows = (c.a_mn ? c.k : c.m) * (c.a_bs ? c.batch : 1), a_cols = c.a_mn ? c.m : c.k, a_pitch = copy_pitch(es, a_rows, a_cols);
+    const uint64_t b_rows = (c.b_mn ? c.k : c.n) * (c.b_bs ? c.batch : 1), b_cols = c.b_mn ? c.n : c.k, b_pitch = copy_pitch(es, b_rows, b_cols);
     const uint64_t a_bytes = c.a_repack ? (a_rows * a_pitch * es + 255) / 256 * 256 : 0, b_bytes = c.b_repack ? b_rows * b_pitch * es : 0;
     if (a_bytes / 16 > 0x7FFFFFFFull || b_bytes / 16 > 0x7FFFFFFFull) return false;  // the copy counts vectors in 32 bits
     if (!ws.take(a_bytes + b_bytes)) return false;
@@ -997,6 +1003,12 @@ static bool plan_ragged(size_t es, TcProduct& c, const void* d, uint64_t least =
     const uint64_t a_cols = c.a_mn ? c.m : c.k, b_cols = c.b_mn ? c.n : c.k;
     c.a_repack = a_cols % q != 0 || (uintptr_t)c.A % 16 != 0;
     c.b_repack = b_cols % q != 0 || (uintptr_t)c.B % 16 != 0;
+    const uint64_t a_rows = (c.a_mn ? c.k : c.m) * (c.a_bs ? c.batch : 1), b_rows = (c.b_mn ? c.k : c.n) * (c.b_bs ? c.batch : 1);
+    const uint64_t a_copy = c.a_repack ? a_rows * tc::copy_pitch(es, a_rows, a_cols) * es : 0, b_copy = c.b_repack ? b_rows * tc::copy_pitch(es, b_rows, b_cols) * es : 0;
+    // The copies are workspace that a caller does not see: at most twice the operands where they are large (rows of one to three
+    // elements grow up to eightfold), and 8 GB in all.  What is beyond runs on the CUDA cores.
+    const uint64_t dense = (c.a_repack ? a_rows * a_cols * es : 0) + (c.b_repack ? b_rows * b_cols * es : 0);
+    if (a_copy + b_copy > 2 * dense + 2 * tc::kCopyFree || a_copy + b_copy > (8ull << 30)) return false;
     if (c.batch > 1) {
         // the batches of a copied operand must lie one after the other; an uncopied one's batch stride is a tensor-map stride
         if (c.a_bs != 0 && c.a_bs != (int64_t)(c.m * c.k)) return false;
@@ -1092,16 +1104,34 @@ static bool aligned_batches(size_t es, const TcProduct& c) {
 // reduction over n, both operands K-major.  2: grad_b[k, n] = sum_m A[m, k] * g[m, n] (x = g, y = A + offset),
 // reduction over m, both operands MN-major.  The backward products read g, A and B as dense row-major matrices
 // (strides ignored, crates/maidenx_cpu/src/ops/matmul.rs:196-261).
+// Few outputs and a long reduction: matmul_longk_kernel (a block per output) is done before 128-row tiles have been cut into runs, copied
+// and summed.  16-bit, longk / tensor cores, both operands K-major: 16 x 64 x 4100 7.9 / 12.1 us, x 8192 12.3 / 8.5; 32 x 32 x 2048 5.1 / 7.3; 1 x 64
+// x 16384 9.0 / 10.7, x 32768 16.1 / 12.2; an MN-major B costs longk a line per element: 16 x 64 x 4100 22.9 / 10.3, 1 x 256 x 8192 11.2 / 11.2, x
+// 16384 19.9 / 13.1.  f32 pays for its drains: 784 x 1 x 65536 70 / 140 us, 5 x 5 x 2^20 333 / 516; only where A lies MN-major does
+// it gain (10 x 64 x 32768 103 / 30, 10 x 32 x 60000 120 / 86).
+static bool longk_better(size_t es, const TcProduct& c) {
+    const uint64_t outputs = c.batch * c.m * c.n;
+    if (c.k < kLongKMinK || outputs > kLongKMaxOutputs) return false;
+    if (es != 2) return !(c.a_mn && outputs >= 256);
+    const bool b_across = c.b_mn && c.n >= 32;
+    return !(c.k >= 32768 || (outputs >= 512 && c.k >= (b_across ? 4096 : 8192)) || (b_across && outputs >= 64 && c.k >= 16384));
+}
+
 bool tc_classify(const MmDesc& d, int which, size_t es, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, const void* out,
                      TcProduct& c) {
     if (which == 0 ? !forward_operands(d, es, num_els, x, y, c) : !backward_operands(d, which, nea, neb, x, y, c)) return false;
+    // a matrix of one column is the same memory as one of one row, and K-major it needs no copy of its one-element rows
+    if (c.m == 1) c.a_mn = false;
+    if (c.n == 1) c.b_mn = false;
     c.ragged = d.out_nd > (which == 0 ? 3 : 2);  // aligned, but new to these kernels: batches beyond rank 3, batched backward
     // 16-bit products far below kTcLeast still gain when their reduction is long: the CUDA-core kernel's time is its chain of
     // k-steps (64 x 64 x 512: 22 us, 128 x 10 x 784: 33), the tensor-core kernel's about 4.5 us, 1.6 us more per copied operand.
     // f32 keeps the line: below it results are bit for bit those of the element-type loop.
     const uint64_t least = es == 2 && c.k >= 256 ? 1ull << 18 : kTcLeast;
     if (es == 4 && c.ragged && c.k < kSplitLeastK) return false;
-    if (aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out, least)) return true;
+    if (aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out, least))
+        return !((c.ragged || c.batch * c.m * c.n * c.k < kTcLeast) && longk_better(es, c));
+    if (longk_better(es, c)) return false;
     // the copy reads whole operands: every batch must be there (a size-1 batch dim passes the contiguity test)
     if (which == 0 && c.batch > 1 && d.a_cont && d.b_cont && (d.a_elems != c.batch * c.m * c.k || d.b_elems != c.batch * c.k * c.n)) return false;
     return plan_ragged(es, c, out, least);

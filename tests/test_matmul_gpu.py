@@ -527,3 +527,24 @@ def test_ragged_f32_products_are_no_less_exact_than_f32_sums(cuda, k):
         ref = a.astype(np.float64) @ b.astype(np.float64)
         err = lambda x: np.linalg.norm(x - ref) / np.linalg.norm(ref)  # noqa: E731
         assert err(got) <= 1.1 * err(serial), (k, positive, err(got), err(serial))
+
+
+@pytest.mark.parametrize("dt", [D.BF16, D.F16, D.F32], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [(1, 1, 1 << 20), (1, 1, 65537), (1, 1003, 8200), (1003, 1, 40001), (700, 1, 33000), (3, 5, 40000), (32, 32, 8191), (30, 30, 9001), (4099, 3, 300), (2, 9001, 1003)],
+                         ids=lambda c: "x".join(map(str, c)))
+def test_vectors_narrow_matrices_and_few_outputs(oracle, cuda, dt, case):
+    """One row or column (K-major whatever its strides say), rows of a few elements (copied to 16-byte rows) and few outputs with long
+    reductions, on both sides of the line to the block-per-output kernel.  Bounds as above."""
+    from oracle import binding
+    m, n, k = case
+    rng = np.random.default_rng(m + n + k)
+    for amaj, bmaj in (("k", "mn"), ("mn", "mn"), ("k", "k")):
+        a, b = H.random_store(rng, dt, m * k, dist="normal"), H.random_store(rng, dt, k * n, dist="normal")
+        meta = H.matmul_metadata([m, n], [m, k], [k, n], [k, 1] if amaj == "k" else [1, m], [n, 1] if bmaj == "mn" else [1, k], 0, 0)
+        got = H.run_matmul(cuda, dt, meta, m * n, a, b)
+        binding.set_wide(True)
+        try:
+            ref = H.run_matmul(oracle, dt, meta, m * n, a, b)
+        finally:
+            binding.set_wide(False)
+        H.assert_same("matmul", dt, got, ref, float_rel=1e-5 if dt.name == "f32" else 1e-2, what=f"{case} {amaj}{bmaj}", scale=np.sqrt(k))

@@ -155,6 +155,27 @@ def test_f32_products_of_short_reductions_stay_where_they_are_more_exact():
     assert mm_plan("f32", [1024, 512], [1024, 64], [64, 512])[0] == 1
 
 
+def test_copies_stay_small_and_few_outputs_stay_with_their_kernel():
+    # a vector is K-major whatever its strides say: nothing is copied where a [K, 1] matrix would grow eightfold
+    assert mm_plan("bf16", [1, 1], [1, 1 << 24], [1 << 24, 1]) == (1, 0, 0, 1, 1, 1 << 24, 4)
+    assert mm_plan("bf16", [1, 4096], [1, 4096], [4096, 4096], ast=[1, 1]) == (1, 0, 1, 1, 4096, 4096, 0)
+    assert mm_plan("f32", [784, 1], [784, 65536], [65536, 1], ast=[1, 784]) == (1, 1, 0, 784, 1, 65536, 4)
+    # rows of two elements: four times their size, taken while that is little memory
+    assert mm_plan("bf16", [2, 4096], [2, 1 << 20], [1 << 20, 4096], ast=[1, 2])[6] == 1
+    assert mm_plan("bf16", [2, 4096], [2, 1 << 22], [1 << 22, 4096], ast=[1, 2]) == 0
+    assert mm_plan("f32", [70000, 40000], [70000, 32767], [32767, 40000]) == 0              # 9 GB of copies
+    # at most 1024 outputs, 2048 terms or more
+    assert mm_plan("bf16", [32, 32], [32, 4095], [4095, 32]) == 0
+    assert mm_plan("bf16", [32, 32], [32, 4096], [4096, 32])[0] == 1
+    assert mm_plan("bf16", [32, 32], [32, 4096], [4096, 32], bst=[1, 4096]) == 0
+    assert mm_plan("bf16", [32, 32], [32, 8192], [8192, 32])[0] == 1
+    assert mm_plan("f16", [8, 8], [8, 16384], [16384, 8]) == 0
+    assert mm_plan("f16", [8, 8], [8, 32768], [32768, 8])[0] == 1
+    assert mm_plan("bf16", [32, 32], [32, 16384], [16384, 32])[0] == 1                       # 2^24 multiply-adds, plain form: as ever
+    assert mm_plan("f32", [5, 5], [5, 1 << 20], [1 << 20, 5]) == 0
+    assert mm_plan("f32", [10, 100], [10, 60000], [60000, 100], ast=[1, 10])[0] == 1
+
+
 def test_small_16_bit_products_with_long_reductions_take_the_tensor_core_kernel():
     assert mm_plan("bf16", [64, 64], [64, 256], [256, 64])[0] == 1
     assert mm_plan("bf16", [64, 64], [64, 255], [255, 64]) == 0        # fewer than 256 terms
