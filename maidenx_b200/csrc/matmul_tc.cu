@@ -68,6 +68,12 @@ struct SmemLayout {
 };
 constexpr int TC_SMEM_BYTES = SmemLayout::total + 1024;  // slack for the 1024-byte alignment
 
+// 16-bit products that the CUDA cores would compute (ragged, rank > 3, batched backward, small) with an f32 sum rounded to nearest.  The
+// tensor core's additions truncate, which pulls a long sum of one sign towards zero: measured 6e-6 of it in 1024 terms, at most an ulp (2^-23)
+// for each instruction's 16.  After runs of these many terms the accumulator is added to f32 totals, so that the pull stays far below the
+// rounding to the type (2.2e-4 f16, 1.8e-3 bf16 for positive sums): f16 K = 16385 2.209e-4 on the CUDA cores, 2.237e-4 in one run.
+constexpr int kRunMostF16 = 1024, kRunMostBf16 = 4096;
+
 // Split-K of a short reduction: what its second launch and the wider partial results cost, in k-blocks (0.27 us each on one CTA)
 constexpr double kSplitFixed16 = 10.0;
 
@@ -105,6 +111,7 @@ struct TcParams {
     // warps copy their staged rows to `d` themselves, in steps of 2 bytes (1) or, for even N, 4 bytes (2).  0: tensor stores.
     int d_plain;
     void* d;
+    int run_kb;      // DRAIN form: k-blocks summed in one accumulator before the epilogue adds them to its own f32 totals
     // Short reductions (num_kb <= STAGES, one batch): `b_keep` CTAs share each column tile, CTA j of them takes the row
     // tiles j, j + b_keep, ...; the B panel of the column tile is loaded once into the B slots of the ring (slot = k-block,
     // the ring is num_kb slots long) and only A streams.  0: the general schedule.
@@ -163,7 +170,9 @@ enum TcMode {
 // BN_T: the tile's columns where they are 256, else 0 (from the parameters).  The ring of full-width tiles is four stages deep and waits
 // out a round trip to L2 in them, so the single producer thread's own instructions between a freed stage and its refill count:
 // with the geometry from the parameters the products of a 16384 x 8192 layer took 12 % longer at full clock.
-template <int MODE, int BN_T>
+// DRAIN (tiles of at most 128 columns): the accumulator is emptied every run_kb k-blocks into totals in registers, added with
+// round-to-nearest, so that the pull of the tensor core's truncating additions stays that of one run whatever K is (see kRunMostF16).
+template <int MODE, int BN_T, bool DRAIN = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                const __grid_constant__ CUtensorMap map_d2, TcParams p, int* err, int tag) {
@@ -253,11 +262,13 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             bool ok = true;
             const int ring = p.b_keep ? p.num_kb : stages;
             int tm, tn, tb;
-            for (int it = 0; ok && next_tile(it, p, tm, tn, tb); it++) {
+            int run = 0;  // first k-block of the accumulator's run (DRAIN: a tile has several)
+            for (int it = 0; ok && next_tile(it, p, tm, tn, tb); it += DRAIN && run ? 0 : 1) {
                 if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1, err, tag, 2)) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
-                for (int kb = 0; kb < p.num_kb; kb++) {
+                const int run_end = DRAIN ? min(run + p.run_kb, p.num_kb) : p.num_kb;
+                for (int kb = run; kb < run_end; kb++) {
                     if (!mbar_wait(full_bar(stage), phase, err, tag, 3)) {
                         ok = false;
                         break;
@@ -266,7 +277,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     const uint32_t sa = smem_base + SmemLayout::ring + stage * stage_bytes;
                     const uint64_t da = smem_desc_sw128(sa, a_lbo, 1024), db = smem_desc_sw128(sa + A_STAGE_BYTES, b_lbo, 1024);
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; k++) umma_f16(d_tmem, da + a_kstep * k, db + b_kstep * k, idesc, (kb | k) != 0);
+                    for (int k = 0; k < BK / UMMA_K; k++) umma_f16(d_tmem, da + a_kstep * k, db + b_kstep * k, idesc, ((kb - run) | k) != 0);
                     umma_commit(empty_bar(stage));  // the stage may be refilled once these MMAs have read it
                     if (++stage == ring) {
                         stage = 0;
@@ -275,6 +286,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 if (!ok) break;
                 umma_commit(tfull_bar(acc));  // accumulator complete
+                if (DRAIN) run = run_end < p.num_kb ? run_end : 0;
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;
@@ -299,9 +311,13 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const int row = tm * BM + quarter * 32 + lane;
                 fused_bias = row < p.M ? (p.is_bf16 ? to_f32(static_cast<const bf16*>(p.bias)[row]) : to_f32(static_cast<const f16*>(p.bias)[row])) : 0.0f;
             }
-            const bool ready = mbar_wait_relaxed(tfull_bar(acc), acc_phase, err, tag, 4, 400);
-            if (!__all_sync(0xFFFFFFFFu, ready)) break;
-            tc_fence_after();
+            auto wait_accumulator = [&] {
+                const bool ready = mbar_wait_relaxed(tfull_bar(acc), acc_phase, err, tag, 4, 400);
+                if (!__all_sync(0xFFFFFFFFu, ready)) return false;
+                tc_fence_after();
+                return true;
+            };
+            if (!DRAIN && !wait_accumulator()) break;
             const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
             const int rows_here = min(32, p.M - (tm * BM + quarter * 32));  // may be <= 0: this warp's rows lie below the matrix
             // Hands the staged 32 rows of 128 bytes (first output column `col`) to the copy engine, or writes them itself.
@@ -427,6 +443,36 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 __syncwarp();
                 if (lane == 0) mbar_arrive(tempty_bar(acc));
             };
+            if constexpr (DRAIN) {
+                uint32_t total[4][32], v[32];
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+#pragma unroll
+                    for (int j = 0; j < 32; j++) total[c][j] = 0;  // 0.0f
+                bool ok = true;
+                for (int run = 0; run < p.num_kb && ok; run += p.run_kb) {
+                    ok = wait_accumulator();
+                    if (!ok) break;
+                    const uint32_t t_run = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        if (c * 32 >= bn) break;
+                        tmem_ld_32x32b_x32(t_run + c * 32, v);
+                        tmem_ld_wait_for(v);
+#pragma unroll
+                        for (int j = 0; j < 32; j++) total[c][j] = __float_as_uint(__uint_as_float(total[c][j]) + __uint_as_float(v[j]));
+                    }
+                    hand_back();
+                    if (++acc == 2) {
+                        acc = 0;
+                        acc_phase ^= 1;
+                    }
+                }
+                if (!ok) break;
+                store_chunk(0, total[0], total[1]);
+                if (chunks > 1) store_chunk(1, total[2], total[3]);
+                continue;
+            }
             uint32_t a0[32], a1[32], b0[32], b1[32];
             tmem_ld_32x32b_x32(t_row, a0);
             tmem_ld_32x32b_x32(t_row + 32, a1);
@@ -493,7 +539,8 @@ bool opt_in_shared_memory() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
-        for (auto kernel : {tc_gemm_kernel<TC_STORE, BN>, tc_gemm_kernel<TC_BIAS, BN>, tc_gemm_kernel<TC_STORE, 0>, tc_gemm_kernel<TC_BIAS, 0>, tc_gemm_kernel<TC_PLAIN, 0>})
+        for (auto kernel : {tc_gemm_kernel<TC_STORE, BN>, tc_gemm_kernel<TC_BIAS, BN>, tc_gemm_kernel<TC_STORE, 0>, tc_gemm_kernel<TC_BIAS, 0>, tc_gemm_kernel<TC_PLAIN, 0>,
+                            tc_gemm_kernel<TC_STORE, 0, true>, tc_gemm_kernel<TC_BIAS, 0, true>, tc_gemm_kernel<TC_PLAIN, 0, true>})
             if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
@@ -631,6 +678,12 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
         p.bn = bn_whole;
         p.tiles_n = (int)((N + p.bn - 1) / p.bn);
     }
+    p.run_kb = c.nearest ? (is_bf16 ? kRunMostBf16 : kRunMostF16) / BK : 0;
+    const bool drain = p.run_kb && p.num_kb > p.run_kb;
+    if (drain && p.bn > 128) {
+        p.bn = 128;
+        p.tiles_n = (int)((N + p.bn - 1) / p.bn);
+    }
     p.tiles_per_batch = p.tiles_m * p.tiles_n;
     p.stages = ring_stages(p.bn);
     p.stage_bytes = A_STAGE_BYTES + p.bn * BK * 2;
@@ -665,7 +718,8 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     if (grid > p.num_tiles) grid = p.num_tiles;
     if (p.b_keep) grid = p.b_keep * p.tiles_n;
     const bool full = p.bn == BN;
-    const auto kernel = p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0>
+    const auto kernel = drain ? (p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0, true> : (fuse ? tc_gemm_kernel<TC_BIAS, 0, true> : tc_gemm_kernel<TC_STORE, 0, true>))
+                        : p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0>
                                   : (fuse ? (full ? tc_gemm_kernel<TC_BIAS, BN> : tc_gemm_kernel<TC_BIAS, 0>) : (full ? tc_gemm_kernel<TC_STORE, BN> : tc_gemm_kernel<TC_STORE, 0>));
     kernel<<<grid, TC_THREADS, TC_SMEM_BYTES, ctx().stream>>>(ma, mb, md, md2, p, err, tag);
     check_launch(where);
@@ -1015,6 +1069,7 @@ static bool plan_ragged(size_t es, TcProduct& c, const void* d, uint64_t least =
         if (c.b_bs != 0 && c.b_bs != (int64_t)(c.k * c.n)) return false;
     }
     c.ragged = true;
+    c.nearest = es == 2;
     const bool plain = c.n % q != 0 || (uintptr_t)d % 16 != 0;
     c.d_plain = !plain ? 0 : (c.n % 2 == 0 && (uintptr_t)d % 4 == 0 ? 2 : 1);
     return true;
@@ -1129,8 +1184,11 @@ bool tc_classify(const MmDesc& d, int which, size_t es, size_t num_els, size_t n
     // f32 keeps the line: below it results are bit for bit those of the element-type loop.
     const uint64_t least = es == 2 && c.k >= 256 ? 1ull << 18 : kTcLeast;
     if (es == 4 && c.ragged && c.k < kSplitLeastK) return false;
-    if (aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out, least))
-        return !((c.ragged || c.batch * c.m * c.n * c.k < kTcLeast) && longk_better(es, c));
+    if (aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out, least)) {
+        const bool plain_form = !c.ragged && c.batch * c.m * c.n * c.k >= kTcLeast;
+        c.nearest = es == 2 && !plain_form;
+        return plain_form || !longk_better(es, c);
+    }
     if (longk_better(es, c)) return false;
     // the copy reads whole operands: every batch must be there (a size-1 batch dim passes the contiguity test)
     if (which == 0 && c.batch > 1 && d.a_cont && d.b_cont && (d.a_elems != c.batch * c.m * c.k || d.b_elems != c.batch * c.k * c.n)) return false;

@@ -19,6 +19,7 @@ struct TcProduct {
     uint64_t a_pitch = 0, b_pitch = 0;        // elements between rows of a copied operand (0: dense)
     bool a_repack = false, b_repack = false;  // the operand has to be copied to 16-byte-multiple rows first
     bool ragged = false;                      // not the plain form: rows or bases off 16 bytes, batches beyond rank 3, batched backward
+    bool nearest = false;                     // 16-bit: a sum that the CUDA cores would round to nearest (see kRunMostF16)
     bool sum_batches = false;                 // D is one [m, n] matrix, the sum of the batches' products
     int d_plain = 0;                          // the output is written without tensor stores: 1 element-wise, 2 in pairs
 };

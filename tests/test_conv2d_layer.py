@@ -160,6 +160,8 @@ RAGGED_TC = [
     (6, 24, 12, 12, 136, 3, 3, 1, 1, 1, 1),   # P = 144: the weight gradient is one product over batch and positions
     (40, 24, 7, 7, 72, 3, 3, 1, 1, 1, 1),
     (10, 16, 15, 15, 72, 5, 5, 2, 2, 2, 2),
+    (40, 128, 7, 7, 72, 3, 3, 1, 1, 1, 1),    # reductions beyond one f16 accumulator run, with the bias in the epilogue
+    (40, 129, 8, 8, 72, 3, 3, 1, 1, 1, 1),    # the same with copied weights and tensor stores
     (33, 64, 8, 8, 40, 1, 1, 1, 1, 0, 0),     # many batches of one k-block each, split over CTAs
 ]
 

@@ -548,3 +548,34 @@ def test_vectors_narrow_matrices_and_few_outputs(oracle, cuda, dt, case):
         finally:
             binding.set_wide(False)
         H.assert_same("matmul", dt, got, ref, float_rel=1e-5 if dt.name == "f32" else 1e-2, what=f"{case} {amaj}{bmaj}", scale=np.sqrt(k))
+
+
+@pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [("plain-stores", [], 1290, 1801, 2100, "k", "k"), ("copies", [], 1289, 1800, 3001, "mn", "mn"), ("one-run", [], 1290, 1801, 1024, "k", "k"),
+                                  ("one-more", [], 1290, 1801, 1025, "k", "k"), ("batched", [3], 264, 517, 8500, "k", "mn"), ("narrow", [2, 2], 515, 40, 3300, "k", "mn"),
+                                  ("split", [], 130, 131, 9001, "k", "k")], ids=lambda c: c[0])
+def test_long_sums_of_one_sign_in_16_bit_products(cuda, dt, case):
+    """The tensor core's additions truncate; after runs of 1024 (f16) or 4096 (bf16) terms the accumulator is emptied into totals rounded to
+    nearest.  Error against 64 bits after the rounding to the type, next to rounding the exact result once.  An instruction adds 16 terms
+    and loses at most an ulp, 2^-23, of the accumulator: 64 of them pull by 7.7e-6 of the result, 256 by 3.1e-5.  Next to 2.2e-4 (f16) and 1.8e-3
+    (bf16) of the rounding that adds 0.06 and 0.02 % to the error's norm."""
+    name, bd, m, n, k, amaj, bmaj = case
+    rng = np.random.default_rng(zlib_seed(name))
+    cs = H.contiguous_strides
+    nb = H.numel(bd) if bd else 1
+    a = D.encode((np.abs(rng.standard_normal((nb, m, k))) / np.sqrt(k)).astype(np.float32).reshape(-1), dt)
+    b = D.encode((np.abs(rng.standard_normal((nb, k, n))) / np.sqrt(k)).astype(np.float32).reshape(-1), dt)
+    av = D.decode(a, dt).astype(np.float64).reshape(nb, m, k)
+    bv = D.decode(b, dt).astype(np.float64).reshape(nb, k, n)
+    ast, bst = cs([*bd, m, k]), cs([*bd, k, n])
+    if amaj == "mn":
+        a, ast = np.ascontiguousarray(a.reshape(m, k).T).reshape(-1), [1, m]
+    if bmaj == "k" and not bd:
+        b, bst = np.ascontiguousarray(b.reshape(k, n).T).reshape(-1), [1, k]
+    meta = H.matmul_metadata([*bd, m, n], [*bd, m, k], [*bd, k, n], ast, bst, 0, 0)
+    got = D.decode(H.run_matmul(cuda, dt, meta, nb * m * n, a, b), dt).astype(np.float64)
+    ref = np.matmul(av, bv).reshape(-1)
+    once = D.decode(D.encode(ref.astype(np.float32), dt), dt).astype(np.float64)
+    err = lambda x: np.linalg.norm(x - ref) / np.linalg.norm(ref)  # noqa: E731
+    assert err(got) <= 1.001 * err(once), (err(got), err(once))
+    assert abs(((got - once) / ref).mean()) < (64 if dt.name == "f16" else 256) * 2.0 ** -23 + 4 * err(once) / np.sqrt(ref.size)
