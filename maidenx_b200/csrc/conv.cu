@@ -207,6 +207,14 @@ __global__ void __launch_bounds__(kConvThreads) col2im_kernel(const T* __restric
     out[bc * HW + pix] = sum;
 }
 
+// The limit is the same in every call, whatever the call needs: with each call setting its own, a thread with small planes
+// took back what a thread with large ones had just asked for, and the larger launch was refused.
+constexpr int kConvSmemMost = 200 * 1024;
+template <class K>
+static void allow_shared_memory(K kernel, size_t bytes) {
+    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmemMost);
+}
+
 static bool conv_params(const size_t* meta, size_t num_els, ConvParams& P, const char* where) {
     const size_t* m = resolve_metadata(meta, 12);
     if (!m) return false;
@@ -286,11 +294,11 @@ void im2col_entry(size_t num_els, const size_t* meta, const T* x, T* col, const 
         Q.num_els = num_els;
         const size_t smem = (size_t)(P.H + 2 * P.PH) * Q.pitch * sizeof(T);
         auto go = [&](auto kernel) {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_shared_memory(kernel, smem);
             kernel<<<grid, kConvS1Threads, smem, s>>>(x, col, Q);
             check_launch(where);
         };
-        if (smem <= 200 * 1024) {
+        if (smem <= kConvSmemMost) {
             switch (P.KW) {
                 case 1: go(im2col_s1_kernel<T, VEC, 1>); return;
                 case 3: if (VEC >= 2) { go(im2col_s1_kernel<T, VEC, 3>); return; } break;
@@ -304,14 +312,14 @@ void im2col_entry(size_t num_els, const size_t* meta, const T* x, T* col, const 
     uint64_t step = 1;
     while (step < VEC && (chunk * step) % VEC != 0) step *= 2;
     const bool col_aligned = (uintptr_t)col % 16 == 0;
-    const uint32_t pb_vec = col_aligned ? planes_per_block(planes_touched, plane_bytes, step, step == 1 ? 200 * 1024 : 48 * 1024) : 0;
-    const uint32_t pb = pb_vec ? pb_vec : planes_per_block(planes_touched, plane_bytes, 1, 200 * 1024);
+    const uint32_t pb_vec = col_aligned ? planes_per_block(planes_touched, plane_bytes, step, step == 1 ? kConvSmemMost : 48 * 1024) : 0;
+    const uint32_t pb = pb_vec ? pb_vec : planes_per_block(planes_touched, plane_bytes, 1, kConvSmemMost);
     if (pb && pb * chunk < 0x7FFFFFFFull) {
         P.planes = (uint32_t)planes_touched;
         P.per_block = pb;
         const size_t smem = pb * plane_bytes;
         auto launch = [&](auto kernel) {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_shared_memory(kernel, smem);
             kernel<<<(unsigned)((planes_touched + pb - 1) / pb), kConvThreads, smem, s>>>(x, col, P);
         };
         if (pb_vec) launch(im2col_planes_kernel<T, VEC>);
@@ -355,7 +363,7 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
             const size_t stage_bytes = (size_t)plane_elems * sizeof(T);
             if (num_els >= planes * plane_elems && stage_bytes % 16 == 0 && stage_bytes <= 112 * 1024 && plane_elems < (1ull << 30)) {
                 auto go = [&](auto kernel) {
-                    if (stage_bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_bytes);
+                    allow_shared_memory(kernel, stage_bytes);
                     kernel<<<(unsigned)planes, kConvS1Threads, stage_bytes, s>>>(col, out, Q, tc::next_wait_report());
                     check_launch(where);
                 };
@@ -385,7 +393,7 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
         P.per_block = pb;
         const size_t smem = pb * col_plane * sizeof(T);
         auto launch = [&](auto kernel) {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_shared_memory(kernel, smem);
             kernel<<<(unsigned)((planes + pb - 1) / pb), kConvThreads, smem, s>>>(col, out, P);
         };
         if (P.SH == 1 && P.SW == 1) launch(col2im_planes_kernel<T, true>);

@@ -111,3 +111,35 @@ def test_planes_sharing_a_block(oracle, cuda, dt, case):
         H.assert_same("conv2d_im2col", dt, H.run_im2col(cuda, dt, meta, n, x), H.run_im2col(oracle, dt, meta, n, x), what=f"{case[0]} {n}")
     for n in (ncol, ncol // 2 + 1):
         H.assert_same("conv2d_col2im", dt, H.run_col2im(cuda, dt, meta, n, col, out_len), H.run_col2im(oracle, dt, meta, n, col, out_len), what=f"{case[0]} {n}")
+
+
+def test_threads_with_planes_of_different_sizes(cuda):
+    """Two threads whose planes need different amounts of shared memory beyond 48 KB: neither may take back the limit that the other
+    has just asked for (its launch would be refused)."""
+    import threading
+
+    dt = D.F32
+    trouble = []
+
+    def work(side, seed):
+        rng = np.random.default_rng(seed)
+        B, C, kh, kw = 1, 2, 3, 3
+        o = (side + 2 - 3) // 2 + 1
+        meta = H.conv_metadata(B, C, side, side, kh, kw, o, o, 1, 1, 2, 2)
+        x = H.random_store(rng, dt, C * side * side, dist="normal")
+        n = C * kh * kw * o * o
+        first = None
+        try:
+            for _ in range(150):
+                got = H.run_im2col(cuda, dt, meta, n, x)
+                first = got if first is None else first
+                assert np.array_equal(got, first)
+        except Exception as e:  # noqa: BLE001
+            trouble.append((side, repr(e)))
+
+    ts = [threading.Thread(target=work, args=a) for a in ((121, 1), (213, 2), (151, 3))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not trouble, trouble
