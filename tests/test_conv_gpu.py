@@ -114,32 +114,35 @@ def test_planes_sharing_a_block(oracle, cuda, dt, case):
 
 
 def test_threads_with_planes_of_different_sizes(cuda):
-    """Two threads whose planes need different amounts of shared memory beyond 48 KB: neither may take back the limit that the other
-    has just asked for (its launch would be refused)."""
+    """Threads whose planes need different amounts of shared memory beyond 48 KB, calling as fast as they can: none may take back the
+    limit that another has just asked for (its launch would be refused)."""
+    import ctypes
     import threading
 
-    dt = D.F32
-    trouble = []
+    from maidenx_b200 import _lib
 
-    def work(side, seed):
-        rng = np.random.default_rng(seed)
-        B, C, kh, kw = 1, 2, 3, 3
-        o = (side + 2 - 3) // 2 + 1
-        meta = H.conv_metadata(B, C, side, side, kh, kw, o, o, 1, 1, 2, 2)
-        x = H.random_store(rng, dt, C * side * side, dist="normal")
-        n = C * kh * kw * o * o
-        first = None
-        try:
-            for _ in range(150):
-                got = H.run_im2col(cuda, dt, meta, n, x)
-                first = got if first is None else first
-                assert np.array_equal(got, first)
-        except Exception as e:  # noqa: BLE001
-            trouble.append((side, repr(e)))
+    dt, lib, op = D.F32, _lib.load(), _lib.op("conv2d_im2col", "f32")
+    start, trouble = threading.Barrier(4), []
 
-    ts = [threading.Thread(target=work, args=a) for a in ((121, 1), (213, 2), (151, 3))]
+    def work(side):
+        C, o = 2, (side + 2 - 3) // 2 + 1
+        meta = np.asarray(H.conv_metadata(1, C, side, side, 3, 3, o, o, 1, 1, 2, 2), dtype=np.uint64)
+        x = H.random_store(np.random.default_rng(side), dt, C * side * side, dist="normal")
+        n = C * 9 * o * o
+        bx, bc = cuda.dev.CudaBuffer.from_host(x), cuda.dev.CudaBuffer.from_host(np.zeros(n, np.float32))
+        start.wait()
+        for _ in range(4000):
+            op(ctypes.c_size_t(n), meta.ctypes.data, bx.ptr, bc.ptr)
+        trouble.append(lib.mx_last_error())
+        lib.mx_clear_error()
+        cuda.dev.synchronize()
+        trouble.append(0 if np.array_equal(bc.to_host(np.float32, n), H.run_im2col(cuda, dt, list(map(int, meta)), n, x)) else side)
+        bx.free()
+        bc.free()
+
+    ts = [threading.Thread(target=work, args=(side,)) for side in (121, 213, 151, 187)]
     for t in ts:
         t.start()
     for t in ts:
         t.join()
-    assert not trouble, trouble
+    assert trouble == [0] * 8
