@@ -256,9 +256,9 @@ static bool conv_params(const size_t* meta, size_t num_els, ConvParams& P, const
 // a multiple of `step`.  0: not even `step` planes fit `most` bytes.
 static uint32_t planes_per_block(uint64_t planes, uint64_t plane_bytes, uint64_t step, uint64_t most) {
     if (step * plane_bytes > most) return 0;
-    uint64_t n = 16 * 1024 / plane_bytes;
     const uint64_t spread = planes / (8 * (uint64_t)sm_count());
-    if (n > spread) n = spread;
+    uint64_t n = spread;
+    if (plane_bytes && n > 16 * 1024 / plane_bytes) n = 16 * 1024 / plane_bytes;  // an image of no pixels is all padding
     n = n / step * step;
     return (uint32_t)(n < step ? step : n);
 }

@@ -146,3 +146,16 @@ def test_threads_with_planes_of_different_sizes(cuda):
     for t in ts:
         t.join()
     assert trouble == [0] * 8
+
+
+@pytest.mark.parametrize("dt", D.FLOATS, ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [(3, 5, 0, 6, 1, 3, 1, 1), (2, 7, 6, 0, 3, 1, 1, 2), (1, 1, 0, 0, 2, 2, 1, 1), (40, 60, 0, 1, 1, 1, 1, 0)], ids=str)
+def test_images_of_no_pixels(cuda, dt, case):
+    """H or W of zero: padding alone gives output positions, and every column entry is a zero of it."""
+    B, C, Hh, W, kh, kw, ph, pw = case
+    oh, ow = Hh + 2 * ph - kh + 1, W + 2 * pw - kw + 1
+    meta = H.conv_metadata(B, C, Hh, W, kh, kw, oh, ow, ph, pw, 1, 1)
+    n = B * C * kh * kw * oh * ow
+    assert n > 0
+    got = H.run_im2col(cuda, dt, meta, n, H.random_store(np.random.default_rng(1), dt, 1, dist="normal"))
+    assert np.array_equal(D.decode(got, dt), np.zeros(n))
