@@ -4,8 +4,8 @@
 //   metadata = [B, C, H, W, kh, kw, out_h, out_w, pad_h, pad_w, stride_h, stride_w]
 //   col layout [B][C, kh, kw][out_h, out_w]
 //
-// im2col: a block takes a few neighbouring (b, c) image planes.  They are read once into shared memory
-// with coalesced loads; the kh*kw shifted copies of all of them are one contiguous run of the column buffer, written
+// im2col: a block takes one or a few neighbouring (b, c) image planes.  They are read once into shared memory
+// with coalesced loads; the kh*kw shifted copies of a plane (of all of them) are one contiguous run of the column buffer, written
 // with 16-byte stores.  DRAM traffic is the algorithmic
 // minimum (input once + col once) where the reference re-reads the input kh*kw times.
 //
@@ -28,8 +28,18 @@ namespace mx {
 struct ConvParams {
     uint32_t B, C, H, W, KH, KW, OH, OW, PH, PW, SH, SW;
     uint64_t num_els;
-    uint32_t planes, per_block;  // planes written, planes of one block (staged kernels)
-    FastDiv ow_div, w_div, ohw_div, hw_div, kk_div, kw_div, sh_div, sw_div;
+    FastDiv ow_div, w_div;
+};
+// the kernels whose blocks take several planes
+struct ConvPlanes : ConvParams {
+    uint32_t planes, per_block;  // planes written, planes of one block
+    FastDiv ohw_div, hw_div, kk_div, kw_div;
+    ConvPlanes(const ConvParams& p, uint64_t n, uint32_t pb) : ConvParams(p), planes((uint32_t)n), per_block(pb) {
+        ohw_div.init(OH * OW);
+        hw_div.init(H * W);
+        kk_div.init(KH * KW);
+        kw_div.init(KW);
+    }
 };
 
 constexpr int kConvThreads = 256;
@@ -51,7 +61,7 @@ __device__ __forceinline__ void stage_run(T* dst, const T* __restrict__ src, uin
 // busy and ragged ones (7 x 7) are written as vectors too.  Bound by HBM / L2 writes: [32, 128, 14, 14] f32, 3 x 3: 12 us, 23 with one
 // plane and one kernel offset at a time.
 template <class T, int VEC>
-__global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* __restrict__ x, T* __restrict__ col, ConvParams P) {
+__global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* __restrict__ x, T* __restrict__ col, ConvPlanes P) {
     extern __shared__ __align__(16) unsigned char conv_smem[];
     T* img = reinterpret_cast<T*>(conv_smem);
     const uint32_t bc0 = blockIdx.x * P.per_block, np = min(P.per_block, P.planes - bc0);
@@ -72,7 +82,7 @@ __global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* __
         for (int j = 0; j < VEC; j++) {
             const int hi = (int)(ho * P.SH + kh) - (int)P.PH, wi = (int)(wo * P.SW + kw) - (int)P.PW;
             r.v[j] = (uint32_t)hi < P.H && (uint32_t)wi < P.W && plane < np ? img[plane * HW + hi * P.W + wi] : zero;
-            if (VEC > 1 && ++wo == P.OW) {
+            if (++wo == P.OW) {
                 wo = 0;
                 if (++ho == P.OH) {
                     ho = 0;
@@ -96,12 +106,20 @@ __global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* __
     }
 }
 
-// Planes too large for shared memory: one block per plane, the input read in place.
-template <class T, int VEC>
+// One block per plane, one kernel offset at a time.  Large maps keep its threads busy with less arithmetic per element than the flat
+// index above takes (see planes_pay).  STAGED: the plane fits shared memory.
+template <class T, int VEC, bool STAGED>
 __global__ void __launch_bounds__(kConvThreads) im2col_kernel(const T* __restrict__ x, T* __restrict__ col, ConvParams P) {
+    extern __shared__ __align__(16) unsigned char conv_smem[];
+    T* plane = reinterpret_cast<T*>(conv_smem);
     const uint64_t bc = blockIdx.x;  // b * C + c
     const uint32_t HW = P.H * P.W, OHW = P.OH * P.OW, KK = P.KH * P.KW;
-    const T* img = x + bc * HW;
+    const T* src = x + bc * HW;
+    if constexpr (STAGED) {
+        for (uint32_t i = threadIdx.x; i < HW; i += kConvThreads) plane[i] = src[i];
+        __syncthreads();
+    }
+    const T* img = STAGED ? plane : src;
     const T zero = zero_of<T>();
     const uint64_t out_base = bc * KK * OHW;
     const uint32_t nvec = (OHW + VEC - 1) / VEC;
@@ -142,9 +160,10 @@ __device__ __forceinline__ T conv_add(T a, T b) {
 }
 
 // The same sums from shared memory: the KH * KW column planes of the block's image planes arrive in one contiguous run; a
-// column entry crosses from L2 once instead of once per term.  UNIT: strides of 1.  [32, 128, 14, 14] f32, 3 x 3: 15 us, 18 from L2.
-template <class T, bool UNIT>
-__global__ void __launch_bounds__(kConvThreads) col2im_planes_kernel(const T* __restrict__ col, T* __restrict__ out, ConvParams P) {
+// column entry crosses from L2 once instead of once per term.  Strides of 1: larger ones touch few entries more than once.
+// [32, 128, 14, 14] f32, 3 x 3: 14 us, 16 from L2.
+template <class T>
+__global__ void __launch_bounds__(kConvThreads) col2im_planes_kernel(const T* __restrict__ col, T* __restrict__ out, ConvPlanes P) {
     extern __shared__ __align__(16) unsigned char conv_smem[];
     T* cols = reinterpret_cast<T*>(conv_smem);
     const uint32_t bc0 = blockIdx.x * P.per_block, np = min(P.per_block, P.planes - bc0);
@@ -160,18 +179,16 @@ __global__ void __launch_bounds__(kConvThreads) col2im_planes_kernel(const T* __
         P.w_div.divmod(pix, h, w);
         const uint32_t hp = h + P.PH, wp = w + P.PW;
         // conv.rs:121-125
-        const uint32_t hs0 = hp >= P.KH - 1 ? hp - (P.KH - 1) : 0, ws0 = wp >= P.KW - 1 ? wp - (P.KW - 1) : 0;
-        const uint32_t hs = UNIT ? hs0 : P.sh_div.div(hs0 + P.SH - 1), ws = UNIT ? ws0 : P.sw_div.div(ws0 + P.SW - 1);
-        const uint32_t he = min((UNIT ? hp : P.sh_div.div(hp)) + 1, P.OH), we = min((UNIT ? wp : P.sw_div.div(wp)) + 1, P.OW);
-        const uint32_t SH = UNIT ? 1 : P.SH, SW = UNIT ? 1 : P.SW;
+        const uint32_t hs = hp >= P.KH - 1 ? hp - (P.KH - 1) : 0, ws = wp >= P.KW - 1 ? wp - (P.KW - 1) : 0;
+        const uint32_t he = min(hp + 1, P.OH), we = min(wp + 1, P.OW);
         const T* mine = cols + plane * KK * OHW;
         T sum = zero_of<T>();
         for (uint32_t ho = hs; ho < he; ho++) {
-            const uint32_t kh = hp - ho * SH;
+            const uint32_t kh = hp - ho;
             if (kh >= P.KH) continue;
             const T* row = mine + kh * P.KW * OHW + ho * P.OW;
             for (uint32_t wo = ws; wo < we; wo++) {
-                const uint32_t kw = wp - wo * SW;
+                const uint32_t kw = wp - wo;
                 if (kw < P.KW) sum = conv_add(sum, row[kw * OHW + wo]);
             }
         }
@@ -242,12 +259,6 @@ static bool conv_params(const size_t* meta, size_t num_els, ConvParams& P, const
     }
     P.ow_div.init(P.OW);
     P.w_div.init(P.W);
-    P.ohw_div.init(P.OH * P.OW);
-    P.hw_div.init(P.H * P.W);
-    P.kk_div.init(P.KH * P.KW);
-    P.kw_div.init(P.KW);
-    P.sh_div.init(P.SH);
-    P.sw_div.init(P.SW);
     return true;
 }
 
@@ -261,6 +272,16 @@ static uint32_t planes_per_block(uint64_t planes, uint64_t plane_bytes, uint64_t
     if (plane_bytes && n > 16 * 1024 / plane_bytes) n = 16 * 1024 / plane_bytes;  // an image of no pixels is all padding
     n = n / step * step;
     return (uint32_t)(n < step ? step : n);
+}
+
+// im2col: is the flat form faster than a block per plane and a kernel offset at a time?  It is where a plane's vectors are whole on
+// their own (step 1: [16, 64, 30, 30] f32 3 x 3 15.1 -> 11.9 us, [64, 64, 29, 29] bf16 7 x 7 stride 4 113 -> 16.6).  Where `step` planes
+// have to share a block to make whole vectors, enough blocks must be left ([4, 64, 27, 27] f32, 64 blocks: 6.3 -> 10.5 us; [16, 64, 21, 21],
+// 256: 11.8 -> 9.0), fewer for maps that do not even fill a block's threads ([2, 64, 7, 7], 32 blocks: 4.0 -> 2.5 us).  8-byte
+// types have two elements a vector, which large maps do not gain from ([32, 64, 35, 35] f64: 39.8 -> 43.4 us).
+static bool planes_pay(size_t es, uint64_t step, uint64_t blocks, uint64_t ohw) {
+    if (es == 8 && ohw > 1100) return false;
+    return step == 1 || blocks >= 192 || (ohw < kConvThreads && blocks >= 32);
 }
 
 template <class T>
@@ -311,22 +332,20 @@ void im2col_entry(size_t num_els, const size_t* meta, const T* x, T* col, const 
     // a block's columns start on a vector boundary when its planes' chunks add up to whole vectors
     uint64_t step = 1;
     while (step < VEC && (chunk * step) % VEC != 0) step *= 2;
-    const bool col_aligned = (uintptr_t)col % 16 == 0;
-    const uint32_t pb_vec = col_aligned ? planes_per_block(planes_touched, plane_bytes, step, step == 1 ? kConvSmemMost : 48 * 1024) : 0;
-    const uint32_t pb = pb_vec ? pb_vec : planes_per_block(planes_touched, plane_bytes, 1, kConvSmemMost);
-    if (pb && pb * chunk < 0x7FFFFFFFull) {
-        P.planes = (uint32_t)planes_touched;
-        P.per_block = pb;
-        const size_t smem = pb * plane_bytes;
+    const uint64_t ohw = (uint64_t)P.OH * P.OW;
+    const uint32_t pb = (uintptr_t)col % 16 == 0 ? planes_per_block(planes_touched, plane_bytes, step, step == 1 ? 48 * 1024 : 40 * 1024) : 0;
+    if (pb && pb * chunk < 0x7FFFFFFFull && planes_pay(sizeof(T), step, (planes_touched + pb - 1) / pb, ohw)) {
+        im2col_planes_kernel<T, VEC><<<(unsigned)((planes_touched + pb - 1) / pb), kConvThreads, pb * plane_bytes, s>>>(x, col, ConvPlanes(P, planes_touched, pb));
+    } else if (plane_bytes <= kConvSmemMost) {
         auto launch = [&](auto kernel) {
-            allow_shared_memory(kernel, smem);
-            kernel<<<(unsigned)((planes_touched + pb - 1) / pb), kConvThreads, smem, s>>>(x, col, P);
+            allow_shared_memory(kernel, plane_bytes);
+            kernel<<<grid, kConvThreads, plane_bytes, s>>>(x, col, P);
         };
-        if (pb_vec) launch(im2col_planes_kernel<T, VEC>);
-        else launch(im2col_planes_kernel<T, 1>);
+        if (vec) launch(im2col_kernel<T, VEC, true>);
+        else launch(im2col_kernel<T, 1, true>);
     } else {
-        if (vec) im2col_kernel<T, VEC><<<grid, kConvThreads, 0, s>>>(x, col, P);
-        else im2col_kernel<T, 1><<<grid, kConvThreads, 0, s>>>(x, col, P);
+        if (vec) im2col_kernel<T, VEC, false><<<grid, kConvThreads, 0, s>>>(x, col, P);
+        else im2col_kernel<T, 1, false><<<grid, kConvThreads, 0, s>>>(x, col, P);
     }
     check_launch(where);
 }
@@ -386,18 +405,14 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
             }
         }
     }
+    // Staged planes: strides of 1, column planes of at most 48 KB (four blocks on an SM, so that one loads while others sum: [16, 64, 50, 50]
+    // f32, 90 KB: 51 -> 65 us; bf16, 45 KB: 40 -> 38), pixels for half of a block's threads, and where a map has more pixels than a block
+    // threads, blocks enough for the whole chip ([32, 64, 35, 35] f32: 48 -> 41 us, [1, 64, 35, 35], 64 blocks: 4.2 -> 8.4), and for 8-byte types
+    // one term a pixel ([64, 64, 33, 33] f64: 1 x 1 29.1 -> 23.6 us; [16, 64, 21, 21] 3 x 3 10.2 -> 11.4).
     const uint64_t col_plane = (uint64_t)P.KH * P.KW * P.OH * P.OW;
-    const uint32_t pb = planes <= 0x7FFFFFFFull && col_plane && HW < 0x7FFFFFFFull ? planes_per_block(planes, col_plane * sizeof(T), 1, 100 * 1024) : 0;
-    if (pb && pb * HW < 0x7FFFFFFFull) {
-        P.planes = (uint32_t)planes;
-        P.per_block = pb;
-        const size_t smem = pb * col_plane * sizeof(T);
-        auto launch = [&](auto kernel) {
-            allow_shared_memory(kernel, smem);
-            kernel<<<(unsigned)((planes + pb - 1) / pb), kConvThreads, smem, s>>>(col, out, P);
-        };
-        if (P.SH == 1 && P.SW == 1) launch(col2im_planes_kernel<T, true>);
-        else launch(col2im_planes_kernel<T, false>);
+    const uint32_t pb = P.SH == 1 && P.SW == 1 && planes <= 0x7FFFFFFFull && col_plane && HW < 0x7FFFFFFFull ? planes_per_block(planes, col_plane * sizeof(T), 1, 48 * 1024) : 0;
+    if (pb && pb * HW < 0x7FFFFFFFull && pb * HW >= kConvThreads / 2 && (HW <= kConvThreads || ((planes + pb - 1) / pb >= 512 && (sizeof(T) < 8 || P.KH * P.KW == 1)))) {
+        col2im_planes_kernel<T><<<(unsigned)((planes + pb - 1) / pb), kConvThreads, pb * col_plane * sizeof(T), s>>>(col, out, ConvPlanes(P, planes, pb));
         check_launch(where);
         return;
     }

@@ -93,6 +93,9 @@ MANY_PLANES = [
     ("7x7-s2", 5, 211, 7, 7, 3, 3, 1, 1, 2, 2),
     ("9x11-5x5", 3, 300, 9, 11, 5, 5, 2, 2, 1, 1),
     ("1x1-odd", 4, 401, 5, 5, 1, 1, 0, 0, 1, 1),
+    ("17x19", 4, 200, 17, 19, 3, 3, 1, 1, 1, 1),      # more pixels than a block has threads, blocks enough
+    ("7x7", 12, 300, 7, 7, 3, 3, 1, 1, 1, 1),
+    ("15x15-few", 1, 9, 15, 15, 3, 3, 1, 1, 1, 1),    # too few planes to share blocks
     ("even-kernel", 3, 257, 6, 10, 2, 4, 1, 0, 1, 3),
     ("plane-beyond-shared-memory", 1, 2, 170, 331, 3, 3, 1, 1, 2, 2),
 ]
