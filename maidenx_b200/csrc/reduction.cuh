@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_block_kernel(const T*
     }
 }
 
-// G lanes of a warp per row (8 <= R <= 32 vectors), G the smallest of 4, 8, 16, 32 that gives every vector of the row a lane: a
+// G lanes of a warp per row (up to 32 vectors), G the smallest of 4, 8, 16, 32 that gives every vector of the row a lane: a
 // row of 56 bf16 is seven vectors, and a whole warp for it left 25 lanes idle.  Q rows per group with their loads in flight
 // together: with one row a block of 256 threads lived for a single load (sums over the last two dims of [64, 256, 56, 56] bf16:
 // 124 us with a warp per row, 55 with eight lanes and one row, 32 with eight lanes and four).
@@ -243,22 +243,34 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_short_kernel(const T*
         if (threadIdx.x % G == 0 && row0 + q * ROWS < rows) out[row0 + q * ROWS] = TR::finalize(acc[q], factor);
 }
 
-// One warp per longer row (R < ~2048), four loads per lane in flight.
+// One warp per longer row (R < ~2048): a lane's loads in flight together, four or, of types with 16 elements a vector (whose adds
+// bound it), two.  Trips that are whole for every lane, then one with a check per load: checks in every trip cost long rows
+// more than they gave (100000 rows of 1023 bf16: 59 us, 46 like this), lanes that leave at different trips the ragged ones.
 template <class T, int KIND, int VEC>
-__global__ void __launch_bounds__(kRedThreads) reduce_rows_warp_kernel(const T* in, T* out, u64 rows, u64 R, u64 factor) {
+__global__ void __launch_bounds__(kRedThreads) reduce_rows_warp_kernel(const T* in, T* out, u64 rows, u32 R, u64 factor) {
     typedef RedTraits<T, KIND> TR;
     const u64 row = (u64)blockIdx.x * (kRedThreads / 32) + threadIdx.x / 32;
     if (row >= rows) return;
-    constexpr int STEP = 32 * VEC;
+    constexpr u32 STEP = 32 * VEC, Q = VEC >= 16 ? 2 : 4;
     const T* p = in + row * R;
     typename TR::Acc acc = TR::init();
-    for (u64 i = (threadIdx.x % 32) * VEC; i < R; i += 4 * STEP) {
-        Vec<T, VEC> v[4];
+    u32 i = (threadIdx.x % 32) * VEC;
+    for (u32 whole = R / (Q * STEP); whole > 0; whole--, i += Q * STEP) {  // the same trips for every lane
+        Vec<T, VEC> v[Q];
 #pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int q = 0; q < Q; q++) v[q] = *reinterpret_cast<const Vec<T, VEC>*>(p + i + q * STEP);
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+#pragma unroll
+            for (int j = 0; j < VEC; j++) acc = TR::combine(acc, TR::load(v[q].v[j]));
+    }
+    if (R % (Q * STEP)) {
+        Vec<T, VEC> v[Q];
+#pragma unroll
+        for (int q = 0; q < Q; q++)
             if (i + q * STEP < R) v[q] = *reinterpret_cast<const Vec<T, VEC>*>(p + i + q * STEP);
 #pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int q = 0; q < Q; q++)
             if (i + q * STEP < R)
 #pragma unroll
                 for (int j = 0; j < VEC; j++) acc = TR::combine(acc, TR::load(v[q].v[j]));
@@ -267,7 +279,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_warp_kernel(const T* 
     if (threadIdx.x % 32 == 0) out[row] = TR::finalize(acc, factor);
 }
 
-// One thread per row (R < 8).
+// One thread per row (R < 32, see red_launch).
 template <class T, int KIND>
 __global__ void __launch_bounds__(kRedThreads) reduce_rows_thread_kernel(const T* in, T* out, u64 rows, u64 R, u64 factor) {
     typedef RedTraits<T, KIND> TR;
@@ -557,7 +569,7 @@ void red_rows_group_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaSt
     else if (lanes <= 8) red_rows_short_launch<T, KIND, VEC, 8>(in, out, O, R, factor, s);
     else if (lanes <= 16) red_rows_short_launch<T, KIND, VEC, 16>(in, out, O, R, factor, s);
     else if (lanes <= 32) red_rows_short_launch<T, KIND, VEC, 32>(in, out, O, R, factor, s);
-    else reduce_rows_warp_kernel<T, KIND, VEC><<<(u32)((O + kRedThreads / 32 - 1) / (kRedThreads / 32)), kRedThreads, 0, s>>>(in, out, O, R, factor);
+    else reduce_rows_warp_kernel<T, KIND, VEC><<<(u32)((O + kRedThreads / 32 - 1) / (kRedThreads / 32)), kRedThreads, 0, s>>>(in, out, O, (u32)R, factor);
 }
 
 template <class T, int KIND>
@@ -576,15 +588,20 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
     const bool base_aligned = ((uintptr_t)in) % 16 == 0;
     if (pl.kind == RP_ROWS) {
         const u64 O = pl.O, R = pl.R;
-        if (R < 8) {
+        // Rows below 32 elements: lane groups where a row is two or more aligned vectors (of 8-byte types, whole 64-byte pieces), a thread
+        // per row otherwise - its loads of neighbouring rows meet in L1, and a row element by element leaves a group little to do (2000000 rows
+        // of 9: f32 10.7 / 43 us in groups, bf16 9.8 / 42; of 16: f32 59 / 22, bf16 31 / 20, u8, one vector, 16.5 / 33; f64 of 12: 35 / 37, of 24: 120 / 75).
+        // Few rows are the latency of one thread's chain, which a group shortens (2000 rows of 31: f32 2.7 / 1.6, f64 3.3 / 1.8; 10000 of 20: bf16 1.9 / 2.1, f64 3.0 / 1.9).
+        const bool vec_rows = base_aligned && R % VEC == 0;
+        if (R < 8 || (R < 32 && O > (sizeof(T) == 8 ? 16384 : 4096) && !(vec_rows && R >= 2 * VEC && (sizeof(T) < 8 || R % 8 == 0)))) {
             u64 blocks = (O + kRedThreads - 1) / kRedThreads;
             reduce_rows_thread_kernel<T, KIND><<<(u32)blocks, kRedThreads, 0, s>>>(in, out, O, R, pl.factor);
         } else if (R < 32 || (R < 2048 && O >= (u64)sms * 4)) {
-            if (base_aligned && R % VEC == 0) red_rows_group_launch<T, KIND, VEC>(in, out, O, R, pl.factor, s);
+            if (vec_rows) red_rows_group_launch<T, KIND, VEC>(in, out, O, R, pl.factor, s);
             else red_rows_group_launch<T, KIND, 1>(in, out, O, R, pl.factor, s);
         } else {
             // block per (row, split); split long rows when there are too few rows to fill the GPU
-            const bool vec = base_aligned && R % VEC == 0;
+            const bool vec = vec_rows;
             const u64 unit = (u64)kRedThreads * VEC * 4;  // one full unrolled trip of a block
             static int occ = 0;  // resident blocks per SM of this instantiation
             if (!occ) occ = resident_blocks((const void*)reduce_rows_block_kernel<T, KIND, VEC>, kRedThreads);

@@ -157,10 +157,11 @@ def test_outer_and_inner_dims_folded_around_a_kept_one(oracle, cuda, shape):
             H.assert_same("sum_to_shape", dt, got, ref, float_rel=SUM_TOL.get(dt.name, 0.0), what=str((shape, off)), scale=np.sqrt(q * i))
 
 
-@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.I32], ids=lambda d: d.name)
-@pytest.mark.parametrize("shape", [(303200, 8), (151600, 56), (76000, 13), (38000, 100), (37900, 30), (700, 31), (700, 33), (700, 1023), (700, 1032)], ids=str)
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.I32, D.U8, D.F64], ids=lambda d: d.name)
+@pytest.mark.parametrize("shape", [(303200, 8), (151600, 56), (76000, 13), (38000, 100), (37900, 30), (700, 31), (700, 33), (700, 1023), (700, 1032), (151700, 16), (9000, 24),
+                                   (700, 128), (700, 129), (700, 255), (700, 2047)], ids=str)
 def test_rows_shared_by_part_of_a_warp(oracle, cuda, shape, dt):
-    """Row lengths around the lanes a row gets (4 to 32, then a warp that walks the row), and row counts on both sides of the
+    """Row lengths around the lanes a row gets (one thread, 4 to 32 lanes, then a warp that walks the row in trips of four or two loads), and row counts on both sides of the
     form with four rows per group; the sum within this file's tolerance, the maximum exact."""
     from oracle import binding
     rows, r = shape
