@@ -1,9 +1,9 @@
 // General batched matmul on the CUDA cores: every dtype, every stride pattern, and the
 // index quirks of the reference (the parity target is crates/maidenx_cpu/src/ops/matmul.rs).
-// The tensor-core path (matmul_tc.cu) takes over for bf16 / f16 shapes it supports; this
-// kernel is the fallback and the only path for f32 / f64 / integers.
+// The tensor-core paths (matmul_tc.cu, matmul_tc_f32.cu) take the larger products of dense bf16 / f16 /
+// f32 operands; these kernels are the rest of those and the only path for f64 and integers.
 //
-// One kernel serves forward and both backward products.  It computes
+// The same index functions serve forward and both backward products.  The kernels compute
 //     out[row * N + col] = sum_{r < K} X[ix(row, r)] * Y[iy(row, r, col)]
 // with affine index functions, row = batch * M + mi:
 //     ix = batch * xs_b + mi * xs_m + r * xs_r        (term skipped when ix >= x_limit)
@@ -140,6 +140,133 @@ __global__ void __launch_bounds__(kMmThreads) matmul_simt_kernel(const T* __rest
     }
 }
 
+// Many small batches: a tile is 64 output rows whatever batch they belong to.  Rows of the tile's first batch multiply from shared
+// memory, the others read their Y element by element, which short reductions of a few rows a batch cost less than a block a
+// batch does ([16000] x 1 x 1 x 16 f32: 16 us, 144 with a block each).  Which one: simt_rows_pay.  The order of additions is the same.
+template <class T>
+__global__ void __launch_bounds__(kMmThreads) matmul_simt_rows_kernel(const T* __restrict__ X, const T* __restrict__ Y, T* __restrict__ out, MmParams P) {
+    typedef typename MmAcc<T>::type Acc;
+    constexpr int TILE = 64, STEP = 16;
+    __shared__ Acc xs[STEP][TILE + 1];  // [r][row]
+    __shared__ Acc ys[STEP][TILE + 1];  // [r][col]
+    const uint64_t row0 = (uint64_t)blockIdx.x * TILE, col0 = (uint64_t)blockIdx.y * TILE;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
+    Acc acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = (Acc)0;
+
+    // loader mapping: pick the fast index along the operand's smaller stride
+    const bool x_r_fast = (P.xs_r <= P.xs_m) || P.xs_m == 0;
+    const bool y_c_fast = (P.ys_c <= P.ys_r) || P.ys_r == 0;
+
+    for (uint64_t k0 = 0; k0 < P.K; k0 += STEP) {
+#pragma unroll
+        for (int it = 0; it < (TILE * STEP) / kMmThreads; it++) {
+            int e = threadIdx.x + it * kMmThreads;
+            int lr, lrow;
+            if (x_r_fast) {
+                lr = e % STEP;
+                lrow = e / STEP;
+            } else {
+                lrow = e % TILE;
+                lr = e / TILE;
+            }
+            uint64_t row = row0 + lrow, r = k0 + lr;
+            Acc v = (Acc)0;
+            if (row < P.rows && r < P.K) {
+                uint64_t batch = row / P.M, mi = row % P.M;
+                uint64_t ix = (uint64_t)((int64_t)batch * P.xs_b + (int64_t)mi * P.xs_m + (int64_t)r * P.xs_r);
+                if (ix < P.x_limit) v = mm_load<T>(X[ix]);
+            }
+            xs[lr][lrow] = v;
+        }
+#pragma unroll
+        for (int it = 0; it < (TILE * STEP) / kMmThreads; it++) {
+            int e = threadIdx.x + it * kMmThreads;
+            int lr, lcol;
+            if (y_c_fast) {
+                lcol = e % TILE;
+                lr = e / TILE;
+            } else {
+                lr = e % STEP;
+                lcol = e / STEP;
+            }
+            // Y is staged for the batch of the tile's first row; rows of other batches read theirs from memory
+            uint64_t col = col0 + lcol, r = k0 + lr;
+            Acc v = (Acc)0;
+            if (col < P.N && r < P.K) {
+                uint64_t batch = row0 / P.M;
+                uint64_t iy = (uint64_t)((int64_t)batch * P.ys_b + (int64_t)r * P.ys_r + (int64_t)col * P.ys_c);
+                if (iy < P.y_limit) v = mm_load<T>(Y[iy]);
+            }
+            ys[lr][lcol] = v;
+        }
+        __syncthreads();
+        const uint64_t batch0 = row0 / P.M;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            uint64_t row = row0 + ty * 4 + i;
+            if (row >= P.rows) continue;
+            uint64_t batch = row / P.M;
+            if (batch == batch0) {
+#pragma unroll
+                for (int kk = 0; kk < STEP; kk++) {
+                    Acc xv = xs[kk][ty * 4 + i];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        if constexpr (is_half_v<T>) acc[i][j] = fmaf(xv, ys[kk][tx * 4 + j], acc[i][j]);  // product exact in f32
+                        else acc[i][j] = acc[i][j] + xv * ys[kk][tx * 4 + j];
+                    }
+                }
+            } else {
+                // this row belongs to a later batch than the staged Y tile: read Y directly
+                for (int kk = 0; kk < STEP; kk++) {
+                    uint64_t r = k0 + kk;
+                    if (r >= P.K) break;
+                    Acc xv = xs[kk][ty * 4 + i];
+                    for (int j = 0; j < 4; j++) {
+                        uint64_t col = col0 + tx * 4 + j;
+                        Acc yv = (Acc)0;
+                        if (col < P.N) {
+                            uint64_t iy = (uint64_t)((int64_t)batch * P.ys_b + (int64_t)r * P.ys_r + (int64_t)col * P.ys_c);
+                            if (iy < P.y_limit) yv = mm_load<T>(Y[iy]);
+                        }
+                        if constexpr (is_half_v<T>) acc[i][j] = fmaf(xv, yv, acc[i][j]);
+                        else acc[i][j] = acc[i][j] + xv * yv;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        uint64_t row = row0 + ty * 4 + i;
+        if (row >= P.rows) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            uint64_t col = col0 + tx * 4 + j;
+            uint64_t o = row * P.N + col;
+            if (col < P.N && o < P.out_elems) out[o] = mm_store<T>(acc[i][j]);
+        }
+    }
+}
+
+// The two kernels' times from their parts, measured over 300 to 100000 batches, M 1 to 33, N 1 to 128 and K 8 to 300: a block of
+// matmul_simt_kernel takes 2.7 ns of the chip and 6.2 more a k-step; 64 shared rows 8 ns and, for every term, 1.6 and 0.5 for each of a
+// thread's four columns and 0.04 for further ones, and their chain of loads cannot be shorter than 2 us and 0.7 to 1.5 us a term.  Of 401
+// products (f32, f64, i32, bf16) two take the slower kernel by more than a tenth, [4000] x 4 x 20 x 200 f64 440 / 519 us.
+inline bool simt_rows_pay(uint64_t rows, uint64_t M, uint64_t N, uint64_t K) {
+    if (rows <= M || M >= 64) return false;
+    const double own = N < 4 ? (double)N : 4.0, more = N < 64 ? (double)N - own : 60.0, tiles_n = (double)((N + 63) / 64), steps = (double)((K + 15) / 16);
+    const double block = (double)((rows + M - 1) / M) * tiles_n * (2.7 + 6.2 * steps);
+    const double shared = (double)((rows + 63) / 64) * tiles_n * (8.0 + (double)K * (1.6 + 0.5 * own + 0.04 * more));
+    const double chain = 2000.0 + (double)K * (400.0 + 275.0 * own);
+    return (shared > chain ? shared : chain) < 0.9 * block;
+}
+
 // Few outputs, long reduction (the weight gradient of a narrow Linear layer: [1, batch] . [batch, in] in the reference's
 // README example): the tiled kernel would run the whole reduction in one or two blocks.  Here one block owns one output
 // element, its threads take k = t, t + 256, ... (each in ascending order) and the partial sums are folded by a fixed
@@ -197,6 +324,14 @@ void mm_launch(const MmParams& P, const T* X, const T* Y, T* out, const char* wh
         matmul_longk_kernel<T><<<(unsigned)P.out_elems, kMmThreads, 0, ctx().stream>>>(X, Y, out, P);
         check_launch(where);
         return;
+    }
+    if (P.M && simt_rows_pay(P.rows, P.M, P.N, P.K)) {
+        const uint64_t gx = (P.rows + 63) / 64, gy = (P.N + 63) / 64;
+        if (gy <= 65535 && gx <= 0x7FFFFFFFull) {
+            matmul_simt_rows_kernel<T><<<dim3((unsigned)gx, (unsigned)gy), kMmThreads, 0, ctx().stream>>>(X, Y, out, P);
+            check_launch(where);
+            return;
+        }
     }
     const uint64_t batches = (P.rows + P.M - 1) / P.M;
     auto go = [&](auto kernel, uint64_t tile) {

@@ -579,3 +579,29 @@ def test_long_sums_of_one_sign_in_16_bit_products(cuda, dt, case):
     err = lambda x: np.linalg.norm(x - ref) / np.linalg.norm(ref)  # noqa: E731
     assert err(got) <= 1.001 * err(once), (err(got), err(once))
     assert abs(((got - once) / ref).mean()) < (64 if dt.name == "f16" else 256) * 2.0 ** -23 + 4 * err(once) / np.sqrt(ref.size)
+
+
+@pytest.mark.parametrize("dt", [D.F32, D.F64, D.BF16, D.I32, D.U8], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [(4001, 1, 1, 16), (4001, 1, 17, 5), (9000, 3, 2, 7), (5000, 5, 3, 33), (3000, 2, 65, 4), (2500, 7, 9, 1), (700, 1, 1, 3), (64, 63, 3, 1)], ids=lambda c: "x".join(map(str, c)))
+def test_many_small_batches(oracle, cuda, dt, case):
+    """Tiles of 64 rows that span batches (few rows a batch, short reductions) and blocks of one batch each: both add in the
+    element-type loop's order, so f32, f64 and integers are bit-exact, and 16-bit types round one f32 sum."""
+    from oracle import binding
+    nb, m, n, k = case
+    rng = np.random.default_rng(nb + k)
+    cs = H.contiguous_strides
+    shapes = [nb, m, k], [nb, k, n], [nb, m, n]
+    a, b, g = (_inputs(rng, dt, H.numel(x)) for x in shapes)
+    binding.set_wide(dt.name == "bf16")
+    try:
+        for bst in (cs(shapes[1]), [0, n, 1]):        # every batch its own B, and one for all
+            meta = H.matmul_metadata(shapes[2], shapes[0], shapes[1], cs(shapes[0]), bst, 0, 0)
+            ref = H.run_matmul(oracle, dt, meta, nb * m * n, a, b)
+            H.assert_same("matmul", dt, H.run_matmul(cuda, dt, meta, nb * m * n, a, b), ref, what=str(bst))
+        meta = H.matmul_metadata(shapes[2], shapes[0], shapes[1], cs(shapes[0]), cs(shapes[1]), 0, 0)
+        ref = H.run_matmul_backward(oracle, dt, meta, nb * m * k, nb * k * n, g, a, b)
+        got = H.run_matmul_backward(cuda, dt, meta, nb * m * k, nb * k * n, g, a, b)
+    finally:
+        binding.set_wide(False)
+    for key in ref:
+        H.assert_same("matmul_backward", dt, got[key], ref[key], what=key)
