@@ -307,7 +307,13 @@ void ew_fill_tile_params(const EwPlan& pl, int tile, EwTileParams& P, uint32_t& 
 
 bool ew_fill_dense_params(const EwPlan& pl, size_t in_size, size_t out_size, const void* out, const void* a, const void* b, EwDenseParams& P) {
     const int vec = (int)(16 / in_size);
-    if (pl.n == 0 || pl.n > 0x7FFFFFFFull - vec || pl.nd < 1 || !aligned_to(out, 0, out_size, vec * out_size)) return false;
+    // A thread makes two vectors where the gather kernel makes an element, so the chip needs vectors enough: 2^15; where rows are shorter
+    // than a vector and its elements are walked one after the other 2^17, of 16 elements 2^18.  Gather / dense, rows of 75: 300000 elements f32 2.9 /
+    // 2.2 us, bf16 2.9 / 2.5, u8 2.9 / 3.3; 30000 f32 1.8 / 2.2; 700000 u8 4.6 / 3.2.  Rows of 3: bf16 300000 2.9 / 4.3, 1800000 7.9 / 4.5; u8 3000000 13.0 /
+    // 13.2 to 16.8 / 37.5 by layout, 30000000 103 / 79.
+    const bool short_rows = pl.nd > 0 && pl.dim[pl.nd - 1] < (uint32_t)vec;
+    if (pl.nd < 1 || pl.n / vec < (short_rows ? (vec >= 16 ? 1u << 18 : 1u << 17) : 1u << 15)) return false;
+    if (pl.n > 0x7FFFFFFFull - vec || !aligned_to(out, 0, out_size, vec * out_size)) return false;
     int64_t acc = 1, span[3] = {0, 0, 0};
     bool flat[3] = {true, true, true};
     for (int d = pl.nd - 1; d >= 0; d--) {

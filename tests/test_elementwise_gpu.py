@@ -453,10 +453,28 @@ def gathered_layouts():
     return out
 
 
+def large_gathered_layouts(vec):
+    """The same where there are vectors enough for the kernel that makes dense outputs vector by vector (2^15; of rows shorter
+    than one 2^17, or 2^18 of 16 elements), and a row fewer."""
+    cs = H.contiguous_strides
+    out = []
+    for q, vectors in ((75, 1 << 15), (vec + 1, 1 << 15), (3, 1 << (15 if vec <= 3 else 18 if vec >= 16 else 17))):
+        rows = -(-vectors * vec // q)
+        for r in (rows, rows - 1):
+            dims, n = [r, q], r * q
+            out.append((f"rows of {q} x {r}/rhs-row", dims, cs(dims), [0, 1], 0, 0, n, q))
+            out.append((f"rows of {q} x {r}/rhs-col-unaligned", dims, cs(dims), [1, 0], 1, 0, n + 1, r))
+    q = 7 if vec <= 4 else 21
+    d = [-(-(1 << 15) * vec // (5 * q)), 5, q]
+    out.append((f"permuted {d}", d, [q, d[0] * q, 1], cs(d), 0, 0, H.numel(d), H.numel(d)))
+    out.append((f"every second of {d}", [d[0] * 5, q], [2 * q, 2], cs([d[0] * 5, q]), 0, 0, 2 * H.numel(d), H.numel(d)))
+    return out
+
+
 @pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16, D.F64, D.I32, D.U8], ids=lambda d: d.name)
 def test_dense_outputs_with_gathered_operands(oracle, cuda, dt):
     rng = np.random.default_rng(zlib.crc32(b"gathered" + dt.name.encode()))
-    for name, dims, ls, rs, lo, ro, ll, rl in gathered_layouts():
+    for name, dims, ls, rs, lo, ro, ll, rl in gathered_layouts() + large_gathered_layouts(16 // dt.np_storage().itemsize):
         lhs, rhs = H.full_range_store(rng, dt, ll), H.full_range_store(rng, dt, rl)
         for op in ("add", "div", "lt"):  # packed, checked-quotient and one-byte-output forms
             ref = H.run_binary(oracle, op, dt, dims, ls, rs, lo, ro, lhs, rhs)
