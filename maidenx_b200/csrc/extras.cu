@@ -863,7 +863,8 @@ __global__ void __launch_bounds__(kExThreads) softmax_cols_kernel(const T* __res
 
 // Rows of any length and alignment: the same one-read form with single elements, lane t holding elements t, t + G, ... of
 // the row in registers.  f32 and f64 keep expf / exp and the quotient of the general kernel, whose rows these were;
-// 16-bit types, whose rounding step is 2^-9, take the hardware exp2 and one reciprocal.  Bound by HBM / L2 with a
+// 16-bit types, whose rounding step is 2^-9 or 2^-12, take the hardware exp2 and one reciprocal: one result in 10^4 is rounded the other
+// way, the error against 64 bits stays the same to six digits (f16 2.0124e-4, bf16 1.6048e-3 at [37824, 197]).  Bound by HBM / L2 with a
 // 64-byte (16-bit) or 128-byte request per warp and load: [192 x 197, 197] bf16 9.9 us, 109 in the general kernel.
 template <class T, int G, int K>
 __global__ void __launch_bounds__(kExThreads) softmax_rows_any_kernel(const T* __restrict__ in, T* __restrict__ out, u64 rows, u32 n) {
@@ -995,11 +996,14 @@ __global__ void __launch_bounds__(kExThreads) softmax_cols_reg_kernel(const T* _
         }
     }
 }
-// false: the columns do not fit (more than 64 32-bit values per thread)
+// false: the columns do not fit (more than 64 32-bit values per thread), or do so at the price of occupancy - all the values, or strips
+// narrower than 128 bytes - while the three-pass kernel has strips for the whole chip, whose later passes come from L2 ([1000, 513, 100]
+// f32 122 -> 161 us; [30, 513, 100], 94 strips, 12.4 -> 7.3).
 template <class T, int VEC, int LANES>
 bool softmax_cols_reg_launch(const T* in, T* out, u64 pre, u64 n, u64 post, cudaStream_t s) {
     constexpr int ROWS = kExThreads / LANES, KMAX = (sizeof(T) == 8 ? 32 : 64) / VEC;
     const u64 per = (n + ROWS - 1) / ROWS;
+    if ((LANES < 8 || per > KMAX / 2) && pre * post / (8 * VEC) > (LANES < 8 ? 2 : 4) * (u64)sm_count()) return false;
     const unsigned blocks = (unsigned)((pre * post / VEC + LANES - 1) / LANES);
     if (per <= KMAX / 4) softmax_cols_reg_kernel<T, VEC, LANES, KMAX / 4><<<blocks, kExThreads, 0, s>>>(in, out, pre, (u32)n, post);
     else if (per <= KMAX / 2) softmax_cols_reg_kernel<T, VEC, LANES, KMAX / 2><<<blocks, kExThreads, 0, s>>>(in, out, pre, (u32)n, post);
@@ -1017,7 +1021,7 @@ bool softmax_rows_any_launch(const T* in, T* out, u64 rows, u32 n, cudaStream_t 
     else if (per <= 8) softmax_rows_any_kernel<T, G, 8><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
     else if (per <= 16) softmax_rows_any_kernel<T, G, 16><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
     else if (per <= 32) softmax_rows_any_kernel<T, G, 32><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (sizeof(T) <= 4 && per <= 64) softmax_rows_any_kernel<T, G, sizeof(T) <= 4 ? 64 : 32><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
+    else if (is_half_v<T> && per <= 64) softmax_rows_any_kernel<T, G, is_half_v<T> ? 64 : 16><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
     else return false;
     return true;
 }
@@ -1081,10 +1085,16 @@ void softmax_entry(size_t num_els, size_t nd, size_t dim, const size_t* meta, co
                 return;
             }
         }
-        // rows that are not whole aligned vectors: a warp up to 1024 elements (32 per lane), a block beyond
-        if (P.post == 1 && P.pre < (1ull << 31) && P.n <= 64ull * kExThreads) {
-            const bool done = P.n <= 1024 ? softmax_rows_any_launch<T, 32>(src, out, P.pre, (u32)P.n, st)
-                                          : softmax_rows_any_launch<T, kExThreads>(src, out, P.pre, (u32)P.n, st);
+        // Rows that are not whole aligned vectors: a warp up to 1024 16-bit elements (32 per lane), a block beyond.  The wider types' exp and
+        // quotient are several times the instructions, so that a lane has less of a row to itself: a warp up to 256 elements, 512 where there are rows
+        // for many blocks ([1000, 1021] f32 8.0 us in the general kernel, 9.7 by a warp, 3.6 by a block; [20000, 257] 71, 13, 26), a block up to
+        // 4096, 8192 where few rows have an SM each, and the general kernel with its three passes from then on ([20000, 4097] f32 300 us,
+        // 632 in registers; [200, 8191] f64 23 and 14).
+        const u64 sms = (u64)sm_count();
+        const u64 warp_most = is_half_v<T> ? 1024 : P.pre >= 16 * sms ? 512 : 256, block_most = is_half_v<T> ? 64ull * kExThreads : P.pre <= 2 * sms ? 8192 : 4096;
+        if (P.post == 1 && P.pre < (1ull << 31) && P.n <= block_most) {
+            const bool done = P.n <= warp_most ? softmax_rows_any_launch<T, 32>(src, out, P.pre, (u32)P.n, st)
+                                               : softmax_rows_any_launch<T, kExThreads>(src, out, P.pre, (u32)P.n, st);
             if (done) {
                 check_launch(where);
                 return;
@@ -1092,9 +1102,9 @@ void softmax_entry(size_t num_els, size_t nd, size_t dim, const size_t* meta, co
         }
         if (P.post >= 16) {
             const bool wide = P.post % VEC == 0 && (reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
-            if (wide ? softmax_cols_reg_launch<T, VEC, 8>(src, out, P.pre, P.n, P.post, st) || softmax_cols_reg_launch<T, VEC, 4>(src, out, P.pre, P.n, P.post, st) ||
-                           softmax_cols_reg_launch<T, VEC, 2>(src, out, P.pre, P.n, P.post, st)
-                     : softmax_cols_reg_launch<T, 1, 32>(src, out, P.pre, P.n, P.post, st)) {
+            // single columns (rows that are no whole vectors) keep the three passes: [1000, 3, 100] bf16 6.7 us, 16.8 in registers
+            if (wide && (softmax_cols_reg_launch<T, VEC, 8>(src, out, P.pre, P.n, P.post, st) || softmax_cols_reg_launch<T, VEC, 4>(src, out, P.pre, P.n, P.post, st) ||
+                         softmax_cols_reg_launch<T, VEC, 2>(src, out, P.pre, P.n, P.post, st))) {
                 check_launch(where);
                 return;
             }

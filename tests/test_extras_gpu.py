@@ -297,12 +297,14 @@ def test_softmax_special_values(oracle, cuda):
 
 @pytest.mark.parametrize("dt", [D.F32, D.F64, D.BF16, D.F16], ids=lambda d: d.name)
 def test_softmax_of_ragged_rows_and_of_columns_in_registers(oracle, cuda, dt):
-    """Row lengths around the steps of the single-element row form (a warp up to 1024, a block up to its registers, the
-    general kernel beyond) and column lengths around those of the one-read column form, vector and scalar strips.  f32
+    """Row lengths around the steps of the single-element row form (a warp up to 256, 512 or 1024, a block up to 4096, 8192 or its
+    registers, the general kernel beyond) and column lengths around those of the one-read column form, vector strips and single columns.  f32
     and f64 keep the general kernel's functions: a few ulp of each quotient; 16-bit results carry one rounding."""
     rng = np.random.default_rng(31)
     tol = {"f32": 2e-6, "f64": 1e-14, "bf16": 2.0 ** -7, "f16": 2.0 ** -10}[dt.name]
-    cases = [([9, n], 1, off) for n, off in ((1, 0), (2, 1), (31, 0), (33, 0), (64, 1), (65, 0), (197, 0), (255, 1), (513, 0), (1023, 0), (1025, 0), (2049, 0), (4097, 1), (8193, 0), (16383, 0), (16391, 0))]
+    cases = [([r, n], 1, 0) for r, n in ((2500, 257), (2500, 511), (2500, 513), (300, 4095), (300, 4097), (9, 8191))]
+    cases += [([9, n], 1, off) for n, off in ((1, 0), (2, 1), (31, 0), (33, 0), (64, 1), (65, 0), (197, 0), (255, 1), (513, 0), (1023, 0), (1025, 0), (2049, 0), (4097, 1), (8193, 0), (16383, 0), (16391, 0))]
+    cases += [([80, n, 128], 1, 0) for n in (257, 300)]   # columns enough for the whole chip
     cases += [([2, n, post], 1, off) for n in (3, 8, 33, 65, 127, 257, 513, 1031) for post, off in ((16, 0), (40, 0), (37, 0), (40, 1))]
     oracle.b.set_wide(True)
     try:
