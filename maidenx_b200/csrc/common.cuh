@@ -125,11 +125,13 @@ void* scratch(size_t bytes);
 // Workspace of one call, in the order of the stream the calling thread launches on: allocated there, freed there when it
 // goes out of scope, so calls on different streams or threads never share it and a stream switch needs no wait.  take()
 // fails, with no error recorded, while that stream is being captured or when memory is short; the caller then takes the
-// route it has without a workspace.
+// route it has without a workspace.  `under_capture` (bounded sizes): a call also reserves that much of the thread's scratch block, and a
+// call under capture lends that, so that a graph does what the direct call before it did.
 struct StreamWorkspace {
     void* ptr = nullptr;
     cudaStream_t stream = 0;
-    bool take(size_t bytes);
+    bool borrowed = false;
+    bool take(size_t bytes, bool under_capture = false);
     StreamWorkspace() {}
     StreamWorkspace(const StreamWorkspace&) = delete;
     StreamWorkspace& operator=(const StreamWorkspace&) = delete;

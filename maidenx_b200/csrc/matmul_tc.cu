@@ -669,7 +669,7 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     }
     StreamWorkspace partial;
     const uint64_t n_pitch = (N + 3) / 4 * 4;
-    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float))) slices = 1;
+    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) slices = 1;
     if (slices > 1) {
         p.split_kb = (p.num_kb + slices - 1) / slices;
         p.num_kb = p.split_kb;

@@ -570,7 +570,7 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     }
     StreamWorkspace partial;
     const uint64_t n_pitch = (N + 3) / 4 * 4;
-    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float))) slices = 1;
+    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) slices = 1;
     if (slices > 1) {
         p.split_kb = (p.num_kb + slices - 1) / slices;
         p.num_kb = p.split_kb;

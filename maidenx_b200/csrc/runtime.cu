@@ -51,6 +51,7 @@ void forget_range_locked(const void* p, size_t bytes) {
 struct ScratchSlot {
     void* ptr = nullptr;
     size_t bytes = 0;
+    bool captured = false;  // a graph may hold the block's address
 };
 thread_local ScratchSlot t_scratch[64];
 thread_local std::vector<size_t> t_meta_copy;
@@ -148,29 +149,36 @@ uint32_t* arrival_counters(uint64_t count) {
     return t_counters[dev];
 }
 
+// At least `bytes` in the thread's block of the device; null and *error when memory is short.
+static void* scratch_block(int dev, size_t bytes, cudaError_t* error) {
+    ScratchSlot& s = t_scratch[dev];
+    if (s.bytes >= bytes && s.ptr) return s.ptr;
+    size_t want = bytes < (size_t)(8u << 20) ? (size_t)(8u << 20) : bytes + bytes / 4;
+    if (s.ptr) {
+        // cudaFree synchronises the device, so earlier kernels that used the old block are done.  One that a graph may write is never
+        // freed; blocks grow by a quarter and more, so that those left behind stay within a few times the last.
+        if (!s.captured) cudaFree(s.ptr);
+        s = ScratchSlot();
+    }
+    *error = cudaMalloc(&s.ptr, want);
+    if (*error != cudaSuccess) {
+        s.ptr = nullptr;
+        return nullptr;
+    }
+    s.bytes = want;
+    return s.ptr;
+}
+
 void* scratch(size_t bytes) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
         set_error(kErrNoDevice, 0, "scratch");
         return nullptr;
     }
-    ScratchSlot& s = t_scratch[dev];
-    if (s.bytes >= bytes && s.ptr) return s.ptr;
-    size_t want = bytes < (size_t)(8u << 20) ? (size_t)(8u << 20) : bytes + bytes / 4;
-    if (s.ptr) {
-        // cudaFree synchronises the device, so earlier kernels that used the old block are done.
-        cudaFree(s.ptr);
-        s.ptr = nullptr;
-        s.bytes = 0;
-    }
-    cudaError_t e = cudaMalloc(&s.ptr, want);
-    if (e != cudaSuccess) {
-        s.ptr = nullptr;
-        set_error(kErrCuda, (int)e, "scratch");
-        return nullptr;
-    }
-    s.bytes = want;
-    return s.ptr;
+    cudaError_t e = cudaSuccess;
+    void* p = scratch_block(dev, bytes, &e);
+    if (!p) set_error(kErrCuda, (int)e, "scratch");
+    return p;
 }
 
 // One pool per device.  Up to kWorkspaceKeep bytes that no call holds stay with the pool across synchronisations (a freed
@@ -207,13 +215,28 @@ static bool workspace_trim() {
     return g_workspace_pools[dev] && cudaDeviceSynchronize() == cudaSuccess && cudaMemPoolTrimTo(g_workspace_pools[dev], 0) == cudaSuccess;
 }
 
-bool StreamWorkspace::take(size_t bytes) {
+constexpr size_t kUnderCaptureMost = 64u << 20;  // a split product's partial results are at most a few tiles an SM: 40 MB
+
+bool StreamWorkspace::take(size_t bytes, bool under_capture) {
     stream = ctx().stream;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     int dev = 0;
-    cudaMemPool_t pool = nullptr;
-    if (ptr || cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone || cudaGetDevice(&dev) != cudaSuccess ||
-        dev < 0 || dev >= 64 || !(pool = workspace_pool(dev)) || cudaMallocFromPoolAsync(&ptr, bytes ? bytes : 1, pool, stream) != cudaSuccess) {
+    if (ptr || cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return false;
+    }
+    under_capture = under_capture && bytes <= kUnderCaptureMost;
+    if (capturing != cudaStreamCaptureStatusNone) {
+        ScratchSlot& s = t_scratch[dev];
+        if (!under_capture || s.bytes < bytes || capturing != cudaStreamCaptureStatusActive) return false;
+        s.captured = borrowed = true;
+        ptr = s.ptr;
+        return true;
+    }
+    cudaError_t e = cudaSuccess;
+    if (under_capture && !scratch_block(dev, bytes, &e)) cudaGetLastError();
+    cudaMemPool_t pool = workspace_pool(dev);
+    if (!pool || cudaMallocFromPoolAsync(&ptr, bytes ? bytes : 1, pool, stream) != cudaSuccess) {
         cudaGetLastError();
         ptr = nullptr;
         return false;
@@ -221,7 +244,7 @@ bool StreamWorkspace::take(size_t bytes) {
     return true;
 }
 StreamWorkspace::~StreamWorkspace() {
-    if (ptr && cudaFreeAsync(ptr, stream) != cudaSuccess) cudaGetLastError();
+    if (ptr && !borrowed && cudaFreeAsync(ptr, stream) != cudaSuccess) cudaGetLastError();
 }
 
 static void side_table_forget(const void* p, size_t bytes) {

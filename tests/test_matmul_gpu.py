@@ -605,3 +605,54 @@ def test_many_small_batches(oracle, cuda, dt, case):
         binding.set_wide(False)
     for key in ref:
         H.assert_same("matmul_backward", dt, got[key], ref[key], what=key)
+
+
+@pytest.mark.parametrize("dt", [D.BF16, D.F32], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [(256, 256, 8192), (128, 264, 1536)], ids=lambda c: "x".join(map(str, c)))
+def test_split_products_under_capture(cuda, dt, case):
+    """A product with few tiles is cut along K in a graph as it is in a direct call: the same bits, also after the thread's scratch block
+    has been replaced by a larger one."""
+    import ctypes
+
+    import torch
+
+    from maidenx_b200 import _lib
+
+    lib, m, n, k = _lib.load(), *case
+    tdt = {"bf16": torch.bfloat16, "f32": torch.float32}[dt.name]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a, b = torch.randn(m, k, device="cuda", generator=g).to(tdt), torch.randn(k, n, device="cuda", generator=g).to(tdt)
+    meta = np.asarray(H.matmul_metadata([m, n], [m, k], [k, n], [k, 1], [n, 1], 0, 0), dtype=np.uint64)
+    direct, replayed = torch.zeros(m, n, device="cuda", dtype=tdt), torch.zeros(m, n, device="cuda", dtype=tdt)
+    op = _lib.op("matmul", dt.name)
+    call = lambda out: op(ctypes.c_size_t(m * n), meta.ctypes.data, a.data_ptr(), b.data_ptr(), out.data_ptr())  # noqa: E731
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    lib.mx_set_stream(s.cuda_stream)
+    graph = torch.cuda.CUDAGraph()
+    try:
+        call(direct)
+        s.synchronize()
+        with torch.cuda.graph(graph, stream=s):
+            call(replayed)
+        for round_ in range(2):
+            replayed.zero_()
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert lib.mx_last_error() == 0
+            assert torch.equal(direct.view(torch.uint8), replayed.view(torch.uint8)), round_
+            # a fold with wide partial results of its own: the block grows
+            x = torch.ones(2, 9, 3000, 4, 700, device="cuda")
+            out = torch.zeros(9, 700, device="cuda")
+            fold = np.asarray([2, 9, 3000, 4, 700, 9 * 3000 * 4 * 700, 3000 * 4 * 700, 4 * 700, 700, 1, 1, 9, 1, 1, 700, 0], dtype=np.uint64)
+            _lib.op("sum_to_shape", "f32")(ctypes.c_size_t(x.numel()), ctypes.c_size_t(5), fold.ctypes.data, x.data_ptr(), out.data_ptr())
+            big = torch.ones(8, 400000, 16, device="cuda")
+            kept = torch.zeros(400000, device="cuda")
+            fold2 = np.asarray([8, 400000, 16, 6400000, 16, 1, 1, 400000, 1, 0], dtype=np.uint64)
+            _lib.op("sum_to_shape", "f32")(ctypes.c_size_t(big.numel()), ctypes.c_size_t(3), fold2.ctypes.data, big.data_ptr(), kept.data_ptr())
+            s.synchronize()
+            assert float(out[0, 0]) == 2 * 3000 * 4 and float(kept[7]) == 128.0
+    finally:
+        lib.mx_set_stream(None)
+        del graph
