@@ -121,6 +121,7 @@ const size_t* resolve_metadata(const size_t* meta, size_t count);
 // Scratch memory for multi-pass kernels: one growable buffer per host thread and device,
 // used in stream order on the thread's current stream.
 void* scratch(size_t bytes);
+constexpr size_t kScratchLeast = 8u << 20;  // the block's first size
 
 // Workspace of one call, in the order of the stream the calling thread launches on: allocated there, freed there when it
 // goes out of scope, so calls on different streams or threads never share it and a stream switch needs no wait.  take()

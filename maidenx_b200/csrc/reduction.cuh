@@ -693,6 +693,9 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
             check_launch(where);
             return;
         }
+        // Many outputs of few elements each: the scatter's atomics hardly meet, and the partial results would be as many bytes as the input
+        // ([2, 100000, 5] f32 17.8 us, 19.7 in two passes; f64 17.9 / 25.5, [2, 1000000, 25] 679 / 839, [2, 65536, 1024] 2281 / 2014; [3, 50000, 10] f32 24 / 15, f64 24 / 20).
+        const bool scatter = O >= 32768 && (R * I <= (sizeof(Acc) < 8 ? 10 : 12) || (sizeof(Acc) == 8 && R <= 2 && I < 512));
         const u64 cols = O * I;
         const bool vec = base_aligned && cols % VEC == 0;
         const int v = vec ? VEC : 1;
@@ -701,9 +704,16 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
         if (splits > max_splits) splits = max_splits;
         u64 seg = (R + splits - 1) / splits;
         splits = (R + seg - 1) / seg;
-        if (splits * I <= 0x7FFFFFFFull && gx <= 0x7FFFFFFFull && splits <= 65535) {
-            Acc* part = static_cast<Acc*>(scratch(sizeof(Acc) * splits * cols));
-            if (!part) return;
+        // The partial results grow with the input: what goes beyond the scratch block every thread has is memory of this call alone, and
+        // where that is not to be had the scatter serves.
+        StreamWorkspace wide;
+        Acc* part = nullptr;
+        if (!scatter && splits * I <= 0x7FFFFFFFull && gx <= 0x7FFFFFFFull && splits <= 65535) {
+            const size_t bytes = sizeof(Acc) * splits * cols;
+            if (bytes > kScratchLeast) part = wide.take(bytes) ? static_cast<Acc*>(wide.ptr) : nullptr;
+            else if (!(part = static_cast<Acc*>(scratch(bytes)))) return;
+        }
+        if (part) {
             dim3 grid((u32)gx, (u32)splits, 1);
             const u32 leave = splits < 2 ? 2 : (u32)splits;
             if (vec) reduce_cols_kernel<T, KIND, VEC><<<grid, kColLanes * kColRows, 0, s>>>(in, out, part, 1, R, cols, seg, leave, pl.factor, nullptr);

@@ -153,7 +153,7 @@ uint32_t* arrival_counters(uint64_t count) {
 static void* scratch_block(int dev, size_t bytes, cudaError_t* error) {
     ScratchSlot& s = t_scratch[dev];
     if (s.bytes >= bytes && s.ptr) return s.ptr;
-    size_t want = bytes < (size_t)(8u << 20) ? (size_t)(8u << 20) : bytes + bytes / 4;
+    size_t want = bytes < kScratchLeast ? kScratchLeast : bytes + bytes / 4;
     if (s.ptr) {
         // cudaFree synchronises the device, so earlier kernels that used the old block are done.  One that a graph may write is never
         // freed; blocks grow by a quarter and more, so that those left behind stay within a few times the last.

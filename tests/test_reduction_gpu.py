@@ -175,3 +175,20 @@ def test_rows_shared_by_part_of_a_warp(oracle, cuda, shape, dt):
             binding.set_wide(False)
         got = _run_dim(cuda, op, dt, [rows, r], None, [1], 0, x)
         H.assert_same(op, dt, got, ref, float_rel=SUM_TOL.get(dt.name, 0.0) if op == "sum" else 0.0, what=str((op, shape)), scale=np.sqrt(r))
+
+
+@pytest.mark.parametrize("shape", [(2, 40000, 5), (2, 40000, 7), (3, 33000, 4), (2, 40000, 60), (5, 700000, 2), (3, 30001, 200)], ids=str)
+def test_outer_folds_of_many_outputs(oracle, cuda, shape):
+    """Both sides of the line between the scatter and the two passes (many outputs of few elements), and partial results beyond the
+    thread's scratch block.  Integers exact; sums of ones of a range that every type holds, so floats are exact too."""
+    q, o, i = shape
+    rng = np.random.default_rng(q * 1000 + o)
+    for dt in (D.F32, D.BF16, D.F64, D.I64, D.U8):
+        n = q * o * i
+        x = D.encode(rng.integers(0, 2, n).astype(np.float32 if dt is not D.F64 else np.float64), dt) if dt.kind == "float" else rng.integers(0, 2, n).astype(dt.np_storage)
+        got = D.decode(H.run_sum_to_shape(cuda, dt, [q, o, i], H.contiguous_strides([q, o, i]), [1, o, 1], 0, x), dt)
+        want = np.asarray(D.decode(x, dt)).reshape(q, o, i).sum(axis=(0, 2), dtype=np.float64)
+        tol = 2.0 ** -8 if dt.name == "bf16" else 0.0          # one rounding of the sum; 256 and more have no exact bf16
+        if dt.name == "u8":
+            want %= 256
+        assert np.all(np.abs(np.asarray(got, dtype=np.float64) - want) <= tol * want), dt.name
