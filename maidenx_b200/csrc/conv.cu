@@ -274,6 +274,13 @@ static uint32_t planes_per_block(uint64_t planes, uint64_t plane_bytes, uint64_t
     return (uint32_t)(n < step ? step : n);
 }
 
+// Bytes of planes that a block of the flat im2col takes at most: large planes leave a block or two on an SM, which 16-bit types (half the vectors to make) and maps of
+// few outputs gain from all the same ([64, 3, 224, 224] 7 x 7 stride 2 bf16 230 -> 206 us, f32 248 -> 325; [32, 3, 224, 224] 16 x 16 stride 16 f32 98 -> 27).
+static uint64_t planes_most(size_t es, uint64_t step, uint64_t ohw) {
+    if (step > 1) return 40 * 1024;
+    return es == 2 || ohw < kConvThreads ? kConvSmemMost : 48 * 1024;
+}
+
 // im2col: is the flat form faster than a block per plane and a kernel offset at a time?  It is where a plane's vectors are whole on
 // their own (step 1: [16, 64, 30, 30] f32 3 x 3 15.1 -> 11.9 us, [64, 64, 29, 29] bf16 7 x 7 stride 4 113 -> 16.6).  Where `step` planes
 // have to share a block to make whole vectors, enough blocks must be left ([4, 64, 27, 27] f32, 64 blocks: 6.3 -> 10.5 us; [16, 64, 21, 21],
@@ -333,8 +340,9 @@ void im2col_entry(size_t num_els, const size_t* meta, const T* x, T* col, const 
     uint64_t step = 1;
     while (step < VEC && (chunk * step) % VEC != 0) step *= 2;
     const uint64_t ohw = (uint64_t)P.OH * P.OW;
-    const uint32_t pb = (uintptr_t)col % 16 == 0 ? planes_per_block(planes_touched, plane_bytes, step, step == 1 ? 48 * 1024 : 40 * 1024) : 0;
+    const uint32_t pb = (uintptr_t)col % 16 == 0 ? planes_per_block(planes_touched, plane_bytes, step, planes_most(sizeof(T), step, ohw)) : 0;
     if (pb && pb * chunk < 0x7FFFFFFFull && planes_pay(sizeof(T), step, (planes_touched + pb - 1) / pb, ohw)) {
+        allow_shared_memory(im2col_planes_kernel<T, VEC>, pb * plane_bytes);
         im2col_planes_kernel<T, VEC><<<(unsigned)((planes_touched + pb - 1) / pb), kConvThreads, pb * plane_bytes, s>>>(x, col, ConvPlanes(P, planes_touched, pb));
     } else if (plane_bytes <= kConvSmemMost) {
         auto launch = [&](auto kernel) {

@@ -96,6 +96,8 @@ MANY_PLANES = [
     ("17x19", 4, 200, 17, 19, 3, 3, 1, 1, 1, 1),      # more pixels than a block has threads, blocks enough
     ("7x7", 12, 300, 7, 7, 3, 3, 1, 1, 1, 1),
     ("15x15-few", 1, 9, 15, 15, 3, 3, 1, 1, 1, 1),    # too few planes to share blocks
+    ("large-planes-few-outputs", 2, 3, 150, 150, 15, 15, 0, 0, 15, 15),
+    ("large-planes", 1, 3, 160, 160, 3, 3, 1, 1, 2, 2),
     ("even-kernel", 3, 257, 6, 10, 2, 4, 1, 0, 1, 3),
     ("plane-beyond-shared-memory", 1, 2, 170, 331, 3, 3, 1, 1, 2, 2),
 ]
