@@ -1025,6 +1025,19 @@ def reference_arm(args):
     print(json.dumps(line))
 
 
+def compact_rows(groups):
+    """The sweeps as they go into the JSON line: [ms, fraction of the measured peak] per case (null where a row is not one kernel's).
+    The whole rows are some 27 KB, and a reader that keeps the last 30 KB of an output loses the head of such a line with the value
+    in it; --rows writes them to a file."""
+    out = {"columns": ["ms", "frac of the measured peak"]}
+    for name, rows in groups.items():
+        if isinstance(rows, list):
+            out[name] = {r["case"]: [r["ms"], r.get("frac", r.get("frac_of_bf16_peak"))] for r in rows}
+        else:
+            out[name] = rows
+    return out
+
+
 def summarize(rows, key="frac"):
     vals = [(r[key], r["case"]) for r in rows if key in r]
     if not vals:
@@ -1050,6 +1063,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--no-sweeps", action="store_true", help="skip the per-case tables (elementwise, reductions, conv, products, movement)")
+    ap.add_argument("--rows", default=None, metavar="PATH", help="also write the whole rows of the per-case tables to this file")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-cpu", action="store_true", help="skip every CPU-oracle timing")
     ap.add_argument("--no-verify", action="store_true", help="skip the output checks against the CPU oracle")
@@ -1200,7 +1214,7 @@ def main():
             gemm_row(torch, lib_mod, "matmul_bf16/16384x8192x8192/nt", "bf16", 16384, 8192, 8192, "k", "k", pk, it, False, "tc_gemm_kernel"),
             gemm_row(torch, lib_mod, "matmul_f16/16384x8192x8192/nt", "f16", 16384, 8192, 8192, "k", "k", pk, it, verify, "tc_gemm_kernel"),
             gemm_row(torch, lib_mod, "matmul_f32/16384x8192x8192/nt", "f32", 16384, 8192, 8192, "k", "k", pk, 3, verify, "tc_gemm_f32_kernel (split tf32)"),
-            gemm_row(torch, lib_mod, "matmul_f32/4096x4098x4096/nn", "f32", 4096, 4098, 4096, "k", "mn", pk, 3, verify, "matmul_simt_kernel (row pitch not a multiple of 16 bytes)"),
+            gemm_row(torch, lib_mod, "matmul_f32/4096x4098x4096/nn", "f32", 4096, 4098, 4096, "k", "mn", pk, 3, verify, "tc_gemm_f32_kernel (rows not a multiple of 16 bytes: copied operand, plain stores)"),
         ]
         sweeps_out["conv2d_layer"] = conv_rows(torch, lib_mod, peaks, 3, verify)
         sweeps_out["movement"] = movement_rows(torch, lib_mod, peaks, 10)
@@ -1240,7 +1254,9 @@ def main():
                            "l2": "per-step working set (weights 0.5 GB + activations 2 GB per GPU at N=1) far exceeds the 126 MB L2; sweep inputs are 0.5-2 GB",
                            "verified": verified if verify else "skipped (--no-verify)"},
                 "loss": loss, "clocks": clocks, "gpu_launches": (MLP_KERNELS_PER_STEP + (3 * MLP_LAYERS - MLP_LAYERS if exch else 0)) * args.steps,
-                "roofline": roofline, "e2e": e2e, "cpu_baseline": cpu, "sweeps": sweeps_out}
+                "roofline": roofline, "e2e": e2e, "cpu_baseline": cpu, "sweeps": compact_rows(sweeps_out)}
+        if args.rows:
+            Path(args.rows).write_text(json.dumps(sweeps_out) + "\n")
         print(json.dumps(line))
 
 
