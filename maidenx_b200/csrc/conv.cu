@@ -9,8 +9,8 @@
 // with 16-byte stores.  DRAM traffic is the algorithmic
 // minimum (input once + col once) where the reference re-reads the input kh*kw times.
 //
-// col2im: gather formulation, the column planes of a few image planes staged in shared memory and one thread per
-// output pixel summing the (at most kh*kw) col entries that map to it in the reference's (h_out, w_out) order and in the element type,
+// col2im: gather formulation, one thread per output pixel (strides of 1 and small planes: the column planes of a few
+// image planes staged in shared memory) summing the (at most kh*kw) col entries that map to it in the reference's (h_out, w_out) order and in the element type,
 // so the result is bit-identical to the CPU backend, deterministic, needs no atomics and
 // overwrites the output (the reference's CUDA kernel scatters with atomicAdd into a
 // pre-zeroed buffer).  `num_els` bounds the readable part of col: entries at or beyond it

@@ -4,14 +4,16 @@
 //
 // One persistent CTA per SM, 192 threads in three roles:
 //   warp 0      TMA producer: one lane issues cp.async.bulk.tensor loads of the A [128 x 64]
-//               and B [256 x 64] k-blocks into a 4-stage shared-memory ring (128-byte swizzle);
-//   warp 1      MMA issuer: one lane issues four tcgen05.mma (M128 N256 K16) per k-block into
-//               one of two 256-column TMEM accumulators, commits the stage back to the
-//               producer and, after the last k-block, the accumulator to the epilogue;
+//               and B [64 to 256 x 64] k-blocks into a shared-memory ring (128-byte swizzle) of four
+//               stages, up to eight of narrower tiles;
+//   warp 1      MMA issuer: one lane issues four tcgen05.mma (M128, N = the tile's columns, K16) per
+//               k-block into one of two 256-column TMEM accumulators, commits the stage back to the
+//               producer and, after the last k-block (or a run of them, see DRAIN), the accumulator
+//               to the epilogue;
 //   warps 2-5   epilogue: each warp owns the 32 TMEM lanes it may address (warp id mod 4),
 //               reads them 64 columns at a time, rounds to bf16 / f16, writes a swizzled
-//               4 KB staging tile and stores it with TMA while the next tile's MMAs run on
-//               the other accumulator.
+//               4 KB staging tile and stores it with TMA (rows that no tensor map can describe:
+//               itself) while the next tile's MMAs run on the other accumulator.
 // No cluster launch: every CTA issues its own (CTA-local) TMA loads; re-use comes from
 // L2 through the order in which output tiles are handed out (16 row-tiles per column sweep).
 //

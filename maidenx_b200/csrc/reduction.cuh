@@ -11,10 +11,11 @@
 //   cols    (I > 1) each thread owns a 16-byte strip of columns and walks down R; R is split
 //           over blockIdx.y so that a [8192,16384] -> [16384] fold still fills 148 SMs;
 // split reductions write per-block partials to scratch and a second launch folds them:
-// the classic two-pass grid reduce.  Every path is atomic-free, so results are
+// the classic two-pass grid reduce.  These paths are atomic-free, so their results are
 // deterministic, and the output is overwritten (no pre-zero contract).
 //   outer   (sum_to_shape of [Q, O, I] to [1, O, 1]: the gradient of a per-channel operand) one of the two above down to
-//           wide partials, [O, I] sums over Q or [Q, O] sums over I, and a second launch that folds those.
+//           wide partials, [O, I] sums over Q or [Q, O] sums over I, and a second launch that folds those; many outputs of
+//           few elements each, and partials that no memory is to be had for, take the scatter below.
 // Accumulation: bf16/f16 in f32 with one final rounding, f32 in f32, f64 in f64, integers
 // wrapping in 32/64 bits (truncation to the element width commutes with wrapping adds).
 // Anything else (several reduced dims, non-contiguous input, partial sum_to_shape
