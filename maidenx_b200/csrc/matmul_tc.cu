@@ -1163,15 +1163,16 @@ static bool aligned_batches(size_t es, const TcProduct& c) {
 // (strides ignored, crates/maidenx_cpu/src/ops/matmul.rs:196-261).
 // Few outputs and a long reduction: matmul_longk_kernel (a block per output) is done before 128-row tiles have been cut into runs, copied
 // and summed.  16-bit, longk / tensor cores, both operands K-major: 16 x 64 x 4100 7.9 / 12.1 us, x 8192 12.3 / 8.5; 32 x 32 x 2048 5.1 / 7.3; 1 x 64
-// x 16384 9.0 / 10.7, x 32768 16.1 / 12.2; an MN-major B costs longk a line per element: 16 x 64 x 4100 22.9 / 10.3, 1 x 256 x 8192 11.2 / 11.2, x
-// 16384 19.9 / 13.1.  f32 pays for its drains: 784 x 1 x 65536 70 / 140 us, 5 x 5 x 2^20 333 / 516; only where A lies MN-major does
+// x 16384 9.0 / 10.7, x 32768 16.1 / 12.2; an MN-major operand costs longk a line per element: 16 x 64 x 4100 22.9 / 10.3, 1 x 256 x 8192
+// 11.2 / 11.2, x 16384 19.9 / 13.1, 100 x 10 x 4100 (A and B) 20.6 / 13.2, and without copies 16 x 64 x 2048 12.5 / 6.9 already.  f32 pays for its drains: 784 x 1 x 65536 70 / 140 us, 5 x 5 x 2^20 333 / 516; only where A lies MN-major does
 // it gain (10 x 64 x 32768 103 / 30, 10 x 32 x 60000 120 / 86).
-static bool longk_better(size_t es, const TcProduct& c) {
+static bool longk_better(size_t es, const TcProduct& c, bool in_place) {
     const uint64_t outputs = c.batch * c.m * c.n;
     if (c.k < kLongKMinK || outputs > kLongKMaxOutputs) return false;
     if (es != 2) return !(c.a_mn && outputs >= 256);
     const bool b_across = c.b_mn && c.n >= 32;
-    return !(c.k >= 32768 || (outputs >= 512 && c.k >= (b_across ? 4096 : 8192)) || (b_across && outputs >= 64 && c.k >= 16384));
+    const uint64_t many = !b_across && !(c.a_mn && c.m >= 32) ? 8192 : in_place ? kLongKMinK : 4096;
+    return !(c.k >= 32768 || (outputs >= 512 && c.k >= many) || (b_across && outputs >= 64 && c.k >= 16384));
 }
 
 bool tc_classify(const MmDesc& d, int which, size_t es, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, const void* out,
@@ -1189,9 +1190,9 @@ bool tc_classify(const MmDesc& d, int which, size_t es, size_t num_els, size_t n
     if (aligned_batches(es, c) && eligible(es, c.m, c.n, c.k, c.batch, c.a_mn, c.b_mn, c.A, c.B, out, least)) {
         const bool plain_form = !c.ragged && c.batch * c.m * c.n * c.k >= kTcLeast;
         c.nearest = es == 2 && !plain_form;
-        return plain_form || !longk_better(es, c);
+        return plain_form || !longk_better(es, c, true);
     }
-    if (longk_better(es, c)) return false;
+    if (longk_better(es, c, false)) return false;
     // the copy reads whole operands: every batch must be there (a size-1 batch dim passes the contiguity test)
     if (which == 0 && c.batch > 1 && d.a_cont && d.b_cont && (d.a_elems != c.batch * c.m * c.k || d.b_elems != c.batch * c.k * c.n)) return false;
     return plan_ragged(es, c, out, least);

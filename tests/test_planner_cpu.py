@@ -169,6 +169,11 @@ def test_copies_stay_small_and_few_outputs_stay_with_their_kernel():
     assert mm_plan("bf16", [32, 32], [32, 4096], [4096, 32])[0] == 1
     assert mm_plan("bf16", [32, 32], [32, 4096], [4096, 32], bst=[1, 4096]) == 0
     assert mm_plan("bf16", [32, 32], [32, 8192], [8192, 32])[0] == 1
+    assert mm_plan("bf16", [16, 64], [16, 2048], [2048, 64])[0] == 1                         # no copies
+    assert mm_plan("bf16", [16, 63], [16, 2048], [2048, 63]) == 0
+    assert mm_plan("bf16", [100, 10], [100, 4096], [4096, 10], ast=[1, 100])[0] == 1
+    assert mm_plan("bf16", [100, 10], [100, 4095], [4095, 10], ast=[1, 100]) == 0
+    assert mm_plan("bf16", [100, 10], [100, 4096], [4096, 10]) == 0
     assert mm_plan("f16", [8, 8], [8, 16384], [16384, 8]) == 0
     assert mm_plan("f16", [8, 8], [8, 32768], [32768, 8])[0] == 1
     assert mm_plan("bf16", [32, 32], [32, 16384], [16384, 32])[0] == 1                       # 2^24 multiply-adds, plain form: as ever
