@@ -1164,12 +1164,13 @@ static bool aligned_batches(size_t es, const TcProduct& c) {
 // Few outputs and a long reduction: matmul_longk_kernel (a block per output) is done before 128-row tiles have been cut into runs, copied
 // and summed.  16-bit, longk / tensor cores, both operands K-major: 16 x 64 x 4100 7.9 / 12.1 us, x 8192 12.3 / 8.5; 32 x 32 x 2048 5.1 / 7.3; 1 x 64
 // x 16384 9.0 / 10.7, x 32768 16.1 / 12.2; an MN-major operand costs longk a line per element: 16 x 64 x 4100 22.9 / 10.3, 1 x 256 x 8192
-// 11.2 / 11.2, x 16384 19.9 / 13.1, 100 x 10 x 4100 (A and B) 20.6 / 13.2, and without copies 16 x 64 x 2048 12.5 / 6.9 already.  f32 pays for its drains: 784 x 1 x 65536 70 / 140 us, 5 x 5 x 2^20 333 / 516; only where A lies MN-major does
-// it gain (10 x 64 x 32768 103 / 30, 10 x 32 x 60000 120 / 86).
+// 11.2 / 11.2, x 16384 19.9 / 13.1, 100 x 10 x 4100 (A and B) 20.6 / 13.2, and without copies 16 x 64 x 2048 12.5 / 6.9 already.  f32 stays: its fixed
+// tree has an error of 5e-8 for values of one sign at any length, the drained tf32 sums 1.9e-7 (normal values 1.9e-7 at K = 20000 to 5.8e-7 at
+// 262144, 2.6e-7 to 3.5e-7), although 100 x 10 x 131072 takes 220 us and would take 84.
 static bool longk_better(size_t es, const TcProduct& c, bool in_place) {
     const uint64_t outputs = c.batch * c.m * c.n;
     if (c.k < kLongKMinK || outputs > kLongKMaxOutputs) return false;
-    if (es != 2) return !(c.a_mn && outputs >= 256);
+    if (es != 2) return true;
     const bool b_across = c.b_mn && c.n >= 32;
     const uint64_t many = !b_across && !(c.a_mn && c.m >= 32) ? 8192 : in_place ? kLongKMinK : 4096;
     return !(c.k >= 32768 || (outputs >= 512 && c.k >= many) || (b_across && outputs >= 64 && c.k >= 16384));

@@ -159,7 +159,7 @@ def test_copies_stay_small_and_few_outputs_stay_with_their_kernel():
     # a vector is K-major whatever its strides say: nothing is copied where a [K, 1] matrix would grow eightfold
     assert mm_plan("bf16", [1, 1], [1, 1 << 24], [1 << 24, 1]) == (1, 0, 0, 1, 1, 1 << 24, 4)
     assert mm_plan("bf16", [1, 4096], [1, 4096], [4096, 4096], ast=[1, 1]) == (1, 0, 1, 1, 4096, 4096, 0)
-    assert mm_plan("f32", [784, 1], [784, 65536], [65536, 1], ast=[1, 784]) == (1, 1, 0, 784, 1, 65536, 4)
+    assert mm_plan("f32", [2048, 1], [2048, 16384], [16384, 1], ast=[1, 2048]) == (1, 1, 0, 2048, 1, 16384, 4)
     # rows of two elements: four times their size, taken while that is little memory
     assert mm_plan("bf16", [2, 4096], [2, 1 << 20], [1 << 20, 4096], ast=[1, 2])[6] == 1
     assert mm_plan("bf16", [2, 4096], [2, 1 << 22], [1 << 22, 4096], ast=[1, 2]) == 0
@@ -178,7 +178,11 @@ def test_copies_stay_small_and_few_outputs_stay_with_their_kernel():
     assert mm_plan("f16", [8, 8], [8, 32768], [32768, 8])[0] == 1
     assert mm_plan("bf16", [32, 32], [32, 16384], [16384, 32])[0] == 1                       # 2^24 multiply-adds, plain form: as ever
     assert mm_plan("f32", [5, 5], [5, 1 << 20], [1 << 20, 5]) == 0
-    assert mm_plan("f32", [10, 100], [10, 60000], [60000, 100], ast=[1, 10])[0] == 1
+    # f32: a block per output is more exact than the drained sums of the forms that are new to the tensor cores
+    assert mm_plan("f32", [10, 100], [10, 60000], [60000, 100])[0] == 1
+    assert mm_plan("f32", [10, 100], [10, 60000], [60000, 100], ast=[1, 10]) == 0
+    assert mm_plan("f32", [20, 50], [20, 1 << 18], [1 << 18, 50]) == 0
+    assert mm_plan("f32", [784, 1], [784, 65536], [65536, 1], ast=[1, 784]) == 0
 
 
 def test_small_16_bit_products_with_long_reductions_take_the_tensor_core_kernel():
