@@ -150,7 +150,24 @@ __global__ void __launch_bounds__(kEwThreads) ew_flat_kernel(F f, const T* a, co
             st_vec<O, VEC>(out + i, apply_vec<F, T, O, NIN, VEC>(f, va[u], vb[u]));
         }
     } else {
-        for (uint64_t i = base + threadIdx.x; i < n; i += kEwThreads) {
+        // The last, incomplete block: vectors as well, all loads in flight together, and only what is left of a vector by elements.
+        // Element by element it walked up to 64 trips to memory one after the other, the length of the whole launch.
+        Vec<T, VEC> va[kEwUnroll], vb[kEwUnroll];
+#pragma unroll
+        for (int u = 0; u < kEwUnroll; u++) {
+            const uint64_t i = base + ((uint64_t)u * kEwThreads + threadIdx.x) * VEC;
+            if (i + VEC <= n) {
+                va[u] = sa ? ld_vec<T, VEC>(a + i) : splat<T, VEC>(a[0]);
+                if constexpr (NIN == 2) vb[u] = sb ? ld_vec<T, VEC>(b + i) : splat<T, VEC>(b[0]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kEwUnroll; u++) {
+            const uint64_t i = base + ((uint64_t)u * kEwThreads + threadIdx.x) * VEC;
+            if (i + VEC <= n) st_vec<O, VEC>(out + i, apply_vec<F, T, O, NIN, VEC>(f, va[u], vb[u]));
+        }
+        const uint64_t i = n - n % VEC + threadIdx.x;
+        if (i < n) {
             T x = a[sa ? i : 0];
             if constexpr (NIN == 2) out[i] = f(x, b[sb ? i : 0]);
             else out[i] = f(x);

@@ -368,6 +368,26 @@ def test_flat_operands_at_unaligned_offsets(oracle, cuda, dt):
     H.assert_same("add", dt, H.run_binary(cuda, *args), H.run_binary(oracle, *args), what="2-d + scalar")
 
 
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F64, D.U8, D.I32], ids=lambda d: d.name)
+def test_last_block_of_flat_operands(oracle, cuda, dt):
+    """The block that is not full works by vectors too: lengths around the vector, a block's 256 threads and its four vectors a thread."""
+    rng = np.random.default_rng(zlib.crc32(dt.name.encode()) + 1)
+    vec = 16 // dt.size
+    row, block = 256 * vec, 1024 * vec
+    for n in (1, vec - 1, vec, vec + 1, row - 1, row + 1, 3 * row + vec, block - vec, block - 1, block, block + 1, 2 * block + row + vec - 1, 3 * block - 1):
+        if n < 1:
+            continue
+        a, b = (H.random_store(rng, dt, n, lo=1, hi=50) if dt.kind != "float" else H.random_store(rng, dt, n, lo=0.5, hi=2.0) for _ in range(2))
+        for op in ("sub", "div", "ge"):
+            for rs in (1, 0):
+                args = (op, dt, [n], [1], [rs], 0, 0, a, b)
+                H.assert_same(op, dt, H.run_binary(cuda, *args), H.run_binary(oracle, *args), what=f"n={n} rhs stride {rs}")
+        args = ("add_inplace", dt, [n], [1], [1], 0, 0, a, b)
+        H.assert_same("add_inplace", dt, H.run_binary_inplace(cuda, *args), H.run_binary_inplace(oracle, *args), what=f"inplace n={n}")
+        got, ref = (H.run_unary(be, "add_scalar", dt, [n], [1], 0, a, scalar=3) for be in (cuda, oracle))
+        H.assert_same("add_scalar", dt, got, ref, what=f"n={n}")
+
+
 @pytest.mark.parametrize("dt", [D.BF16, D.F16, D.I16, D.U16], ids=lambda d: d.name)
 def test_two_byte_transposed_tiles(oracle, cuda, dt):
     """2-byte types with vector-aligned transposed operands run on the tensor-copy tile kernel (64 x 64 boxes, ldmatrix
