@@ -110,7 +110,7 @@ struct TcParams {
     int stages, stage_bytes;  // of the operand ring
     int split_kb;    // > 0: split-K; batch s of the launch reduces the k-blocks [s * split_kb, (s + 1) * split_kb) of one product
     // The output's rows are not 16-byte multiples (or its base is not aligned), which no tensor map can describe: the epilogue
-    // warps copy their staged rows to `d` themselves, in steps of 2 bytes (1) or, for even N, 4 bytes (2).  0: tensor stores.
+    // warps copy their staged rows to `d` themselves (store_rows).  0: tensor stores.
     int d_plain;
     void* d;
     int run_kb;      // DRAIN form: k-blocks summed in one accumulator before the epilogue adds them to its own f32 totals
@@ -159,6 +159,58 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi, int is_bf16) {
 // v rounded to the operand type and widened again
 __device__ __forceinline__ float round16(float v, int is_bf16) {
     return is_bf16 ? to_f32(from_f32<bf16>(v)) : to_f32(from_f32<f16>(v));
+}
+
+// The 16 bytes that start 16 - 2 * sh bytes into (lo, hi), sh = 0 .. 7.
+__device__ __forceinline__ uint4 vector_before(const uint4& lo, const uint4& hi, uint32_t sh) {
+    const uint32_t words = 4 - (sh + 1) / 2, bits = (sh & 1) * 16;
+    uint32_t w[9] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w, 0};
+#pragma unroll
+    for (int s = 4; s; s >>= 1)  // word-wise shift with compile-time indices
+#pragma unroll
+        for (int i = 0; i + s < 9; i++)
+            if (words & s) w[i] = w[i + s];
+    return make_uint4(__funnelshift_r(w[0], w[1], bits), __funnelshift_r(w[1], w[2], bits), __funnelshift_r(w[2], w[3], bits), __funnelshift_r(w[3], w[4], bits));
+}
+
+// Chunk `c` (64 columns) of a warp's 32 rows of a tile, written to an output whose rows start anywhere: `tile` is the first element of
+// row 0, `ld` the elements between rows, `cols` the tile's columns inside the matrix; `cur` is the staged chunk (XOR-swizzled rows of 128 bytes), `prev` the
+// chunk before.  A row that starts sh elements behind a 16-byte boundary is cut at the boundaries: its vector v holds the elements 8 v - sh and following, so that
+// every chunk completes exactly eight vectors a row, the first of them with the last sh elements of the chunk before.  Only the
+// up to seven elements before a tile's first boundary and after its last are written by themselves.  Stores of one element
+// each bound the tiles of short reductions.
+__device__ __forceinline__ void store_rows(uint16_t* tile, size_t ld, int rows, int cols, int c, const unsigned char* cur, const unsigned char* prev, int lane) {
+    if (c * 64 >= cols) return;
+    const int r_lane = lane >> 3, j = lane & 7;
+    const bool first = c == 0, last = c * 64 + 64 >= cols;
+    uint16_t* dst = tile + r_lane * ld;
+#pragma unroll 1
+    for (int r0 = 0; r0 < 32; r0 += 16) {
+        uint4 lo[4], hi[4];
+        // four rows a step, all loads before the first store: the compiler cannot tell the staging tile from the output
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = r0 + 4 * i + r_lane;
+            lo[i] = *reinterpret_cast<const uint4*>((j ? cur : prev) + r * 128 + ((((j - 1) & 7) ^ (r & 7)) << 4));
+            hi[i] = *reinterpret_cast<const uint4*>(cur + r * 128 + ((j ^ (r & 7)) << 4));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++, dst += 4 * ld) {
+            const int r = r0 + 4 * i + r_lane;
+            const int sh = (int)(reinterpret_cast<uintptr_t>(dst) >> 1) & 7, e0 = c * 64 + j * 8 - sh;
+            if (r < rows && e0 >= 0 && e0 + 8 <= cols) *reinterpret_cast<uint4*>(dst + e0) = vector_before(lo[i], hi[i], (uint32_t)sh);
+            auto single = [&](int e) {
+                const int x = e & 63;
+                dst[e] = *reinterpret_cast<const uint16_t*>((e >> 6 == c ? cur : prev) + r * 128 + (((x >> 3) ^ (r & 7)) << 4) + (x & 7) * 2);
+            };
+            const int head = sh ? 8 - sh : 0;
+            if (first && r < rows && j < head && j < cols) single(j);
+            if (last) {
+                const int e = max(head, ((cols + sh) & ~7) - sh) + j;
+                if (r < rows && e < cols) single(e);
+            }
+        }
+    }
 }
 
 // What the epilogue does is compiled in: each form keeps its registers and its code to itself, and the plain product's loop is
@@ -333,35 +385,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                     return;
                 }
-                uint16_t* dst = static_cast<uint16_t*>(p.d) + ((size_t)tb * p.M + tm * BM + quarter * 32) * p.N + col;
-                const int cols = min(64, p.N - col);
-                // Eight rows at a time, all loads before the first store: the compiler cannot tell the staging tile from `d`, and a
-                // load behind a store waits for it.
-                if (p.d_plain == 2) {
-                    for (int r0 = 0; r0 < 32; r0 += 8) {
-                        uint32_t v[8];
-#pragma unroll
-                        for (int r = 0; r < 8; r++) v[r] = *reinterpret_cast<const uint32_t*>(src + (r0 + r) * 128 + (((lane >> 2) ^ r) << 4) + (lane & 3) * 4);
-#pragma unroll
-                        for (int r = 0; r < 8; r++)
-                            if (r0 + r < rows_here && 2 * lane < cols) *reinterpret_cast<uint32_t*>(dst + (size_t)(r0 + r) * p.N + 2 * lane) = v[r];
-                    }
-                    return;
-                }
-                const int c0 = lane, c1 = lane + 32;
-                for (int r0 = 0; r0 < 32; r0 += 8) {
-                    uint16_t v0[8], v1[8];
-#pragma unroll
-                    for (int r = 0; r < 8; r++) {
-                        v0[r] = *reinterpret_cast<const uint16_t*>(src + (r0 + r) * 128 + (((c0 >> 3) ^ r) << 4) + (c0 & 7) * 2);
-                        v1[r] = *reinterpret_cast<const uint16_t*>(src + (r0 + r) * 128 + (((c1 >> 3) ^ r) << 4) + (c1 & 7) * 2);
-                    }
-#pragma unroll
-                    for (int r = 0; r < 8; r++) {
-                        if (r0 + r < rows_here && c0 < cols) dst[(size_t)(r0 + r) * p.N + c0] = v0[r];
-                        if (r0 + r < rows_here && c1 < cols) dst[(size_t)(r0 + r) * p.N + c1] = v1[r];
-                    }
-                }
+                store_rows(static_cast<uint16_t*>(p.d) + ((size_t)tb * p.M + tm * BM + quarter * 32) * p.N + tn * bn, (size_t)p.N, rows_here,
+                           min(bn, p.N - tn * bn), (col - tn * bn) / 64, src, stage_buf + buf * EPI_STAGE_BYTES, lane);
             };
             // One 64-column chunk: round, stage in shared memory (XOR-swizzled rows), hand to the copy engine.
             auto store_chunk = [&](int c, uint32_t (&v0)[32], uint32_t (&v1)[32]) {

@@ -402,6 +402,25 @@ def test_products_with_ragged_rows(oracle, cuda, dt, case):
     H.assert_same("matmul", dt, got, ref, float_rel=1e-5 if dt.name == "f32" else 1e-2, what=name, scale=np.sqrt(k))
 
 
+@pytest.mark.parametrize("off", [0, 1, 3, 4, 6, 7])
+@pytest.mark.parametrize("n", [1, 7, 9, 63, 65, 71, 127, 130, 191, 194, 257, 260, 391])
+def test_ragged_output_rows_are_written_whole_and_alone(cuda, n, off):
+    """16-bit output rows that start anywhere: cut at the 16-byte boundaries, across the 64-column chunks and the tiles' edges.  Whole
+    numbers, so that the result is exact; what lies before and behind the output stays as it was."""
+    from maidenx_b200 import device
+    m, k = 1100, 256
+    rng = np.random.default_rng(n * 8 + off)
+    a, b = rng.integers(-2, 3, (m, k)).astype(np.float32), rng.integers(-2, 3, (n, k)).astype(np.float32)
+    for dt in (D.BF16, D.F16):
+        fill = np.full(m * n + 16, 0x1234, dtype=np.uint16)
+        bufs = [device.CudaBuffer.from_host(x) for x in (D.encode(a.reshape(-1), dt), D.encode(b.reshape(-1), dt), fill)]
+        device.dispatch("matmul", dt.name, [2, 2, 2, m, n, m, k, k, n, k, 1, 1, k, 0, 0], m * n, "META", bufs[0].ptr, bufs[1].ptr, bufs[2].ptr + 2 * off)
+        got = bufs[2].to_host(np.uint16, m * n + 16)
+        want = fill.copy()
+        want[off:off + m * n] = D.encode((a @ b.T).reshape(-1), dt).view(np.uint16)
+        assert np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("dt", [D.BF16, D.F16, D.F32], ids=lambda d: d.name)
 @pytest.mark.parametrize("case", [("batched", [4], 152, 136, 216), ("batched-odd", [4], 151, 133, 219), ("rank-4", [2, 2], 152, 136, 216), ("odd", [], 301, 259, 227),
                                   ("broadcast-b", None, 150, 136, 216)], ids=lambda c: c[0])
