@@ -2,7 +2,7 @@
 // tensor memory (TMEM), operands staged in shared memory by TMA, epilogue read back with
 // tcgen05.ld, converted and written with TMA stores.
 //
-// One persistent CTA per SM, 192 threads in three roles:
+// One persistent CTA per SM, 320 threads in three roles:
 //   warp 0      TMA producer: one lane issues cp.async.bulk.tensor loads of the A [128 x 64]
 //               and B [64 to 256 x 64] k-blocks into a shared-memory ring (128-byte swizzle) of four
 //               stages, up to eight of narrower tiles;
@@ -10,10 +10,10 @@
 //               k-block into one of two 256-column TMEM accumulators, commits the stage back to the
 //               producer and, after the last k-block (or a run of them, see DRAIN), the accumulator
 //               to the epilogue;
-//   warps 2-5   epilogue: each warp owns the 32 TMEM lanes it may address (warp id mod 4),
-//               reads them 64 columns at a time, rounds to bf16 / f16, writes a swizzled
-//               4 KB staging tile and stores it with TMA (rows that no tensor map can describe:
-//               itself) while the next tile's MMAs run on the other accumulator.
+//   warps 2-9   epilogue: two warps own the 32 TMEM lanes that both may address (warp id mod 4),
+//               read them 64 columns at a time, each 32, round to bf16 / f16, write a swizzled
+//               4 KB staging tile and store it with TMA (rows that no tensor map can describe:
+//               themselves) while the next tile's MMAs run on the other accumulator.
 // No cluster launch: every CTA issues its own (CTA-local) TMA loads; re-use comes from
 // L2 through the order in which output tiles are handed out (16 row-tiles per column sweep).
 //
@@ -54,9 +54,9 @@ constexpr int STAGES = 4;                     // ring stages of full-width tiles
 constexpr int MAX_STAGES = 8;
 constexpr int A_STAGE_BYTES = BM * BK * 2;    // 16 KB
 constexpr int B_STAGE_BYTES = BN * BK * 2;    // 32 KB
-constexpr int EPI_WARPS = 4;
+constexpr int EPI_WARPS = 8;                  // two for each quarter of the accumulator's lanes
 constexpr int EPI_CHUNK_COLS = 64;            // columns per TMA store (128 bytes of 16-bit)
-constexpr int EPI_STAGE_BYTES = 32 * EPI_CHUNK_COLS * 2;  // 4 KB per warp per buffer
+constexpr int EPI_STAGE_BYTES = 32 * EPI_CHUNK_COLS * 2;  // 4 KB: 32 rows of a chunk; two such buffers per quarter
 constexpr int TC_THREADS = 32 * (2 + EPI_WARPS);
 constexpr int TMEM_COLS = 512;                // two 256-column f32 accumulators
 constexpr int GROUP_M = 16;                   // row-tiles per column sweep (L2 re-use)
@@ -65,7 +65,7 @@ struct SmemLayout {
     // offsets inside the dynamic shared memory block (base aligned to 1024 bytes)
     static constexpr int ring = 0;  // stage s: A block, then B block (bn rows of 128 bytes), s * stage_bytes further
     static constexpr int epi = ring + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES);
-    static constexpr int bars = epi + EPI_WARPS * 2 * EPI_STAGE_BYTES;
+    static constexpr int bars = epi + 4 * 2 * EPI_STAGE_BYTES;
     static constexpr int total = bars + 256;
 };
 constexpr int TC_SMEM_BYTES = SmemLayout::total + 1024;  // slack for the 1024-byte alignment
@@ -173,42 +173,39 @@ __device__ __forceinline__ uint4 vector_before(const uint4& lo, const uint4& hi,
     return make_uint4(__funnelshift_r(w[0], w[1], bits), __funnelshift_r(w[1], w[2], bits), __funnelshift_r(w[2], w[3], bits), __funnelshift_r(w[3], w[4], bits));
 }
 
-// Chunk `c` (64 columns) of a warp's 32 rows of a tile, written to an output whose rows start anywhere: `tile` is the first element of
+// Chunk `c` (64 columns) of 16 rows from r0 on of a quarter's 32 (those below `rows`), written to an output whose rows start anywhere: `tile` is the first element of
 // row 0, `ld` the elements between rows, `cols` the tile's columns inside the matrix; `cur` is the staged chunk (XOR-swizzled rows of 128 bytes), `prev` the
 // chunk before.  A row that starts sh elements behind a 16-byte boundary is cut at the boundaries: its vector v holds the elements 8 v - sh and following, so that
 // every chunk completes exactly eight vectors a row, the first of them with the last sh elements of the chunk before.  Only the
 // up to seven elements before a tile's first boundary and after its last are written by themselves.  Stores of one element
 // each bound the tiles of short reductions.
-__device__ __forceinline__ void store_rows(uint16_t* tile, size_t ld, int rows, int cols, int c, const unsigned char* cur, const unsigned char* prev, int lane) {
+__device__ __forceinline__ void store_rows(uint16_t* tile, size_t ld, int r0, int rows, int cols, int c, const unsigned char* cur, const unsigned char* prev, int lane) {
     if (c * 64 >= cols) return;
     const int r_lane = lane >> 3, j = lane & 7;
     const bool first = c == 0, last = c * 64 + 64 >= cols;
-    uint16_t* dst = tile + r_lane * ld;
-#pragma unroll 1
-    for (int r0 = 0; r0 < 32; r0 += 16) {
-        uint4 lo[4], hi[4];
-        // four rows a step, all loads before the first store: the compiler cannot tell the staging tile from the output
+    uint16_t* dst = tile + (r0 + r_lane) * ld;
+    uint4 lo[4], hi[4];
+    // all loads before the first store: the compiler cannot tell the staging tile from the output
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int r = r0 + 4 * i + r_lane;
-            lo[i] = *reinterpret_cast<const uint4*>((j ? cur : prev) + r * 128 + ((((j - 1) & 7) ^ (r & 7)) << 4));
-            hi[i] = *reinterpret_cast<const uint4*>(cur + r * 128 + ((j ^ (r & 7)) << 4));
-        }
+    for (int i = 0; i < 4; i++) {
+        const int r = r0 + 4 * i + r_lane;
+        lo[i] = *reinterpret_cast<const uint4*>((j ? cur : prev) + r * 128 + ((((j - 1) & 7) ^ (r & 7)) << 4));
+        hi[i] = *reinterpret_cast<const uint4*>(cur + r * 128 + ((j ^ (r & 7)) << 4));
+    }
 #pragma unroll
-        for (int i = 0; i < 4; i++, dst += 4 * ld) {
-            const int r = r0 + 4 * i + r_lane;
-            const int sh = (int)(reinterpret_cast<uintptr_t>(dst) >> 1) & 7, e0 = c * 64 + j * 8 - sh;
-            if (r < rows && e0 >= 0 && e0 + 8 <= cols) *reinterpret_cast<uint4*>(dst + e0) = vector_before(lo[i], hi[i], (uint32_t)sh);
-            auto single = [&](int e) {
-                const int x = e & 63;
-                dst[e] = *reinterpret_cast<const uint16_t*>((e >> 6 == c ? cur : prev) + r * 128 + (((x >> 3) ^ (r & 7)) << 4) + (x & 7) * 2);
-            };
-            const int head = sh ? 8 - sh : 0;
-            if (first && r < rows && j < head && j < cols) single(j);
-            if (last) {
-                const int e = max(head, ((cols + sh) & ~7) - sh) + j;
-                if (r < rows && e < cols) single(e);
-            }
+    for (int i = 0; i < 4; i++, dst += 4 * ld) {
+        const int r = r0 + 4 * i + r_lane;
+        const int sh = (int)(reinterpret_cast<uintptr_t>(dst) >> 1) & 7, e0 = c * 64 + j * 8 - sh;
+        if (r < rows && e0 >= 0 && e0 + 8 <= cols) *reinterpret_cast<uint4*>(dst + e0) = vector_before(lo[i], hi[i], (uint32_t)sh);
+        auto single = [&](int e) {
+            const int x = e & 63;
+            dst[e] = *reinterpret_cast<const uint16_t*>((e >> 6 == c ? cur : prev) + r * 128 + (((x >> 3) ^ (r & 7)) << 4) + (x & 7) * 2);
+        };
+        const int head = sh ? 8 - sh : 0;
+        if (first && r < rows && j < head && j < cols) single(j);
+        if (last) {
+            const int e = max(head, ((cols + sh) & ~7) - sh) + j;
+            if (r < rows && e < cols) single(e);
         }
     }
 }
@@ -348,120 +345,114 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else {
-        // ------------------------------------------------------------ epilogue (warps 2..5)
+        // ------------------------------------------------------------ epilogue (warps 2..9)
+        // Two warps share a quarter of the accumulator's lanes: each reads, rounds and stages 32 of a chunk's 64 columns, and the chunk leaves as one
+        // copy.  With one warp a quarter the epilogue of a 256-column tile took about as long as a reduction of 256
+        // (its warps wait for TMEM, shared memory and the copy engine in turn).
         const int quarter = warp & 3;  // TMEM lanes [32 * quarter, 32 * quarter + 32)
-        const int ew = warp - 2;
-        unsigned char* stage_buf = smem + SmemLayout::epi + ew * 2 * EPI_STAGE_BYTES;
+        const int half = (warp - 2) >> 2;
+        const bool lead = half == 0 && lane == 0;  // the thread that hands a quarter's chunks to the copy engine
+        unsigned char* stage_buf = smem + SmemLayout::epi + quarter * 2 * EPI_STAGE_BYTES;
+        auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory"); };
         int acc = 0, buf = 0;
         uint32_t acc_phase = 0;
         float fused_bias = 0.0f;
         if (MODE == TC_BIAS && p.fuse != 3) fused_bias = p.is_bf16 ? to_f32(*static_cast<const bf16*>(p.bias)) : to_f32(*static_cast<const f16*>(p.bias));
         int tm, tn, tb;
         for (int it = 0; next_tile(it, p, tm, tn, tb); it++) {
-            // the TMEM loads below are warp-collective: leave the loop only as a whole warp
-            // four warps wait here for most of a tile's reduction: they sleep between polls, so that their polling does not
+            // eight warps wait here for most of a tile's reduction: they sleep between polls, so that their polling does not
             // take shared-memory cycles from the TMA writes and the tensor core's operand reads
             if (MODE != TC_STORE && p.fuse == 3) {  // this thread's output row inside the batch's matrix
                 const int row = tm * BM + quarter * 32 + lane;
                 fused_bias = row < p.M ? (p.is_bf16 ? to_f32(static_cast<const bf16*>(p.bias)[row]) : to_f32(static_cast<const f16*>(p.bias)[row])) : 0.0f;
             }
+            // The TMEM loads below take whole warps and the staging both warps of a quarter: these leave the loop together, by a vote that each
+            // of them reaches, its own wait being bounded.
             auto wait_accumulator = [&] {
                 const bool ready = mbar_wait_relaxed(tfull_bar(acc), acc_phase, err, tag, 4, 400);
-                if (!__all_sync(0xFFFFFFFFu, ready)) return false;
+                uint32_t both;
+                __syncwarp();
+                asm volatile(
+                    "{\n\t.reg .pred p, q;\n\t"
+                    "setp.ne.u32 p, %2, 0;\n\t"
+                    "barrier.cta.red.and.pred q, %1, 64, p;\n\t"
+                    "selp.u32 %0, 1, 0, q;\n\t}"
+                    : "=r"(both)
+                    : "r"(1 + quarter), "r"((uint32_t)ready)
+                    : "memory");
+                if (!both) return false;
                 tc_fence_after();
                 return true;
             };
             if (!DRAIN && !wait_accumulator()) break;
-            const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
+            const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * 32);
             const int rows_here = min(32, p.M - (tm * BM + quarter * 32));  // may be <= 0: this warp's rows lie below the matrix
-            // Hands the staged 32 rows of 128 bytes (first output column `col`) to the copy engine, or writes them itself.
-            auto flush = [&](const CUtensorMap* map, int col) {
+            // Stages 32 columns of a row: 16-byte pieces, XOR-swizzled by the row; the chunk (first output column `col`) then goes to the copy engine, or the
+            // warps write its rows themselves.
+            auto flush = [&](const CUtensorMap* map, int col, const uint4 (&q)[4]) {
+                if (lead) tma_store_wait_read<1>();  // the buffer's previous chunk has been read
+                __syncwarp();
+                pair_sync();
                 unsigned char* src = stage_buf + buf * EPI_STAGE_BYTES;
+#pragma unroll
+                for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(src + lane * 128 + (((half * 4 + j) ^ (lane & 7)) << 4)) = q[j];
+                if (MODE != TC_PLAIN) fence_proxy_async_smem();
+                pair_sync();
                 buf ^= 1;
                 if constexpr (MODE != TC_PLAIN) {
-                    if (lane == 0) {
+                    if (lead) {
                         tma_store_3d(map, smem_u32(src), col, tm * BM + quarter * 32, tb);
+                        tma_store_commit();
+                    }
+                } else {
+                    store_rows(static_cast<uint16_t*>(p.d) + ((size_t)tb * p.M + tm * BM + quarter * 32) * p.N + tn * bn, (size_t)p.N, half * 16, rows_here,
+                               min(bn, p.N - tn * bn), (col - tn * bn) / 64, src, stage_buf + buf * EPI_STAGE_BYTES, lane);
+                }
+            };
+            auto pack = [&](const float (&e)[32], uint4 (&q)[4]) {
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    q[j] = make_uint4(pack2(e[8 * j], e[8 * j + 1], p.is_bf16), pack2(e[8 * j + 2], e[8 * j + 3], p.is_bf16), pack2(e[8 * j + 4], e[8 * j + 5], p.is_bf16),
+                                      pack2(e[8 * j + 6], e[8 * j + 7], p.is_bf16));
+            };
+            // This warp's 32 columns of a chunk.
+            auto store_chunk = [&](int c, const uint32_t (&v)[32]) {
+                const int col = tn * bn + c * EPI_CHUNK_COLS;
+                if (MODE == TC_STORE && p.out_f32) {
+                    // f32: 32 columns are the 128 bytes a row of a copy has, so each warp stages and stores its own
+                    if (lane == 0) tma_store_wait_read<0>();
+                    __syncwarp();
+                    unsigned char* src = stage_buf + half * EPI_STAGE_BYTES;
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        *reinterpret_cast<uint4*>(src + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tma_store_3d(&map_d, smem_u32(src), col + half * 32, tm * BM + quarter * 32, tb);
                         tma_store_commit();
                     }
                     return;
                 }
-                store_rows(static_cast<uint16_t*>(p.d) + ((size_t)tb * p.M + tm * BM + quarter * 32) * p.N + tn * bn, (size_t)p.N, rows_here,
-                           min(bn, p.N - tn * bn), (col - tn * bn) / 64, src, stage_buf + buf * EPI_STAGE_BYTES, lane);
-            };
-            // One 64-column chunk: round, stage in shared memory (XOR-swizzled rows), hand to the copy engine.
-            auto store_chunk = [&](int c, uint32_t (&v0)[32], uint32_t (&v1)[32]) {
+                float e[32];
+                uint4 q[4];
+#pragma unroll
+                for (int j = 0; j < 32; j++) e[j] = __uint_as_float(v[j]);
                 if (MODE == TC_BIAS || (MODE == TC_PLAIN && p.fuse)) {
                     // Linear + bias (+ GELU) in one pass, with the roundings of the separate ops: the product is rounded to
                     // the operand type, the bias is added in f32 and rounded (u), the activation is evaluated on u in f32
                     // and rounded (act) - bit for bit what cuda_matmul, cuda_add and cuda_gelu give one after the other.
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        v0[j] = __float_as_uint(round16(round16(__uint_as_float(v0[j]), p.is_bf16) + fused_bias, p.is_bf16));
-                        v1[j] = __float_as_uint(round16(round16(__uint_as_float(v1[j]), p.is_bf16) + fused_bias, p.is_bf16));
-                    }
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        if (h == 1 && (MODE == TC_PLAIN || p.fuse != 2)) break;
-                        if (lane == 0) tma_store_wait_read<1>();
-                        __syncwarp();
-                        unsigned char* dst = stage_buf + buf * EPI_STAGE_BYTES + lane * 128;
-#pragma unroll
-                        for (int j = 0; j < 8; j++) {
-                            const uint32_t* src = j < 4 ? &v0[j * 8] : &v1[(j - 4) * 8];
-                            float e[8];
-#pragma unroll
-                            for (int k = 0; k < 8; k++) e[k] = h ? gelu_f32_fast(__uint_as_float(src[k])) : __uint_as_float(src[k]);  // second pass: the activation of u
-                            uint4 q;
-                            q.x = pack2(e[0], e[1], p.is_bf16);
-                            q.y = pack2(e[2], e[3], p.is_bf16);
-                            q.z = pack2(e[4], e[5], p.is_bf16);
-                            q.w = pack2(e[6], e[7], p.is_bf16);
-                            *reinterpret_cast<uint4*>(dst + ((j ^ (lane & 7)) << 4)) = q;
-                        }
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        flush(h ? &map_d2 : &map_d, tn * bn + c * EPI_CHUNK_COLS);
-                    }
-                    return;
+                    for (int j = 0; j < 32; j++) e[j] = round16(round16(e[j], p.is_bf16) + fused_bias, p.is_bf16);
                 }
-                if (MODE == TC_STORE && p.out_f32) {
-                    // two 32-column f32 chunks (128 bytes per row each), one per staging buffer
+                pack(e, q);
+                flush(&map_d, col, q);
+                if (MODE == TC_BIAS && p.fuse == 2) {
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const uint32_t* v = h ? v1 : v0;
-                        if (lane == 0) tma_store_wait_read<1>();
-                        __syncwarp();
-                        unsigned char* dst = stage_buf + buf * EPI_STAGE_BYTES + lane * 128;
-#pragma unroll
-                        for (int j = 0; j < 8; j++)
-                            *reinterpret_cast<uint4*>(dst + ((j ^ (lane & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            tma_store_3d(&map_d, smem_u32(stage_buf + buf * EPI_STAGE_BYTES), tn * bn + c * EPI_CHUNK_COLS + h * 32, tm * BM + quarter * 32, tb);
-                            tma_store_commit();
-                        }
-                        buf ^= 1;
-                    }
-                    return;
+                    for (int j = 0; j < 32; j++) e[j] = gelu_f32_fast(e[j]);
+                    pack(e, q);
+                    flush(&map_d2, col, q);
                 }
-                // the staging buffer must have been read by its previous TMA store
-                if (lane == 0) tma_store_wait_read<1>();
-                __syncwarp();
-                unsigned char* dst = stage_buf + buf * EPI_STAGE_BYTES + lane * 128;  // row `lane` of the 32 x 64 tile
-#pragma unroll
-                for (int j = 0; j < 8; j++) {  // eight 16-byte chunks per row, XOR-swizzled by the row index
-                    const uint32_t* src = j < 4 ? &v0[j * 8] : &v1[(j - 4) * 8];
-                    uint4 q;
-                    q.x = pack2(__uint_as_float(src[0]), __uint_as_float(src[1]), p.is_bf16);
-                    q.y = pack2(__uint_as_float(src[2]), __uint_as_float(src[3]), p.is_bf16);
-                    q.z = pack2(__uint_as_float(src[4]), __uint_as_float(src[5]), p.is_bf16);
-                    q.w = pack2(__uint_as_float(src[6]), __uint_as_float(src[7]), p.is_bf16);
-                    *reinterpret_cast<uint4*>(dst + ((j ^ (lane & 7)) << 4)) = q;
-                }
-                fence_proxy_async_smem();
-                __syncwarp();
-                flush(&map_d, tn * bn + c * EPI_CHUNK_COLS);
             };
             // The TMEM loads of chunk c + 1 are in flight while chunk c is converted and stored.
             const int chunks = bn / EPI_CHUNK_COLS;
@@ -471,20 +462,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if (lane == 0) mbar_arrive(tempty_bar(acc));
             };
             if constexpr (DRAIN) {
-                uint32_t total[4][32], v[32];
+                uint32_t total[2][32], v[32];  // tiles of at most 128 columns
 #pragma unroll
-                for (int c = 0; c < 4; c++)
+                for (int c = 0; c < 2; c++)
 #pragma unroll
                     for (int j = 0; j < 32; j++) total[c][j] = 0;  // 0.0f
                 bool ok = true;
                 for (int run = 0; run < p.num_kb && ok; run += p.run_kb) {
                     ok = wait_accumulator();
                     if (!ok) break;
-                    const uint32_t t_run = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
+                    const uint32_t t_run = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * 32);
 #pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        if (c * 32 >= bn) break;
-                        tmem_ld_32x32b_x32(t_run + c * 32, v);
+                    for (int c = 0; c < 2; c++) {
+                        if (c >= chunks) break;
+                        tmem_ld_32x32b_x32(t_run + c * EPI_CHUNK_COLS, v);
                         tmem_ld_wait_for(v);
 #pragma unroll
                         for (int j = 0; j < 32; j++) total[c][j] = __float_as_uint(__uint_as_float(total[c][j]) + __uint_as_float(v[j]));
@@ -496,35 +487,24 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 }
                 if (!ok) break;
-                store_chunk(0, total[0], total[1]);
-                if (chunks > 1) store_chunk(1, total[2], total[3]);
+                store_chunk(0, total[0]);
+                if (chunks > 1) store_chunk(1, total[1]);
                 continue;
             }
-            uint32_t a0[32], a1[32], b0[32], b1[32];
-            tmem_ld_32x32b_x32(t_row, a0);
-            tmem_ld_32x32b_x32(t_row + 32, a1);
+            uint32_t va[32], vb[32];
+            tmem_ld_32x32b_x32(t_row, va);
 #pragma unroll
             for (int c = 0; c < BN / EPI_CHUNK_COLS; c += 2) {
                 if (c >= chunks) break;
-                tmem_ld_wait_for(a0);
-                reg_fence(a1);
-                if (c + 1 < chunks) {
-                    tmem_ld_32x32b_x32(t_row + (c + 1) * EPI_CHUNK_COLS, b0);
-                    tmem_ld_32x32b_x32(t_row + (c + 1) * EPI_CHUNK_COLS + 32, b1);
-                } else {
-                    hand_back();
-                }
-                store_chunk(c, a0, a1);
+                tmem_ld_wait_for(va);
+                if (c + 1 < chunks) tmem_ld_32x32b_x32(t_row + (c + 1) * EPI_CHUNK_COLS, vb);
+                else hand_back();
+                store_chunk(c, va);
                 if (c + 1 >= chunks) break;
-                tmem_ld_wait_for(b0);
-                reg_fence(b1);
-                if (c + 2 < chunks) {
-                    tmem_ld_32x32b_x32(t_row + (c + 2) * EPI_CHUNK_COLS, a0);
-                    tmem_ld_32x32b_x32(t_row + (c + 2) * EPI_CHUNK_COLS + 32, a1);
-                } else {
-                    hand_back();
-                }
-                store_chunk(c + 1, b0, b1);
+                tmem_ld_wait_for(vb);
+                if (c + 2 < chunks) tmem_ld_32x32b_x32(t_row + (c + 2) * EPI_CHUNK_COLS, va);
+                else hand_back();
+                store_chunk(c + 1, vb);
             }
             if (++acc == 2) {
                 acc = 0;
