@@ -118,6 +118,9 @@ struct TcParams {
     // tiles j, j + b_keep, ...; the B panel of the column tile is loaded once into the B slots of the ring (slot = k-block,
     // the ring is num_kb slots long) and only A streams.  0: the general schedule.
     int b_keep;
+    // Short reductions of a batch: the tiles in the order batch, column tile, row tile, an equal run of them for each CTA, which loads a B panel
+    // once for all row tiles of it.
+    int panels;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, const TcParams& p, int& tm, int& tn, int& tb) {
@@ -140,6 +143,15 @@ __device__ __forceinline__ bool next_tile(int it, const TcParams& p, int& tm, in
         tm = (int)blockIdx.x % p.b_keep + it * p.b_keep;
         tb = 0;
         return tn < p.tiles_n && tm < p.tiles_m;
+    }
+    if (p.panels) {
+        const int tile = (int)((long long)blockIdx.x * p.num_tiles / gridDim.x) + it;
+        if (tile >= (int)((long long)(blockIdx.x + 1) * p.num_tiles / gridDim.x)) return false;
+        const int panel = tile / p.tiles_m;
+        tm = tile - panel * p.tiles_m;
+        tb = panel / p.tiles_n;
+        tn = panel - tb * p.tiles_n;
+        return true;
     }
     const int tile = (int)blockIdx.x + it * (int)gridDim.x;
     if (tile >= p.num_tiles) return false;
@@ -268,12 +280,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            const int ring = p.b_keep ? p.num_kb : stages;
+            const int ring = p.b_keep || p.panels ? p.num_kb : stages;
             int tm, tn, tb;
             for (int it = 0; ok && next_tile(it, p, tm, tn, tb); it++) {
                 const int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
                 int k = tb * p.split_kb * BK;              // a k-block past the end of K is all fill: zeros
-                const bool load_b = !p.b_keep || it == 0;  // the kept B panel arrives with the first tile's A blocks
+                const bool load_b = it == 0 || (p.panels ? tm == 0 : !p.b_keep);  // a kept B panel arrives with its first tile's A blocks
                 for (int kb = 0; kb < p.num_kb; kb++, k += BK) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, err, tag, 1)) {
                         ok = false;
@@ -311,7 +323,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
-            const int ring = p.b_keep ? p.num_kb : stages;
+            const int ring = p.b_keep || p.panels ? p.num_kb : stages;
             int tm, tn, tb;
             int run = 0;  // first k-block of the accumulator's run (DRAIN: a tile has several)
             for (int it = 0; ok && next_tile(it, p, tm, tn, tb); it += DRAIN && run ? 0 : 1) {
@@ -572,6 +584,11 @@ int keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, int ctas) {
     return tiles_m >= 4 * per_col ? per_col : 0;
 }
 
+// The same for a batch: with four row tiles and more to a panel and enough tiles that the runs' ends do not count.
+bool keep_panels(uint64_t tiles_m, uint64_t tiles_n, int num_kb, uint64_t batch, int ctas) {
+    return g_keep_b.load(std::memory_order_relaxed) && batch > 1 && num_kb <= STAGES && tiles_m >= 4 && tiles_m * tiles_n * batch >= 8 * (uint64_t)ctas;
+}
+
 // The two-CTA kernel: B is staged in halves of 128 columns, a pair of CTAs owns a 256 x 256 tile.  Its split-K slices are
 // sub-matrices behind the third coordinate of the tensor maps.  false: nothing was launched.
 bool launch_two_cta(bool is_bf16, const TcProduct& c, void* D, const char* where, int grid) {
@@ -668,6 +685,7 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     // few output tiles: cut K into slices that run as the batches of this launch
     int slices = 1;
     const int bn_whole = p.b_keep ? p.bn : tile_columns((uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid);
+    p.panels = p.bn == BN && bn_whole == BN && keep_panels((uint64_t)p.tiles_m, (uint64_t)p.tiles_n, p.num_kb, batch, grid) ? 1 : 0;
     if (batch == 1 && !fuse && !p.b_keep) {
         slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
         if (slices == 1)
