@@ -66,15 +66,18 @@ __global__ void __launch_bounds__(kFusedThreads) bias_gelu_kernel(const T* __res
         }
 }
 
+// d/dx of x * sigmoid(2t), t = sqrt(2/pi) (x + 0.044715 x^3) - the tanh form's derivative, 0.5 (1 + tanh t) being sigmoid(2t):
+//   sigmoid + x sigmoid (1 - sigmoid) (2t)'
+// Ten instructions and two of the special-function unit, where tanh, its square and the separately rounded products took thirty.
+// For negative x the sigmoid keeps its relative accuracy, which 1 + tanh t loses.
 __device__ __forceinline__ float gelu_grad_f32(float x) {
-    const float s = 0.7978845608028654f, c = 0.044715f;
+    const float k1 = -2.302208198f, k2 = -0.102943240f;  // exp(-2t) = 2^(x (k1 + k2 x^2)), as in gelu_f32_fast
+    const float c1 = 1.5957691216f, c2 = 0.2140644488f;  // (2t)' = c1 + c2 x^2: 2 sqrt(2/pi), three times 0.044715 of that
     const float x2 = x * x;
-    const float t = s * (x + c * x2 * x);
-    // tanh(t) = 1 - 2 / (1 + exp(2t)); sech^2 = 1 - tanh^2
-    const float e = __expf(2.0f * t);
-    const float th = 1.0f - __fdividef(2.0f, 1.0f + e);
-    const float sech2 = 1.0f - th * th;
-    return 0.5f * (1.0f + th) + 0.5f * x * sech2 * s * (1.0f + 3.0f * c * x2);
+    float e, sig;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * fmaf(k2, x2, k1)));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(sig) : "f"(1.0f + e));
+    return fmaf(fmaf(-sig, sig, sig) * x, fmaf(c2, x2, c1), sig);
 }
 
 // The block's sum of v; valid in thread 0.
@@ -89,22 +92,49 @@ __device__ __forceinline__ float fused_block_sum(float v) {
     return v;
 }
 
-// SUM: per-block partial sums of du into `partial` (the bias gradient), which the pass over du that used to follow read it back for.
+// A pass that leaves a sum over everything it writes ends with it: every block leaves its part in `partial`, and the last one to arrive
+// folds the parts in block order.  (A launch of its own for that took 2 to 4 us.)  True in every thread of the last block, which then sees all parts.
+// `arrived` is a zeroed word, left zeroed.
+__device__ __forceinline__ bool fused_last_block(uint32_t* arrived) {
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+        if (last) *arrived = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// SUM: the sum of du (the bias gradient), which a pass over du used to read it back for.  Two vectors of each operand in flight
+// per thread.
 template <class T, bool SUM>
 __global__ void __launch_bounds__(kFusedThreads) gelu_backward_kernel(const T* __restrict__ dy, const T* __restrict__ u, T* __restrict__ du,
-                                                                     uint64_t n, float* __restrict__ partial) {
+                                                                     uint64_t n, float* __restrict__ partial, uint32_t* arrived, T* grad_sum) {
     float acc = 0.0f;
-    constexpr int VEC = 16 / sizeof(T);
+    constexpr int VEC = 16 / sizeof(T), UN = 2;
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
-    for (uint64_t v = (uint64_t)blockIdx.x * kFusedThreads + threadIdx.x; v < nvec; v += stride) {
-        Vec<T, VEC> g = *reinterpret_cast<const Vec<T, VEC>*>(dy + v * VEC), x = *reinterpret_cast<const Vec<T, VEC>*>(u + v * VEC), o;
+    for (uint64_t v0 = (uint64_t)blockIdx.x * kFusedThreads + threadIdx.x; v0 < nvec; v0 += UN * stride) {
+        Vec<T, VEC> g[UN], x[UN];
 #pragma unroll
-        for (int j = 0; j < VEC; j++) {
-            o.v[j] = st_from_f32<T>(up(g.v[j]) * gelu_grad_f32(up(x.v[j])));
-            if (SUM) acc += up(o.v[j]);
-        }
-        *reinterpret_cast<Vec<T, VEC>*>(du + v * VEC) = o;
+        for (int i = 0; i < UN; i++)
+            if (v0 + i * stride < nvec) {
+                g[i] = *reinterpret_cast<const Vec<T, VEC>*>(dy + (v0 + i * stride) * VEC);
+                x[i] = *reinterpret_cast<const Vec<T, VEC>*>(u + (v0 + i * stride) * VEC);
+            }
+#pragma unroll
+        for (int i = 0; i < UN; i++)
+            if (v0 + i * stride < nvec) {
+                Vec<T, VEC> o;
+#pragma unroll
+                for (int j = 0; j < VEC; j++) {
+                    o.v[j] = st_from_f32<T>(up(g[i].v[j]) * gelu_grad_f32(up(x[i].v[j])));
+                    if (SUM) acc += up(o.v[j]);
+                }
+                *reinterpret_cast<Vec<T, VEC>*>(du + (v0 + i * stride) * VEC) = o;
+            }
     }
     if (blockIdx.x == 0)
         for (uint64_t i = nvec * VEC + threadIdx.x; i < n; i += kFusedThreads) {
@@ -114,21 +144,34 @@ __global__ void __launch_bounds__(kFusedThreads) gelu_backward_kernel(const T* _
     if constexpr (SUM) {
         acc = fused_block_sum(acc);
         if (threadIdx.x == 0) partial[blockIdx.x] = acc;
+        if (!fused_last_block(arrived)) return;
+        acc = 0.0f;
+        for (uint32_t i = threadIdx.x; i < gridDim.x; i += kFusedThreads) acc += __ldcg(partial + i);
+        acc = fused_block_sum(acc);
+        if (threadIdx.x == 0) *grad_sum = st_from_f32<T>(acc);
     }
 }
-// One block: the rounded sum of the partial sums, in a fixed order.
-template <class T>
-__global__ void __launch_bounds__(kFusedThreads) sum_finish_kernel(const float* __restrict__ partial, int count, T* __restrict__ out) {
+
+// The sum of the blocks' parts in a fixed order; valid in thread 0.
+__device__ __forceinline__ float mse_fold(const float* partial, uint32_t count) {
+    __shared__ float sm[kFusedThreads];
     float acc = 0.0f;
-    for (int i = threadIdx.x; i < count; i += kFusedThreads) acc += partial[i];
-    acc = fused_block_sum(acc);
-    if (threadIdx.x == 0) *out = st_from_f32<T>(acc);
+    for (uint32_t i = threadIdx.x; i < count; i += kFusedThreads) acc += __ldcg(partial + i);
+    __syncthreads();  // an earlier fold's result has been read
+    sm[threadIdx.x] = acc;
+    __syncthreads();
+    for (int o = kFusedThreads / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
+        __syncthreads();
+    }
+    return sm[0];
 }
 
-// Pass 1: grad = 2 (p - t) / n, per-block partial sums of (p - t)^2 into `partial` and, with SUM, of grad behind them.
+// grad = 2 (p - t) / n, per-block partial sums of (p - t)^2 into `partial` and, with SUM, of grad behind them; with SUM the last block folds both.
 template <class T, bool SUM>
 __global__ void __launch_bounds__(kFusedThreads) mse_kernel(const T* __restrict__ p, const T* __restrict__ t, T* __restrict__ grad,
-                                                           float* __restrict__ partial, uint64_t n, float two_over_n) {
+                                                           float* __restrict__ partial, uint64_t n, float two_over_n, float inv_n, float* loss,
+                                                           T* grad_sum, uint32_t* arrived) {
     constexpr int VEC = 16 / sizeof(T);
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
@@ -168,24 +211,24 @@ __global__ void __launch_bounds__(kFusedThreads) mse_kernel(const T* __restrict_
         float v = lane < kFusedThreads / 32 ? warp_part[which][lane] : 0.0f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        if (lane == 0) partial[which * gridDim.x + blockIdx.x] = v;
+        if (lane == 0) {
+            partial[which * gridDim.x + blockIdx.x] = v;
+            __threadfence();
+        }
+    }
+    if constexpr (SUM) {
+        __syncthreads();
+        if (!fused_last_block(arrived)) return;
+        const float l = mse_fold(partial, gridDim.x), g = mse_fold(partial + gridDim.x, gridDim.x);
+        if (threadIdx.x) return;
+        *loss = l * inv_n;
+        *grad_sum = st_from_f32<T>(g);
     }
 }
-// Pass 2: one block per output folds its partials in a fixed order: block 0 the loss, block 1 the gradient's sum.
-template <class T>
-__global__ void __launch_bounds__(kFusedThreads) mse_finish_kernel(const float* __restrict__ partial, int count, float inv_n, float* __restrict__ loss, T* __restrict__ grad_sum) {
-    __shared__ float sm[kFusedThreads];
-    float acc = 0.0f;
-    for (int i = threadIdx.x; i < count; i += kFusedThreads) acc += partial[(int)blockIdx.x * count + i];
-    sm[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = kFusedThreads / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x) return;
-    if (blockIdx.x == 0) *loss = sm[0] * inv_n;
-    else *grad_sum = st_from_f32<T>(sm[0]);
+// Without an arrival word (the exported pass, whose caller has none): the loss folded by a launch of one block.
+__global__ void __launch_bounds__(kFusedThreads) mse_finish_kernel(const float* __restrict__ partial, int count, float inv_n, float* __restrict__ loss) {
+    const float l = mse_fold(partial, (uint32_t)count);
+    if (threadIdx.x == 0) *loss = l * inv_n;
 }
 
 template <class T>
@@ -228,8 +271,11 @@ __global__ void __launch_bounds__(kFusedThreads) sgd_kernel(float* __restrict__ 
         }
 }
 
+// Four vectors per thread, up to 16 blocks an SM; small tensors one vector per thread, since four trips to memory one after the other are
+// longer than what more blocks cost.
 static unsigned fused_grid(uint64_t n, int vec) {
     uint64_t blocks = (n / vec + kFusedThreads * 4 - 1) / (kFusedThreads * 4);
+    if (blocks < (uint64_t)sm_count() * 2) blocks = (n / vec + kFusedThreads - 1) / kFusedThreads;
     uint64_t cap = (uint64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
     return blocks ? (unsigned)blocks : 1u;
@@ -247,7 +293,7 @@ void bias_gelu_launch(size_t n, const T* z, const T* bias, T* u, T* a, const cha
     check_launch(where);
 }
 template <class T>
-void gelu_backward_launch(size_t n, const T* dy, const T* u, T* du, T* grad_sum, const char* where) {
+void gelu_backward_launch(size_t n, const T* dy, const T* u, T* du, T* grad_sum, uint32_t* arrived, const char* where) {
     if (!n) return;
     if (!aligned16(dy) || !aligned16(u) || !aligned16(du)) {
         set_error(kErrUnsupported, 0, where);
@@ -255,17 +301,16 @@ void gelu_backward_launch(size_t n, const T* dy, const T* u, T* du, T* grad_sum,
     }
     const unsigned blocks = fused_grid(n, 16 / sizeof(T));
     if (!grad_sum) {
-        gelu_backward_kernel<T, false><<<blocks, kFusedThreads, 0, ctx().stream>>>(dy, u, du, n, nullptr);
+        gelu_backward_kernel<T, false><<<blocks, kFusedThreads, 0, ctx().stream>>>(dy, u, du, n, nullptr, nullptr, nullptr);
     } else {
         float* partial = static_cast<float*>(scratch(sizeof(float) * blocks));
         if (!partial) return;
-        gelu_backward_kernel<T, true><<<blocks, kFusedThreads, 0, ctx().stream>>>(dy, u, du, n, partial);
-        sum_finish_kernel<T><<<1, kFusedThreads, 0, ctx().stream>>>(partial, (int)blocks, grad_sum);
+        gelu_backward_kernel<T, true><<<blocks, kFusedThreads, 0, ctx().stream>>>(dy, u, du, n, partial, arrived, grad_sum);
     }
     check_launch(where);
 }
 template <class T>
-void mse_launch(size_t n, const T* p, const T* t, T* grad, float* loss, T* grad_sum, const char* where) {
+void mse_launch(size_t n, const T* p, const T* t, T* grad, float* loss, T* grad_sum, uint32_t* arrived, const char* where) {
     if (!n) return;
     if (!aligned16(p) || !aligned16(t) || !aligned16(grad)) {
         set_error(kErrUnsupported, 0, where);
@@ -274,9 +319,13 @@ void mse_launch(size_t n, const T* p, const T* t, T* grad, float* loss, T* grad_
     unsigned blocks = fused_grid(n, 16 / sizeof(T));
     float* partial = static_cast<float*>(scratch(sizeof(float) * blocks * (grad_sum ? 2 : 1)));
     if (!partial) return;
-    if (grad_sum) mse_kernel<T, true><<<blocks, kFusedThreads, 0, ctx().stream>>>(p, t, grad, partial, n, 2.0f / (float)n);
-    else mse_kernel<T, false><<<blocks, kFusedThreads, 0, ctx().stream>>>(p, t, grad, partial, n, 2.0f / (float)n);
-    mse_finish_kernel<T><<<grad_sum ? 2 : 1, kFusedThreads, 0, ctx().stream>>>(partial, (int)blocks, 1.0f / (float)n, loss, grad_sum);
+    const float two_over_n = 2.0f / (float)n, inv_n = 1.0f / (float)n;
+    if (grad_sum) {
+        mse_kernel<T, true><<<blocks, kFusedThreads, 0, ctx().stream>>>(p, t, grad, partial, n, two_over_n, inv_n, loss, grad_sum, arrived);
+    } else {
+        mse_kernel<T, false><<<blocks, kFusedThreads, 0, ctx().stream>>>(p, t, grad, partial, n, two_over_n, inv_n, nullptr, nullptr, nullptr);
+        mse_finish_kernel<<<1, kFusedThreads, 0, ctx().stream>>>(partial, (int)blocks, inv_n, loss);
+    }
     check_launch(where);
 }
 template <class T>
@@ -291,21 +340,21 @@ void sgd_launch(size_t n, float* w32, const T* g, T* w16, float lr, float grad_s
 }
 
 template <class T>
-void mse_loss_grad_sum(size_t n, const T* pred, const T* target, T* grad, float* loss, T* grad_sum, const char* where) {
-    mse_launch<T>(n, pred, target, grad, loss, grad_sum, where);
+void mse_loss_grad_sum(size_t n, const T* pred, const T* target, T* grad, float* loss, T* grad_sum, uint32_t* arrived, const char* where) {
+    mse_launch<T>(n, pred, target, grad, loss, grad_sum, arrived, where);
 }
 template <class T>
-void gelu_backward_sum(size_t n, const T* dy, const T* u, T* du, T* grad_sum, const char* where) {
-    gelu_backward_launch<T>(n, dy, u, du, grad_sum, where);
+void gelu_backward_sum(size_t n, const T* dy, const T* u, T* du, T* grad_sum, uint32_t* arrived, const char* where) {
+    gelu_backward_launch<T>(n, dy, u, du, grad_sum, arrived, where);
 }
 template <class T>
 void sgd_update_layer(size_t n, float* w32, const T* grad, T* w16, float* b32, const T* grad_b, T* b16, float lr, float grad_scale, const char* where) {
     sgd_launch<T>(n, w32, grad, w16, lr, grad_scale, where, b32, grad_b, b16);
 }
-template void mse_loss_grad_sum<bf16>(size_t, const bf16*, const bf16*, bf16*, float*, bf16*, const char*);
-template void mse_loss_grad_sum<f16>(size_t, const f16*, const f16*, f16*, float*, f16*, const char*);
-template void gelu_backward_sum<bf16>(size_t, const bf16*, const bf16*, bf16*, bf16*, const char*);
-template void gelu_backward_sum<f16>(size_t, const f16*, const f16*, f16*, f16*, const char*);
+template void mse_loss_grad_sum<bf16>(size_t, const bf16*, const bf16*, bf16*, float*, bf16*, uint32_t*, const char*);
+template void mse_loss_grad_sum<f16>(size_t, const f16*, const f16*, f16*, float*, f16*, uint32_t*, const char*);
+template void gelu_backward_sum<bf16>(size_t, const bf16*, const bf16*, bf16*, bf16*, uint32_t*, const char*);
+template void gelu_backward_sum<f16>(size_t, const f16*, const f16*, f16*, f16*, uint32_t*, const char*);
 template void sgd_update_layer<bf16>(size_t, float*, const bf16*, bf16*, float*, const bf16*, bf16*, float, float, const char*);
 template void sgd_update_layer<f16>(size_t, float*, const f16*, f16*, float*, const f16*, f16*, float, float, const char*);
 
@@ -316,10 +365,10 @@ template void sgd_update_layer<f16>(size_t, float*, const f16*, f16*, float*, co
         mx::bias_gelu_launch<mx_##T>(n, z, bias, u, a, "mx_bias_gelu_" #T);                                                             \
     }                                                                                                                                   \
     void mx_gelu_backward_##T(size_t n, const mx_##T* dy, const mx_##T* u, mx_##T* du) {                                                \
-        mx::gelu_backward_launch<mx_##T>(n, dy, u, du, nullptr, "mx_gelu_backward_" #T);                                                \
+        mx::gelu_backward_launch<mx_##T>(n, dy, u, du, nullptr, nullptr, "mx_gelu_backward_" #T);                                                \
     }                                                                                                                                   \
     void mx_mse_loss_grad_##T(size_t n, const mx_##T* pred, const mx_##T* target, mx_##T* grad, float* loss) {                          \
-        mx::mse_launch<mx_##T>(n, pred, target, grad, loss, nullptr, "mx_mse_loss_grad_" #T);                                           \
+        mx::mse_launch<mx_##T>(n, pred, target, grad, loss, nullptr, nullptr, "mx_mse_loss_grad_" #T);                                           \
     }                                                                                                                                   \
     void mx_sgd_update_##T(size_t n, float* w32, const mx_##T* grad, mx_##T* w16, float lr, float grad_scale) {                         \
         mx::sgd_launch<mx_##T>(n, w32, grad, w16, lr, grad_scale, "mx_sgd_update_" #T);                                                 \

@@ -55,6 +55,7 @@ struct Mlp {
                                          // data-parallel step can finish layer 0 before it computes layer 1's weight gradient
     const uint16_t* x = nullptr;         // input batch of the current step
     float* loss = nullptr;               // device scalar
+    uint32_t* arrived = nullptr;         // zeroed word for the passes whose last block folds a sum
     std::vector<void*> owned;
     // data-parallel mode over peer-mapped arenas (dp_sync.cu); world == 1 and dp == false otherwise
     bool dp = false;
@@ -143,7 +144,7 @@ static void loss_backward_t(Mlp* m, const T* y) {
     const size_t n = m->batch * m->dim;
     const T* pred = reinterpret_cast<const T*>(m->u[m->layers - 1]);
     // the same pass leaves the last layer's bias gradient, the sum of the gradient it writes
-    mse_loss_grad_sum<T>(n, pred, y, reinterpret_cast<T*>(m->du[(m->layers - 1) & 1]), m->loss, reinterpret_cast<T*>(m->gb[m->layers - 1]), "mx_mlp_loss_backward");
+    mse_loss_grad_sum<T>(n, pred, y, reinterpret_cast<T*>(m->du[(m->layers - 1) & 1]), m->loss, reinterpret_cast<T*>(m->gb[m->layers - 1]), m->arrived, "mx_mlp_loss_backward");
 }
 
 // Backward of layer l, first part: the gradient w.r.t. the pre-activation, the bias gradient, and the gradient
@@ -156,7 +157,7 @@ static void backward_input_t(Mlp* m, int l) {
     // of du over all elements (the scalar bias broadcasts over the whole output); the last layer's came with its du.
     // At 16384 x 8192 the sums' own passes took 51 us a layer.
     if (l != m->layers - 1)
-        gelu_backward_sum<T>(n, reinterpret_cast<const T*>(m->d_act), reinterpret_cast<const T*>(m->u[l]), du, reinterpret_cast<T*>(m->gb[l]), "mx_mlp_backward_layer");
+        gelu_backward_sum<T>(n, reinterpret_cast<const T*>(m->d_act), reinterpret_cast<const T*>(m->u[l]), du, reinterpret_cast<T*>(m->gb[l]), m->arrived, "mx_mlp_backward_layer");
     // gradient for the layer below: da_prev [B, D_in] = du [B, D_out] . W [D_out, D_in]
     if (l > 0) {
         const size_t meta[] = {2, 2, 2, B, D, B, D, D, D, D, 1, D, 1, 0, 0};
@@ -246,8 +247,9 @@ static Mlp* mlp_create_impl(int layers, size_t dim, size_t batch, int dtype, uin
     m->du[0] = static_cast<uint16_t*>(dmalloc(m, an * 2));
     m->du[1] = static_cast<uint16_t*>(dmalloc(m, an * 2));
     m->loss = static_cast<float*>(dmalloc(m, 256));
+    m->arrived = static_cast<uint32_t*>(dmalloc(m, 256));
     m->dp_err = static_cast<uint32_t*>(dmalloc(m, 256));
-    ok = ok && m->z && m->d_act && m->du[0] && m->du[1] && m->loss && m->dp_err;
+    ok = ok && m->z && m->d_act && m->du[0] && m->du[1] && m->loss && m->arrived && m->dp_err;
     if (ok) {
         int lo = 0, hi = 0;
         cudaDeviceGetStreamPriorityRange(&lo, &hi);
@@ -267,6 +269,7 @@ static Mlp* mlp_create_impl(int layers, size_t dim, size_t batch, int dtype, uin
     const float bound = 1.0f / std::sqrt((float)dim);
     cudaStream_t s = ctx().stream;
     cudaMemsetAsync(m->dp_err, 0, 256, s);
+    cudaMemsetAsync(m->arrived, 0, 256, s);
     for (int l = 0; l < layers; l++) {
         cudaMemsetAsync(m->b32[l], 0, 256, s);
         cudaMemsetAsync(m->b16[l], 0, 256, s);
