@@ -898,9 +898,83 @@ __global__ void __launch_bounds__(kEwThreads) ew_dense_kernel(F f, const T* a, c
         if (w[u].live) ew_dense_store<F, T, O, NIN, VEC>(f, out, w[u], va[u], vb[u]);
 }
 
+// Two inputs, each either the output's own layout (vector loads) or constant along the innermost dim of at most three - a per-row or a per-channel
+// operand whose rows are no whole vectors, the commonest call of the kernel above.  What bounds that one there is its instructions (loops over the
+// dims, every element's own choice): here the place of a vector costs two divisions by multiplication, the row behind comes from
+// the one before it without another, both values a vector can see are loaded whether or not its rows change inside it, and a thread has
+// four vectors' loads in flight.
+struct FastDiv31 {  // floor(n / d) for n < 2^31 and d >= 2: with 2^s < d <= 2^(s+1) and m = ceil(2^(32+s) / d), n (m d - 2^(32+s)) < 2^(32+s)
+    uint32_t d, m, s;
+    void init(uint32_t div) {
+        d = div;
+        for (s = 0; (2ull << s) < d; s++) {
+        }
+        m = (uint32_t)(((1ull << (32 + s)) + d - 1) / d);
+    }
+    __device__ __forceinline__ uint32_t div(uint32_t n) const { return __umulhi(n, m) >> s; }
+};
+struct EwChanParams {
+    uint32_t n, q, channels;    // elements; extent of the innermost dim and of the middle one
+    FastDiv31 q_div, channel_div;
+    int vector[3];              // [1], [2]: the input has the output's layout
+    int s_outer[3], s_channel[3];
+};
+constexpr int kEwChanUnroll = 4;
+template <class F, class T, class O, int VEC>
+__global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, const T* b, O* out, EwChanParams P) {
+    constexpr int U = kEwChanUnroll;
+    const uint32_t first = (blockIdx.x * U * kEwThreads + threadIdx.x) * VEC;
+    Vec<T, VEC> va[U], vb[U];
+    T xa[U][2], xb[U][2];
+    int left[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const uint32_t i0 = first + u * kEwThreads * VEC;
+        if (i0 >= P.n) continue;
+        const uint32_t row = P.q_div.div(i0), outer = P.channel_div.div(row), channel = row - outer * P.channels;
+        left[u] = (int)(P.q - (i0 - row * P.q));  // elements of the vector's first row from i0 on
+        const bool wraps = channel + 1 == P.channels, ends = left[u] < VEC && i0 + left[u] < P.n;
+        auto load = [&](const T* p, int k, Vec<T, VEC>& v, T(&x)[2]) {
+            if (P.vector[k]) {
+                if (i0 + VEC <= P.n) v = ld_vec<T, VEC>(p + i0);
+                else
+#pragma unroll
+                    for (int j = 0; j < VEC; j++)
+                        if (i0 + j < P.n) v.v[j] = p[i0 + j];
+            } else {
+                const int o0 = (int)outer * P.s_outer[k] + (int)channel * P.s_channel[k];
+                const int o1 = wraps ? (int)(outer + 1) * P.s_outer[k] : o0 + P.s_channel[k];
+                x[0] = p[o0];
+                x[1] = p[ends ? o1 : o0];
+            }
+        };
+        load(a, 1, va[u], xa[u]);
+        load(b, 2, vb[u], xb[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const uint32_t i0 = first + u * kEwThreads * VEC;
+        if (i0 >= P.n) continue;
+        auto spread = [&](int k, Vec<T, VEC>& v, const T(&x)[2]) {
+            if (!P.vector[k])
+#pragma unroll
+                for (int j = 0; j < VEC; j++) v.v[j] = j < left[u] ? x[0] : x[1];
+        };
+        spread(1, va[u], xa[u]);
+        spread(2, vb[u], xb[u]);
+        if (i0 + VEC <= P.n) st_vec<O, VEC>(out + i0, apply_vec<F, T, O, 2, VEC>(f, va[u], vb[u]));
+        else
+#pragma unroll
+            for (int j = 0; j < VEC; j++)
+                if (i0 + j < P.n) out[i0 + j] = f(va[u].v[j], vb[u].v[j]);
+    }
+}
+
 // ---------------------------------------------------------------------------------
 // launcher
 // ---------------------------------------------------------------------------------
+// The dense-output kernel's parameters as those of the kernel of rows and channels; false when they are not of its form.
+bool ew_fill_chan_params(const EwDenseParams& D, int vec, EwChanParams& P);
 // Fills the parameters for the dense-output kernel; false when the output is not dense from `out` on or not vector-aligned, or
 // an offset does not fit 31 bits.
 bool ew_fill_dense_params(const EwPlan& pl, size_t in_size, size_t out_size, const void* out, const void* a, const void* b, EwDenseParams& P);
@@ -1046,6 +1120,13 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
             EwDenseParams D;
             if (pl.kind == EW_GENERIC && ew_fill_dense_params(pl, sizeof(T), sizeof(O), out, a, b, D)) {
                 const uint64_t vecs = (pl.n + VEC - 1) / VEC;
+                if constexpr (NIN == 2 && VEC <= 8) {  // 16 elements a vector would take 145 registers
+                    EwChanParams C;
+                    if (ew_fill_chan_params(D, VEC, C)) {
+                        ew_chan_kernel<F, T, O, VEC><<<(uint32_t)((vecs + kEwThreads * kEwChanUnroll - 1) / (kEwThreads * kEwChanUnroll)), kEwThreads, 0, s>>>(f, a, b, out, C);
+                        break;
+                    }
+                }
                 ew_dense_kernel<F, T, O, NIN, VEC><<<(uint32_t)((vecs + kEwThreads * kEwDenseUnroll - 1) / (kEwThreads * kEwDenseUnroll)), kEwThreads, 0, s>>>(f, a, b, out, D);
                 break;
             }

@@ -344,6 +344,23 @@ bool ew_fill_dense_params(const EwPlan& pl, size_t in_size, size_t out_size, con
     return true;
 }
 
+bool ew_fill_chan_params(const EwDenseParams& D, int vec, EwChanParams& P) {
+    if (D.nd < 2 || D.nd > 3 || D.q < (uint32_t)vec) return false;  // a vector has elements of two rows at most
+    for (int k = 1; k < 3; k++) {
+        if (D.kind[k] != EWD_VECTOR && D.kind[k] != EWD_CONST) return false;
+        P.vector[k] = D.kind[k] == EWD_VECTOR ? 1 : 0;
+        P.s_outer[k] = D.nd == 3 ? D.st[k][0] : 0;
+        P.s_channel[k] = D.st[k][D.nd - 2];
+    }
+    P.n = D.n;
+    P.q = D.q;
+    P.channels = D.div[D.nd - 2].d;
+    if (P.channels < 2) return false;
+    P.q_div.init(P.q);
+    P.channel_div.init(P.channels);
+    return true;
+}
+
 void ew_fill_gen_params(const EwPlan& pl, EwGenParams& P) {
     P.nd = pl.nd;
     P.n = pl.n;

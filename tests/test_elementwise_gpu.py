@@ -368,6 +368,33 @@ def test_flat_operands_at_unaligned_offsets(oracle, cuda, dt):
     H.assert_same("add", dt, H.run_binary(cuda, *args), H.run_binary(oracle, *args), what="2-d + scalar")
 
 
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16, D.F64, D.I16], ids=lambda d: d.name)
+@pytest.mark.parametrize("q", ["vec", "vec+1", 49, 197, 1023])
+def test_operands_constant_along_ragged_rows(oracle, cuda, dt, q):
+    """Per-row and per-channel operands of rows that are no whole vectors, on either side and on both, with an outer stride of their own, as a
+    comparison and in place; tensors that end inside a vector, whose last vector starts in the row before, and whose rows are two."""
+    vec = 16 // dt.size
+    q = {"vec": vec, "vec+1": vec + 1}.get(q, q)
+    rng = np.random.default_rng(q * dt.size)
+    least = (1 << 15) * vec
+    r = least // q + 3
+    c = 7
+    o = r // c + 1
+    layouts = [("row", [r, q], [q, 1], [1, 0]), ("row-strided", [r, q], [q, 1], [3, 0]), ("channel", [o, c, q], [c * q, q, 1], [0, 1, 0]),
+               ("outer", [o, c, q], [c * q, q, 1], [1, 0, 0]), ("both", [o, c, q], [c * q, q, 1], [c + 2, 1, 0]), ("two-rows", [2, least + 5], [least + 5, 1], [1, 0])]
+    for name, dims, dense, const in layouts:
+        n = H.numel(dims)
+        size = 1 + sum((d - 1) * s for d, s in zip(dims, const))
+        full = H.random_store(rng, dt, n, lo=1, hi=50) if dt.kind != "float" else H.random_store(rng, dt, n, lo=0.5, hi=2.0)
+        part = H.random_store(rng, dt, size + 2, lo=1, hi=50) if dt.kind != "float" else H.random_store(rng, dt, size + 2, lo=0.5, hi=2.0)
+        for op, sa, sb, off, a, b in (("sub", dense, const, 0, full, part), ("div", const, dense, 0, part, full), ("mul", const, const, 0, part, part), ("lt", dense, const, 1, full, part)):
+            loff, roff = (0, off) if sa is dense else (off, 0)
+            args = (op, dt, dims, sa, sb, loff, roff, a, b)
+            H.assert_same(op, dt, H.run_binary(cuda, *args), H.run_binary(oracle, *args), what=f"{name} {op} q={q}")
+        args = ("add_inplace", dt, dims, dense, const, 0, 2, full, part)
+        H.assert_same("add_inplace", dt, H.run_binary_inplace(cuda, *args), H.run_binary_inplace(oracle, *args), what=f"{name} in place q={q}")
+
+
 @pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F64, D.U8, D.I32], ids=lambda d: d.name)
 def test_last_block_of_flat_operands(oracle, cuda, dt):
     """The block that is not full works by vectors too: lengths around the vector, a block's 256 threads and its four vectors a thread."""
