@@ -265,9 +265,11 @@ MX_DTYPES_ALL(MX_DECL_CAST_FROM, _)
  * 0 turns both off: every request goes to cudaMalloc / cudaFree / cudaMemcpy, as in the reference. */
 void mx_set_small_pool(int enabled);
 
-/* What a dispatch layer does around an op, in two calls: select `device`, cuda_malloc a metadata block and cuda_memcpy_h2d
- * `count` words into it (returns the first failing call's code, 0 = ok); after the op, cuda_free the block (returns the
- * sticky status of mx_last_error). */
+/* What a dispatch layer does around an op, in two calls: select `device` and provide a metadata block of `count` words, readable by
+ * the host and the device (returns the first failing call's code, 0 = ok); after the op, give the block back (returns the
+ * sticky status of mx_last_error).  The block is for the op calls in between: small ones are pinned host memory, which the launcher
+ * reads in place and which is used again once it is given back, so device work of the caller's own that reads it must have finished
+ * by then; longer ones are cuda_malloc and cuda_memcpy_h2d, as all are after mx_set_small_pool(0). */
 int mx_dispatch_begin(int device, const size_t* host_metadata, size_t count, void** block);
 int mx_dispatch_end(void* block);
 

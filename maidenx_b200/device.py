@@ -88,22 +88,29 @@ def _raise_last_error(op: str, dtype_name: str):
     raise CudaError(f"cuda_{op}_{dtype_name}: {err}")
 
 
+_packers = {}  # words of a metadata block -> packing function
+
+
 def dispatch(op: str, dtype_name: str, metadata, *args, device: int = 0, metadata_on_host: bool = False, check: bool = True):
     """Call cuda_<op>_<dtype> the way maidenx_core does.  `args` is the op's argument list
     with the string "META" standing where the metadata pointer goes."""
     lib = _lib.load()
     if not metadata_on_host and type(metadata) is list and metadata:
         # The usual call.  Host time per call is what small workloads are made of (the README example is 17 such calls):
-        # packing with struct and two native calls around the op take 7.4 us
-        # where numpy's conversion and six native calls took 10.8.
+        # packing with struct and two native calls around the op, whose metadata block is read where it is written.
+        pack = _packers.get(len(metadata))
+        if pack is None:
+            pack = _packers[len(metadata)] = struct.Struct(f"{len(metadata)}Q").pack
         try:
-            words = struct.pack(f"{len(metadata)}Q", *metadata)
+            words = pack(*metadata)
         except struct.error:
             words = None  # not whole 64-bit numbers: numpy's conversion below decides
         if words is not None:
             fn = _lib.op(op, dtype_name)
             block = ctypes.c_void_p()
-            _check(lib.mx_dispatch_begin(device, words, len(metadata), ctypes.byref(block)), "metadata upload")
+            status = lib.mx_dispatch_begin(device, words, len(metadata), ctypes.byref(block))
+            if status:
+                _check(status, "metadata upload")
             try:
                 fn(*[block if type(a) is str and a == "META" else a for a in args])
             finally:

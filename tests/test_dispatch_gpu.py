@@ -1,0 +1,70 @@
+"""The metadata blocks of mx_dispatch_begin / mx_dispatch_end: slots the launcher reads where they lie, and device blocks for what does not fit."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _begin(lib, words):
+    block = ctypes.c_void_p()
+    raw = np.asarray(words, dtype=np.uint64).tobytes()
+    assert lib.mx_dispatch_begin(0, raw, len(words), ctypes.byref(block)) == 0 and block.value
+    return block
+
+
+def test_blocks_open_at_once_read_back_and_given_back(cuda):
+    from maidenx_b200 import _lib, device
+    lib = _lib.load()
+    neg = _lib.op("neg", "f32")
+    x = np.arange(1, 401, dtype=np.float32)
+    src, dst = device.CudaBuffer.from_host(x), device.CudaBuffer(4 * 400)
+    try:
+        blocks = [_begin(lib, [n + 1, 1, 0]) for n in range(300)]        # more than there are slots
+        assert len({b.value for b in blocks}) == 300
+        for n, b in enumerate(blocks):
+            back = np.zeros(3, dtype=np.uint64)
+            assert lib.cuda_memcpy_d2h(back.ctypes.data, b, 24) == 0 and list(back) == [n + 1, 1, 0]
+            dst.fill_from(np.zeros(400, np.float32))
+            neg(n + 1, 1, b, src.ptr, dst.ptr)
+            got = dst.to_host(np.float32, 400)
+            assert np.array_equal(got[:n + 1], -x[:n + 1]) and not got[n + 1:].any()
+        assert lib.cuda_free(blocks.pop()) == 0                          # the call that mx_dispatch_end makes
+        assert all(lib.mx_dispatch_end(b) == 0 for b in blocks)
+        b = _begin(lib, [2, 3, 100, 1, 0])                               # dims [2, 3]
+        new = np.array([3, 2, 1, 3, 0], dtype=np.uint64)                 # the transposed view, written over it
+        assert lib.cuda_memcpy_h2d(b, new.ctypes.data, 40) == 0
+        neg(6, 2, b, src.ptr, dst.ptr)
+        assert np.array_equal(dst.to_host(np.float32, 6), -x[:6].reshape(2, 3).T.reshape(-1)) and lib.mx_dispatch_end(b) == 0
+        long = _begin(lib, [1] * 300 + [4] + [1] * 300 + [1, 0])         # beyond a slot: a device block, refused for its rank
+        neg(4, 301, long, src.ptr, dst.ptr)
+        assert lib.mx_dispatch_end(long) == 2
+        lib.mx_clear_error()
+        short = _begin(lib, [4])                                         # fewer words than the op reads
+        neg(4, 1, short, src.ptr, dst.ptr)
+        assert lib.mx_dispatch_end(short) == 2
+    finally:
+        lib.mx_clear_error()
+        src.free()
+        dst.free()
+
+
+def test_threads_share_the_slots(cuda):
+    from maidenx_b200 import device
+    bad = []
+
+    def work(seed):
+        n = 100 + seed
+        x = np.arange(n, dtype=np.float32) + seed
+        a, o = device.CudaBuffer.from_host(x), device.CudaBuffer(4 * n)
+        for _ in range(300):
+            device.dispatch("neg", "f32", [n, 1, 0], n, 1, "META", a.ptr, o.ptr)
+        if not np.array_equal(o.to_host(np.float32, n), -x):
+            bad.append(seed)
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not bad
