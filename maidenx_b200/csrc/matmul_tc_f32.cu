@@ -36,12 +36,10 @@
 // Every mbarrier wait is bounded (see tc_ptx.cuh); on expiry all roles fall through to the common exit.
 #include <cuda.h>
 
-#include <algorithm>
-#include <atomic>
 #include <mutex>
 
 #include "matmul_tc.cuh"
-#include "tc_pair.cuh"
+#include "tc_ptx.cuh"
 
 namespace mx {
 
@@ -78,12 +76,7 @@ struct Smem {
 constexpr int SMEM_BYTES = Smem::total + 1024;  // slack for the 1024-byte alignment
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 
-// What TMA delivers per stage to a CTA, and the stages of the ring: raw and small tiles share the bytes of STAGES 128-column stages.
-__host__ __device__ constexpr int raw_stage_bytes(int bn, bool pair) { return A_TILE + (pair ? bn / 2 : bn) * BK * 4; }
-__host__ __device__ constexpr int ring_stages(int bn, bool pair) { return STAGES * STAGE_BYTES / (2 * raw_stage_bytes(bn, pair)); }
-static_assert(ring_stages(BN, true) == MAX_STAGES && ring_stages(64, false) == MAX_STAGES, "barrier slots");
-
-__host__ __device__ constexpr uint32_t make_idesc_tf32(bool a_mn_major, bool b_mn_major, int bn, int bm) {
+__host__ __device__ constexpr uint32_t make_idesc_tf32(bool a_mn_major, bool b_mn_major, int bn) {
     uint32_t d = 0;
     d |= 1u << 4;                               // D format: f32
     d |= 2u << 7;                               // A format: tf32
@@ -91,12 +84,12 @@ __host__ __device__ constexpr uint32_t make_idesc_tf32(bool a_mn_major, bool b_m
     d |= (a_mn_major ? 1u : 0u) << 15;
     d |= (b_mn_major ? 1u : 0u) << 16;
     d |= (uint32_t)(bn >> 3) << 17;
-    d |= (uint32_t)(bm >> 4) << 24;
+    d |= (uint32_t)(BM >> 4) << 24;
     return d;
 }
 
 struct Params {
-    int tiles_m, tiles_n, num_tiles, num_kb;  // PAIR: tiles_m counts pairs of row tiles
+    int tiles_m, tiles_n, num_tiles, num_kb;
     int tiles_per_batch;       // tiles_m * tiles_n; num_tiles = batch * tiles_per_batch
     int a_batched, b_batched;  // 0: the operand is one matrix shared by every batch (third TMA coordinate stays 0)
     int a_mn, b_mn;
@@ -104,7 +97,7 @@ struct Params {
     int chunk_kb;   // k-blocks summed inside TMEM before the registers take over
     int bn;         // columns of an output tile: 64 or 128
     int stages;     // of the ring
-    int raw_bytes;  // what TMA delivers per stage and CTA: A and bn rows of B (PAIR: half of them)
+    int raw_bytes;  // what TMA delivers per stage: A and bn rows of B
     int split_kb;   // > 0: split-K; batch s of the launch reduces the k-blocks [s * split_kb, (s + 1) * split_kb) of one product
     int kb_per_z;   // > 0: the reduction runs over the operands' batches too: k-block i is block i % kb_per_z of batch i / kb_per_z
     int d_plain;    // != 0: the output's rows (or base) are not 16-byte multiples: the epilogue warps write them to `out` themselves
@@ -200,13 +193,7 @@ __device__ __forceinline__ void redo_tile(const Params& p, int bn, int tm, int t
 // BN_T = 128: the form of 128-column tiles, long chunks and tensor stores, all known to the compiler; 0: everything from the
 // parameters.  The difference is the splitter's: with the distance between a raw and its small tile a constant, its loads run
 // ahead of its stores (8192 x 4096 x 4096: 164 TFLOP/s, 148 in batches of four).
-//
-// PAIR: two CTAs of a cluster compute a 256 x 128 tile with cta_group::2 instructions (M256): each stages and splits its own 128 rows of A and
-// HALF of the B tile, and the pair's tensor cores read both halves.  Per k-block of 128 x 128 x 32 a CTA then writes 24 KB (TMA), reads and
-// writes 24 KB (splitter) and reads 72 KB (three products) of shared memory instead of 32, 32 and 96, which is what bounds
-// the kernel, and the ring is four stages deep instead of three.  The sums and their order are the same, bit for bit.  Signals: a CTA's loads and splitter use its own barriers;
-// the splitters of both arrive on the leader's (rank 0) split barrier, whose thread issues the pair's instructions, and its commits go to both CTAs.
-template <int BN_T, bool PAIR>
+template <int BN_T>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                    Params p, int* err, int tag) {
@@ -224,58 +211,28 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int chunk_kb = BN_T ? CHUNK_FAST : p.chunk_kb;
-    const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? ring_stages(BN_T, PAIR) : p.stages, raw_bytes = BN_T ? raw_stage_bytes(BN_T, PAIR) : p.raw_bytes;
-    const int bn_own = PAIR ? bn / 2 : bn;  // columns of the B tile that this CTA stages
-    const int rank = PAIR ? (int)cluster_ctarank() : 0, first_tile = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, tile_step = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
-    // this CTA's 128-row tile
-    auto place = [&](int tile, int& tm, int& tn, int& tb) {
-        tile_coords(tile, p, tm, tn, tb);
-        if (PAIR) tm = 2 * tm + rank;
-    };
-    auto arrive_at_leader = [&](uint32_t bar) {
-        if constexpr (PAIR) mbar_arrive_cluster(map_to_cta(bar, 0));
-        else mbar_arrive(bar);
-    };
-    auto commit = [&](uint32_t bar) {
-        if constexpr (PAIR) {
-            umma2_commit(bar);
-            umma2_commit(map_to_cta(bar, 1));
-        } else {
-            umma_commit(bar);
-        }
-    };
-    auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-        if constexpr (PAIR) umma2_tf32(d, a, b, idesc, accumulate);
-        else umma_tf32(d, a, b, idesc, accumulate);
-    };
+    const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? STAGES : p.stages, raw_bytes = BN_T ? A_TILE + BN_T * BK * 4 : p.raw_bytes;
 
     auto redo = [&] { return reinterpret_cast<uint32_t*>(smem + Smem::redo); };
     if (threadIdx.x <= REDO_BITS / 32) redo()[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < MAX_STAGES; s++) {
             mbar_init(full_bar(s), 1);
-            mbar_init(split_bar(s), (PAIR ? 2 : 1) * SPLIT_WARPS);
+            mbar_init(split_bar(s), SPLIT_WARPS);
             mbar_init(empty_bar(s), 1);
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(tfull_bar(a), 1);
-            mbar_init(tempty_bar(a), (PAIR ? 2 : 1) * EPI_WARPS);
+            mbar_init(tempty_bar(a), EPI_WARPS);
         }
         fence_barrier_init();
     }
     if (warp == 1) {
-        const uint32_t slot = smem_u32(const_cast<uint32_t*>(tmem_base_slot));
-        if constexpr (PAIR) {
-            tmem_alloc2(slot, TMEM_COLS);
-            tmem_relinquish2();
-        } else {
-            tmem_alloc(slot, TMEM_COLS);
-            tmem_relinquish();
-        }
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_base_slot)), TMEM_COLS);
+        tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
-    if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers exist before anything arrives on them from the other
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
 
@@ -285,9 +242,9 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int tile = first_tile; tile < p.num_tiles && ok; tile += tile_step) {
+            for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
                 int tm, tn, tb;
-                place(tile, tm, tn, tb);
+                tile_coords(tile, p, tm, tn, tb);
                 int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
                 for (int kb = 0; kb < p.num_kb; kb++) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, err, tag, 1)) {
@@ -310,9 +267,9 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         for (int h = 0; h < BM / 32; h++) tma_load_3d(sa + h * MN_CHUNK_BYTES, &map_a, tm * BM + h * 32, k, za, full_bar(stage));
                     }
                     if (!p.b_mn) {
-                        tma_load_3d(sb, &map_b, k, tn * bn + rank * bn_own, zb, full_bar(stage));
+                        tma_load_3d(sb, &map_b, k, tn * bn, zb, full_bar(stage));
                     } else {
-                        for (int h = 0; h < bn_own / 32; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * bn + rank * bn_own + h * 32, k, zb, full_bar(stage));
+                        for (int h = 0; h < bn / 32; h++) tma_load_3d(sb + h * MN_CHUNK_BYTES, &map_b, tn * bn + h * 32, k, zb, full_bar(stage));
                     }
                     if (++stage == stages) {
                         stage = 0;
@@ -322,17 +279,17 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer (PAIR: the leader's)
-        if (lane == 0 && rank == 0) {
-            const uint32_t idesc = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, bn, PAIR ? 2 * BM : BM);
+        // ------------------------------------------------------------ MMA issuer
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, bn);
             // K-major: 8 floats further along the 128-byte row; MN-major: the next group of eight K-rows
             const uint64_t a_kstep = p.a_mn ? (1024 >> 4) : (32 >> 4), b_kstep = p.b_mn ? (1024 >> 4) : (32 >> 4);
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
-            for (int tile = first_tile; tile < p.num_tiles && ok; tile += tile_step) {
+            for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
                 for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += chunk_kb) {
-                    if (!(PAIR ? mbar_wait_cluster(tempty_bar(acc), acc_phase ^ 1, err, tag, 2) : mbar_wait(tempty_bar(acc), acc_phase ^ 1, err, tag, 2))) {
+                    if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1, err, tag, 2)) {
                         ok = false;
                         break;
                     }
@@ -341,9 +298,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     const int kb1 = min(kb0 + chunk_kb, p.num_kb);
                     for (int kb = kb0; kb < kb1; kb++) {
                         // the raw tiles (TMA) and the small tiles (splitter) are both operands
-                        // PAIR: every splitter warp of both CTAs has seen its own loads land before it arrives
-                        if (PAIR ? !mbar_wait_cluster(split_bar(stage), phase, err, tag, 6)
-                                 : !mbar_wait(full_bar(stage), phase, err, tag, 3) || !mbar_wait(split_bar(stage), phase, err, tag, 6)) {
+                        if (!mbar_wait(full_bar(stage), phase, err, tag, 3) || !mbar_wait(split_bar(stage), phase, err, tag, 6)) {
                             ok = false;
                             break;
                         }
@@ -360,27 +315,27 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         if (chunk_kb == 1) {
 #pragma unroll
                             for (int k = 0; k < BK / UMMA_K; k++) {
-                                mma(d_tmem, a_small + a_kstep * k, b_big + b_kstep * k, idesc, k != 0);
-                                mma(d_tmem, a_big + a_kstep * k, b_small + b_kstep * k, idesc, 1);
+                                umma_tf32(d_tmem, a_small + a_kstep * k, b_big + b_kstep * k, idesc, k != 0);
+                                umma_tf32(d_tmem, a_big + a_kstep * k, b_small + b_kstep * k, idesc, 1);
                             }
 #pragma unroll
-                            for (int k = 0; k < BK / UMMA_K; k++) mma(d_tmem, a_big + a_kstep * k, b_big + b_kstep * k, idesc, 1);
+                            for (int k = 0; k < BK / UMMA_K; k++) umma_tf32(d_tmem, a_big + a_kstep * k, b_big + b_kstep * k, idesc, 1);
                         } else {
 #pragma unroll
                             for (int k = 0; k < BK / UMMA_K; k++) {
-                                mma(d_tmem, a_small + a_kstep * k, b_big + b_kstep * k, idesc, (kb != kb0) || (k != 0));
-                                mma(d_tmem, a_big + a_kstep * k, b_small + b_kstep * k, idesc, 1);
-                                mma(d_tmem, a_big + a_kstep * k, b_big + b_kstep * k, idesc, 1);
+                                umma_tf32(d_tmem, a_small + a_kstep * k, b_big + b_kstep * k, idesc, (kb != kb0) || (k != 0));
+                                umma_tf32(d_tmem, a_big + a_kstep * k, b_small + b_kstep * k, idesc, 1);
+                                umma_tf32(d_tmem, a_big + a_kstep * k, b_big + b_kstep * k, idesc, 1);
                             }
                         }
-                        commit(empty_bar(stage));
+                        umma_commit(empty_bar(stage));
                         if (++stage == stages) {
                             stage = 0;
                             phase ^= 1;
                         }
                     }
                     if (!ok) break;
-                    commit(tfull_bar(acc));  // this chunk's partial sums are complete
+                    umma_commit(tfull_bar(acc));  // this chunk's partial sums are complete
                     if (++acc == 2) {
                         acc = 0;
                         acc_phase ^= 1;
@@ -396,9 +351,9 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         int acc = 0, buf = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
-        for (int tile = first_tile; tile < p.num_tiles && ok; tile += tile_step) {
+        for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
             int tm, tn, tb;
-            place(tile, tm, tn, tb);
+            tile_coords(tile, p, tm, tn, tb);
             float total[BN];  // this thread's row of the tile (registers: every index below is a compile-time constant)
 #pragma unroll
             for (int j = 0; j < BN; j++) total[j] = 0.0f;
@@ -423,7 +378,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 // every TMEM read of this accumulator is done: hand it back to the MMA warp
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) arrive_at_leader(tempty_bar(acc));
+                if (lane == 0) mbar_arrive(tempty_bar(acc));
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;
@@ -470,7 +425,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 buf ^= 1;
             }
             if (__any_sync(0xFFFFFFFFu, zero != 0.0f) && lane == 0) {
-                const int it = (tile - first_tile) / tile_step;
+                const int it = (tile - (int)blockIdx.x) / (int)gridDim.x;
                 atomicOr(&redo()[it % REDO_BITS / 32], 1u << it % 32);
                 redo()[REDO_BITS / 32] = 1;
             }
@@ -482,7 +437,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        for (int tile = first_tile; tile < p.num_tiles && ok; tile += tile_step) {
+        for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
             for (int kb = 0; kb < p.num_kb; kb++) {
                 const bool landed = mbar_wait_relaxed(full_bar(stage), phase, err, tag, 5, 40);
                 if (!__all_sync(0xFFFFFFFFu, landed)) {
@@ -492,7 +447,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 const uint4* raw = reinterpret_cast<const uint4*>(smem + Smem::stages + stage * 2 * raw_bytes);
                 uint4* small = reinterpret_cast<uint4*>(smem + Smem::stages + stage * 2 * raw_bytes + raw_bytes);
                 if constexpr (BN_T != 0) {
-                    constexpr int STEPS = raw_stage_bytes(BN_T, PAIR) / 16 / (32 * SPLIT_WARPS);
+                    constexpr int STEPS = (A_TILE + BN_T * BK * 4) / 16 / (32 * SPLIT_WARPS);
 #pragma unroll 8
                     for (int i = 0; i < STEPS; i++) {
                         const uint4 q = raw[t + i * 32 * SPLIT_WARPS];
@@ -511,7 +466,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 }
                 fence_proxy_async_smem();  // the tensor core reads these through the async proxy
                 __syncwarp();
-                if (lane == 0) arrive_at_leader(split_bar(stage));
+                if (lane == 0) mbar_arrive(split_bar(stage));
                 if (++stage == stages) {
                     stage = 0;
                     phase ^= 1;
@@ -529,21 +484,19 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
         __syncthreads();
     }
-    if constexpr (PAIR) cluster_sync_all();  // neither CTA leaves, reuses its ring or frees tensor memory before both are done
     if (warp == 1) {
         __syncwarp();
         tc_fence_after();
-        if constexpr (PAIR) tmem_dealloc2(tmem_base, TMEM_COLS);
-        else tmem_dealloc(tmem_base, TMEM_COLS);
+        tmem_dealloc(tmem_base, TMEM_COLS);
     }
 
     // the tile stores have completed (tma_store_wait_all before the barrier above): their places may be written again
     if (!redo()[REDO_BITS / 32]) return;
     fence_proxy_async();
-    for (int tile = first_tile, it = 0; tile < p.num_tiles; tile += tile_step, it++) {
+    for (int tile = blockIdx.x, it = 0; tile < p.num_tiles; tile += gridDim.x, it++) {
         if (!(redo()[it % REDO_BITS / 32] >> it % 32 & 1)) continue;
         int tm, tn, tb;
-        place(tile, tm, tn, tb);
+        tile_coords(tile, p, tm, tn, tb);
         redo_tile(p, bn, tm, tn, tb, reinterpret_cast<float*>(smem + Smem::stages));
     }
 }
@@ -555,7 +508,7 @@ bool opt_in_shared_memory() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
-        for (auto kernel : {tc_gemm_f32_kernel<BN, false>, tc_gemm_f32_kernel<0, false>, tc_gemm_f32_kernel<BN, true>, tc_gemm_f32_kernel<0, true>})
+        for (auto kernel : {tc_gemm_f32_kernel<BN>, tc_gemm_f32_kernel<0>})
             if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
@@ -583,41 +536,6 @@ int tile_columns(uint64_t tiles_m, uint64_t N, uint64_t batch, int grid) {
 }
 // what the second launch of a split-K product costs, in k-blocks (about 0.9 us each on one CTA)
 constexpr double kSplitFixed32 = 3.0;
-// a k-block of a 256 x 128 tile of two CTAs, in the same unit (see PAIR at the kernel)
-constexpr double kPairKb = 0.75;
-std::atomic<int> g_pair{-1};  // 0 / 1: never / wherever there are two row tiles (tests, A/B timing); -1: by plan()
-
-struct Plan {
-    bool pair;
-    int bn, slices;  // slices > 1: K cut into that many runs of k-blocks, each a batch of the launch, summed by a second one
-    double cost;
-};
-Plan plan_form(bool pair, uint64_t tiles_m, uint64_t N, uint64_t K, uint64_t num_kb, uint64_t batch, bool sum_batches, int grid) {
-    Plan f;
-    f.pair = pair;
-    const uint64_t rows = pair ? (tiles_m + 1) / 2 : tiles_m;
-    const int units = pair ? grid / 2 : grid, bn_split = !pair && N <= 64 ? 64 : BN, bn_whole = pair ? BN : tile_columns(rows, N, batch, grid);
-    const double kb = pair ? kPairKb : (128 + bn_split) / 256.0;
-    const double whole = (pair ? kPairKb * (double)((rows * ((N + BN - 1) / BN) * batch + units - 1) / units) : tile_cost(bn_whole, rows, N, batch, grid)) * (double)num_kb;
-    f.slices = 1;
-    if (batch == 1) {
-        const uint64_t tiles = rows * ((N + bn_split - 1) / bn_split);
-        if (!sum_batches) f.slices = splitk_slices(tiles, K, BK, units);
-        if (f.slices == 1) f.slices = splitk_short(tiles, num_kb, units, kb, whole - kSplitFixed32);
-        if (f.slices > 1) f.cost = (double)((tiles * f.slices + units - 1) / units * ((num_kb + f.slices - 1) / f.slices)) * kb + kSplitFixed32 + 0.1 * f.slices;
-    }
-    f.bn = f.slices > 1 ? bn_split : bn_whole;
-    if (f.slices == 1) f.cost = whole;
-    return f;
-}
-// Pairs of CTAs where their estimate is lower: two row tiles and more, unless a pair's larger tile leaves too many SMs without one.
-Plan plan(uint64_t tiles_m, uint64_t N, uint64_t K, uint64_t num_kb, uint64_t batch, bool sum_batches, int grid) {
-    const Plan one = plan_form(false, tiles_m, N, K, num_kb, batch, sum_batches, grid);
-    const int force = g_pair.load(std::memory_order_relaxed);
-    if (force == 0 || tiles_m < 2 || grid < 2) return one;
-    const Plan two = plan_form(true, tiles_m, N, K, num_kb, batch, sum_batches, grid);
-    return force == 1 || two.cost < 0.97 * one.cost ? two : one;
-}
 
 // D[M,N] = sum_k Aop[m,k] * Bop[n,k]; K-major operand = row-major [MN, K], MN-major = row-major [K, MN].
 bool launch(const TcProduct& c, void* D, const char* where) {
@@ -629,6 +547,9 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.M = (int)M;
     p.N = (int)N;
     p.chunk_kb = c.ragged ? 1 : CHUNK_FAST;
+    p.bn = N <= 64 ? 64 : BN;
+    p.tiles_m = (int)((M + BM - 1) / BM);
+    p.tiles_n = (int)((N + p.bn - 1) / p.bn);
     p.num_kb = (int)((K + BK - 1) / BK);
     p.split_kb = 0;
     p.kb_per_z = 0;
@@ -639,33 +560,36 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     }
     int grid = sm_count();
     if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
-    const uint64_t row_tiles = (M + BM - 1) / BM;
-    const Plan f = plan(row_tiles, N, K, (uint64_t)p.num_kb, batch, c.sum_batches, grid);
-    int slices = f.slices;
+    // few output tiles: cut K into slices that run as the batches of this launch (see tc_ptx.cuh)
+    int slices = 1;
+    const int bn_whole = tile_columns((uint64_t)p.tiles_m, N, batch, grid);
+    if (batch == 1) {
+        if (!c.sum_batches) slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
+        if (slices == 1)
+            slices = splitk_short((uint64_t)p.tiles_m * p.tiles_n, (uint64_t)p.num_kb, grid, (128 + p.bn) / 256.0,
+                                  tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, grid) * p.num_kb - kSplitFixed32);
+    }
     StreamWorkspace partial;
     const uint64_t n_pitch = (N + 3) / 4 * 4;
-    p.bn = f.bn;
-    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) {
-        slices = 1;
-        if (!f.pair) p.bn = tile_columns(row_tiles, N, batch, grid);
-    }
+    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) slices = 1;
     if (slices > 1) {
         p.split_kb = (p.num_kb + slices - 1) / slices;
         p.num_kb = p.split_kb;
         batch = (uint64_t)slices;
+    } else {
+        p.bn = bn_whole;
+        p.tiles_n = (int)((N + p.bn - 1) / p.bn);
     }
-    p.tiles_m = (int)(f.pair ? (row_tiles + 1) / 2 : row_tiles);
-    p.tiles_n = (int)((N + p.bn - 1) / p.bn);
     p.tiles_per_batch = p.tiles_m * p.tiles_n;
-    p.raw_bytes = raw_stage_bytes(p.bn, f.pair);
-    p.stages = ring_stages(p.bn, f.pair);
+    p.raw_bytes = A_TILE + p.bn * BK * 4;
+    p.stages = STAGES * STAGE_BYTES / (2 * p.raw_bytes);
     int tag = 0;
     int* err = next_launch_error_word(&tag);
     if (!err) return false;
     CUtensorMap ma, mb, md;
     const uint64_t a_bs = (uint64_t)c.a_bs, b_bs = (uint64_t)c.b_bs;
     const bool oka = a_mn ? make_map(&ma, c.A, K, M, c.batch, a_bs, BK, true, c.a_pitch) : make_map(&ma, c.A, M, K, c.batch, a_bs, BM, false, c.a_pitch);
-    const bool okb = b_mn ? make_map(&mb, c.B, K, N, c.batch, b_bs, BK, true, c.b_pitch) : make_map(&mb, c.B, N, K, c.batch, b_bs, (uint32_t)(f.pair ? p.bn / 2 : p.bn), false, c.b_pitch);
+    const bool okb = b_mn ? make_map(&mb, c.B, K, N, c.batch, b_bs, BK, true, c.b_pitch) : make_map(&mb, c.B, N, K, c.batch, b_bs, (uint32_t)p.bn, false, c.b_pitch);
     if (!oka || !okb) return false;
     p.d_plain = slices > 1 ? 0 : c.d_plain;
     if (p.d_plain) md = ma;  // not used
@@ -688,24 +612,9 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.zs = (int)c.batch;
     p.out = static_cast<float*>(slices > 1 ? partial.ptr : D);
     p.out_ld = (int64_t)(slices > 1 ? n_pitch : N);
-    const bool fixed = p.bn == BN && !p.d_plain && p.chunk_kb == CHUNK_FAST;
-    if (f.pair) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * (unsigned)std::min(grid / 2, p.num_tiles));
-        cfg.blockDim = dim3(THREADS);
-        cfg.dynamicSmemBytes = SMEM_BYTES;
-        cfg.stream = ctx().stream;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;
-        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, fixed ? tc_gemm_f32_kernel<BN, true> : tc_gemm_f32_kernel<0, true>, ma, mb, md, p, err, tag);
-    } else {
-        const auto kernel = fixed ? tc_gemm_f32_kernel<BN, false> : tc_gemm_f32_kernel<0, false>;
-        kernel<<<std::min(grid, p.num_tiles), THREADS, SMEM_BYTES, ctx().stream>>>(ma, mb, md, p, err, tag);
-    }
+    if (grid > p.num_tiles) grid = p.num_tiles;
+    const auto kernel = p.bn == BN && !p.d_plain && p.chunk_kb == CHUNK_FAST ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>;
+    kernel<<<grid, THREADS, SMEM_BYTES, ctx().stream>>>(ma, mb, md, p, err, tag);
     check_launch(where);
     if (slices > 1) splitk_reduce(2, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
     return true;
@@ -723,6 +632,3 @@ bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t 
 }
 
 }  // namespace mx
-
-// -1 (default): f32 products run on one CTA or on pairs of CTAs by an estimate; 0 / 1: never / always on pairs where there are two row tiles
-extern "C" void mx_debug_set_gemm_f32_pair(int form) { mx::g_pair.store(form, std::memory_order_relaxed); }

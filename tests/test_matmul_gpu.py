@@ -421,45 +421,6 @@ def test_ragged_output_rows_are_written_whole_and_alone(cuda, n, off):
         assert np.array_equal(got, want)
 
 
-@pytest.mark.parametrize("case", [
-    # M, N, K, majors: row tiles odd and even, the last one of one row and of all, N below and above a tile, one k-block and a short last one
-    (129, 128, 512, "kk"), (256, 300, 452, "kk"), (385, 132, 260, "mk"), (512, 64, 324, "km"), (1000, 388, 32, "mm"), (264, 516, 1156, "mm"),
-    (257, 515, 193, "kk"), (391, 133, 227, "mm"), (640, 129, 200, "km"), (300, 7, 5001, "kk")], ids=lambda c: "x".join(map(str, c)))
-def test_f32_pairs_of_ctas_give_the_bits_of_one(cuda, case):
-    """A 256-row tile of two CTAs adds in the order of two 128-row tiles.  Three batches, so that K is not cut into runs; dense and ragged
-    rows, every operand order, an infinity in one row (its tile is computed again), and nothing written around the output."""
-    from maidenx_b200 import _lib, device
-    lib = _lib.load()
-    m, n, k, majors = case
-    nb = 3
-    rng = np.random.default_rng(m * n + k)
-    a, b = (rng.standard_normal((nb, *x)).astype(np.float32) for x in ((m, k), (k, n)))
-    a[1, m - 1, k // 2] = np.inf
-    ast, bst = [m * k, k, 1] if majors[0] == "k" else [m * k, 1, m], [k * n, 1, k] if majors[1] == "k" else [k * n, n, 1]
-    am, bm = a if majors[0] == "k" else np.swapaxes(a, 1, 2), np.swapaxes(b, 1, 2) if majors[1] == "k" else b
-    guard = 4
-    fill = np.full(nb * m * n + 2 * guard, 7.25, dtype=np.float32)
-    meta = [3, 3, 3, nb, m, n, nb, m, k, nb, k, n, *ast, *bst, 0, 0]
-    got = {}
-    try:
-        for form in (0, 1):
-            lib.mx_debug_set_gemm_f32_pair(form)
-            bufs = [device.CudaBuffer.from_host(np.ascontiguousarray(x).reshape(-1)) for x in (am, bm, fill)]
-            device.dispatch("matmul", "f32", meta, nb * m * n, "META", bufs[0].ptr, bufs[1].ptr, bufs[2].ptr + 4 * guard)
-            got[form] = bufs[2].to_host(np.float32, fill.size)
-    finally:
-        lib.mx_debug_set_gemm_f32_pair(-1)
-    assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
-    out = got[1][guard:-guard].reshape(nb, m, n)
-    assert (got[1][:guard] == 7.25).all() and (got[1][-guard:] == 7.25).all()
-    with np.errstate(invalid="ignore"):
-        ref = np.matmul(a.astype(np.float64), b.astype(np.float64))
-    bad = np.zeros((nb, m, n), dtype=bool)
-    bad[1, m - 1] = True
-    assert np.array_equal(np.sign(out[bad]), np.sign(ref[bad])) and np.isinf(out[bad]).all()
-    assert np.linalg.norm(out[~bad] - ref[~bad]) <= 2e-6 * np.linalg.norm(ref[~bad])
-
-
 @pytest.mark.parametrize("dt", [D.BF16, D.F16, D.F32], ids=lambda d: d.name)
 @pytest.mark.parametrize("case", [("batched", [4], 152, 136, 216), ("batched-odd", [4], 151, 133, 219), ("rank-4", [2, 2], 152, 136, 216), ("odd", [], 301, 259, 227),
                                   ("broadcast-b", None, 150, 136, 216)], ids=lambda c: c[0])
