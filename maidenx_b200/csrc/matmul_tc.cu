@@ -2,7 +2,7 @@
 // tensor memory (TMEM), operands staged in shared memory by TMA, epilogue read back with
 // tcgen05.ld, converted and written with TMA stores.
 //
-// One persistent CTA per SM, 320 threads in three roles:
+// One persistent CTA per SM, 192 threads (320 where the warps write the rows themselves) in three roles:
 //   warp 0      TMA producer: one lane issues cp.async.bulk.tensor loads of the A [128 x 64]
 //               and B [64 to 256 x 64] k-blocks into a shared-memory ring (128-byte swizzle) of four
 //               stages, up to eight of narrower tiles;
@@ -10,8 +10,8 @@
 //               k-block into one of two 256-column TMEM accumulators, commits the stage back to the
 //               producer and, after the last k-block (or a run of them, see DRAIN), the accumulator
 //               to the epilogue;
-//   warps 2-9   epilogue: two warps own the 32 TMEM lanes that both may address (warp id mod 4),
-//               read them 64 columns at a time, each 32, round to bf16 / f16, write a swizzled
+//   the others  epilogue: one or two warps own the 32 TMEM lanes that they may address (warp id mod 4),
+//               read them 64 columns at a time, round to bf16 / f16, write a swizzled
 //               4 KB staging tile and store it with TMA (rows that no tensor map can describe:
 //               themselves) while the next tile's MMAs run on the other accumulator.
 // No cluster launch: every CTA issues its own (CTA-local) TMA loads; re-use comes from
@@ -54,10 +54,8 @@ constexpr int STAGES = 4;                     // ring stages of full-width tiles
 constexpr int MAX_STAGES = 8;
 constexpr int A_STAGE_BYTES = BM * BK * 2;    // 16 KB
 constexpr int B_STAGE_BYTES = BN * BK * 2;    // 32 KB
-constexpr int EPI_WARPS = 8;                  // two for each quarter of the accumulator's lanes
 constexpr int EPI_CHUNK_COLS = 64;            // columns per TMA store (128 bytes of 16-bit)
 constexpr int EPI_STAGE_BYTES = 32 * EPI_CHUNK_COLS * 2;  // 4 KB: 32 rows of a chunk; two such buffers per quarter
-constexpr int TC_THREADS = 32 * (2 + EPI_WARPS);
 constexpr int TMEM_COLS = 512;                // two 256-column f32 accumulators
 constexpr int GROUP_M = 16;                   // row-tiles per column sweep (L2 re-use)
 
@@ -118,9 +116,6 @@ struct TcParams {
     // tiles j, j + b_keep, ...; the B panel of the column tile is loaded once into the B slots of the ring (slot = k-block,
     // the ring is num_kb slots long) and only A streams.  0: the general schedule.
     int b_keep;
-    // Short reductions of a batch: the tiles in the order batch, column tile, row tile, an equal run of them for each CTA, which loads a B panel
-    // once for all row tiles of it.
-    int panels;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, const TcParams& p, int& tm, int& tn, int& tb) {
@@ -136,15 +131,11 @@ __device__ __forceinline__ void tile_coords(int tile, const TcParams& p, int& tm
     tn = in_group / rows;
 }
 
-// The it-th tile of this CTA; false when it has none left.
+// The it-th tile of this CTA; false when it has none left.  PANELS (short reductions of a batch): the tiles in the order batch, column tile, row
+// tile, an equal run of them for each CTA, which loads a B panel once for all row tiles of it.
+template <bool PANELS>
 __device__ __forceinline__ bool next_tile(int it, const TcParams& p, int& tm, int& tn, int& tb) {
-    if (p.b_keep) {
-        tn = (int)blockIdx.x / p.b_keep;
-        tm = (int)blockIdx.x % p.b_keep + it * p.b_keep;
-        tb = 0;
-        return tn < p.tiles_n && tm < p.tiles_m;
-    }
-    if (p.panels) {
+    if constexpr (PANELS) {
         const int tile = (int)((long long)blockIdx.x * p.num_tiles / gridDim.x) + it;
         if (tile >= (int)((long long)(blockIdx.x + 1) * p.num_tiles / gridDim.x)) return false;
         const int panel = tile / p.tiles_m;
@@ -152,6 +143,12 @@ __device__ __forceinline__ bool next_tile(int it, const TcParams& p, int& tm, in
         tb = panel / p.tiles_n;
         tn = panel - tb * p.tiles_n;
         return true;
+    }
+    if (p.b_keep) {
+        tn = (int)blockIdx.x / p.b_keep;
+        tm = (int)blockIdx.x % p.b_keep + it * p.b_keep;
+        tb = 0;
+        return tn < p.tiles_n && tm < p.tiles_m;
     }
     const int tile = (int)blockIdx.x + it * (int)gridDim.x;
     if (tile >= p.num_tiles) return false;
@@ -235,10 +232,17 @@ enum TcMode {
 // with the geometry from the parameters the products of a 16384 x 8192 layer took 12 % longer at full clock.
 // DRAIN (tiles of at most 128 columns): the accumulator is emptied every run_kb k-blocks into totals in registers, added with
 // round-to-nearest, so that the pull of the tensor core's truncating additions stays that of one run whatever K is (see kRunMostF16).
-template <int MODE, int BN_T, bool DRAIN = false>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+// PANELS: TcParams::panels, an instantiation of its own for the same reason (as a branch of the common schedule it cost 4096^3 19 %).
+//
+// Epilogue warps for each quarter of the accumulator's lanes.  Rows that the warps write themselves take two (4096 x 2050 x 512 bf16: 25 us, 36
+// with one); products that leave through the copy engine gain nothing from a second one (16384 x 4096 x 256: 55 us, 50 with one).
+constexpr int epi_warps(int mode) { return mode == TC_PLAIN ? 2 : 1; }
+constexpr int tc_threads(int mode) { return 32 * (2 + 4 * epi_warps(mode)); }
+template <int MODE, int BN_T, bool DRAIN = false, bool PANELS = false>
+__global__ void __launch_bounds__(tc_threads(MODE), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                const __grid_constant__ CUtensorMap map_d2, TcParams p, int* err, int tag) {
+    constexpr int W = epi_warps(MODE), CW = EPI_CHUNK_COLS / W;  // columns of a chunk that a warp has
     extern __shared__ unsigned char tc_smem_raw[];
     // 128-byte swizzled TMA tiles and UMMA descriptors want 1024-byte aligned bases
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -261,7 +265,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(tfull_bar(a), 1);
-            mbar_init(tempty_bar(a), EPI_WARPS);
+            mbar_init(tempty_bar(a), 4 * W);
         }
         fence_barrier_init();
     }
@@ -280,12 +284,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            const int ring = p.b_keep || p.panels ? p.num_kb : stages;
+            const int ring = PANELS || p.b_keep ? p.num_kb : stages;
             int tm, tn, tb;
-            for (int it = 0; ok && next_tile(it, p, tm, tn, tb); it++) {
+            for (int it = 0; ok && next_tile<PANELS>(it, p, tm, tn, tb); it++) {
                 const int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
                 int k = tb * p.split_kb * BK;              // a k-block past the end of K is all fill: zeros
-                const bool load_b = it == 0 || (p.panels ? tm == 0 : !p.b_keep);  // a kept B panel arrives with its first tile's A blocks
+                const bool load_b = PANELS ? tm == 0 || it == 0 : !p.b_keep || it == 0;  // a kept B panel arrives with its first tile's A blocks
                 for (int kb = 0; kb < p.num_kb; kb++, k += BK) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, err, tag, 1)) {
                         ok = false;
@@ -323,10 +327,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
-            const int ring = p.b_keep || p.panels ? p.num_kb : stages;
+            const int ring = PANELS || p.b_keep ? p.num_kb : stages;
             int tm, tn, tb;
             int run = 0;  // first k-block of the accumulator's run (DRAIN: a tile has several)
-            for (int it = 0; ok && next_tile(it, p, tm, tn, tb); it += DRAIN && run ? 0 : 1) {
+            for (int it = 0; ok && next_tile<PANELS>(it, p, tm, tn, tb); it += DRAIN && run ? 0 : 1) {
                 if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1, err, tag, 2)) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
@@ -357,59 +361,65 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else {
-        // ------------------------------------------------------------ epilogue (warps 2..9)
-        // Two warps share a quarter of the accumulator's lanes: each reads, rounds and stages 32 of a chunk's 64 columns, and the chunk leaves as one
-        // copy.  With one warp a quarter the epilogue of a 256-column tile took about as long as a reduction of 256
-        // (its warps wait for TMEM, shared memory and the copy engine in turn).
+        // ------------------------------------------------------------ epilogue (warps 2 to 5 or 9)
+        // W warps share a quarter of the accumulator's lanes: each reads, rounds and stages its CW columns of a 64-column chunk, which
+        // leaves as one copy.
         const int quarter = warp & 3;  // TMEM lanes [32 * quarter, 32 * quarter + 32)
-        const int half = (warp - 2) >> 2;
+        const int half = W == 2 ? (warp - 2) >> 2 : 0;
         const bool lead = half == 0 && lane == 0;  // the thread that hands a quarter's chunks to the copy engine
         unsigned char* stage_buf = smem + SmemLayout::epi + quarter * 2 * EPI_STAGE_BYTES;
-        auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory"); };
+        auto quarter_sync = [&] {
+            if constexpr (W == 2) asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
+            else __syncwarp();
+        };
         int acc = 0, buf = 0;
         uint32_t acc_phase = 0;
         float fused_bias = 0.0f;
         if (MODE == TC_BIAS && p.fuse != 3) fused_bias = p.is_bf16 ? to_f32(*static_cast<const bf16*>(p.bias)) : to_f32(*static_cast<const f16*>(p.bias));
         int tm, tn, tb;
-        for (int it = 0; next_tile(it, p, tm, tn, tb); it++) {
-            // eight warps wait here for most of a tile's reduction: they sleep between polls, so that their polling does not
+        for (int it = 0; next_tile<PANELS>(it, p, tm, tn, tb); it++) {
+            // four or eight warps wait here for most of a tile's reduction: they sleep between polls, so that their polling does not
             // take shared-memory cycles from the TMA writes and the tensor core's operand reads
             if (MODE != TC_STORE && p.fuse == 3) {  // this thread's output row inside the batch's matrix
                 const int row = tm * BM + quarter * 32 + lane;
                 fused_bias = row < p.M ? (p.is_bf16 ? to_f32(static_cast<const bf16*>(p.bias)[row]) : to_f32(static_cast<const f16*>(p.bias)[row])) : 0.0f;
             }
-            // The TMEM loads below take whole warps and the staging both warps of a quarter: these leave the loop together, by a vote that each
+            // The TMEM loads below take whole warps and the staging all warps of a quarter: these leave the loop together, two by a vote that each
             // of them reaches, its own wait being bounded.
             auto wait_accumulator = [&] {
                 const bool ready = mbar_wait_relaxed(tfull_bar(acc), acc_phase, err, tag, 4, 400);
-                uint32_t both;
-                __syncwarp();
-                asm volatile(
-                    "{\n\t.reg .pred p, q;\n\t"
-                    "setp.ne.u32 p, %2, 0;\n\t"
-                    "barrier.cta.red.and.pred q, %1, 64, p;\n\t"
-                    "selp.u32 %0, 1, 0, q;\n\t}"
-                    : "=r"(both)
-                    : "r"(1 + quarter), "r"((uint32_t)ready)
-                    : "memory");
-                if (!both) return false;
+                if constexpr (W == 2) {
+                    uint32_t both;
+                    __syncwarp();
+                    asm volatile(
+                        "{\n\t.reg .pred p, q;\n\t"
+                        "setp.ne.u32 p, %2, 0;\n\t"
+                        "barrier.cta.red.and.pred q, %1, 64, p;\n\t"
+                        "selp.u32 %0, 1, 0, q;\n\t}"
+                        : "=r"(both)
+                        : "r"(1 + quarter), "r"((uint32_t)ready)
+                        : "memory");
+                    if (!both) return false;
+                } else if (!__all_sync(0xFFFFFFFFu, ready)) {
+                    return false;
+                }
                 tc_fence_after();
                 return true;
             };
             if (!DRAIN && !wait_accumulator()) break;
-            const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * 32);
+            const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * CW);
             const int rows_here = min(32, p.M - (tm * BM + quarter * 32));  // may be <= 0: this warp's rows lie below the matrix
-            // Stages 32 columns of a row: 16-byte pieces, XOR-swizzled by the row; the chunk (first output column `col`) then goes to the copy engine, or the
-            // warps write its rows themselves.
-            auto flush = [&](const CUtensorMap* map, int col, const uint4 (&q)[4]) {
+            // Stages a warp's columns of a chunk (16-byte pieces, XOR-swizzled by the row); the chunk (first output column `col`) then goes to the copy
+            // engine, or the warps write its rows themselves.
+            auto flush = [&](const CUtensorMap* map, int col, const uint4 (&q)[CW / 8]) {
                 if (lead) tma_store_wait_read<1>();  // the buffer's previous chunk has been read
-                __syncwarp();
-                pair_sync();
+                if (W == 2) __syncwarp();
+                quarter_sync();
                 unsigned char* src = stage_buf + buf * EPI_STAGE_BYTES;
 #pragma unroll
-                for (int j = 0; j < 4; j++) *reinterpret_cast<uint4*>(src + lane * 128 + (((half * 4 + j) ^ (lane & 7)) << 4)) = q[j];
+                for (int j = 0; j < CW / 8; j++) *reinterpret_cast<uint4*>(src + lane * 128 + (((half * (CW / 8) + j) ^ (lane & 7)) << 4)) = q[j];
                 if (MODE != TC_PLAIN) fence_proxy_async_smem();
-                pair_sync();
+                quarter_sync();
                 buf ^= 1;
                 if constexpr (MODE != TC_PLAIN) {
                     if (lead) {
@@ -421,50 +431,64 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                min(bn, p.N - tn * bn), (col - tn * bn) / 64, src, stage_buf + buf * EPI_STAGE_BYTES, lane);
                 }
             };
-            auto pack = [&](const float (&e)[32], uint4 (&q)[4]) {
+            auto pack = [&](const float (&e)[CW], uint4 (&q)[CW / 8]) {
 #pragma unroll
-                for (int j = 0; j < 4; j++)
+                for (int j = 0; j < CW / 8; j++)
                     q[j] = make_uint4(pack2(e[8 * j], e[8 * j + 1], p.is_bf16), pack2(e[8 * j + 2], e[8 * j + 3], p.is_bf16), pack2(e[8 * j + 4], e[8 * j + 5], p.is_bf16),
                                       pack2(e[8 * j + 6], e[8 * j + 7], p.is_bf16));
             };
-            // This warp's 32 columns of a chunk.
-            auto store_chunk = [&](int c, const uint32_t (&v)[32]) {
+            auto store_chunk = [&](int c, const uint32_t (&v)[CW / 32][32]) {
                 const int col = tn * bn + c * EPI_CHUNK_COLS;
-                if (MODE == TC_STORE && p.out_f32) {
-                    // f32: 32 columns are the 128 bytes a row of a copy has, so each warp stages and stores its own
-                    if (lane == 0) tma_store_wait_read<0>();
-                    __syncwarp();
-                    unsigned char* src = stage_buf + half * EPI_STAGE_BYTES;
+                if constexpr (MODE == TC_STORE) {
+                    static_assert(W == 1, "f32 results: a warp stages both halves of a chunk");
+                    if (p.out_f32) {
+                        // two 32-column f32 chunks (128 bytes per row each), one per staging buffer
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        *reinterpret_cast<uint4*>(src + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-                        tma_store_3d(&map_d, smem_u32(src), col + half * 32, tm * BM + quarter * 32, tb);
-                        tma_store_commit();
+                        for (int h = 0; h < CW / 32; h++) {
+                            if (lane == 0) tma_store_wait_read<1>();
+                            __syncwarp();
+                            unsigned char* src = stage_buf + buf * EPI_STAGE_BYTES;
+#pragma unroll
+                            for (int j = 0; j < 8; j++)
+                                *reinterpret_cast<uint4*>(src + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(v[h][4 * j], v[h][4 * j + 1], v[h][4 * j + 2], v[h][4 * j + 3]);
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (lane == 0) {
+                                tma_store_3d(&map_d, smem_u32(src), col + h * 32, tm * BM + quarter * 32, tb);
+                                tma_store_commit();
+                            }
+                            buf ^= 1;
+                        }
+                        return;
                     }
-                    return;
                 }
-                float e[32];
-                uint4 q[4];
+                float e[CW];
+                uint4 q[CW / 8];
 #pragma unroll
-                for (int j = 0; j < 32; j++) e[j] = __uint_as_float(v[j]);
+                for (int j = 0; j < CW; j++) e[j] = __uint_as_float(v[j / 32][j % 32]);
                 if (MODE == TC_BIAS || (MODE == TC_PLAIN && p.fuse)) {
                     // Linear + bias (+ GELU) in one pass, with the roundings of the separate ops: the product is rounded to
                     // the operand type, the bias is added in f32 and rounded (u), the activation is evaluated on u in f32
                     // and rounded (act) - bit for bit what cuda_matmul, cuda_add and cuda_gelu give one after the other.
 #pragma unroll
-                    for (int j = 0; j < 32; j++) e[j] = round16(round16(e[j], p.is_bf16) + fused_bias, p.is_bf16);
+                    for (int j = 0; j < CW; j++) e[j] = round16(round16(e[j], p.is_bf16) + fused_bias, p.is_bf16);
                 }
                 pack(e, q);
                 flush(&map_d, col, q);
                 if (MODE == TC_BIAS && p.fuse == 2) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) e[j] = gelu_f32_fast(e[j]);
+                    for (int j = 0; j < CW; j++) e[j] = gelu_f32_fast(e[j]);
                     pack(e, q);
                     flush(&map_d2, col, q);
                 }
+            };
+            auto load_chunk = [&](uint32_t at, uint32_t (&v)[CW / 32][32]) {
+#pragma unroll
+                for (int h = 0; h < CW / 32; h++) tmem_ld_32x32b_x32(at + h * 32, v[h]);
+            };
+            auto wait_chunk = [&](uint32_t (&v)[CW / 32][32]) {
+                tmem_ld_wait_for(v[0]);
+                if constexpr (CW > 32) reg_fence(v[CW / 32 - 1]);
             };
             // The TMEM loads of chunk c + 1 are in flight while chunk c is converted and stored.
             const int chunks = bn / EPI_CHUNK_COLS;
@@ -474,23 +498,24 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if (lane == 0) mbar_arrive(tempty_bar(acc));
             };
             if constexpr (DRAIN) {
-                uint32_t total[2][32], v[32];  // tiles of at most 128 columns
+                uint32_t total[2][CW / 32][32], v[32];  // tiles of at most 128 columns
 #pragma unroll
-                for (int c = 0; c < 2; c++)
-#pragma unroll
-                    for (int j = 0; j < 32; j++) total[c][j] = 0;  // 0.0f
+                for (int c = 0; c < 2 * CW; c++) total[c / CW][c % CW / 32][c % 32] = 0;  // 0.0f
                 bool ok = true;
                 for (int run = 0; run < p.num_kb && ok; run += p.run_kb) {
                     ok = wait_accumulator();
                     if (!ok) break;
-                    const uint32_t t_run = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * 32);
+                    const uint32_t t_run = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * CW);
 #pragma unroll
                     for (int c = 0; c < 2; c++) {
                         if (c >= chunks) break;
-                        tmem_ld_32x32b_x32(t_run + c * EPI_CHUNK_COLS, v);
-                        tmem_ld_wait_for(v);
 #pragma unroll
-                        for (int j = 0; j < 32; j++) total[c][j] = __float_as_uint(__uint_as_float(total[c][j]) + __uint_as_float(v[j]));
+                        for (int h = 0; h < CW / 32; h++) {
+                            tmem_ld_32x32b_x32(t_run + c * EPI_CHUNK_COLS + h * 32, v);
+                            tmem_ld_wait_for(v);
+#pragma unroll
+                            for (int j = 0; j < 32; j++) total[c][h][j] = __float_as_uint(__uint_as_float(total[c][h][j]) + __uint_as_float(v[j]));
+                        }
                     }
                     hand_back();
                     if (++acc == 2) {
@@ -503,18 +528,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if (chunks > 1) store_chunk(1, total[1]);
                 continue;
             }
-            uint32_t va[32], vb[32];
-            tmem_ld_32x32b_x32(t_row, va);
+            uint32_t va[CW / 32][32], vb[CW / 32][32];
+            load_chunk(t_row, va);
 #pragma unroll
             for (int c = 0; c < BN / EPI_CHUNK_COLS; c += 2) {
                 if (c >= chunks) break;
-                tmem_ld_wait_for(va);
-                if (c + 1 < chunks) tmem_ld_32x32b_x32(t_row + (c + 1) * EPI_CHUNK_COLS, vb);
+                wait_chunk(va);
+                if (c + 1 < chunks) load_chunk(t_row + (c + 1) * EPI_CHUNK_COLS, vb);
                 else hand_back();
                 store_chunk(c, va);
                 if (c + 1 >= chunks) break;
-                tmem_ld_wait_for(vb);
-                if (c + 2 < chunks) tmem_ld_32x32b_x32(t_row + (c + 2) * EPI_CHUNK_COLS, va);
+                wait_chunk(vb);
+                if (c + 2 < chunks) load_chunk(t_row + (c + 2) * EPI_CHUNK_COLS, va);
                 else hand_back();
                 store_chunk(c + 1, vb);
             }
@@ -558,7 +583,7 @@ bool opt_in_shared_memory() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
-        for (auto kernel : {tc_gemm_kernel<TC_STORE, BN>, tc_gemm_kernel<TC_BIAS, BN>, tc_gemm_kernel<TC_STORE, 0>, tc_gemm_kernel<TC_BIAS, 0>, tc_gemm_kernel<TC_PLAIN, 0>,
+        for (auto kernel : {tc_gemm_kernel<TC_STORE, BN>, tc_gemm_kernel<TC_BIAS, BN>, tc_gemm_kernel<TC_STORE, 0>, tc_gemm_kernel<TC_BIAS, 0>, tc_gemm_kernel<TC_PLAIN, 0>, tc_gemm_kernel<TC_STORE, BN, false, true>, tc_gemm_kernel<TC_BIAS, BN, false, true>,
                             tc_gemm_kernel<TC_STORE, 0, true>, tc_gemm_kernel<TC_BIAS, 0, true>, tc_gemm_kernel<TC_PLAIN, 0, true>})
             if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess) {
                 cudaGetLastError();
@@ -685,7 +710,7 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     // few output tiles: cut K into slices that run as the batches of this launch
     int slices = 1;
     const int bn_whole = p.b_keep ? p.bn : tile_columns((uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid);
-    p.panels = p.bn == BN && bn_whole == BN && keep_panels((uint64_t)p.tiles_m, (uint64_t)p.tiles_n, p.num_kb, batch, grid) ? 1 : 0;
+    const bool panels = p.bn == BN && bn_whole == BN && !c.d_plain && keep_panels((uint64_t)p.tiles_m, (uint64_t)p.tiles_n, p.num_kb, batch, grid);
     if (batch == 1 && !fuse && !p.b_keep) {
         slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
         if (slices == 1)
@@ -743,10 +768,11 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     if (grid > p.num_tiles) grid = p.num_tiles;
     if (p.b_keep) grid = p.b_keep * p.tiles_n;
     const bool full = p.bn == BN;
-    const auto kernel = drain ? (p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0, true> : (fuse ? tc_gemm_kernel<TC_BIAS, 0, true> : tc_gemm_kernel<TC_STORE, 0, true>))
+    const auto kernel = panels ? (fuse ? tc_gemm_kernel<TC_BIAS, BN, false, true> : tc_gemm_kernel<TC_STORE, BN, false, true>)
+                        : drain ? (p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0, true> : (fuse ? tc_gemm_kernel<TC_BIAS, 0, true> : tc_gemm_kernel<TC_STORE, 0, true>))
                         : p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0>
                                   : (fuse ? (full ? tc_gemm_kernel<TC_BIAS, BN> : tc_gemm_kernel<TC_BIAS, 0>) : (full ? tc_gemm_kernel<TC_STORE, BN> : tc_gemm_kernel<TC_STORE, 0>));
-    kernel<<<grid, TC_THREADS, TC_SMEM_BYTES, ctx().stream>>>(ma, mb, md, md2, p, err, tag);
+    kernel<<<grid, tc_threads(p.d_plain ? TC_PLAIN : TC_STORE), TC_SMEM_BYTES, ctx().stream>>>(ma, mb, md, md2, p, err, tag);
     check_launch(where);
     if (slices > 1) splitk_reduce(is_bf16 ? 0 : 1, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
     return true;
