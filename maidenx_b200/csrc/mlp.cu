@@ -351,6 +351,9 @@ void mx_mlp_sgd_layer(void* h, int l, float lr, float grad_scale) {
     if (m->is_bf16) sgd_layer_t<bf16>(m, l, lr, grad_scale);
     else sgd_layer_t<f16>(m, l, lr, grad_scale);
 }
+// Weights of a layer up to which its update stays on the main stream of mx_mlp_train_step: a pass of 4 us then, which the way to the side
+// stream (two event calls of the host, a wait between streams on the device) would not repay.
+static constexpr size_t kSideLeast = (size_t)1 << 21;
 // One whole training step of the single-device engine.  The optimizer update of layer l is memory-bound and nothing
 // below it in the backward pass needs its result, so it runs on the side stream beside the backward products of the
 // layers below (which are bound by the tensor cores, not by HBM); the next forward waits, per layer, for that layer's
@@ -366,13 +369,16 @@ void mx_mlp_train_step(void* h, const void* x, const void* y, float lr, float gr
     mx_mlp_loss_backward(h, y);
     for (int l = m->layers - 1; l >= 0; l--) {
         mx_mlp_backward_layer(h, l);
-        cudaEventRecord(m->ev_grad[l], main_stream);
-        cudaStreamWaitEvent(m->side, m->ev_grad[l], 0);
-        ctx().stream = m->side;
+        const cudaStream_t update = m->dim * m->dim < kSideLeast ? main_stream : m->side;
+        if (update != main_stream) {
+            cudaEventRecord(m->ev_grad[l], main_stream);
+            cudaStreamWaitEvent(update, m->ev_grad[l], 0);
+        }
+        ctx().stream = update;
         if (m->is_bf16) sgd_layer_t<bf16>(m, l, lr, grad_scale);
         else sgd_layer_t<f16>(m, l, lr, grad_scale);
         ctx().stream = main_stream;
-        cudaEventRecord(m->ev_done[l], m->side);
+        cudaEventRecord(m->ev_done[l], update);
     }
     check_launch("mx_mlp_train_step");
 }
