@@ -36,10 +36,12 @@
 // Every mbarrier wait is bounded (see tc_ptx.cuh); on expiry all roles fall through to the common exit.
 #include <cuda.h>
 
+#include <atomic>
+#include <algorithm>
 #include <mutex>
 
 #include "matmul_tc.cuh"
-#include "tc_ptx.cuh"
+#include "tc_cluster.cuh"
 
 namespace mx {
 
@@ -107,6 +109,10 @@ struct Params {
     int K, zs;      // zs: batches of the operands (kb_per_z > 0)
     float* out;     // D or the split-K partial results, rows `out_ld` elements apart
     int64_t out_ld;
+    // > 0: the K slices of an output tile are the CTAs of one cluster; each leaves its partial result in its own shared memory and adds the
+    // rows that fall to it over all of them, in slice order (the sums of the form with a second launch, bit for bit)
+    int cluster;
+    int vec_out;    // cluster: the rows of `out` may be written by 16-byte vectors
 };
 
 __device__ __forceinline__ void tile_coords(int tile, const Params& p, int& tm, int& tn, int& tb) {
@@ -130,6 +136,11 @@ __device__ __forceinline__ uint32_t small_part(uint32_t bits) {
     const uint32_t s = (__float_as_uint(x - big) + 0x1000u) & 0xFFFFE000u;
     return (bits & 0x7F800000u) == 0x7F800000u ? 0u : s;
 }
+
+// Where a CTA of a cluster keeps its partial result: behind what redo_tile stages; a row is 16 bytes longer than 128 floats, so that the threads of a
+// warp, a row each, store to different banks.
+constexpr int PART_OFF = 64 * 1024, PART_LD = BN + 4;
+static_assert(PART_OFF + BM * PART_LD * 4 <= STAGES * STAGE_BYTES && 2 * BK * (BM + 4) * 4 <= PART_OFF, "partial result inside the ring");
 
 // A tile whose result is not finite, again and in f32 arithmetic: the split has no form for infinities (inf times the zero `small` of
 // an operand that tf32 holds exactly is NaN) and the tensor core reads a NaN whose payload sits in the low bits as one.  An
@@ -185,7 +196,9 @@ __device__ __forceinline__ void redo_tile(const Params& p, int bn, int tm, int t
 #pragma unroll
         for (int j = 0; j < BN / T; j++) {
             const int c = tx + T * j;
-            if (row < p.M && c < bn && tn * bn + c < p.N) p.out[((int64_t)tb * p.M + row) * p.out_ld + tn * bn + c] = acc[i][j];
+            if (row >= p.M || c >= bn || tn * bn + c >= p.N) continue;
+            if (p.cluster) stage[PART_OFF / 4 + (ty + T * i) * PART_LD + c] = acc[i][j];
+            else p.out[((int64_t)tb * p.M + row) * p.out_ld + tn * bn + c] = acc[i][j];
         }
     }
 }
@@ -193,7 +206,8 @@ __device__ __forceinline__ void redo_tile(const Params& p, int bn, int tm, int t
 // BN_T = 128: the form of 128-column tiles, long chunks and tensor stores, all known to the compiler; 0: everything from the
 // parameters.  The difference is the splitter's: with the distance between a raw and its small tile a constant, its loads run
 // ahead of its stores (8192 x 4096 x 4096: 164 TFLOP/s, 148 in batches of four).
-template <int BN_T>
+// CLUSTER: Params::cluster.
+template <int BN_T, bool CLUSTER = false>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                    Params p, int* err, int tag) {
@@ -212,6 +226,9 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int chunk_kb = BN_T ? CHUNK_FAST : p.chunk_kb;
     const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? STAGES : p.stages, raw_bytes = BN_T ? A_TILE + BN_T * BK * 4 : p.raw_bytes;
+
+    // a CTA of a cluster of slices has one tile and slice: its rank is the batch, and the grid is as long as the tiles
+    const int first_tile = CLUSTER ? (int)blockIdx.x % p.cluster * p.tiles_per_batch + (int)blockIdx.x / p.cluster : (int)blockIdx.x;
 
     auto redo = [&] { return reinterpret_cast<uint32_t*>(smem + Smem::redo); };
     if (threadIdx.x <= REDO_BITS / 32) redo()[threadIdx.x] = 0;
@@ -242,7 +259,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
+            for (int tile = first_tile; tile < p.num_tiles && ok; tile += gridDim.x) {
                 int tm, tn, tb;
                 tile_coords(tile, p, tm, tn, tb);
                 int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
@@ -287,7 +304,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
+            for (int tile = first_tile; tile < p.num_tiles && ok; tile += gridDim.x) {
                 for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += chunk_kb) {
                     if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1, err, tag, 2)) {
                         ok = false;
@@ -351,7 +368,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         int acc = 0, buf = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
+        for (int tile = first_tile; tile < p.num_tiles && ok; tile += gridDim.x) {
             int tm, tn, tb;
             tile_coords(tile, p, tm, tn, tb);
             float total[BN];  // this thread's row of the tile (registers: every index below is a compile-time constant)
@@ -386,6 +403,17 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
             if (!ok) break;
             float zero = 0.0f;  // NaN from the first total on that is not finite
+            if constexpr (CLUSTER) {
+                float* part = reinterpret_cast<float*>(smem + Smem::stages + PART_OFF) + (quarter * 32 + lane) * PART_LD;  // the ring is done with
+#pragma unroll
+                for (int j = 0; j < BN; j += 4) {
+                    if (j >= bn) break;
+                    *reinterpret_cast<float4*>(part + j) = make_float4(total[j], total[j + 1], total[j + 2], total[j + 3]);
+                    zero += fmaf(total[j], 0.0f, fmaf(total[j + 1], 0.0f, fmaf(total[j + 2], 0.0f, total[j + 3] * 0.0f)));
+                }
+                if (__any_sync(0xFFFFFFFFu, zero != 0.0f) && lane == 0) redo()[REDO_BITS / 32] = 1;
+                continue;
+            }
 #pragma unroll
             for (int c = 0; c < BN / EPI_CHUNK_COLS; c++) {
                 if (c * EPI_CHUNK_COLS >= bn) break;
@@ -425,7 +453,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 buf ^= 1;
             }
             if (__any_sync(0xFFFFFFFFu, zero != 0.0f) && lane == 0) {
-                const int it = (tile - (int)blockIdx.x) / (int)gridDim.x;
+                const int it = (tile - first_tile) / (int)gridDim.x;
                 atomicOr(&redo()[it % REDO_BITS / 32], 1u << it % 32);
                 redo()[REDO_BITS / 32] = 1;
             }
@@ -437,7 +465,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
+        for (int tile = first_tile; tile < p.num_tiles && ok; tile += gridDim.x) {
             for (int kb = 0; kb < p.num_kb; kb++) {
                 const bool landed = mbar_wait_relaxed(full_bar(stage), phase, err, tag, 5, 40);
                 if (!__all_sync(0xFFFFFFFFu, landed)) {
@@ -490,6 +518,30 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
 
+    if constexpr (CLUSTER) {
+        int tm, tn, tb;
+        tile_coords(first_tile, p, tm, tn, tb);
+        if (redo()[REDO_BITS / 32]) redo_tile(p, bn, tm, tn, tb, reinterpret_cast<float*>(smem + Smem::stages));
+        cluster_sync_all();
+        const int r0 = BM * tb / p.cluster, rows = BM * (tb + 1) / p.cluster - r0, vecs = bn / 4;
+        for (int e = threadIdx.x; e < rows * vecs; e += THREADS) {
+            const int r = r0 + e / vecs, c = e % vecs * 4, row = tm * BM + r, col = tn * bn + c;
+            if (row >= p.M || col >= p.N) continue;
+            const float4 sum = sum_slices(smem_base + Smem::stages + PART_OFF + (uint32_t)(r * PART_LD + c) * 4, p.cluster);
+            float* out = p.out + (int64_t)row * p.out_ld + col;
+            if (p.vec_out) {
+                *reinterpret_cast<float4*>(out) = sum;
+            } else {
+                out[0] = sum.x;
+                if (col + 1 < p.N) out[1] = sum.y;
+                if (col + 2 < p.N) out[2] = sum.z;
+                if (col + 3 < p.N) out[3] = sum.w;
+            }
+        }
+        cluster_sync_all();  // the others have read this CTA's part
+        return;
+    }
+
     // the tile stores have completed (tma_store_wait_all before the barrier above): their places may be written again
     if (!redo()[REDO_BITS / 32]) return;
     fence_proxy_async();
@@ -508,7 +560,7 @@ bool opt_in_shared_memory() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
-        for (auto kernel : {tc_gemm_f32_kernel<BN>, tc_gemm_f32_kernel<0>})
+        for (auto kernel : {tc_gemm_f32_kernel<BN>, tc_gemm_f32_kernel<0>, tc_gemm_f32_kernel<BN, true>, tc_gemm_f32_kernel<0, true>})
             if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
@@ -536,6 +588,9 @@ int tile_columns(uint64_t tiles_m, uint64_t N, uint64_t batch, int grid) {
 }
 // what the second launch of a split-K product costs, in k-blocks (about 0.9 us each on one CTA)
 constexpr double kSplitFixed32 = 3.0;
+// and the sum inside a cluster
+constexpr double kClusterFixed32 = 1.5;
+std::atomic<int> g_cluster{1};  // 0: no clusters of slices (tests, A/B timing)
 
 // D[M,N] = sum_k Aop[m,k] * Bop[n,k]; K-major operand = row-major [MN, K], MN-major = row-major [K, MN].
 bool launch(const TcProduct& c, void* D, const char* where) {
@@ -563,15 +618,22 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     // few output tiles: cut K into slices that run as the batches of this launch (see tc_ptx.cuh)
     int slices = 1;
     const int bn_whole = tile_columns((uint64_t)p.tiles_m, N, batch, grid);
+    p.cluster = 0;
     if (batch == 1) {
-        if (!c.sum_batches) slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
-        if (slices == 1)
-            slices = splitk_short((uint64_t)p.tiles_m * p.tiles_n, (uint64_t)p.num_kb, grid, (128 + p.bn) / 256.0,
-                                  tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, grid) * p.num_kb - kSplitFixed32);
+        const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n;
+        const double kb = (128 + p.bn) / 256.0, whole = tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, grid) * p.num_kb;
+        if (!c.sum_batches) slices = splitk_slices(tiles, K, BK, grid);
+        if (slices == 1) slices = splitk_short(tiles, (uint64_t)p.num_kb, grid, kb, whole - kSplitFixed32);
+        double cost = whole;
+        if (slices > 1) cost = std::min(cost, (double)((tiles * slices + grid - 1) / grid * ((p.num_kb + slices - 1) / slices)) * kb + kSplitFixed32 + 0.1 * slices);
+        if (g_cluster.load(std::memory_order_relaxed))
+            p.cluster = cluster_slices(tiles, (uint64_t)p.num_kb, grid, kb, kClusterFixed32, cost,
+                                       [](int n) { return resident_clusters(reinterpret_cast<const void*>(tc_gemm_f32_kernel<0, true>), THREADS, SMEM_BYTES, n); });
+        if (p.cluster) slices = p.cluster;
     }
     StreamWorkspace partial;
     const uint64_t n_pitch = (N + 3) / 4 * 4;
-    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) slices = 1;
+    if (slices > 1 && !p.cluster && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) slices = 1;
     if (slices > 1) {
         p.split_kb = (p.num_kb + slices - 1) / slices;
         p.num_kb = p.split_kb;
@@ -592,7 +654,8 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     const bool okb = b_mn ? make_map(&mb, c.B, K, N, c.batch, b_bs, BK, true, c.b_pitch) : make_map(&mb, c.B, N, K, c.batch, b_bs, (uint32_t)p.bn, false, c.b_pitch);
     if (!oka || !okb) return false;
     p.d_plain = slices > 1 ? 0 : c.d_plain;
-    if (p.d_plain) md = ma;  // not used
+    p.vec_out = N % 4 == 0 && (uintptr_t)D % 16 == 0 ? 1 : 0;
+    if (p.d_plain || p.cluster) md = ma;  // not used
     else if (slices > 1 ? !make_map(&md, partial.ptr, M, N, batch, M * n_pitch, 32, false, n_pitch) : !make_map(&md, D, M, N, batch, M * N, 32)) return false;
     p.num_tiles = (int)batch * p.tiles_per_batch;
     p.a_batched = (c.batch > 1 && a_bs != 0) ? 1 : 0;
@@ -610,13 +673,14 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.b_ks = b_mn ? b_ld : 1;
     p.K = (int)K;
     p.zs = (int)c.batch;
-    p.out = static_cast<float*>(slices > 1 ? partial.ptr : D);
-    p.out_ld = (int64_t)(slices > 1 ? n_pitch : N);
+    p.out = static_cast<float*>(slices > 1 && !p.cluster ? partial.ptr : D);
+    p.out_ld = (int64_t)(slices > 1 && !p.cluster ? n_pitch : N);
     if (grid > p.num_tiles) grid = p.num_tiles;
-    const auto kernel = p.bn == BN && !p.d_plain && p.chunk_kb == CHUNK_FAST ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>;
-    kernel<<<grid, THREADS, SMEM_BYTES, ctx().stream>>>(ma, mb, md, p, err, tag);
+    const bool fixed = p.bn == BN && !p.d_plain && p.chunk_kb == CHUNK_FAST;
+    const auto kernel = p.cluster ? (fixed ? tc_gemm_f32_kernel<BN, true> : tc_gemm_f32_kernel<0, true>) : (fixed ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>);
+    launch_clusters(kernel, p.cluster ? p.num_tiles : grid, THREADS, SMEM_BYTES, p.cluster, ma, mb, md, p, err, tag);
     check_launch(where);
-    if (slices > 1) splitk_reduce(2, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
+    if (slices > 1 && !p.cluster) splitk_reduce(2, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
     return true;
 }
 
@@ -632,3 +696,6 @@ bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t 
 }
 
 }  // namespace mx
+
+// 1 (default): the slices of a split f32 product are summed inside a cluster where they fit one; 0: always by a second launch
+extern "C" void mx_debug_set_gemm_f32_cluster(int on) { mx::g_cluster.store(on ? 1 : 0, std::memory_order_relaxed); }

@@ -402,6 +402,51 @@ def test_products_with_ragged_rows(oracle, cuda, dt, case):
     H.assert_same("matmul", dt, got, ref, float_rel=1e-5 if dt.name == "f32" else 1e-2, what=name, scale=np.sqrt(k))
 
 
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [
+    # M, N, K, majors: two to eight slices, the last one short; ragged rows and edges of tiles; one row and one column of tiles; reductions that are emptied in runs
+    (128, 300, 784, "kk"), (128, 784, 300, "km"), (300, 784, 1024, "mm"), (130, 131, 9001, "kk"), (257, 64, 2049, "mk"), (100, 1000, 4100, "km"), (1, 4099, 4099, "km"),
+    (512, 72, 8200, "mm"), (1543, 200, 2000, "mm")], ids=lambda c: "x".join(map(str, c)))
+def test_slices_summed_in_a_cluster(cuda, dt, case):
+    """A split product whose slices are the CTAs of a cluster, next to float64 and to the form with a second launch; an infinity reaches its own row and
+    nothing else, and nothing is written around the output."""
+    from maidenx_b200 import _lib, device
+    lib = _lib.load()
+    m, n, k, majors = case
+    rng = np.random.default_rng(m + n + k)
+    a, b = (D.encode(rng.standard_normal(x).astype(np.float32).reshape(-1), dt).reshape(x) for x in ((m, k), (k, n)))
+    inf = m > 64
+    if inf:
+        a[m - 1, k // 2] = D.encode(np.array([np.inf], np.float32), dt)[0]
+    am, bm = a if majors[0] == "k" else a.T, b.T if majors[1] == "k" else b
+    meta = [2, 2, 2, m, n, m, k, k, n, *([k, 1] if majors[0] == "k" else [1, m]), *([1, k] if majors[1] == "k" else [n, 1]), 0, 0]
+    guard = 16
+    fill = np.full(m * n + 2 * guard, 3, dtype=dt.np_storage)
+    got = {}
+    try:
+        for on in (0, 1):
+            lib.mx_debug_set_gemm_cluster(on)
+            lib.mx_debug_set_gemm_f32_cluster(on)
+            bufs = [device.CudaBuffer.from_host(np.ascontiguousarray(x).reshape(-1)) for x in (am, bm, fill)]
+            device.dispatch("matmul", dt.name, meta, m * n, "META", bufs[0].ptr, bufs[1].ptr, bufs[2].ptr + guard * dt.size)
+            raw = bufs[2].to_host(dt.np_storage, fill.size)
+            assert (raw[:guard] == 3).all() and (raw[-guard:] == 3).all()
+            got[on] = D.decode(raw[guard:-guard], dt).astype(np.float64).reshape(m, n)
+            for x in bufs:
+                x.free()
+    finally:
+        lib.mx_debug_set_gemm_cluster(1)
+        lib.mx_debug_set_gemm_f32_cluster(1)
+    ref = np.matmul(D.decode(a.reshape(-1), dt).astype(np.float64).reshape(m, k)[:m - inf], D.decode(b.reshape(-1), dt).astype(np.float64).reshape(k, n))
+    once = D.decode(D.encode(ref.astype(np.float32).reshape(-1), dt), dt).astype(np.float64).reshape(ref.shape)
+    for out in got.values():
+        if inf:
+            assert np.isinf(out[m - 1]).all()
+        # f32: the split product's error; 16 bits: what rounding the exact result once gives, and a few sums that round the other way
+        err = np.linalg.norm(out[:m - inf] - ref) / np.linalg.norm(ref)
+        assert err <= (2e-6 if dt.name == "f32" else 1.01 * np.linalg.norm(once - ref) / np.linalg.norm(ref)), err
+
+
 @pytest.mark.parametrize("off", [0, 1, 3, 4, 6, 7])
 @pytest.mark.parametrize("n", [1, 7, 9, 63, 65, 71, 127, 130, 191, 194, 257, 260, 391])
 def test_ragged_output_rows_are_written_whole_and_alone(cuda, n, off):
