@@ -139,6 +139,30 @@ struct StreamWorkspace {
     ~StreamWorkspace();
 };
 
+// Launches `kernel` so that it is scheduled as soon as the blocks of the kernel before it in the stream have ended, without the launch's own latency
+// between the two (programmatic dependent launch): 2 us less for each of a chain of kernels on small tensors (1e6 floats 5.1 us a launch, now 3.1), up to a
+// third of a small layer's time.  The kernel's threads call after_previous_kernel() before they touch global memory.  The kernels do not
+// let their successors in any earlier (griddepcontrol.launch_dependents): blocks that wait take the places of blocks that work (8e6 floats 33 us
+// instead of 17).  A kernel that is launched the ordinary way waits for whole kernels as ever.
+template <class... P, class... A>
+inline void launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t stream, const A&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = shared;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+// Every thread of a kernel that launch_kernel starts, before its first access to global memory: waits until the kernel before has completed and its
+// writes are visible.  Such kernels have no __restrict__ const pointers: what is read through one counts as constant for the whole kernel, and its
+// loads need not stay behind this.
+__device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 int sm_count();
 // Blocks of `kernel` that stay resident on one SM at this block size and dynamic shared memory (at least 1).
 int resident_blocks(const void* kernel, int threads, size_t dynamic_smem = 0);

@@ -46,7 +46,7 @@ constexpr int kConvThreads = 256;
 
 // `count` consecutive elements into shared memory, as 16-byte vectors where the source allows.
 template <class T>
-__device__ __forceinline__ void stage_run(T* dst, const T* __restrict__ src, uint32_t count) {
+__device__ __forceinline__ void stage_run(T* dst, const T* src, uint32_t count) {
     constexpr uint32_t VEC = 16 / sizeof(T);
     uint32_t done = 0;
     if ((uintptr_t)src % 16 == 0) {
@@ -61,7 +61,8 @@ __device__ __forceinline__ void stage_run(T* dst, const T* __restrict__ src, uin
 // busy and ragged ones (7 x 7) are written as vectors too.  Bound by HBM / L2 writes: [32, 128, 14, 14] f32, 3 x 3: 12 us, 23 with one
 // plane and one kernel offset at a time.
 template <class T, int VEC>
-__global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* __restrict__ x, T* __restrict__ col, ConvPlanes P) {
+__global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* x, T* col, ConvPlanes P) {
+    after_previous_kernel();
     extern __shared__ __align__(16) unsigned char conv_smem[];
     T* img = reinterpret_cast<T*>(conv_smem);
     const uint32_t bc0 = blockIdx.x * P.per_block, np = min(P.per_block, P.planes - bc0);
@@ -109,7 +110,8 @@ __global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* __
 // One block per plane, one kernel offset at a time.  Large maps keep its threads busy with less arithmetic per element than the flat
 // index above takes (see planes_pay).  STAGED: the plane fits shared memory.
 template <class T, int VEC, bool STAGED>
-__global__ void __launch_bounds__(kConvThreads) im2col_kernel(const T* __restrict__ x, T* __restrict__ col, ConvParams P) {
+__global__ void __launch_bounds__(kConvThreads) im2col_kernel(const T* x, T* col, ConvParams P) {
+    after_previous_kernel();
     extern __shared__ __align__(16) unsigned char conv_smem[];
     T* plane = reinterpret_cast<T*>(conv_smem);
     const uint64_t bc = blockIdx.x;  // b * C + c
@@ -163,7 +165,8 @@ __device__ __forceinline__ T conv_add(T a, T b) {
 // column entry crosses from L2 once instead of once per term.  Strides of 1: larger ones touch few entries more than once.
 // [32, 128, 14, 14] f32, 3 x 3: 14 us, 16 from L2.
 template <class T>
-__global__ void __launch_bounds__(kConvThreads) col2im_planes_kernel(const T* __restrict__ col, T* __restrict__ out, ConvPlanes P) {
+__global__ void __launch_bounds__(kConvThreads) col2im_planes_kernel(const T* col, T* out, ConvPlanes P) {
+    after_previous_kernel();
     extern __shared__ __align__(16) unsigned char conv_smem[];
     T* cols = reinterpret_cast<T*>(conv_smem);
     const uint32_t bc0 = blockIdx.x * P.per_block, np = min(P.per_block, P.planes - bc0);
@@ -197,7 +200,8 @@ __global__ void __launch_bounds__(kConvThreads) col2im_planes_kernel(const T* __
 }
 
 template <class T>
-__global__ void __launch_bounds__(kConvThreads) col2im_kernel(const T* __restrict__ col, T* __restrict__ out, ConvParams P) {
+__global__ void __launch_bounds__(kConvThreads) col2im_kernel(const T* col, T* out, ConvParams P) {
+    after_previous_kernel();
     const uint64_t bc = blockIdx.y;  // b * C + c
     const uint32_t HW = P.H * P.W, OHW = P.OH * P.OW, KK = P.KH * P.KW;
     const uint32_t pix = blockIdx.x * kConvThreads + threadIdx.x;
@@ -323,7 +327,7 @@ void im2col_entry(size_t num_els, const size_t* meta, const T* x, T* col, const 
         const size_t smem = (size_t)(P.H + 2 * P.PH) * Q.pitch * sizeof(T);
         auto go = [&](auto kernel) {
             allow_shared_memory(kernel, smem);
-            kernel<<<grid, kConvS1Threads, smem, s>>>(x, col, Q);
+            launch_kernel(kernel, grid, kConvS1Threads, smem, s, x, col, Q);
             check_launch(where);
         };
         if (smem <= kConvSmemMost) {
@@ -343,17 +347,17 @@ void im2col_entry(size_t num_els, const size_t* meta, const T* x, T* col, const 
     const uint32_t pb = (uintptr_t)col % 16 == 0 ? planes_per_block(planes_touched, plane_bytes, step, planes_most(sizeof(T), step, ohw)) : 0;
     if (pb && pb * chunk < 0x7FFFFFFFull && planes_pay(sizeof(T), step, (planes_touched + pb - 1) / pb, ohw)) {
         allow_shared_memory(im2col_planes_kernel<T, VEC>, pb * plane_bytes);
-        im2col_planes_kernel<T, VEC><<<(unsigned)((planes_touched + pb - 1) / pb), kConvThreads, pb * plane_bytes, s>>>(x, col, ConvPlanes(P, planes_touched, pb));
+        launch_kernel(im2col_planes_kernel<T, VEC>, (unsigned)((planes_touched + pb - 1) / pb), kConvThreads, pb * plane_bytes, s, x, col, ConvPlanes(P, planes_touched, pb));
     } else if (plane_bytes <= kConvSmemMost) {
         auto launch = [&](auto kernel) {
             allow_shared_memory(kernel, plane_bytes);
-            kernel<<<grid, kConvThreads, plane_bytes, s>>>(x, col, P);
+            launch_kernel(kernel, grid, kConvThreads, plane_bytes, s, x, col, P);
         };
         if (vec) launch(im2col_kernel<T, VEC, true>);
         else launch(im2col_kernel<T, 1, true>);
     } else {
-        if (vec) im2col_kernel<T, VEC, false><<<grid, kConvThreads, 0, s>>>(x, col, P);
-        else im2col_kernel<T, 1, false><<<grid, kConvThreads, 0, s>>>(x, col, P);
+        if (vec) launch_kernel(im2col_kernel<T, VEC, false>, grid, kConvThreads, 0, s, x, col, P);
+        else launch_kernel(im2col_kernel<T, 1, false>, grid, kConvThreads, 0, s, x, col, P);
     }
     check_launch(where);
 }
@@ -391,7 +395,7 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
             if (num_els >= planes * plane_elems && stage_bytes % 16 == 0 && stage_bytes <= 112 * 1024 && plane_elems < (1ull << 30)) {
                 auto go = [&](auto kernel) {
                     allow_shared_memory(kernel, stage_bytes);
-                    kernel<<<(unsigned)planes, kConvS1Threads, stage_bytes, s>>>(col, out, Q, tc::next_wait_report());
+                    launch_kernel(kernel, (unsigned)planes, kConvS1Threads, stage_bytes, s, col, out, Q, tc::next_wait_report());
                     check_launch(where);
                 };
                 if (kw == 1 && pw == 0) { go(col2im_s1_staged_kernel<T, VEC, 1, 0>); return; }
@@ -401,11 +405,11 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
                 if (kw == 7 && pw == 3 && VEC > 3) { go(col2im_s1_staged_kernel<T, VEC, 7, 3>); return; }
             }
             bool done = true;
-            if (kw == 1 && pw == 0) col2im_s1_kernel<T, VEC, 1, 0><<<grid, kConvS1Threads, 0, s>>>(col, out, Q);
-            else if (kw == 3 && pw == 1) col2im_s1_kernel<T, VEC, 3, 1><<<grid, kConvS1Threads, 0, s>>>(col, out, Q);
-            else if (kw == 3 && pw == 0 && VEC > 2) col2im_s1_kernel<T, VEC, 3, 0><<<grid, kConvS1Threads, 0, s>>>(col, out, Q);
-            else if (kw == 5 && pw == 2 && VEC > 2) col2im_s1_kernel<T, VEC, 5, 2><<<grid, kConvS1Threads, 0, s>>>(col, out, Q);
-            else if (kw == 7 && pw == 3 && VEC > 3) col2im_s1_kernel<T, VEC, 7, 3><<<grid, kConvS1Threads, 0, s>>>(col, out, Q);
+            if (kw == 1 && pw == 0) launch_kernel(col2im_s1_kernel<T, VEC, 1, 0>, grid, kConvS1Threads, 0, s, col, out, Q);
+            else if (kw == 3 && pw == 1) launch_kernel(col2im_s1_kernel<T, VEC, 3, 1>, grid, kConvS1Threads, 0, s, col, out, Q);
+            else if (kw == 3 && pw == 0 && VEC > 2) launch_kernel(col2im_s1_kernel<T, VEC, 3, 0>, grid, kConvS1Threads, 0, s, col, out, Q);
+            else if (kw == 5 && pw == 2 && VEC > 2) launch_kernel(col2im_s1_kernel<T, VEC, 5, 2>, grid, kConvS1Threads, 0, s, col, out, Q);
+            else if (kw == 7 && pw == 3 && VEC > 3) launch_kernel(col2im_s1_kernel<T, VEC, 7, 3>, grid, kConvS1Threads, 0, s, col, out, Q);
             else done = false;
             if (done) {
                 check_launch(where);
@@ -420,7 +424,7 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
     const uint64_t col_plane = (uint64_t)P.KH * P.KW * P.OH * P.OW;
     const uint32_t pb = P.SH == 1 && P.SW == 1 && planes <= 0x7FFFFFFFull && col_plane && HW < 0x7FFFFFFFull ? planes_per_block(planes, col_plane * sizeof(T), 1, 48 * 1024) : 0;
     if (pb && pb * HW < 0x7FFFFFFFull && pb * HW >= kConvThreads / 2 && (HW <= kConvThreads || ((planes + pb - 1) / pb >= 512 && (sizeof(T) < 8 || P.KH * P.KW == 1)))) {
-        col2im_planes_kernel<T><<<(unsigned)((planes + pb - 1) / pb), kConvThreads, pb * col_plane * sizeof(T), s>>>(col, out, ConvPlanes(P, planes, pb));
+        launch_kernel(col2im_planes_kernel<T>, (unsigned)((planes + pb - 1) / pb), kConvThreads, pb * col_plane * sizeof(T), s, col, out, ConvPlanes(P, planes, pb));
         check_launch(where);
         return;
     }
@@ -432,7 +436,7 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
         // shift the views instead of the plane index: col entries of plane p start at p*KK*OHW
         const uint64_t col_shift = p0 * P.KH * P.KW * P.OH * P.OW;
         Q.num_els = num_els > col_shift ? num_els - col_shift : 0;
-        col2im_kernel<T><<<dim3(gx, (unsigned)cnt), kConvThreads, 0, s>>>(col + col_shift, out + p0 * HW, Q);
+        launch_kernel(col2im_kernel<T>, dim3(gx, (unsigned)cnt), kConvThreads, 0, s, col + col_shift, out + p0 * HW, Q);
     }
     check_launch(where);
 }

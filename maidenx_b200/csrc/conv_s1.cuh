@@ -32,7 +32,8 @@ __device__ __forceinline__ T window_at(const Vec<T, VEC>& lo, const Vec<T, VEC>&
 }
 
 template <class T, int VEC, int KW>
-__global__ void __launch_bounds__(kConvS1Threads) im2col_s1_kernel(const T* __restrict__ x, T* __restrict__ col, ConvS1Params P) {
+__global__ void __launch_bounds__(kConvS1Threads) im2col_s1_kernel(const T* x, T* col, ConvS1Params P) {
+    after_previous_kernel();
     extern __shared__ __align__(16) unsigned char conv_s1_smem[];
     T* plane = reinterpret_cast<T*>(conv_s1_smem);
     const uint64_t bc = blockIdx.x;
@@ -82,7 +83,7 @@ __device__ __forceinline__ T conv_s1_add(T a, T b) {
 // the window shift PW - KWI is a compile-time constant; the recursion walks kw from KW-1 down to 0
 // (w_out ascending).
 template <class T, int VEC, int KW, int PW, int KWI>
-__device__ __forceinline__ void col2im_s1_terms(const T* __restrict__ col, const ConvS1Params& P, uint64_t kh_base, uint32_t w0, uint32_t OHW,
+__device__ __forceinline__ void col2im_s1_terms(const T* col, const ConvS1Params& P, uint64_t kh_base, uint32_t w0, uint32_t OHW,
                                                 const Vec<T, VEC>& zero_vec, Vec<T, VEC>& sum) {
     // pixel w0 + j reads col column w0 + j + SH
     constexpr int SH = PW - KWI;                          // |SH| < VEC on this path
@@ -110,7 +111,8 @@ __device__ __forceinline__ void col2im_s1_terms(const T* __restrict__ col, const
 }
 
 template <class T, int VEC, int KW, int PW>
-__global__ void __launch_bounds__(kConvS1Threads) col2im_s1_kernel(const T* __restrict__ col, T* __restrict__ out, ConvS1Params P) {
+__global__ void __launch_bounds__(kConvS1Threads) col2im_s1_kernel(const T* col, T* out, ConvS1Params P) {
+    after_previous_kernel();
     const uint64_t bc = blockIdx.y;
     const uint32_t wv = P.W / VEC;  // output vectors per image row (W % VEC == 0 on this path)
     const uint32_t item = blockIdx.x * kConvS1Threads + threadIdx.x;
@@ -139,7 +141,8 @@ __global__ void __launch_bounds__(kConvS1Threads) col2im_s1_kernel(const T* __re
 // term walk as above (same order, same rounding).  Needs the whole column buffer readable (num_els covers every plane) and
 // KH * KW * OH * OW elements to fit the shared memory of at least two resident blocks.
 template <class T, int VEC, int KW, int PW>
-__global__ void __launch_bounds__(kConvS1Threads) col2im_s1_staged_kernel(const T* __restrict__ col, T* __restrict__ out, ConvS1Params P, tc::WaitReport rep) {
+__global__ void __launch_bounds__(kConvS1Threads) col2im_s1_staged_kernel(const T* col, T* out, ConvS1Params P, tc::WaitReport rep) {
+    after_previous_kernel();
     extern __shared__ __align__(128) unsigned char conv_s1_stage[];
     __shared__ __align__(8) unsigned long long stage_bar;
     const T* planes = reinterpret_cast<const T*>(conv_s1_stage);

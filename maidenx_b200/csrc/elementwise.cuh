@@ -134,6 +134,7 @@ __device__ __forceinline__ Vec<O, VEC> apply_vec(const F& f, const Vec<T, VEC>& 
 // sa / sb: 1 = contiguous, 0 = broadcast scalar
 template <class F, class T, class O, int NIN, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_flat_kernel(F f, const T* a, const T* b, O* out, uint64_t n, int sa, int sb) {
+    after_previous_kernel();
     constexpr uint64_t kChunk = (uint64_t)kEwThreads * VEC * kEwUnroll;
     const uint64_t base = (uint64_t)blockIdx.x * kChunk;
     if (base + kChunk <= n) {
@@ -217,6 +218,7 @@ __device__ __forceinline__ Vec<T, VEC> ld_vec_shifted(const T* p, uint32_t sh) {
 template <class F, class T, class O, int NIN, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_flat_shift_kernel(F f, const T* a, const T* b, O* out, uint64_t n, uint64_t head, uint64_t body_vecs,
                                                                    int sa, int sb, uint32_t sha, uint32_t shb) {
+    after_previous_kernel();
     const uint64_t v0 = (uint64_t)blockIdx.x * kEwThreads * kEwUnroll + threadIdx.x;
     Vec<T, VEC> va[kEwUnroll], vb[kEwUnroll];
 #pragma unroll
@@ -271,6 +273,7 @@ __device__ __forceinline__ bool ew_stage_wait(uint32_t bar, const tc::WaitReport
 template <class F, class T, class O, int NIN, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_flat_shift_staged_kernel(F f, const T* a, const T* b, O* out, uint64_t n, uint64_t head,
                                                                           uint64_t body_vecs, int sa, int sb, uint32_t sha, uint32_t shb, int stage_aligned, tc::WaitReport rep) {
+    after_previous_kernel();
     extern __shared__ __align__(128) unsigned char ew_stage[];
     __shared__ __align__(8) unsigned long long stage_bar;
     const uint64_t block_v0 = (uint64_t)blockIdx.x * kEwThreads * kEwUnroll;
@@ -374,6 +377,7 @@ struct EwRowParams {
 // index — the same instruction stream as the flat kernel.
 template <class F, class T, class O, int NIN, int VEC>
 __global__ void __launch_bounds__(kEwThreads, 4) ew_row_long_kernel(F f, const T* a, const T* b, O* out, EwRowParams P) {
+    after_previous_kernel();
     uint32_t r, chunk;
     P.chunk_div.divmod(blockIdx.x, r, chunk);
     int64_t o_out = 0, o_a = 0, o_b = 0;
@@ -421,6 +425,7 @@ __global__ void __launch_bounds__(kEwThreads, 4) ew_row_long_kernel(F f, const T
 // them to a slab of output rows — the kernel is a pure store stream.
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_bcast_rows_kernel(F f, const T* a, O* out, uint32_t qv, uint32_t rows, uint32_t rows_per_block) {
+    after_previous_kernel();
     const uint32_t v0 = blockIdx.x * (kEwThreads * kEwUnroll) + threadIdx.x;
     const uint32_t r0 = blockIdx.y * rows_per_block;
     const uint32_t r1 = min(rows, r0 + rows_per_block);
@@ -447,6 +452,7 @@ __global__ void __launch_bounds__(kEwThreads) ew_bcast_rows_kernel(F f, const T*
 // input type); rows are VEC * sizeof(O)-byte multiples here, so every copy is 16-byte aligned and sized.
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_bcast_rows_bulk_kernel(F f, const T* a, O* out, uint32_t qv, uint32_t rows, uint32_t rows_per_block) {
+    after_previous_kernel();
     extern __shared__ __align__(128) unsigned char ew_stage[];
     const uint32_t chunk_v0 = blockIdx.x * (kEwThreads * kEwUnroll);
     const uint32_t nv = min(qv - chunk_v0, (uint32_t)(kEwThreads * kEwUnroll));
@@ -477,6 +483,7 @@ __global__ void __launch_bounds__(kEwThreads) ew_bcast_rows_bulk_kernel(F f, con
 // Short rows: one fast-divmod per vector to find its row.
 template <class F, class T, class O, int NIN, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_row_kernel(F f, const T* a, const T* b, O* out, EwRowParams P) {
+    after_previous_kernel();
     const uint32_t base = blockIdx.x * (kEwThreads * kEwUnroll);
 #pragma unroll
     for (int u = 0; u < kEwUnroll; u++) {
@@ -538,6 +545,7 @@ __device__ __forceinline__ void ew_tile_coord(int i, int& row, int& vcol) {
 
 template <class F, class T, class O, int NIN, int VEC>
 __global__ void __launch_bounds__(kEwThreads, sizeof(T) == 2 ? 6 : 4) ew_tile_kernel(F f, const T* a, const T* b, O* out, EwTileParams P) {
+    after_previous_kernel();
     constexpr int TILE = EwTile<T>::kTile;
     constexpr int PITCH = EwTile<T>::kPitch;
     constexpr int VPR = TILE / VEC;                       // vectors per tile row
@@ -689,6 +697,7 @@ struct EwTile16Params {
 template <class F, class T, class O, int NIN>
 __global__ void __launch_bounds__(kEwThreads) ew_tile16_kernel(F f, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                                                const __grid_constant__ CUtensorMap map_o, EwTile16Params P, tc::WaitReport rep) {
+    after_previous_kernel();
     static_assert(sizeof(T) == 2 && sizeof(O) == 2, "2-byte elements on both sides");
     extern __shared__ unsigned char ew_smem_raw[];
     __shared__ __align__(8) unsigned long long tile_bar;
@@ -764,6 +773,7 @@ struct EwGenParams {
 
 template <class F, class T, class O, int NIN>
 __global__ void __launch_bounds__(kEwThreads) ew_generic_kernel(F f, const T* a, const T* b, O* out, EwGenParams P) {
+    after_previous_kernel();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.n; i += stride) {
         int64_t o0 = 0, o1 = 0, o2 = 0;
@@ -842,6 +852,7 @@ __device__ __forceinline__ void ew_dense_store(const F& f, O* out, const EwDense
 }
 template <class F, class T, class O, int NIN, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_dense_kernel(F f, const T* a, const T* b, O* out, EwDenseParams P) {
+    after_previous_kernel();
     auto row_offsets = [&](uint32_t r, int& oa, int& ob) {
         oa = ob = 0;
         for (int d = P.nd - 2; d > 0; d--) {
@@ -922,6 +933,7 @@ struct EwChanParams {
 constexpr int kEwChanUnroll = 4;
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, const T* b, O* out, EwChanParams P) {
+    after_previous_kernel();
     constexpr int U = kEwChanUnroll;
     const uint32_t first = (blockIdx.x * U * kEwThreads + threadIdx.x) * VEC;
     Vec<T, VEC> va[U], vb[U];
@@ -1010,7 +1022,7 @@ bool ew_launch_tile16(const EwPlan& pl, const EwTileParams& TP, uint32_t blocks,
         maps[2] = maps[1];
         P.transposed[2] = P.batched[2] = 0;
     }
-    ew_tile16_kernel<F, T, O, NIN><<<blocks, kEwThreads, (NIN + 1) * kEwT16Bytes + 1024, s>>>(f, maps[1], maps[2], maps[0], P, tc::next_wait_report());
+    launch_kernel(ew_tile16_kernel<F, T, O, NIN>, blocks, kEwThreads, (NIN + 1) * kEwT16Bytes + 1024, s, f, maps[1], maps[2], maps[0], P, tc::next_wait_report());
     return true;
 }
 
@@ -1037,12 +1049,11 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                 const int sa = (int)pl.st[1][0], sb = NIN == 2 ? (int)pl.st[2][0] : 0;
                 const int staged = (sa ? 1 : 0) + (sb ? 1 : 0);
                 if (staged && pl.n / VEC >= 4096) {
-                    ew_flat_shift_staged_kernel<F, T, O, NIN, VEC>
-                        <<<(uint32_t)blocks, kEwThreads, (size_t)staged * kEwStageBytes, s>>>(f, a, b, out, pl.n, 0, pl.n / VEC, sa, sb, 0, 0, 1, tc::next_wait_report());
+                    launch_kernel(ew_flat_shift_staged_kernel<F, T, O, NIN, VEC>, (uint32_t)blocks, kEwThreads, (size_t)staged * kEwStageBytes, s, f, a, b, out, pl.n, 0, pl.n / VEC, sa, sb, 0, 0, 1, tc::next_wait_report());
                     break;
                 }
             }
-            ew_flat_kernel<F, T, O, NIN, VEC><<<(uint32_t)blocks, kEwThreads, 0, s>>>(f, a, b, out, pl.n, (int)pl.st[1][0], NIN == 2 ? (int)pl.st[2][0] : 0);
+            launch_kernel(ew_flat_kernel<F, T, O, NIN, VEC>, (uint32_t)blocks, kEwThreads, 0, s, f, a, b, out, pl.n, (int)pl.st[1][0], NIN == 2 ? (int)pl.st[2][0] : 0);
             break;
         }
         case EW_FLAT_SHIFT: {
@@ -1064,11 +1075,10 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
             const int staged = (sa && sha != 0 ? 1 : 0) + (NIN == 2 && sb && shb != 0 ? 1 : 0);
             if (staged && body_vecs >= 4096) {
                 // large operands: the shifted ones go through shared memory, one bulk copy per block and operand
-                ew_flat_shift_staged_kernel<F, T, O, NIN, VEC>
-                    <<<(uint32_t)blocks, kEwThreads, (size_t)staged * kEwStageBytes, s>>>(f, a, b, out, pl.n, head, body_vecs, sa, sb, sha, shb, 0, tc::next_wait_report());
+                launch_kernel(ew_flat_shift_staged_kernel<F, T, O, NIN, VEC>, (uint32_t)blocks, kEwThreads, (size_t)staged * kEwStageBytes, s, f, a, b, out, pl.n, head, body_vecs, sa, sb, sha, shb, 0, tc::next_wait_report());
                 break;
             }
-            ew_flat_shift_kernel<F, T, O, NIN, VEC><<<(uint32_t)blocks, kEwThreads, 0, s>>>(f, a, b, out, pl.n, head, body_vecs, sa, sb, sha, shb);
+            launch_kernel(ew_flat_shift_kernel<F, T, O, NIN, VEC>, (uint32_t)blocks, kEwThreads, 0, s, f, a, b, out, pl.n, head, body_vecs, sa, sb, sha, shb);
             break;
         }
         case EW_ROW: {
@@ -1087,18 +1097,18 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                     gy = (uint32_t)((rows + rpb - 1) / rpb);
                     if ((VEC * sizeof(O)) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
                         const size_t stage = (size_t)kEwThreads * kEwUnroll * VEC * sizeof(O);
-                        ew_bcast_rows_bulk_kernel<F, T, O, VEC><<<dim3(P.chunks_per_row, gy), kEwThreads, stage, s>>>(f, a, out, P.qv, (uint32_t)rows, rpb);
+                        launch_kernel(ew_bcast_rows_bulk_kernel<F, T, O, VEC>, dim3(P.chunks_per_row, gy), kEwThreads, stage, s, f, a, out, P.qv, (uint32_t)rows, rpb);
                         break;
                     }
-                    ew_bcast_rows_kernel<F, T, O, VEC><<<dim3(P.chunks_per_row, gy), kEwThreads, 0, s>>>(f, a, out, P.qv, (uint32_t)rows, rpb);
+                    launch_kernel(ew_bcast_rows_kernel<F, T, O, VEC>, dim3(P.chunks_per_row, gy), kEwThreads, 0, s, f, a, out, P.qv, (uint32_t)rows, rpb);
                     break;
                 }
             }
             if (P.qv >= (uint32_t)kEwThreads && rows * P.chunks_per_row < 0x7FFFFFFFull) {
-                ew_row_long_kernel<F, T, O, NIN, VEC><<<(uint32_t)(rows * P.chunks_per_row), kEwThreads, 0, s>>>(f, a, b, out, P);
+                launch_kernel(ew_row_long_kernel<F, T, O, NIN, VEC>, (uint32_t)(rows * P.chunks_per_row), kEwThreads, 0, s, f, a, b, out, P);
             } else {
                 uint32_t blocks = ceil_div_u32(P.total_vecs, kEwThreads * kEwUnroll);
-                ew_row_kernel<F, T, O, NIN, VEC><<<blocks, kEwThreads, 0, s>>>(f, a, b, out, P);
+                launch_kernel(ew_row_kernel<F, T, O, NIN, VEC>, blocks, kEwThreads, 0, s, f, a, b, out, P);
             }
             break;
         }
@@ -1111,8 +1121,8 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
             if constexpr (sizeof(T) == 2 && sizeof(O) == 2) {
                 if (pl.vec && ew_launch_tile16<F, T, O, NIN>(pl, P, blocks, f, a, b, out, s)) break;
             }
-            if (pl.vec) ew_tile_kernel<F, T, O, NIN, VEC><<<blocks, kEwThreads, smem, s>>>(f, a, b, out, P);
-            else ew_tile_kernel<F, T, O, NIN, 1><<<blocks, kEwThreads, smem, s>>>(f, a, b, out, P);
+            if (pl.vec) launch_kernel(ew_tile_kernel<F, T, O, NIN, VEC>, blocks, kEwThreads, smem, s, f, a, b, out, P);
+            else launch_kernel(ew_tile_kernel<F, T, O, NIN, 1>, blocks, kEwThreads, smem, s, f, a, b, out, P);
             break;
         }
         case EW_GENERIC:
@@ -1123,22 +1133,22 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                 if constexpr (NIN == 2 && VEC <= 8) {  // 16 elements a vector would take 145 registers
                     EwChanParams C;
                     if (ew_fill_chan_params(D, VEC, C)) {
-                        ew_chan_kernel<F, T, O, VEC><<<(uint32_t)((vecs + kEwThreads * kEwChanUnroll - 1) / (kEwThreads * kEwChanUnroll)), kEwThreads, 0, s>>>(f, a, b, out, C);
+                        launch_kernel(ew_chan_kernel<F, T, O, VEC>, (uint32_t)((vecs + kEwThreads * kEwChanUnroll - 1) / (kEwThreads * kEwChanUnroll)), kEwThreads, 0, s, f, a, b, out, C);
                         break;
                     }
                 }
-                ew_dense_kernel<F, T, O, NIN, VEC><<<(uint32_t)((vecs + kEwThreads * kEwDenseUnroll - 1) / (kEwThreads * kEwDenseUnroll)), kEwThreads, 0, s>>>(f, a, b, out, D);
+                launch_kernel(ew_dense_kernel<F, T, O, NIN, VEC>, (uint32_t)((vecs + kEwThreads * kEwDenseUnroll - 1) / (kEwThreads * kEwDenseUnroll)), kEwThreads, 0, s, f, a, b, out, D);
                 break;
             }
             EwGenParams P;
             ew_fill_gen_params(pl, P);
             if (pl.kind == EW_SERIAL) {
-                ew_generic_kernel<F, T, O, NIN><<<1, 1, 0, s>>>(f, a, b, out, P);
+                launch_kernel(ew_generic_kernel<F, T, O, NIN>, 1, 1, 0, s, f, a, b, out, P);
             } else {
                 uint64_t blocks = (pl.n + kEwThreads - 1) / kEwThreads;
                 uint64_t cap = (uint64_t)sm_count() * 32;
                 if (blocks > cap) blocks = cap;
-                ew_generic_kernel<F, T, O, NIN><<<(uint32_t)blocks, kEwThreads, 0, s>>>(f, a, b, out, P);
+                launch_kernel(ew_generic_kernel<F, T, O, NIN>, (uint32_t)blocks, kEwThreads, 0, s, f, a, b, out, P);
             }
             break;
         }

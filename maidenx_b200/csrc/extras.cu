@@ -641,6 +641,7 @@ __device__ __forceinline__ u64 softmax_index(const SoftmaxParams& P, u64 pre_idx
 
 template <class T>
 __global__ void __launch_bounds__(kExThreads) softmax_kernel(const T* in, T* out, SoftmaxParams P) {
+    after_previous_kernel();
     typedef typename std::conditional<std::is_same<T, f64>::value, f64, f32>::type A;
     typedef RedTraits<A, RED_MAX> MaxT;
     typedef RedTraits<A, RED_SUM> SumT;
@@ -714,6 +715,7 @@ __device__ __forceinline__ A softmax_group_all(A v, A* part) {
 
 template <class T, int G, int K>
 __global__ void __launch_bounds__(kExThreads, (K * 16 / (int)sizeof(T) <= 32) ? 5 : 1) softmax_rows_kernel(const T* __restrict__ in, T* __restrict__ out, u64 rows, u32 n) {
+    after_previous_kernel();
     typedef typename std::conditional<std::is_same<T, f64>::value, f64, f32>::type A;
     constexpr int VEC = 16 / (int)sizeof(T);
     __shared__ A part_max[kExThreads / 32], part_sum[kExThreads / 32];
@@ -783,7 +785,8 @@ __global__ void __launch_bounds__(kExThreads, (K * 16 / (int)sizeof(T) <= 32) ? 
 // else 32 lanes of single elements - with 256 / LANES threads per column group, which take every (256 / LANES)-th
 // element of the dim, four loads in flight each, and combine through shared memory; three passes as in the general kernel.
 template <class T, int VEC, int LANES>
-__global__ void __launch_bounds__(kExThreads) softmax_cols_kernel(const T* __restrict__ in, T* __restrict__ out, u64 pre, u64 n, u64 post) {
+__global__ void __launch_bounds__(kExThreads) softmax_cols_kernel(const T* in, T* out, u64 pre, u64 n, u64 post) {
+    after_previous_kernel();
     typedef typename std::conditional<std::is_same<T, f64>::value, f64, f32>::type A;
     constexpr int kSmColLanes = LANES, kSmColRows = kExThreads / LANES;
     __shared__ A part[kSmColRows][kSmColLanes][VEC];
@@ -867,7 +870,8 @@ __global__ void __launch_bounds__(kExThreads) softmax_cols_kernel(const T* __res
 // way, the error against 64 bits stays the same to six digits (f16 2.0124e-4, bf16 1.6048e-3 at [37824, 197]).  Bound by HBM / L2 with a
 // 64-byte (16-bit) or 128-byte request per warp and load: [192 x 197, 197] bf16 9.9 us, 109 in the general kernel.
 template <class T, int G, int K>
-__global__ void __launch_bounds__(kExThreads) softmax_rows_any_kernel(const T* __restrict__ in, T* __restrict__ out, u64 rows, u32 n) {
+__global__ void __launch_bounds__(kExThreads) softmax_rows_any_kernel(const T* in, T* out, u64 rows, u32 n) {
+    after_previous_kernel();
     typedef typename std::conditional<std::is_same<T, f64>::value, f64, f32>::type A;
     __shared__ A part_max[kExThreads / 32], part_sum[kExThreads / 32];
     const u32 t = threadIdx.x % G;
@@ -915,7 +919,8 @@ __global__ void __launch_bounds__(kExThreads) softmax_rows_any_kernel(const T* _
 // VEC neighbouring columns, so each element is read once instead of three times, with the formulas of softmax_cols_kernel.
 // The widest strip whose columns fit: 128, 64 or 32 bytes of each row.
 template <class T, int VEC, int LANES, int K>
-__global__ void __launch_bounds__(kExThreads) softmax_cols_reg_kernel(const T* __restrict__ in, T* __restrict__ out, u64 pre, u32 n, u64 post) {
+__global__ void __launch_bounds__(kExThreads) softmax_cols_reg_kernel(const T* in, T* out, u64 pre, u32 n, u64 post) {
+    after_previous_kernel();
     typedef typename std::conditional<std::is_same<T, f64>::value, f64, f32>::type A;
     constexpr int ROWS = kExThreads / LANES;
     __shared__ A part[kExThreads / 32][LANES][VEC];
@@ -1005,9 +1010,9 @@ bool softmax_cols_reg_launch(const T* in, T* out, u64 pre, u64 n, u64 post, cuda
     const u64 per = (n + ROWS - 1) / ROWS;
     if ((LANES < 8 || per > KMAX / 2) && pre * post / (8 * VEC) > (LANES < 8 ? 2 : 4) * (u64)sm_count()) return false;
     const unsigned blocks = (unsigned)((pre * post / VEC + LANES - 1) / LANES);
-    if (per <= KMAX / 4) softmax_cols_reg_kernel<T, VEC, LANES, KMAX / 4><<<blocks, kExThreads, 0, s>>>(in, out, pre, (u32)n, post);
-    else if (per <= KMAX / 2) softmax_cols_reg_kernel<T, VEC, LANES, KMAX / 2><<<blocks, kExThreads, 0, s>>>(in, out, pre, (u32)n, post);
-    else if (per <= KMAX) softmax_cols_reg_kernel<T, VEC, LANES, KMAX><<<blocks, kExThreads, 0, s>>>(in, out, pre, (u32)n, post);
+    if (per <= KMAX / 4) launch_kernel(softmax_cols_reg_kernel<T, VEC, LANES, KMAX / 4>, blocks, kExThreads, 0, s, in, out, pre, (u32)n, post);
+    else if (per <= KMAX / 2) launch_kernel(softmax_cols_reg_kernel<T, VEC, LANES, KMAX / 2>, blocks, kExThreads, 0, s, in, out, pre, (u32)n, post);
+    else if (per <= KMAX) launch_kernel(softmax_cols_reg_kernel<T, VEC, LANES, KMAX>, blocks, kExThreads, 0, s, in, out, pre, (u32)n, post);
     else return false;
     return true;
 }
@@ -1016,12 +1021,12 @@ template <class T, int G>
 bool softmax_rows_any_launch(const T* in, T* out, u64 rows, u32 n, cudaStream_t s) {
     const u32 per = (n + G - 1) / G;  // elements per thread
     const unsigned blocks = (unsigned)((rows + kExThreads / G - 1) / (kExThreads / G));
-    if (per <= 2) softmax_rows_any_kernel<T, G, 2><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (per <= 4) softmax_rows_any_kernel<T, G, 4><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (per <= 8) softmax_rows_any_kernel<T, G, 8><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (per <= 16) softmax_rows_any_kernel<T, G, 16><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (per <= 32) softmax_rows_any_kernel<T, G, 32><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (is_half_v<T> && per <= 64) softmax_rows_any_kernel<T, G, is_half_v<T> ? 64 : 16><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
+    if (per <= 2) launch_kernel(softmax_rows_any_kernel<T, G, 2>, blocks, kExThreads, 0, s, in, out, rows, n);
+    else if (per <= 4) launch_kernel(softmax_rows_any_kernel<T, G, 4>, blocks, kExThreads, 0, s, in, out, rows, n);
+    else if (per <= 8) launch_kernel(softmax_rows_any_kernel<T, G, 8>, blocks, kExThreads, 0, s, in, out, rows, n);
+    else if (per <= 16) launch_kernel(softmax_rows_any_kernel<T, G, 16>, blocks, kExThreads, 0, s, in, out, rows, n);
+    else if (per <= 32) launch_kernel(softmax_rows_any_kernel<T, G, 32>, blocks, kExThreads, 0, s, in, out, rows, n);
+    else if (is_half_v<T> && per <= 64) launch_kernel(softmax_rows_any_kernel<T, G, is_half_v<T> ? 64 : 16>, blocks, kExThreads, 0, s, in, out, rows, n);
     else return false;
     return true;
 }
@@ -1032,11 +1037,11 @@ bool softmax_rows_launch(const T* in, T* out, u64 rows, u32 n, cudaStream_t s) {
     constexpr int KMAX = sizeof(T) == 2 ? 8 : 16;  // at most 64 values per thread
     const u32 vecs = (n / VEC + G - 1) / G;          // vectors per thread
     const unsigned blocks = (unsigned)((rows + kExThreads / G - 1) / (kExThreads / G));
-    if (vecs <= 1) softmax_rows_kernel<T, G, 1><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (vecs <= 2) softmax_rows_kernel<T, G, 2><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (vecs <= 4) softmax_rows_kernel<T, G, 4><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (vecs <= 8) softmax_rows_kernel<T, G, 8><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
-    else if (KMAX >= 16 && vecs <= 16) softmax_rows_kernel<T, G, (KMAX >= 16 ? 16 : 8)><<<blocks, kExThreads, 0, s>>>(in, out, rows, n);
+    if (vecs <= 1) launch_kernel(softmax_rows_kernel<T, G, 1>, blocks, kExThreads, 0, s, in, out, rows, n);
+    else if (vecs <= 2) launch_kernel(softmax_rows_kernel<T, G, 2>, blocks, kExThreads, 0, s, in, out, rows, n);
+    else if (vecs <= 4) launch_kernel(softmax_rows_kernel<T, G, 4>, blocks, kExThreads, 0, s, in, out, rows, n);
+    else if (vecs <= 8) launch_kernel(softmax_rows_kernel<T, G, 8>, blocks, kExThreads, 0, s, in, out, rows, n);
+    else if (KMAX >= 16 && vecs <= 16) launch_kernel(softmax_rows_kernel<T, G, (KMAX >= 16 ? 16 : 8)>, blocks, kExThreads, 0, s, in, out, rows, n);
     else return false;
     return true;
 }
@@ -1108,14 +1113,14 @@ void softmax_entry(size_t num_els, size_t nd, size_t dim, const size_t* meta, co
                 check_launch(where);
                 return;
             }
-            if (wide) softmax_cols_kernel<T, VEC, 8><<<(unsigned)((slices / VEC + 7) / 8), kExThreads, 0, st>>>(src, out, P.pre, P.n, P.post);
-            else softmax_cols_kernel<T, 1, 32><<<(unsigned)((slices + 31) / 32), kExThreads, 0, st>>>(src, out, P.pre, P.n, P.post);
+            if (wide) launch_kernel(softmax_cols_kernel<T, VEC, 8>, (unsigned)((slices / VEC + 7) / 8), kExThreads, 0, st, src, out, P.pre, P.n, P.post);
+            else launch_kernel(softmax_cols_kernel<T, 1, 32>, (unsigned)((slices + 31) / 32), kExThreads, 0, st, src, out, P.pre, P.n, P.post);
             check_launch(where);
             return;
         }
     }
     u64 blocks = slices < (u64)sm_count() * 16 ? slices : (u64)sm_count() * 16;
-    softmax_kernel<T><<<(unsigned)blocks, kExThreads, 0, ctx().stream>>>(in, out, P);
+    launch_kernel(softmax_kernel<T>, (unsigned)blocks, kExThreads, 0, ctx().stream, in, out, P);
     check_launch(where);
 }
 

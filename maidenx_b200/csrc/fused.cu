@@ -42,8 +42,9 @@ __device__ __forceinline__ float gelu_fwd(float x) {
 // u = round(z + b), a = round(gelu(u)); `a` may be NULL (bias add only).  The sum is rounded to
 // T before the activation, exactly as the two separate ops would.
 template <class T>
-__global__ void __launch_bounds__(kFusedThreads) bias_gelu_kernel(const T* __restrict__ z, const T* __restrict__ bias, T* __restrict__ u,
-                                                                 T* __restrict__ a, uint64_t n) {
+__global__ void __launch_bounds__(kFusedThreads) bias_gelu_kernel(const T* z, const T* bias, T* u,
+                                                                 T* a, uint64_t n) {
+    after_previous_kernel();
     constexpr int VEC = 16 / sizeof(T);
     const float b = ld_scalar_f32(bias);
     const uint64_t nvec = n / VEC;
@@ -112,8 +113,9 @@ __device__ __forceinline__ bool fused_last_block(uint32_t* arrived) {
 // SUM: the sum of du (the bias gradient), which a pass over du used to read it back for.  Two vectors of each operand in flight
 // per thread.
 template <class T, bool SUM>
-__global__ void __launch_bounds__(kFusedThreads) gelu_backward_kernel(const T* __restrict__ dy, const T* __restrict__ u, T* __restrict__ du,
-                                                                     uint64_t n, float* __restrict__ partial, uint32_t* arrived, T* grad_sum) {
+__global__ void __launch_bounds__(kFusedThreads) gelu_backward_kernel(const T* dy, const T* u, T* du,
+                                                                     uint64_t n, float* partial, uint32_t* arrived, T* grad_sum) {
+    after_previous_kernel();
     float acc = 0.0f;
     constexpr int VEC = 16 / sizeof(T), UN = 2;
     const uint64_t nvec = n / VEC;
@@ -171,9 +173,10 @@ __device__ __forceinline__ float mse_fold(const float* partial, uint32_t count) 
 
 // grad = 2 (p - t) / n, per-block partial sums of (p - t)^2 into `partial` and, with SUM, of grad behind them; with SUM the last block folds both.
 template <class T, bool SUM>
-__global__ void __launch_bounds__(kFusedThreads) mse_kernel(const T* __restrict__ p, const T* __restrict__ t, T* __restrict__ grad,
-                                                           float* __restrict__ partial, uint64_t n, float two_over_n, float inv_n, float* loss,
+__global__ void __launch_bounds__(kFusedThreads) mse_kernel(const T* p, const T* t, T* grad,
+                                                           float* partial, uint64_t n, float two_over_n, float inv_n, float* loss,
                                                            T* grad_sum, uint32_t* arrived) {
+    after_previous_kernel();
     constexpr int VEC = 16 / sizeof(T);
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
@@ -228,14 +231,16 @@ __global__ void __launch_bounds__(kFusedThreads) mse_kernel(const T* __restrict_
     }
 }
 // Without an arrival word (the exported pass, whose caller has none): the loss folded by a launch of one block.
-__global__ void __launch_bounds__(kFusedThreads) mse_finish_kernel(const float* __restrict__ partial, int count, float inv_n, float* __restrict__ loss) {
+__global__ void __launch_bounds__(kFusedThreads) mse_finish_kernel(const float* partial, int count, float inv_n, float* loss) {
+    after_previous_kernel();
     const float l = mse_fold(partial, (uint32_t)count);
     if (threadIdx.x == 0) *loss = l * inv_n;
 }
 
 template <class T>
-__global__ void __launch_bounds__(kFusedThreads) sgd_kernel(float* __restrict__ w32, const T* __restrict__ g, T* __restrict__ w16, uint64_t n,
-                                                           float step, float* __restrict__ b32, const T* __restrict__ gb, T* __restrict__ b16) {
+__global__ void __launch_bounds__(kFusedThreads) sgd_kernel(float* w32, const T* g, T* w16, uint64_t n,
+                                                           float step, float* b32, const T* gb, T* b16) {
+    after_previous_kernel();
     constexpr int VEC = 16 / sizeof(T);  // elements per 16-byte vector of the gradient; w32 moves as VEC floats
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
@@ -291,7 +296,7 @@ void bias_gelu_launch(size_t n, const T* z, const T* bias, T* u, T* a, const cha
         set_error(kErrUnsupported, 0, where);
         return;
     }
-    bias_gelu_kernel<T><<<fused_grid(n, 16 / sizeof(T)), kFusedThreads, 0, ctx().stream>>>(z, bias, u, a, n);
+    launch_kernel(bias_gelu_kernel<T>, fused_grid(n, 16 / sizeof(T)), kFusedThreads, 0, ctx().stream, z, bias, u, a, n);
     check_launch(where);
 }
 template <class T>
@@ -303,11 +308,11 @@ void gelu_backward_launch(size_t n, const T* dy, const T* u, T* du, T* grad_sum,
     }
     const unsigned blocks = fused_grid(n, 16 / sizeof(T));
     if (!grad_sum) {
-        gelu_backward_kernel<T, false><<<blocks, kFusedThreads, 0, ctx().stream>>>(dy, u, du, n, nullptr, nullptr, nullptr);
+        launch_kernel(gelu_backward_kernel<T, false>, blocks, kFusedThreads, 0, ctx().stream, dy, u, du, n, nullptr, nullptr, nullptr);
     } else {
         float* partial = static_cast<float*>(scratch(sizeof(float) * blocks));
         if (!partial) return;
-        gelu_backward_kernel<T, true><<<blocks, kFusedThreads, 0, ctx().stream>>>(dy, u, du, n, partial, arrived, grad_sum);
+        launch_kernel(gelu_backward_kernel<T, true>, blocks, kFusedThreads, 0, ctx().stream, dy, u, du, n, partial, arrived, grad_sum);
     }
     check_launch(where);
 }
@@ -323,10 +328,10 @@ void mse_launch(size_t n, const T* p, const T* t, T* grad, float* loss, T* grad_
     if (!partial) return;
     const float two_over_n = 2.0f / (float)n, inv_n = 1.0f / (float)n;
     if (grad_sum) {
-        mse_kernel<T, true><<<blocks, kFusedThreads, 0, ctx().stream>>>(p, t, grad, partial, n, two_over_n, inv_n, loss, grad_sum, arrived);
+        launch_kernel(mse_kernel<T, true>, blocks, kFusedThreads, 0, ctx().stream, p, t, grad, partial, n, two_over_n, inv_n, loss, grad_sum, arrived);
     } else {
-        mse_kernel<T, false><<<blocks, kFusedThreads, 0, ctx().stream>>>(p, t, grad, partial, n, two_over_n, inv_n, nullptr, nullptr, nullptr);
-        mse_finish_kernel<<<1, kFusedThreads, 0, ctx().stream>>>(partial, (int)blocks, inv_n, loss);
+        launch_kernel(mse_kernel<T, false>, blocks, kFusedThreads, 0, ctx().stream, p, t, grad, partial, n, two_over_n, inv_n, nullptr, nullptr, nullptr);
+        launch_kernel(mse_finish_kernel, 1, kFusedThreads, 0, ctx().stream, partial, (int)blocks, inv_n, loss);
     }
     check_launch(where);
 }
@@ -337,7 +342,7 @@ void sgd_launch(size_t n, float* w32, const T* g, T* w16, float lr, float grad_s
         set_error(kErrUnsupported, 0, where);
         return;
     }
-    sgd_kernel<T><<<fused_grid(n, 16 / sizeof(T)), kFusedThreads, 0, ctx().stream>>>(w32, g, w16, n, lr * grad_scale, b32, gb, b16);
+    launch_kernel(sgd_kernel<T>, fused_grid(n, 16 / sizeof(T)), kFusedThreads, 0, ctx().stream, w32, g, w16, n, lr * grad_scale, b32, gb, b16);
     check_launch(where);
 }
 

@@ -55,7 +55,8 @@ constexpr int kMmThreads = 256;
 // the next k-step's operands are on their way from memory while the current one is multiplied.  Bound by that latency
 // for small products, by the separate multiply and add for large ones.  f32: 64 x 64 x 512 17 us (163 before), 256 x 256 x 128 5.8 (42).
 template <class T, int TILE>
-__global__ void __launch_bounds__(kMmThreads) matmul_simt_kernel(const T* __restrict__ X, const T* __restrict__ Y, T* __restrict__ out, MmParams P, uint32_t tiles_m, uint64_t first) {
+__global__ void __launch_bounds__(kMmThreads) matmul_simt_kernel(const T* X, const T* Y, T* out, MmParams P, uint32_t tiles_m, uint64_t first) {
+    after_previous_kernel();
     typedef typename MmAcc<T>::type Acc;
     constexpr int kMmK = TILE == 32 ? (sizeof(Acc) == 8 ? 32 : 64) : 16;  // reduction step: the narrow tile is for products with few blocks, which wait for memory once per step
     constexpr int PER = TILE / 16, LOADS = TILE * kMmK / kMmThreads;
@@ -144,7 +145,8 @@ __global__ void __launch_bounds__(kMmThreads) matmul_simt_kernel(const T* __rest
 // memory, the others read their Y element by element, which short reductions of a few rows a batch cost less than a block a
 // batch does ([16000] x 1 x 1 x 16 f32: 16 us, 144 with a block each).  Which one: simt_rows_pay.  The order of additions is the same.
 template <class T>
-__global__ void __launch_bounds__(kMmThreads) matmul_simt_rows_kernel(const T* __restrict__ X, const T* __restrict__ Y, T* __restrict__ out, MmParams P) {
+__global__ void __launch_bounds__(kMmThreads) matmul_simt_rows_kernel(const T* X, const T* Y, T* out, MmParams P) {
+    after_previous_kernel();
     typedef typename MmAcc<T>::type Acc;
     constexpr int TILE = 64, STEP = 16;
     __shared__ Acc xs[STEP][TILE + 1];  // [r][row]
@@ -273,7 +275,8 @@ inline bool simt_rows_pay(uint64_t rows, uint64_t M, uint64_t N, uint64_t K) {
 // shuffle tree, so the result is reproducible; integers stay exact (wrapping addition is associative), floats are summed
 // in a different order than the element-type loop of the reference and agree with it within the reduction tolerance.
 template <class T>
-__global__ void __launch_bounds__(kMmThreads) matmul_longk_kernel(const T* __restrict__ X, const T* __restrict__ Y, T* __restrict__ out, MmParams P) {
+__global__ void __launch_bounds__(kMmThreads) matmul_longk_kernel(const T* X, const T* Y, T* out, MmParams P) {
+    after_previous_kernel();
     typedef typename MmAcc<T>::type Acc;
     const uint64_t o = blockIdx.x;
     const uint64_t row = o / P.N, col = o % P.N;
@@ -321,14 +324,14 @@ template <class T>
 void mm_launch(const MmParams& P, const T* X, const T* Y, T* out, const char* where) {
     if (P.rows == 0 || P.N == 0) return;
     if (P.K >= kLongKMinK && P.out_elems <= kLongKMaxOutputs && P.rows * P.N <= kLongKMaxOutputs) {
-        matmul_longk_kernel<T><<<(unsigned)P.out_elems, kMmThreads, 0, ctx().stream>>>(X, Y, out, P);
+        launch_kernel(matmul_longk_kernel<T>, (unsigned)P.out_elems, kMmThreads, 0, ctx().stream, X, Y, out, P);
         check_launch(where);
         return;
     }
     if (P.M && simt_rows_pay(P.rows, P.M, P.N, P.K)) {
         const uint64_t gx = (P.rows + 63) / 64, gy = (P.N + 63) / 64;
         if (gy <= 65535 && gx <= 0x7FFFFFFFull) {
-            matmul_simt_rows_kernel<T><<<dim3((unsigned)gx, (unsigned)gy), kMmThreads, 0, ctx().stream>>>(X, Y, out, P);
+            launch_kernel(matmul_simt_rows_kernel<T>, dim3((unsigned)gx, (unsigned)gy), kMmThreads, 0, ctx().stream, X, Y, out, P);
             check_launch(where);
             return;
         }
@@ -342,7 +345,7 @@ void mm_launch(const MmParams& P, const T* X, const T* Y, T* out, const char* wh
         }
         for (uint64_t first = 0; first < gx; first += 0x7FFFFFFFull) {
             const uint64_t count = gx - first < 0x7FFFFFFFull ? gx - first : 0x7FFFFFFFull;
-            kernel<<<dim3((unsigned)count, (unsigned)gy), kMmThreads, 0, ctx().stream>>>(X, Y, out, P, (uint32_t)tiles_m, first);
+            launch_kernel(kernel, dim3((unsigned)count, (unsigned)gy), kMmThreads, 0, ctx().stream, X, Y, out, P, (uint32_t)tiles_m, first);
         }
         check_launch(where);
     };

@@ -297,6 +297,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    after_previous_kernel();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -954,8 +955,9 @@ int splitk_short(uint64_t tiles, uint64_t num_kb, int sms, double kb_cost, doubl
 
 // `vec` elements per step: 4 when the output's rows are whole vectors (then rows and padded rows coincide), else 1.
 template <class T, int VEC>
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, int slices, size_t rows, uint32_t cols, uint32_t pitch, FastDiv div,
-                                                            T* __restrict__ out) {
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* partial, int slices, size_t rows, uint32_t cols, uint32_t pitch, FastDiv div,
+                                                            T* out) {
+    after_previous_kernel();
     const size_t nvec = rows * cols / VEC, stride = (size_t)gridDim.x * 256, slice = rows * pitch;
     for (size_t v = (size_t)blockIdx.x * 256 + threadIdx.x; v < nvec; v += stride) {
         size_t src = VEC * v;
@@ -988,8 +990,8 @@ static void splitk_reduce_t(const float* partial, int slices, uint64_t rows, uin
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     const FastDiv div((uint32_t)cols);
-    if (vec) splitk_reduce_kernel<T, 4><<<(unsigned)blocks, 256, 0, ctx().stream>>>(partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out));
-    else splitk_reduce_kernel<T, 1><<<(unsigned)blocks, 256, 0, ctx().stream>>>(partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out));
+    if (vec) launch_kernel(splitk_reduce_kernel<T, 4>, (unsigned)blocks, 256, 0, ctx().stream, partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out));
+    else launch_kernel(splitk_reduce_kernel<T, 1>, (unsigned)blocks, 256, 0, ctx().stream, partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out));
 }
 
 void splitk_reduce(int dtype, const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out, const char* where) {
@@ -1004,7 +1006,8 @@ void splitk_reduce(int dtype, const float* partial, int slices, uint64_t rows, u
 // source it straddles.  The words read all hold at least one element of the vector, so nothing outside the aligned words
 // of the source's own elements is touched.  Bound by HBM (or L2): reads and writes the operand once.
 template <class W>
-__global__ void __launch_bounds__(256) repack_rows_kernel(const W* __restrict__ in, W* __restrict__ out, uint32_t vecs, FastDiv per_row, uint32_t cols, uint32_t pitch) {
+__global__ void __launch_bounds__(256) repack_rows_kernel(const W* in, W* out, uint32_t vecs, FastDiv per_row, uint32_t cols, uint32_t pitch) {
+    after_previous_kernel();
     constexpr uint32_t VEC = 16 / sizeof(W);
     const uint32_t stride = gridDim.x * 256;
     for (uint32_t v = blockIdx.x * 256 + threadIdx.x; v < vecs; v += stride) {
@@ -1049,10 +1052,10 @@ static bool repack_rows(size_t es, const void* in, void* out, uint64_t rows, uin
     if (blocks > cap) blocks = cap;
     const FastDiv div((uint32_t)per_row);
     if (es == 2)
-        repack_rows_kernel<uint16_t><<<(unsigned)blocks, 256, 0, ctx().stream>>>(static_cast<const uint16_t*>(in), static_cast<uint16_t*>(out), (uint32_t)vecs, div, (uint32_t)cols,
+        launch_kernel(repack_rows_kernel<uint16_t>, (unsigned)blocks, 256, 0, ctx().stream, static_cast<const uint16_t*>(in), static_cast<uint16_t*>(out), (uint32_t)vecs, div, (uint32_t)cols,
                                                                                  (uint32_t)pitch);
     else
-        repack_rows_kernel<uint32_t><<<(unsigned)blocks, 256, 0, ctx().stream>>>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), (uint32_t)vecs, div, (uint32_t)cols,
+        launch_kernel(repack_rows_kernel<uint32_t>, (unsigned)blocks, 256, 0, ctx().stream, static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), (uint32_t)vecs, div, (uint32_t)cols,
                                                                                  (uint32_t)pitch);
     return true;
 }

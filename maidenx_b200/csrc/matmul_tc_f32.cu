@@ -252,6 +252,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    after_previous_kernel();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer

@@ -203,6 +203,7 @@ __device__ __forceinline__ typename TR::Acc fold_published(const typename TR::Ac
 template <class T, int KIND, int VEC>
 __global__ void __launch_bounds__(kRedThreads) reduce_rows_block_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial,
                                                                       u64 R, u64 seg, u32 splits, u64 factor, u32* counters, int tree_fold) {
+    after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
     typedef typename TR::Acc Acc;
     const u64 row = blockIdx.y;
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_block_kernel(const T*
 // 124 us with a warp per row, 55 with eight lanes and one row, 32 with eight lanes and four).
 template <class T, int KIND, int VEC, int G, int Q>
 __global__ void __launch_bounds__(kRedThreads) reduce_rows_short_kernel(const T* in, T* out, u64 rows, u32 R, u64 factor) {
+    after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
     constexpr u32 ROWS = kRedThreads / G;  // rows a block has in one step
     const u64 row0 = (u64)blockIdx.x * ROWS * Q + threadIdx.x / G;
@@ -265,6 +267,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_short_kernel(const T*
 // more than they gave (100000 rows of 1023 bf16: 59 us, 46 like this), lanes that leave at different trips the ragged ones.
 template <class T, int KIND, int VEC>
 __global__ void __launch_bounds__(kRedThreads) reduce_rows_warp_kernel(const T* in, T* out, u64 rows, u32 R, u64 factor) {
+    after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
     const u64 row = (u64)blockIdx.x * (kRedThreads / 32) + threadIdx.x / 32;
     if (row >= rows) return;
@@ -299,6 +302,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_warp_kernel(const T* 
 // One thread per row (R < 32, see red_launch).
 template <class T, int KIND>
 __global__ void __launch_bounds__(kRedThreads) reduce_rows_thread_kernel(const T* in, T* out, u64 rows, u64 R, u64 factor) {
+    after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
     const u64 row = (u64)blockIdx.x * kRedThreads + threadIdx.x;
     if (row >= rows) return;
@@ -313,6 +317,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_thread_kernel(const T
 template <class T, int KIND>
 __global__ void __launch_bounds__(kRedThreads) reduce_partials_kernel(const typename RedTraits<T, KIND>::Acc* partial, T* out, u64 count,
                                                                     u32 S, int cols_layout, u64 factor) {
+    after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
     const u64 j = (u64)blockIdx.x * kRedThreads + threadIdx.x;
     if (j >= count) return;
@@ -329,6 +334,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_partials_kernel(const type
 // split over ~1000 blocks): threads stride over the partials, then a fixed-shape block tree.
 template <class T, int KIND>
 __global__ void __launch_bounds__(kRedThreads) reduce_partials_block_kernel(const typename RedTraits<T, KIND>::Acc* partial, T* out, u32 S, u64 factor) {
+    after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
     const u64 j = blockIdx.x;
     typename TR::Acc acc = TR::init();
@@ -348,6 +354,7 @@ constexpr int kColRows = 8;    // threads along the reduced dim
 template <class T, int KIND, int VEC>
 __global__ void __launch_bounds__(kColLanes* kColRows) reduce_cols_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial, u64 O,
                                                                          u64 R, u64 I, u64 seg, u32 splits, u64 factor, u32* counters) {
+    after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
     typedef typename TR::Acc Acc;
     __shared__ Acc sm[kColRows][kColLanes * VEC + 1];
@@ -416,8 +423,9 @@ __global__ void __launch_bounds__(kColLanes* kColRows) reduce_cols_kernel(const 
 // Second pass of an "outer" reduction: out[o] = fold of partial[o * so + i * si + j], i < ni, j < nj.  G = 32: a warp per
 // output; G = kRedThreads: a block per output.
 template <class T, int KIND, int G>
-__global__ void __launch_bounds__(kRedThreads) reduce_outer_fold_kernel(const typename RedTraits<T, KIND>::Acc* __restrict__ partial, T* out, u64 count, u64 so, u32 ni,
+__global__ void __launch_bounds__(kRedThreads) reduce_outer_fold_kernel(const typename RedTraits<T, KIND>::Acc* partial, T* out, u64 count, u64 so, u32 ni,
                                                                       u64 si, u32 nj, FastDiv nj_div, u64 factor) {
+    after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
     const u64 o = (u64)blockIdx.x * (kRedThreads / G) + threadIdx.x / G;
     if (G == 32 && o >= count) return;
@@ -486,16 +494,19 @@ __device__ __forceinline__ void atomic_combine_minmax(Acc* p, Acc v) {
 
 template <class T, int KIND>
 __global__ void __launch_bounds__(kRedThreads) reduce_fill_kernel(typename RedTraits<T, KIND>::Acc* ws, u64 count) {
+    after_previous_kernel();
     for (u64 j = (u64)blockIdx.x * kRedThreads + threadIdx.x; j < count; j += (u64)gridDim.x * kRedThreads) ws[j] = RedTraits<T, KIND>::init();
 }
 template <class T, int KIND>
 __global__ void __launch_bounds__(kRedThreads) reduce_finalize_kernel(const typename RedTraits<T, KIND>::Acc* ws, T* out, u64 count, u64 factor) {
+    after_previous_kernel();
     for (u64 j = (u64)blockIdx.x * kRedThreads + threadIdx.x; j < count; j += (u64)gridDim.x * kRedThreads)
         out[j] = RedTraits<T, KIND>::finalize(ws[j], factor);
 }
 
 template <class T, int KIND>
 __global__ void __launch_bounds__(kRedThreads) reduce_scatter_kernel(const T* in, typename RedTraits<T, KIND>::Acc* ws, RedGenParams P) {
+    after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
     for (u64 i = (u64)blockIdx.x * kRedThreads + threadIdx.x; i < P.n; i += (u64)gridDim.x * kRedThreads) {
         u64 src, dst;
@@ -574,8 +585,8 @@ template <class T, int KIND, int VEC, int G>
 void red_rows_short_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaStream_t s) {
     constexpr u64 ROWS = kRedThreads / G;
     // four rows per group while that leaves every SM its eight blocks
-    if (O >= 4 * ROWS * 8 * (u64)sm_count()) reduce_rows_short_kernel<T, KIND, VEC, G, 4><<<(u32)((O + 4 * ROWS - 1) / (4 * ROWS)), kRedThreads, 0, s>>>(in, out, O, (u32)R, factor);
-    else reduce_rows_short_kernel<T, KIND, VEC, G, 1><<<(u32)((O + ROWS - 1) / ROWS), kRedThreads, 0, s>>>(in, out, O, (u32)R, factor);
+    if (O >= 4 * ROWS * 8 * (u64)sm_count()) launch_kernel(reduce_rows_short_kernel<T, KIND, VEC, G, 4>, (u32)((O + 4 * ROWS - 1) / (4 * ROWS)), kRedThreads, 0, s, in, out, O, (u32)R, factor);
+    else launch_kernel(reduce_rows_short_kernel<T, KIND, VEC, G, 1>, (u32)((O + ROWS - 1) / ROWS), kRedThreads, 0, s, in, out, O, (u32)R, factor);
 }
 template <class T, int KIND, int VEC>
 void red_rows_group_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaStream_t s) {
@@ -584,7 +595,7 @@ void red_rows_group_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaSt
     else if (lanes <= 8) red_rows_short_launch<T, KIND, VEC, 8>(in, out, O, R, factor, s);
     else if (lanes <= 16) red_rows_short_launch<T, KIND, VEC, 16>(in, out, O, R, factor, s);
     else if (lanes <= 32) red_rows_short_launch<T, KIND, VEC, 32>(in, out, O, R, factor, s);
-    else reduce_rows_warp_kernel<T, KIND, VEC><<<(u32)((O + kRedThreads / 32 - 1) / (kRedThreads / 32)), kRedThreads, 0, s>>>(in, out, O, (u32)R, factor);
+    else launch_kernel(reduce_rows_warp_kernel<T, KIND, VEC>, (u32)((O + kRedThreads / 32 - 1) / (kRedThreads / 32)), kRedThreads, 0, s, in, out, O, (u32)R, factor);
 }
 
 template <class T, int KIND>
@@ -610,7 +621,7 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
         const bool vec_rows = base_aligned && R % VEC == 0;
         if (R < 8 || (R < 32 && O > (sizeof(T) == 8 ? 16384 : 4096) && !(vec_rows && R >= 2 * VEC && (sizeof(T) < 8 || R % 8 == 0)))) {
             u64 blocks = (O + kRedThreads - 1) / kRedThreads;
-            reduce_rows_thread_kernel<T, KIND><<<(u32)blocks, kRedThreads, 0, s>>>(in, out, O, R, pl.factor);
+            launch_kernel(reduce_rows_thread_kernel<T, KIND>, (u32)blocks, kRedThreads, 0, s, in, out, O, R, pl.factor);
         } else if (R < 32 || (R < 2048 && O >= (u64)sms * 4)) {
             if (vec_rows) red_rows_group_launch<T, KIND, VEC>(in, out, O, R, pl.factor, s);
             else red_rows_group_launch<T, KIND, 1>(in, out, O, R, pl.factor, s);
@@ -639,12 +650,12 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
                 }
                 const int tree_fold = O <= 64 && splits >= 64;
                 dim3 grid((u32)splits, (u32)O);
-                if (vec) reduce_rows_block_kernel<T, KIND, VEC><<<grid, kRedThreads, 0, s>>>(in, out, part, R, seg, (u32)splits, pl.factor, counters, tree_fold);
-                else reduce_rows_block_kernel<T, KIND, 1><<<grid, kRedThreads, 0, s>>>(in, out, part, R, seg, (u32)splits, pl.factor, counters, tree_fold);
+                if (vec) launch_kernel(reduce_rows_block_kernel<T, KIND, VEC>, grid, kRedThreads, 0, s, in, out, part, R, seg, (u32)splits, pl.factor, counters, tree_fold);
+                else launch_kernel(reduce_rows_block_kernel<T, KIND, 1>, grid, kRedThreads, 0, s, in, out, part, R, seg, (u32)splits, pl.factor, counters, tree_fold);
                 if (splits > 1 && !counters) {
                     check_launch(where);
-                    if (tree_fold) reduce_partials_block_kernel<T, KIND><<<(u32)O, kRedThreads, 0, s>>>(part, out, (u32)splits, pl.factor);
-                    else reduce_partials_kernel<T, KIND><<<(u32)((O + kRedThreads - 1) / kRedThreads), kRedThreads, 0, s>>>(part, out, O, (u32)splits, 0, pl.factor);
+                    if (tree_fold) launch_kernel(reduce_partials_block_kernel<T, KIND>, (u32)O, kRedThreads, 0, s, part, out, (u32)splits, pl.factor);
+                    else launch_kernel(reduce_partials_kernel<T, KIND>, (u32)((O + kRedThreads - 1) / kRedThreads), kRedThreads, 0, s, part, out, O, (u32)splits, 0, pl.factor);
                 }
             }
         }
@@ -674,12 +685,12 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
             counters = arrival_counters(O * gx);
         }
         dim3 grid((u32)gx, (u32)splits, (u32)gz);
-        if (vec) reduce_cols_kernel<T, KIND, VEC><<<grid, kColLanes * kColRows, 0, s>>>(in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
-        else reduce_cols_kernel<T, KIND, 1><<<grid, kColLanes * kColRows, 0, s>>>(in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
+        if (vec) launch_kernel(reduce_cols_kernel<T, KIND, VEC>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
+        else launch_kernel(reduce_cols_kernel<T, KIND, 1>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
         if (splits > 1 && !counters) {
             check_launch(where);
             u64 count = O * I;
-            reduce_partials_kernel<T, KIND><<<(u32)((count + kRedThreads - 1) / kRedThreads), kRedThreads, 0, s>>>(part, out, count, (u32)splits, 1, pl.factor);
+            launch_kernel(reduce_partials_kernel<T, KIND>, (u32)((count + kRedThreads - 1) / kRedThreads), kRedThreads, 0, s, part, out, count, (u32)splits, 1, pl.factor);
         }
         check_launch(where);
         return;
@@ -701,10 +712,10 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
             Acc* part = static_cast<Acc*>(scratch(sizeof(Acc) * rows * pitch));
             if (!part) return;
             dim3 grid((u32)splits, (u32)rows);
-            if (base_aligned && I % VEC == 0) reduce_rows_block_kernel<T, KIND, VEC><<<grid, kRedThreads, 0, s>>>(in, out, part, I, seg, pitch, pl.factor, nullptr, 0);
-            else reduce_rows_block_kernel<T, KIND, 1><<<grid, kRedThreads, 0, s>>>(in, out, part, I, seg, pitch, pl.factor, nullptr, 0);
+            if (base_aligned && I % VEC == 0) launch_kernel(reduce_rows_block_kernel<T, KIND, VEC>, grid, kRedThreads, 0, s, in, out, part, I, seg, pitch, pl.factor, nullptr, 0);
+            else launch_kernel(reduce_rows_block_kernel<T, KIND, 1>, grid, kRedThreads, 0, s, in, out, part, I, seg, pitch, pl.factor, nullptr, 0);
             check_launch(where);
-            reduce_outer_fold_kernel<T, KIND, 32><<<(u32)((O + 7) / 8), kRedThreads, 0, s>>>(part, out, O, pitch, (u32)R, O * pitch, (u32)splits, FastDiv((u32)splits), pl.factor);
+            launch_kernel(reduce_outer_fold_kernel<T, KIND, 32>, (u32)((O + 7) / 8), kRedThreads, 0, s, part, out, O, pitch, (u32)R, O * pitch, (u32)splits, FastDiv((u32)splits), pl.factor);
             check_launch(where);
             return;
         }
@@ -731,12 +742,12 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
         if (part) {
             dim3 grid((u32)gx, (u32)splits, 1);
             const u32 leave = splits < 2 ? 2 : (u32)splits;
-            if (vec) reduce_cols_kernel<T, KIND, VEC><<<grid, kColLanes * kColRows, 0, s>>>(in, out, part, 1, R, cols, seg, leave, pl.factor, nullptr);
-            else reduce_cols_kernel<T, KIND, 1><<<grid, kColLanes * kColRows, 0, s>>>(in, out, part, 1, R, cols, seg, leave, pl.factor, nullptr);
+            if (vec) launch_kernel(reduce_cols_kernel<T, KIND, VEC>, grid, kColLanes * kColRows, 0, s, in, out, part, 1, R, cols, seg, leave, pl.factor, nullptr);
+            else launch_kernel(reduce_cols_kernel<T, KIND, 1>, grid, kColLanes * kColRows, 0, s, in, out, part, 1, R, cols, seg, leave, pl.factor, nullptr);
             check_launch(where);
             const FastDiv div((u32)I);
-            if (splits * I <= 2048) reduce_outer_fold_kernel<T, KIND, 32><<<(u32)((O + 7) / 8), kRedThreads, 0, s>>>(part, out, O, I, (u32)splits, cols, (u32)I, div, pl.factor);
-            else reduce_outer_fold_kernel<T, KIND, kRedThreads><<<(u32)O, kRedThreads, 0, s>>>(part, out, O, I, (u32)splits, cols, (u32)I, div, pl.factor);
+            if (splits * I <= 2048) launch_kernel(reduce_outer_fold_kernel<T, KIND, 32>, (u32)((O + 7) / 8), kRedThreads, 0, s, part, out, O, I, (u32)splits, cols, (u32)I, div, pl.factor);
+            else launch_kernel(reduce_outer_fold_kernel<T, KIND, kRedThreads>, (u32)O, kRedThreads, 0, s, part, out, O, I, (u32)splits, cols, (u32)I, div, pl.factor);
             check_launch(where);
             return;
         }
@@ -747,11 +758,11 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
     u32 fill_blocks = (u32)((pl.out_count + kRedThreads - 1) / kRedThreads);
     if (fill_blocks > (u32)sms * 16) fill_blocks = sms * 16;
     if (fill_blocks == 0) fill_blocks = 1;
-    reduce_fill_kernel<T, KIND><<<fill_blocks, kRedThreads, 0, s>>>(ws, pl.out_count);
+    launch_kernel(reduce_fill_kernel<T, KIND>, fill_blocks, kRedThreads, 0, s, ws, pl.out_count);
     u64 sb = (pl.gen.n + kRedThreads - 1) / kRedThreads;
     if (sb > (u64)sms * 16) sb = (u64)sms * 16;
-    if (sb) reduce_scatter_kernel<T, KIND><<<(u32)sb, kRedThreads, 0, s>>>(in, ws, pl.gen);
-    reduce_finalize_kernel<T, KIND><<<fill_blocks, kRedThreads, 0, s>>>(ws, out, pl.out_count, pl.factor);
+    if (sb) launch_kernel(reduce_scatter_kernel<T, KIND>, (u32)sb, kRedThreads, 0, s, in, ws, pl.gen);
+    launch_kernel(reduce_finalize_kernel<T, KIND>, fill_blocks, kRedThreads, 0, s, ws, out, pl.out_count, pl.factor);
     check_launch(where);
 }
 

@@ -49,12 +49,14 @@ inline void launch_clusters(void (*kernel)(P...), int grid, int threads, size_t 
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = shared;
     cfg.stream = ctx().stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)cluster;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = cluster ? 1 : 0;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_kernel
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster ? 2 : 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 // Clusters of n CTAs of `kernel` that can be resident at once; 0: cannot be asked.
