@@ -299,6 +299,83 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_warp_kernel(const T* 
     if (threadIdx.x % 32 == 0) out[row] = TR::finalize(acc, factor);
 }
 
+// Rows that are no whole aligned vectors, by the aligned 16-byte words they lie in: a lane loads a word (which holds at least one element of its row, so
+// that nothing outside the tensor's own words is touched) and leaves out the neighbours' elements.  Element by element a row of 197 bf16 took
+// seven loads of two bytes a lane, where one of 16 does.  G lanes per row with Q rows in flight where a row has up to G words, else a warp with four words
+// of it in flight.
+template <class T, int KIND>
+struct RowWords {
+    typedef RedTraits<T, KIND> TR;
+    static constexpr int VEC = 16 / (int)sizeof(T);
+    const Vec<T, VEC>* first;
+    u32 before, words;  // elements of the first word that belong to the row before; words
+    __device__ __forceinline__ RowWords(const T* row, u32 R) {
+        const uintptr_t at = reinterpret_cast<uintptr_t>(row), base = at & ~(uintptr_t)15;
+        first = reinterpret_cast<const Vec<T, VEC>*>(base);
+        before = (u32)(at - base) / (u32)sizeof(T);
+        words = (before + R + VEC - 1) / VEC;
+    }
+    __device__ __forceinline__ typename TR::Acc add(typename TR::Acc acc, const Vec<T, VEC>& v, u32 w, u32 R) const {
+        const u32 e0 = w * VEC - before;  // wraps below zero: then not below R
+#pragma unroll
+        for (int j = 0; j < VEC; j++) acc = TR::combine(acc, e0 + j < R ? TR::load(v.v[j]) : TR::init());
+        return acc;
+    }
+};
+template <class T, int KIND, int G, int Q>
+__global__ void __launch_bounds__(kRedThreads) reduce_rows_words_kernel(const T* in, T* out, u64 rows, u32 R, u64 factor) {
+    after_previous_kernel();
+    typedef RedTraits<T, KIND> TR;
+    typedef RowWords<T, KIND> RW;
+    constexpr u32 ROWS = kRedThreads / G;
+    const u64 row0 = (u64)blockIdx.x * ROWS * Q + threadIdx.x / G;
+    const u32 lane = threadIdx.x % G;
+    Vec<T, RW::VEC> v[Q];
+    typename TR::Acc acc[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+        if (row0 + q * ROWS < rows) {
+            const RW w(in + (row0 + q * ROWS) * R, R);
+            if (lane < w.words) v[q] = w.first[lane];
+        }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        acc[q] = TR::init();
+        if (row0 + q * ROWS < rows) {
+            const RW w(in + (row0 + q * ROWS) * R, R);
+            if (lane < w.words) acc[q] = w.add(acc[q], v[q], lane, R);
+        }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1)  // the shuffles take the whole warp
+#pragma unroll
+        for (int q = 0; q < Q; q++) acc[q] = TR::combine(acc[q], __shfl_xor_sync(0xFFFFFFFFu, acc[q], o));
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+        if (lane == 0 && row0 + q * ROWS < rows) out[row0 + q * ROWS] = TR::finalize(acc[q], factor);
+}
+template <class T, int KIND>
+__global__ void __launch_bounds__(kRedThreads) reduce_rows_long_words_kernel(const T* in, T* out, u64 rows, u32 R, u64 factor) {
+    after_previous_kernel();
+    typedef RedTraits<T, KIND> TR;
+    typedef RowWords<T, KIND> RW;
+    const u64 row = (u64)blockIdx.x * (kRedThreads / 32) + threadIdx.x / 32;
+    if (row >= rows) return;
+    const RW w(in + row * R, R);
+    typename TR::Acc acc = TR::init();
+    for (u32 i = threadIdx.x % 32; i < w.words; i += 4 * 32) {
+        Vec<T, RW::VEC> v[4];
+#pragma unroll
+        for (u32 q = 0; q < 4; q++)
+            if (i + q * 32 < w.words) v[q] = w.first[i + q * 32];
+#pragma unroll
+        for (u32 q = 0; q < 4; q++)
+            if (i + q * 32 < w.words) acc = w.add(acc, v[q], i + q * 32, R);
+    }
+    acc = warp_reduce<TR>(acc);
+    if (threadIdx.x % 32 == 0) out[row] = TR::finalize(acc, factor);
+}
+
 // One thread per row (R < 32, see red_launch).
 template <class T, int KIND>
 __global__ void __launch_bounds__(kRedThreads) reduce_rows_thread_kernel(const T* in, T* out, u64 rows, u64 R, u64 factor) {
@@ -598,6 +675,19 @@ void red_rows_group_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaSt
     else launch_kernel(reduce_rows_warp_kernel<T, KIND, VEC>, (u32)((O + kRedThreads / 32 - 1) / (kRedThreads / 32)), kRedThreads, 0, s, in, out, O, (u32)R, factor);
 }
 
+// Rows of at least 128 bytes that are no whole aligned vectors (see RowWords).
+template <class T, int KIND>
+void red_rows_words_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaStream_t s) {
+    constexpr u64 VEC = 16 / sizeof(T);
+    const u64 words = (R + 2 * VEC - 2) / VEC;  // at most, wherever a row starts
+    auto blocks = [&](u64 rows) { return (u32)((O + rows - 1) / rows); };
+    const bool many = O >= 4 * 8 * 8 * (u64)sm_count();
+    if (words <= 16) launch_kernel(reduce_rows_words_kernel<T, KIND, 16, 4>, blocks(4 * kRedThreads / 16), kRedThreads, 0, s, in, out, O, (u32)R, factor);
+    else if (words <= 32 && many) launch_kernel(reduce_rows_words_kernel<T, KIND, 32, 4>, blocks(4 * kRedThreads / 32), kRedThreads, 0, s, in, out, O, (u32)R, factor);
+    else if (words <= 32) launch_kernel(reduce_rows_words_kernel<T, KIND, 32, 1>, blocks(kRedThreads / 32), kRedThreads, 0, s, in, out, O, (u32)R, factor);
+    else launch_kernel(reduce_rows_long_words_kernel<T, KIND>, blocks(kRedThreads / 32), kRedThreads, 0, s, in, out, O, (u32)R, factor);
+}
+
 template <class T, int KIND>
 void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
     typedef RedTraits<T, KIND> TR;
@@ -624,6 +714,7 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
             launch_kernel(reduce_rows_thread_kernel<T, KIND>, (u32)blocks, kRedThreads, 0, s, in, out, O, R, pl.factor);
         } else if (R < 32 || (R < 2048 && O >= (u64)sms * 4)) {
             if (vec_rows) red_rows_group_launch<T, KIND, VEC>(in, out, O, R, pl.factor, s);
+            else if (sizeof(T) < 8 && R * sizeof(T) >= 128 && (uintptr_t)in % sizeof(T) == 0) red_rows_words_launch<T, KIND>(in, out, O, R, pl.factor, s);
             else red_rows_group_launch<T, KIND, 1>(in, out, O, R, pl.factor, s);
         } else {
             // block per (row, split); split long rows when there are too few rows to fill the GPU

@@ -192,3 +192,26 @@ def test_outer_folds_of_many_outputs(oracle, cuda, shape):
         if dt.name == "u8":
             want %= 256
         assert np.all(np.abs(np.asarray(got, dtype=np.float64) - want) <= tol * want), dt.name
+
+
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16, D.U8, D.I16, D.I32], ids=lambda d: d.name)
+def test_ragged_rows_by_the_words_they_lie_in(oracle, cuda, dt):
+    """Rows that are no whole aligned vectors, from an aligned base and from every place inside a word: the first and last word of a row belong to its
+    neighbours too, whose elements (the largest and smallest values) must not count."""
+    from oracle import binding
+    rng = np.random.default_rng(dt.size)
+    vec = 16 // dt.size
+    for r in (8 * vec + 1, 9 * vec - 1, 15 * vec + 1, 17 * vec + 2, 31 * vec + 1, 32 * vec + 1, 33 * vec - 1, 2047):
+        o = 701
+        for off in (0, 1, vec - 1):
+            x = H.random_store(rng, dt, o * r + off, dist="normal") if dt.kind == "float" else H.random_store(rng, dt, o * r + off)
+            for op in ("sum", "mean", "max"):
+                if op == "mean" and dt.kind != "float":
+                    continue
+                binding.set_wide(dt.kind == "float" and op != "max")
+                try:
+                    ref = H.run_reduce(oracle, op, dt, [o, r], [r, 1], [r], [1], off, x)
+                finally:
+                    binding.set_wide(False)
+                got = H.run_reduce(cuda, op, dt, [o, r], [r, 1], [r], [1], off, x)
+                H.assert_same(op, dt, got, ref, float_rel=SUM_TOL.get(dt.name, 0.0) if op != "max" else 0.0, what=str((op, r, off)), scale=np.sqrt(r) if op == "sum" else 1.0)
