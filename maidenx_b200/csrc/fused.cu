@@ -70,8 +70,8 @@ __global__ void __launch_bounds__(kFusedThreads) bias_gelu_kernel(const T* z, co
 // d/dx of x * sigmoid(2t), t = sqrt(2/pi) (x + 0.044715 x^3) - the tanh form's derivative, 0.5 (1 + tanh t) being sigmoid(2t):
 //   sigmoid + x sigmoid (1 - sigmoid) (2t)'
 // A dozen instructions and two of the special-function unit, where tanh, its square and the separately rounded products took thirty.  With
-// e = exp(-2|t|) and r = 1 / (1 + e) the sigmoid is r or e r and its product with the rest e r^2: no difference of near values on either side
-// (f32 error against 64 bits GELU_ERR, 1.0e-7 and 4.5e-6 of the norm for positive and negative x by tanh).
+// e = exp(-2|t|) and r = 1 / (1 + e) the sigmoid is r or e r and its product with the rest e r^2: no difference of near values on either side.
+// Error against 64 bits, of the norm, over [0, 12]: 4.0e-8 (by tanh 1.0e-7); [-12, 0]: 1.05e-7 (4.6e-6); [-6, 6]: 5.7e-8 (5.1e-7); 16-bit results alike.
 __device__ __forceinline__ float gelu_grad_f32(float x) {
     const float k1 = -2.302208198f, k2 = -0.102943240f;  // exp(-2t) = 2^(x (k1 + k2 x^2)), as in gelu_f32_fast
     const float c1 = 1.5957691216f, c2 = 0.2140644488f;  // (2t)' = c1 + c2 x^2: 2 sqrt(2/pi), three times 0.044715 of that

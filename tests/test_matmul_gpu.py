@@ -352,6 +352,37 @@ def test_short_reductions_with_the_b_panel_resident(oracle, cuda, dt, case):
     assert np.array_equal(kept, general)
 
 
+@pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [
+    # batch, M, N, K, majors, whether A is the same for all batches: edges of row and column tiles, one to four k-blocks, runs of tiles that end inside a panel
+    (97, 520, 760, 64, "kk", False), (149, 513, 504, 136, "km", False), (160, 512, 512, 256, "mm", True)], ids=lambda c: "x".join(map(str, c[:4])))
+def test_short_reductions_of_a_batch_with_the_b_panel_resident(cuda, dt, case):
+    """Batched products of K <= 256 load a B panel once for all its row tiles: bit for bit the general schedule, and next to float64 in the first, a middle and the
+    last batch (one rounding of an f32 sum: half a step of the type and the sum's own error)."""
+    from maidenx_b200 import _lib
+    lib = _lib.load()
+    nb, m, n, k, majors, shared = case
+    rng = np.random.default_rng(nb + m + n + k)
+    na = 1 if shared else nb
+    a, b = H.random_store(rng, dt, na * m * k, dist="normal"), H.random_store(rng, dt, nb * k * n, dist="normal")
+    sa, sb = [0 if shared else m * k, *([k, 1] if majors[0] == "k" else [1, m])], [k * n, *([1, k] if majors[1] == "k" else [n, 1])]
+    meta = H.matmul_metadata([nb, m, n], [nb, m, k], [nb, k, n], sa, sb, 0, 0)
+    kept = H.run_matmul(cuda, dt, meta, nb * m * n, a, b)
+    lib.mx_debug_set_gemm_keep_b(0)
+    try:
+        general = H.run_matmul(cuda, dt, meta, nb * m * n, a, b)
+    finally:
+        lib.mx_debug_set_gemm_keep_b(1)
+    assert np.array_equal(kept, general)
+    got = D.decode(kept, dt).reshape(nb, m, n)
+    for i in (0, nb // 2, nb - 1):
+        x = D.decode(a.reshape(na, m * k)[0 if shared else i], dt).astype(np.float64)
+        y = D.decode(b.reshape(nb, k * n)[i], dt).astype(np.float64)
+        x, y = x.reshape(m, k) if majors[0] == "k" else x.reshape(k, m).T, y.reshape(k, n) if majors[1] == "k" else y.reshape(n, k).T
+        ref, bound = x @ y, np.abs(x) @ np.abs(y)
+        assert np.all(np.abs(got[i] - ref) <= (2.0**-8 if dt.name == "bf16" else 2.0**-11) * np.abs(ref) + k * 2.0**-23 * bound + 2.0**-24)
+
+
 # ---------------------------------------------------------------------------------------
 # Products whose matrices are not 16-byte multiples: operands copied to padded rows, output rows
 # written without tensor stores; and the plain tensor-core products that have more than one batch
