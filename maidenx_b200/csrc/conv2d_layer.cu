@@ -21,8 +21,6 @@
 //
 // The caller owns every buffer, as everywhere in this ABI: `cols` (B*P*K elements) is written by forward and read
 // by backward; `workspace` holds the intermediates (sizes from mx_conv2d_workspace_elems).
-#include <algorithm>
-
 #include "abi_common.cuh"
 #include "matmul_tc.cuh"
 
@@ -111,19 +109,6 @@ void bias_gradient(const Ops& ops, const Geometry& g, size_t es, const void* gra
     sum_dim(ops, d2, 2, 0, t2, grad_bias);
 }
 
-// Images that mode 1 takes at a time.  A column matrix larger than L2 (126 MB) goes out to HBM when it is written and comes back for the
-// op behind it; in groups of images whose columns stay below this it is read from L2 where it was just written, and in the backward pass, where all
-// groups use the same place of the workspace, the most of it is overwritten before it ever leaves.  Each image's results are the same whatever
-// the group (a group of one would be an unbatched product, which may add in another order: not taken).
-constexpr size_t kGroupBytes = (size_t)80 << 20;
-size_t images_at_a_time(const Geometry& g, size_t es) {
-    const size_t image = g.K * g.P * es, most = kGroupBytes / (image ? image : 1);
-    if (g.B * image <= 2 * kGroupBytes || most < 2) return g.B;
-    const size_t groups = (g.B + most - 1) / most;
-    const size_t per = (g.B + groups - 1) / groups;
-    return g.B % per == 1 ? g.B : per;
-}
-
 size_t workspace_elems(const Geometry& g, int mode, int backward) {
     const size_t sums = round16(g.B * g.Co * g.oh) + round16(g.B * g.Co);
     if (mode == 0) {
@@ -168,24 +153,17 @@ void forward(const Ops& ops, size_t es, const MxConv2d* c, int mode, const void*
         }
         return;
     }
-    auto at = [&](const void* p, size_t elems) { return static_cast<const char*>(p) + elems * es; };
-    const size_t per = images_at_a_time(g, es);
-    for (size_t b0 = 0; b0 < g.B; b0 += per) {
-        const size_t B = std::min(per, g.B - b0);
-        char* cols_b = static_cast<char*>(cols) + b0 * g.K * g.P * es;
-        char* out_b = static_cast<char*>(out) + b0 * g.Co * g.P * es;
-        const size_t cm[12] = {B, g.C, g.H, g.W, g.kh, g.kw, g.oh, g.ow, g.ph, g.pw, g.sh, g.sw};
-        ops.im2col(B * g.P * g.K, cm, at(x, b0 * g.C * g.H * g.W), cols_b);
-        // out[B, Co, P] = W[Co, K] (shared by every batch) . cols[B, K, P]
-        const size_t mm[20] = {3, 3, 3, B, g.Co, g.P, B, g.Co, g.K, B, g.K, g.P, 0, g.K, 1, g.K * g.P, g.P, 1, 0, 0};
-        // 16-bit types: the bias add rides in the product's epilogue (same roundings as the two ops below) when the
-        // tensor-core kernel takes the shape
-        if (bias && ops.half_kind && tc_batched_row_bias(ops.half_kind == 1, B, g.Co, g.K, g.P, w, cols_b, bias, out_b, "mx_conv2d_forward")) continue;
-        ops.matmul(B * g.Co * g.P, mm, w, cols_b, out_b);
-        if (bias) {
-            const size_t am[11] = {B, g.Co, g.P, g.Co * g.P, g.P, 1, 0, 1, 0, 0, 0};
-            ops.add_inplace(B * g.Co * g.P, 3, am, out_b, bias);
-        }
+    const size_t cm[12] = {g.B, g.C, g.H, g.W, g.kh, g.kw, g.oh, g.ow, g.ph, g.pw, g.sh, g.sw};
+    ops.im2col(ncol, cm, x, cols);
+    // out[B, Co, P] = W[Co, K] (shared by every batch) . cols[B, K, P]
+    const size_t mm[20] = {3, 3, 3, g.B, g.Co, g.P, g.B, g.Co, g.K, g.B, g.K, g.P, 0, g.K, 1, g.K * g.P, g.P, 1, 0, 0};
+    // 16-bit types: the bias add rides in the product's epilogue (same roundings as the two ops below) when the
+    // tensor-core kernel takes the shape
+    if (bias && ops.half_kind && tc_batched_row_bias(ops.half_kind == 1, g.B, g.Co, g.K, g.P, w, cols, bias, out, "mx_conv2d_forward")) return;
+    ops.matmul(g.B * g.Co * g.P, mm, w, cols, out);
+    if (bias) {
+        const size_t am[11] = {g.B, g.Co, g.P, g.Co * g.P, g.P, 1, 0, 1, 0, 0, 0};
+        ops.add_inplace(g.B * g.Co * g.P, 3, am, out, bias);
     }
 }
 
@@ -231,15 +209,11 @@ void backward(const Ops& ops, size_t es, const MxConv2d* c, int mode, const void
     char* gw_batch = grad_cols + round16(g.B * g.K * g.P) * es;
     char* sums = gw_batch + round16(g.B * g.Co * g.K) * es;
     if (grad_x) {
-        const size_t per = images_at_a_time(g, es);
-        for (size_t b0 = 0; b0 < g.B; b0 += per) {
-            const size_t B = std::min(per, g.B - b0);
-            // grad_cols[B, K, P] = W^T (the transposed view of [Co, K], shared by every batch) . grad_out[B, Co, P]
-            const size_t mm[20] = {3, 3, 3, B, g.K, g.P, B, g.K, g.Co, B, g.Co, g.P, 0, 1, g.K, g.Co * g.P, g.P, 1, 0, 0};
-            ops.matmul(B * g.K * g.P, mm, w, static_cast<const char*>(grad_out) + b0 * g.Co * g.P * es, grad_cols);
-            const size_t cm[12] = {B, g.C, g.H, g.W, g.kh, g.kw, g.oh, g.ow, g.ph, g.pw, g.sh, g.sw};
-            ops.col2im(B * g.K * g.P, cm, grad_cols, static_cast<char*>(grad_x) + b0 * g.C * g.H * g.W * es);
-        }
+        // grad_cols[B, K, P] = W^T (the transposed view of [Co, K], shared by every batch) . grad_out[B, Co, P]
+        const size_t mm[20] = {3, 3, 3, g.B, g.K, g.P, g.B, g.K, g.Co, g.B, g.Co, g.P, 0, 1, g.K, g.Co * g.P, g.P, 1, 0, 0};
+        ops.matmul(g.B * g.K * g.P, mm, w, grad_out, grad_cols);
+        const size_t cm[12] = {g.B, g.C, g.H, g.W, g.kh, g.kw, g.oh, g.ow, g.ph, g.pw, g.sh, g.sw};
+        ops.col2im(g.B * g.K * g.P, cm, grad_cols, grad_x);
     }
     // f32: the sum over the batch is part of the product's reduction where the tensor-core kernel takes it; no per-batch
     // gradient is written and read back (38 MB at 32 x 128 x 14 x 14, 256 channels: product and sum 45 us, now 37).  16-bit types keep the composition's rounding

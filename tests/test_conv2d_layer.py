@@ -7,8 +7,6 @@ GPU: the library's composition (mx_conv2d_forward / backward through the C ABI) 
 the same calls, for the literal reference call sequence (mode 0) and the direct one (mode 1), and mode 1 against
 the float64 convolution.  Tolerances: f32 1e-4 and bf16 / f16 2e-2 of max(|ref|, sqrt(terms)).
 """
-import ctypes
-
 import numpy as np
 import pytest
 
@@ -180,36 +178,3 @@ def test_direct_layer_on_ragged_maps(cuda, dt, shape):
     sc = _scales(shape)
     for key in ("out", "grad_x", "grad_w", "grad_bias"):
         H.assert_same("conv2d", dt, got[key], D.encode(ref[key], dt), float_rel={"f32": 1e-5}.get(dt.name, 2e-2), what=key, scale=sc[key])
-
-
-@pytest.mark.gpu
-@pytest.mark.parametrize("dt", [D.BF16, D.F32], ids=lambda d: d.name)
-def test_images_taken_in_groups_give_the_bits_of_all_at_once(cuda, dt):
-    """A column matrix larger than L2 is made and used a group of images at a time; the parts of the batch, small enough to be taken at once, give the same bits."""
-    from maidenx_b200 import _lib, device
-    c, hw, co, k = (64, 112, 40, 3) if dt.size == 2 else (32, 112, 24, 3)
-    n = 13
-    rng = np.random.default_rng(n)
-    x, w, b, g = (D.encode(rng.standard_normal(e).astype(np.float32) * f, dt) for e, f in ((n * c * hw * hw, 1.0), (co * c * k * k, 0.05), (co, 1.0), (n * co * hw * hw, 1.0)))
-    fwd, bwd = _lib.conv2d(dt.name)
-    lib = _lib.load()
-
-    def run(i0, i1):
-        conv = _lib.MxConv2d(i1 - i0, c, hw, hw, co, k, k, 1, 1, 1, 1)
-        ref = ctypes.byref(conv)
-        parts = [x[i0 * c * hw * hw:i1 * c * hw * hw], w, b, g[i0 * co * hw * hw:i1 * co * hw * hw]]
-        xb, wb, bb, gb = (device.CudaBuffer.from_host(p) for p in parts)
-        cols = device.CudaBuffer(lib.mx_conv2d_cols_elems(ref) * dt.size)
-        ws = device.CudaBuffer(max(lib.mx_conv2d_workspace_elems(ref, 1, 0), lib.mx_conv2d_workspace_elems(ref, 1, 1)) * dt.size)
-        y, dx, dw, db = (device.CudaBuffer(max(e, 1) * dt.size) for e in (parts[3].size, parts[0].size, w.size, co))
-        fwd(ref, 1, xb.ptr, wb.ptr, bb.ptr, cols.ptr, ws.ptr, y.ptr)
-        bwd(ref, 1, gb.ptr, wb.ptr, cols.ptr, ws.ptr, dx.ptr, dw.ptr, db.ptr)
-        out = [y.to_host(dt.np_storage, parts[3].size), dx.to_host(dt.np_storage, parts[0].size), cols.to_host(dt.np_storage, lib.mx_conv2d_cols_elems(ref))]
-        for buf in (xb, wb, bb, gb, cols, ws, y, dx, dw, db):
-            buf.free()
-        assert device.last_error() is None
-        return out
-
-    whole = run(0, n)
-    for got, a, b2 in zip(whole, run(0, 7), run(7, n)):
-        assert np.array_equal(got.view(np.uint8), np.concatenate([a, b2]).view(np.uint8))
