@@ -1017,84 +1017,6 @@ bool softmax_cols_reg_launch(const T* in, T* out, u64 pre, u64 n, u64 post, cuda
     return true;
 }
 
-// The same rows by the aligned 16-byte words they lie in: a lane has up to K words (each with at least one element of the row), reads them
-// whole and writes them whole but for the row's two ends.  Element by element, rows of 197 bf16 took seven loads and seven stores of two bytes a lane.
-template <class T, int K>
-__global__ void __launch_bounds__(kExThreads) softmax_rows_words_kernel(const T* in, T* out, u64 rows, u32 n) {
-    after_previous_kernel();
-    constexpr int VEC = 16 / (int)sizeof(T);
-    const u32 lane = threadIdx.x % 32;
-    const u64 row = (u64)blockIdx.x * (kExThreads / 32) + threadIdx.x / 32;
-    if (row >= rows) return;  // whole warps
-    const uintptr_t at = reinterpret_cast<uintptr_t>(in + row * n), base = at & ~(uintptr_t)15;
-    const u32 before = (u32)(at - base) / (u32)sizeof(T), words = (before + n + VEC - 1) / VEC;
-    Vec<T, VEC> v[K];
-#pragma unroll
-    for (int k = 0; k < K; k++)
-        if (k * 32 + lane < words) v[k] = reinterpret_cast<const Vec<T, VEC>*>(base)[k * 32 + lane];
-    f32 x[K][VEC], mx = -INFINITY;
-    auto place = [&](int k, int j) { return (k * 32 + lane) * VEC + j - before; };  // in the row; not below n: another row's, or none
-#pragma unroll
-    for (int k = 0; k < K; k++)
-#pragma unroll
-        for (int j = 0; j < VEC; j++) {
-            x[k][j] = -INFINITY;
-            if (place(k, j) < n) {
-                if constexpr (is_half_v<T>) x[k][j] = to_f32(v[k].v[j]);
-                else x[k][j] = (f32)v[k].v[j];
-            }
-            mx = x[k][j] > mx ? x[k][j] : mx;  // a NaN never becomes the maximum
-        }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const f32 other = __shfl_xor_sync(0xFFFFFFFFu, mx, o);
-        mx = other > mx ? other : mx;
-    }
-    f32 sum = 0.0f;
-#pragma unroll
-    for (int k = 0; k < K; k++)
-#pragma unroll
-        for (int j = 0; j < VEC; j++) {
-            if constexpr (is_half_v<T>) x[k][j] = exp2_approx((x[k][j] - mx) * 1.4426950408889634f);
-            else x[k][j] = expf(x[k][j] - mx);
-            if (place(k, j) < n) sum += x[k][j];
-        }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    const f32 inv = 1.0f / sum;
-    T* dst = out + row * n;
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        Vec<T, VEC> r;
-#pragma unroll
-        for (int j = 0; j < VEC; j++) {
-            if constexpr (is_half_v<T>) r.v[j] = from_f32<T>(x[k][j] * inv);
-            else r.v[j] = (T)(x[k][j] / sum);
-        }
-        const u32 e0 = place(k, 0);
-        if (e0 < n && e0 + VEC <= n) {
-            *reinterpret_cast<Vec<T, VEC>*>(dst + e0) = r;
-        } else {
-#pragma unroll
-            for (int j = 0; j < VEC; j++)
-                if (e0 + j < n) dst[e0 + j] = r.v[j];
-        }
-    }
-}
-// false: rows too long for a warp's registers, or in- and output are not the same distance from a 16-byte boundary
-template <class T>
-bool softmax_rows_words_launch(const T* in, T* out, u64 rows, u32 n, cudaStream_t s) {
-    constexpr u32 VEC = 16 / (u32)sizeof(T);
-    if ((reinterpret_cast<uintptr_t>(in) ^ reinterpret_cast<uintptr_t>(out)) % 16 || reinterpret_cast<uintptr_t>(in) % sizeof(T) || n * sizeof(T) < 128) return false;
-    const u32 words = (n + 2 * VEC - 2) / VEC;  // at most, wherever a row starts
-    const unsigned blocks = (unsigned)((rows + kExThreads / 32 - 1) / (kExThreads / 32));
-    if (words <= 32) launch_kernel(softmax_rows_words_kernel<T, 1>, blocks, kExThreads, 0, s, in, out, rows, n);
-    else if (words <= 64) launch_kernel(softmax_rows_words_kernel<T, 2>, blocks, kExThreads, 0, s, in, out, rows, n);
-    else if (words <= 128) launch_kernel(softmax_rows_words_kernel<T, 4>, blocks, kExThreads, 0, s, in, out, rows, n);
-    else return false;
-    return true;
-}
-
 template <class T, int G>
 bool softmax_rows_any_launch(const T* in, T* out, u64 rows, u32 n, cudaStream_t s) {
     const u32 per = (n + G - 1) / G;  // elements per thread
@@ -1176,9 +1098,7 @@ void softmax_entry(size_t num_els, size_t nd, size_t dim, const size_t* meta, co
         const u64 sms = (u64)sm_count();
         const u64 warp_most = is_half_v<T> ? 1024 : P.pre >= 16 * sms ? 512 : 256, block_most = is_half_v<T> ? 64ull * kExThreads : P.pre <= 2 * sms ? 8192 : 4096;
         if (P.post == 1 && P.pre < (1ull << 31) && P.n <= block_most) {
-            bool done = false;
-            if constexpr (sizeof(T) <= 4) done = P.n <= warp_most && softmax_rows_words_launch<T>(src, out, P.pre, (u32)P.n, st);
-            if (!done) done = P.n <= warp_most ? softmax_rows_any_launch<T, 32>(src, out, P.pre, (u32)P.n, st)
+            const bool done = P.n <= warp_most ? softmax_rows_any_launch<T, 32>(src, out, P.pre, (u32)P.n, st)
                                                : softmax_rows_any_launch<T, kExThreads>(src, out, P.pre, (u32)P.n, st);
             if (done) {
                 check_launch(where);

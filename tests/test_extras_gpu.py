@@ -317,34 +317,3 @@ def test_softmax_of_ragged_rows_and_of_columns_in_registers(oracle, cuda, dt):
             assert np.all(np.abs(got - ref) <= tol * np.maximum(np.abs(ref), floor)), (dims, off, np.abs(got / np.maximum(ref, 1e-30) - 1).max())
     finally:
         oracle.b.set_wide(False)
-
-
-@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16], ids=lambda d: d.name)
-def test_softmax_of_rows_by_the_words_they_lie_in(oracle, cuda, dt):
-    """Rows that start anywhere in a 16-byte word, one word to four a lane; rows with infinities at their ends, next to rows of large values, and nothing written
-    outside the output."""
-    from maidenx_b200 import device
-    from oracle import binding
-    rng = np.random.default_rng(dt.size)
-    vec = 16 // dt.size
-    for n in (8 * vec + 1, 31 * vec + 1, 32 * vec - 1, 33 * vec + 1, 63 * vec + 3, 100 * vec + 1, 127 * vec + 1):
-        for off in (0, 1, vec - 1):
-            rows = 37
-            v = rng.standard_normal((rows, n)).astype(np.float32) * 4
-            v[1::4] += 40
-            v[2, 0] = v[2, -1] = -np.inf
-            x = D.encode(np.concatenate([np.full(off, 60, np.float32), v.reshape(-1)]), dt)
-            binding.set_wide(True)
-            try:
-                ref = D.decode(H.run_softmax(oracle, dt, [rows, n], [n, 1], off, 1, x), dt).astype(np.float64)
-            finally:
-                binding.set_wide(False)
-            guard = 16 // dt.size
-            src, dst = device.CudaBuffer.from_host(x), device.CudaBuffer.from_host(np.full(rows * n + 2 * guard + off, 3, dt.np_storage))
-            device.dispatch("softmax", dt.name, [rows, n, n, 1, off], rows * n, 2, 1, "META", src.ptr, dst.ptr + (guard + off) * dt.size)
-            raw = dst.to_host(dt.np_storage, rows * n + 2 * guard + off)
-            assert (raw[:guard + off] == 3).all() and (raw[guard + off + rows * n:] == 3).all()
-            got = D.decode(raw[guard + off:guard + off + rows * n], dt).astype(np.float64)
-            assert np.all(np.abs(got - ref.reshape(-1)) <= (1e-5 if dt.name == "f32" else 2e-2) * np.maximum(np.abs(ref.reshape(-1)), 1e-3)), (n, off)
-            src.free()
-            dst.free()

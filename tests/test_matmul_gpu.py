@@ -378,7 +378,7 @@ def test_short_reductions_of_a_batch_with_the_b_panel_resident(cuda, dt, case):
     for i in (0, nb // 2, nb - 1):
         x = D.decode(a.reshape(na, m * k)[0 if shared else i], dt).astype(np.float64)
         y = D.decode(b.reshape(nb, k * n)[i], dt).astype(np.float64)
-        x, y = x.reshape(m, k) if majors[0] == "k" else x.reshape(k, m).T, y.reshape(k, n) if majors[1] == "k" else y.reshape(n, k).T
+        x, y = x.reshape(m, k) if majors[0] == "k" else x.reshape(k, m).T, y.reshape(n, k).T if majors[1] == "k" else y.reshape(k, n)
         ref, bound = x @ y, np.abs(x) @ np.abs(y)
         assert np.all(np.abs(got[i] - ref) <= (2.0**-8 if dt.name == "bf16" else 2.0**-11) * np.abs(ref) + k * 2.0**-23 * bound + 2.0**-24)
 
