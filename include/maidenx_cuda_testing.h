@@ -44,9 +44,8 @@ int mx_debug_gemm_keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, i
 /* How many K slices the tensor-core path cuts a product with `tiles` output tiles and reduction length `k` into
  * (1 = no split) on `sms` SMs; block_k = 64 for bf16 / f16, 32 for f32. */
 int mx_debug_splitk_slices(size_t tiles, size_t k, int block_k, int sms);
-/* Tensor-core products (16-bit, f32) whose reduction is cut into slices: 1 = summed inside a cluster of CTAs where they fit one (default), 0 =
- * by a second launch. */
-void mx_debug_set_gemm_cluster(int on);
+/* f32 tensor-core products whose reduction is cut into the CTAs of a cluster: 1 = where that pays and a second launch does not (default), 0 =
+ * nowhere, 2 = wherever one fits. */
 void mx_debug_set_gemm_f32_cluster(int on);
 /* Writes `value` (0 clears) into the calling thread's tensor-core error word the way a kernel of an earlier launch
  * whose bounded wait ran out would have left it.  Returns 0, or -1 without a usable device. */

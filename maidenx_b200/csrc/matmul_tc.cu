@@ -35,7 +35,7 @@
 
 #include "matmul_tc.cuh"
 #include "matmul_tc2.cuh"
-#include "tc_cluster.cuh"
+#include "tc_ptx.cuh"
 
 namespace mx {
 
@@ -79,13 +79,6 @@ constexpr double kSplitFixed16 = 10.0;
 
 constexpr int MN_CHUNK_BYTES = 64 * BK * 2;  // one [64 K-rows x 64 MN] box
 
-// A split product whose slices are the CTAs of a cluster (TcParams::cluster): the partial result in the ring's place, rows 16 bytes longer than
-// 256 floats, so that the threads of a warp, a row each, store to different banks.
-constexpr int PART_LD = BN + 4;
-static_assert(BM * PART_LD * 4 <= STAGES * (A_STAGE_BYTES + B_STAGE_BYTES), "partial result inside the ring");
-// what the sum inside a cluster costs, in the unit of kSplitFixed16
-constexpr double kClusterFixed16 = 5.0;
-
 // Instruction descriptor of tcgen05.mma kind::f16 with f32 accumulation.
 __host__ __device__ constexpr uint32_t make_idesc(bool is_bf16, bool a_mn_major, bool b_mn_major, int bn) {
     uint32_t d = 0;
@@ -106,10 +99,6 @@ struct TcParams {
     int a_batched, b_batched;  // 0: the operand is one matrix shared by every batch (third TMA coordinate stays 0)
     int is_bf16;
     int out_f32;  // split-K partial results: the epilogue stores the f32 accumulators unrounded
-    // > 0: the K slices of an output tile are the CTAs of one cluster: each leaves its partial result in its own shared memory and rounds the sums of
-    // the rows that fall to it, added in slice order (the bits of the form with a second launch).  out_f32 is set too.
-    int cluster;
-    int vec_out;  // cluster: the output's rows may be written four elements at a time
     int fuse;     // 0: store the product; 1: u = round(round(product) + bias) through map_d; 2: also act = round(gelu(u)) through map_d2;
                   // 3: as 1 with one bias element per output ROW (bias[row of the batch's matrix]): a convolution's per-channel bias
     const void* bias;  // fuse != 0: one element of the operand type in device memory
@@ -142,16 +131,11 @@ __device__ __forceinline__ void tile_coords(int tile, const TcParams& p, int& tm
     tn = in_group / rows;
 }
 
-// Which tiles a CTA computes.
-enum TcSched {
-    SCHED_TILES = 0,  // every gridDim.x-th of tile_coords' order, or those of TcParams::b_keep
-    SCHED_PANELS,     // short reductions of a batch: an equal run of the order batch, column tile, row tile, with a B panel loaded once for all its row tiles
-    SCHED_CLUSTER,    // TcParams::cluster: one tile and slice; the rank in the cluster is the slice
-};
-// The it-th tile of this CTA; false when it has none left.
-template <int SCHED>
+// The it-th tile of this CTA; false when it has none left.  PANELS (short reductions of a batch): the tiles in the order batch, column tile, row
+// tile, an equal run of them for each CTA, which loads a B panel once for all row tiles of it.
+template <bool PANELS>
 __device__ __forceinline__ bool next_tile(int it, const TcParams& p, int& tm, int& tn, int& tb) {
-    if constexpr (SCHED == SCHED_PANELS) {
+    if constexpr (PANELS) {
         const int tile = (int)((long long)blockIdx.x * p.num_tiles / gridDim.x) + it;
         if (tile >= (int)((long long)(blockIdx.x + 1) * p.num_tiles / gridDim.x)) return false;
         const int panel = tile / p.tiles_m;
@@ -159,10 +143,6 @@ __device__ __forceinline__ bool next_tile(int it, const TcParams& p, int& tm, in
         tb = panel / p.tiles_n;
         tn = panel - tb * p.tiles_n;
         return true;
-    }
-    if constexpr (SCHED == SCHED_CLUSTER) {
-        tile_coords((int)blockIdx.x % p.cluster * p.tiles_per_batch + (int)blockIdx.x / p.cluster, p, tm, tn, tb);
-        return it == 0;
     }
     if (p.b_keep) {
         tn = (int)blockIdx.x / p.b_keep;
@@ -252,13 +232,13 @@ enum TcMode {
 // with the geometry from the parameters the products of a 16384 x 8192 layer took 12 % longer at full clock.
 // DRAIN (tiles of at most 128 columns): the accumulator is emptied every run_kb k-blocks into totals in registers, added with
 // round-to-nearest, so that the pull of the tensor core's truncating additions stays that of one run whatever K is (see kRunMostF16).
-// SCHED: TcSched.  Instantiations of their own for the same reason (the panels as a branch of the common schedule cost 4096^3 19 %).
+// PANELS: TcParams::panels, an instantiation of its own for the same reason (as a branch of the common schedule it cost 4096^3 19 %).
 //
 // Epilogue warps for each quarter of the accumulator's lanes.  Rows that the warps write themselves take two (4096 x 2050 x 512 bf16: 25 us, 36
 // with one); products that leave through the copy engine gain nothing from a second one (16384 x 4096 x 256: 55 us, 50 with one).
 constexpr int epi_warps(int mode) { return mode == TC_PLAIN ? 2 : 1; }
 constexpr int tc_threads(int mode) { return 32 * (2 + 4 * epi_warps(mode)); }
-template <int MODE, int BN_T, bool DRAIN = false, int SCHED = SCHED_TILES>
+template <int MODE, int BN_T, bool DRAIN = false, bool PANELS = false>
 __global__ void __launch_bounds__(tc_threads(MODE), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                const __grid_constant__ CUtensorMap map_d2, TcParams p, int* err, int tag) {
@@ -305,12 +285,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            const int ring = SCHED == SCHED_PANELS || p.b_keep ? p.num_kb : stages;
+            const int ring = PANELS || p.b_keep ? p.num_kb : stages;
             int tm, tn, tb;
-            for (int it = 0; ok && next_tile<SCHED>(it, p, tm, tn, tb); it++) {
+            for (int it = 0; ok && next_tile<PANELS>(it, p, tm, tn, tb); it++) {
                 const int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
                 int k = tb * p.split_kb * BK;              // a k-block past the end of K is all fill: zeros
-                const bool load_b = SCHED == SCHED_PANELS ? tm == 0 || it == 0 : !p.b_keep || it == 0;  // a kept B panel arrives with its first tile's A blocks
+                const bool load_b = PANELS ? tm == 0 || it == 0 : !p.b_keep || it == 0;  // a kept B panel arrives with its first tile's A blocks
                 for (int kb = 0; kb < p.num_kb; kb++, k += BK) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, err, tag, 1)) {
                         ok = false;
@@ -348,10 +328,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
-            const int ring = SCHED == SCHED_PANELS || p.b_keep ? p.num_kb : stages;
+            const int ring = PANELS || p.b_keep ? p.num_kb : stages;
             int tm, tn, tb;
             int run = 0;  // first k-block of the accumulator's run (DRAIN: a tile has several)
-            for (int it = 0; ok && next_tile<SCHED>(it, p, tm, tn, tb); it += DRAIN && run ? 0 : 1) {
+            for (int it = 0; ok && next_tile<PANELS>(it, p, tm, tn, tb); it += DRAIN && run ? 0 : 1) {
                 if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1, err, tag, 2)) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
@@ -398,7 +378,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         float fused_bias = 0.0f;
         if (MODE == TC_BIAS && p.fuse != 3) fused_bias = p.is_bf16 ? to_f32(*static_cast<const bf16*>(p.bias)) : to_f32(*static_cast<const f16*>(p.bias));
         int tm, tn, tb;
-        for (int it = 0; next_tile<SCHED>(it, p, tm, tn, tb); it++) {
+        for (int it = 0; next_tile<PANELS>(it, p, tm, tn, tb); it++) {
             // four or eight warps wait here for most of a tile's reduction: they sleep between polls, so that their polling does not
             // take shared-memory cycles from the TMA writes and the tensor core's operand reads
             if (MODE != TC_STORE && p.fuse == 3) {  // this thread's output row inside the batch's matrix
@@ -462,13 +442,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const int col = tn * bn + c * EPI_CHUNK_COLS;
                 if constexpr (MODE == TC_STORE) {
                     static_assert(W == 1, "f32 results: a warp stages both halves of a chunk");
-                    if constexpr (SCHED == SCHED_CLUSTER) {  // the ring is done with: every product that read it has been committed
-                        float* part = reinterpret_cast<float*>(smem + SmemLayout::ring) + (quarter * 32 + lane) * PART_LD + c * EPI_CHUNK_COLS;
-#pragma unroll
-                        for (int j = 0; j < CW; j += 4)
-                            *reinterpret_cast<uint4*>(part + j) = make_uint4(v[j / 32][j % 32], v[j / 32][j % 32 + 1], v[j / 32][j % 32 + 2], v[j / 32][j % 32 + 3]);
-                        return;
-                    }
                     if (p.out_f32) {
                         // two 32-column f32 chunks (128 bytes per row each), one per staging buffer
 #pragma unroll
@@ -594,28 +567,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
-    if constexpr (SCHED == SCHED_CLUSTER) {
-        int tm, tn, tb;
-        next_tile<SCHED>(0, p, tm, tn, tb);
-        cluster_sync_all();
-        const int r0 = BM * tb / p.cluster, rows = BM * (tb + 1) / p.cluster - r0, vecs = bn / 4;
-        for (int e = threadIdx.x; e < rows * vecs; e += tc_threads(MODE)) {
-            const int r = r0 + e / vecs, c = e % vecs * 4, row = tm * BM + r, col = tn * bn + c;
-            if (row >= p.M || col >= p.N) continue;
-            const float4 sum = sum_slices(smem_base + SmemLayout::ring + (uint32_t)(r * PART_LD + c) * 4, p.cluster);
-            const uint2 q = make_uint2(pack2(sum.x, sum.y, p.is_bf16), pack2(sum.z, sum.w, p.is_bf16));
-            uint16_t* out = static_cast<uint16_t*>(p.d) + (size_t)row * p.N + col;
-            if (p.vec_out) {
-                *reinterpret_cast<uint2*>(out) = q;
-            } else {
-                out[0] = (uint16_t)q.x;
-                if (col + 1 < p.N) out[1] = (uint16_t)(q.x >> 16);
-                if (col + 2 < p.N) out[2] = (uint16_t)q.y;
-                if (col + 3 < p.N) out[3] = (uint16_t)(q.y >> 16);
-            }
-        }
-        cluster_sync_all();  // the others have read this CTA's part
-    }
 }
 
 // ---------------------------------------------------------------------------------
@@ -633,9 +584,7 @@ bool opt_in_shared_memory() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
-        for (auto kernel : {tc_gemm_kernel<TC_STORE, BN>, tc_gemm_kernel<TC_BIAS, BN>, tc_gemm_kernel<TC_STORE, 0>, tc_gemm_kernel<TC_BIAS, 0>, tc_gemm_kernel<TC_PLAIN, 0>, tc_gemm_kernel<TC_STORE, BN, false, SCHED_PANELS>,
-                            tc_gemm_kernel<TC_BIAS, BN, false, SCHED_PANELS>, tc_gemm_kernel<TC_STORE, BN, false, SCHED_CLUSTER>, tc_gemm_kernel<TC_STORE, 0, false, SCHED_CLUSTER>,
-                            tc_gemm_kernel<TC_STORE, 0, true, SCHED_CLUSTER>,
+        for (auto kernel : {tc_gemm_kernel<TC_STORE, BN>, tc_gemm_kernel<TC_BIAS, BN>, tc_gemm_kernel<TC_STORE, 0>, tc_gemm_kernel<TC_BIAS, 0>, tc_gemm_kernel<TC_PLAIN, 0>, tc_gemm_kernel<TC_STORE, BN, false, true>, tc_gemm_kernel<TC_BIAS, BN, false, true>,
                             tc_gemm_kernel<TC_STORE, 0, true>, tc_gemm_kernel<TC_BIAS, 0, true>, tc_gemm_kernel<TC_PLAIN, 0, true>})
             if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess) {
                 cudaGetLastError();
@@ -735,8 +684,6 @@ int tile_columns(uint64_t tiles_m, uint64_t N, uint64_t batch, uint64_t num_kb, 
     return best;
 }
 
-std::atomic<int> g_cluster{1};  // 0: no clusters of slices (tests, A/B timing)
-
 bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, int fuse = 0, const void* bias = nullptr, void* D2 = nullptr) {
     const void *A = c.A, *B = c.B;
     const bool a_mn = c.a_mn, b_mn = c.b_mn;
@@ -763,25 +710,17 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     p.b_keep = keep_b_ctas(p.tiles_m, p.tiles_n, p.num_kb, (int)batch, std::min(grid, (int)std::min<uint64_t>(batch * p.tiles_m * p.tiles_n, 1u << 30)));
     // few output tiles: cut K into slices that run as the batches of this launch
     int slices = 1;
-    p.cluster = 0;
     const int bn_whole = p.b_keep ? p.bn : tile_columns((uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid);
     const bool panels = p.bn == BN && bn_whole == BN && !c.d_plain && keep_panels((uint64_t)p.tiles_m, (uint64_t)p.tiles_n, p.num_kb, batch, grid);
     if (batch == 1 && !fuse && !p.b_keep) {
-        const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n;
-        const double kb = kb_cost(p.bn), whole = tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid);
-        slices = splitk_slices(tiles, K, BK, grid);
-        if (slices == 1) slices = splitk_short(tiles, (uint64_t)p.num_kb, grid, kb, whole - kSplitFixed16);
-        double cost = whole;
-        if (slices > 1) cost = std::min(cost, (double)((tiles * slices + grid - 1) / grid * ((p.num_kb + slices - 1) / slices)) * kb + kSplitFixed16 + 0.1 * slices);
-        if (g_cluster.load(std::memory_order_relaxed))
-            p.cluster = cluster_slices(tiles, (uint64_t)p.num_kb, grid, kb, kClusterFixed16, cost, [](int n) {
-                return resident_clusters(reinterpret_cast<const void*>(tc_gemm_kernel<TC_STORE, BN, false, SCHED_CLUSTER>), tc_threads(TC_STORE), TC_SMEM_BYTES, n);
-            });
-        if (p.cluster) slices = p.cluster;
+        slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
+        if (slices == 1)
+            slices = splitk_short((uint64_t)p.tiles_m * p.tiles_n, (uint64_t)p.num_kb, grid, kb_cost(p.bn),
+                                  tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid) - kSplitFixed16);
     }
     StreamWorkspace partial;
     const uint64_t n_pitch = (N + 3) / 4 * 4;
-    if (slices > 1 && !p.cluster && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) slices = 1;
+    if (slices > 1 && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) slices = 1;
     if (slices > 1) {
         p.split_kb = (p.num_kb + slices - 1) / slices;
         p.num_kb = p.split_kb;
@@ -808,10 +747,7 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     if (!oka || !okb) return false;
     p.d_plain = slices > 1 ? 0 : c.d_plain;
     p.d = D;
-    p.vec_out = N % 4 == 0 && (uintptr_t)D % 8 == 0 ? 1 : 0;
-    if (p.cluster) {
-        md = ma;  // not used
-    } else if (slices > 1) {
+    if (slices > 1) {
         if (!make_map_3d(&md, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, partial.ptr, M, N, batch, M * n_pitch, 32, sw, n_pitch)) return false;
     } else if (p.d_plain) {
         md = ma;  // not used
@@ -833,14 +769,13 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     if (grid > p.num_tiles) grid = p.num_tiles;
     if (p.b_keep) grid = p.b_keep * p.tiles_n;
     const bool full = p.bn == BN;
-    const auto kernel = p.cluster ? (drain ? tc_gemm_kernel<TC_STORE, 0, true, SCHED_CLUSTER> : full ? tc_gemm_kernel<TC_STORE, BN, false, SCHED_CLUSTER> : tc_gemm_kernel<TC_STORE, 0, false, SCHED_CLUSTER>)
-                        : panels ? (fuse ? tc_gemm_kernel<TC_BIAS, BN, false, SCHED_PANELS> : tc_gemm_kernel<TC_STORE, BN, false, SCHED_PANELS>)
+    const auto kernel = panels ? (fuse ? tc_gemm_kernel<TC_BIAS, BN, false, true> : tc_gemm_kernel<TC_STORE, BN, false, true>)
                         : drain ? (p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0, true> : (fuse ? tc_gemm_kernel<TC_BIAS, 0, true> : tc_gemm_kernel<TC_STORE, 0, true>))
                         : p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0>
                                   : (fuse ? (full ? tc_gemm_kernel<TC_BIAS, BN> : tc_gemm_kernel<TC_BIAS, 0>) : (full ? tc_gemm_kernel<TC_STORE, BN> : tc_gemm_kernel<TC_STORE, 0>));
-    launch_clusters(kernel, p.cluster ? p.num_tiles : grid, tc_threads(p.d_plain ? TC_PLAIN : TC_STORE), TC_SMEM_BYTES, p.cluster, ma, mb, md, md2, p, err, tag);
+    launch_kernel(kernel, grid, tc_threads(p.d_plain ? TC_PLAIN : TC_STORE), TC_SMEM_BYTES, ctx().stream, ma, mb, md, md2, p, err, tag);
     check_launch(where);
-    if (slices > 1 && !p.cluster) splitk_reduce(is_bf16 ? 0 : 1, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
+    if (slices > 1) splitk_reduce(is_bf16 ? 0 : 1, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
     return true;
 }
 
@@ -888,32 +823,6 @@ bool make_map_3d(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes, con
     CUresult r = enc(map, type, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
-}
-
-int resident_clusters(const void* kernel, int threads, size_t shared, int n) {
-    static std::mutex mu;
-    static std::unordered_map<const void*, int> known[64][CLUSTER_MOST + 1];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    std::lock_guard<std::mutex> lock(mu);
-    const auto it = known[dev][n].find(kernel);
-    if (it != known[dev][n].end()) return it->second;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(sm_count() / n * n));
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = shared;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)n;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int most = 0;
-    if (cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        most = 0;
-    }
-    return known[dev][n][kernel] = most;
 }
 
 int splitk_slices(uint64_t tiles, uint64_t K, int block_k, int sms) {
@@ -1427,8 +1336,6 @@ extern "C" int mx_debug_gemm_max_resident_pairs(void) { return mx::tc2::max_resi
 extern "C" void mx_debug_set_gemm_group_m(int rows) { mx::g_group_m.store(rows > 0 ? rows : 16, std::memory_order_relaxed); }
 // 1 (default): products with a reduction of at most 256 run with the B panel resident in shared memory; 0: general schedule
 extern "C" void mx_debug_set_gemm_keep_b(int on) { mx::g_keep_b.store(on ? 1 : 0, std::memory_order_relaxed); }
-// 1 (default): the slices of a split 16-bit product are summed inside a cluster where they fit one; 0: always by a second launch
-extern "C" void mx_debug_set_gemm_cluster(int on) { mx::g_cluster.store(on ? 1 : 0, std::memory_order_relaxed); }
 extern "C" int mx_debug_gemm_keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, int ctas) { return mx::keep_b_ctas(tiles_m, tiles_n, num_kb, batch, ctas); }
 extern "C" int mx_debug_splitk_slices(size_t tiles, size_t k, int block_k, int sms) { return mx::tc::splitk_slices(tiles, k, block_k, sms); }
 extern "C" int mx_debug_matmul_forward_path(size_t num_els, const size_t* host_metadata, const void* a, const void* b, const void* out, int* a_mn_major,

@@ -589,9 +589,11 @@ int tile_columns(uint64_t tiles_m, uint64_t N, uint64_t batch, int grid) {
 }
 // what the second launch of a split-K product costs, in k-blocks (about 0.9 us each on one CTA)
 constexpr double kSplitFixed32 = 3.0;
-// and the sum inside a cluster
-constexpr double kClusterFixed32 = 1.5;
-std::atomic<int> g_cluster{1};  // 0: no clusters of slices (tests, A/B timing)
+// and the sum inside a cluster.  Where both forms split, the one with a second launch is the faster since that closes up with the first (128 x 300 x 784
+// 10.9 us, 12.2 in a cluster; 512 x 1024 x 1024 15.5, 15.9); a cluster takes what it leaves whole: 300 x 784 x 8192 70 us whole, 50 in
+// clusters; ragged 1001 x 1003 x 1005 33, 31.
+constexpr double kClusterFixed32 = 4.0;
+std::atomic<int> g_cluster{1};  // 0: no clusters of slices, 2: wherever they fit (tests, A/B timing)
 
 // D[M,N] = sum_k Aop[m,k] * Bop[n,k]; K-major operand = row-major [MN, K], MN-major = row-major [K, MN].
 bool launch(const TcProduct& c, void* D, const char* where) {
@@ -625,9 +627,9 @@ bool launch(const TcProduct& c, void* D, const char* where) {
         const double kb = (128 + p.bn) / 256.0, whole = tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, grid) * p.num_kb;
         if (!c.sum_batches) slices = splitk_slices(tiles, K, BK, grid);
         if (slices == 1) slices = splitk_short(tiles, (uint64_t)p.num_kb, grid, kb, whole - kSplitFixed32);
-        double cost = whole;
-        if (slices > 1) cost = std::min(cost, (double)((tiles * slices + grid - 1) / grid * ((p.num_kb + slices - 1) / slices)) * kb + kSplitFixed32 + 0.1 * slices);
-        if (g_cluster.load(std::memory_order_relaxed))
+        const int form = g_cluster.load(std::memory_order_relaxed);
+        double cost = form == 2 ? 1e30 : whole;
+        if (form == 2 || (form && slices == 1))
             p.cluster = cluster_slices(tiles, (uint64_t)p.num_kb, grid, kb, kClusterFixed32, cost,
                                        [](int n) { return resident_clusters(reinterpret_cast<const void*>(tc_gemm_f32_kernel<0, true>), THREADS, SMEM_BYTES, n); });
         if (p.cluster) slices = p.cluster;
@@ -698,5 +700,5 @@ bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t 
 
 }  // namespace mx
 
-// 1 (default): the slices of a split f32 product are summed inside a cluster where they fit one; 0: always by a second launch
+// 1 (default): f32 products that are not split in two launches are split into the CTAs of a cluster where that pays; 0: never; 2: wherever they fit
 extern "C" void mx_debug_set_gemm_f32_cluster(int on) { mx::g_cluster.store(on ? 1 : 0, std::memory_order_relaxed); }

