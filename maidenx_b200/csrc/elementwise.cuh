@@ -930,6 +930,11 @@ struct EwChanParams {
     int vector[3];              // [1], [2]: the input has the output's layout
     int s_outer[3], s_channel[3];
 };
+struct EwRepeatParams {
+    uint32_t n, q;    // elements; extent of the innermost dim
+    FastDiv31 q_div;
+    int repeated[3];  // [1], [2]: the input is one row for all rows, else it has the output's layout
+};
 constexpr int kEwChanUnroll = 4;
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, const T* b, O* out, EwChanParams P) {
@@ -982,11 +987,54 @@ __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, co
     }
 }
 
+// Two inputs of ragged rows, each the output's own layout or the same row for all of them (a bias, a norm's weights): one division by multiplication a
+// vector, the repeated row from L1 by elements, four vectors a thread.  An instantiation of the kernel above for it would have the constants'
+// registers too (94 instead of 79 in 16 bits).
+template <class F, class T, class O, int VEC>
+__global__ void __launch_bounds__(kEwThreads) ew_repeat_kernel(F f, const T* a, const T* b, O* out, EwRepeatParams P) {
+    after_previous_kernel();
+    constexpr int U = kEwChanUnroll;
+    const uint32_t first = (blockIdx.x * U * kEwThreads + threadIdx.x) * VEC;
+    Vec<T, VEC> va[U], vb[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const uint32_t i0 = first + u * kEwThreads * VEC;
+        if (i0 >= P.n) continue;
+        const uint32_t col = i0 - P.q_div.div(i0) * P.q;
+        auto load = [&](const T* p, int repeated, Vec<T, VEC>& v) {
+            if (repeated) {
+#pragma unroll
+                for (int j = 0; j < VEC; j++) v.v[j] = p[col + j < P.q ? col + j : col + j - P.q];
+            } else if (i0 + VEC <= P.n) {
+                v = ld_vec<T, VEC>(p + i0);
+            } else {
+#pragma unroll
+                for (int j = 0; j < VEC; j++)
+                    if (i0 + j < P.n) v.v[j] = p[i0 + j];
+            }
+        };
+        load(a, P.repeated[1], va[u]);
+        load(b, P.repeated[2], vb[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const uint32_t i0 = first + u * kEwThreads * VEC;
+        if (i0 + VEC <= P.n) {
+            st_vec<O, VEC>(out + i0, apply_vec<F, T, O, 2, VEC>(f, va[u], vb[u]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < VEC; j++)
+                if (i0 + j < P.n) out[i0 + j] = f(va[u].v[j], vb[u].v[j]);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------
 // launcher
 // ---------------------------------------------------------------------------------
 // The dense-output kernel's parameters as those of the kernel of rows and channels; false when they are not of its form.
 bool ew_fill_chan_params(const EwDenseParams& D, int vec, EwChanParams& P);
+bool ew_fill_repeat_params(const EwDenseParams& D, int vec, EwRepeatParams& P);
 // Fills the parameters for the dense-output kernel; false when the output is not dense from `out` on or not vector-aligned, or
 // an offset does not fit 31 bits.
 bool ew_fill_dense_params(const EwPlan& pl, size_t in_size, size_t out_size, const void* out, const void* a, const void* b, EwDenseParams& P);
@@ -1134,6 +1182,11 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                     EwChanParams C;
                     if (ew_fill_chan_params(D, VEC, C)) {
                         launch_kernel(ew_chan_kernel<F, T, O, VEC>, (uint32_t)((vecs + kEwThreads * kEwChanUnroll - 1) / (kEwThreads * kEwChanUnroll)), kEwThreads, 0, s, f, a, b, out, C);
+                        break;
+                    }
+                    EwRepeatParams Q;
+                    if (ew_fill_repeat_params(D, VEC, Q)) {
+                        launch_kernel(ew_repeat_kernel<F, T, O, VEC>, (uint32_t)((vecs + kEwThreads * kEwChanUnroll - 1) / (kEwThreads * kEwChanUnroll)), kEwThreads, 0, s, f, a, b, out, Q);
                         break;
                     }
                 }

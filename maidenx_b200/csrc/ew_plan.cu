@@ -361,6 +361,21 @@ bool ew_fill_chan_params(const EwDenseParams& D, int vec, EwChanParams& P) {
     return true;
 }
 
+// The same for rows that repeat: the plan has merged the dims before the innermost one where no operand tells them apart.
+bool ew_fill_repeat_params(const EwDenseParams& D, int vec, EwRepeatParams& P) {
+    if (D.nd < 2 || D.q < (uint32_t)vec) return false;
+    for (int k = 1; k < 3; k++) {
+        bool repeated = D.kind[k] == EWD_STEP && D.st[k][D.nd - 1] == 1;
+        for (int d = 0; d < D.nd - 1; d++) repeated = repeated && D.st[k][d] == 0;
+        if (D.kind[k] != EWD_VECTOR && !repeated) return false;
+        P.repeated[k] = repeated ? 1 : 0;
+    }
+    P.n = D.n;
+    P.q = D.q;
+    P.q_div.init(P.q);
+    return true;
+}
+
 void ew_fill_gen_params(const EwPlan& pl, EwGenParams& P) {
     P.nd = pl.nd;
     P.n = pl.n;

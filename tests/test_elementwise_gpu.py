@@ -371,7 +371,7 @@ def test_flat_operands_at_unaligned_offsets(oracle, cuda, dt):
 @pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16, D.F64, D.I16], ids=lambda d: d.name)
 @pytest.mark.parametrize("q", ["vec", "vec+1", 49, 197, 1023])
 def test_operands_constant_along_ragged_rows(oracle, cuda, dt, q):
-    """Per-row and per-channel operands of rows that are no whole vectors, on either side and on both, with an outer stride of their own, as a
+    """Per-row and per-channel operands of rows that are no whole vectors, and a row that is the same for all of them, on either side and on both, with an outer stride of their own, as a
     comparison and in place; tensors that end inside a vector, whose last vector starts in the row before, and whose rows are two."""
     vec = 16 // dt.size
     q = {"vec": vec, "vec+1": vec + 1}.get(q, q)
@@ -381,7 +381,8 @@ def test_operands_constant_along_ragged_rows(oracle, cuda, dt, q):
     c = 7
     o = r // c + 1
     layouts = [("row", [r, q], [q, 1], [1, 0]), ("row-strided", [r, q], [q, 1], [3, 0]), ("channel", [o, c, q], [c * q, q, 1], [0, 1, 0]),
-               ("outer", [o, c, q], [c * q, q, 1], [1, 0, 0]), ("both", [o, c, q], [c * q, q, 1], [c + 2, 1, 0]), ("two-rows", [2, least + 5], [least + 5, 1], [1, 0])]
+               ("outer", [o, c, q], [c * q, q, 1], [1, 0, 0]), ("both", [o, c, q], [c * q, q, 1], [c + 2, 1, 0]), ("two-rows", [2, least + 5], [least + 5, 1], [1, 0]),
+               ("repeated", [r, q], [q, 1], [0, 1]), ("repeated-two-rows", [2, least + 5], [least + 5, 1], [0, 1])]
     for name, dims, dense, const in layouts:
         n = H.numel(dims)
         size = 1 + sum((d - 1) * s for d, s in zip(dims, const))
