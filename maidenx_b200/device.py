@@ -4,8 +4,8 @@
 58-75): `cuda_malloc` on creation, `cuda_free` on release, base pointer handed to the ops,
 element offsets travelling in the metadata.  `dispatch` mirrors what every generated
 function of crates/maidenx_core/src/be/ops/*.rs does around an op call: select the device,
-upload the metadata block with cuda_malloc + cuda_memcpy_h2d, call `cuda_<op>_<dtype>`,
-free the block.
+provide the metadata block (mx_dispatch_begin: a slot of pinned memory, or cuda_malloc +
+cuda_memcpy_h2d), call `cuda_<op>_<dtype>`, give the block back.
 """
 from __future__ import annotations
 
