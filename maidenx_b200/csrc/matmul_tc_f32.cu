@@ -31,7 +31,7 @@
 //   warps 2-5   the epilogue: per chunk tcgen05.ld of the warp's 32 rows x BN columns, added into BN registers per
 //               thread; after the tile's last chunk the totals go through a swizzled 4 KB staging tile to TMA stores.
 // Operands may be K-major ([MN, K] row-major) or MN-major ([K, MN] row-major, loaded as [32 K-rows x 32 MN] boxes),
-// which covers x . W^T, g . W and x^T . g without transposed copies.  No cluster launch, no multicast.
+// which covers x . W^T, g . W and x^T . g without transposed copies.  Clusters only for the slices of one product; no multicast.
 // Infinities and NaNs, for which the split has no form, are found in the totals and their tiles computed again (redo_tile).
 // Every mbarrier wait is bounded (see tc_ptx.cuh); on expiry all roles fall through to the common exit.
 #include <cuda.h>
