@@ -39,6 +39,7 @@
 #include <atomic>
 #include <algorithm>
 #include <mutex>
+#include <unordered_map>
 
 #include "matmul_tc.cuh"
 #include "tc_cluster.cuh"
@@ -688,6 +689,34 @@ bool launch(const TcProduct& c, void* D, const char* where) {
 }
 
 }  // namespace
+
+namespace tc {
+int resident_clusters(const void* kernel, int threads, size_t shared, int n) {
+    static std::mutex mu;
+    static std::unordered_map<const void*, int> known[64][CLUSTER_MOST + 1];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = known[dev][n].find(kernel);
+    if (it != known[dev][n].end()) return it->second;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sm_count() / n * n));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = shared;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)n;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int most = 0;
+    if (cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        most = 0;
+    }
+    return known[dev][n][kernel] = most;
+}
+}  // namespace tc
 
 bool tc_launch_f32(const TcProduct& c, void* out, const char* where) { return launch(c, out, where); }
 
