@@ -47,6 +47,8 @@ int mx_debug_splitk_slices(size_t tiles, size_t k, int block_k, int sms);
 /* f32 tensor-core products whose reduction is cut into the CTAs of a cluster: 1 = where that pays and a second launch does not (default), 0 =
  * nowhere, 2 = wherever one fits. */
 void mx_debug_set_gemm_f32_cluster(int on);
+/* 1 (default): long f32 reductions multiply the large part of A by both parts of B in one instruction; 0: never. */
+void mx_debug_set_gemm_f32_wide(int on);
 /* Writes `value` (0 clears) into the calling thread's tensor-core error word the way a kernel of an earlier launch
  * whose bounded wait ran out would have left it.  Returns 0, or -1 without a usable device. */
 int mx_debug_tc_gemm_poke_status(int value);

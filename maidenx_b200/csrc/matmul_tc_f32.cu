@@ -4,8 +4,10 @@
 // Every f32 operand element x is used as two tf32 values
 //     big   = x with the low 13 significand bits dropped (what the tensor core reads from the raw f32 bits),
 //     small = x - big   (exact in f32; its own low bits are again dropped by the tensor core),
-// and each k-step issues three MMAs into the same TMEM accumulator:
-//     a_small * b_big  +  a_big * b_small  +  a_big * b_big.
+// and each k-step multiplies
+//     a_small * b_big  +  a_big * b_small  +  a_big * b_big
+// by three MMAs into one TMEM accumulator, or (long reductions, Params::wide) by two: a_big by [b_big | b_small], which lie behind one another, into an
+// accumulator of twice the columns, and a_small * b_big into its second half; the halves meet in the epilogue's registers.
 // The dropped term a_small * b_small and the truncation of `small` are each below 2^-21 of |a * b|, so a dot
 // product agrees with f32 arithmetic to a few 1e-7 relative to sum |a_k * b_k| (the stated f32 matmul tolerance is
 // 1e-4).
@@ -25,7 +27,7 @@
 //               into a ring of stages;
 //   warps 6-9   splitter: when a stage has landed, read the raw tiles and write the `small` tiles beside them
 //               (element-wise, so the swizzled placement carries over unchanged), then hand the stage to
-//   warp 1      the MMA issuer: 4 k-steps x 3 tcgen05.mma (M128, N up to BN, K8) per k-block into one of two TMEM
+//   warp 1      the MMA issuer: 4 k-steps x 3 (wide: 2) tcgen05.mma (M128, N up to BN, wide 2 BN, K8) per k-block into one of two TMEM
 //               accumulators, switching accumulator every chunk_kb k-blocks; commits the stage back to the
 //               producer and each finished chunk to
 //   warps 2-5   the epilogue: per chunk tcgen05.ld of the warp's 32 rows x BN columns, added into BN registers per
@@ -55,12 +57,12 @@ constexpr int UMMA_K = 8;                      // tf32: 32 bytes of K per instru
 constexpr int STAGES = 3, MAX_STAGES = 4;      // of 128- and of 64-column tiles
 constexpr int A_TILE = BM * BK * 4;            // 16 KB
 constexpr int B_TILE = BN * BK * 4;
-constexpr int STAGE_BYTES = 2 * (A_TILE + B_TILE);  // [A raw | B raw | A small | B small] of a 128-column tile
+constexpr int STAGE_BYTES = 2 * (A_TILE + B_TILE);  // [A raw | A small | B raw | B small] of a 128-column tile
 constexpr int EPI_WARPS = 4, SPLIT_WARPS = 4;
 constexpr int EPI_CHUNK_COLS = 32;             // 32 f32 = 128 bytes per staged row
 constexpr int EPI_STAGE_BYTES = 32 * EPI_CHUNK_COLS * 4;  // 4 KB per warp per buffer
 constexpr int THREADS = 32 * (2 + EPI_WARPS + SPLIT_WARPS);
-constexpr int TMEM_COLS = 2 * BN;              // two f32 accumulators
+constexpr int TMEM_COLS = 4 * BN;              // two f32 accumulators, each [big x big | products with a small factor] (Params::wide)
 constexpr int GROUP_M = 16;
 constexpr int CHUNK_FAST = 4;
 constexpr int MN_CHUNK_BYTES = BK * 128;       // one [32 K-rows x 32 MN-elements] box
@@ -101,6 +103,7 @@ struct Params {
     int bn;         // columns of an output tile: 64 or 128
     int stages;     // of the ring
     int raw_bytes;  // what TMA delivers per stage: A and bn rows of B
+    int wide;       // 1: big x [big | small] in one instruction, the products with a small factor in an accumulator of their own (see kWideLeast)
     int split_kb;   // > 0: split-K; batch s of the launch reduces the k-blocks [s * split_kb, (s + 1) * split_kb) of one product
     int kb_per_z;   // > 0: the reduction runs over the operands' batches too: k-block i is block i % kb_per_z of batch i / kb_per_z
     int d_plain;    // != 0: the output's rows (or base) are not 16-byte multiples: the epilogue warps write them to `out` themselves
@@ -272,7 +275,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     }
                     mbar_expect_tx(full_bar(stage), raw_bytes);
                     const uint32_t sa = smem_base + Smem::stages + stage * 2 * raw_bytes;
-                    const uint32_t sb = sa + A_TILE;
+                    const uint32_t sb = sa + 2 * A_TILE;
                     int block = tb * p.split_kb + kb;  // a block past the end of K (or of the batches) is all fill: zeros
                     if (p.kb_per_z) {
                         za = zb = block / p.kb_per_z;
@@ -300,7 +303,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (lane == 0) {
-            const uint32_t idesc = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, bn);
+            const uint32_t idesc = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, bn), idesc_wide = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, 2 * bn);
             // K-major: 8 floats further along the 128-byte row; MN-major: the next group of eight K-rows
             const uint64_t a_kstep = p.a_mn ? (1024 >> 4) : (32 >> 4), b_kstep = p.b_mn ? (1024 >> 4) : (32 >> 4);
             int stage = 0, acc = 0;
@@ -313,7 +316,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
+                    const uint32_t d_tmem = tmem_base + (uint32_t)acc * 2 * BN;
                     const int kb1 = min(kb0 + chunk_kb, p.num_kb);
                     for (int kb = kb0; kb < kb1; kb++) {
                         // the raw tiles (TMA) and the small tiles (splitter) are both operands
@@ -326,12 +329,17 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         // K-major: rows of 32 floats, groups of eight rows 1024 bytes apart.  MN-major: 32-byte-atom swizzle,
                         // groups of four K-rows 512 bytes apart, 128-byte-wide MN chunks one box (4 KB) apart.
                         const uint64_t a_big = p.a_mn ? smem_desc_sw128_atom32(s0, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0, 16, 1024);
-                        const uint64_t b_big = p.b_mn ? smem_desc_sw128_atom32(s0 + A_TILE, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + A_TILE, 16, 1024);
-                        const uint64_t a_small =
-                            p.a_mn ? smem_desc_sw128_atom32(s0 + raw_bytes, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + raw_bytes, 16, 1024);
-                        const uint64_t b_small = p.b_mn ? smem_desc_sw128_atom32(s0 + raw_bytes + A_TILE, MN_CHUNK_BYTES, 512)
-                                                        : smem_desc_sw128(s0 + raw_bytes + A_TILE, 16, 1024);
-                        if (chunk_kb == 1) {
+                        const uint32_t s_b = s0 + 2 * A_TILE, s_bs = s_b + (raw_bytes - A_TILE);
+                        const uint64_t b_big = p.b_mn ? smem_desc_sw128_atom32(s_b, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s_b, 16, 1024);
+                        const uint64_t a_small = p.a_mn ? smem_desc_sw128_atom32(s0 + A_TILE, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + A_TILE, 16, 1024);
+                        const uint64_t b_small = p.b_mn ? smem_desc_sw128_atom32(s_bs, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s_bs, 16, 1024);
+                        if (p.wide) {  // the small part of B lies behind the raw one: one instruction of twice the columns multiplies a_big by both
+#pragma unroll
+                            for (int k = 0; k < BK / UMMA_K; k++) {
+                                umma_tf32(d_tmem, a_big + a_kstep * k, b_big + b_kstep * k, idesc_wide, (kb != kb0) || (k != 0));
+                                umma_tf32(d_tmem + bn, a_small + a_kstep * k, b_big + b_kstep * k, idesc, 1);
+                            }
+                        } else if (chunk_kb == 1) {
 #pragma unroll
                             for (int k = 0; k < BK / UMMA_K; k++) {
                                 umma_tf32(d_tmem, a_small + a_kstep * k, b_big + b_kstep * k, idesc, k != 0);
@@ -384,11 +392,17 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     break;
                 }
                 tc_fence_after();
-                const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * BN;
+                const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)acc * 2 * BN;
 #pragma unroll
                 for (int c = 0; c < BN / 32; c++) {
                     if (c * 32 >= bn) break;
                     uint32_t v[32];
+                    if (p.wide) {  // the sum of the small products first
+                        tmem_ld_32x32b_x32(t_row + bn + c * 32, v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; j++) total[c * 32 + j] += __uint_as_float(v[j]);
+                    }
                     tmem_ld_32x32b_x32(t_row + c * 32, v);
                     tmem_ld_wait();
 #pragma unroll
@@ -474,24 +488,25 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     ok = false;
                     break;
                 }
-                const uint4* raw = reinterpret_cast<const uint4*>(smem + Smem::stages + stage * 2 * raw_bytes);
-                uint4* small = reinterpret_cast<uint4*>(smem + Smem::stages + stage * 2 * raw_bytes + raw_bytes);
+                uint4* words = reinterpret_cast<uint4*>(smem + Smem::stages + stage * 2 * raw_bytes) + t;  // [A raw | A small | B raw | B small]
+                constexpr int A_WORDS = A_TILE / 16, STEP = 32 * SPLIT_WARPS;
+                auto split = [](const uint4& q) { return make_uint4(small_part(q.x), small_part(q.y), small_part(q.z), small_part(q.w)); };
                 if constexpr (BN_T != 0) {
-                    constexpr int STEPS = (A_TILE + BN_T * BK * 4) / 16 / (32 * SPLIT_WARPS);
+                    constexpr int B_WORDS = BN_T * BK * 4 / 16;
 #pragma unroll 8
-                    for (int i = 0; i < STEPS; i++) {
-                        const uint4 q = raw[t + i * 32 * SPLIT_WARPS];
-                        small[t + i * 32 * SPLIT_WARPS] = make_uint4(small_part(q.x), small_part(q.y), small_part(q.z), small_part(q.w));
-                    }
+                    for (int i = 0; i < A_WORDS; i += STEP) words[i + A_WORDS] = split(words[i]);
+#pragma unroll 8
+                    for (int i = 0; i < B_WORDS; i += STEP) words[2 * A_WORDS + i + B_WORDS] = split(words[2 * A_WORDS + i]);
                 } else {
-                    const int steps = raw_bytes / 16 / (32 * SPLIT_WARPS);
-                    for (int i0 = 0; i0 < steps; i0 += 4) {  // 12 or 16 steps; loads first: the compiler cannot tell the two tiles apart
+                    const int b_words = bn * BK * 4 / 16;
+                    for (int i0 = 0; i0 < A_WORDS + b_words; i0 += 4 * STEP) {  // loads first: the compiler cannot tell the tiles apart
+                        uint4* from = words + (i0 < A_WORDS ? i0 : A_WORDS + i0);
+                        const int to = i0 < A_WORDS ? A_WORDS : b_words;
                         uint4 q[4];
 #pragma unroll
-                        for (int i = 0; i < 4; i++) q[i] = raw[t + (i0 + i) * 32 * SPLIT_WARPS];
+                        for (int i = 0; i < 4; i++) q[i] = from[i * STEP];
 #pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            small[t + (i0 + i) * 32 * SPLIT_WARPS] = make_uint4(small_part(q[i].x), small_part(q[i].y), small_part(q[i].z), small_part(q[i].w));
+                        for (int i = 0; i < 4; i++) from[i * STEP + to] = split(q[i]);
                     }
                 }
                 fence_proxy_async_smem();  // the tensor core reads these through the async proxy
@@ -590,6 +605,12 @@ int tile_columns(uint64_t tiles_m, uint64_t N, uint64_t batch, int grid) {
 }
 // what the second launch of a split-K product costs, in k-blocks (about 0.9 us each on one CTA)
 constexpr double kSplitFixed32 = 3.0;
+// k-blocks from which on big x [big | small] is one instruction of twice the columns: two instructions a k-step instead of three and a third fewer reads of A,
+// for twice the accumulator columns to empty every four k-blocks.  32 x (1152 x 196 x 256) 37.3 us, 35.7 so; 4096 x 4096 x 256 59.0, 57.3, x 64 22.6,
+// 24.0.  Slices of a split product are short and gain nothing (256 x 512 x 2048 12.9, 13.1).  Error of 32 convolutions [256 x 1152] . [1152 x 196]
+// against 64 bits 9.2e-7 (1.0e-6 by three).
+constexpr int kWideLeast = 8;
+std::atomic<int> g_wide{1};  // 0: never (tests, A/B timing)
 // and the sum inside a cluster.  Where both forms split, the one with a second launch is the faster since that closes up with the first (128 x 300 x 784
 // 10.9 us, 12.2 in a cluster; 512 x 1024 x 1024 15.5, 15.9); a cluster takes what it leaves whole: 300 x 784 x 8192 70 us whole, 50 in
 // clusters; ragged 1001 x 1003 x 1005 33, 31.
@@ -680,6 +701,7 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.out = static_cast<float*>(slices > 1 && !p.cluster ? partial.ptr : D);
     p.out_ld = (int64_t)(slices > 1 && !p.cluster ? n_pitch : N);
     if (grid > p.num_tiles) grid = p.num_tiles;
+    p.wide = p.chunk_kb == CHUNK_FAST && slices == 1 && p.num_kb >= kWideLeast && g_wide.load(std::memory_order_relaxed) ? 1 : 0;
     const bool fixed = p.bn == BN && !p.d_plain && p.chunk_kb == CHUNK_FAST;
     const auto kernel = p.cluster ? (fixed ? tc_gemm_f32_kernel<BN, true> : tc_gemm_f32_kernel<0, true>) : (fixed ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>);
     launch_clusters(kernel, p.cluster ? p.num_tiles : grid, THREADS, SMEM_BYTES, p.cluster, ma, mb, md, p, err, tag);
@@ -731,3 +753,4 @@ bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t 
 
 // 1 (default): f32 products that are not split in two launches are split into the CTAs of a cluster where that pays; 0: never; 2: wherever they fit
 extern "C" void mx_debug_set_gemm_f32_cluster(int on) { mx::g_cluster.store(on ? 1 : 0, std::memory_order_relaxed); }
+extern "C" void mx_debug_set_gemm_f32_wide(int on) { mx::g_wide.store(on ? 1 : 0, std::memory_order_relaxed); }

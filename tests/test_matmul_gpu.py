@@ -474,6 +474,35 @@ def test_slices_summed_in_a_cluster(cuda, dt, case):
         assert err <= 2e-6, err  # the split product's
 
 
+@pytest.mark.parametrize("case", [
+    # M, N, K, majors: the shortest reduction of the form, one chunk more and less than whole, a last k-block that is not full; tiles of 64 and 128 columns with edges; no split
+    (2048, 1600, 256, "kk"), (1800, 1540, 260, "km"), (2048, 1600, 392, "mm"), (5000, 64, 512, "mk"), (2432, 1664, 1000, "km"), (130, 19000, 288, "kk")],
+    ids=lambda c: "x".join(map(str, c)))
+def test_f32_products_with_both_parts_of_b_in_one_instruction(cuda, case):
+    """Next to float64: within the split product's bound, and no further off than the form of three instructions by more than rounding."""
+    from maidenx_b200 import _lib, device
+    lib = _lib.load()
+    m, n, k, majors = case
+    rng = np.random.default_rng(m + n + k)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    am, bm = a if majors[0] == "k" else a.T, b.T if majors[1] == "k" else b
+    meta = [2, 2, 2, m, n, m, k, k, n, *([k, 1] if majors[0] == "k" else [1, m]), *([1, k] if majors[1] == "k" else [n, 1]), 0, 0]
+    ref = a.astype(np.float64) @ b.astype(np.float64)
+    err = []
+    try:
+        for on in (0, 1):
+            lib.mx_debug_set_gemm_f32_wide(on)
+            bufs = [device.CudaBuffer.from_host(np.ascontiguousarray(x).reshape(-1)) for x in (am, bm, np.zeros(m * n, np.float32))]
+            device.dispatch("matmul", "f32", meta, m * n, "META", bufs[0].ptr, bufs[1].ptr, bufs[2].ptr)
+            out = bufs[2].to_host(np.float32, m * n).reshape(m, n)
+            err.append(np.linalg.norm(out - ref) / np.linalg.norm(ref))
+            for x in bufs:
+                x.free()
+    finally:
+        lib.mx_debug_set_gemm_f32_wide(1)
+    assert max(err) <= 2e-6 and err[1] <= 1.02 * err[0], err
+
+
 @pytest.mark.parametrize("off", [0, 1, 3, 4, 6, 7])
 @pytest.mark.parametrize("n", [1, 7, 9, 63, 65, 71, 127, 130, 191, 194, 257, 260, 391])
 def test_ragged_output_rows_are_written_whole_and_alone(cuda, n, off):
