@@ -44,7 +44,7 @@ int mx_debug_gemm_keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, i
 /* How many K slices the tensor-core path cuts a product with `tiles` output tiles and reduction length `k` into
  * (1 = no split) on `sms` SMs; block_k = 64 for bf16 / f16, 32 for f32. */
 int mx_debug_splitk_slices(size_t tiles, size_t k, int block_k, int sms);
-/* f32 tensor-core products whose reduction is cut into the CTAs of a cluster: 1 = where that pays and a second launch does not (default), 0 =
+/* f32 tensor-core products whose reduction is cut into the CTAs of a cluster: 1 = where that is the cheapest form (default), 0 =
  * nowhere, 2 = wherever one fits. */
 void mx_debug_set_gemm_f32_cluster(int on);
 /* 1 (default): long f32 reductions multiply the large part of A by both parts of B in one instruction; 0: never. */

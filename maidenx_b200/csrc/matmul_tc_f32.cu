@@ -611,9 +611,8 @@ constexpr double kSplitFixed32 = 3.0;
 // against 64 bits 9.2e-7 (1.0e-6 by three).
 constexpr int kWideLeast = 8;
 std::atomic<int> g_wide{1};  // 0: never (tests, A/B timing)
-// and the sum inside a cluster.  Where both forms split, the one with a second launch is the faster since that closes up with the first (128 x 300 x 784
-// 10.9 us, 12.2 in a cluster; 512 x 1024 x 1024 15.5, 15.9); a cluster takes what it leaves whole: 300 x 784 x 8192 70 us whole, 50 in
-// clusters; ragged 1001 x 1003 x 1005 33, 31.
+// and the sum inside a cluster: more, since the second launch closes up with the first (128 x 300 x 784 10.9 us, 12.2 in a cluster; 512 x 1024 x 1024
+// 15.5, 15.9).  A cluster takes products that the other form cuts into few slices or none: 300 x 784 x 8192 68 us, 50 in clusters of seven.
 constexpr double kClusterFixed32 = 4.0;
 std::atomic<int> g_cluster{1};  // 0: no clusters of slices, 2: wherever they fit (tests, A/B timing)
 
@@ -651,7 +650,9 @@ bool launch(const TcProduct& c, void* D, const char* where) {
         if (slices == 1) slices = splitk_short(tiles, (uint64_t)p.num_kb, grid, kb, whole - kSplitFixed32);
         const int form = g_cluster.load(std::memory_order_relaxed);
         double cost = form == 2 ? 1e30 : whole;
-        if (form == 2 || (form && slices == 1))
+        if (form != 2 && slices > 1)
+            cost = std::min(cost, (double)((tiles * slices + grid - 1) / grid * ((p.num_kb + slices - 1) / slices)) * kb + kSplitFixed32 + 0.1 * slices);
+        if (form)
             p.cluster = cluster_slices(tiles, (uint64_t)p.num_kb, grid, kb, kClusterFixed32, cost,
                                        [](int n) { return resident_clusters(reinterpret_cast<const void*>(tc_gemm_f32_kernel<0, true>), THREADS, SMEM_BYTES, n); });
         if (p.cluster) slices = p.cluster;
@@ -751,6 +752,6 @@ bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t 
 
 }  // namespace mx
 
-// 1 (default): f32 products that are not split in two launches are split into the CTAs of a cluster where that pays; 0: never; 2: wherever they fit
+// 1 (default): the slices of an f32 product are the CTAs of a cluster where that is the cheapest form; 0: never; 2: wherever they fit
 extern "C" void mx_debug_set_gemm_f32_cluster(int on) { mx::g_cluster.store(on ? 1 : 0, std::memory_order_relaxed); }
 extern "C" void mx_debug_set_gemm_f32_wide(int on) { mx::g_wide.store(on ? 1 : 0, std::memory_order_relaxed); }
