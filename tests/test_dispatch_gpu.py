@@ -68,3 +68,25 @@ def test_threads_share_the_slots(cuda):
     [t.start() for t in ts]
     [t.join() for t in ts]
     assert not bad
+
+
+@pytest.mark.parametrize("n", [1, 1000, 300000, 3000001])
+def test_each_launch_of_a_chain_sees_the_one_before(cuda, n):
+    """Kernels are scheduled when the one before them ends: a chain in which every launch reads what the last one wrote, of sums (whose last block folds the others'
+    parts), passes over vectors and small ones after large ones.  Whole numbers below 2^24: exact."""
+    from maidenx_b200 import device
+    x = np.arange(n, dtype=np.float32) % 5
+    a, b, s = device.CudaBuffer.from_host(x), device.CudaBuffer(4 * n), device.CudaBuffer.from_host(np.zeros(1, np.float32))
+    total = 0.0
+    try:
+        for _ in range(20):
+            device.dispatch("neg", "f32", [n, 1, 0], n, 1, "META", a.ptr, b.ptr)
+            device.dispatch("sub", "f32", [n, 1, 1, 0, 0], n, 1, "META", a.ptr, b.ptr, a.ptr)          # a = 2 a
+            device.dispatch("neg", "f32", [n, 1, 0], n, 1, "META", b.ptr, b.ptr)                        # b = the a before
+            device.dispatch("sub", "f32", [n, 1, 1, 0, 0], n, 1, "META", a.ptr, b.ptr, a.ptr)          # a as it was
+            device.dispatch("sum_to_shape", "f32", [n, 1, 1, 0], n, 1, "META", a.ptr, s.ptr)
+        total = float(s.to_host(np.float32, 1)[0])
+        assert total == x.sum(dtype=np.float64) and np.array_equal(a.to_host(np.float32, n), x)
+    finally:
+        for buf in (a, b, s):
+            buf.free()
