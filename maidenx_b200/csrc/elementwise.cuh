@@ -989,7 +989,7 @@ __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, co
 }
 
 // Two inputs of ragged rows, each the output's own layout or the same row for all of them (a bias, a norm's weights): one division by multiplication a
-// vector, the repeated row from L1 by elements, four vectors a thread.  A norm of [8191, 1023] f32, two such passes in nine: 62.4 us, 64.5 with the dense kernel.  An instantiation of the kernel above for it would have the constants'
+// vector, the repeated row from L1 by elements, four vectors a thread.  [8191, 1023] f32 10.3 us (11.8 by the dense kernel), [4099, 1543] bf16 7.0 (8.1).  An instantiation of the kernel above for it would have the constants'
 // registers too (94 instead of 79 in 16 bits).
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_repeat_kernel(F f, const T* a, const T* b, O* out, EwRepeatParams P) {
