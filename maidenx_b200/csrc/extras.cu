@@ -714,7 +714,7 @@ __device__ __forceinline__ A softmax_group_all(A v, A* part) {
 }
 
 template <class T, int G, int K>
-__global__ void __launch_bounds__(kExThreads, (K * 16 / (int)sizeof(T) <= 32) ? 5 : 1) softmax_rows_kernel(const T* __restrict__ in, T* __restrict__ out, u64 rows, u32 n) {
+__global__ void __launch_bounds__(kExThreads, (K * 16 / (int)sizeof(T) <= 32) ? 5 : 1) softmax_rows_kernel(const T* in, T* out, u64 rows, u32 n) {
     after_previous_kernel();
     typedef typename std::conditional<std::is_same<T, f64>::value, f64, f32>::type A;
     constexpr int VEC = 16 / (int)sizeof(T);

@@ -90,3 +90,43 @@ def test_each_launch_of_a_chain_sees_the_one_before(cuda, n):
     finally:
         for buf in (a, b, s):
             buf.free()
+
+
+READERS = {  # name: elements read, elements written, words and arguments of the call (x: what it reads, out: what it writes)
+    "softmax_rows": (2048 * 1024, 2048 * 1024, lambda x, out: ("softmax", [2048, 1024, 1024, 1, 0], 2048 * 1024, 2, 1, "META", x, out)),
+    "softmax_rows_of_a_block": (256 * 8192, 256 * 8192, lambda x, out: ("softmax", [256, 8192, 8192, 1, 0], 256 * 8192, 2, 1, "META", x, out)),
+    "softmax_ragged": (2047 * 197, 2047 * 197, lambda x, out: ("softmax", [2047, 197, 197, 1, 0], 2047 * 197, 2, 1, "META", x, out)),
+    "softmax_columns": (512 * 1024, 512 * 1024, lambda x, out: ("softmax", [512, 1024, 1024, 1, 0], 512 * 1024, 2, 0, "META", x, out)),
+    "product": (1024 * 512, 1024 * 1024, lambda x, out: ("matmul", [2, 2, 2, 1024, 1024, 1024, 512, 512, 1024, 512, 1, 1, 512, 0, 0], 1024 * 1024, "META", x, x, out)),
+    "im2col": (16 * 32 * 28 * 28, 16 * 32 * 9 * 28 * 28, lambda x, out: ("conv2d_im2col", [16, 32, 28, 28, 3, 3, 28, 28, 1, 1, 1, 1], 16 * 32 * 9 * 28 * 28, "META", x, out)),
+    "col2im": (16 * 32 * 9 * 28 * 28, 16 * 32 * 28 * 28, lambda x, out: ("conv2d_col2im", [16, 32, 28, 28, 3, 3, 28, 28, 1, 1, 1, 1], 16 * 32 * 9 * 28 * 28, "META", x, out)),
+}
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("name", READERS)
+def test_readers_see_what_the_launch_before_them_wrote(cuda, name, dt):
+    """An op that reads, right behind it, the whole buffer that a pass over vectors has just written, twenty times with other values each time: bit for bit what it
+    gives with the device idle in between.  A load ahead of the kernel's wait would find the values of the time before."""
+    from maidenx_b200 import _lib, device, dtypes as D
+    lib = _lib.load()
+    t = D.BY_NAME[dt]
+    n_in, n_out, call = READERS[name]
+    rng = np.random.default_rng(n_in)
+    bufs = [device.CudaBuffer.from_host(D.encode(rng.standard_normal(n_in).astype(np.float32), t)) for _ in range(3)]
+    x = device.CudaBuffer.from_host(np.zeros(n_in, t.np_storage))
+    outs = [[device.CudaBuffer.from_host(np.zeros(n_out, t.np_storage)) for _ in range(3)] for _ in range(2)]
+    try:
+        for idle in (True, False):
+            for i in range(20):
+                device.dispatch("neg", dt, [n_in, 1, 0], n_in, 1, "META", bufs[i % 3].ptr, x.ptr)
+                if idle:
+                    assert lib.mx_device_synchronize() == 0
+                op, *args = call(x.ptr, outs[idle][i % 3].ptr)
+                device.dispatch(op, dt, *args)
+        for i in range(3):
+            a, b = (outs[k][i].to_host(t.np_storage, n_out) for k in range(2))
+            assert a.any() and np.array_equal(a, b)
+    finally:
+        for b in [x, *bufs, *outs[0], *outs[1]]:
+            b.free()
