@@ -49,6 +49,9 @@ int mx_debug_splitk_slices(size_t tiles, size_t k, int block_k, int sms);
 void mx_debug_set_gemm_f32_cluster(int on);
 /* 1 (default): long f32 reductions multiply the large part of A by both parts of B in one instruction; 0: never. */
 void mx_debug_set_gemm_f32_wide(int on);
+/* What the calling thread's last f32 product on the tensor cores was: form[0] K slices, form[1] CTAs of a cluster of slices (0: none), form[2]
+ * 1 = both parts of B in one instruction, form[3] columns of a tile. */
+void mx_debug_gemm_f32_last_form(int form[4]);
 /* Writes `value` (0 clears) into the calling thread's tensor-core error word the way a kernel of an earlier launch
  * whose bounded wait ran out would have left it.  Returns 0, or -1 without a usable device. */
 int mx_debug_tc_gemm_poke_status(int value);

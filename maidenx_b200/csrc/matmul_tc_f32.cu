@@ -615,6 +615,7 @@ std::atomic<int> g_wide{1};  // 0: never (tests, A/B timing)
 // 15.5, 15.9).  A cluster takes products that the other form cuts into few slices or none: 300 x 784 x 8192 68 us, 50 in clusters of seven.
 constexpr double kClusterFixed32 = 4.0;
 std::atomic<int> g_cluster{1};  // 0: no clusters of slices, 2: wherever they fit (tests, A/B timing)
+thread_local int t_last_form[4] = {0, 0, 0, 0};  // of the thread's last launch: slices, CTAs of a cluster (0: none), wide, columns of a tile (tests)
 
 // D[M,N] = sum_k Aop[m,k] * Bop[n,k]; K-major operand = row-major [MN, K], MN-major = row-major [K, MN].
 bool launch(const TcProduct& c, void* D, const char* where) {
@@ -703,6 +704,10 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.out_ld = (int64_t)(slices > 1 && !p.cluster ? n_pitch : N);
     if (grid > p.num_tiles) grid = p.num_tiles;
     p.wide = p.chunk_kb == CHUNK_FAST && slices == 1 && p.num_kb >= kWideLeast && g_wide.load(std::memory_order_relaxed) ? 1 : 0;
+    t_last_form[0] = slices;
+    t_last_form[1] = p.cluster;
+    t_last_form[2] = p.wide;
+    t_last_form[3] = p.bn;
     const bool fixed = p.bn == BN && !p.d_plain && p.chunk_kb == CHUNK_FAST;
     const auto kernel = p.cluster ? (fixed ? tc_gemm_f32_kernel<BN, true> : tc_gemm_f32_kernel<0, true>) : (fixed ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>);
     launch_clusters(kernel, p.cluster ? p.num_tiles : grid, THREADS, SMEM_BYTES, p.cluster, ma, mb, md, p, err, tag);
@@ -753,5 +758,8 @@ bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t 
 }  // namespace mx
 
 // 1 (default): the slices of an f32 product are the CTAs of a cluster where that is the cheapest form; 0: never; 2: wherever they fit
-extern "C" void mx_debug_set_gemm_f32_cluster(int on) { mx::g_cluster.store(on ? 1 : 0, std::memory_order_relaxed); }
+extern "C" void mx_debug_set_gemm_f32_cluster(int on) { mx::g_cluster.store(on < 0 ? 0 : on > 2 ? 2 : on, std::memory_order_relaxed); }
 extern "C" void mx_debug_set_gemm_f32_wide(int on) { mx::g_wide.store(on ? 1 : 0, std::memory_order_relaxed); }
+extern "C" void mx_debug_gemm_f32_last_form(int* form) {
+    for (int i = 0; i < 4; i++) form[i] = mx::t_last_form[i];
+}

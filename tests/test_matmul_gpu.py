@@ -11,6 +11,8 @@ index reaches num_els * k are skipped (crates/maidenx_cpu/src/ops/matmul.rs:55-1
 """
 import zlib
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -433,14 +435,21 @@ def test_products_with_ragged_rows(oracle, cuda, dt, case):
     H.assert_same("matmul", dt, got, ref, float_rel=1e-5 if dt.name == "f32" else 1e-2, what=name, scale=np.sqrt(k))
 
 
+def _last_f32_form(lib):
+    """Slices, CTAs of a cluster, both parts of B in one instruction, columns of a tile: of the thread's last f32 product on the tensor cores."""
+    form = (ctypes.c_int * 4)()
+    lib.mx_debug_gemm_f32_last_form(form)
+    return tuple(form)
+
+
 @pytest.mark.parametrize("dt", [D.F32], ids=lambda d: d.name)
 @pytest.mark.parametrize("case", [
     # M, N, K, majors: two to eight slices, the last one short; ragged rows and edges of tiles; one row and one column of tiles; reductions that are emptied in runs
     (128, 300, 784, "kk"), (128, 784, 300, "km"), (300, 784, 1024, "mm"), (130, 131, 9001, "kk"), (257, 64, 2049, "mk"), (100, 1000, 4100, "km"), (1, 4099, 4099, "km"),
-    (512, 72, 8200, "mm"), (1543, 200, 2000, "mm")], ids=lambda c: "x".join(map(str, c)))
+    (512, 72, 8200, "mm"), (1543, 200, 2000, "mm"), (300, 784, 8192, "kk")], ids=lambda c: "x".join(map(str, c)))
 def test_slices_summed_in_a_cluster(cuda, dt, case):
-    """A split product whose slices are the CTAs of a cluster, next to float64 and to the form with a second launch; an infinity reaches its own row and
-    nothing else, and nothing is written around the output."""
+    """A split product whose slices are the CTAs of a cluster, next to float64 and to the form with a second launch (the same bits where both cut alike); an
+    infinity reaches its own row and nothing else, and nothing is written around the output.  300 x 784 x 8192 takes the form by itself."""
     from maidenx_b200 import _lib, device
     lib = _lib.load()
     m, n, k, majors = case
@@ -453,12 +462,13 @@ def test_slices_summed_in_a_cluster(cuda, dt, case):
     meta = [2, 2, 2, m, n, m, k, k, n, *([k, 1] if majors[0] == "k" else [1, m]), *([1, k] if majors[1] == "k" else [n, 1]), 0, 0]
     guard = 16
     fill = np.full(m * n + 2 * guard, 3, dtype=dt.np_storage)
-    got = {}
+    got, form = {}, {}
     try:
-        for on in (0, 2):
+        for on in (0, 1, 2):
             lib.mx_debug_set_gemm_f32_cluster(on)
             bufs = [device.CudaBuffer.from_host(np.ascontiguousarray(x).reshape(-1)) for x in (am, bm, fill)]
             device.dispatch("matmul", dt.name, meta, m * n, "META", bufs[0].ptr, bufs[1].ptr, bufs[2].ptr + guard * dt.size)
+            form[on] = _last_f32_form(lib)
             raw = bufs[2].to_host(dt.np_storage, fill.size)
             assert (raw[:guard] == 3).all() and (raw[-guard:] == 3).all()
             got[on] = D.decode(raw[guard:-guard], dt).astype(np.float64).reshape(m, n)
@@ -466,17 +476,22 @@ def test_slices_summed_in_a_cluster(cuda, dt, case):
                 x.free()
     finally:
         lib.mx_debug_set_gemm_f32_cluster(1)
+    assert form[0][1] == 0 and 2 <= form[2][1] <= 8 and form[2][0] == form[2][1], form
+    assert case[:3] != (300, 784, 8192) or form[1][1] > 0, form
     ref = np.matmul(D.decode(a.reshape(-1), dt).astype(np.float64).reshape(m, k)[:m - inf], D.decode(b.reshape(-1), dt).astype(np.float64).reshape(k, n))
     for out in got.values():
         if inf:
             assert np.isinf(out[m - 1]).all()
         err = np.linalg.norm(out[:m - inf] - ref) / np.linalg.norm(ref)
         assert err <= 2e-6, err  # the split product's
+    for on in (1, 2):
+        if form[on][0] == form[0][0] and form[on][3] == form[0][3]:
+            assert np.array_equal(got[on], got[0])
 
 
 @pytest.mark.parametrize("case", [
     # M, N, K, majors: the shortest reduction of the form, one chunk more and less than whole, a last k-block that is not full; tiles of 64 and 128 columns with edges; no split
-    (2048, 1600, 256, "kk"), (1800, 1540, 260, "km"), (2048, 1600, 392, "mm"), (5000, 64, 512, "mk"), (2432, 1664, 1000, "km"), (130, 19000, 288, "kk")],
+    (2048, 1600, 256, "kk"), (1800, 1540, 260, "km"), (2048, 1600, 392, "mm"), (12000, 64, 512, "mk"), (9700, 52, 392, "km"), (2432, 1664, 1000, "km"), (130, 19000, 288, "kk")],
     ids=lambda c: "x".join(map(str, c)))
 def test_f32_products_with_both_parts_of_b_in_one_instruction(cuda, case):
     """Next to float64: within the split product's bound, and no further off than the form of three instructions by more than rounding."""
@@ -494,6 +509,7 @@ def test_f32_products_with_both_parts_of_b_in_one_instruction(cuda, case):
             lib.mx_debug_set_gemm_f32_wide(on)
             bufs = [device.CudaBuffer.from_host(np.ascontiguousarray(x).reshape(-1)) for x in (am, bm, np.zeros(m * n, np.float32))]
             device.dispatch("matmul", "f32", meta, m * n, "META", bufs[0].ptr, bufs[1].ptr, bufs[2].ptr)
+            assert _last_f32_form(lib)[:3] == (1, 0, on) and (n > 64 or _last_f32_form(lib)[3] == 64)
             out = bufs[2].to_host(np.float32, m * n).reshape(m, n)
             err.append(np.linalg.norm(out - ref) / np.linalg.norm(ref))
             for x in bufs:
