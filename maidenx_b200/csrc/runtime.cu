@@ -61,11 +61,27 @@ int g_slot_free[kDispatchSlots], g_slots_free = 0;  // under g_slot_mutex
 bool g_slot_open[kDispatchSlots];                   // under g_slot_mutex
 size_t g_slot_words[kDispatchSlots];                // of an open slot: written before its address is handed out, read by its owner
 
-int dispatch_slot_of(const void* p) {  // -1: not a slot
+int dispatch_slot_around(const void* p, size_t* offset) {  // the slot that holds the byte at `p`; -1: none does
     const char* base = g_slot_base.load(std::memory_order_acquire);
     if (!base || (uintptr_t)p < (uintptr_t)base) return -1;
     const uintptr_t off = (uintptr_t)p - (uintptr_t)base;
-    return off < kDispatchSlots * kSideTableMaxBytes && off % kSideTableMaxBytes == 0 ? (int)(off / kSideTableMaxBytes) : -1;
+    *offset = off % kSideTableMaxBytes;
+    return off < kDispatchSlots * kSideTableMaxBytes ? (int)(off / kSideTableMaxBytes) : -1;
+}
+int dispatch_slot_of(const void* p) {  // -1: not the start of a slot
+    size_t offset = 0;
+    const int slot = dispatch_slot_around(p, &offset);
+    return offset == 0 ? slot : -1;
+}
+
+// A copy to `dst` by the host, complete when it returns: the launcher reads a slot without waiting for the stream.  The block has at least the words that
+// were ever written to it.  cudaErrorInvalidValue when it runs out of the slot.
+template <class Copy>
+cudaError_t dispatch_slot_write(int slot, size_t offset, size_t size, Copy copy) {
+    if (size > kSideTableMaxBytes - offset) return cudaErrorInvalidValue;
+    const cudaError_t e = copy();
+    if (e == cudaSuccess && g_slot_words[slot] < (offset + size) / sizeof(size_t)) g_slot_words[slot] = (offset + size) / sizeof(size_t);
+    return e;
 }
 
 void* dispatch_slot_take(const size_t* words, size_t count) {
@@ -565,10 +581,12 @@ bool staged_upload(void* dst, const void* src, size_t size, cudaError_t* result)
 
 int cuda_memcpy_h2d(void* dst, const void* src, size_t size) {
     cudaError_t e;
-    if (size <= kSideTableMaxBytes && dispatch_slot_of(dst) >= 0) {  // a block of mx_dispatch_begin, written anew
-        std::memcpy(dst, src, size);
-        return (int)cudaSuccess;
-    }
+    size_t offset = 0;
+    if (const int slot = dispatch_slot_around(dst, &offset); slot >= 0)  // a block of mx_dispatch_begin, or words of it, written anew
+        return (int)dispatch_slot_write(slot, offset, size, [&] {
+            std::memcpy(dst, src, size);
+            return cudaSuccess;
+        });
     if (!(size > 0 && size <= kStageSlotBytes && g_stage_enabled.load(std::memory_order_relaxed) && staged_upload(dst, src, size, &e)))
         e = cudaMemcpy(dst, src, size, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && size > 0 && size <= kSideTableMaxBytes && size % sizeof(size_t) == 0) {
@@ -605,8 +623,12 @@ int cuda_memcpy_d2h(void* dst, const void* src, size_t size) {
 
 int cuda_memcpy_d2d(void* dst, const void* src, size_t size) {
     drain_thread_stream();
+    size_t offset = 0;
+    if (const int slot = dispatch_slot_around(dst, &offset); slot >= 0)
+        return (int)dispatch_slot_write(slot, offset, size, [&] { return cudaMemcpy(dst, src, size, cudaMemcpyDeviceToHost); });
     side_table_forget(dst, size);
-    return (int)cudaMemcpy(dst, src, size, cudaMemcpyDeviceToDevice);
+    // from a block of mx_dispatch_begin: complete when it returns, since the block may be given back and used again at once
+    return (int)cudaMemcpy(dst, src, size, dispatch_slot_around(src, &offset) >= 0 ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice);
 }
 
 // The calls around an op in the dispatch pattern, folded into two (fewer crossings for callers behind a foreign-function layer).

@@ -51,6 +51,55 @@ def test_blocks_open_at_once_read_back_and_given_back(cuda):
         dst.free()
 
 
+def test_words_of_a_block_written_anew(cuda):
+    """A block may be written in part, and past the words it was given, from the host or the device, with work queued on the stream: the next op reads what was
+    written, and a block that is handed out again holds nothing of it."""
+    from maidenx_b200 import _lib, device
+    lib = _lib.load()
+    neg, x = _lib.op("neg", "f32"), np.arange(1, 1 << 25, dtype=np.float32)
+    src, dst, busy = device.CudaBuffer.from_host(x), device.CudaBuffer(4 * 16), device.CudaBuffer(4 * x.size)
+    try:
+        def words(*v):
+            return np.array(v, dtype=np.uint64)
+
+        for i in range(100):
+            block = _begin(lib, [4, 1, 0])
+            for _ in range(3):  # the device is busy when the words arrive
+                neg(x.size, 1, None, src.ptr, busy.ptr)
+            offset = words(3 * i)
+            if i % 2:
+                on_device = device.CudaBuffer.from_host(offset)
+                assert lib.cuda_memcpy_d2d(block.value + 16, on_device.ptr, 8) == 0
+                on_device.free()
+            else:
+                assert lib.cuda_memcpy_h2d(block.value + 16, offset.ctypes.data, 8) == 0
+            neg(4, 1, block, src.ptr, dst.ptr)
+            assert lib.mx_dispatch_end(block) == 0
+            assert np.array_equal(dst.to_host(np.float32, 4), -x[3 * i:3 * i + 4]), i
+        table = lib.mx_metadata_table_size()
+        block = _begin(lib, [4])                                          # fewer words than the op reads, completed afterwards
+        rest = words(1, 7)
+        assert lib.cuda_memcpy_h2d(block.value + 8, rest.ctypes.data, 16) == 0
+        neg(4, 1, block, src.ptr, dst.ptr)
+        assert lib.mx_last_error() == 0 and np.array_equal(dst.to_host(np.float32, 4), -x[7:11])
+        copy = device.CudaBuffer(24)
+        assert lib.cuda_memcpy_d2d(copy.ptr, block, 24) == 0 and lib.mx_dispatch_end(block) == 0
+        block = _begin(lib, [9, 9, 9])
+        assert list(copy.to_host(np.uint64, 3)) == [4, 1, 7] and lib.mx_dispatch_end(block) == 0
+        copy.free()
+        assert lib.mx_metadata_table_size() == table                      # nothing is remembered for addresses inside a slot
+        block = _begin(lib, [9])
+        neg(4, 1, block, src.ptr, dst.ptr)                                # the words of its last use do not count
+        assert lib.mx_dispatch_end(block) == 2
+        block, long = _begin(lib, [4, 1, 0]), np.zeros(300, np.uint64)
+        assert lib.cuda_memcpy_h2d(block.value, long.ctypes.data, 2400) != 0  # past the end of the slot: refused, nothing written
+    finally:
+        lib.mx_clear_error()
+        for b in (src, dst, busy):
+            b.free()
+    assert lib.mx_dispatch_end(block) == 0
+
+
 def test_threads_share_the_slots(cuda):
     from maidenx_b200 import device
     bad = []
