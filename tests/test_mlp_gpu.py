@@ -285,3 +285,42 @@ def test_loss_reader_returns_every_steps_loss_one_step_later(cuda):
     b.close()
     xb.free()
     yb.free()
+
+
+@pytest.mark.parametrize("dim", [1440, 1456, 2048])
+def test_updates_beside_the_backward_pass_give_the_same_bits(cuda, dim):
+    """mx_mlp_train_step against a twin engine stepped through the separate entry points on one stream, eight steps with other inputs each: layers whose update runs
+    on the main stream (1440) and on the side stream, whose writes the next forward pass has to wait for."""
+    from maidenx_b200.mlp import Mlp
+    L, B, seed, lr = 3, 200, 9, 0.05
+    rng = np.random.default_rng(dim)
+    xs = [device.CudaBuffer.from_host(H.random_store(rng, D.BF16, B * dim, dist="normal")) for _ in range(6)]
+    a, b = Mlp(L, dim, B, "bf16", seed), Mlp(L, dim, B, "bf16", seed)
+    loss = []
+    for i in range(8):
+        x, y = xs[i % 3].ptr, xs[3 + i % 2].ptr
+        a.train_step(x, y, lr)
+    a.join()
+    for i in range(8):
+        x, y = xs[i % 3].ptr, xs[3 + i % 2].ptr
+        b.forward(x)
+        b.loss_backward(y)
+        for l in reversed(range(L)):
+            b.backward_layer(l)
+            device.synchronize()
+            b.sgd_layer(l, lr)
+        loss.append(b.loss())
+    assert a.loss() == loss[-1] != loss[0]
+    for l in range(L):
+        for what, count, dt in (("master_weight", dim * dim, np.float32), ("master_bias", 1, np.float32), ("weight_grad", dim * dim, np.uint16), ("bias_grad", 1, np.uint16)):
+            got = []
+            for m in (a, b):
+                host = np.empty(count, dt)
+                assert m.lib.cuda_memcpy_d2h(host.ctypes.data, m.ptr(what, l), host.nbytes) == 0
+                got.append(host)
+            assert np.array_equal(*got), (what, l)
+    assert device.last_error() is None
+    a.close()
+    b.close()
+    for v in xs:
+        v.free()
