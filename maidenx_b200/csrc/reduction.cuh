@@ -300,9 +300,8 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_warp_kernel(const T* 
 }
 
 // Rows that are no whole aligned vectors, by the aligned 16-byte words they lie in: a lane loads a word (which holds at least one element of its row, so
-// that nothing outside the tensor's own words is touched) and leaves out the neighbours' elements.  Element by element a row of 197 bf16 took
-// seven loads of two bytes a lane, where one of 16 does (192 x 197 of them 6.8 us, now 5.9).  G lanes per row with Q rows in flight where a row has up to G words, else a warp with four words
-// of it in flight.
+// that nothing outside the tensor's own words is touched) and leaves out the neighbours' elements.  Element by element a row of 197 bf16 takes
+// seven loads of two bytes a lane, where one of 16 does (40000 rows of 193 5.5 us, 5.0 so).  G lanes per row with Q rows in flight; which: red_rows_words_launch.
 template <class T, int KIND>
 struct RowWords {
     typedef RedTraits<T, KIND> TR;
@@ -353,27 +352,6 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_words_kernel(const T*
 #pragma unroll
     for (int q = 0; q < Q; q++)
         if (lane == 0 && row0 + q * ROWS < rows) out[row0 + q * ROWS] = TR::finalize(acc[q], factor);
-}
-template <class T, int KIND>
-__global__ void __launch_bounds__(kRedThreads) reduce_rows_long_words_kernel(const T* in, T* out, u64 rows, u32 R, u64 factor) {
-    after_previous_kernel();
-    typedef RedTraits<T, KIND> TR;
-    typedef RowWords<T, KIND> RW;
-    const u64 row = (u64)blockIdx.x * (kRedThreads / 32) + threadIdx.x / 32;
-    if (row >= rows) return;
-    const RW w(in + row * R, R);
-    typename TR::Acc acc = TR::init();
-    for (u32 i = threadIdx.x % 32; i < w.words; i += 4 * 32) {
-        Vec<T, RW::VEC> v[4];
-#pragma unroll
-        for (u32 q = 0; q < 4; q++)
-            if (i + q * 32 < w.words) v[q] = w.first[i + q * 32];
-#pragma unroll
-        for (u32 q = 0; q < 4; q++)
-            if (i + q * 32 < w.words) acc = w.add(acc, v[q], i + q * 32, R);
-    }
-    acc = warp_reduce<TR>(acc);
-    if (threadIdx.x % 32 == 0) out[row] = TR::finalize(acc, factor);
 }
 
 // One thread per row (R < 32, see red_launch).
@@ -675,17 +653,42 @@ void red_rows_group_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaSt
     else launch_kernel(reduce_rows_warp_kernel<T, KIND, VEC>, (u32)((O + kRedThreads / 32 - 1) / (kRedThreads / 32)), kRedThreads, 0, s, in, out, O, (u32)R, factor);
 }
 
-// Rows of at least 128 bytes that are no whole aligned vectors (see RowWords).
+// Rows of at least 128 bytes that are no whole aligned vectors (see RowWords); false: they are summed element by element.  Leaving out the neighbours costs
+// two instructions an element, for one load instead of up to 16, so it pays while a lane has one word.  Elements / words, us (sums; maxima alike):
+//   up to 16 words   bf16 65: 600 rows 1.20 / 1.19, 19200 2.63 / 1.90, 300000 22.3 / 14.6; u8 225: 600 1.54 / 1.31, 300000 36.5 / 22.6; f32 57: 9600 1.70 / 1.37
+//     four rows a group, f32 57: 600 1.73, 9600 1.83 instead of 1.37, 40000 2.62 instead of 2.71, 300000 10.5 instead of 12.6; 16-bit and bytes no gain at 300000
+//   up to 32         bf16 193: 600 1.43 / 1.21, 40000 5.50 / 5.02, 300000 42.0 / 35.4 (four rows a group 5.19, 31.1); f32 97: 9600 1.72 / 1.81, 30000 3.28 / 3.44, four
+//                    rows a group 40000 3.99 / 3.83, 300000 31.7 / 26.9; u8 385: 9600 2.40 / 2.52, 40000 6.24 / 7.06, 100000 13.1 / 15.7
+//   a warp a row with its words in steps of four a lane was slower than elements over most of what is longer (bf16 263: 40000 5.7 / 9.0; u8 527: 15.1 / 45.7; f32
+//   1023: 9600 3.9 / 4.3) and is gone.
 template <class T, int KIND>
-void red_rows_words_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaStream_t s) {
+bool red_rows_words_launch(const T* in, T* out, u64 O, u64 R, u64 factor, cudaStream_t s) {
     constexpr u64 VEC = 16 / sizeof(T);
     const u64 words = (R + 2 * VEC - 2) / VEC;  // at most, wherever a row starts
-    auto blocks = [&](u64 rows) { return (u32)((O + rows - 1) / rows); };
-    const bool many = O >= 4 * 8 * 8 * (u64)sm_count();
-    if (words <= 16) launch_kernel(reduce_rows_words_kernel<T, KIND, 16, 4>, blocks(4 * kRedThreads / 16), kRedThreads, 0, s, in, out, O, (u32)R, factor);
-    else if (words <= 32 && many) launch_kernel(reduce_rows_words_kernel<T, KIND, 32, 4>, blocks(4 * kRedThreads / 32), kRedThreads, 0, s, in, out, O, (u32)R, factor);
-    else if (words <= 32) launch_kernel(reduce_rows_words_kernel<T, KIND, 32, 1>, blocks(kRedThreads / 32), kRedThreads, 0, s, in, out, O, (u32)R, factor);
-    else launch_kernel(reduce_rows_long_words_kernel<T, KIND>, blocks(kRedThreads / 32), kRedThreads, 0, s, in, out, O, (u32)R, factor);
+    auto launch = [&](auto kernel, u64 rows) { launch_kernel(kernel, (u32)((O + rows - 1) / rows), kRedThreads, 0, s, in, out, O, (u32)R, factor); };
+    const u64 sms = (u64)sm_count();
+    if constexpr (sizeof(T) == 4) {
+        const bool many = O >= 256 * sms;
+        if (words <= 16 && many) launch(reduce_rows_words_kernel<T, KIND, 16, 4>, 4 * kRedThreads / 16);
+        else if (words <= 16) launch(reduce_rows_words_kernel<T, KIND, 16, 1>, kRedThreads / 16);
+        else if (words <= 32 && many) launch(reduce_rows_words_kernel<T, KIND, 32, 4>, 4 * kRedThreads / 32);
+        else return false;
+        return true;
+    }
+    if constexpr (sizeof(T) < 4) {
+        if (words <= 16) {
+            launch(reduce_rows_words_kernel<T, KIND, 16, 1>, kRedThreads / 16);
+            return true;
+        }
+    }
+    if constexpr (sizeof(T) == 2) {
+        if (words <= 32) {
+            if (O >= 1024 * sms) launch(reduce_rows_words_kernel<T, KIND, 32, 4>, 4 * kRedThreads / 32);
+            else launch(reduce_rows_words_kernel<T, KIND, 32, 1>, kRedThreads / 32);
+            return true;
+        }
+    }
+    return false;
 }
 
 template <class T, int KIND>
@@ -714,8 +717,8 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
             launch_kernel(reduce_rows_thread_kernel<T, KIND>, (u32)blocks, kRedThreads, 0, s, in, out, O, R, pl.factor);
         } else if (R < 32 || (R < 2048 && O >= (u64)sms * 4)) {
             if (vec_rows) red_rows_group_launch<T, KIND, VEC>(in, out, O, R, pl.factor, s);
-            else if (sizeof(T) < 8 && R * sizeof(T) >= 128 && (uintptr_t)in % sizeof(T) == 0) red_rows_words_launch<T, KIND>(in, out, O, R, pl.factor, s);
-            else red_rows_group_launch<T, KIND, 1>(in, out, O, R, pl.factor, s);
+            else if (!(R * sizeof(T) >= 128 && (uintptr_t)in % sizeof(T) == 0 && red_rows_words_launch<T, KIND>(in, out, O, R, pl.factor, s)))
+                red_rows_group_launch<T, KIND, 1>(in, out, O, R, pl.factor, s);
         } else {
             // block per (row, split); split long rows when there are too few rows to fill the GPU
             const bool vec = vec_rows;

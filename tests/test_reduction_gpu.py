@@ -215,3 +215,24 @@ def test_ragged_rows_by_the_words_they_lie_in(oracle, cuda, dt):
                     binding.set_wide(False)
                 got = H.run_reduce(cuda, op, dt, [o, r], [r, 1], [r], [1], off, x)
                 H.assert_same(op, dt, got, ref, float_rel=SUM_TOL.get(dt.name, 0.0) if op != "max" else 0.0, what=str((op, r, off)), scale=np.sqrt(r) if op == "sum" else 1.0)
+
+
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.U8, D.I32], ids=lambda d: d.name)
+def test_ragged_rows_on_both_sides_of_the_rules_lines(oracle, cuda, dt):
+    """Rows of up to 16, up to 32 and more words, in counts on both sides of where a group of lanes takes four rows at a time (256 and 1024 rows an SM); a last
+    group that is not full."""
+    from oracle import binding
+    rng = np.random.default_rng(dt.size + 5)
+    vec = 16 // dt.size
+    rows = {4: (37887, 37889), 2: (37889, 151551, 151555), 1: (37889,)}[dt.size]
+    for r in (8 * vec + 1, 14 * vec + 3, 15 * vec + 3, 30 * vec + 1, 31 * vec + 3):
+        for o in rows:
+            x = H.random_store(rng, dt, o * r + 1, dist="normal") if dt.kind == "float" else H.random_store(rng, dt, o * r + 1)
+            for op in ("sum", "max"):
+                binding.set_wide(dt.kind == "float" and op != "max")
+                try:
+                    ref = H.run_reduce(oracle, op, dt, [o, r], [r, 1], [r], [1], 1, x)
+                finally:
+                    binding.set_wide(False)
+                got = H.run_reduce(cuda, op, dt, [o, r], [r, 1], [r], [1], 1, x)
+                H.assert_same(op, dt, got, ref, float_rel=SUM_TOL.get(dt.name, 0.0) if op != "max" else 0.0, what=str((op, r, o)), scale=np.sqrt(r) if op == "sum" else 1.0)
