@@ -41,6 +41,9 @@ int mx_debug_gemm_max_resident_pairs(void);
  * with these tile counts takes (0 = general schedule). */
 void mx_debug_set_gemm_keep_b(int on);
 int mx_debug_gemm_keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, int ctas);
+/* The schedule of the calling thread's last launch of the one-CTA tensor-core kernel: 0 = general, 1 = the B panel of a column tile kept, 2 = the same for a
+ * batch that shares A. */
+int mx_debug_gemm_last_schedule(void);
 /* How many K slices the tensor-core path cuts a product with `tiles` output tiles and reduction length `k` into
  * (1 = no split) on `sms` SMs; block_k = 64 for bf16 / f16, 32 for f32. */
 int mx_debug_splitk_slices(size_t tiles, size_t k, int block_k, int sms);

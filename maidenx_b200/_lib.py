@@ -85,6 +85,7 @@ RUNTIME_SIGNATURES = {
     "mx_debug_set_gemm_f32_wide": ([ctypes.c_int], None),
     "mx_debug_gemm_f32_last_form": ([ctypes.POINTER(ctypes.c_int)], None),
     "mx_debug_gemm_keep_b_ctas": ([ctypes.c_int] * 5, ctypes.c_int),
+    "mx_debug_gemm_last_schedule": ([], ctypes.c_int),
     "mx_debug_splitk_slices": ([ctypes.c_size_t, ctypes.c_size_t, ctypes.c_int, ctypes.c_int], ctypes.c_int),
     "mx_debug_reduce_plan": ([ctypes.c_size_t, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_size_t),
                               ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_size_t)], ctypes.c_int),

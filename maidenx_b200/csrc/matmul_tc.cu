@@ -610,11 +610,14 @@ int keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, int ctas) {
     return tiles_m >= 4 * per_col ? per_col : 0;
 }
 
-// The same for a batch: with four row tiles and more to a panel and enough tiles that the runs' ends do not count (64 x (2304 x 3136 x 256) bf16 364 us
-// in the common order, 318 so at the same clock).
-bool keep_panels(uint64_t tiles_m, uint64_t tiles_n, int num_kb, uint64_t batch, int ctas) {
-    return g_keep_b.load(std::memory_order_relaxed) && batch > 1 && num_kb <= STAGES && tiles_m >= 4 && tiles_m * tiles_n * batch >= 8 * (uint64_t)ctas;
+// The same for a batch whose products share A, with five row tiles and more to a panel and enough tiles that the runs' ends do not count.  General schedule /
+// panels, bf16, us: A shared 64 x (2304 x 3136 x 256) 316 / 266, 64 x (2304 x 784 x 256) 93 / 80, 300 x (520 x 256 x 256) 36 / 33.  Four row tiles gain nothing (160 x (512 x
+// 512 x 256) 32.6 / 33.3), nor does what loads little of B (64 x (1152 x 3136 x 128) 114 / 125, 128 x (1024 x 1024 x 64) 57 / 59), and an A of its own
+// for each product is read again for every panel by CTAs that are batches apart (64 x (2304 x 3136 x 256) 285 / 365, 160 x (512 x 512 x 256) 34.6 / 39.5).
+bool keep_panels(uint64_t tiles_m, uint64_t tiles_n, int num_kb, uint64_t batch, bool a_shared, int ctas) {
+    return g_keep_b.load(std::memory_order_relaxed) && batch > 1 && a_shared && num_kb == STAGES && tiles_m >= 5 && tiles_m * tiles_n * batch >= 8 * (uint64_t)ctas;
 }
+thread_local int t_last_schedule = 0;  // of the thread's last launch of this kernel: 1 = one B panel kept, 2 = panels of a batch, 0 = general (tests)
 
 // The two-CTA kernel: B is staged in halves of 128 columns, a pair of CTAs owns a 256 x 256 tile.  Its split-K slices are
 // sub-matrices behind the third coordinate of the tensor maps.  false: nothing was launched.
@@ -712,7 +715,7 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     // few output tiles: cut K into slices that run as the batches of this launch
     int slices = 1;
     const int bn_whole = p.b_keep ? p.bn : tile_columns((uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid);
-    const bool panels = p.bn == BN && bn_whole == BN && !c.d_plain && keep_panels((uint64_t)p.tiles_m, (uint64_t)p.tiles_n, p.num_kb, batch, grid);
+    const bool panels = p.bn == BN && bn_whole == BN && !c.d_plain && keep_panels((uint64_t)p.tiles_m, (uint64_t)p.tiles_n, p.num_kb, batch, c.a_bs == 0, grid);
     if (batch == 1 && !fuse && !p.b_keep) {
         slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
         if (slices == 1)
@@ -769,6 +772,7 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     p.b_mn = b_mn ? 1 : 0;
     if (grid > p.num_tiles) grid = p.num_tiles;
     if (p.b_keep) grid = p.b_keep * p.tiles_n;
+    t_last_schedule = panels ? 2 : p.b_keep ? 1 : 0;
     const bool full = p.bn == BN;
     const auto kernel = panels ? (fuse ? tc_gemm_kernel<TC_BIAS, BN, false, true> : tc_gemm_kernel<TC_STORE, BN, false, true>)
                         : drain ? (p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0, true> : (fuse ? tc_gemm_kernel<TC_BIAS, 0, true> : tc_gemm_kernel<TC_STORE, 0, true>))
@@ -1338,6 +1342,7 @@ extern "C" void mx_debug_set_gemm_group_m(int rows) { mx::g_group_m.store(rows >
 // 1 (default): products with a reduction of at most 256 run with the B panel resident in shared memory; 0: general schedule
 extern "C" void mx_debug_set_gemm_keep_b(int on) { mx::g_keep_b.store(on ? 1 : 0, std::memory_order_relaxed); }
 extern "C" int mx_debug_gemm_keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, int ctas) { return mx::keep_b_ctas(tiles_m, tiles_n, num_kb, batch, ctas); }
+extern "C" int mx_debug_gemm_last_schedule(void) { return mx::t_last_schedule; }
 extern "C" int mx_debug_splitk_slices(size_t tiles, size_t k, int block_k, int sms) { return mx::tc::splitk_slices(tiles, k, block_k, sms); }
 extern "C" int mx_debug_matmul_forward_path(size_t num_els, const size_t* host_metadata, const void* a, const void* b, const void* out, int* a_mn_major,
                                             int* b_mn_major, size_t* m, size_t* n, size_t* k) {

@@ -356,10 +356,12 @@ def test_short_reductions_with_the_b_panel_resident(oracle, cuda, dt, case):
 
 @pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
 @pytest.mark.parametrize("case", [
-    # batch, M, N, K, majors, whether A is the same for all batches: edges of row and column tiles, one to four k-blocks, runs of tiles that end inside a panel
-    (97, 520, 760, 64, "kk", False), (149, 513, 504, 136, "km", False), (160, 512, 512, 256, "mm", True)], ids=lambda c: "x".join(map(str, c[:4])))
+    # batch, M, N, K, majors, whether A is the same for all batches: edges of row and column tiles, a last k-block that is not full, runs of tiles that end inside a
+    # panel; and what the rule leaves to the general schedule
+    (97, 600, 760, 256, "kk", True), (149, 641, 504, 200, "km", True), (300, 520, 256, 248, "mm", True), (97, 600, 760, 256, "kk", False), (160, 512, 512, 256, "mm", True),
+    (149, 641, 504, 136, "km", True)], ids=lambda c: "x".join(map(str, c)))
 def test_short_reductions_of_a_batch_with_the_b_panel_resident(cuda, dt, case):
-    """Batched products of K <= 256 load a B panel once for all its row tiles: bit for bit the general schedule, and next to float64 in the first, a middle and the
+    """Batched products of K <= 256 that share A load a B panel once for all its row tiles: bit for bit the general schedule, and next to float64 in the first, a middle and the
     last batch (one rounding of an f32 sum: half a step of the type and the sum's own error)."""
     from maidenx_b200 import _lib
     lib = _lib.load()
@@ -370,9 +372,11 @@ def test_short_reductions_of_a_batch_with_the_b_panel_resident(cuda, dt, case):
     sa, sb = [0 if shared else m * k, *([k, 1] if majors[0] == "k" else [1, m])], [k * n, *([1, k] if majors[1] == "k" else [n, 1])]
     meta = H.matmul_metadata([nb, m, n], [nb, m, k], [nb, k, n], sa, sb, 0, 0)
     kept = H.run_matmul(cuda, dt, meta, nb * m * n, a, b)
+    assert lib.mx_debug_gemm_last_schedule() == (2 if shared and k > 192 and m > 512 else 0)
     lib.mx_debug_set_gemm_keep_b(0)
     try:
         general = H.run_matmul(cuda, dt, meta, nb * m * n, a, b)
+        assert lib.mx_debug_gemm_last_schedule() == 0
     finally:
         lib.mx_debug_set_gemm_keep_b(1)
     assert np.array_equal(kept, general)
