@@ -181,17 +181,18 @@ __device__ __forceinline__ Acc load_published(const Acc* p) {
     return *reinterpret_cast<const volatile Acc*>(p);  // not through L1: written by other blocks of this launch
 }
 
-// The fold of `splits` published parts, `stride` apart, in split order, eight of them in flight: one thread folds an output while the
-// rest of the launch is over, so each trip to L2 counts in full.
+// The fold of a row's `splits` published parts in split order, eight of them in flight: one thread folds an output while the
+// rest of the launch is over, so each trip to L2 counts in full.  Not in the kernel of columns, where it takes registers from the main loop (bf16
+// 52, 80 with it; 130 x 300000 8.8 us, 10.1; 100001 x 16 f32 32.0, 37.2; 2047 x 20000 f64 49.7, 54.5; only 2047 x 20000 bf16 10.2, 9.6).
 template <class TR>
-__device__ __forceinline__ typename TR::Acc fold_published(const typename TR::Acc* p, u64 stride, u32 splits) {
+__device__ __forceinline__ typename TR::Acc fold_published(const typename TR::Acc* p, u32 splits) {
     typedef typename TR::Acc Acc;
     Acc acc = TR::init();
     for (u32 s = 0; s < splits; s += 8) {
         Acc v[8];
 #pragma unroll
         for (u32 q = 0; q < 8; q++)
-            if (s + q < splits) v[q] = load_published(p + (s + q) * stride);
+            if (s + q < splits) v[q] = load_published(p + s + q);
 #pragma unroll
         for (u32 q = 0; q < 8; q++)
             if (s + q < splits) acc = TR::combine(acc, v[q]);
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_block_kernel(const T*
         acc = block_reduce<TR, kRedThreads>(acc);
         if (threadIdx.x == 0) out[row] = TR::finalize(acc, factor);
     } else if (threadIdx.x == 0) {  // same order as reduce_partials_kernel
-        out[row] = TR::finalize(fold_published<TR>(mine, 1, splits), factor);
+        out[row] = TR::finalize(fold_published<TR>(mine, splits), factor);
     }
 }
 
@@ -466,7 +467,9 @@ __global__ void __launch_bounds__(kColLanes* kColRows) reduce_cols_kernel(const 
                 for (int c = threadIdx.x; c < kColLanes * VEC; c += kColLanes * kColRows) {
                     u64 gc = (u64)blockIdx.x * kColLanes * VEC + c;
                     if (gc < I) {
-                        out[o * I + gc] = TR::finalize(fold_published<TR>(partial + o * I + gc, O * I, splits), factor);
+                        Acc v = TR::init();
+                        for (u32 s2 = 0; s2 < splits; s2++) v = TR::combine(v, load_published(partial + ((u64)s2 * O + o) * I + gc));
+                        out[o * I + gc] = TR::finalize(v, factor);
                     }
                 }
             }
