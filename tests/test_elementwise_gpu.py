@@ -416,6 +416,20 @@ def test_last_block_of_flat_operands(oracle, cuda, dt):
         H.assert_same("add_scalar", dt, got, ref, what=f"n={n}")
 
 
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F64, D.U8, D.I32], ids=lambda d: d.name)
+def test_short_last_block_by_elements(oracle, cuda, dt):
+    """Last blocks on both sides of where elements give way to vectors (one to three trips of 256 threads), alone and behind whole blocks."""
+    rng = np.random.default_rng(zlib.crc32(dt.name.encode()) + 2)
+    block = 1024 * (16 // dt.size)
+    for n in (17, 255, 256, 257, 511, 512, 513, 767, 768, 769, block + 1, block + 256, block + 257, block + 513, 2 * block + 768, 2 * block + 769):
+        a, b = (H.random_store(rng, dt, n, lo=1, hi=50) if dt.kind != "float" else H.random_store(rng, dt, n, lo=0.5, hi=2.0) for _ in range(2))
+        for rs in (1, 0):
+            args = ("div", dt, [n], [1], [rs], 0, 0, a, b)
+            H.assert_same("div", dt, H.run_binary(cuda, *args), H.run_binary(oracle, *args), what=f"n={n} rhs stride {rs}")
+        got, ref = (H.run_unary(be, "add_scalar", dt, [n], [1], 0, a, scalar=3) for be in (cuda, oracle))
+        H.assert_same("add_scalar", dt, got, ref, what=f"n={n}")
+
+
 @pytest.mark.parametrize("dt", [D.BF16, D.F16, D.I16, D.U16], ids=lambda d: d.name)
 def test_two_byte_transposed_tiles(oracle, cuda, dt):
     """2-byte types with vector-aligned transposed operands run on the tensor-copy tile kernel (64 x 64 boxes, ldmatrix
