@@ -269,7 +269,8 @@ void mx_set_small_pool(int enabled);
  * the host and the device (returns the first failing call's code, 0 = ok); after the op, give the block back (returns the
  * sticky status of mx_last_error).  The block is for the op calls in between: small ones are pinned host memory, which the launcher
  * reads in place and which is used again once it is given back, so device work of the caller's own that reads it must have finished
- * by then; longer ones are cuda_malloc and cuda_memcpy_h2d, as all are after mx_set_small_pool(0). */
+ * by then; longer ones are cuda_malloc and cuda_memcpy_h2d, as all are after mx_set_small_pool(0).  The block's words may be written anew while
+ * it is open (cuda_memcpy_h2d, cuda_memcpy_d2d). */
 int mx_dispatch_begin(int device, const size_t* host_metadata, size_t count, void** block);
 int mx_dispatch_end(void* block);
 

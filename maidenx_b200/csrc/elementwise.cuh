@@ -819,7 +819,8 @@ __global__ void __launch_bounds__(kEwThreads) ew_generic_kernel(F f, const T* a,
 // whose offsets are both known up front, so that all loads are independent; an input that is constant along the rows costs
 // two loads per vector.  Shorter rows walk the vector row by row.
 // Bound by HBM / L2 where rows are long enough: [8191, 1023] f32 with a per-row operand 12 us (33 on the gather
-// kernel; a flat op on the same data 9); [256, 512, 7, 7] bf16 with a per-channel one 9.9 us (33).
+// kernel; a flat op on the same data 9); [256, 512, 7, 7] bf16 with a per-channel one 9.9 us (33).  These two and a row that repeats have kernels of
+// their own below; here stay ops of one input, operands at odd addresses, more than three dims, rows shorter than a vector and vectors of 16 elements.
 enum EwDenseKind { EWD_VECTOR = 0, EWD_ELEMENT, EWD_CONST, EWD_STEP };
 constexpr int kEwDenseUnroll = 2;
 struct EwDenseParams {
@@ -926,7 +927,8 @@ __global__ void __launch_bounds__(kEwThreads) ew_dense_kernel(F f, const T* a, c
 // dims, every element's own choice): here the place of a vector costs two divisions by multiplication, the row behind comes from
 // the one before it without another, both values a vector can see are loaded whether or not its rows change inside it, and a thread has
 // four vectors' loads in flight.  [256, 512, 7, 7] bf16 with a per-channel operand 5.3 us (10.2 by the kernel above), [8191, 1023] f32 with a per-row
-// one 8.5 (11.6).
+// one 8.5 (11.6).  Wherever the kernel above would take a call of this form, from 2^15 vectors on, this one is faster: rows of 5 to 1023 f32, 9 to 1023 bf16, 3 to 1023 f64,
+// per row 2^15 vectors 1.9 to 2.1 / 1.8 to 1.9 us, 2^17 2.0 to 2.3 / 1.8 to 2.0, 2^20 5.3 to 6.7 / 4.2 to 4.8; per channel 2.3 to 2.5 / 1.7 to 1.9 and 6.9 to 8.7 / 4.2 to 4.7.
 struct FastDiv31 {  // floor(n / d) for n < 2^31 and d >= 2: with 2^s < d <= 2^(s+1) and m = ceil(2^(32+s) / d), n (m d - 2^(32+s)) < 2^(32+s)
     uint32_t d, m, s;
     void init(uint32_t div) {
@@ -1001,7 +1003,8 @@ __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, co
 }
 
 // Two inputs of ragged rows, each the output's own layout or the same row for all of them (a bias, a norm's weights): one division by multiplication a
-// vector, the repeated row from L1 by elements, four vectors a thread.  [8191, 1023] f32 10.3 us (11.8 by the dense kernel), [4099, 1543] bf16 7.0 (8.1).  An instantiation of the kernel above for it would have the constants'
+// vector, the repeated row from L1 by elements, four vectors a thread.  [8191, 1023] f32 10.3 us (11.8 by the dense kernel), [4099, 1543] bf16 7.0 (8.1); 2^15 vectors
+// 1.7 to 2.3 by either (bf16 rows of 197 2.10 / 2.18), 2^18 2.5 to 3.4 / 2.0 to 3.0, 2^20 5.3 to 8.2 / 4.2 to 7.5.  An instantiation of the kernel above for it would have the constants'
 // registers too (94 instead of 79 in 16 bits).
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_repeat_kernel(F f, const T* a, const T* b, O* out, EwRepeatParams P) {
