@@ -131,19 +131,27 @@ __device__ __forceinline__ Vec<O, VEC> apply_vec(const F& f, const Vec<T, VEC>& 
     return r;
 }
 
-// What the last, incomplete block still does element by element: one, two or three trips.  Vectors give a few threads the work of all and take a second
+// What an incomplete block still does element by element: one, two or three trips.  Vectors give a few threads the work of all and take a second
 // path for the rest.  Elements / vectors, us: difference of 100 u8 0.95 / 1.84, bf16 0.94 / 1.33, quotient 1.04 / 2.64, 1.10 / 1.93, f32 1.00 / 1.32; 300 u8 1.20 / 1.84,
 // bf16 1.14 / 1.19, quotient 1.39 / 1.78, f32 difference 1.15 / 1.02; 700 u8 1.38 / 1.68, bf16 1.33 / 1.21; square of 1000 u8 1.50 / 1.30, bf16 1.73 / 1.04.
 template <int VEC>
 constexpr uint64_t kEwTailElements = kEwThreads * (VEC >= 16 ? 3 : VEC == 8 ? 2 : 1);
+// Elements of a block: four vectors a thread, all loads in flight together, or one while that leaves an SM two blocks at most: those blocks, and the last of
+// the others, take their vectors one after the other in a loop of its own, which costs the main one no registers (with all of an incomplete block's loads
+// in flight it had 142 instead of 42, product of i16, 74 instead of 32, comparison of bf16, and fewer blocks an SM for it).  One / four vectors a
+// thread, us: difference of 2048 vectors f32 1.3 / 1.5, u8 1.7 / 3.7; 60000 1.5 / 1.9, 2.8 / 3.8; 150000 1.84 / 1.79, 5.1 / 3.8; square root of 8191 f32 1.3 / 2.3, 6.4 by elements.
+template <int VEC>
+inline uint32_t ew_flat_chunk(uint64_t n) {
+    return (uint32_t)(kEwThreads * VEC) * (n / VEC <= 2 * (uint64_t)kEwThreads * sm_count() ? 1 : kEwUnroll);
+}
 
-// sa / sb: 1 = contiguous, 0 = broadcast scalar
+// sa / sb: 1 = contiguous, 0 = broadcast scalar; chunk: ew_flat_chunk
 template <class F, class T, class O, int NIN, int VEC>
-__global__ void __launch_bounds__(kEwThreads) ew_flat_kernel(F f, const T* a, const T* b, O* out, uint64_t n, int sa, int sb) {
+__global__ void __launch_bounds__(kEwThreads) ew_flat_kernel(F f, const T* a, const T* b, O* out, uint64_t n, int sa, int sb, uint32_t chunk) {
     after_previous_kernel();
-    constexpr uint64_t kChunk = (uint64_t)kEwThreads * VEC * kEwUnroll;
-    const uint64_t base = (uint64_t)blockIdx.x * kChunk;
-    if (base + kChunk <= n) {
+    constexpr uint32_t kChunk = (uint32_t)kEwThreads * VEC * kEwUnroll;
+    const uint64_t base = (uint64_t)blockIdx.x * chunk;
+    if (chunk == kChunk && base + kChunk <= n) {
         Vec<T, VEC> va[kEwUnroll], vb[kEwUnroll];
 #pragma unroll
         for (int u = 0; u < kEwUnroll; u++) {
@@ -156,35 +164,24 @@ __global__ void __launch_bounds__(kEwThreads) ew_flat_kernel(F f, const T* a, co
             uint64_t i = base + ((uint64_t)u * kEwThreads + threadIdx.x) * VEC;
             st_vec<O, VEC>(out + i, apply_vec<F, T, O, NIN, VEC>(f, va[u], vb[u]));
         }
-    } else if (n - base <= kEwTailElements<VEC>) {
-        for (uint64_t i = base + threadIdx.x; i < n; i += kEwThreads) {
-            T x = a[sa ? i : 0];
-            if constexpr (NIN == 2) out[i] = f(x, b[sb ? i : 0]);
-            else out[i] = f(x);
+        return;
+    }
+    const uint64_t end = base + chunk < n ? base + chunk : n;
+    uint64_t rest = base;
+    if (end - base > kEwTailElements<VEC>) {
+#pragma unroll 1
+        for (uint64_t i = base + (uint64_t)threadIdx.x * VEC; i + VEC <= end; i += kEwThreads * VEC) {
+            const Vec<T, VEC> va = sa ? ld_vec<T, VEC>(a + i) : splat<T, VEC>(a[0]);
+            Vec<T, VEC> vb;
+            if constexpr (NIN == 2) vb = sb ? ld_vec<T, VEC>(b + i) : splat<T, VEC>(b[0]);
+            st_vec<O, VEC>(out + i, apply_vec<F, T, O, NIN, VEC>(f, va, vb));
         }
-    } else {
-        // The last, incomplete block: vectors as well, all loads in flight together, and only what is left of a vector by elements.
-        // Element by element it walked up to 64 trips to memory one after the other, the length of the whole launch (square root of 8191 f32: 6.4 us, 2.5 so).
-        Vec<T, VEC> va[kEwUnroll], vb[kEwUnroll];
-#pragma unroll
-        for (int u = 0; u < kEwUnroll; u++) {
-            const uint64_t i = base + ((uint64_t)u * kEwThreads + threadIdx.x) * VEC;
-            if (i + VEC <= n) {
-                va[u] = sa ? ld_vec<T, VEC>(a + i) : splat<T, VEC>(a[0]);
-                if constexpr (NIN == 2) vb[u] = sb ? ld_vec<T, VEC>(b + i) : splat<T, VEC>(b[0]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kEwUnroll; u++) {
-            const uint64_t i = base + ((uint64_t)u * kEwThreads + threadIdx.x) * VEC;
-            if (i + VEC <= n) st_vec<O, VEC>(out + i, apply_vec<F, T, O, NIN, VEC>(f, va[u], vb[u]));
-        }
-        const uint64_t i = n - n % VEC + threadIdx.x;
-        if (i < n) {
-            T x = a[sa ? i : 0];
-            if constexpr (NIN == 2) out[i] = f(x, b[sb ? i : 0]);
-            else out[i] = f(x);
-        }
+        rest = end - end % VEC;  // blocks start at whole vectors
+    }
+    for (uint64_t i = rest + threadIdx.x; i < end; i += kEwThreads) {
+        T x = a[sa ? i : 0];
+        if constexpr (NIN == 2) out[i] = f(x, b[sb ? i : 0]);
+        else out[i] = f(x);
     }
 }
 
@@ -1117,7 +1114,8 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                     break;
                 }
             }
-            launch_kernel(ew_flat_kernel<F, T, O, NIN, VEC>, (uint32_t)blocks, kEwThreads, 0, s, f, a, b, out, pl.n, (int)pl.st[1][0], NIN == 2 ? (int)pl.st[2][0] : 0);
+            const uint32_t block = ew_flat_chunk<VEC>(pl.n);
+            launch_kernel(ew_flat_kernel<F, T, O, NIN, VEC>, (uint32_t)((pl.n + block - 1) / block), kEwThreads, 0, s, f, a, b, out, pl.n, (int)pl.st[1][0], NIN == 2 ? (int)pl.st[2][0] : 0, block);
             break;
         }
         case EW_FLAT_SHIFT: {
