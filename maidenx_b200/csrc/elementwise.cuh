@@ -923,9 +923,8 @@ __global__ void __launch_bounds__(kEwThreads) ew_dense_kernel(F f, const T* a, c
 // operand whose rows are no whole vectors, the commonest call of the kernel above.  What bounds that one there is its instructions (loops over the
 // dims, every element's own choice): here the place of a vector costs two divisions by multiplication, the row behind comes from
 // the one before it without another, both values a vector can see are loaded whether or not its rows change inside it, and a thread has
-// four vectors' loads in flight.  [256, 512, 7, 7] bf16 with a per-channel operand 5.3 us (10.2 by the kernel above), [8191, 1023] f32 with a per-row
-// one 8.5 (11.6).  Wherever the kernel above would take a call of this form, from 2^15 vectors on, this one is faster: rows of 5 to 1023 f32, 9 to 1023 bf16, 3 to 1023 f64,
-// per row 2^15 vectors 1.9 to 2.1 / 1.8 to 1.9 us, 2^17 2.0 to 2.3 / 1.8 to 2.0, 2^20 5.3 to 6.7 / 4.2 to 4.8; per channel 2.3 to 2.5 / 1.7 to 1.9 and 6.9 to 8.7 / 4.2 to 4.7.
+// up to four vectors' loads in flight (ew_chan_units).  [256, 512, 7, 7] bf16 with a per-channel operand 5.3 us (10.2 by the kernel above), [8191, 1023] f32 with a per-row
+// one 8.5 (11.6).
 struct FastDiv31 {  // floor(n / d) for n < 2^31 and d >= 2: with 2^s < d <= 2^(s+1) and m = ceil(2^(32+s) / d), n (m d - 2^(32+s)) < 2^(32+s)
     uint32_t d, m, s;
     void init(uint32_t div) {
@@ -941,25 +940,46 @@ struct EwChanParams {
     FastDiv31 q_div, channel_div;
     int vector[3];              // [1], [2]: the input has the output's layout
     int s_outer[3], s_channel[3];
+    int units;                  // vectors a thread (ew_chan_units)
 };
 struct EwRepeatParams {
     uint32_t n, q;    // elements; extent of the innermost dim
     FastDiv31 q_div;
     int repeated[3];  // [1], [2]: the input is one row for all rows, else it has the output's layout
+    int units;
 };
 constexpr int kEwChanUnroll = 4;
+// Vectors a thread of the two kernels below; 0: the dense kernel.  One while that leaves an SM two blocks at most, two up to three blocks an SM (94 registers: the
+// next would wait), then four.  Divisions are bound by their instructions and keep two longer: f32 to eight blocks an SM, 16-bit floats always; integer
+// ones have nothing to hide behind the loads and leave.  Dense / one / two / four, us, a row's or a channel's operand beside rows of 1023:
+//   f32 difference    33000 vectors 1.84 1.33 1.54 1.91    220000 2.33 2.13 1.94 2.33    1200000 5.92 5.99 5.02 4.90
+//   f32 quotient      33000 2.35 1.83 2.08 2.87            300000 2.96 3.48 2.74 3.17    2400000 17.2 20.9 16.7 14.6
+//   bf16 quotient     33000 4.91 2.83 4.60 8.10            300000 7.68 7.37 6.85 9.13    2400000 47.2 47.1 42.9 43.5
+//   bf16 comparison   33000 2.34 1.62 1.94 2.85            300000 3.15 3.68 3.47 3.38    1200000 9.93 11.1 9.61 8.81
+//   i16 quotient      33000 4.50 2.66 4.09 7.27            300000 6.53 7.78 8.39 8.38    2400000 42.6 51.7 47.2 48.4
+template <class F, class T>
+inline int ew_chan_units(uint64_t vecs) {
+    const uint64_t sms = sm_count();
+    if (vecs <= 2 * kEwThreads * sms) return 1;
+    if (vecs <= 6 * kEwThreads * sms) return 2;
+    if constexpr (F::kDivides) {
+        if (is_int_v<T>) return 0;
+        if (is_half_v<T> || vecs <= 16 * kEwThreads * sms) return 2;
+    }
+    return 4;
+}
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, const T* b, O* out, EwChanParams P) {
     after_previous_kernel();
     constexpr int U = kEwChanUnroll;
-    const uint32_t first = (blockIdx.x * U * kEwThreads + threadIdx.x) * VEC;
+    const uint32_t first = (blockIdx.x * P.units * kEwThreads + threadIdx.x) * VEC;
     Vec<T, VEC> va[U], vb[U];
     T xa[U][2], xb[U][2];
     int left[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
         const uint32_t i0 = first + u * kEwThreads * VEC;
-        if (i0 >= P.n) continue;
+        if (u >= P.units || i0 >= P.n) continue;
         const uint32_t row = P.q_div.div(i0), outer = P.channel_div.div(row), channel = row - outer * P.channels;
         left[u] = (int)(P.q - (i0 - row * P.q));  // elements of the vector's first row from i0 on
         const bool wraps = channel + 1 == P.channels, ends = left[u] < VEC && i0 + left[u] < P.n;
@@ -983,7 +1003,7 @@ __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, co
 #pragma unroll
     for (int u = 0; u < U; u++) {
         const uint32_t i0 = first + u * kEwThreads * VEC;
-        if (i0 >= P.n) continue;
+        if (u >= P.units || i0 >= P.n) continue;
         auto spread = [&](int k, Vec<T, VEC>& v, const T(&x)[2]) {
             if (!P.vector[k])
 #pragma unroll
@@ -1000,19 +1020,18 @@ __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, co
 }
 
 // Two inputs of ragged rows, each the output's own layout or the same row for all of them (a bias, a norm's weights): one division by multiplication a
-// vector, the repeated row from L1 by elements, four vectors a thread.  [8191, 1023] f32 10.3 us (11.8 by the dense kernel), [4099, 1543] bf16 7.0 (8.1); 2^15 vectors
-// 1.7 to 2.3 by either (bf16 rows of 197 2.10 / 2.18), 2^18 2.5 to 3.4 / 2.0 to 3.0, 2^20 5.3 to 8.2 / 4.2 to 7.5.  An instantiation of the kernel above for it would have the constants'
-// registers too (94 instead of 79 in 16 bits).
+// vector, the repeated row from L1 by elements, up to four vectors a thread.  [8191, 1023] f32 10.3 us (11.8 by the dense kernel), [4099, 1543] bf16 7.0 (8.1).  An
+// instantiation of the kernel above for it would have the constants' registers too (94 instead of 79 in 16 bits).
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_repeat_kernel(F f, const T* a, const T* b, O* out, EwRepeatParams P) {
     after_previous_kernel();
     constexpr int U = kEwChanUnroll;
-    const uint32_t first = (blockIdx.x * U * kEwThreads + threadIdx.x) * VEC;
+    const uint32_t first = (blockIdx.x * P.units * kEwThreads + threadIdx.x) * VEC;
     Vec<T, VEC> va[U], vb[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
         const uint32_t i0 = first + u * kEwThreads * VEC;
-        if (i0 >= P.n) continue;
+        if (u >= P.units || i0 >= P.n) continue;
         const uint32_t col = i0 - P.q_div.div(i0) * P.q;
         auto load = [&](const T* p, int repeated, Vec<T, VEC>& v) {
             if (repeated) {
@@ -1032,6 +1051,7 @@ __global__ void __launch_bounds__(kEwThreads) ew_repeat_kernel(F f, const T* a, 
 #pragma unroll
     for (int u = 0; u < U; u++) {
         const uint32_t i0 = first + u * kEwThreads * VEC;
+        if (u >= P.units) continue;
         if (i0 + VEC <= P.n) {
             st_vec<O, VEC>(out + i0, apply_vec<F, T, O, 2, VEC>(f, va[u], vb[u]));
         } else {
@@ -1194,13 +1214,15 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                 const uint64_t vecs = (pl.n + VEC - 1) / VEC;
                 if constexpr (NIN == 2 && VEC <= 8) {  // 16 elements a vector would take 145 registers
                     EwChanParams C;
-                    if (ew_fill_chan_params(D, VEC, C)) {
-                        launch_kernel(ew_chan_kernel<F, T, O, VEC>, (uint32_t)((vecs + kEwThreads * kEwChanUnroll - 1) / (kEwThreads * kEwChanUnroll)), kEwThreads, 0, s, f, a, b, out, C);
+                    EwRepeatParams Q;
+                    C.units = Q.units = ew_chan_units<F, T>(vecs);
+                    const uint32_t blocks = C.units ? (uint32_t)((vecs + kEwThreads * C.units - 1) / (kEwThreads * C.units)) : 0;
+                    if (blocks && ew_fill_chan_params(D, VEC, C)) {
+                        launch_kernel(ew_chan_kernel<F, T, O, VEC>, blocks, kEwThreads, 0, s, f, a, b, out, C);
                         break;
                     }
-                    EwRepeatParams Q;
-                    if (ew_fill_repeat_params(D, VEC, Q)) {
-                        launch_kernel(ew_repeat_kernel<F, T, O, VEC>, (uint32_t)((vecs + kEwThreads * kEwChanUnroll - 1) / (kEwThreads * kEwChanUnroll)), kEwThreads, 0, s, f, a, b, out, Q);
+                    if (blocks && ew_fill_repeat_params(D, VEC, Q)) {
+                        launch_kernel(ew_repeat_kernel<F, T, O, VEC>, blocks, kEwThreads, 0, s, f, a, b, out, Q);
                         break;
                     }
                 }
