@@ -237,11 +237,13 @@ __global__ void __launch_bounds__(kFusedThreads) mse_finish_kernel(const float* 
     if (threadIdx.x == 0) *loss = l * inv_n;
 }
 
+// Bound by HBM.  Two vectors of each operand are loaded before the first store: without restricted pointers, which kernels that wait may not have, the
+// compiler leaves the loads of the next step behind the stores of this one (40e6 elements f16 90.9 us, 75.1 so, bf16 80.0, 75.1).
 template <class T>
 __global__ void __launch_bounds__(kFusedThreads) sgd_kernel(float* w32, const T* g, T* w16, uint64_t n,
                                                            float step, float* b32, const T* gb, T* b16) {
     after_previous_kernel();
-    constexpr int VEC = 16 / sizeof(T);  // elements per 16-byte vector of the gradient; w32 moves as VEC floats
+    constexpr int VEC = 16 / sizeof(T), UN = 2;  // elements per 16-byte vector of the gradient; w32 moves as VEC floats
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
     if (b32 && blockIdx.x == 0 && threadIdx.x == 0) {  // the layer's one-element bias
@@ -249,26 +251,37 @@ __global__ void __launch_bounds__(kFusedThreads) sgd_kernel(float* w32, const T*
         *b32 = w;
         *b16 = st_from_f32<T>(w);
     }
-    for (uint64_t v = (uint64_t)blockIdx.x * kFusedThreads + threadIdx.x; v < nvec; v += stride) {
-        Vec<T, VEC> gi = *reinterpret_cast<const Vec<T, VEC>*>(g + v * VEC), wo;
+    for (uint64_t v0 = (uint64_t)blockIdx.x * kFusedThreads + threadIdx.x; v0 < nvec; v0 += UN * stride) {
+        Vec<T, VEC> gi[UN], wo;
         // the master weights are promised 16-byte aligned only: move them as float4 quads, never as one 32-byte access
-        float4 w[VEC / 4];
+        float4 w[UN][VEC / 4];
 #pragma unroll
-        for (int q = 0; q < VEC / 4; q++) w[q] = *reinterpret_cast<const float4*>(w32 + v * VEC + 4 * q);
+        for (int i = 0; i < UN; i++)
+            if (v0 + i * stride < nvec) {
+                const uint64_t at = (v0 + i * stride) * VEC;
+                gi[i] = *reinterpret_cast<const Vec<T, VEC>*>(g + at);
 #pragma unroll
-        for (int q = 0; q < VEC / 4; q++) {
-            w[q].x = w[q].x - step * up(gi.v[4 * q + 0]);
-            w[q].y = w[q].y - step * up(gi.v[4 * q + 1]);
-            w[q].z = w[q].z - step * up(gi.v[4 * q + 2]);
-            w[q].w = w[q].w - step * up(gi.v[4 * q + 3]);
-            wo.v[4 * q + 0] = st_from_f32<T>(w[q].x);
-            wo.v[4 * q + 1] = st_from_f32<T>(w[q].y);
-            wo.v[4 * q + 2] = st_from_f32<T>(w[q].z);
-            wo.v[4 * q + 3] = st_from_f32<T>(w[q].w);
-        }
+                for (int q = 0; q < VEC / 4; q++) w[i][q] = *reinterpret_cast<const float4*>(w32 + at + 4 * q);
+            }
 #pragma unroll
-        for (int q = 0; q < VEC / 4; q++) *reinterpret_cast<float4*>(w32 + v * VEC + 4 * q) = w[q];
-        *reinterpret_cast<Vec<T, VEC>*>(w16 + v * VEC) = wo;
+        for (int i = 0; i < UN; i++)
+            if (v0 + i * stride < nvec) {
+                const uint64_t at = (v0 + i * stride) * VEC;
+#pragma unroll
+                for (int q = 0; q < VEC / 4; q++) {
+                    float4& x = w[i][q];
+                    x.x = x.x - step * up(gi[i].v[4 * q + 0]);
+                    x.y = x.y - step * up(gi[i].v[4 * q + 1]);
+                    x.z = x.z - step * up(gi[i].v[4 * q + 2]);
+                    x.w = x.w - step * up(gi[i].v[4 * q + 3]);
+                    wo.v[4 * q + 0] = st_from_f32<T>(x.x);
+                    wo.v[4 * q + 1] = st_from_f32<T>(x.y);
+                    wo.v[4 * q + 2] = st_from_f32<T>(x.z);
+                    wo.v[4 * q + 3] = st_from_f32<T>(x.w);
+                    *reinterpret_cast<float4*>(w32 + at + 4 * q) = x;
+                }
+                *reinterpret_cast<Vec<T, VEC>*>(w16 + at) = wo;
+            }
     }
     if (blockIdx.x == 0)
         for (uint64_t i = nvec * VEC + threadIdx.x; i < n; i += kFusedThreads) {
