@@ -182,19 +182,21 @@ __device__ __forceinline__ Acc load_published(const Acc* p) {
 }
 
 // The fold of a row's `splits` published parts in split order, eight of them in flight: one thread folds an output while the
-// rest of the launch is over, so each trip to L2 counts in full.  Not in the kernel of columns, where it takes registers from the main loop (bf16
-// 52, 80 with it; 130 x 300000 8.8 us, 10.1; 100001 x 16 f32 32.0, 37.2; 2047 x 20000 f64 49.7, 54.5; only 2047 x 20000 bf16 10.2, 9.6).
+// rest of the launch is over, so each trip to L2 counts in full.  One by one where eight take registers from the main loop: f64 (means 34, 52 with eight),
+// and in the kernel of columns, which has its own (bf16 52, 80; 130 x 300000 8.8 us, 10.1; 100001 x 16 f32 32.0, 37.2; 2047 x 20000 f64 49.7, 54.5; only 2047 x
+// 20000 bf16 10.2, 9.6).
 template <class TR>
 __device__ __forceinline__ typename TR::Acc fold_published(const typename TR::Acc* p, u32 splits) {
     typedef typename TR::Acc Acc;
+    constexpr u32 UN = std::is_same<Acc, f64>::value ? 1 : 8;
     Acc acc = TR::init();
-    for (u32 s = 0; s < splits; s += 8) {
-        Acc v[8];
+    for (u32 s = 0; s < splits; s += UN) {
+        Acc v[UN];
 #pragma unroll
-        for (u32 q = 0; q < 8; q++)
+        for (u32 q = 0; q < UN; q++)
             if (s + q < splits) v[q] = load_published(p + s + q);
 #pragma unroll
-        for (u32 q = 0; q < 8; q++)
+        for (u32 q = 0; q < UN; q++)
             if (s + q < splits) acc = TR::combine(acc, v[q]);
     }
     return acc;
@@ -407,8 +409,9 @@ constexpr int kColRows = 8;    // threads along the reduced dim
 
 // grid = (ceil(I / (32 * VEC)), splits, min(O, 65535)).  VEC > 1 requires I % VEC == 0 and an
 // aligned base.
+// Eight-byte types keep to the registers of five blocks an SM (maxima of u64 took 54 of them since the wait at the top, four blocks: [48950, 873] 66 us before, 74, 54 so).
 template <class T, int KIND, int VEC>
-__global__ void __launch_bounds__(kColLanes* kColRows) reduce_cols_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial, u64 O,
+__global__ void __launch_bounds__(kColLanes* kColRows, sizeof(T) == 8 ? 5 : 1) reduce_cols_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial, u64 O,
                                                                          u64 R, u64 I, u64 seg, u32 splits, u64 factor, u32* counters) {
     after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
