@@ -6,7 +6,7 @@
 //     small = x - big   (exact in f32; its own low bits are again dropped by the tensor core),
 // and each k-step multiplies
 //     a_small * b_big  +  a_big * b_small  +  a_big * b_big
-// by three MMAs into one TMEM accumulator, or (long reductions, Params::wide) by two: a_big by [b_big | b_small], which lie behind one another, into an
+// by three MMAs into one TMEM accumulator, or (long reductions, WIDE) by two: a_big by [b_big | b_small], which lie behind one another, into an
 // accumulator of twice the columns, and a_small * b_big into its second half; the halves meet in the epilogue's registers.
 // The dropped term a_small * b_small and the truncation of `small` are each below 2^-21 of |a * b|, so a dot
 // product agrees with f32 arithmetic to a few 1e-7 relative to sum |a_k * b_k| (the stated f32 matmul tolerance is
@@ -62,7 +62,7 @@ constexpr int EPI_WARPS = 4, SPLIT_WARPS = 4;
 constexpr int EPI_CHUNK_COLS = 32;             // 32 f32 = 128 bytes per staged row
 constexpr int EPI_STAGE_BYTES = 32 * EPI_CHUNK_COLS * 4;  // 4 KB per warp per buffer
 constexpr int THREADS = 32 * (2 + EPI_WARPS + SPLIT_WARPS);
-constexpr int TMEM_COLS = 4 * BN;              // two f32 accumulators, each [big x big | products with a small factor] (Params::wide)
+constexpr int TMEM_COLS = 4 * BN;              // two f32 accumulators, each [big x big | products with a small factor] (WIDE)
 constexpr int GROUP_M = 16;
 constexpr int CHUNK_FAST = 4;
 constexpr int MN_CHUNK_BYTES = BK * 128;       // one [32 K-rows x 32 MN-elements] box
@@ -103,7 +103,6 @@ struct Params {
     int bn;         // columns of an output tile: 64 or 128
     int stages;     // of the ring
     int raw_bytes;  // what TMA delivers per stage: A and bn rows of B
-    int wide;       // 1: big x [big | small] in one instruction, the products with a small factor in an accumulator of their own (see kWideLeast)
     int split_kb;   // > 0: split-K; batch s of the launch reduces the k-blocks [s * split_kb, (s + 1) * split_kb) of one product
     int kb_per_z;   // > 0: the reduction runs over the operands' batches too: k-block i is block i % kb_per_z of batch i / kb_per_z
     int d_plain;    // != 0: the output's rows (or base) are not 16-byte multiples: the epilogue warps write them to `out` themselves
@@ -151,6 +150,7 @@ static_assert(PART_OFF + BM * PART_LD * 4 <= STAGES * STAGE_BYTES && 2 * BK * (B
 // infinity or NaN among the operands always leaves a non-finite sum here, whatever becomes of it, so the epilogue's look at its totals
 // finds every such tile at the cost of one FMA per output, and finite operands cost nothing else (products of K = 64: 4 to 7 %; of
 // K = 1024 and more: none).  k ascending with separate multiply and add, as on the CUDA cores.  All threads of the block; `stage` is the operand ring, which nothing uses any more.
+template <bool INTO_PART>  // into the partial result of a CTA of a cluster
 __device__ __forceinline__ void redo_tile(const Params& p, int bn, int tm, int tn, int tb, float* stage) {
     constexpr int LD = BM + 4, T = 16;  // 16 x 16 threads, rows ty + 16 i, columns tx + 16 j
     float *xs = stage, *ys = stage + BK * LD;  // [k][row], [k][column]
@@ -201,7 +201,7 @@ __device__ __forceinline__ void redo_tile(const Params& p, int bn, int tm, int t
         for (int j = 0; j < BN / T; j++) {
             const int c = tx + T * j;
             if (row >= p.M || c >= bn || tn * bn + c >= p.N) continue;
-            if (p.cluster) stage[PART_OFF / 4 + (ty + T * i) * PART_LD + c] = acc[i][j];
+            if constexpr (INTO_PART) stage[PART_OFF / 4 + (ty + T * i) * PART_LD + c] = acc[i][j];
             else p.out[((int64_t)tb * p.M + row) * p.out_ld + tn * bn + c] = acc[i][j];
         }
     }
@@ -210,8 +210,10 @@ __device__ __forceinline__ void redo_tile(const Params& p, int bn, int tm, int t
 // BN_T = 128: the form of 128-column tiles, long chunks and tensor stores, all known to the compiler; 0: everything from the
 // parameters.  The difference is the splitter's: with the distance between a raw and its small tile a constant, its loads run
 // ahead of its stores (8192 x 4096 x 4096: 164 TFLOP/s, 148 in batches of four).
-// CLUSTER: Params::cluster.
-template <int BN_T, bool CLUSTER = false>
+// FORM: what the slices and the parts of B take is compiled in.  As a parameter the wide form cost the others' epilogue registers (24 bytes spilled, 40 with
+// it) and time where a tile is little else: 165 x (8 x 4008 x 8) 75.8 us, 88.9.
+enum Form { PLAIN = 0, WIDE = 1, CLUSTERED = 2 };  // WIDE: see kWideLeast; CLUSTERED: Params::cluster
+template <int BN_T, int FORM = PLAIN>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                    Params p, int* err, int tag) {
@@ -232,7 +234,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? STAGES : p.stages, raw_bytes = BN_T ? A_TILE + BN_T * BK * 4 : p.raw_bytes;
 
     // a CTA of a cluster of slices has one tile and slice: its rank is the batch, and the grid is as long as the tiles
-    const int first_tile = CLUSTER ? (int)blockIdx.x % p.cluster * p.tiles_per_batch + (int)blockIdx.x / p.cluster : (int)blockIdx.x;
+    const int first_tile = FORM == CLUSTERED ? (int)blockIdx.x % p.cluster * p.tiles_per_batch + (int)blockIdx.x / p.cluster : (int)blockIdx.x;
 
     auto redo = [&] { return reinterpret_cast<uint32_t*>(smem + Smem::redo); };
     if (threadIdx.x <= REDO_BITS / 32) redo()[threadIdx.x] = 0;
@@ -333,7 +335,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                         const uint64_t b_big = p.b_mn ? smem_desc_sw128_atom32(s_b, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s_b, 16, 1024);
                         const uint64_t a_small = p.a_mn ? smem_desc_sw128_atom32(s0 + A_TILE, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s0 + A_TILE, 16, 1024);
                         const uint64_t b_small = p.b_mn ? smem_desc_sw128_atom32(s_bs, MN_CHUNK_BYTES, 512) : smem_desc_sw128(s_bs, 16, 1024);
-                        if (p.wide) {  // the small part of B lies behind the raw one: one instruction of twice the columns multiplies a_big by both
+                        if constexpr (FORM == WIDE) {  // the small part of B lies behind the raw one: one instruction of twice the columns multiplies a_big by both
 #pragma unroll
                             for (int k = 0; k < BK / UMMA_K; k++) {
                                 umma_tf32(d_tmem, a_big + a_kstep * k, b_big + b_kstep * k, idesc_wide, (kb != kb0) || (k != 0));
@@ -397,7 +399,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 for (int c = 0; c < BN / 32; c++) {
                     if (c * 32 >= bn) break;
                     uint32_t v[32];
-                    if (p.wide) {  // the sum of the small products first
+                    if constexpr (FORM == WIDE) {  // the sum of the small products first
                         tmem_ld_32x32b_x32(t_row + bn + c * 32, v);
                         tmem_ld_wait();
 #pragma unroll
@@ -419,7 +421,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
             if (!ok) break;
             float zero = 0.0f;  // NaN from the first total on that is not finite
-            if constexpr (CLUSTER) {
+            if constexpr (FORM == CLUSTERED) {
                 float* part = reinterpret_cast<float*>(smem + Smem::stages + PART_OFF) + (quarter * 32 + lane) * PART_LD;  // the ring is done with
 #pragma unroll
                 for (int j = 0; j < BN; j += 4) {
@@ -535,10 +537,10 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
 
-    if constexpr (CLUSTER) {
+    if constexpr (FORM == CLUSTERED) {
         int tm, tn, tb;
         tile_coords(first_tile, p, tm, tn, tb);
-        if (redo()[REDO_BITS / 32]) redo_tile(p, bn, tm, tn, tb, reinterpret_cast<float*>(smem + Smem::stages));
+        if (redo()[REDO_BITS / 32]) redo_tile<true>(p, bn, tm, tn, tb, reinterpret_cast<float*>(smem + Smem::stages));
         cluster_sync_all();
         const int r0 = BM * tb / p.cluster, rows = BM * (tb + 1) / p.cluster - r0, vecs = bn / 4;
         for (int e = threadIdx.x; e < rows * vecs; e += THREADS) {
@@ -566,7 +568,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         if (!(redo()[it % REDO_BITS / 32] >> it % 32 & 1)) continue;
         int tm, tn, tb;
         tile_coords(tile, p, tm, tn, tb);
-        redo_tile(p, bn, tm, tn, tb, reinterpret_cast<float*>(smem + Smem::stages));
+        redo_tile<false>(p, bn, tm, tn, tb, reinterpret_cast<float*>(smem + Smem::stages));
     }
 }
 
@@ -577,7 +579,8 @@ bool opt_in_shared_memory() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
-        for (auto kernel : {tc_gemm_f32_kernel<BN>, tc_gemm_f32_kernel<0>, tc_gemm_f32_kernel<BN, true>, tc_gemm_f32_kernel<0, true>})
+        for (auto kernel : {tc_gemm_f32_kernel<BN>, tc_gemm_f32_kernel<0>, tc_gemm_f32_kernel<BN, WIDE>, tc_gemm_f32_kernel<0, WIDE>, tc_gemm_f32_kernel<BN, CLUSTERED>,
+                            tc_gemm_f32_kernel<0, CLUSTERED>})
             if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
@@ -655,7 +658,7 @@ bool launch(const TcProduct& c, void* D, const char* where) {
             cost = std::min(cost, (double)((tiles * slices + grid - 1) / grid * ((p.num_kb + slices - 1) / slices)) * kb + kSplitFixed32 + 0.1 * slices);
         if (form)
             p.cluster = cluster_slices(tiles, (uint64_t)p.num_kb, grid, kb, kClusterFixed32, cost,
-                                       [](int n) { return resident_clusters(reinterpret_cast<const void*>(tc_gemm_f32_kernel<0, true>), THREADS, SMEM_BYTES, n); });
+                                       [](int n) { return resident_clusters(reinterpret_cast<const void*>(tc_gemm_f32_kernel<0, CLUSTERED>), THREADS, SMEM_BYTES, n); });
         if (p.cluster) slices = p.cluster;
     }
     StreamWorkspace partial;
@@ -703,13 +706,15 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.out = static_cast<float*>(slices > 1 && !p.cluster ? partial.ptr : D);
     p.out_ld = (int64_t)(slices > 1 && !p.cluster ? n_pitch : N);
     if (grid > p.num_tiles) grid = p.num_tiles;
-    p.wide = p.chunk_kb == CHUNK_FAST && slices == 1 && p.num_kb >= kWideLeast && g_wide.load(std::memory_order_relaxed) ? 1 : 0;
+    const int form = p.cluster ? CLUSTERED : p.chunk_kb == CHUNK_FAST && slices == 1 && p.num_kb >= kWideLeast && g_wide.load(std::memory_order_relaxed) ? WIDE : PLAIN;
     t_last_form[0] = slices;
     t_last_form[1] = p.cluster;
-    t_last_form[2] = p.wide;
+    t_last_form[2] = form == WIDE;
     t_last_form[3] = p.bn;
     const bool fixed = p.bn == BN && !p.d_plain && p.chunk_kb == CHUNK_FAST;
-    const auto kernel = p.cluster ? (fixed ? tc_gemm_f32_kernel<BN, true> : tc_gemm_f32_kernel<0, true>) : (fixed ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>);
+    const auto kernel = form == CLUSTERED ? (fixed ? tc_gemm_f32_kernel<BN, CLUSTERED> : tc_gemm_f32_kernel<0, CLUSTERED>)
+                        : form == WIDE ? (fixed ? tc_gemm_f32_kernel<BN, WIDE> : tc_gemm_f32_kernel<0, WIDE>)
+                                       : (fixed ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>);
     launch_clusters(kernel, p.cluster ? p.num_tiles : grid, THREADS, SMEM_BYTES, p.cluster, ma, mb, md, p, err, tag);
     check_launch(where);
     if (slices > 1 && !p.cluster) splitk_reduce(2, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
