@@ -409,9 +409,12 @@ constexpr int kColRows = 8;    // threads along the reduced dim
 
 // grid = (ceil(I / (32 * VEC)), splits, min(O, 65535)).  VEC > 1 requires I % VEC == 0 and an
 // aligned base.
-// Eight-byte types keep to the registers of five blocks an SM (maxima of u64 took 54 of them since the wait at the top, four blocks: [48950, 873] 66 us before, 74, 54 so).
+// Maxima of eight-byte integers are held to five blocks an SM (they took 54 registers instead of 44 since the wait at the top, four blocks: [48950, 873] u64 66 us before,
+// 74, 54 so).  0: the compiler's own choice for all others; 1 would let it take every register (bf16 [130, 300000] 9.0 us, 9.8; minima of f32 [811, 2, 13536] 403, 888).
+template <class T, int KIND>
+constexpr int kColBlocks = KIND >= RED_MAX && std::is_integral<T>::value && sizeof(T) == 8 ? 5 : 0;
 template <class T, int KIND, int VEC>
-__global__ void __launch_bounds__(kColLanes* kColRows, sizeof(T) == 8 ? 5 : 1) reduce_cols_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial, u64 O,
+__global__ void __launch_bounds__(kColLanes* kColRows, VEC > 1 ? kColBlocks<T, KIND> : 0) reduce_cols_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial, u64 O,
                                                                          u64 R, u64 I, u64 seg, u32 splits, u64 factor, u32* counters) {
     after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
