@@ -136,22 +136,23 @@ __device__ __forceinline__ Vec<O, VEC> apply_vec(const F& f, const Vec<T, VEC>& 
 // bf16 1.14 / 1.19, quotient 1.39 / 1.78, f32 difference 1.15 / 1.02; 700 u8 1.38 / 1.68, bf16 1.33 / 1.21; square of 1000 u8 1.50 / 1.30, bf16 1.73 / 1.04.
 template <int VEC>
 constexpr uint64_t kEwTailElements = kEwThreads * (VEC >= 16 ? 3 : VEC == 8 ? 2 : 1);
-// Elements of a block: four vectors a thread, all loads in flight together, or one while that leaves an SM two blocks at most: those blocks, and the last of
-// the others, take their vectors one after the other in a loop of its own, which costs the main one no registers (with all of an incomplete block's loads
-// in flight it had 142 instead of 42, product of i16, 74 instead of 32, comparison of bf16, and fewer blocks an SM for it).  One / four vectors a
-// thread, us: difference of 2048 vectors f32 1.3 / 1.5, u8 1.7 / 3.7; 60000 1.5 / 1.9, 2.8 / 3.8; 150000 1.84 / 1.79, 5.1 / 3.8; square root of 8191 f32 1.3 / 2.3, 6.4 by elements.
+// `full` blocks of four vectors a thread, all loads in flight together, then blocks of one vector a thread: all of a tensor that would leave an SM half a
+// block the other way, the last, incomplete block of a larger one.  Each is one trip to memory; with its four vectors in a loop an incomplete block was
+// the length of the launch (3.4 MB f32 3.3 us, 3.9 so), with all of them in flight it cost the main path registers (product of i16 42, 142 so: 40 MB 21 us, 33).
+// One / four vectors a thread, us: difference of 2048 vectors f32 1.3 / 1.5, u8 1.7 / 3.7; 60000 1.5 / 1.9, 2.8 / 3.8; 150000 1.84 / 1.79, 5.1 / 3.8; square root of 8191 f32
+// 1.3 / 2.3, 6.4 by elements.
 template <int VEC>
-inline uint32_t ew_flat_chunk(uint64_t n) {
-    return (uint32_t)(kEwThreads * VEC) * (n / VEC <= 2 * (uint64_t)kEwThreads * sm_count() ? 1 : kEwUnroll);
+inline uint32_t ew_flat_full_blocks(uint64_t n) {
+    return n / VEC <= 2 * (uint64_t)kEwThreads * sm_count() ? 0 : (uint32_t)(n / ((uint64_t)kEwThreads * VEC * kEwUnroll));
 }
 
-// sa / sb: 1 = contiguous, 0 = broadcast scalar; chunk: ew_flat_chunk
+// sa / sb: 1 = contiguous, 0 = broadcast scalar
 template <class F, class T, class O, int NIN, int VEC>
-__global__ void __launch_bounds__(kEwThreads) ew_flat_kernel(F f, const T* a, const T* b, O* out, uint64_t n, int sa, int sb, uint32_t chunk) {
+__global__ void __launch_bounds__(kEwThreads) ew_flat_kernel(F f, const T* a, const T* b, O* out, uint64_t n, int sa, int sb, uint32_t full) {
     after_previous_kernel();
-    constexpr uint32_t kChunk = (uint32_t)kEwThreads * VEC * kEwUnroll;
-    const uint64_t base = (uint64_t)blockIdx.x * chunk;
-    if (chunk == kChunk && base + kChunk <= n) {
+    constexpr uint64_t kChunk = (uint64_t)kEwThreads * VEC * kEwUnroll, kPiece = (uint64_t)kEwThreads * VEC;
+    if (blockIdx.x < full) {
+        const uint64_t base = (uint64_t)blockIdx.x * kChunk;
         Vec<T, VEC> va[kEwUnroll], vb[kEwUnroll];
 #pragma unroll
         for (int u = 0; u < kEwUnroll; u++) {
@@ -166,11 +167,11 @@ __global__ void __launch_bounds__(kEwThreads) ew_flat_kernel(F f, const T* a, co
         }
         return;
     }
-    const uint64_t end = base + chunk < n ? base + chunk : n;
+    const uint64_t base = full * kChunk + (blockIdx.x - full) * kPiece, end = base + kPiece < n ? base + kPiece : n;
     uint64_t rest = base;
     if (end - base > kEwTailElements<VEC>) {
-#pragma unroll 1
-        for (uint64_t i = base + (uint64_t)threadIdx.x * VEC; i + VEC <= end; i += kEwThreads * VEC) {
+        const uint64_t i = base + (uint64_t)threadIdx.x * VEC;
+        if (i + VEC <= end) {
             const Vec<T, VEC> va = sa ? ld_vec<T, VEC>(a + i) : splat<T, VEC>(a[0]);
             Vec<T, VEC> vb;
             if constexpr (NIN == 2) vb = sb ? ld_vec<T, VEC>(b + i) : splat<T, VEC>(b[0]);
@@ -1134,8 +1135,9 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                     break;
                 }
             }
-            const uint32_t block = ew_flat_chunk<VEC>(pl.n);
-            launch_kernel(ew_flat_kernel<F, T, O, NIN, VEC>, (uint32_t)((pl.n + block - 1) / block), kEwThreads, 0, s, f, a, b, out, pl.n, (int)pl.st[1][0], NIN == 2 ? (int)pl.st[2][0] : 0, block);
+            const uint32_t full = ew_flat_full_blocks<VEC>(pl.n);
+            const uint64_t piece = (uint64_t)kEwThreads * VEC, pieces = (pl.n - full * chunk + piece - 1) / piece;
+            launch_kernel(ew_flat_kernel<F, T, O, NIN, VEC>, full + (uint32_t)pieces, kEwThreads, 0, s, f, a, b, out, pl.n, (int)pl.st[1][0], NIN == 2 ? (int)pl.st[2][0] : 0, full);
             break;
         }
         case EW_FLAT_SHIFT: {
