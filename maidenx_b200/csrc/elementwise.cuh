@@ -924,8 +924,8 @@ __global__ void __launch_bounds__(kEwThreads) ew_dense_kernel(F f, const T* a, c
 // operand whose rows are no whole vectors, the commonest call of the kernel above.  What bounds that one there is its instructions (loops over the
 // dims, every element's own choice): here the place of a vector costs two divisions by multiplication, the row behind comes from
 // the one before it without another, both values a vector can see are loaded whether or not its rows change inside it, and a thread has
-// up to four vectors' loads in flight (ew_chan_units).  [256, 512, 7, 7] bf16 with a per-channel operand 5.3 us (10.2 by the kernel above), [8191, 1023] f32 with a per-row
-// one 8.5 (11.6).
+// up to two vectors' loads in flight (ew_chan_units).  [256, 512, 7, 7] bf16 with a per-channel operand 4.3 us (8.1 by the kernel above), [8191, 1023] f32 with a per-row
+// one 7.8 (10.7).
 struct FastDiv31 {  // floor(n / d) for n < 2^31 and d >= 2: with 2^s < d <= 2^(s+1) and m = ceil(2^(32+s) / d), n (m d - 2^(32+s)) < 2^(32+s)
     uint32_t d, m, s;
     void init(uint32_t div) {
@@ -949,26 +949,12 @@ struct EwRepeatParams {
     int repeated[3];  // [1], [2]: the input is one row for all rows, else it has the output's layout
     int units;
 };
-constexpr int kEwChanUnroll = 4;
-// Vectors a thread of the two kernels below; 0: the dense kernel.  One while that leaves an SM two blocks at most, two up to three blocks an SM (94 registers: the
-// next would wait), then four.  Divisions are bound by their instructions and keep two longer: f32 to eight blocks an SM, 16-bit floats always; integer
-// ones have nothing to hide behind the loads and leave.  Dense / one / two / four, us, a row's or a channel's operand beside rows of 1023:
-//   f32 difference    33000 vectors 1.84 1.33 1.54 1.91    220000 2.33 2.13 1.94 2.33    1200000 5.92 5.99 5.02 4.90
-//   f32 quotient      33000 2.35 1.83 2.08 2.87            300000 2.96 3.48 2.74 3.17    2400000 17.2 20.9 16.7 14.6
-//   bf16 quotient     33000 4.91 2.83 4.60 8.10            300000 7.68 7.37 6.85 9.13    2400000 47.2 47.1 42.9 43.5
-//   bf16 comparison   33000 2.34 1.62 1.94 2.85            300000 3.15 3.68 3.47 3.38    1200000 9.93 11.1 9.61 8.81
-//   i16 quotient      33000 4.50 2.66 4.09 7.27            300000 6.53 7.78 8.39 8.38    2400000 42.6 51.7 47.2 48.4
-template <class F, class T>
-inline int ew_chan_units(uint64_t vecs) {
-    const uint64_t sms = sm_count();
-    if (vecs <= 2 * kEwThreads * sms) return 1;
-    if (vecs <= 6 * kEwThreads * sms) return 2;
-    if constexpr (F::kDivides) {
-        if (is_int_v<T>) return 0;
-        if (is_half_v<T> || vecs <= 16 * kEwThreads * sms) return 2;
-    }
-    return 4;
-}
+// Two vectors a thread at most, one while that leaves an SM four blocks at most.  Compiled for four the kernels have 46 (f32) to 94 registers (16 bits) instead of 30 to
+// 48: fewer blocks an SM, and below 150000 vectors most SMs had none.  Dense kernel / one / two / four, geometric mean and worst over layouts and rows of 92 and 1023,
+// of the dense kernel's time: 33000 vectors f32 difference 0.81 0.84 0.93, worst 1.04; bf16 quotient 0.58 0.87 1.44, worst 1.60; i16 comparison 0.60 0.71 1.05, worst
+// 1.19; 220000 bf16 quotient 0.84 0.87 1.26; 2400000 f32 difference 0.89 0.85 0.86, bf16 quotient 0.77 0.76 0.84, comparison 0.69 0.62 0.77.  One or two: worst 1.03.
+constexpr int kEwChanUnroll = 2;
+inline int ew_chan_units(uint64_t vecs) { return vecs <= 4 * (uint64_t)kEwThreads * sm_count() ? 1 : kEwChanUnroll; }
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, const T* b, O* out, EwChanParams P) {
     after_previous_kernel();
@@ -1021,8 +1007,8 @@ __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, co
 }
 
 // Two inputs of ragged rows, each the output's own layout or the same row for all of them (a bias, a norm's weights): one division by multiplication a
-// vector, the repeated row from L1 by elements, up to four vectors a thread.  [8191, 1023] f32 10.3 us (11.8 by the dense kernel), [4099, 1543] bf16 7.0 (8.1).  An
-// instantiation of the kernel above for it would have the constants' registers too (94 instead of 79 in 16 bits).
+// vector, the repeated row from L1 by elements, up to two vectors a thread.  [8191, 1023] f32 9.5 us (10.8 by the dense kernel), [4099, 1543] bf16 5.9 (7.0).  An
+// instantiation of the kernel above for it would have the constants' registers too.
 template <class F, class T, class O, int VEC>
 __global__ void __launch_bounds__(kEwThreads) ew_repeat_kernel(F f, const T* a, const T* b, O* out, EwRepeatParams P) {
     after_previous_kernel();
@@ -1217,13 +1203,13 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                 if constexpr (NIN == 2 && VEC <= 8) {  // 16 elements a vector would take 145 registers
                     EwChanParams C;
                     EwRepeatParams Q;
-                    C.units = Q.units = ew_chan_units<F, T>(vecs);
-                    const uint32_t blocks = C.units ? (uint32_t)((vecs + kEwThreads * C.units - 1) / (kEwThreads * C.units)) : 0;
-                    if (blocks && ew_fill_chan_params(D, VEC, C)) {
+                    C.units = Q.units = ew_chan_units(vecs);
+                    const uint32_t blocks = (uint32_t)((vecs + kEwThreads * C.units - 1) / (kEwThreads * C.units));
+                    if (ew_fill_chan_params(D, VEC, C)) {
                         launch_kernel(ew_chan_kernel<F, T, O, VEC>, blocks, kEwThreads, 0, s, f, a, b, out, C);
                         break;
                     }
-                    if (blocks && ew_fill_repeat_params(D, VEC, Q)) {
+                    if (ew_fill_repeat_params(D, VEC, Q)) {
                         launch_kernel(ew_repeat_kernel<F, T, O, VEC>, blocks, kEwThreads, 0, s, f, a, b, out, Q);
                         break;
                     }

@@ -592,7 +592,6 @@ __device__ __forceinline__ uint32_t pack2_rn(f32 lo, f32 hi) {
 // Adapters giving every family the call shape the kernels use.
 template <class Op, class T, class O>
 struct Binary {  // out = Op(a, b)
-    static constexpr bool kDivides = std::is_same<Op, OpDiv>::value;
     static constexpr bool kCore = HalfCore<Op>::ok && is_half_v<T> && std::is_same<O, T>::value;
     static constexpr bool kNative = HalfNative<Op>::ok && is_half_v<T> && std::is_same<O, T>::value;
     // division of 16-bit floats: fast quotient per element, flagged elements redone exactly
