@@ -136,14 +136,15 @@ __device__ __forceinline__ Vec<O, VEC> apply_vec(const F& f, const Vec<T, VEC>& 
 // bf16 1.14 / 1.19, quotient 1.39 / 1.78, f32 difference 1.15 / 1.02; 700 u8 1.38 / 1.68, bf16 1.33 / 1.21; square of 1000 u8 1.50 / 1.30, bf16 1.73 / 1.04.
 template <int VEC>
 constexpr uint64_t kEwTailElements = kEwThreads * (VEC >= 16 ? 3 : VEC == 8 ? 2 : 1);
-// `full` blocks of four vectors a thread, all loads in flight together, then blocks of one vector a thread: all of a tensor that would leave an SM half a
-// block the other way, the last, incomplete block of a larger one.  Each is one trip to memory; with its four vectors in a loop an incomplete block was
+// `full` blocks of four vectors a thread, all loads in flight together, then blocks of one vector a thread: all of a tensor that would leave an SM one
+// block the other way (half of one, with 16 elements a vector), the last, incomplete block of a larger one.  Each is one trip to memory; with its four vectors in a loop an incomplete block was
 // the length of the launch (3.4 MB f32 3.3 us, 3.9 so), with all of them in flight it cost the main path registers (product of i16 42, 142 so: 40 MB 21 us, 33).
-// One / four vectors a thread, us: difference of 2048 vectors f32 1.3 / 1.5, u8 1.7 / 3.7; 60000 1.5 / 1.9, 2.8 / 3.8; 150000 1.84 / 1.79, 5.1 / 3.8; square root of 8191 f32
+// One / four vectors a thread, us: difference of 2048 vectors f32 1.3 / 1.5, u8 1.7 / 3.7; 60000 1.5 / 1.9, 2.8 / 3.8; 100000 f32 1.74 / 1.94, bf16 1.73 / 2.04, u8 3.96 /
+// 3.77; 150000 1.84 / 1.79, 1.82 / 2.05, 5.1 / 3.8; square root of 8191 f32
 // 1.3 / 2.3, 6.4 by elements.
 template <int VEC>
 inline uint32_t ew_flat_full_blocks(uint64_t n) {
-    return n / VEC <= 2 * (uint64_t)kEwThreads * sm_count() ? 0 : (uint32_t)(n / ((uint64_t)kEwThreads * VEC * kEwUnroll));
+    return n / VEC <= (VEC > 8 ? 2 : 4) * (uint64_t)kEwThreads * sm_count() ? 0 : (uint32_t)(n / ((uint64_t)kEwThreads * VEC * kEwUnroll));
 }
 
 // sa / sb: 1 = contiguous, 0 = broadcast scalar
