@@ -430,6 +430,44 @@ def test_short_last_block_by_elements(oracle, cuda, dt):
         H.assert_same("add_scalar", dt, got, ref, what=f"n={n}")
 
 
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F64, D.U8], ids=lambda d: d.name)
+def test_whole_blocks_and_what_is_left_of_flat_operands(oracle, cuda, dt):
+    """Lengths around the line from which blocks have four vectors a thread, and what they leave for blocks of one: nothing, an element, parts of a block, one to four
+    blocks."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(zlib.crc32(dt.name.encode()) + 3)
+    vec = 16 // dt.size
+    piece, block = 256 * vec, 1024 * vec
+    line = (2 if vec > 8 else 4) * sms * piece
+    whole = -(-(line + vec) // block) * block
+    a, b = (H.random_store(rng, dt, whole + 2 * block, lo=1, hi=50) if dt.kind != "float" else H.random_store(rng, dt, whole + 2 * block, lo=0.5, hi=2.0) for _ in range(2))
+    for n in (line + vec - 1, line + vec, whole, whole + 1, whole + piece - 1, whole + piece + 1, whole + 2 * piece + 300, whole + block - 1, whole + block + 769):
+        for rs in (1, 0):
+            args = ("sub", dt, [n], [1], [rs], 0, 0, a[:n], b[:n])
+            H.assert_same("sub", dt, H.run_binary(cuda, *args), H.run_binary(oracle, *args), what=f"n={n} rhs stride {rs}")
+        got, ref = (H.run_unary(be, "add_scalar", dt, [n], [1], 0, a[:n], scalar=3) for be in (cuda, oracle))
+        H.assert_same("add_scalar", dt, got, ref, what=f"n={n}")
+
+
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F64, D.I16], ids=lambda d: d.name)
+def test_constant_and_repeated_operands_by_one_and_two_vectors_a_thread(oracle, cuda, dt):
+    """Both sides of the line between one vector a thread and two, tensors that end inside a vector and inside a block."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    vec = 16 // dt.size
+    rng = np.random.default_rng(dt.size + 40)
+    line = 4 * sms * 256 * vec
+    for q in (vec + 1, 197):
+        for r in (line // q, line // q + 2, (line + 700 * vec) // q + 1):
+            for name, dims, dense, const in (("row", [r, q], [q, 1], [1, 0]), ("repeated", [r, q], [q, 1], [0, 1]), ("channel", [r // 3 + 1, 3, q], [3 * q, q, 1], [0, 1, 0])):
+                size = 1 + sum((d - 1) * s for d, s in zip(dims, const))
+                full, part = (H.random_store(rng, dt, n, lo=1, hi=50) if dt.kind != "float" else H.random_store(rng, dt, n, lo=0.5, hi=2.0) for n in (H.numel(dims), size))
+                for op, sa, sb, x, y in (("div", dense, const, full, part), ("sub", const, dense, part, full)):
+                    args = (op, dt, dims, sa, sb, 0, 0, x, y)
+                    H.assert_same(op, dt, H.run_binary(cuda, *args), H.run_binary(oracle, *args), what=f"{name} {op} {dims}")
+
+
 @pytest.mark.parametrize("dt", [D.BF16, D.F16, D.I16, D.U16], ids=lambda d: d.name)
 def test_two_byte_transposed_tiles(oracle, cuda, dt):
     """2-byte types with vector-aligned transposed operands run on the tensor-copy tile kernel (64 x 64 boxes, ldmatrix
