@@ -182,19 +182,18 @@ __device__ __forceinline__ Acc load_published(const Acc* p) {
 }
 
 // The fold of a row's `splits` published parts in split order, eight of them in flight: one thread folds an output while the
-// rest of the launch is over, so each trip to L2 counts in full.  One by one where eight take registers from the main loop: f64 (means 34, 52 with eight),
-// and in the kernel of columns, which has its own (bf16 52, 80; 130 x 300000 8.8 us, 10.1; 100001 x 16 f32 32.0, 37.2; 2047 x 20000 f64 49.7, 54.5; only 2047 x
-// 20000 bf16 10.2, 9.6).
-template <class TR>
-__device__ __forceinline__ typename TR::Acc fold_published(const typename TR::Acc* p, u32 splits) {
+// rest of the launch is over, so each trip to L2 counts in full.  One by one (UN = 1) where eight take registers from the main loop: f64 (means of rows 34, 52 with
+// eight), and columns (100001 x 16 f32 32.0 us, 37.2; 2047 x 20000 f64 49.7, 54.5) but for vectors of 16-bit floats, whose kernel is held to four blocks an
+// SM (bf16 52 registers, 80 without the bound: 130 x 300000 8.8 us, 10.1; with it 2.5 % faster than one by one over 25 shapes, at most 3 % slower).
+template <class TR, u32 UN>
+__device__ __forceinline__ typename TR::Acc fold_published(const typename TR::Acc* p, u64 stride, u32 splits) {
     typedef typename TR::Acc Acc;
-    constexpr u32 UN = std::is_same<Acc, f64>::value ? 1 : 8;
     Acc acc = TR::init();
     for (u32 s = 0; s < splits; s += UN) {
         Acc v[UN];
 #pragma unroll
         for (u32 q = 0; q < UN; q++)
-            if (s + q < splits) v[q] = load_published(p + s + q);
+            if (s + q < splits) v[q] = load_published(p + (s + q) * stride);
 #pragma unroll
         for (u32 q = 0; q < UN; q++)
             if (s + q < splits) acc = TR::combine(acc, v[q]);
@@ -229,7 +228,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_rows_block_kernel(const T*
         acc = block_reduce<TR, kRedThreads>(acc);
         if (threadIdx.x == 0) out[row] = TR::finalize(acc, factor);
     } else if (threadIdx.x == 0) {  // same order as reduce_partials_kernel
-        out[row] = TR::finalize(fold_published<TR>(mine, splits), factor);
+        out[row] = TR::finalize(fold_published<TR, std::is_same<Acc, f64>::value ? 1 : 8>(mine, 1, splits), factor);
     }
 }
 
@@ -409,10 +408,10 @@ constexpr int kColRows = 8;    // threads along the reduced dim
 
 // grid = (ceil(I / (32 * VEC)), splits, min(O, 65535)).  VEC > 1 requires I % VEC == 0 and an
 // aligned base.
-// Maxima of eight-byte integers are held to five blocks an SM (they took 54 registers instead of 44 since the wait at the top, four blocks: [48950, 873] u64 66 us before,
-// 74, 54 so).  0: the compiler's own choice for all others; 1 would let it take every register (bf16 [130, 300000] 9.0 us, 9.8; minima of f32 [811, 2, 13536] 403, 888).
+// Vectors of 16-bit floats are held to four blocks an SM (see fold_published), maxima of eight-byte integers to five (they took 54 registers instead of 44 since
+// the wait at the top, four blocks: [48950, 873] u64 66 us before, 74, 54 so).  0: the compiler's own choice for all others; 1 would let it take every register (bf16 [130, 300000] 9.0 us, 9.8; minima of f32 [811, 2, 13536] 403, 888).
 template <class T, int KIND>
-constexpr int kColBlocks = KIND >= RED_MAX && std::is_integral<T>::value && sizeof(T) == 8 ? 5 : 0;
+constexpr int kColBlocks = is_half_v<T> ? 4 : KIND >= RED_MAX && std::is_integral<T>::value && sizeof(T) == 8 ? 5 : 0;
 template <class T, int KIND, int VEC>
 __global__ void __launch_bounds__(kColLanes* kColRows, VEC > 1 ? kColBlocks<T, KIND> : 0) reduce_cols_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial, u64 O,
                                                                          u64 R, u64 I, u64 seg, u32 splits, u64 factor, u32* counters) {
@@ -473,8 +472,11 @@ __global__ void __launch_bounds__(kColLanes* kColRows, VEC > 1 ? kColBlocks<T, K
                 for (int c = threadIdx.x; c < kColLanes * VEC; c += kColLanes * kColRows) {
                     u64 gc = (u64)blockIdx.x * kColLanes * VEC + c;
                     if (gc < I) {
+                        const Acc* parts = partial + o * I + gc;
                         Acc v = TR::init();
-                        for (u32 s2 = 0; s2 < splits; s2++) v = TR::combine(v, load_published(partial + ((u64)s2 * O + o) * I + gc));
+                        if constexpr (is_half_v<T> && VEC > 1) v = fold_published<TR, 8>(parts, O * I, splits);
+                        else
+                            for (u32 s2 = 0; s2 < splits; s2++) v = TR::combine(v, load_published(partial + ((u64)s2 * O + o) * I + gc));
                         out[o * I + gc] = TR::finalize(v, factor);
                     }
                 }
