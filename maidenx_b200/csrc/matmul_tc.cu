@@ -255,7 +255,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * MAX_STAGES + 2 + a); };
     volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(smem + SmemLayout::bars + 8 * (2 * MAX_STAGES + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? STAGES : p.stages, stage_bytes = BN_T ? A_STAGE_BYTES + BN_T * BK * 2 : p.stage_bytes;
 
     if (threadIdx.x == 0) {
@@ -269,6 +269,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         fence_barrier_init();
     }
+    if (warp == 2 && elect_one()) {
+        prefetch_map(&map_a);
+        prefetch_map(&map_b);
+        if (MODE != TC_PLAIN) prefetch_map(&map_d);
+    }
     if (warp == 1) {  // the MMA warp owns the TMEM allocation
         tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_base_slot)), TMEM_COLS);
         tmem_relinquish();
@@ -281,7 +286,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -320,7 +325,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(p.is_bf16 != 0, p.a_mn != 0, p.b_mn != 0, bn);
             // per-operand descriptor geometry: (leading, stride) byte offsets and the K step in 16-byte units
             const uint32_t a_lbo = p.a_mn ? MN_CHUNK_BYTES : 16, b_lbo = p.b_mn ? MN_CHUNK_BYTES : 16;

@@ -229,7 +229,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     auto tempty_bar = [&](int a) { return bar_base + 8u * (3 * MAX_STAGES + 2 + a); };
     volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(smem + Smem::bars + 8 * (3 * MAX_STAGES + 4));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const int chunk_kb = BN_T ? CHUNK_FAST : p.chunk_kb;
     const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? STAGES : p.stages, raw_bytes = BN_T ? A_TILE + BN_T * BK * 4 : p.raw_bytes;
 
@@ -250,6 +250,10 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
         fence_barrier_init();
     }
+    if (warp == 2 && elect_one()) {
+        prefetch_map(&map_a);
+        prefetch_map(&map_b);
+    }
     if (warp == 1) {
         tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_base_slot)), TMEM_COLS);
         tmem_relinquish();
@@ -262,7 +266,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -304,7 +308,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, bn), idesc_wide = make_idesc_tf32(p.a_mn != 0, p.b_mn != 0, 2 * bn);
             // K-major: 8 floats further along the 128-byte row; MN-major: the next group of eight K-rows
             const uint64_t a_kstep = p.a_mn ? (1024 >> 4) : (32 >> 4), b_kstep = p.b_mn ? (1024 >> 4) : (32 >> 4);

@@ -16,6 +16,22 @@ constexpr long long TC_WAIT_BUDGET_CYCLES = 4000000000ll;  // about two seconds
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One thread of a whole warp, the same one each time.  What a role's only thread issues stands behind this and not behind a comparison of the
+// lane: the compiler then knows that one thread runs it and keeps what tcgen05 and the copy engine take in uniform registers.  Chains of
+// tcgen05.mma M128 K16, cycles each, behind `lane == 0` / behind this: N = 64 65 / 48, 128 65 / 64, 256 128 / 128, and 135 and more behind `lane == 0`
+// where the accumulator's address is not a constant.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(one));
+    return one != 0;
+}
+// The warp's number in its block, in a form that the compiler knows to be the same for all its threads.
+__device__ __forceinline__ int warp_number() { return __shfl_sync(0xFFFFFFFFu, (int)threadIdx.x >> 5, 0); }
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
@@ -94,6 +110,8 @@ __device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity,
     }
 }
 
+// Brings a tensor map into the copy engine's cache.  The map is a parameter of the launch: nothing of it waits for the kernel before.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
                  "l"(map), "r"(x), "r"(y), "r"(bar)
