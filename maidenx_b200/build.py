@@ -14,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -22,6 +23,7 @@ CSRC = PKG_DIR / "csrc"
 INCLUDE = PKG_DIR.parent / "include"
 BUILD = CSRC / "build"
 LIB_PATH = PKG_DIR / "libmaidenx_cuda.so"
+DISPATCH_PATH = PKG_DIR / "_dispatch.so"  # extension module: device.dispatch as one native call
 
 # suffix -> class id (see abi_common.cuh)
 DTYPES = {
@@ -128,7 +130,18 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False, p
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_dispatch(force)
     return LIB_PATH
+
+
+def build_dispatch(force: bool = False) -> Path:
+    src = CSRC / "pydispatch.cpp"
+    if force or not DISPATCH_PATH.exists() or DISPATCH_PATH.stat().st_mtime < max(src.stat().st_mtime, Path(__file__).stat().st_mtime):
+        cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(DISPATCH_PATH)]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"building {DISPATCH_PATH.name} failed:\n{r.stdout}\n{r.stderr}")
+    return DISPATCH_PATH
 
 
 def main(argv=None):

@@ -91,13 +91,11 @@ def _raise_last_error(op: str, dtype_name: str):
 _packers = {}  # words of a metadata block -> packing function
 
 
-def dispatch(op: str, dtype_name: str, metadata, *args, device: int = 0, metadata_on_host: bool = False, check: bool = True):
-    """Call cuda_<op>_<dtype> the way maidenx_core does.  `args` is the op's argument list
-    with the string "META" standing where the metadata pointer goes."""
+def _dispatch_general(op: str, dtype_name: str, metadata, *args, device: int = 0, metadata_on_host: bool = False, check: bool = True):
+    """`dispatch` with any arguments that ctypes and numpy take; the usual call is csrc/pydispatch.cpp's."""
     lib = _lib.load()
     if not metadata_on_host and type(metadata) is list and metadata:
-        # The usual call.  Host time per call is what small workloads are made of (the README example is 17 such calls):
-        # packing with struct and two native calls around the op, whose metadata block is read where it is written.
+        # packing with struct and two native calls around the op, whose metadata block is read where it is written
         pack = _packers.get(len(metadata))
         if pack is None:
             pack = _packers[len(metadata)] = struct.Struct(f"{len(metadata)}Q").pack
@@ -136,6 +134,30 @@ def dispatch(op: str, dtype_name: str, metadata, *args, device: int = 0, metadat
         mbuf.free()
     if check and lib.mx_last_error():
         _raise_last_error(op, dtype_name)
+
+
+def _register(op: str, dtype_name: str):
+    """Makes an entry point known to the native dispatch; raises where there is none."""
+    lib = _lib.load()
+    fn = _lib.op(op, dtype_name)
+    address = lambda f: ctypes.cast(f, ctypes.c_void_p).value  # noqa: E731
+    _native.bind(address(lib.mx_dispatch_begin), address(lib.mx_dispatch_end))
+    types = "".join("P" if t is ctypes.c_void_p else "S" if t is ctypes.c_size_t else t._type_ for t in fn.argtypes)
+    # the first pointer is the metadata block, by-value u64 scalars (the same C type as sizes) stand where the family says
+    family, _ = _lib._ops.family[(op, dtype_name)]
+    at = {"unary_const": 4, "unary_const_bool": 4, "pad_const": 6}.get(family)
+    if at is not None:
+        types = types[:at] + fn.argtypes[at]._type_ + types[at + 1:]
+    _native.register(op, dtype_name, address(fn), types, types.index("P"))
+
+
+try:
+    from . import _dispatch as _native
+except ImportError:  # not built: the interpreted form does the same
+    dispatch = _dispatch_general
+else:
+    _native.setup(_dispatch_general, _register, _check, _raise_last_error)
+    dispatch = _native.dispatch
 
 
 def synchronize():
