@@ -36,6 +36,9 @@ int mx_debug_matmul_forward_path_f32(size_t num_els, const size_t* host_metadata
 void mx_debug_set_gemm_group_m(int rows);
 /* Pairs of CTAs of the two-CTA tensor-core kernel that can be resident at once on the current device (-1: query failed). */
 int mx_debug_gemm_max_resident_pairs(void);
+/* 16-bit operands whose rows are 16-byte multiples but no whole 128-byte lines are copied in lines where that pays: 1 = by the rule (default), 0 = never, 2 =
+ * always. */
+void mx_debug_set_gemm_realign(int mode);
 /* Short reductions (K <= 256, one batch, many row tiles) keep the B panel of a column tile in shared memory and stream
  * only A.  set: 1 = on (default), 0 = always the general schedule.  The query returns the CTAs per column tile a launch
  * with these tile counts takes (0 = general schedule). */

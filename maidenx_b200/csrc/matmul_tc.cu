@@ -923,36 +923,49 @@ void splitk_reduce(int dtype, const float* partial, int slices, uint64_t rows, u
 // Rows of `cols` elements, dense and starting anywhere, copied to rows of `pitch` elements (a multiple of 128 bytes): one
 // 16-byte vector of a destination row per thread and step, assembled from the one or two aligned 16-byte words of the
 // source it straddles.  The words read all hold at least one element of the vector, so nothing outside the aligned words
-// of the source's own elements is touched.  Bound by HBM (or L2): reads and writes the operand once.
+// of the source's own elements is touched.  Bound by HBM (or L2): reads and writes the operand once.  Both operands of a product in one launch.
 template <class W>
-__global__ void __launch_bounds__(256) repack_rows_kernel(const W* in, W* out, uint32_t vecs, FastDiv per_row, uint32_t cols, uint32_t pitch) {
-    after_previous_kernel();
+struct RowCopy {
+    const W* in;
+    W* out;
+    uint32_t vecs;  // 0: nothing to copy
+    FastDiv per_row;
+    uint32_t cols, pitch;
+};
+template <class W>
+__device__ __forceinline__ void repack_vector(const RowCopy<W>& p, uint32_t v) {
     constexpr uint32_t VEC = 16 / sizeof(W);
-    const uint32_t stride = gridDim.x * 256;
-    for (uint32_t v = blockIdx.x * 256 + threadIdx.x; v < vecs; v += stride) {
-        uint32_t row, c;
-        per_row.divmod(v, row, c);
-        c *= VEC;
-        const uint32_t need = min(VEC, cols - c) * (uint32_t)sizeof(W);
-        const uintptr_t src = reinterpret_cast<uintptr_t>(in + (size_t)row * cols + c);
-        const uint32_t sh = (uint32_t)(src & 15);
-        const uint4* words = reinterpret_cast<const uint4*>(src - sh);
-        const uint4 lo = words[0];
-        uint4 hi = make_uint4(0, 0, 0, 0);
-        if (sh + need > 16) hi = words[1];
-        uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-        uint4 r;
-        const uint32_t bits = (sh & 3) * 8;
+    uint32_t row, c;
+    p.per_row.divmod(v, row, c);
+    c *= VEC;
+    const uint32_t need = min(VEC, p.cols - c) * (uint32_t)sizeof(W);
+    const uintptr_t src = reinterpret_cast<uintptr_t>(p.in + (size_t)row * p.cols + c);
+    const uint32_t sh = (uint32_t)(src & 15);
+    const uint4* words = reinterpret_cast<const uint4*>(src - sh);
+    const uint4 lo = words[0];
+    uint4 hi = make_uint4(0, 0, 0, 0);
+    if (sh + need > 16) hi = words[1];
+    uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    uint4 r;
+    const uint32_t bits = (sh & 3) * 8;
 #pragma unroll
-        for (int k = 0; k < 2; k++)  // word-wise shift by sh / 4 in two steps with compile-time indices
+    for (int k = 0; k < 2; k++)  // word-wise shift by sh / 4 in two steps with compile-time indices
 #pragma unroll
-            for (int i = 0; i < 8; i++)
-                if ((sh >> 2) & (2 >> k)) w[i] = i + (2 >> k) < 8 ? w[i + (2 >> k)] : 0;
-        r.x = __funnelshift_r(w[0], w[1], bits);
-        r.y = __funnelshift_r(w[1], w[2], bits);
-        r.z = __funnelshift_r(w[2], w[3], bits);
-        r.w = __funnelshift_r(w[3], w[4], bits);
-        *reinterpret_cast<uint4*>(out + (size_t)row * pitch + c) = r;
+        for (int i = 0; i < 8; i++)
+            if ((sh >> 2) & (2 >> k)) w[i] = i + (2 >> k) < 8 ? w[i + (2 >> k)] : 0;
+    r.x = __funnelshift_r(w[0], w[1], bits);
+    r.y = __funnelshift_r(w[1], w[2], bits);
+    r.z = __funnelshift_r(w[2], w[3], bits);
+    r.w = __funnelshift_r(w[3], w[4], bits);
+    *reinterpret_cast<uint4*>(p.out + (size_t)row * p.pitch + c) = r;
+}
+template <class W>
+__global__ void __launch_bounds__(256) repack_rows_kernel(RowCopy<W> a, RowCopy<W> b) {
+    after_previous_kernel();
+    const uint32_t stride = gridDim.x * 256, all = a.vecs + b.vecs;
+    for (uint32_t v = blockIdx.x * 256 + threadIdx.x; v < all; v += stride) {
+        if (v < a.vecs) repack_vector(a, v);
+        else repack_vector(b, v - a.vecs);
     }
 }
 
@@ -964,38 +977,67 @@ uint64_t copy_pitch(size_t es, uint64_t rows, uint64_t cols) {
     return (cols + q - 1) / q * q;
 }
 
-static bool repack_rows(size_t es, const void* in, void* out, uint64_t rows, uint64_t cols, uint64_t pitch) {
-    const uint64_t per_row = (cols * es + 15) / 16, vecs = rows * per_row;  // the padding itself is never read
-    uint64_t blocks = (vecs + 255) / 256;
+// A 16-bit operand whose rows lie 16-byte multiples apart, but no whole 128-byte lines: each row of a tensor copy's box reads parts of two lines.  What that costs a
+// product is counted in us a KB of the box and k-block (bf16 4096 x 1536 x 1024 15.0 us; x 1000, 16 bytes off, 24.4, x 1008 18.3, x 992 16.6), on as many
+// k-blocks as a CTA has (of long reductions cut into slices at least a quarter); a copy in lines costs its bytes, read and written, at 5 TB/s, and 1.5 us where
+// no other operand has to be copied.  In place / by the rule, us: 4104^3 209 / 137, 4112^3 135 / 127, 4128^3 both 126, 4096 x 1536 x 1000 24.6 / 19.9, 16384 x 4088 x
+// 520 97 / 79, 8192 x 1000 x 1000 25.0 / 20.4, and both alike 1024 x 1024 x 1000 8.2, 16384 x 200 x 200 10.2.  The products' sums are the same either way.
+std::atomic<int> g_realign{1};  // 0: never, 2: always (tests, A/B timing)
+constexpr uint64_t kRealignMost = 256ull << 20;  // what the workspace pool keeps between calls, halved: beyond it a call would map memory anew
+static double misaligned_us(const TcProduct& c, uint64_t pitch, int box_kb) {
+    const uint64_t off = pitch * 2 % 128;
+    const double us_kb = off == 0 ? 0.0 : off % 32 ? 0.006 : off % 64 ? 0.0025 : 0.00125;
+    const double tiles = (double)c.batch * (double)((c.m + 127) / 128) * (double)((c.n + 255) / 256);
+    return us_kb * box_kb * (double)((c.k + 63) / 64) * std::max(0.25, tiles / sm_count());
+}
+static double copy_us(uint64_t rows, uint64_t cols) { return (double)rows * (double)cols * 4.0 / 5.0e6; }
+
+template <class W>
+static void repack_launch(const RowCopy<W>& a, const RowCopy<W>& b) {
+    uint64_t blocks = ((uint64_t)a.vecs + b.vecs + 255) / 256;
     const uint64_t cap = (uint64_t)sm_count() * 32;
     if (blocks > cap) blocks = cap;
-    const FastDiv div((uint32_t)per_row);
-    if (es == 2)
-        launch_kernel(repack_rows_kernel<uint16_t>, (unsigned)blocks, 256, 0, ctx().stream, static_cast<const uint16_t*>(in), static_cast<uint16_t*>(out), (uint32_t)vecs, div, (uint32_t)cols,
-                                                                                 (uint32_t)pitch);
-    else
-        launch_kernel(repack_rows_kernel<uint32_t>, (unsigned)blocks, 256, 0, ctx().stream, static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), (uint32_t)vecs, div, (uint32_t)cols,
-                                                                                 (uint32_t)pitch);
-    return true;
+    launch_kernel(repack_rows_kernel<W>, (unsigned)blocks, 256, 0, ctx().stream, a, b);
 }
 
 bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* where) {
-    if (!c.a_repack && !c.b_repack) return true;
     const uint64_t a_rows = (c.a_mn ? c.k : c.m) * (c.a_bs ? c.batch : 1), a_cols = c.a_mn ? c.m : c.k, a_pitch = copy_pitch(es, a_rows, a_cols);
     const uint64_t b_rows = (c.b_mn ? c.k : c.n) * (c.b_bs ? c.batch : 1), b_cols = c.b_mn ? c.n : c.k, b_pitch = copy_pitch(es, b_rows, b_cols);
-    const uint64_t a_bytes = c.a_repack ? (a_rows * a_pitch * es + 255) / 256 * 256 : 0, b_bytes = c.b_repack ? b_rows * b_pitch * es : 0;
-    if (a_bytes / 16 > 0x7FFFFFFFull || b_bytes / 16 > 0x7FFFFFFFull) return false;  // the copy counts vectors in 32 bits
-    if (!ws.take(a_bytes + b_bytes)) return false;
-    if (c.a_repack) {
-        repack_rows(es, c.A, ws.ptr, a_rows, a_cols, a_pitch);
-        c.A = static_cast<const char*>(ws.ptr);
+    bool a_copy = c.a_repack, b_copy = c.b_repack;
+    const bool needed = a_copy || b_copy;
+    const int mode = g_realign.load(std::memory_order_relaxed);
+    if (es == 2 && mode) {
+        const bool a_dense = !c.a_bs || c.a_bs == (int64_t)(c.m * c.k), b_dense = !c.b_bs || c.b_bs == (int64_t)(c.k * c.n);
+        const auto fits = [&](uint64_t rows, uint64_t pitch) { return rows * pitch * es <= kRealignMost / 2; };
+        const bool a_may = !a_copy && a_dense && a_pitch != a_cols && fits(a_rows, a_pitch), b_may = !b_copy && b_dense && b_pitch != b_cols && fits(b_rows, b_pitch);
+        const double a_gain = a_may ? std::max(0.0, misaligned_us(c, a_cols, 16) - copy_us(a_rows, a_cols)) : 0.0;
+        const double b_gain = b_may ? std::max(0.0, misaligned_us(c, b_cols, 32) - copy_us(b_rows, b_cols)) : 0.0;
+        const bool pays = mode == 2 || a_gain + b_gain > (needed ? 0.0 : 1.5);
+        a_copy = a_copy || (pays && a_may && (mode == 2 || a_gain > 0.0));
+        b_copy = b_copy || (pays && b_may && (mode == 2 || b_gain > 0.0));
+    }
+    if (!a_copy && !b_copy) return true;
+    const uint64_t a_bytes = a_copy ? (a_rows * a_pitch * es + 255) / 256 * 256 : 0, b_bytes = b_copy ? b_rows * b_pitch * es : 0;
+    if (a_bytes / 16 + b_bytes / 16 > 0x7FFFFFFFull) return !needed;  // the copy counts vectors in 32 bits
+    if (!ws.take(a_bytes + b_bytes)) return !needed;
+    char *const a_dst = static_cast<char*>(ws.ptr), *const b_dst = a_dst + a_bytes;
+    auto launch = [&](auto w) {
+        typedef decltype(w) W;
+        const auto copy = [&](bool yes, const char* in, char* out, uint64_t rows, uint64_t cols, uint64_t pitch) {
+            const uint64_t per_row = (cols * es + 15) / 16;  // the padding itself is never read
+            return RowCopy<W>{reinterpret_cast<const W*>(in), reinterpret_cast<W*>(out), yes ? (uint32_t)(rows * per_row) : 0u, FastDiv((uint32_t)per_row), (uint32_t)cols, (uint32_t)pitch};
+        };
+        repack_launch<W>(copy(a_copy, c.A, a_dst, a_rows, a_cols, a_pitch), copy(b_copy, c.B, b_dst, b_rows, b_cols, b_pitch));
+    };
+    if (es == 2) launch(uint16_t());
+    else launch(uint32_t());
+    if (a_copy) {
+        c.A = a_dst;
         c.a_pitch = a_pitch;
         if (c.a_bs) c.a_bs = (int64_t)((c.a_mn ? c.k : c.m) * a_pitch);
     }
-    if (c.b_repack) {
-        char* dst = static_cast<char*>(ws.ptr) + a_bytes;
-        repack_rows(es, c.B, dst, b_rows, b_cols, b_pitch);
-        c.B = dst;
+    if (b_copy) {
+        c.B = b_dst;
         c.b_pitch = b_pitch;
         if (c.b_bs) c.b_bs = (int64_t)((c.b_mn ? c.k : c.n) * b_pitch);
     }
@@ -1346,6 +1388,7 @@ extern "C" int mx_debug_gemm_max_resident_pairs(void) { return mx::tc2::max_resi
 extern "C" void mx_debug_set_gemm_group_m(int rows) { mx::g_group_m.store(rows > 0 ? rows : 16, std::memory_order_relaxed); }
 // 1 (default): products with a reduction of at most 256 run with the B panel resident in shared memory; 0: general schedule
 extern "C" void mx_debug_set_gemm_keep_b(int on) { mx::g_keep_b.store(on ? 1 : 0, std::memory_order_relaxed); }
+extern "C" void mx_debug_set_gemm_realign(int mode) { mx::tc::g_realign.store(mode, std::memory_order_relaxed); }
 extern "C" int mx_debug_gemm_keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, int ctas) { return mx::keep_b_ctas(tiles_m, tiles_n, num_kb, batch, ctas); }
 extern "C" int mx_debug_gemm_last_schedule(void) { return mx::t_last_schedule; }
 extern "C" int mx_debug_splitk_slices(size_t tiles, size_t k, int block_k, int sms) { return mx::tc::splitk_slices(tiles, k, block_k, sms); }

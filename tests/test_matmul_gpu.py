@@ -356,6 +356,44 @@ def test_short_reductions_with_the_b_panel_resident(oracle, cuda, dt, case):
 
 @pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
 @pytest.mark.parametrize("case", [
+    # batch, M, N, K, majors, whether A is the same for all batches: rows 16, 32 and 64 bytes off a line, on one side and on both, a ragged side that is copied
+    # anyway, slices of a long reduction, and what the rule leaves in place
+    (1, 2056, 1544, 1000, "kk", False), (1, 1000, 1032, 1032, "mm", False), (1, 1536, 1544, 1543, "km", False), (1, 520, 1008, 992, "kk", False), (1, 136, 264, 16392, "mk", False),
+    (5, 520, 776, 328, "km", False), (7, 264, 520, 200, "kk", True)], ids=lambda c: "x".join(map(str, c)))
+def test_operands_off_whole_lines(cuda, dt, case):
+    """Copies in whole lines, always and by the rule, change nothing in the sums: bit for bit what the operands give in place; the sums themselves next to float64 (one rounding of an
+    f32 sum: half a step of the type and the sum's own error)."""
+    from maidenx_b200 import _lib
+    lib = _lib.load()
+    nb, m, n, k, majors, shared = case
+    rng = np.random.default_rng(nb + m + n + k)
+    na = 1 if shared else nb
+    a, b = H.random_store(rng, dt, na * m * k, dist="normal"), H.random_store(rng, dt, nb * k * n, dist="normal")
+    lead = [nb] if nb > 1 else []
+    sa, sb = ([0 if shared else m * k] if lead else []) + ([k, 1] if majors[0] == "k" else [1, m]), ([k * n] if lead else []) + ([1, k] if majors[1] == "k" else [n, 1])
+    meta = H.matmul_metadata(lead + [m, n], lead + [m, k], lead + [k, n], sa, sb, 0, 0)
+    got = {}
+    for mode in (0, 2, 1):
+        lib.mx_debug_set_gemm_realign(mode)
+        try:
+            got[mode] = H.run_matmul(cuda, dt, meta, nb * m * n, a, b)
+        finally:
+            lib.mx_debug_set_gemm_realign(1)
+    assert np.array_equal(got[0], got[2]) and np.array_equal(got[0], got[1])
+    fa, fb = D.decode(a, dt).astype(np.float64), D.decode(b, dt).astype(np.float64)
+    for z in {0, nb - 1}:
+        za = fa[(0 if shared else z) * m * k:][:m * k]
+        x = za.reshape(m, k) if majors[0] == "k" else za.reshape(k, m).T
+        zb = fb[z * k * n:][:k * n]
+        y = zb.reshape(n, k).T if majors[1] == "k" else zb.reshape(k, n)
+        ref = x @ y
+        res = D.decode(got[0], dt).reshape(nb, m, n)[z]
+        step = 2.0 ** -8 if dt is D.BF16 else 2.0 ** -11
+        assert np.all(np.abs(res - ref) <= step * np.abs(ref) + 2e-5 * np.sqrt(k))
+
+
+@pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [
     # batch, M, N, K, majors, whether A is the same for all batches: edges of row and column tiles, a last k-block that is not full, runs of tiles that end inside a
     # panel; and what the rule leaves to the general schedule
     (97, 600, 760, 256, "kk", True), (149, 641, 504, 200, "km", True), (300, 520, 256, 248, "mm", True), (97, 600, 760, 256, "kk", False), (160, 512, 512, 256, "mm", True),
