@@ -960,8 +960,9 @@ __device__ __forceinline__ void repack_vector(const RowCopy<W>& p, uint32_t v) {
     *reinterpret_cast<uint4*>(p.out + (size_t)row * p.pitch + c) = r;
 }
 template <class W>
-__global__ void __launch_bounds__(256) repack_rows_kernel(RowCopy<W> a, RowCopy<W> b) {
+__global__ void __launch_bounds__(256) repack_rows_kernel(RowCopy<W> a, RowCopy<W> b, Gate gate) {
     after_previous_kernel();
+    if (gate.shut()) return;
     const uint32_t stride = gridDim.x * 256, all = a.vecs + b.vecs;
     for (uint32_t v = blockIdx.x * 256 + threadIdx.x; v < all; v += stride) {
         if (v < a.vecs) repack_vector(a, v);
@@ -993,11 +994,11 @@ static double misaligned_us(const TcProduct& c, uint64_t pitch, int box_kb) {
 static double copy_us(uint64_t rows, uint64_t cols) { return (double)rows * (double)cols * 4.0 / 5.0e6; }
 
 template <class W>
-static void repack_launch(const RowCopy<W>& a, const RowCopy<W>& b) {
+static void repack_launch(const RowCopy<W>& a, const RowCopy<W>& b, const Gate& gate) {
     uint64_t blocks = ((uint64_t)a.vecs + b.vecs + 255) / 256;
     const uint64_t cap = (uint64_t)sm_count() * 32;
     if (blocks > cap) blocks = cap;
-    launch_kernel(repack_rows_kernel<W>, (unsigned)blocks, 256, 0, ctx().stream, a, b);
+    launch_kernel(repack_rows_kernel<W>, (unsigned)blocks, 256, 0, ctx().stream, a, b, gate);
 }
 
 bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* where) {
@@ -1027,7 +1028,7 @@ bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* w
             const uint64_t per_row = (cols * es + 15) / 16;  // the padding itself is never read
             return RowCopy<W>{reinterpret_cast<const W*>(in), reinterpret_cast<W*>(out), yes ? (uint32_t)(rows * per_row) : 0u, FastDiv((uint32_t)per_row), (uint32_t)cols, (uint32_t)pitch};
         };
-        repack_launch<W>(copy(a_copy, c.A, a_dst, a_rows, a_cols, a_pitch), copy(b_copy, c.B, b_dst, b_rows, b_cols, b_pitch));
+        repack_launch<W>(copy(a_copy, c.A, a_dst, a_rows, a_cols, a_pitch), copy(b_copy, c.B, b_dst, b_rows, b_cols, b_pitch), c.gate);
     };
     if (es == 2) launch(uint16_t());
     else launch(uint32_t());

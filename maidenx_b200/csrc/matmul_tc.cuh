@@ -7,6 +7,13 @@
 
 namespace mx {
 
+// What a launch looks for before it does anything: it runs when the word holds the tag.  No word: it runs.
+struct Gate {
+    const unsigned long long* word = nullptr;
+    unsigned long long tag = 0;
+    __device__ __forceinline__ bool shut() const { return word && *word != tag; }
+};
+
 // A product the tensor-core kernels accept: D[m, n] = sum_k Aop[m, k] * Bop[n, k] with dense operands that are
 // K-major ([MN, K] row-major) or MN-major ([K, MN] row-major).
 struct TcProduct {
@@ -21,6 +28,7 @@ struct TcProduct {
     bool ragged = false;                      // not the plain form: rows or bases off 16 bytes, batches beyond rank 3, batched backward
     bool nearest = false;                     // 16-bit: a sum that the CUDA cores would round to nearest (see kRunMostF16)
     bool sum_batches = false;                 // D is one [m, n] matrix, the sum of the batches' products
+    Gate gate;                                // f32: the launches for this product run only if it is open
     int d_plain = 0;                          // the output is written without tensor stores: 1 element-wise, 2 in pairs
 };
 // Every product the kernels compute, with the fields that say what has to be prepared for it: dense and transposed operands, ragged
@@ -44,6 +52,9 @@ bool tc_batched_row_bias(bool is_bf16, uint64_t batch, uint64_t rows, uint64_t k
 // false = not taken (rows of k or n that are not 16-byte multiples, a small product).
 bool tc_batch_sum_f32(uint64_t batch, uint64_t m, uint64_t n, uint64_t k, const float* a, const float* b, float* out, const char* where);
 bool tc_launch_f32(const TcProduct& c, void* out, const char* where);
+// The product in pairs of f16 (matmul_tc_pairs.cu), if that is estimated to take less than `tf32_us`.  true: launched, and whoever called runs the product behind
+// `gate`, which is open when an operand was not fit for pairs and lies in `ws`; false: nothing launched.
+bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* out, Gate& gate, StreamWorkspace& ws, const char* where);
 bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out, const char* where);
 
 template <class T>

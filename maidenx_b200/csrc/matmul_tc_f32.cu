@@ -116,6 +116,7 @@ struct Params {
     // rows that fall to it over all of them, in slice order (the sums of the form with a second launch, bit for bit)
     int cluster;
     int vec_out;    // cluster: the rows of `out` may be written by 16-byte vectors
+    Gate gate;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, const Params& p, int& tm, int& tn, int& tb) {
@@ -217,6 +218,10 @@ template <int BN_T, int FORM = PLAIN>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                    Params p, int* err, int tag) {
+    if (p.gate.word) {  // behind a product in pairs: almost always shut
+        after_previous_kernel();
+        if (p.gate.shut()) return;
+    }
     extern __shared__ unsigned char tcf_smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)tcf_smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t smem_base = smem_u32(smem);
@@ -624,6 +629,21 @@ constexpr double kClusterFixed32 = 4.0;
 std::atomic<int> g_cluster{1};  // 0: no clusters of slices, 2: wherever they fit (tests, A/B timing)
 thread_local int t_last_form[4] = {0, 0, 0, 0};  // of the thread's last launch: slices, CTAs of a cluster (0: none), wide, columns of a tile (tests)
 
+// What a product is estimated to take here: 0.9 us for 128 columns of a k-block (1.2 where the accumulator is emptied after each), whole or cut into slices, and
+// the copies of ragged operands.
+double estimate_us(const TcProduct& c) {
+    int grid = sm_count();
+    if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
+    const uint64_t tiles_m = (c.m + BM - 1) / BM, tiles = tiles_m * ((c.n + BN - 1) / BN);
+    const double num_kb = (double)((c.k + BK - 1) / BK) * (c.sum_batches ? (double)c.batch : 1.0);
+    const uint64_t batch = c.sum_batches ? 1 : c.batch;
+    double kb = tile_cost(tile_columns(tiles_m, c.n, batch, grid), tiles_m, c.n, batch, grid) * num_kb;
+    if (batch == 1)  // 3 us more than in the choice of slices: the second launch's own
+        for (int s = 2; s <= 32; s++) kb = std::min(kb, (double)((tiles * s + grid - 1) / grid) * (double)(int)((num_kb + s - 1) / s) + kSplitFixed32 + 3.0 + 0.1 * s);
+    const double copies = (c.a_repack ? (double)c.m * c.k : 0.0) + (c.b_repack ? (double)c.n * c.k : 0.0);
+    return kb * (c.ragged ? 1.2 : 0.9) + 3.0 + (copies > 0 ? 1.5 + copies * 8 * c.batch / 5e6 : 0.0);
+}
+
 // D[M,N] = sum_k Aop[m,k] * Bop[n,k]; K-major operand = row-major [MN, K], MN-major = row-major [K, MN].
 bool launch(const TcProduct& c, void* D, const char* where) {
     const bool a_mn = c.a_mn, b_mn = c.b_mn;
@@ -651,6 +671,7 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     int slices = 1;
     const int bn_whole = tile_columns((uint64_t)p.tiles_m, N, batch, grid);
     p.cluster = 0;
+    p.gate = c.gate;
     if (batch == 1) {
         const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n;
         const double kb = (128 + p.bn) / 256.0, whole = tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, grid) * p.num_kb;
@@ -664,6 +685,7 @@ bool launch(const TcProduct& c, void* D, const char* where) {
             p.cluster = cluster_slices(tiles, (uint64_t)p.num_kb, grid, kb, kClusterFixed32, cost,
                                        [](int n) { return resident_clusters(reinterpret_cast<const void*>(tc_gemm_f32_kernel<0, CLUSTERED>), THREADS, SMEM_BYTES, n); });
         if (p.cluster) slices = p.cluster;
+        else if (c.gate.word) slices = 1;  // behind a gate in one launch
     }
     StreamWorkspace partial;
     const uint64_t n_pitch = (N + 3) / 4 * 4;
@@ -755,13 +777,22 @@ int resident_clusters(const void* kernel, int threads, size_t shared, int n) {
 }
 }  // namespace tc
 
-bool tc_launch_f32(const TcProduct& c, void* out, const char* where) { return launch(c, out, where); }
+// Pairs of f16 where they are faster, with the kernel above behind them for operands that are not fit; else, and where there is no workspace for pairs, that kernel alone.
+// Whatever fails here has launched no less than the product's own kernels would overwrite: the caller computes it another way.
+static bool repack_and_launch(TcProduct& c, void* out, const char* where) {
+    StreamWorkspace pairs, ws;
+    tc_launch_f32_pairs(c, estimate_us(c), out, c.gate, pairs, where);
+    return repack_operands(4, c, ws, where) && launch(c, out, where);
+}
+
+bool tc_launch_f32(const TcProduct& c, void* out, const char* where) {
+    TcProduct mine = c;
+    return repack_and_launch(mine, out, where);
+}
 
 bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out, const char* where) {
     TcProduct c;
-    if (!tc_classify(d, which, 4, num_els, nea, neb, x, y, out, c)) return false;
-    StreamWorkspace ws;
-    return repack_operands(4, c, ws, where) && launch(c, out, where);
+    return tc_classify(d, which, 4, num_els, nea, neb, x, y, out, c) && repack_and_launch(c, out, where);
 }
 
 }  // namespace mx

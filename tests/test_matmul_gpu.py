@@ -834,3 +834,99 @@ def test_split_products_under_capture(cuda, dt, case):
     finally:
         lib.mx_set_stream(None)
         del graph
+
+
+# batch, M, N, K, majors, operand shared by the batch, base offset in elements: edges of tiles and of scales' blocks (128 values of K, 64 of a k-block), a lone k-block,
+# slices of a long reduction, batches, ragged rows and bases
+PAIRS = [(1, 384, 384, 128, "kk", "", 0), (1, 385, 260, 196, "km", "", 0), (1, 516, 532, 64, "mm", "", 0), (1, 132, 136, 4100, "mk", "", 0), (5, 256, 200, 320, "km", "a", 0),
+         (6, 160, 256, 448, "kk", "b", 0), (9, 130, 132, 200, "mm", "", 0), (1, 257, 331, 333, "kk", "", 0), (1, 131, 257, 1001, "mm", "", 1), (3, 129, 233, 205, "km", "a", 0)]
+
+
+def _pairs_product(cuda, lib, case, a, b, mode):
+    nb, m, n, k, majors, shared, off = case
+    lead = [nb] if nb > 1 else []
+    sa = ([0 if "a" in shared else m * k] if lead else []) + ([k, 1] if majors[0] == "k" else [1, m])
+    sb = ([0 if "b" in shared else k * n] if lead else []) + ([1, k] if majors[1] == "k" else [n, 1])
+    lib.mx_debug_set_gemm_f32_pairs(mode)
+    try:
+        got = H.run_matmul(cuda, D.F32, H.matmul_metadata(lead + [m, n], lead + [m, k], lead + [k, n], sa, sb, off, off), nb * m * n, a, b)
+        return got.reshape(nb, m, n), lib.mx_debug_gemm_f32_last_pairs()
+    finally:
+        lib.mx_debug_set_gemm_f32_pairs(1)
+
+
+def _pairs_operands(case, rng, dist):
+    nb, m, n, k, majors, shared, off = case
+    draw = (lambda s: rng.standard_normal(s)) if dist == "normal" else (lambda s: rng.random(s))
+    a, b = (draw(off + (1 if s in shared else nb) * r * k).astype(np.float32) for s, r in (("a", m), ("b", n)))
+    x = a[off:].reshape(-1, m, k) if majors[0] == "k" else a[off:].reshape(-1, k, m).transpose(0, 2, 1)
+    y = b[off:].reshape(-1, n, k).transpose(0, 2, 1) if majors[1] == "k" else b[off:].reshape(-1, k, n)
+    return a, b, x, y
+
+
+@pytest.mark.parametrize("dist", ["normal", "positive"])
+@pytest.mark.parametrize("case", PAIRS, ids=lambda c: "x".join(map(str, c)))
+def test_f32_products_as_pairs_of_f16(cuda, case, dist):
+    """Next to float64, relative to the sums' size: 2^-23 of each factor, a truncation of at most 2^-24 of the running sum for each of a chunk's eight instructions, the totals' own
+    rounding - and no further from float64 than the tf32 kernel (a tenth for chance)."""
+    from maidenx_b200 import _lib
+    lib = _lib.load()
+    a, b, x, y = _pairs_operands(case, np.random.default_rng(sum(case[:4])), dist)
+    ref = x.astype(np.float64) @ y.astype(np.float64)
+    err = {}
+    ragged = any(v % 4 for v in ((case[3] if case[4][0] == "k" else case[1]), case[2], case[6])) or (case[4][1] == "k" and case[3] % 4)
+    for mode in (0, 2, 3):
+        got, pairs = _pairs_product(cuda, lib, case, a, b, mode)
+        assert (pairs > 0) == (mode > 0)
+        err[mode] = np.linalg.norm(got - ref) / np.linalg.norm(ref)
+    assert err[2] < 6e-7 and err[3] < 3e-7
+    assert err[3 if ragged else 2] <= 1.1 * err[0]
+
+
+@pytest.mark.parametrize("case", [(2048, 1600, 256, "kk"), (1800, 1540, 260, "km"), (2048, 1600, 392, "mm"), (2432, 1664, 1000, "km")], ids=lambda c: "x".join(map(str, c)))
+def test_the_tf32_kernel_s_forms_where_pairs_are_faster(cuda, case):
+    from maidenx_b200 import _lib
+    lib = _lib.load()
+    lib.mx_debug_set_gemm_f32_pairs(0)
+    try:
+        test_f32_products_with_both_parts_of_b_in_one_instruction(cuda, case)
+    finally:
+        lib.mx_debug_set_gemm_f32_pairs(1)
+
+
+@pytest.mark.parametrize("what", ["tiny", "tiny_k", "huge", "small_all", "denormal", "inf", "nan", "zeros"])
+@pytest.mark.parametrize("case", [(1, 300, 260, 400, "km", "", 0), (4, 132, 136, 260, "kk", "a", 0), (1, 257, 231, 333, "kk", "", 0)], ids=lambda c: "x".join(map(str, c)))
+def test_operands_that_are_not_fit_for_pairs(cuda, case, what):
+    """Elements far below their block's largest, blocks out of range, infinities and NaNs: the result is the tf32 kernel's, launched behind the pairs."""
+    from maidenx_b200 import _lib
+    lib = _lib.load()
+    rng = np.random.default_rng(7)
+    a, b, x, y = _pairs_operands(case, rng, "normal")
+    k, off = case[3], case[6]
+    if what == "tiny":  # all of one row of A, which only a block's common scale would lose
+        a[off:off + k] *= np.float32(1e-13)
+    elif what == "tiny_k":  # every third value of K, made up for in B
+        if case[4] == "km":
+            a.reshape(-1, k)[:, ::3] *= np.float32(1e12)
+            b.reshape(k, -1)[::3] *= np.float32(1e-12)
+    elif what == "huge":
+        a[off + 5], b[off + 7] = 3e38, 1e-37
+    elif what == "small_all":
+        a *= np.float32(1e-20)
+    elif what == "denormal":
+        a[off + 3] = 1e-42
+    elif what == "inf":
+        a[off + 1], b[off + 2 * k + 1] = np.inf, -np.inf
+    elif what == "nan":
+        b[off + 11] = np.nan
+    else:
+        a[off:off + 200 * 64] = 0.0
+    got, pairs = _pairs_product(cuda, lib, case, a, b, 2)
+    want, _ = _pairs_product(cuda, lib, case, a, b, 0)
+    assert pairs > 0
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+    with np.errstate(all="ignore"):
+        ref = x.astype(np.float64) @ y.astype(np.float64)
+        size = np.abs(x).astype(np.float64) @ np.abs(y).astype(np.float64)
+    fine = np.isfinite(want) & np.isfinite(ref)
+    assert np.all(np.abs(got - ref)[fine] <= 4e-6 * size[fine] + 1e-42)
