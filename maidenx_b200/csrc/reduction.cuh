@@ -406,13 +406,33 @@ __global__ void __launch_bounds__(kRedThreads) reduce_partials_block_kernel(cons
 constexpr int kColLanes = 32;  // threads along the columns
 constexpr int kColRows = 8;    // threads along the reduced dim
 
+// The fold of a strip of single columns by the last block, where it has many parts: a column by eight threads, each every eighth part, and then theirs in order, since the trips to L2 are what
+// this costs ([17683, 43] bf16, 148 parts, 41.6 us by one thread a column, 7.0 so; [9999, 100] 10.7, 6.0; vectors of f32 [3000, 1000] 7.2, 6.1).  A function of its own and an instantiation of its own
+// (TOGETHER): in the kernel that all columns take it cost those without a fold up to 6 %, and vectors' strips, whose main loop it took registers from, up to 30 %.
+constexpr u32 kColFoldTogether = 12;
+template <class T, int KIND, int VEC>
+__device__ __noinline__ void fold_columns(const typename RedTraits<T, KIND>::Acc* parts, T* out, u64 cols, u64 stride, u32 splits, u64 factor, typename RedTraits<T, KIND>::Acc* sm) {
+    typedef RedTraits<T, KIND> TR;
+    constexpr int LD = kColLanes * VEC, P = kColRows / VEC;  // threads of a column
+    const int c = threadIdx.x % LD, y = threadIdx.x / LD;
+    typename TR::Acc v = TR::init();
+    if ((u64)c < cols && (u32)y < splits) v = fold_published<TR, VEC>(parts + c + (u64)y * stride, P * stride, (splits - y + P - 1) / P);
+    sm[y * (LD + 1) + c] = v;
+    __syncthreads();
+    if (y == 0 && (u64)c < cols) {
+#pragma unroll
+        for (int q = 1; q < P; q++) v = TR::combine(v, sm[q * (LD + 1) + c]);
+        out[c] = TR::finalize(v, factor);
+    }
+}
+
 // grid = (ceil(I / (32 * VEC)), splits, min(O, 65535)).  VEC > 1 requires I % VEC == 0 and an
 // aligned base.
 // Vectors of 16-bit floats are held to four blocks an SM (see fold_published), maxima of eight-byte integers to five (they took 54 registers instead of 44 since
 // the wait at the top, four blocks: [48950, 873] u64 66 us before, 74, 54 so).  0: the compiler's own choice for all others; 1 would let it take every register (bf16 [130, 300000] 9.0 us, 9.8; minima of f32 [811, 2, 13536] 403, 888).
 template <class T, int KIND>
 constexpr int kColBlocks = is_half_v<T> ? 4 : KIND >= RED_MAX && std::is_integral<T>::value && sizeof(T) == 8 ? 5 : 0;
-template <class T, int KIND, int VEC>
+template <class T, int KIND, int VEC, bool TOGETHER = false>
 __global__ void __launch_bounds__(kColLanes* kColRows, VEC > 1 ? kColBlocks<T, KIND> : 0) reduce_cols_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial, u64 O,
                                                                          u64 R, u64 I, u64 seg, u32 splits, u64 factor, u32* counters) {
     after_previous_kernel();
@@ -469,15 +489,20 @@ __global__ void __launch_bounds__(kColLanes* kColRows, VEC > 1 ? kColBlocks<T, K
         if (splits > 1 && counters) {
             // fold in the same launch: the last block of this (o, column strip) to arrive
             if (last_arrival(counters + o * gridDim.x + blockIdx.x, splits)) {
-                for (int c = threadIdx.x; c < kColLanes * VEC; c += kColLanes * kColRows) {
-                    u64 gc = (u64)blockIdx.x * kColLanes * VEC + c;
-                    if (gc < I) {
-                        const Acc* parts = partial + o * I + gc;
-                        Acc v = TR::init();
-                        if constexpr (is_half_v<T> && VEC > 1) v = fold_published<TR, 8>(parts, O * I, splits);
-                        else
-                            for (u32 s2 = 0; s2 < splits; s2++) v = TR::combine(v, load_published(partial + ((u64)s2 * O + o) * I + gc));
-                        out[o * I + gc] = TR::finalize(v, factor);
+                if constexpr (TOGETHER) {
+                    const u64 c0 = (u64)blockIdx.x * kColLanes * VEC;
+                    fold_columns<T, KIND, VEC>(partial + o * I + c0, out + o * I + c0, I - c0, O * I, splits, factor, &sm[0][0]);
+                } else {
+                    for (int c = threadIdx.x; c < kColLanes * VEC; c += kColLanes * kColRows) {
+                        u64 gc = (u64)blockIdx.x * kColLanes * VEC + c;
+                        if (gc < I) {
+                            const Acc* parts = partial + o * I + gc;
+                            Acc v = TR::init();
+                            if constexpr (is_half_v<T> && VEC > 1) v = fold_published<TR, 8>(parts, O * I, splits);
+                            else
+                                for (u32 s2 = 0; s2 < splits; s2++) v = TR::combine(v, load_published(partial + ((u64)s2 * O + o) * I + gc));
+                            out[o * I + gc] = TR::finalize(v, factor);
+                        }
                     }
                 }
             }
@@ -790,7 +815,10 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
             counters = arrival_counters(O * gx);
         }
         dim3 grid((u32)gx, (u32)splits, (u32)gz);
-        if (vec) launch_kernel(reduce_cols_kernel<T, KIND, VEC>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
+        constexpr int TV = VEC < kColRows ? VEC : 1;  // a wider vector's columns have a thread each
+        if (vec && TV == VEC && splits >= 2 * kColFoldTogether) launch_kernel(reduce_cols_kernel<T, KIND, TV, true>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
+        else if (vec) launch_kernel(reduce_cols_kernel<T, KIND, VEC>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
+        else if (splits >= kColFoldTogether) launch_kernel(reduce_cols_kernel<T, KIND, 1, true>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
         else launch_kernel(reduce_cols_kernel<T, KIND, 1>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
         if (splits > 1 && !counters) {
             check_launch(where);

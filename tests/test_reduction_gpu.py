@@ -236,3 +236,28 @@ def test_ragged_rows_on_both_sides_of_the_rules_lines(oracle, cuda, dt):
                     binding.set_wide(False)
                 got = H.run_reduce(cuda, op, dt, [o, r], [r, 1], [r], [1], 1, x)
                 H.assert_same(op, dt, got, ref, float_rel=SUM_TOL.get(dt.name, 0.0) if op != "max" else 0.0, what=str((op, r, o)), scale=np.sqrt(r) if op == "sum" else 1.0)
+
+
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F64, D.I32, D.U8, D.U64], ids=lambda d: d.name)
+@pytest.mark.parametrize("shape", [(769, 33), (1600, 1), (17683, 43), (9999, 100), (20011, 129), (3, 5000, 31), (6500, 132), (40000, 2)], ids=str)
+def test_columns_cut_into_many_parts(oracle, cuda, shape, dt):
+    """The last block of a strip folds its parts with several threads a column: on both sides of the number of parts from which on, strips with columns missing, fewer parts than threads
+    would share, several outer indices; twice, with the same bits (float sums: the file's bounds)."""
+    rng = np.random.default_rng(sum(shape))
+    a = H.random_store(rng, dt, int(np.prod(shape)), dist="normal") if dt.kind == "float" else H.random_store(rng, dt, int(np.prod(shape)))
+    dim = len(shape) - 2
+    from oracle import binding
+    for op in ("sum", "max", "min") + (("mean",) if dt.kind == "float" else ()):
+        got = _run_dim(cuda, op, dt, list(shape), None, [dim], 0, a)
+        binding.set_wide(True)
+        try:
+            ref = _run_dim(oracle, op, dt, list(shape), None, [dim], 0, a)
+        finally:
+            binding.set_wide(False)
+        exact = dt.kind != "float" or op in ("max", "min")
+        if exact:
+            assert np.array_equal(got, ref), op
+        else:
+            scale = np.sqrt(shape[dim]) / (shape[dim] if op == "mean" else 1.0)
+            H.assert_same(op, dt, got, ref, float_rel=SUM_TOL[dt.name], scale=scale, what=f"{op} {shape}")
+        assert np.array_equal(got, _run_dim(cuda, op, dt, list(shape), None, [dim], 0, a)), op
