@@ -150,7 +150,13 @@ __global__ void __launch_bounds__(kFusedThreads) gelu_backward_kernel(const T* d
         if (threadIdx.x == 0) partial[blockIdx.x] = acc;
         if (!fused_last_block(arrived)) return;
         acc = 0.0f;
-        for (uint32_t i = threadIdx.x; i < gridDim.x; i += kFusedThreads) acc += __ldcg(partial + i);
+        for (uint32_t i = threadIdx.x; i < gridDim.x; i += 4 * kFusedThreads) {
+            float v[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++) v[q] = i + q * kFusedThreads < gridDim.x ? __ldcg(partial + i + q * kFusedThreads) : 0.0f;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++) acc += v[q];
+        }
         acc = fused_block_sum(acc);
         if (threadIdx.x == 0) *grad_sum = st_from_f32<T>(acc);
     }
@@ -169,6 +175,28 @@ __device__ __forceinline__ float mse_fold(const float* partial, uint32_t count) 
         __syncthreads();
     }
     return sm[0];
+}
+
+// The same by half a block, in a tree of its own; valid in the half's first thread.
+__device__ __forceinline__ float fused_half_sum(const float* partial, uint32_t count) {
+    constexpr uint32_t HALF = kFusedThreads / 2;
+    __shared__ float warp_part[kFusedThreads / 32];
+    const uint32_t t = threadIdx.x % HALF;
+    float acc = 0.0f;
+    for (uint32_t i = t; i < count; i += 4 * HALF) {  // four parts in flight: what a trip to L2 takes is the length of this
+        float v[4];
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++) v[q] = i + q * HALF < count ? __ldcg(partial + i + q * HALF) : 0.0f;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++) acc += v[q];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (t == 0)
+        for (uint32_t w = 1; w < HALF / 32; w++) acc += warp_part[(threadIdx.x >> 5) + w];
+    return acc;
 }
 
 // grad = 2 (p - t) / n, per-block partial sums of (p - t)^2 into `partial` and, with SUM, of grad behind them; with SUM the last block folds both.
@@ -216,18 +244,16 @@ __global__ void __launch_bounds__(kFusedThreads) mse_kernel(const T* p, const T*
         float v = lane < kFusedThreads / 32 ? warp_part[which][lane] : 0.0f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        if (lane == 0) {
-            partial[which * gridDim.x + blockIdx.x] = v;
-            __threadfence();
-        }
+        if (lane == 0) partial[which * gridDim.x + blockIdx.x] = v;
     }
     if constexpr (SUM) {
-        __syncthreads();
+        __syncthreads();  // both parts are written: the fence of the thread that counts is behind them
         if (!fused_last_block(arrived)) return;
-        const float l = mse_fold(partial, gridDim.x), g = mse_fold(partial + gridDim.x, gridDim.x);
-        if (threadIdx.x) return;
-        *loss = l * inv_n;
-        *grad_sum = st_from_f32<T>(g);
+        // two halves of the block, a sum each
+        const uint32_t half = threadIdx.x / (kFusedThreads / 2);
+        float v = fused_half_sum(partial + half * gridDim.x, gridDim.x);
+        if (threadIdx.x == 0) *loss = v * inv_n;
+        if (threadIdx.x == kFusedThreads / 2) *grad_sum = st_from_f32<T>(v);
     }
 }
 // Without an arrival word (the exported pass, whose caller has none): the loss folded by a launch of one block.

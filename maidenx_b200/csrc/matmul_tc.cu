@@ -235,14 +235,16 @@ enum TcMode {
 // PANELS: TcParams::panels, an instantiation of its own for the same reason (as a branch of the common schedule it cost 4096^3 19 %).
 //
 // Epilogue warps for each quarter of the accumulator's lanes.  Rows that the warps write themselves take two (4096 x 2050 x 512 bf16: 25 us, 36
-// with one); products that leave through the copy engine gain nothing from a second one (16384 x 4096 x 256: 55 us, 50 with one).
-constexpr int epi_warps(int mode) { return mode == TC_PLAIN ? 2 : 1; }
-constexpr int tc_threads(int mode) { return 32 * (2 + 4 * epi_warps(mode)); }
+// with one), and so do narrow tiles with a bias or an activation, whose arithmetic a wave of few tiles ends with (training step of two layers 1024 x 2048 x 2048 96.2 us, 94.5 so;
+// 256 x 256 x 256 34.9, 33.9); products that only leave through the copy engine gain nothing from a second one (16384 x 4096 x 256: 55 us, 50 with one; 128 x
+// (384 x 384 x 64) and its gradients 31.1, 29.8).
+constexpr int epi_warps(int mode, int bn_t, bool drain) { return mode == TC_PLAIN || (mode == TC_BIAS && !bn_t && !drain) ? 2 : 1; }
+constexpr int tc_threads(int w) { return 32 * (2 + 4 * w); }
 template <int MODE, int BN_T, bool DRAIN = false, bool PANELS = false>
-__global__ void __launch_bounds__(tc_threads(MODE), 1)
+__global__ void __launch_bounds__(tc_threads(epi_warps(MODE, BN_T, DRAIN)), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                const __grid_constant__ CUtensorMap map_d2, TcParams p, int* err, int tag) {
-    constexpr int W = epi_warps(MODE), CW = EPI_CHUNK_COLS / W;  // columns of a chunk that a warp has
+    constexpr int W = epi_warps(MODE, BN_T, DRAIN), CW = EPI_CHUNK_COLS / W;  // columns of a chunk that a warp has
     extern __shared__ unsigned char tc_smem_raw[];
     // 128-byte swizzled TMA tiles and UMMA descriptors want 1024-byte aligned bases
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -554,7 +556,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 acc_phase ^= 1;
             }
         }
-        if (lane == 0) tma_store_wait_all();
+        // the staging has been read; the writes themselves belong to the launch, and what follows it waits for them
+        if (lane == 0) tma_store_wait_read<0>();
     }
 
     // common exit: TMEM is released by the warp that allocated it, after everyone is done with it
@@ -783,7 +786,8 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
                         : drain ? (p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0, true> : (fuse ? tc_gemm_kernel<TC_BIAS, 0, true> : tc_gemm_kernel<TC_STORE, 0, true>))
                         : p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0>
                                   : (fuse ? (full ? tc_gemm_kernel<TC_BIAS, BN> : tc_gemm_kernel<TC_BIAS, 0>) : (full ? tc_gemm_kernel<TC_STORE, BN> : tc_gemm_kernel<TC_STORE, 0>));
-    launch_kernel(kernel, grid, tc_threads(p.d_plain ? TC_PLAIN : TC_STORE), TC_SMEM_BYTES, ctx().stream, ma, mb, md, md2, p, err, tag);
+    const int warps = epi_warps(p.d_plain ? TC_PLAIN : fuse ? TC_BIAS : TC_STORE, panels || full ? BN : 0, drain);
+    launch_kernel(kernel, grid, tc_threads(warps), TC_SMEM_BYTES, ctx().stream, ma, mb, md, md2, p, err, tag);
     check_launch(where);
     if (slices > 1) splitk_reduce(is_bf16 ? 0 : 1, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
     return true;

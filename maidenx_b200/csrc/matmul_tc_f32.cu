@@ -485,7 +485,7 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 redo()[REDO_BITS / 32] = 1;
             }
         }
-        if (lane == 0) tma_store_wait_all();
+        if (lane == 0) tma_store_wait_read<0>();  // the staging has been read; the writes themselves belong to the launch, and what follows it waits for them
     } else {
         // ------------------------------------------------------------ splitter (warps 6..9)
         const int t = threadIdx.x - 32 * (2 + EPI_WARPS);
@@ -570,8 +570,10 @@ tc_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         return;
     }
 
-    // the tile stores have completed (tma_store_wait_all before the barrier above): their places may be written again
     if (!redo()[REDO_BITS / 32]) return;
+    // the tile stores have to be made before their places are written again
+    if (warp >= 2 && warp < 2 + EPI_WARPS && lane == 0) tma_store_wait_all();
+    __syncthreads();
     fence_proxy_async();
     for (int tile = blockIdx.x, it = 0; tile < p.num_tiles; tile += gridDim.x, it++) {
         if (!(redo()[it % REDO_BITS / 32] >> it % 32 & 1)) continue;

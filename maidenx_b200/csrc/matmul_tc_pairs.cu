@@ -322,7 +322,7 @@ tc_gemm_pairs_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 }
             }
         }
-        if (lane == 0) tma_store_wait_all();
+        if (lane == 0) tma_store_wait_read<0>();
     }
 
     tc_fence_before();
