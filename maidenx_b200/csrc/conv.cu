@@ -44,24 +44,28 @@ struct ConvPlanes : ConvParams {
 
 constexpr int kConvThreads = 256;
 
-// `count` consecutive elements into shared memory, as 16-byte vectors where the source allows.
+// `count` consecutive elements into shared memory, as 16-byte vectors where the source allows, all of them in flight; complete behind the caller's barrier.
 template <class T>
 __device__ __forceinline__ void stage_run(T* dst, const T* src, uint32_t count) {
     constexpr uint32_t VEC = 16 / sizeof(T);
     uint32_t done = 0;
     if ((uintptr_t)src % 16 == 0) {
         done = count / VEC * VEC;
-        for (uint32_t i = threadIdx.x * VEC; i < done; i += kConvThreads * VEC) *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+        for (uint32_t i = threadIdx.x * VEC; i < done; i += kConvThreads * VEC)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + i * (uint32_t)sizeof(T)), "l"(src + i) : "memory");
     }
     for (uint32_t i = done + threadIdx.x; i < count; i += kConvThreads) dst[i] = src[i];
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// The block's planes share one flat index over [plane, kh, kw, out_h, out_w], a thread takes VEC consecutive columns of it from
-// one index computation and walks on from there, so that small maps (14 x 14: 49 vectors of a plane's 441) keep every thread
-// busy and ragged ones (7 x 7) are written as vectors too.  Bound by HBM / L2 writes: [32, 128, 14, 14] f32, 3 x 3: 12 us, 23 with one
-// plane and one kernel offset at a time.
-template <class T, int VEC>
-__global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* x, T* col, ConvPlanes P) {
+// The block's planes share one flat index over [plane, kh, kw, out_h, out_w], which repeats from group to group of `step` planes, the fewest that make whole vectors: a thread takes VEC
+// consecutive columns of a group, finds where they come from once and writes them for all groups of the block.  So small maps (14 x 14: 49 vectors of a
+// plane's 441) keep every thread busy and ragged ones (7 x 7) are written as vectors too.  Bound by HBM / L2 writes and by the reads from shared memory (vectors of neighbouring
+// lanes meet in its banks): [32, 128, 14, 14] f32, 3 x 3: 7 us, 12 with the places found anew for every plane, 23 with one plane and one kernel offset at a time.
+// GROUPS: the block has more than one group; with a single one places kept for later cost what they take ([39, 170, 25, 25] bf16 45.7 us, 48.4).
+template <class T, int VEC, bool GROUPS>
+__global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* x, T* col, ConvPlanes P, uint32_t step) {
     after_previous_kernel();
     extern __shared__ __align__(16) unsigned char conv_smem[];
     T* img = reinterpret_cast<T*>(conv_smem);
@@ -72,17 +76,54 @@ __global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* x,
     const T zero = zero_of<T>();
     const uint64_t base = (uint64_t)bc0 * KK * OHW;
     const uint32_t total = (uint32_t)min((uint64_t)np * KK * OHW, P.num_els - base);
-    for (uint32_t e = threadIdx.x * VEC; e < total; e += kConvThreads * VEC) {
+    if constexpr (!GROUPS) {
+        for (uint32_t e = threadIdx.x * VEC; e < total; e += kConvThreads * VEC) {
+            uint32_t row, o, plane, kk, kh, kw, ho, wo;
+            P.ohw_div.divmod(e, row, o);
+            P.kk_div.divmod(row, plane, kk);
+            P.kw_div.divmod(kk, kh, kw);
+            P.ow_div.divmod(o, ho, wo);
+            Vec<T, VEC> r;
+#pragma unroll
+            for (int j = 0; j < VEC; j++) {
+                const int hi = (int)(ho * P.SH + kh) - (int)P.PH, wi = (int)(wo * P.SW + kw) - (int)P.PW;
+                r.v[j] = (uint32_t)hi < P.H && (uint32_t)wi < P.W && plane < np ? img[plane * HW + hi * P.W + wi] : zero;
+                if (++wo == P.OW) {
+                    wo = 0;
+                    if (++ho == P.OH) {
+                        ho = 0;
+                        if (++kw == P.KW) {
+                            kw = 0;
+                            if (++kh == P.KH) {
+                                kh = 0;
+                                plane++;
+                            }
+                        }
+                    }
+                }
+            }
+            if (e + VEC <= total) {
+                *reinterpret_cast<Vec<T, VEC>*>(col + base + e) = r;
+            } else {
+#pragma unroll
+                for (int j = 0; j < VEC; j++)
+                    if (e + j < total) col[base + e + j] = r.v[j];
+            }
+        }
+        return;
+    }
+    const uint32_t period = step * KK * OHW, hop = step * HW;
+    for (uint32_t e0 = threadIdx.x * VEC; e0 < min(total, period); e0 += kConvThreads * VEC) {
         uint32_t row, o, plane, kk, kh, kw, ho, wo;
-        P.ohw_div.divmod(e, row, o);
+        P.ohw_div.divmod(e0, row, o);
         P.kk_div.divmod(row, plane, kk);
         P.kw_div.divmod(kk, kh, kw);
         P.ow_div.divmod(o, ho, wo);
-        Vec<T, VEC> r;
+        int at[VEC];  // the element's place in the group's planes, -1 in the padding
 #pragma unroll
         for (int j = 0; j < VEC; j++) {
             const int hi = (int)(ho * P.SH + kh) - (int)P.PH, wi = (int)(wo * P.SW + kw) - (int)P.PW;
-            r.v[j] = (uint32_t)hi < P.H && (uint32_t)wi < P.W && plane < np ? img[plane * HW + hi * P.W + wi] : zero;
+            at[j] = (uint32_t)hi < P.H && (uint32_t)wi < P.W ? (int)(plane * HW) + hi * (int)P.W + wi : -1;
             if (++wo == P.OW) {
                 wo = 0;
                 if (++ho == P.OH) {
@@ -97,12 +138,19 @@ __global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* x,
                 }
             }
         }
-        if (e + VEC <= total) {
-            *reinterpret_cast<Vec<T, VEC>*>(col + base + e) = r;
-        } else {
+        const T* from = img;
+#pragma unroll 2
+        for (uint32_t e = e0; e < total; e += period, from += hop) {
+            Vec<T, VEC> r;  // elements behind the last plane are read from the block's memory all the same, and not written
 #pragma unroll
-            for (int j = 0; j < VEC; j++)
-                if (e + j < total) col[base + e + j] = r.v[j];
+            for (int j = 0; j < VEC; j++) r.v[j] = at[j] < 0 ? zero : from[at[j]];
+            if (e + VEC <= total) {
+                *reinterpret_cast<Vec<T, VEC>*>(col + base + e) = r;
+            } else {
+#pragma unroll
+                for (int j = 0; j < VEC; j++)
+                    if (e + j < total) col[base + e + j] = r.v[j];
+            }
         }
     }
 }
@@ -162,9 +210,10 @@ __device__ __forceinline__ T conv_add(T a, T b) {
 }
 
 // The same sums from shared memory: the KH * KW column planes of the block's image planes arrive in one contiguous run; a
-// column entry crosses from L2 once instead of once per term.  Strides of 1: larger ones touch few entries more than once.
-// [32, 128, 14, 14] f32, 3 x 3: 14 us, 16 from L2.
-template <class T>
+// column entry crosses from L2 once instead of once per term.  Strides of 1: larger ones touch few entries more than once.  K > 0: a K x K kernel, whose terms are so many reads at
+// distances known up front, each under a bit of the pixel's row or column; 0: any kernel, by the ranges of its output rows and columns.
+// [32, 128, 14, 14] f32, 3 x 3: 8 us, 14 by the ranges, 16 from L2.
+template <class T, int K>
 __global__ void __launch_bounds__(kConvThreads) col2im_planes_kernel(const T* col, T* out, ConvPlanes P) {
     after_previous_kernel();
     extern __shared__ __align__(16) unsigned char conv_smem[];
@@ -181,18 +230,39 @@ __global__ void __launch_bounds__(kConvThreads) col2im_planes_kernel(const T* co
         P.hw_div.divmod(i, plane, pix);
         P.w_div.divmod(pix, h, w);
         const uint32_t hp = h + P.PH, wp = w + P.PW;
-        // conv.rs:121-125
-        const uint32_t hs = hp >= P.KH - 1 ? hp - (P.KH - 1) : 0, ws = wp >= P.KW - 1 ? wp - (P.KW - 1) : 0;
-        const uint32_t he = min(hp + 1, P.OH), we = min(wp + 1, P.OW);
         const T* mine = cols + plane * KK * OHW;
         T sum = zero_of<T>();
-        for (uint32_t ho = hs; ho < he; ho++) {
-            const uint32_t kh = hp - ho;
-            if (kh >= P.KH) continue;
-            const T* row = mine + kh * P.KW * OHW + ho * P.OW;
-            for (uint32_t wo = ws; wo < we; wo++) {
-                const uint32_t kw = wp - wo;
-                if (kw < P.KW) sum = conv_add(sum, row[kw * OHW + wo]);
+        if constexpr (K > 0) {
+            // output row hp - kh, output column wp - kw; ascending, as conv.rs:121-135 goes through them
+            const T* top = mine + hp * P.OW + wp;
+            const int kh_step = (int)(K * OHW) - (int)P.OW, kw_step = (int)OHW - 1;
+            uint32_t cols_in = 0;
+#pragma unroll
+            for (int kw = 0; kw < K; kw++) cols_in |= (wp - kw < P.OW ? 1u : 0u) << kw;
+#pragma unroll
+            for (int kh = K - 1; kh >= 0; kh--) {
+                if (hp - kh < P.OH) {
+                    T v[K];
+#pragma unroll
+                    for (int kw = K - 1; kw >= 0; kw--)
+                        if (cols_in >> kw & 1) v[kw] = top[kh * kh_step + kw * kw_step];
+#pragma unroll
+                    for (int kw = K - 1; kw >= 0; kw--)
+                        if (cols_in >> kw & 1) sum = conv_add(sum, v[kw]);
+                }
+            }
+        } else {
+            // conv.rs:121-125
+            const uint32_t hs = hp >= P.KH - 1 ? hp - (P.KH - 1) : 0, ws = wp >= P.KW - 1 ? wp - (P.KW - 1) : 0;
+            const uint32_t he = min(hp + 1, P.OH), we = min(wp + 1, P.OW);
+            for (uint32_t ho = hs; ho < he; ho++) {
+                const uint32_t kh = hp - ho;
+                if (kh >= P.KH) continue;
+                const T* row = mine + kh * P.KW * OHW + ho * P.OW;
+                for (uint32_t wo = ws; wo < we; wo++) {
+                    const uint32_t kw = wp - wo;
+                    if (kw < P.KW) sum = conv_add(sum, row[kw * OHW + wo]);
+                }
             }
         }
         out[(uint64_t)bc0 * HW + i] = sum;
@@ -344,10 +414,13 @@ void im2col_entry(size_t num_els, const size_t* meta, const T* x, T* col, const 
     uint64_t step = 1;
     while (step < VEC && (chunk * step) % VEC != 0) step *= 2;
     const uint64_t ohw = (uint64_t)P.OH * P.OW;
-    const uint32_t pb = (uintptr_t)col % 16 == 0 ? planes_per_block(planes_touched, plane_bytes, step, planes_most(sizeof(T), step, ohw)) : 0;
+    uint32_t pb = (uintptr_t)col % 16 == 0 ? planes_per_block(planes_touched, plane_bytes, step, planes_most(sizeof(T), step, ohw)) : 0;
+    // four groups share their places where two blocks an SM are left ([32, 128, 14, 14] bf16, a group of two planes: 10.0 us with one group a block)
+    if (pb && pb < 4 * step && 4 * step * plane_bytes <= 16 * 1024 && planes_touched >= 4 * step * 2 * (uint64_t)sm_count()) pb = (uint32_t)(4 * step);
     if (pb && pb * chunk < 0x7FFFFFFFull && planes_pay(sizeof(T), step, (planes_touched + pb - 1) / pb, ohw)) {
-        allow_shared_memory(im2col_planes_kernel<T, VEC>, pb * plane_bytes);
-        launch_kernel(im2col_planes_kernel<T, VEC>, (unsigned)((planes_touched + pb - 1) / pb), kConvThreads, pb * plane_bytes, s, x, col, ConvPlanes(P, planes_touched, pb));
+        const auto kernel = pb > step ? im2col_planes_kernel<T, VEC, true> : im2col_planes_kernel<T, VEC, false>;
+        allow_shared_memory(kernel, pb * plane_bytes);
+        launch_kernel(kernel, (unsigned)((planes_touched + pb - 1) / pb), kConvThreads, pb * plane_bytes, s, x, col, ConvPlanes(P, planes_touched, pb), (uint32_t)step);
     } else if (plane_bytes <= kConvSmemMost) {
         auto launch = [&](auto kernel) {
             allow_shared_memory(kernel, plane_bytes);
@@ -424,7 +497,9 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
     const uint64_t col_plane = (uint64_t)P.KH * P.KW * P.OH * P.OW;
     const uint32_t pb = P.SH == 1 && P.SW == 1 && planes <= 0x7FFFFFFFull && col_plane && HW < 0x7FFFFFFFull ? planes_per_block(planes, col_plane * sizeof(T), 1, 48 * 1024) : 0;
     if (pb && pb * HW < 0x7FFFFFFFull && pb * HW >= kConvThreads / 2 && (HW <= kConvThreads || ((planes + pb - 1) / pb >= 512 && (sizeof(T) < 8 || P.KH * P.KW == 1)))) {
-        launch_kernel(col2im_planes_kernel<T>, (unsigned)((planes + pb - 1) / pb), kConvThreads, pb * col_plane * sizeof(T), s, col, out, ConvPlanes(P, planes, pb));
+        const uint32_t k = P.KH == P.KW ? P.KH : 0;
+        const auto kernel = k == 3 ? col2im_planes_kernel<T, 3> : k == 5 ? col2im_planes_kernel<T, 5> : k == 7 ? col2im_planes_kernel<T, 7> : col2im_planes_kernel<T, 0>;
+        launch_kernel(kernel, (unsigned)((planes + pb - 1) / pb), kConvThreads, pb * col_plane * sizeof(T), s, col, out, ConvPlanes(P, planes, pb));
         check_launch(where);
         return;
     }

@@ -164,3 +164,16 @@ def test_images_of_no_pixels(cuda, dt, case):
     assert n > 0
     got = H.run_im2col(cuda, dt, meta, n, H.random_store(np.random.default_rng(1), dt, 1, dist="normal"))
     assert np.array_equal(D.decode(got, dt), np.zeros(n))
+
+
+GROUPS = [
+    # several groups of planes a block, the last block and the last group incomplete; groups of one, two and four planes; kernels of 3, 5, 7 (terms at fixed distances) and others
+    ("14x14-3", 9, 277, 14, 14, 3, 3, 1, 1, 1, 1), ("13x13-5", 8, 313, 13, 13, 5, 5, 2, 2, 1, 1), ("7x7-7", 11, 223, 7, 7, 7, 7, 3, 3, 1, 1), ("6x10-3-nopad", 10, 251, 6, 10, 3, 3, 0, 0, 1, 1),
+    ("9x9-7-wide-pad", 7, 350, 9, 9, 7, 7, 5, 4, 1, 1), ("8x9-3x5", 6, 401, 8, 9, 3, 5, 1, 2, 1, 1), ("11x7-3-s2", 9, 301, 11, 7, 3, 3, 1, 1, 2, 2), ("4x4-5", 3, 797, 4, 4, 5, 5, 2, 2, 1, 1),
+]
+
+
+@pytest.mark.parametrize("dt", D.FLOATS, ids=lambda d: d.name)
+@pytest.mark.parametrize("case", GROUPS, ids=lambda c: c[0])
+def test_groups_of_planes_in_a_block(oracle, cuda, dt, case):
+    test_planes_sharing_a_block(oracle, cuda, dt, case)
