@@ -1010,7 +1010,16 @@ __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, co
 // Two inputs of ragged rows, each the output's own layout or the same row for all of them (a bias, a norm's weights): one division by multiplication a
 // vector, the repeated row from L1 by elements, up to two vectors a thread.  [8191, 1023] f32 9.5 us (10.8 by the dense kernel), [4099, 1543] bf16 5.9 (7.0).  An
 // instantiation of the kernel above for it would have the constants' registers too.
-template <class F, class T, class O, int VEC>
+// SHIFTED, for rows of kEwRepeatLong and more: the repeated row's vectors from the two aligned words they lie in instead of by elements, which meet in L1's banks ([4099, 1543] bf16 6.1 us,
+// 4.9 so, [2277, 5799] 10.5, 7.8; f32 [8191, 1023] 9.7, 8.9).  In shorter rows the vectors that wrap, which go by elements, are in too many warps ([30000, 197] bf16 5.2,
+// 6.1), below two vectors a thread the way to the words is longer than what they save ([3, 100001] bf16 1.7, 2.0), and quotients and saturating sums of 16 bits have
+// no registers for it ([5789, 3853] f32 28.1, 31.6; [12489, 523] i16 7.5, 8.4).
+constexpr uint32_t kEwRepeatLong = 512;
+template <class F>
+struct EwShiftsRepeated : std::true_type {};
+template <class T, class O>
+struct EwShiftsRepeated<Binary<OpDiv, T, O>> : std::false_type {};
+template <class F, class T, class O, int VEC, bool SHIFTED = false>
 __global__ void __launch_bounds__(kEwThreads) ew_repeat_kernel(F f, const T* a, const T* b, O* out, EwRepeatParams P) {
     after_previous_kernel();
     constexpr int U = kEwChanUnroll;
@@ -1023,8 +1032,12 @@ __global__ void __launch_bounds__(kEwThreads) ew_repeat_kernel(F f, const T* a, 
         const uint32_t col = i0 - P.q_div.div(i0) * P.q;
         auto load = [&](const T* p, int repeated, Vec<T, VEC>& v) {
             if (repeated) {
+                if (SHIFTED && col + VEC <= P.q) {
+                    v = ld_vec_shifted<T, VEC>(p + col, (uint32_t)reinterpret_cast<uintptr_t>(p + col) & 15);
+                } else {
 #pragma unroll
-                for (int j = 0; j < VEC; j++) v.v[j] = p[col + j < P.q ? col + j : col + j - P.q];
+                    for (int j = 0; j < VEC; j++) v.v[j] = p[col + j < P.q ? col + j : col + j - P.q];
+                }
             } else if (i0 + VEC <= P.n) {
                 v = ld_vec<T, VEC>(p + i0);
             } else {
@@ -1211,7 +1224,9 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                         break;
                     }
                     if (ew_fill_repeat_params(D, VEC, Q)) {
-                        launch_kernel(ew_repeat_kernel<F, T, O, VEC>, blocks, kEwThreads, 0, s, f, a, b, out, Q);
+                        constexpr bool kShifts = EwShiftsRepeated<F>::value && (is_half_v<T> || std::is_same<T, f32>::value);
+                        if (kShifts && Q.q >= kEwRepeatLong && Q.units > 1) launch_kernel(ew_repeat_kernel<F, T, O, VEC, kShifts>, blocks, kEwThreads, 0, s, f, a, b, out, Q);
+                        else launch_kernel(ew_repeat_kernel<F, T, O, VEC>, blocks, kEwThreads, 0, s, f, a, b, out, Q);
                         break;
                     }
                 }

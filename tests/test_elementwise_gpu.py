@@ -396,6 +396,20 @@ def test_operands_constant_along_ragged_rows(oracle, cuda, dt, q):
         H.assert_same("add_inplace", dt, H.run_binary_inplace(cuda, *args), H.run_binary_inplace(oracle, *args), what=f"{name} in place q={q}")
 
 
+@pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("shape", [(2500, 513), (1211, 1023), (3, 500001), (700, 2049)], ids=str)
+def test_a_long_row_repeated_from_any_place(oracle, cuda, dt, shape):
+    """Large tensors of long ragged rows: the repeated row's vectors come from the aligned words they lie in, at every distance from a 16-byte boundary, and by elements where a row ends."""
+    rows, q = shape
+    rng = np.random.default_rng(rows + q)
+    n = rows * q
+    full = H.random_store(rng, dt, n, dist="normal")
+    for off in range(16 // dt.size):
+        part = H.random_store(rng, dt, q + off, dist="normal")
+        args = ("sub", dt, [rows, q], [q, 1], [0, 1], 0, off, full, part) if off % 2 else ("mul", dt, [rows, q], [0, 1], [q, 1], off, 0, part, full)
+        H.assert_same(args[0], dt, H.run_binary(cuda, *args), H.run_binary(oracle, *args), what=f"{shape} {off}")
+
+
 @pytest.mark.parametrize("dt", [D.F32, D.BF16, D.F64, D.U8, D.I32], ids=lambda d: d.name)
 def test_last_block_of_flat_operands(oracle, cuda, dt):
     """The block that is not full works by vectors too: lengths around the vector, a block's 256 threads and its four vectors a thread."""
