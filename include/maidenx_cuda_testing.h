@@ -36,6 +36,9 @@ int mx_debug_matmul_forward_path_f32(size_t num_els, const size_t* host_metadata
 void mx_debug_set_gemm_group_m(int rows);
 /* Pairs of CTAs of the two-CTA tensor-core kernel that can be resident at once on the current device (-1: query failed). */
 int mx_debug_gemm_max_resident_pairs(void);
+/* The 16-bit Conv2d layer's input gradient (direct form, strides of 1) as one product without a column matrix: 1 = by the rule (default), 0 = never, 2 = wherever
+ * possible. */
+void mx_debug_set_conv_implicit(int mode);
 /* f32 products as pairs of f16 values: 1 = by the rule on their cost (default), 0 = never, 2 = wherever possible, 3 = the same, emptying the accumulator after
  * every k-block of 64.  The query: the calling thread's last f32 product ran as pairs in this many slices (0: not as pairs). */
 void mx_debug_set_gemm_f32_pairs(int mode);

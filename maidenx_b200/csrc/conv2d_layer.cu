@@ -2,7 +2,8 @@
 // composes them (crates/maidenx_nn/src/layers/conv.rs:185-307 with the im2col / col2im wrappers at :333-420):
 // im2col -> matmul -> (views) -> bias add, and in backward matmul -> col2im for the input gradient, matmul for
 // the weight gradient and three sums for the bias gradient.  Every step is a call of a cuda_<op>_<dtype> symbol of
-// this library with the metadata the reference's tensor layer would build; nothing here launches a kernel itself.
+// this library with the metadata the reference's tensor layer would build, but for 16-bit types' input gradient (one product without columns, where that is faster) and
+// the first two of their bias sums (one pass with the roundings of both).
 //
 // Two compositions are offered (argument `mode`):
 //
@@ -21,6 +22,8 @@
 //
 // The caller owns every buffer, as everywhere in this ABI: `cols` (B*P*K elements) is written by forward and read
 // by backward; `workspace` holds the intermediates (sizes from mx_conv2d_workspace_elems).
+#include <atomic>
+
 #include "abi_common.cuh"
 #include "matmul_tc.cuh"
 
@@ -99,13 +102,69 @@ void sum_dim(const Ops& ops, const size_t* dims, size_t nd, size_t dim, const vo
     ops.sum(n, nd, 1, meta, in, out);
 }
 
+// The first two of the bias gradient's sums, over rows and over their sums, each rounded: out[plane] = round(sum_h round(sum_w in[plane][h][w])).  A warp has a plane, G lanes a row of `nv`
+// vectors, four rows in flight.  Bound by HBM: one read of grad_out, where the sums as two launches took more than that ([64, 256, 56, 56] bf16 33 us, 26 so; rows of 14 [32, 256, 14, 14] 25 us, 4).
+constexpr int kPlaneThreads = 256;
+template <class T, int VEC, int G>
+__global__ void __launch_bounds__(kPlaneThreads) plane_sums_kernel(const T* in, T* out, size_t planes, uint32_t h, uint32_t w) {
+    after_previous_kernel();
+    constexpr int Q = 4;
+    constexpr uint32_t ROWS = 32 / G;
+    const size_t plane = (size_t)blockIdx.x * (kPlaneThreads / 32) + threadIdx.x / 32;
+    if (plane >= planes) return;
+    const uint32_t lane = threadIdx.x % 32, nv = w / VEC, rounds = (nv + G - 1) / G;
+    const T* p = in + plane * h * w;
+    float sum = 0.0f;
+    for (uint32_t r0 = lane / G; r0 - lane / G < h; r0 += Q * ROWS) {  // the same trips for every lane: the shuffles take the whole warp
+        float acc[Q];
+#pragma unroll
+        for (int q = 0; q < Q; q++) acc[q] = 0.0f;
+        for (uint32_t k = 0, v = lane % G; k < rounds; k++, v += G) {
+            Vec<T, VEC> x[Q];
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+                if (r0 + q * ROWS < h && v < nv) x[q] = *reinterpret_cast<const Vec<T, VEC>*>(p + (size_t)(r0 + q * ROWS) * w + v * VEC);
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+                if (r0 + q * ROWS < h && v < nv)
+#pragma unroll
+                    for (int j = 0; j < VEC; j++) acc[q] += to_f32(x[q].v[j]);
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < Q; q++) acc[q] += __shfl_xor_sync(0xFFFFFFFFu, acc[q], o);
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+            if (r0 + q * ROWS < h) sum += to_f32(from_f32<T>(acc[q]));
+    }
+#pragma unroll
+    for (int o = 16; o >= G; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    if (lane == 0) out[plane] = from_f32<T>(sum);
+}
+template <class T>
+void plane_sums(const Geometry& g, const void* grad_out, void* out) {
+    const bool vec = g.ow % 8 == 0 && (uintptr_t)grad_out % 16 == 0;
+    const size_t planes = g.B * g.Co, nv = vec ? g.ow / 8 : g.ow;
+    const auto kernel = vec ? (nv <= 4 ? plane_sums_kernel<T, 8, 4> : nv <= 8 ? plane_sums_kernel<T, 8, 8> : nv <= 16 ? plane_sums_kernel<T, 8, 16> : plane_sums_kernel<T, 8, 32>)
+                            : (nv <= 8 ? plane_sums_kernel<T, 1, 8> : nv <= 16 ? plane_sums_kernel<T, 1, 16> : plane_sums_kernel<T, 1, 32>);
+    launch_kernel(kernel, (unsigned)((planes + kPlaneThreads / 32 - 1) / (kPlaneThreads / 32)), kPlaneThreads, 0, ctx().stream, static_cast<const T*>(grad_out), static_cast<T*>(out), planes,
+                  (uint32_t)g.oh, (uint32_t)g.ow);
+    check_launch("mx_conv2d_backward");
+}
+
 // grad_bias = grad_out.sum(3).sum(2).sum(0) (conv.rs:283-288); tmp holds B*Co*oh + B*Co elements
 void bias_gradient(const Ops& ops, const Geometry& g, size_t es, const void* grad_out, char* tmp, void* grad_bias) {
     const size_t d4[4] = {g.B, g.Co, g.oh, g.ow}, d3[3] = {g.B, g.Co, g.oh}, d2[2] = {g.B, g.Co};
     char* t1 = tmp;
     char* t2 = tmp + round16(g.B * g.Co * g.oh) * es;
-    sum_dim(ops, d4, 4, 3, grad_out, t1);
-    sum_dim(ops, d3, 3, 2, t1, t2);
+    if (ops.half_kind && g.B * g.Co <= 0x7FFFFFFFull && g.oh <= 0x7FFFFFFFull && g.ow <= 0x7FFFFFFFull) {
+        if (ops.half_kind == 1) plane_sums<bf16>(g, grad_out, t2);
+        else plane_sums<f16>(g, grad_out, t2);
+    } else {
+        sum_dim(ops, d4, 4, 3, grad_out, t1);
+        sum_dim(ops, d3, 3, 2, t1, t2);
+    }
     sum_dim(ops, d2, 2, 0, t2, grad_bias);
 }
 
@@ -167,6 +226,27 @@ void forward(const Ops& ops, size_t es, const MxConv2d* c, int mode, const void*
     }
 }
 
+std::atomic<int> g_implicit{1};  // 0: never, 2: wherever possible (tests, A/B timing)
+
+// 16-bit types, strides of 1: the input gradient without its columns, from grad_out with the channels last and the transposed weights, both in the place of the columns.
+bool implicit_grad_x(const Ops& ops, const Geometry& g, const void* grad_out, const void* w, char* place, void* grad_x) {
+    const int mode = g_implicit.load(std::memory_order_relaxed);
+    if (!mode || !ops.half_kind || g.sh != 1 || g.sw != 1 || !conv_grad_input_fits(g.B, g.C, g.H, g.W, g.Co, g.kh, g.kw, g.ph, g.pw)) return false;
+    const size_t g_elems = (g.B * g.P * g.Co + 63) / 64 * 64;
+    char* base = reinterpret_cast<char*>(((uintptr_t)place + 127) & ~(uintptr_t)127);
+    if (g_elems + g.K * g.Co + 64 > g.B * g.K * g.P) return false;
+    // Half a tile's rows and a third of the SMs: columns / in one product, the whole backward pass and forward of a bf16 layer 3 x 3, us: 64 x 256 x 56 x 56 -> 256 1024 / 854, 64 x 64 x 7 x 7 -> 64 (64
+    // tiles) 45.2 / 41.5, 16 x 128 x 20 x 20 -> 96 (32) 43.4 / 44.5, 2 x 256 x 14 x 14 -> 256 (4) 48.8 / 58.6, 64 x 16 x 28 x 28 -> 32 58.8 / 65.7; 1 x 1: 64 x 256 x 14 x 14 -> 64 57.8 / 46.0.
+    const size_t rows = 256 / g.W < g.H ? 256 / g.W : g.H, tiles = g.B * ((g.C + 127) / 128) * ((g.H + rows - 1) / rows);
+    if (mode == 1 && (g.C < 64 || tiles * 3 < (size_t)sm_count())) return false;
+    char *last = base, *wt = base + g_elems * 2;
+    const size_t gm[7] = {g.B, g.P, g.Co, g.Co * g.P, 1, g.P, 0};
+    ops.contiguous(g.B * g.P * g.Co, 3, gm, grad_out, last);
+    const size_t wm[5] = {g.K, g.Co, 1, g.K, 0};
+    ops.contiguous(g.K * g.Co, 2, wm, w, wt);
+    return tc_conv_grad_input(ops.half_kind == 1, g.B, g.C, g.H, g.W, g.Co, g.kh, g.kw, g.ph, g.pw, g.oh, g.ow, last, wt, grad_x, "mx_conv2d_backward");
+}
+
 void backward(const Ops& ops, size_t es, const MxConv2d* c, int mode, const void* grad_out, const void* w, const void* cols, void* workspace,
               void* grad_x, void* grad_w, void* grad_bias) {
     Geometry g;
@@ -208,7 +288,7 @@ void backward(const Ops& ops, size_t es, const MxConv2d* c, int mode, const void
     char* grad_cols = ws;
     char* gw_batch = grad_cols + round16(g.B * g.K * g.P) * es;
     char* sums = gw_batch + round16(g.B * g.Co * g.K) * es;
-    if (grad_x) {
+    if (grad_x && !implicit_grad_x(ops, g, grad_out, w, grad_cols, grad_x)) {
         // grad_cols[B, K, P] = W^T (the transposed view of [Co, K], shared by every batch) . grad_out[B, Co, P]
         const size_t mm[20] = {3, 3, 3, g.B, g.K, g.P, g.B, g.K, g.Co, g.B, g.Co, g.P, 0, 1, g.K, g.Co * g.P, g.P, 1, 0, 0};
         ops.matmul(g.B * g.K * g.P, mm, w, grad_out, grad_cols);
@@ -266,5 +346,8 @@ DEF_CONV2D(bf16)
 DEF_CONV2D(f16)
 DEF_CONV2D(f32)
 DEF_CONV2D(f64)
+
+// 1 (default): a 16-bit layer's input gradient is one product without columns by the rule on its sizes; 0: never; 2: wherever possible
+void mx_debug_set_conv_implicit(int mode) { mx::g_implicit.store(mode, std::memory_order_relaxed); }
 
 }  // extern "C"

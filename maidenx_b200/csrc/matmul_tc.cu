@@ -116,6 +116,9 @@ struct TcParams {
     // tiles j, j + b_keep, ...; the B panel of the column tile is loaded once into the B slots of the ring (slot = k-block,
     // the ring is num_kb slots long) and only A streams.  0: the general schedule.
     int b_keep;
+    // CONV: the product's B is read out of images, K runs over a kernel's taps and, for each, over the channels of B's images in k-blocks (conv_cb of them); a column tile
+    // is conv_rows whole rows of an output image of width conv_w, whose source pixels for tap (i, j) begin at row + conv_y - i, column conv_x - j.
+    int conv_cb, conv_kw, conv_rows, conv_w, conv_x, conv_y;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, const TcParams& p, int& tm, int& tn, int& tb) {
@@ -240,7 +243,8 @@ enum TcMode {
 // (384 x 384 x 64) and its gradients 31.1, 29.8).
 constexpr int epi_warps(int mode, int bn_t, bool drain) { return mode == TC_PLAIN || (mode == TC_BIAS && !bn_t && !drain) ? 2 : 1; }
 constexpr int tc_threads(int w) { return 32 * (2 + 4 * w); }
-template <int MODE, int BN_T, bool DRAIN = false, bool PANELS = false>
+// CONV (TC_PLAIN): TcParams::conv_*; an instantiation of its own for the producer's sake too.
+template <int MODE, int BN_T, bool DRAIN = false, bool PANELS = false, bool CONV = false>
 __global__ void __launch_bounds__(tc_threads(epi_warps(MODE, BN_T, DRAIN)), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                const __grid_constant__ CUtensorMap map_d2, TcParams p, int* err, int tag) {
@@ -298,13 +302,31 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const int za = p.a_batched ? tb : 0, zb = p.b_batched ? tb : 0;
                 int k = tb * p.split_kb * BK;              // a k-block past the end of K is all fill: zeros
                 const bool load_b = PANELS ? tm == 0 || it == 0 : !p.b_keep || it == 0;  // a kept B panel arrives with its first tile's A blocks
+                int cb = 0, ki = 0, kj = 0;  // CONV: k-block of the channels, tap
                 for (int kb = 0; kb < p.num_kb; kb++, k += BK) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, err, tag, 1)) {
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(full_bar(stage), A_STAGE_BYTES + (load_b ? bn * BK * 2 : 0));
                     const uint32_t sa = smem_base + SmemLayout::ring + stage * stage_bytes, sb = sa + A_STAGE_BYTES;
+                    if constexpr (CONV) {  // what lies outside an image, or behind the last channel of either operand, arrives as zeros
+                        mbar_expect_tx(full_bar(stage), A_STAGE_BYTES + p.conv_rows * p.conv_w * BK * 2);
+                        tma_load_3d(sa, &map_a, cb * BK, ki * p.conv_kw + kj, tm * BM, full_bar(stage));
+                        tma_load_4d(sb, &map_b, cb * BK, p.conv_x - kj, tn * p.conv_rows + p.conv_y - ki, tb, full_bar(stage));
+                        if (++cb == p.conv_cb) {
+                            cb = 0;
+                            if (++kj == p.conv_kw) {
+                                kj = 0;
+                                ki++;
+                            }
+                        }
+                        if (++stage == ring) {
+                            stage = 0;
+                            phase ^= 1;
+                        }
+                        continue;
+                    }
+                    mbar_expect_tx(full_bar(stage), A_STAGE_BYTES + (load_b ? bn * BK * 2 : 0));
                     if (!p.a_mn) {
                         tma_load_3d(sa, &map_a, k, tm * BM, za, full_bar(stage));
                     } else {
@@ -435,8 +457,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         tma_store_commit();
                     }
                 } else {
-                    store_rows(static_cast<uint16_t*>(p.d) + ((size_t)tb * p.M + tm * BM + quarter * 32) * p.N + tn * bn, (size_t)p.N, half * 16, rows_here,
-                               min(bn, p.N - tn * bn), (col - tn * bn) / 64, src, stage_buf + buf * EPI_STAGE_BYTES, lane);
+                    const int width = CONV ? p.conv_rows * p.conv_w : bn;  // columns from one tile to the next
+                    store_rows(static_cast<uint16_t*>(p.d) + ((size_t)tb * p.M + tm * BM + quarter * 32) * p.N + tn * width, (size_t)p.N, half * 16, rows_here,
+                               min(width, p.N - tn * width), (col - tn * bn) / 64, src, stage_buf + buf * EPI_STAGE_BYTES, lane);
                 }
             };
             auto pack = [&](const float (&e)[CW], uint4 (&q)[CW / 8]) {
@@ -499,7 +522,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if constexpr (CW > 32) reg_fence(v[CW / 32 - 1]);
             };
             // The TMEM loads of chunk c + 1 are in flight while chunk c is converted and stored.
-            const int chunks = bn / EPI_CHUNK_COLS;
+            const int chunks = CONV ? (bn + EPI_CHUNK_COLS - 1) / EPI_CHUNK_COLS : bn / EPI_CHUNK_COLS;
             auto hand_back = [&] {  // every TMEM read of this accumulator is done: hand it back to the MMA warp
                 tc_fence_before();
                 __syncwarp();
@@ -593,7 +616,8 @@ bool opt_in_shared_memory() {
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
         for (auto kernel : {tc_gemm_kernel<TC_STORE, BN>, tc_gemm_kernel<TC_BIAS, BN>, tc_gemm_kernel<TC_STORE, 0>, tc_gemm_kernel<TC_BIAS, 0>, tc_gemm_kernel<TC_PLAIN, 0>, tc_gemm_kernel<TC_STORE, BN, false, true>, tc_gemm_kernel<TC_BIAS, BN, false, true>,
-                            tc_gemm_kernel<TC_STORE, 0, true>, tc_gemm_kernel<TC_BIAS, 0, true>, tc_gemm_kernel<TC_PLAIN, 0, true>})
+                            tc_gemm_kernel<TC_STORE, 0, true>, tc_gemm_kernel<TC_BIAS, 0, true>, tc_gemm_kernel<TC_PLAIN, 0, true>,
+                            tc_gemm_kernel<TC_PLAIN, 0, false, false, true>})
             if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
@@ -1354,6 +1378,65 @@ bool tc_batched_row_bias(bool is_bf16, uint64_t batch, uint64_t rows, uint64_t k
     if (!eligible(2, c.m, c.n, c.k, batch, false, true, w, cols, out) && !plan_ragged(2, c, out)) return false;
     StreamWorkspace ws;
     return repack_operands(2, c, ws, where) && launch_gemm(is_bf16, c, out, where, 3, bias, nullptr);
+}
+
+// Rows of whole output images in at most 256 columns of a tile, channels that tensor maps can describe, sizes that the kernel indexes in 32 bits.
+bool conv_grad_input_fits(uint64_t batch, uint64_t c, uint64_t h, uint64_t w, uint64_t co, uint64_t kh, uint64_t kw, uint64_t ph, uint64_t pw) {
+    return batch && c && h && w && co && kh && kw && w <= 256 && co % 8 == 0 && batch <= 0x7FFF && h * w <= 0x3FFFFFFF && c <= 0x3FFFFFFF && kh * kw * ((co + BK - 1) / BK) <= 0xFFFF && ph <= 0x7FFF &&
+           pw <= 0x7FFF && batch * ((c + BM - 1) / BM) * h <= 0x3FFFFFFF;
+}
+// The gradient of a convolution's input, strides of 1: grad_x[b][c] = sum over taps (i, j) and output channels o of w[o][c][i][j] grad_out[b][o] shifted by the tap.  `g` holds
+// grad_out with the channels last, `wt` the weights as [c][tap][o]: then every tap is a product whose second operand is a box of neighbouring pixels, zeros outside
+// the image, and all of them are one reduction in the f32 accumulator.  No column matrix is written and read, and nothing is rounded on the way.
+bool tc_conv_grad_input(bool is_bf16, uint64_t batch, uint64_t c, uint64_t h, uint64_t w, uint64_t co, uint64_t kh, uint64_t kw, uint64_t ph, uint64_t pw, uint64_t oh, uint64_t ow,
+                        const void* g, const void* wt, void* grad_x, const char* where) {
+    if (!conv_grad_input_fits(batch, c, h, w, co, kh, kw, ph, pw) || ((uintptr_t)g | (uintptr_t)wt) % 16 != 0 || (uintptr_t)grad_x % 2 != 0 || !opt_in_shared_memory()) return false;
+    TcParams p = {};
+    const uint64_t blocks = (h + 256 / w - 1) / (256 / w);
+    p.conv_rows = (int)((h + blocks - 1) / blocks);
+    p.conv_w = (int)w;
+    p.conv_kw = (int)kw;
+    p.conv_cb = (int)((co + BK - 1) / BK);
+    p.conv_x = (int)pw;
+    p.conv_y = (int)ph;
+    p.M = (int)c;
+    p.N = (int)(h * w);
+    p.num_kb = (int)(kh * kw) * p.conv_cb;
+    p.K = p.num_kb * BK;
+    p.bn = (p.conv_rows * p.conv_w + 15) / 16 * 16;
+    p.tiles_m = (int)((c + BM - 1) / BM);
+    p.tiles_n = (int)((h + p.conv_rows - 1) / p.conv_rows);
+    p.tiles_per_batch = p.tiles_m * p.tiles_n;
+    p.num_tiles = (int)batch * p.tiles_per_batch;
+    p.a_batched = p.b_batched = 1;
+    p.is_bf16 = is_bf16 ? 1 : 0;
+    p.group_m = g_group_m.load(std::memory_order_relaxed);
+    p.stages = ring_stages(p.bn);
+    p.stage_bytes = A_STAGE_BYTES + p.bn * BK * 2;
+    p.d_plain = 1;
+    p.d = grad_x;
+    int tag = 0;
+    int* err = next_launch_error_word(&tag);
+    EncodeTiledFn enc = encode_fn();
+    if (!err || !enc) return false;
+    const CUtensorMapDataType t16 = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    auto encode = [&](CUtensorMap& map, const void* base, int rank, const cuuint64_t* dims, const cuuint32_t* box) {  // dense
+        cuuint64_t strides[3];
+        const cuuint32_t ones[4] = {1, 1, 1, 1};
+        for (int i = 0; i + 1 < rank; i++) strides[i] = (i ? strides[i - 1] : 2) * dims[i];
+        return enc(&map, t16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    CUtensorMap ma, mb;
+    const cuuint64_t a_dims[3] = {co, kh * kw, c}, b_dims[4] = {co, ow, oh, batch};
+    const cuuint32_t a_box[3] = {BK, 1, BM}, b_box[4] = {BK, (cuuint32_t)w, (cuuint32_t)p.conv_rows, 1};
+    if (!encode(ma, wt, 3, a_dims, a_box) || !encode(mb, g, 4, b_dims, b_box)) return false;
+    int grid = sm_count();
+    if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
+    if (grid > p.num_tiles) grid = p.num_tiles;
+    launch_kernel(tc_gemm_kernel<TC_PLAIN, 0, false, false, true>, grid, tc_threads(epi_warps(TC_PLAIN, 0, false)), TC_SMEM_BYTES, ctx().stream, ma, mb, ma, ma, p, err, tag);
+    check_launch(where);
+    return true;
 }
 
 bool tc_batch_sum_f32(uint64_t batch, uint64_t m, uint64_t n, uint64_t k, const float* a, const float* b, float* out, const char* where) {

@@ -51,6 +51,11 @@ bool tc_batched_row_bias(bool is_bf16, uint64_t batch, uint64_t rows, uint64_t k
 // out[m, n] = sum_b a[b][m, k] . b[b][n, k]^T over the whole batch in one reduction: the weight gradient of a convolution.
 // false = not taken (rows of k or n that are not 16-byte multiples, a small product).
 bool tc_batch_sum_f32(uint64_t batch, uint64_t m, uint64_t n, uint64_t k, const float* a, const float* b, float* out, const char* where);
+// The gradient of a convolution's input in one product, strides of 1, 16-bit types: g = grad_out as [batch][oh][ow][co], wt = the weights as [c][kh * kw][co].
+// false: not taken, nothing launched.
+bool conv_grad_input_fits(uint64_t batch, uint64_t c, uint64_t h, uint64_t w, uint64_t co, uint64_t kh, uint64_t kw, uint64_t ph, uint64_t pw);
+bool tc_conv_grad_input(bool is_bf16, uint64_t batch, uint64_t c, uint64_t h, uint64_t w, uint64_t co, uint64_t kh, uint64_t kw, uint64_t ph, uint64_t pw, uint64_t oh, uint64_t ow,
+                        const void* g, const void* wt, void* grad_x, const char* where);
 bool tc_launch_f32(const TcProduct& c, void* out, const char* where);
 // The product in pairs of f16 (matmul_tc_pairs.cu), if that is estimated to take less than `tf32_us`.  true: launched, and whoever called runs the product behind
 // `gate`, which is open when an operand was not fit for pairs and lies in `ws`; false: nothing launched.

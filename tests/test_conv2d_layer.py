@@ -178,3 +178,38 @@ def test_direct_layer_on_ragged_maps(cuda, dt, shape):
     sc = _scales(shape)
     for key in ("out", "grad_x", "grad_w", "grad_bias"):
         H.assert_same("conv2d", dt, got[key], D.encode(ref[key], dt), float_rel={"f32": 1e-5}.get(dt.name, 2e-2), what=key, scale=sc[key])
+
+
+# input channels beyond and below a tile's 128 rows, maps of one and of several row blocks a tile, widths that leave columns of the tile unused, output channels that end inside a k-block,
+# kernels that are not square, paddings from none to more than the kernel's half, output maps larger and smaller than the input
+IMPLICIT = [
+    (3, 64, 14, 14, 72, 3, 3, 1, 1, 1, 1), (2, 130, 9, 31, 64, 3, 3, 1, 1, 1, 1), (5, 8, 7, 7, 8, 5, 5, 1, 1, 2, 2), (2, 200, 28, 28, 136, 3, 3, 1, 1, 1, 1), (1, 64, 17, 130, 136, 1, 3, 1, 1, 0, 1),
+    (2, 72, 12, 20, 64, 4, 2, 1, 1, 3, 0), (2, 64, 10, 10, 24, 3, 3, 1, 1, 0, 0), (1, 65, 5, 256, 16, 2, 2, 1, 1, 1, 1), (40, 128, 7, 7, 72, 3, 3, 1, 1, 1, 1), (1, 64, 33, 56, 64, 7, 7, 1, 1, 3, 3),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("shape", IMPLICIT, ids=lambda s: "x".join(map(str, s)))
+def test_input_gradient_without_columns(cuda, dt, shape):
+    """One product over taps and channels: next to float64 one rounding of an f32 sum (half a step of the type, and 2^-22 of the sums' scale for the sum itself), and no further off than the columns'
+    form, which rounds each of them; nothing else of the layer changes."""
+    from maidenx_b200 import _lib
+    lib = _lib.load()
+    x, w, b, g = _data(16, dt, shape)
+    ref = CC.direct_conv_f64(shape, D.decode(x, dt), D.decode(w, dt), D.decode(b, dt), D.decode(g, dt))
+    got = {}
+    for mode in (0, 2, 1):
+        lib.mx_debug_set_conv_implicit(mode)
+        try:
+            got[mode] = CC.run_layer(dt, 1, shape, x, w, b, g)
+        finally:
+            lib.mx_debug_set_conv_implicit(1)
+    for key in ("out", "grad_w", "grad_bias", "cols"):
+        assert np.array_equal(got[0][key], got[2][key]), key
+    want = ref["grad_x"].reshape(-1)
+    err = {m: np.linalg.norm(D.decode(got[m]["grad_x"], dt) - want) for m in got}
+    assert err[2] <= err[0] * 1.0001 and err[1] <= err[0] * 1.0001
+    step = 2.0 ** -9 if dt is D.BF16 else 2.0 ** -12
+    terms = shape[4] * shape[5] * shape[6]
+    assert np.all(np.abs(D.decode(got[2]["grad_x"], dt) - want) <= 1.001 * step * 2 * np.abs(want) + 2.0 ** -20 * _scales(shape)["grad_x"] * np.sqrt(terms) + 1e-7)
