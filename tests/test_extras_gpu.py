@@ -317,3 +317,37 @@ def test_softmax_of_ragged_rows_and_of_columns_in_registers(oracle, cuda, dt):
             assert np.all(np.abs(got - ref) <= tol * np.maximum(np.abs(ref), floor)), (dims, off, np.abs(got / np.maximum(ref, 1e-30) - 1).max())
     finally:
         oracle.b.set_wide(False)
+
+
+@pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("rows,n,off", [(5, 1, 0), (301, 3, 1), (1000, 15, 0), (700, 17, 1), (500, 31, 0), (400, 33, 1), (400, 63, 0), (19000, 65, 1), (19001, 127, 0), (19000, 159, 1), (19003, 197, 0),
+                                        (18999, 255, 0), (3700, 257, 1), (3701, 383, 0), (3702, 511, 1), (9, 513, 0), (1200, 1021, 1)], ids=str)
+def test_softmax_of_ragged_rows_by_words(cuda, dt, rows, n, off):
+    """16-bit rows by the 4-byte words they lie in, at even and odd places, around the words a lane takes and the lanes a row takes: next to float64 with one rounding; -inf at a row's ends, a row of
+    nothing else, +inf and NaN stay in their rows; elements before and behind the output stay as they were."""
+    from maidenx_b200 import device
+    rng = np.random.default_rng(rows + n)
+    x = rng.standard_normal((rows, n)) * 3.0
+    if n > 1:
+        x[0, 0] = x[1, n - 1] = -np.inf
+        x[2] = -np.inf
+        x[3, n // 2] = np.inf
+        x[4, 1] = np.nan
+    enc = D.encode(np.concatenate([np.full(off, 50.0), x.reshape(-1)]), dt)  # what lies before the first row is large
+    fill = np.full(rows * n + off + 4, 0x1234, np.uint16)
+    src, dst = device.CudaBuffer.from_host(enc), device.CudaBuffer.from_host(fill)
+    device.dispatch("softmax", dt.name, [rows, n, n, 1, off], rows * n, 2, 1, "META", src.ptr, dst.ptr + 2 * off)
+    raw = dst.to_host(np.uint16, fill.size)
+    src.free(), dst.free()
+    assert (raw[:off] == 0x1234).all() and (raw[off + rows * n:] == 0x1234).all()
+    got = D.decode(raw[off:off + rows * n].view(dt.np_storage), dt).astype(np.float64).reshape(rows, n)
+    v = D.decode(enc[off:], dt).astype(np.float64).reshape(rows, n)
+    with np.errstate(all="ignore"):
+        e = np.exp(v - v.max(axis=1, keepdims=True))
+        ref = e / e.sum(axis=1, keepdims=True)
+    if n > 1:
+        assert np.isnan(got[2]).all() and np.isnan(got[4]).all() and np.isnan(got[3, n // 2]) and np.isfinite(got[5:]).all()
+    keep = [r for r in range(rows) if n == 1 or r not in (2, 3, 4)]
+    step = 2.0 ** -8 if dt is D.BF16 else 2.0 ** -11
+    least = 0.0 if dt is D.BF16 else 2.0 ** -25  # half a step of the smallest f16
+    assert np.all(np.abs(got - ref)[keep] <= 1.01 * step * ref[keep] + least + 1e-38)
