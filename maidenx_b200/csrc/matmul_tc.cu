@@ -704,22 +704,30 @@ bool launch_two_cta(bool is_bf16, const TcProduct& c, void* D, const char* where
 int ring_stages(int bn) { return std::min(MAX_STAGES, STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) / (A_STAGE_BYTES + bn * BK * 2)); }
 // k-blocks of tensor-core time (M128 N256 K64: 512 cycles) that one k-block of a bn-wide tile takes: the columns' share; the
 // operand reads from shared memory (a k-step of N64 needs 48 cycles for its 6 KB, 32 for its multiplications); or the ring, whose
-// stages all wait out one round trip to L2 of about 1.2 us.
-double kb_cost(int bn) { return std::max(std::max(bn / 256.0, (128 + bn) / 512.0), 4.4 / ring_stages(bn)); }
+// stages all wait out one round trip to L2 of about 1.2 us.  The four stages of 192 columns do not: measured, 0.212 us a k-block
+// against 0.306 of a 256-wide tile, 0.27 with B MN-major (a copy for each 64 columns); 128 columns 0.200.
+double kb_cost(int bn, bool b_mn) {
+    if (bn == 192) return b_mn ? 0.87 : 0.70;
+    if (bn == 128 && !b_mn) return 0.65;
+    return std::max(std::max(bn / 256.0, (128 + bn) / 512.0), 4.4 / ring_stages(bn));
+}
 // Columns of an output tile.  256 feeds the tensor core best, so narrower tiles are for products that 256-wide tiles serve
 // badly: an N that fills its last tile poorly (N = 64 would compute 256 columns, N = 384 512) or too few tiles to reach every
 // SM.  The estimate is in k-blocks of a 256-wide tile: a wave's reduction, and its epilogue in proportion to the columns.
-// From two waves of 256-wide tiles on only the columns count: at the power cap a part-filled last wave costs nothing.
-// bf16 512 x 1024 x 1024 (64 tiles of 64 columns instead of 16): 8.7 us, 10.0 on full-width tiles.
-double tile_cost(int bn, uint64_t tiles_m, uint64_t N, uint64_t batch, uint64_t num_kb, int grid) {
+// From two waves of 256-wide tiles on only the columns count, and all that narrow tiles load besides: at the power cap a
+// part-filled last wave costs nothing (12856 x 2856 x 760 58 us, 65 on tiles of 192).
+// bf16 512 x 1024 x 1024 (64 tiles of 64 columns instead of 16): 8.7 us, 10.0 on full-width tiles;
+// 4096 x 1536 x 1024 (256 of 192 columns instead of 192) 13.1, 15.4; 2432 x 1008 x 1504 with B MN-major 11.6, 15.3.
+double tile_cost(int bn, bool b_mn, uint64_t tiles_m, uint64_t N, uint64_t batch, uint64_t num_kb, int grid) {
     const uint64_t tiles = tiles_m * ((N + bn - 1) / bn) * batch, tiles_256 = tiles_m * ((N + 255) / 256) * batch;
-    const double waves = tiles_256 > 2 * (uint64_t)grid ? (double)tiles / grid : (double)((tiles + grid - 1) / grid);
-    return waves * ((double)num_kb * kb_cost(bn) + 3.0 * bn / 256.0);
+    const double epilogue = 3.0 * bn / 256.0;
+    if (tiles_256 > 2 * (uint64_t)grid) return (double)tiles / grid * ((double)num_kb * std::max((128 + bn) / 512.0, 4.4 / ring_stages(bn)) + epilogue);
+    return (double)((tiles + grid - 1) / grid) * ((double)num_kb * kb_cost(bn, b_mn) + epilogue);
 }
-int tile_columns(uint64_t tiles_m, uint64_t N, uint64_t batch, uint64_t num_kb, int grid) {
+int tile_columns(bool b_mn, uint64_t tiles_m, uint64_t N, uint64_t batch, uint64_t num_kb, int grid) {
     int best = 256;
     for (int bn : {192, 128, 64})
-        if (tile_cost(bn, tiles_m, N, batch, num_kb, grid) < 0.93 * tile_cost(best, tiles_m, N, batch, num_kb, grid)) best = bn;
+        if (tile_cost(bn, b_mn, tiles_m, N, batch, num_kb, grid) < 0.93 * tile_cost(best, b_mn, tiles_m, N, batch, num_kb, grid)) best = bn;
     return best;
 }
 
@@ -749,13 +757,13 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
     p.b_keep = keep_b_ctas(p.tiles_m, p.tiles_n, p.num_kb, (int)batch, std::min(grid, (int)std::min<uint64_t>(batch * p.tiles_m * p.tiles_n, 1u << 30)));
     // few output tiles: cut K into slices that run as the batches of this launch
     int slices = 1;
-    const int bn_whole = p.b_keep ? p.bn : tile_columns((uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid);
+    const int bn_whole = p.b_keep ? p.bn : tile_columns(b_mn, (uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid);
     const bool panels = p.bn == BN && bn_whole == BN && !c.d_plain && keep_panels((uint64_t)p.tiles_m, (uint64_t)p.tiles_n, p.num_kb, batch, c.a_bs == 0, grid);
     if (batch == 1 && !fuse && !p.b_keep) {
         slices = splitk_slices((uint64_t)p.tiles_m * p.tiles_n, K, BK, grid);
         if (slices == 1)
-            slices = splitk_short((uint64_t)p.tiles_m * p.tiles_n, (uint64_t)p.num_kb, grid, kb_cost(p.bn),
-                                  tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid) - kSplitFixed16);
+            slices = splitk_short((uint64_t)p.tiles_m * p.tiles_n, (uint64_t)p.num_kb, grid, kb_cost(p.bn, b_mn),
+                                  tile_cost(bn_whole, b_mn, (uint64_t)p.tiles_m, N, batch, (uint64_t)p.num_kb, grid) - kSplitFixed16);
     }
     StreamWorkspace partial;
     const uint64_t n_pitch = (N + 3) / 4 * 4;
