@@ -83,6 +83,70 @@ __device__ __forceinline__ float gelu_grad_f32(float x) {
     return fmaf(er * r * x, fmaf(c2, x2, c1), x < 0.0f ? er : r);
 }
 
+// Two elements at a time: multiplications and additions in the packed form (each half rounds as the scalar instruction does), which halves what the kernel
+// issues.  At the clocks that the products around it leave under the power cap the issue slots, not HBM, bounded it: 16384 x 8192 bf16
+// with its sum, behind two products of that size, 222 us by single instructions, 172 so (alone 148 and 131; at 6553 GB/s 123).  f32 elements, half as many a byte, are at HBM's rate as they are.
+struct Pair {
+    unsigned long long v;
+};
+__device__ __forceinline__ Pair make_pair(float lo, float hi) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ Pair both(float v) { return make_pair(v, v); }
+__device__ __forceinline__ float2 halves(Pair p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p.v));
+    return r;
+}
+__device__ __forceinline__ Pair operator*(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Pair operator+(Pair a, Pair b) {
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ Pair gelu_grad_pair(float2 x) {
+    const float k1 = -2.302208198f, k2 = -0.102943240f, c1 = 1.5957691216f, c2 = 0.2140644488f;
+    const Pair xx = make_pair(x.x, x.y), x2 = xx * xx;
+    const float2 k = halves(fma2(both(k2), x2, both(k1)));
+    float2 e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(fabsf(x.x) * k.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(fabsf(x.y) * k.y));
+    const Pair ep = make_pair(e.x, e.y);
+    const float2 d = halves(both(1.0f) + ep);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
+    const Pair rp = make_pair(r.x, r.y), er = ep * rp;
+    const float2 s = halves(er);
+    return fma2(er * rp * xx, fma2(both(c2), x2, both(c1)), make_pair(x.x < 0.0f ? s.x : r.x, x.y < 0.0f ? s.y : r.y));
+}
+
+// Elements 2 i and 2 i + 1 of a vector of a 16-bit type as f32, and back with one rounding each.
+template <class T, int VEC>
+__device__ __forceinline__ float2 pair_of(const Vec<T, VEC>& v, int i) {
+    if constexpr (std::is_same<T, bf16>::value) {
+        const uint32_t w = reinterpret_cast<const uint32_t*>(&v)[i];
+        return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+    } else {
+        return __half22float2(reinterpret_cast<const __half2*>(&v)[i]);
+    }
+}
+template <class T, int VEC>
+__device__ __forceinline__ void set_pair(Vec<T, VEC>& v, int i, float2 x) {
+    if constexpr (std::is_same<T, bf16>::value) reinterpret_cast<__nv_bfloat162*>(&v)[i] = __float22bfloat162_rn(x);
+    else reinterpret_cast<__half2*>(&v)[i] = __float22half2_rn(x);
+}
+
 // The block's sum of v; valid in thread 0.
 __device__ __forceinline__ float fused_block_sum(float v) {
     __shared__ float warp_part[kFusedThreads / 32];
@@ -111,12 +175,13 @@ __device__ __forceinline__ bool fused_last_block(uint32_t* arrived) {
 }
 
 // SUM: the sum of du (the bias gradient), which a pass over du used to read it back for.  Two vectors of each operand in flight
-// per thread.
+// per thread.  Registers for five blocks: the pairs without the bound took 58 and four blocks (2^24 f16 16.2 us, 15.2 so).
 template <class T, bool SUM>
-__global__ void __launch_bounds__(kFusedThreads) gelu_backward_kernel(const T* dy, const T* u, T* du,
+__global__ void __launch_bounds__(kFusedThreads, is_half_v<T> || SUM ? 5 : 6) gelu_backward_kernel(const T* dy, const T* u, T* du,
                                                                      uint64_t n, float* partial, uint32_t* arrived, T* grad_sum) {
     after_previous_kernel();
     float acc = 0.0f;
+    Pair sums = both(0.0f);
     constexpr int VEC = 16 / sizeof(T), UN = 2;
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
@@ -132,14 +197,27 @@ __global__ void __launch_bounds__(kFusedThreads) gelu_backward_kernel(const T* d
         for (int i = 0; i < UN; i++)
             if (v0 + i * stride < nvec) {
                 Vec<T, VEC> o;
+if constexpr (is_half_v<T>) {
 #pragma unroll
-                for (int j = 0; j < VEC; j++) {
-                    o.v[j] = st_from_f32<T>(up(g[i].v[j]) * gelu_grad_f32(up(x[i].v[j])));
-                    if (SUM) acc += up(o.v[j]);
+                    for (int j = 0; j < VEC / 2; j++) {
+                        const float2 gj = pair_of(g[i], j);
+                        set_pair(o, j, halves(make_pair(gj.x, gj.y) * gelu_grad_pair(pair_of(x[i], j))));
+                        if (SUM) {
+                            const float2 oj = pair_of(o, j);
+                            sums = sums + make_pair(oj.x, oj.y);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < VEC; j++) {
+                        o.v[j] = g[i].v[j] * gelu_grad_f32(x[i].v[j]);
+                        if (SUM) acc += o.v[j];
+                    }
                 }
                 *reinterpret_cast<Vec<T, VEC>*>(du + (v0 + i * stride) * VEC) = o;
             }
     }
+    acc += halves(sums).x + halves(sums).y;
     if (blockIdx.x == 0)
         for (uint64_t i = nvec * VEC + threadIdx.x; i < n; i += kFusedThreads) {
             du[i] = st_from_f32<T>(up(dy[i]) * gelu_grad_f32(up(u[i])));

@@ -96,6 +96,29 @@ def test_fused_passes_match_the_single_op_chain(cuda):
     assert device.last_error() is None
 
 
+@pytest.mark.parametrize("n", [1, 7, 8, 4103, 400_006])
+@pytest.mark.parametrize("dt", [D.BF16, D.F16])
+def test_gelu_backward_by_pairs(cuda, dt, n):
+    """16-bit elements are taken two at a time, what is behind the last vector one at a time, with the same results: the derivative in f32 (error below 4e-6: the exponent's
+    rounding, 2^-23 of at most 16 where the sigmoid's derivative is not negligible, and the approximate exp2 and reciprocal), one rounding at the end."""
+    lib = _lib.load()
+    rng = np.random.default_rng(n)
+    u, dy = D.encode(rng.uniform(-12, 12, n).astype(np.float32), dt), D.encode(rng.standard_normal(n).astype(np.float32), dt)
+    ub, dyb, dub = device.CudaBuffer.from_host(np.resize(u, n + 8)), device.CudaBuffer.from_host(np.resize(dy, n + 8)), device.CudaBuffer.from_host(np.full(n + 8, 0x1234, np.uint16))
+    (lib.mx_gelu_backward_bf16 if dt == D.BF16 else lib.mx_gelu_backward_f16)(n, dyb.ptr, ub.ptr, dub.ptr)
+    device.synchronize()
+    out = dub.to_host(np.uint16, n + 8)
+    u64, dy64 = D.decode(u, dt).astype(np.float64), D.decode(dy, dt).astype(np.float64)
+    want, got = dy64 * gelu_grad64(u64), D.decode(out[:n].view(u.dtype), dt)
+    half_ulp, smallest = (2.0 ** -8, 2.0 ** -134) if dt == D.BF16 else (2.0 ** -11, 2.0 ** -25)
+    # half_ulp: the relative rounding of 8 (bf16) and 11 (f16) significant bits
+    bound = (np.abs(want) + 4e-6 * np.abs(dy64)) * half_ulp + 4e-6 * np.abs(dy64) + smallest
+    assert np.all(np.abs(got - want) <= bound) and np.all(out[n:] == 0x1234)
+    for x in (ub, dyb, dub):
+        x.free()
+    assert device.last_error() is None
+
+
 def test_one_training_step_matches_f64_model(cuda):
     from maidenx_b200.mlp import Mlp
     L, Dm, B, seed, lr = 3, 256, 512, 6, 0.05
