@@ -11,6 +11,7 @@
 // All are HBM-bound: 16-byte vector accesses, four vectors in flight per thread, math in f32,
 // one rounding per stored value.
 #include "fused.cuh"
+#include "f32x2.cuh"
 #include "abi_common.cuh"
 #include "ops.cuh"
 #include "matmul_tc.cuh"
@@ -86,65 +87,26 @@ __device__ __forceinline__ float gelu_grad_f32(float x) {
 // Two elements at a time: multiplications and additions in the packed form (each half rounds as the scalar instruction does), which halves what the kernel
 // issues.  At the clocks that the products around it leave under the power cap the issue slots, not HBM, bounded it: 16384 x 8192 bf16
 // with its sum, behind two products of that size, 222 us by single instructions, 172 so (alone 148 and 131; at 6553 GB/s 123).  f32 elements, half as many a byte, are at HBM's rate as they are.
-struct Pair {
-    unsigned long long v;
-};
-__device__ __forceinline__ Pair make_pair(float lo, float hi) {
-    Pair r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ Pair both(float v) { return make_pair(v, v); }
-__device__ __forceinline__ float2 halves(Pair p) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p.v));
-    return r;
-}
-__device__ __forceinline__ Pair operator*(Pair a, Pair b) {
-    Pair r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ Pair operator+(Pair a, Pair b) {
-    Pair r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
-    Pair r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-__device__ __forceinline__ Pair gelu_grad_pair(float2 x) {
+__device__ __forceinline__ F32x2 gelu_grad_pair(float2 x) {
     const float k1 = -2.302208198f, k2 = -0.102943240f, c1 = 1.5957691216f, c2 = 0.2140644488f;
-    const Pair xx = make_pair(x.x, x.y), x2 = xx * xx;
-    const float2 k = halves(fma2(both(k2), x2, both(k1)));
+    const F32x2 xx = pair_of(x), x2 = xx * xx;
+    const float2 k = halves(fma2(twice(k2), x2, twice(k1)));
     float2 e, r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(fabsf(x.x) * k.x));
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(fabsf(x.y) * k.y));
-    const Pair ep = make_pair(e.x, e.y);
-    const float2 d = halves(both(1.0f) + ep);
+    const F32x2 ep = pair_of(e);
+    const float2 d = halves(twice(1.0f) + ep);
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d.x));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
-    const Pair rp = make_pair(r.x, r.y), er = ep * rp;
+    const F32x2 rp = pair_of(r), er = ep * rp;
     const float2 s = halves(er);
-    return fma2(er * rp * xx, fma2(both(c2), x2, both(c1)), make_pair(x.x < 0.0f ? s.x : r.x, x.y < 0.0f ? s.y : r.y));
+    return fma2(er * rp * xx, fma2(twice(c2), x2, twice(c1)), pair_of(make_float2(x.x < 0.0f ? s.x : r.x, x.y < 0.0f ? s.y : r.y)));
 }
 
-// Elements 2 i and 2 i + 1 of a vector of a 16-bit type as f32, and back with one rounding each.
+// The 32-bit words of a vector of 16-bit elements.
 template <class T, int VEC>
-__device__ __forceinline__ float2 pair_of(const Vec<T, VEC>& v, int i) {
-    if constexpr (std::is_same<T, bf16>::value) {
-        const uint32_t w = reinterpret_cast<const uint32_t*>(&v)[i];
-        return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
-    } else {
-        return __half22float2(reinterpret_cast<const __half2*>(&v)[i]);
-    }
-}
-template <class T, int VEC>
-__device__ __forceinline__ void set_pair(Vec<T, VEC>& v, int i, float2 x) {
-    if constexpr (std::is_same<T, bf16>::value) reinterpret_cast<__nv_bfloat162*>(&v)[i] = __float22bfloat162_rn(x);
-    else reinterpret_cast<__half2*>(&v)[i] = __float22half2_rn(x);
+__device__ __forceinline__ uint32_t* words(Vec<T, VEC>& v) {
+    return reinterpret_cast<uint32_t*>(&v);
 }
 
 // The block's sum of v; valid in thread 0.
@@ -181,7 +143,7 @@ __global__ void __launch_bounds__(kFusedThreads, is_half_v<T> || SUM ? 5 : 6) ge
                                                                      uint64_t n, float* partial, uint32_t* arrived, T* grad_sum) {
     after_previous_kernel();
     float acc = 0.0f;
-    Pair sums = both(0.0f);
+    F32x2 sums = twice(0.0f);
     constexpr int VEC = 16 / sizeof(T), UN = 2;
     const uint64_t nvec = n / VEC;
     const uint64_t stride = (uint64_t)gridDim.x * kFusedThreads;
@@ -200,12 +162,9 @@ __global__ void __launch_bounds__(kFusedThreads, is_half_v<T> || SUM ? 5 : 6) ge
 if constexpr (is_half_v<T>) {
 #pragma unroll
                     for (int j = 0; j < VEC / 2; j++) {
-                        const float2 gj = pair_of(g[i], j);
-                        set_pair(o, j, halves(make_pair(gj.x, gj.y) * gelu_grad_pair(pair_of(x[i], j))));
-                        if (SUM) {
-                            const float2 oj = pair_of(o, j);
-                            sums = sums + make_pair(oj.x, oj.y);
-                        }
+                        const float2 r = halves(pair_of(unpack2<T>(words(g[i])[j])) * gelu_grad_pair(unpack2<T>(words(x[i])[j])));
+                        words(o)[j] = pack2_rn<T>(r.x, r.y);
+                        if (SUM) sums = sums + pair_of(unpack2<T>(words(o)[j]));
                     }
                 } else {
 #pragma unroll

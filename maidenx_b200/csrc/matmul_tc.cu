@@ -2,7 +2,7 @@
 // tensor memory (TMEM), operands staged in shared memory by TMA, epilogue read back with
 // tcgen05.ld, converted and written with TMA stores.
 //
-// One persistent CTA per SM, 192 threads (320 where the warps write the rows themselves) in three roles:
+// One persistent CTA per SM, 192 threads (320 where the warps write the rows themselves or add a bias) in three roles:
 //   warp 0      TMA producer: one lane issues cp.async.bulk.tensor loads of the A [128 x 64]
 //               and B [64 to 256 x 64] k-blocks into a shared-memory ring (128-byte swizzle) of four
 //               stages, up to eight of narrower tiles;
@@ -33,6 +33,7 @@
 #include <mutex>
 #include <unordered_map>
 
+#include "f32x2.cuh"
 #include "matmul_tc.cuh"
 #include "matmul_tc2.cuh"
 #include "tc_ptx.cuh"
@@ -174,6 +175,28 @@ __device__ __forceinline__ float round16(float v, int is_bf16) {
     return is_bf16 ? to_f32(from_f32<bf16>(v)) : to_f32(from_f32<f16>(v));
 }
 
+// The epilogue's arithmetic of Linear + bias (+ GELU) on N elements, with the roundings of the separate ops: u = round(round(product) + bias) as 16-byte pieces, and what GELU of u is
+// before its rounding.  By pairs, with one branch on the type a chunk: element by element, the type chosen at each, 8192 x 4096 x 512 bf16 took 48.7 us (with GELU, on the same warps, 84.6), 30.1 (58.3) so;
+// 512 x 1024 x 1024 7.2 (8.1), 6.8 (7.6).  Without arithmetic the one branch gains nothing (128 x (384 x 384 x 64) 10.9 us, 11.4).
+template <class T, bool GELU, int N>
+__device__ __forceinline__ void bias_gelu(float (&e)[N], float bias, uint4 (&u)[N / 8]) {
+#pragma unroll
+    for (int j = 0; j < N / 8; j++) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float* x = e + 8 * j + 2 * i;
+            float2 f = halves(pair_of(unpack2<T>(pack2_rn<T>(x[0], x[1]))) + twice(bias));
+            w[i] = pack2_rn<T>(f.x, f.y);
+            if (!GELU) continue;
+            f = gelu_f32x2(unpack2<T>(w[i]));
+            x[0] = f.x;
+            x[1] = f.y;
+        }
+        u[j] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
 // The 16 bytes that start 16 - 2 * sh bytes into (lo, hi), sh = 0 .. 7.
 __device__ __forceinline__ uint4 vector_before(const uint4& lo, const uint4& hi, uint32_t sh) {
     const uint32_t words = 4 - (sh + 1) / 2, bits = (sh & 1) * 16;
@@ -239,10 +262,10 @@ enum TcMode {
 // PANELS: TcParams::panels, an instantiation of its own for the same reason (as a branch of the common schedule it cost 4096^3 19 %).
 //
 // Epilogue warps for each quarter of the accumulator's lanes.  Rows that the warps write themselves take two (4096 x 2050 x 512 bf16: 25 us, 36
-// with one), and so do narrow tiles with a bias or an activation, whose arithmetic a wave of few tiles ends with (training step of two layers 1024 x 2048 x 2048 96.2 us, 94.5 so;
-// 256 x 256 x 256 34.9, 33.9); products that only leave through the copy engine gain nothing from a second one (16384 x 4096 x 256: 55 us, 50 with one; 128 x
-// (384 x 384 x 64) and its gradients 31.1, 29.8).
-constexpr int epi_warps(int mode, int bn_t, bool drain) { return mode == TC_PLAIN || (mode == TC_BIAS && !bn_t && !drain) ? 2 : 1; }
+// with one), and so do tiles with a bias or an activation: their arithmetic is what a wave of few narrow tiles ends with (training step of two layers 1024 x 2048 x 2048 96.2 us, 94.5 so;
+// 256 x 256 x 256 34.9, 33.9) and what full-width tiles of a short reduction wait for (8192 x 4096 x 512 with GELU 58.3 us, 46.9 so; 4096 x 4096 x 1024 39.5, 35.2); products that only leave
+// through the copy engine gain nothing from a second one (16384 x 4096 x 256: 55 us, 50 with one; 128 x (384 x 384 x 64) and its gradients 31.1, 29.8).
+constexpr int epi_warps(int mode, int bn_t, bool drain) { return mode == TC_PLAIN || (mode == TC_BIAS && !drain) ? 2 : 1; }
 constexpr int tc_threads(int w) { return 32 * (2 + 4 * w); }
 // CONV (TC_PLAIN): TcParams::conv_*; an instantiation of its own for the producer's sake too.
 template <int MODE, int BN_T, bool DRAIN = false, bool PANELS = false, bool CONV = false>
@@ -498,20 +521,23 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 uint4 q[CW / 8];
 #pragma unroll
                 for (int j = 0; j < CW; j++) e[j] = __uint_as_float(v[j / 32][j % 32]);
-                if (MODE == TC_BIAS || (MODE == TC_PLAIN && p.fuse)) {
-                    // Linear + bias (+ GELU) in one pass, with the roundings of the separate ops: the product is rounded to
-                    // the operand type, the bias is added in f32 and rounded (u), the activation is evaluated on u in f32
-                    // and rounded (act) - bit for bit what cuda_matmul, cuda_add and cuda_gelu give one after the other.
+                if constexpr (MODE == TC_BIAS) {
+                    // Linear + bias (+ GELU) in one pass: bit for bit what cuda_matmul, cuda_add and cuda_gelu give one after the other.
+                    const bool gelu = p.fuse == 2;
+                    if (p.is_bf16) gelu ? bias_gelu<bf16, true>(e, fused_bias, q) : bias_gelu<bf16, false>(e, fused_bias, q);
+                    else gelu ? bias_gelu<f16, true>(e, fused_bias, q) : bias_gelu<f16, false>(e, fused_bias, q);
+                    flush(&map_d, col, q);
+                    if (gelu) {
+                        pack(e, q);
+                        flush(&map_d2, col, q);
+                    }
+                } else {
+                    if (MODE == TC_PLAIN && p.fuse) {
 #pragma unroll
-                    for (int j = 0; j < CW; j++) e[j] = round16(round16(e[j], p.is_bf16) + fused_bias, p.is_bf16);
-                }
-                pack(e, q);
-                flush(&map_d, col, q);
-                if (MODE == TC_BIAS && p.fuse == 2) {
-#pragma unroll
-                    for (int j = 0; j < CW; j++) e[j] = gelu_f32_fast(e[j]);
+                        for (int j = 0; j < CW; j++) e[j] = round16(round16(e[j], p.is_bf16) + fused_bias, p.is_bf16);
+                    }
                     pack(e, q);
-                    flush(&map_d2, col, q);
+                    flush(&map_d, col, q);
                 }
             };
             auto load_chunk = [&](uint32_t at, uint32_t (&v)[CW / 32][32]) {

@@ -119,6 +119,28 @@ def test_gelu_backward_by_pairs(cuda, dt, n):
     assert device.last_error() is None
 
 
+@pytest.mark.parametrize("rows", [256, 51200])  # narrow tiles in one wave, full-width ones in several
+@pytest.mark.parametrize("dt", [D.BF16, D.F16])
+def test_linear_epilogue_of_every_16_bit_value(cuda, dt, rows):
+    """x . I + 0 through the product's epilogue, for every finite value that u can have: u is x and act the bits of cuda_gelu."""
+    lib = _lib.load()
+    n = 256
+    x = np.arange(65536, dtype=np.uint16).view(D.encode([0], dt).dtype)
+    x = np.resize(np.where(np.isfinite(D.decode(x, dt)), x, x[:1]), rows * n)
+    w = D.encode(np.eye(n, dtype=np.float32).ravel(), dt)
+    xb, wb, bb = device.CudaBuffer.from_host(x), device.CudaBuffer.from_host(w), device.CudaBuffer.from_host(D.encode(np.zeros(128, np.float32), dt))
+    ub, ab = device.CudaBuffer(rows * n * 2), device.CudaBuffer(rows * n * 2)
+    (lib.mx_linear_bias_gelu_bf16 if dt == D.BF16 else lib.mx_linear_bias_gelu_f16)(rows, n, n, xb.ptr, wb.ptr, bb.ptr, ub.ptr, ab.ptr)
+    device.synchronize()
+    u = ub.to_host(np.uint16, rows * n).view(x.dtype)
+    assert np.array_equal(D.decode(u, dt), D.decode(x, dt))
+    want = H.run_unary(cuda, "gelu", dt, [65536], [1], 0, u[:65536])
+    assert np.array_equal(ab.to_host(np.uint16, rows * n), np.resize(want.view(np.uint16), rows * n))
+    for b in (xb, wb, bb, ub, ab):
+        b.free()
+    assert device.last_error() is None
+
+
 def test_one_training_step_matches_f64_model(cuda):
     from maidenx_b200.mlp import Mlp
     L, Dm, B, seed, lr = 3, 256, 512, 6, 0.05
