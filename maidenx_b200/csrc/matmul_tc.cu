@@ -170,14 +170,9 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi, int is_bf16) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// v rounded to the operand type and widened again
-__device__ __forceinline__ float round16(float v, int is_bf16) {
-    return is_bf16 ? to_f32(from_f32<bf16>(v)) : to_f32(from_f32<f16>(v));
-}
-
 // The epilogue's arithmetic of Linear + bias (+ GELU) on N elements, with the roundings of the separate ops: u = round(round(product) + bias) as 16-byte pieces, and what GELU of u is
 // before its rounding.  By pairs, with one branch on the type a chunk: element by element, the type chosen at each, 8192 x 4096 x 512 bf16 took 48.7 us (with GELU, on the same warps, 84.6), 30.1 (58.3) so;
-// 512 x 1024 x 1024 7.2 (8.1), 6.8 (7.6).  Without arithmetic the one branch gains nothing (128 x (384 x 384 x 64) 10.9 us, 11.4).
+// 512 x 1024 x 1024 7.2 (8.1), 6.8 (7.6); a 1 x 1 convolution 64 x 256 x 55 x 55 -> 64, whose warps write the rows, forward and backward 340 us, 325.  Without arithmetic the one branch gains nothing (128 x (384 x 384 x 64) 10.9 us, 11.4).
 template <class T, bool GELU, int N>
 __device__ __forceinline__ void bias_gelu(float (&e)[N], float bias, uint4 (&u)[N / 8]) {
 #pragma unroll
@@ -533,10 +528,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 } else {
                     if (MODE == TC_PLAIN && p.fuse) {
-#pragma unroll
-                        for (int j = 0; j < CW; j++) e[j] = round16(round16(e[j], p.is_bf16) + fused_bias, p.is_bf16);
+                        if (p.is_bf16) bias_gelu<bf16, false>(e, fused_bias, q);
+                        else bias_gelu<f16, false>(e, fused_bias, q);
+                    } else {
+                        pack(e, q);
                     }
-                    pack(e, q);
                     flush(&map_d, col, q);
                 }
             };
