@@ -164,8 +164,7 @@ extern "C" void mx_sum_f32_noalloc(size_t num_els, size_t num_dims, size_t num_r
         splits = (R + seg - 1) / seg;
         u32* counters = splits > 1 && O * gx <= kNoAllocCounters ? all_counters : nullptr;
         dim3 grid((u32)gx, (u32)splits, (u32)gz);
-        if (vec) reduce_cols_kernel<f32, RED_SUM, VEC><<<grid, kColLanes * kColRows, 0, s>>>(inp, out, ws, O, R, I, seg, (u32)splits, pl.factor, counters);
-        else reduce_cols_kernel<f32, RED_SUM, 1><<<grid, kColLanes * kColRows, 0, s>>>(inp, out, ws, O, R, I, seg, (u32)splits, pl.factor, counters);
+        reduce_cols_choice<f32, RED_SUM, VEC>(vec, splits)<<<grid, kColLanes * kColRows, 0, s>>>(inp, out, ws, O, R, I, seg, (u32)splits, pl.factor, counters);
         if (splits > 1 && !counters) {
             u64 count = O * I;
             reduce_partials_kernel<f32, RED_SUM><<<(u32)((count + kRedThreads - 1) / kRedThreads), kRedThreads, 0, s>>>(ws, out, count, (u32)splits, 1, pl.factor);

@@ -511,6 +511,14 @@ __global__ void __launch_bounds__(kColLanes* kColRows, VEC > 1 ? kColBlocks<T, K
     }
 }
 
+// The instantiation for a fold of `splits` parts: every entry point that promises another's bits takes it from here.
+template <class T, int KIND, int VEC>
+auto reduce_cols_choice(bool vec, u64 splits) {
+    constexpr int TV = VEC < kColRows ? VEC : 1;  // a wider vector's columns have a thread each
+    if (vec) return TV == VEC && splits >= 2 * kColFoldTogether ? reduce_cols_kernel<T, KIND, TV, true> : reduce_cols_kernel<T, KIND, VEC>;
+    return splits >= kColFoldTogether ? reduce_cols_kernel<T, KIND, 1, true> : reduce_cols_kernel<T, KIND, 1>;
+}
+
 // Second pass of an "outer" reduction: out[o] = fold of partial[o * so + i * si + j], i < ni, j < nj.  G = 32: a warp per
 // output; G = kRedThreads: a block per output.
 template <class T, int KIND, int G>
@@ -815,11 +823,7 @@ void red_launch(const RedPlan& pl, const T* in, T* out, const char* where) {
             counters = arrival_counters(O * gx);
         }
         dim3 grid((u32)gx, (u32)splits, (u32)gz);
-        constexpr int TV = VEC < kColRows ? VEC : 1;  // a wider vector's columns have a thread each
-        if (vec && TV == VEC && splits >= 2 * kColFoldTogether) launch_kernel(reduce_cols_kernel<T, KIND, TV, true>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
-        else if (vec) launch_kernel(reduce_cols_kernel<T, KIND, VEC>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
-        else if (splits >= kColFoldTogether) launch_kernel(reduce_cols_kernel<T, KIND, 1, true>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
-        else launch_kernel(reduce_cols_kernel<T, KIND, 1>, grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
+        launch_kernel(reduce_cols_choice<T, KIND, VEC>(vec, splits), grid, kColLanes * kColRows, 0, s, in, out, part, O, R, I, seg, (u32)splits, pl.factor, counters);
         if (splits > 1 && !counters) {
             check_launch(where);
             u64 count = O * I;
