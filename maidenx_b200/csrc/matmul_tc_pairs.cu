@@ -496,8 +496,9 @@ bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* D, Gate& gate
     if (!ws.take(part_at + partial_bytes)) return false;
     char* base = static_cast<char*>(ws.ptr);
     // a tag is never given twice, and what the workspace held before does not look like one
-    gate.word = reinterpret_cast<unsigned long long*>(base);
-    gate.tag = 0x5A17C3E900000000ull ^ g_next_tag.fetch_add(1, std::memory_order_relaxed);
+    Gate mine;
+    mine.word = reinterpret_cast<unsigned long long*>(base);
+    mine.tag = 0x5A17C3E900000000ull ^ g_next_tag.fetch_add(1, std::memory_order_relaxed);
     int tag = 0;
     int* err = next_launch_error_word(&tag);
     if (!err) return false;
@@ -541,9 +542,10 @@ bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* D, Gate& gate
     p.a_scale = oa.scale, p.b_scale = ob.scale;
     p.d_plain = d_plain;
     p.out = static_cast<float*>(D);
-    p.unfit = gate.word, p.tag = gate.tag;
+    p.unfit = mine.word, p.tag = mine.tag;
     t_last_pairs = q.slices;
-    launch_kernel(split_pairs_kernel, oa.blocks + ob.blocks, SPLIT_THREADS, 0, ctx().stream, oa, ob, reinterpret_cast<unsigned long long*>(base), gate.tag);
+    gate = mine;  // only here: a caller whose product was not launched goes on without a gate, for nothing would open it
+    launch_kernel(split_pairs_kernel, oa.blocks + ob.blocks, SPLIT_THREADS, 0, ctx().stream, oa, ob, reinterpret_cast<unsigned long long*>(base), mine.tag);
     launch_kernel(tc_gemm_pairs_kernel, std::min(q.grid, p.num_tiles), THREADS, SMEM_BYTES, ctx().stream, ma, mb, md, p, err, tag);
     check_launch(where);
     if (q.slices > 1) splitk_reduce(2, reinterpret_cast<const float*>(base + part_at), q.slices, c.m, c.n, n_pitch, D, where);
