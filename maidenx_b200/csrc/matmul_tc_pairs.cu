@@ -9,9 +9,11 @@
 // only ever holds 128 values of K (as in the tf32 kernel, whose reason - truncating additions - holds here too), and the epilogue warps add it to their totals
 // in registers with the scales of the two blocks.
 //
-// An element far below its block's largest one would lose bits: h2 ends at 2^-24.  Blocks with a nonzero element below 2^-32 of the largest (there a pair
-// still has 2^-19 of the element), with a largest element outside 2^+-45, or with an infinity or NaN are counted as unfit; then the whole product is computed by the tf32
-// kernel instead.  The host does not wait to know: the split pass leaves the call's tag in a word of the call's workspace, this kernel gives up
+// An element far below its block's largest one would lose bits: h2 ends at 2^-24.  Blocks with a nonzero element below 2^-28 of the largest, with a
+// largest element outside 2^+-45, or with an infinity or NaN are counted as unfit; then the whole product is computed by the tf32 kernel instead.  Down to 2^-28 h1 is
+// a normal f16 and a pair holds 2^-23 of the element; from there on it loses a bit with each power of two, and an element must not be held worse than there
+// (elements of one binade by an identity, largest error and rms: tf32 2.4e-7, 7.9e-8 everywhere; pairs 1.2e-7, 4.2e-8 to 2^-27, 6.0e-8 at 2^-28, then 2.4e-7, 1.0e-7 and 4.8e-7, 2.0e-7).
+// The host does not wait to know: the split pass leaves the call's tag in a word of the call's workspace, this kernel gives up
 // when it finds it there, and the tf32 kernel, launched behind it, gives up when it does not.
 //
 // tf32 kernel / pairs, all launches, us: 4096^3 745 to 850 / 380, 2048 x 2048 x 1024 62 / 34, 4100 x 1544 x 1000 85 / 48, ragged 4099 x 1543 x 1000 124 / 62, 32 x (1152 x
@@ -35,6 +37,7 @@ namespace {
 
 constexpr int BM = 128, BN = 128, BK = 64;
 constexpr int BLOCK = 128;                          // a scale's block: 128 rows or columns by 128 values of K
+constexpr int FIT = 28;                             // powers of two that a block's nonzero elements may lie below its largest
 constexpr int STAGES = 3;
 constexpr int TILE_BYTES = BM * BK * 2;             // 16 KB: one half of the pairs of an operand's tile
 constexpr int STAGE_BYTES = 4 * TILE_BYTES;         // [A h1 | A h2 | B h1 | B h2]
@@ -394,7 +397,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_pairs_kernel(SplitOperand
     most = __reduce_max_sync(0xFFFFFFFFu, part[0][lane % (SPLIT_THREADS / 32)]);
     least = __reduce_min_sync(0xFFFFFFFFu, part[1][lane % (SPLIT_THREADS / 32)]);
     const int e = (int)(most >> 23) - 127, low = (int)((least + 1) >> 23) - 127;  // of the largest and of the smallest nonzero element
-    const bool zero = most == 0, fit = zero || (e >= -45 && e <= 45 && low >= e - 32);
+    const bool zero = most == 0, fit = zero || (e >= -45 && e <= 45 && low >= e - FIT);
     const float up = zero || !fit ? 1.0f : __uint_as_float((uint32_t)(127 + 14 - e) << 23);
     if (threadIdx.x == 0) {
         const uint32_t mb = o.k_rows ? cb : rb, kc = o.k_rows ? rb : cb, mbs = o.k_rows ? o.col_blocks : o.row_blocks, kcs = o.k_rows ? o.row_blocks : o.col_blocks;

@@ -930,3 +930,19 @@ def test_operands_that_are_not_fit_for_pairs(cuda, case, what):
         size = np.abs(x).astype(np.float64) @ np.abs(y).astype(np.float64)
     fine = np.isfinite(want) & np.isfinite(ref)
     assert np.all(np.abs(got - ref)[fine] <= 4e-6 * size[fine] + 1e-42)
+
+
+@pytest.mark.parametrize("where", ["rows", "k"])
+@pytest.mark.parametrize("depth", [20, 27, 28, 29, 30, 32])
+@pytest.mark.parametrize("majors", ["kk", "mm"])
+def test_elements_far_below_their_block_s_largest(cuda, majors, depth, where):
+    """A product that selects elements gives each of them to 2^-22, as the tf32 kernel does, however small it is next to its neighbours: 2^-23 as pairs (h1 normal), or left to that kernel."""
+    from maidenx_b200 import _lib
+    m, k, n = 320, 256, 256
+    rng = np.random.default_rng(depth)
+    x = ((rng.random((m, k)) + 1) * rng.choice([-1, 1], (m, k))).astype(np.float32)
+    x[(slice(1, None, 3),) if where == "rows" else (slice(None), slice(1, None, 3))] *= np.float32(2.0 ** -depth)
+    y = np.eye(k, n, dtype=np.float32)
+    a, b = (x if majors[0] == "k" else x.T.copy()).ravel(), y.ravel()
+    got, pairs = _pairs_product(cuda, _lib.load(), (1, m, n, k, majors, "", 0), a, b, 2)
+    assert pairs > 0 and np.all(np.abs(got[0] - x) <= 2.0 ** -22 * np.abs(x))
