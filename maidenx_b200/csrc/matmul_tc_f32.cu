@@ -631,23 +631,50 @@ constexpr double kClusterFixed32 = 4.0;
 std::atomic<int> g_cluster{1};  // 0: no clusters of slices, 2: wherever they fit (tests, A/B timing)
 thread_local int t_last_form[4] = {0, 0, 0, 0};  // of the thread's last launch: slices, CTAs of a cluster (0: none), wide, columns of a tile (tests)
 
-// What a product is estimated to take here: 0.9 us for 128 columns of a k-block (1.2 where the accumulator is emptied after each), whole or cut into slices, and
-// the copies of ragged operands.
-double estimate_us(const TcProduct& c) {
-    int grid = sm_count();
-    if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
-    const uint64_t tiles_m = (c.m + BM - 1) / BM, tiles = tiles_m * ((c.n + BN - 1) / BN);
-    const double num_kb = (double)((c.k + BK - 1) / BK) * (c.sum_batches ? (double)c.batch : 1.0);
-    const uint64_t batch = c.sum_batches ? 1 : c.batch;
-    double kb = tile_cost(tile_columns(tiles_m, c.n, batch, grid), tiles_m, c.n, batch, grid) * num_kb;
-    if (batch == 1)  // 3 us more than in the choice of slices: the second launch's own
-        for (int s = 2; s <= 32; s++) kb = std::min(kb, (double)((tiles * s + grid - 1) / grid) * (double)(int)((num_kb + s - 1) / s) + kSplitFixed32 + 3.0 + 0.1 * s);
-    const double copies = (c.a_repack ? (double)c.m * c.k : 0.0) + (c.b_repack ? (double)c.n * c.k : 0.0);
-    return kb * (c.ragged ? 1.2 : 0.9) + 3.0 + (copies > 0 ? 1.5 + copies * 8 * c.batch / 5e6 : 0.0);
+// How a product runs here: in how many slices of K, as CTAs of a cluster or through a second launch, and on which tiles.
+struct Choice {
+    int grid;
+    int slices, cluster;
+    int bn_cut, bn_whole;  // columns of a tile where the product is cut along K, where it is not
+    double us;             // what it is estimated to take
+};
+Choice choose(const TcProduct& c) {
+    Choice f;
+    f.grid = sm_count();
+    if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < f.grid) f.grid = ctx().gemm_sm_limit;
+    const uint64_t batch = c.sum_batches ? 1 : c.batch, tiles_m = (c.m + BM - 1) / BM;
+    const int num_kb = (int)((c.k + BK - 1) / BK) * (c.sum_batches ? (int)c.batch : 1);
+    // few output tiles: cut K into slices that run as the batches of the launch (see tc_ptx.cuh)
+    f.bn_cut = c.n <= 64 ? 64 : BN;
+    f.bn_whole = tile_columns(tiles_m, c.n, batch, f.grid);
+    f.slices = 1;
+    f.cluster = 0;
+    if (batch == 1) {
+        const uint64_t tiles = tiles_m * ((c.n + f.bn_cut - 1) / f.bn_cut);
+        const double kb = (128 + f.bn_cut) / 256.0, whole = tile_cost(f.bn_whole, tiles_m, c.n, batch, f.grid) * num_kb;
+        if (!c.sum_batches) f.slices = splitk_slices(tiles, c.k, BK, f.grid);
+        if (f.slices == 1) f.slices = splitk_short(tiles, (uint64_t)num_kb, f.grid, kb, whole - kSplitFixed32);
+        const int form = g_cluster.load(std::memory_order_relaxed);
+        double cost = form == 2 ? 1e30 : whole;
+        if (form != 2 && f.slices > 1)
+            cost = std::min(cost, (double)((tiles * f.slices + f.grid - 1) / f.grid * ((num_kb + f.slices - 1) / f.slices)) * kb + kSplitFixed32 + 0.1 * f.slices);
+        if (form)
+            f.cluster = cluster_slices(tiles, (uint64_t)num_kb, f.grid, kb, kClusterFixed32, cost,
+                                       [](int n) { return resident_clusters(reinterpret_cast<const void*>(tc_gemm_f32_kernel<0, CLUSTERED>), THREADS, SMEM_BYTES, n); });
+        if (f.cluster) f.slices = f.cluster;
+    }
+    // us of a k-block of 128 columns, of a tile's end, of the launch and of what else is launched, fitted to 1400 products of 1.6e7 to 3e11 multiply-adds (four of five within 11 %)
+    const int bn = f.slices > 1 ? f.bn_cut : f.bn_whole, per = (num_kb + f.slices - 1) / f.slices;
+    const double waves = (double)((batch * tiles_m * ((c.n + bn - 1) / bn) * f.slices + f.grid - 1) / f.grid), columns = bn / 128.0;
+    const bool wide = !c.ragged && f.slices == 1 && num_kb >= kWideLeast;
+    const double copies = (c.a_repack ? (double)(c.a_bs ? c.batch : 1) * c.m * c.k : 0.0) + (c.b_repack ? (double)(c.b_bs ? c.batch : 1) * c.n * c.k : 0.0);
+    f.us = waves * ((c.ragged ? 1.09 : 0.87) * per * (128 + bn) / 256.0 + (c.d_plain && f.slices == 1 ? 4.5 : wide ? 0.25 : 0.73) * columns) + 5.0 + (f.cluster ? 3.4 : f.slices > 1 ? 2.5 : 0.0) +
+           (copies > 0 ? 1.6 + copies * 8 / 8.6e6 : 0.0);
+    return f;
 }
 
 // D[M,N] = sum_k Aop[m,k] * Bop[n,k]; K-major operand = row-major [MN, K], MN-major = row-major [K, MN].
-bool launch(const TcProduct& c, void* D, const char* where) {
+bool launch(const TcProduct& c, const Choice& f, void* D, const char* where) {
     const bool a_mn = c.a_mn, b_mn = c.b_mn;
     const uint64_t M = c.m, N = c.n, K = c.k;
     uint64_t batch = c.batch;
@@ -656,7 +683,7 @@ bool launch(const TcProduct& c, void* D, const char* where) {
     p.M = (int)M;
     p.N = (int)N;
     p.chunk_kb = c.ragged ? 1 : CHUNK_FAST;
-    p.bn = N <= 64 ? 64 : BN;
+    p.bn = f.bn_cut;
     p.tiles_m = (int)((M + BM - 1) / BM);
     p.tiles_n = (int)((N + p.bn - 1) / p.bn);
     p.num_kb = (int)((K + BK - 1) / BK);
@@ -667,28 +694,11 @@ bool launch(const TcProduct& c, void* D, const char* where) {
         p.num_kb *= (int)batch;
         batch = 1;
     }
-    int grid = sm_count();
-    if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
-    // few output tiles: cut K into slices that run as the batches of this launch (see tc_ptx.cuh)
-    int slices = 1;
-    const int bn_whole = tile_columns((uint64_t)p.tiles_m, N, batch, grid);
-    p.cluster = 0;
+    int grid = f.grid;
     p.gate = c.gate;
-    if (batch == 1) {
-        const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n;
-        const double kb = (128 + p.bn) / 256.0, whole = tile_cost(bn_whole, (uint64_t)p.tiles_m, N, batch, grid) * p.num_kb;
-        if (!c.sum_batches) slices = splitk_slices(tiles, K, BK, grid);
-        if (slices == 1) slices = splitk_short(tiles, (uint64_t)p.num_kb, grid, kb, whole - kSplitFixed32);
-        const int form = g_cluster.load(std::memory_order_relaxed);
-        double cost = form == 2 ? 1e30 : whole;
-        if (form != 2 && slices > 1)
-            cost = std::min(cost, (double)((tiles * slices + grid - 1) / grid * ((p.num_kb + slices - 1) / slices)) * kb + kSplitFixed32 + 0.1 * slices);
-        if (form)
-            p.cluster = cluster_slices(tiles, (uint64_t)p.num_kb, grid, kb, kClusterFixed32, cost,
-                                       [](int n) { return resident_clusters(reinterpret_cast<const void*>(tc_gemm_f32_kernel<0, CLUSTERED>), THREADS, SMEM_BYTES, n); });
-        if (p.cluster) slices = p.cluster;
-        else if (c.gate.word) slices = 1;  // behind a gate in one launch
-    }
+    p.cluster = f.cluster;
+    int slices = f.slices;
+    if (c.gate.word && !p.cluster) slices = 1;  // behind a gate in one launch
     StreamWorkspace partial;
     const uint64_t n_pitch = (N + 3) / 4 * 4;
     if (slices > 1 && !p.cluster && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) slices = 1;
@@ -697,7 +707,7 @@ bool launch(const TcProduct& c, void* D, const char* where) {
         p.num_kb = p.split_kb;
         batch = (uint64_t)slices;
     } else {
-        p.bn = bn_whole;
+        p.bn = f.bn_whole;
         p.tiles_n = (int)((N + p.bn - 1) / p.bn);
     }
     p.tiles_per_batch = p.tiles_m * p.tiles_n;
@@ -783,8 +793,9 @@ int resident_clusters(const void* kernel, int threads, size_t shared, int n) {
 // Whatever fails here has launched no less than the product's own kernels would overwrite: the caller computes it another way.
 static bool repack_and_launch(TcProduct& c, void* out, const char* where) {
     StreamWorkspace pairs, ws;
-    tc_launch_f32_pairs(c, estimate_us(c), out, c.gate, pairs, where);
-    return repack_operands(4, c, ws, where) && launch(c, out, where);
+    const Choice choice = choose(c);
+    tc_launch_f32_pairs(c, choice.us, out, c.gate, pairs, where);
+    return repack_operands(4, c, ws, where) && launch(c, choice, out, where);
 }
 
 bool tc_launch_f32(const TcProduct& c, void* out, const char* where) {

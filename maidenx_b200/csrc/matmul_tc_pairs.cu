@@ -447,6 +447,12 @@ std::atomic<unsigned long long> g_next_tag{1};
 
 constexpr uint64_t kPairsMost = 512ull << 20;  // bytes of pairs: what the workspace pool keeps between calls
 
+// From which time in the tf32 kernel on pairs are considered, and by a seventh they have to be faster there, what the estimates are off by.  The two to four launches more, their tensor maps and
+// the workspace are 5 us of the calling thread (3.4 to 9.6 us a call, 8.7 to 14.4 as pairs): below this line a pass that is issued from the host waits for them.
+// Linear layers op by op, forward and gradients, tf32 / pairs, us: 550 x 192 -> 630 41.9 / 52.2, 596 x 53 -> 3816 62.4 / 75.2, 880 x 43 -> 792 39.2 / 46.9; 162 x (635 x 16 x 88) and its
+// gradients 92.7 / 120.
+constexpr double kPairsLeastUs = 28.0;
+
 struct Plan {
     uint64_t a_rows, a_cols, b_rows, b_cols, a_zs, b_zs, a_pitch, b_pitch, a_bytes, b_bytes, a_scales, b_scales;
     int tiles_m, tiles_n, kb_z, chunks_z, all_chunks, slices, grid;
@@ -466,16 +472,21 @@ Plan make_plan(const TcProduct& c) {
     q.grid = sm_count();
     if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < q.grid) q.grid = ctx().gemm_sm_limit;
     const uint64_t tiles = (uint64_t)q.tiles_m * q.tiles_n * (c.sum_batches ? 1 : c.batch);
-    auto cost = [&](int s) {  // us of the product kernel: 1.4 a chunk, 1 for a tile's end, 2.5 for the launch; 5 and the partial results for a second one
-        return (double)((tiles * s + q.grid - 1) / q.grid) * (1.4 * ((q.all_chunks + s - 1) / s) + 1.0) + 2.5 + (s > 1 ? 5.0 + (double)s * c.m * c.n * 8 / 8e6 : 0.0);
+    const uint64_t blocks = q.a_zs * q.tiles_m * q.chunks_z + q.b_zs * q.tiles_n * q.chunks_z;
+    const double most = 0.5 * q.kb_z * (c.sum_batches ? (double)c.batch : 1.0);  // chunks, the last one of a matrix by its k-blocks
+    // us of a chunk, of a tile's end, of all launches (the split pass, this kernel, the copies and the kernel behind the gate), of the sum over slices and of the split pass's bytes, fitted as
+    // the tf32 kernel's (choose; four of five products within 13 %)
+    auto cost = [&](int s) {
+        const double waves = (double)((tiles * s + q.grid - 1) / q.grid), per = std::min((double)((q.all_chunks + s - 1) / s), most);
+        return waves * (1.32 * per + (c.d_plain && s == 1 ? 3.4 : 1.4)) + 6.8 + (c.a_repack || c.b_repack ? 2.0 : 0.0) + (s > 1 ? 2.0 + (double)s * c.m * c.n * 8 / 1e7 : 0.0) +
+               (double)blocks * BLOCK * BLOCK * 8 / 7.4e6;
     };
     q.slices = 1;
     if (c.batch == 1 || c.sum_batches)
         for (int s = 2; s <= std::min(q.all_chunks, 16); s++)
             if (cost(s) < cost(q.slices)) q.slices = s;
     q.slices = (q.all_chunks + (q.all_chunks + q.slices - 1) / q.slices - 1) / ((q.all_chunks + q.slices - 1) / q.slices);
-    // the split pass, which reads and writes four bytes an element, and the tf32 kernel behind that finds its gate shut
-    q.cost = cost(q.slices) + 2.5 + (double)(q.a_zs * q.a_rows * q.a_cols + q.b_zs * q.b_rows * q.b_cols) * 8 / 6e6 + 1.5;
+    q.cost = cost(q.slices);
     return q;
 }
 
@@ -489,8 +500,7 @@ bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* D, Gate& gate
     if (!mode) return false;
     if (c.batch > 0x3FFF || c.m > 0x3FFFFFFF || c.n > 0x3FFFFFFF || c.k > 0x3FFFFFFF) return false;
     const Plan q = make_plan(c);
-    // 5 % in the pairs' favour: both estimates are high where a product is cut into slices, the tf32 kernel's less so ([256 x 6272] x 1152 28.1 us as pairs, 33.1)
-    if (q.a_bytes + q.b_bytes > kPairsMost || (mode == 1 && q.cost > 1.05 * tf32_us)) return false;
+    if (q.a_bytes + q.b_bytes > kPairsMost || (mode == 1 && (tf32_us < kPairsLeastUs || 1.15 * q.cost > tf32_us))) return false;
     if (q.a_zs * ((q.a_rows + 127) / 128) * ((q.a_cols + 127) / 128) + q.b_zs * ((q.b_rows + 127) / 128) * ((q.b_cols + 127) / 128) > 0x7FFFFFFFull) return false;
     if (!opt_in_shared_memory()) return false;
     auto line = [](uint64_t bytes) { return (bytes + 255) / 256 * 256; };

@@ -946,3 +946,17 @@ def test_elements_far_below_their_block_s_largest(cuda, majors, depth, where):
     a, b = (x if majors[0] == "k" else x.T.copy()).ravel(), y.ravel()
     got, pairs = _pairs_product(cuda, _lib.load(), (1, m, n, k, majors, "", 0), a, b, 2)
     assert pairs > 0 and np.all(np.abs(got[0] - x) <= 2.0 ** -22 * np.abs(x))
+
+
+@pytest.mark.parametrize("batch,fan_in,fan_out", [(550, 192, 630), (596, 53, 3816), (880, 43, 792), (504, 24, 3087), (91, 4000, 200)], ids=str)
+def test_short_f32_products_run_without_the_launches_of_pairs(cuda, batch, fan_in, fan_out):
+    """Layers whose products take less than the host takes for a split pass, a product in pairs and a kernel behind it stay with one kernel; products of several times that run as pairs."""
+    from maidenx_b200 import _lib
+    lib = _lib.load()
+
+    def ran_as_pairs(m, n, k, majors):
+        _pairs_product(cuda, lib, (1, 256, 256, 512, "kk", "", 0), np.ones(1 << 17, np.float32), np.ones(1 << 17, np.float32), 0)
+        return _pairs_product(cuda, lib, (1, m, n, k, majors, "", 0), np.ones(m * k, np.float32), np.ones(n * k, np.float32), 1)[1] > 0
+
+    assert not ran_as_pairs(batch, fan_out, fan_in, "kk") and not ran_as_pairs(batch, fan_in, fan_out, "km") and not ran_as_pairs(fan_out, fan_in, batch, "mm")
+    assert ran_as_pairs(2048, 2048, 1024, "kk") and ran_as_pairs(2100, 1500, 1001, "km")
