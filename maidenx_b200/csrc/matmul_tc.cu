@@ -1074,7 +1074,7 @@ static void repack_launch(const RowCopy<W>& a, const RowCopy<W>& b, const Gate& 
     launch_kernel(repack_rows_kernel<W>, a_blocks + b_blocks, 256, 0, ctx().stream, a, b, gate, a_blocks);
 }
 
-bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* where) {
+bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* where, char* place, uint64_t room) {
     const uint64_t a_rows = (c.a_mn ? c.k : c.m) * (c.a_bs ? c.batch : 1), a_cols = c.a_mn ? c.m : c.k, a_pitch = copy_pitch(es, a_rows, a_cols);
     const uint64_t b_rows = (c.b_mn ? c.k : c.n) * (c.b_bs ? c.batch : 1), b_cols = c.b_mn ? c.n : c.k, b_pitch = copy_pitch(es, b_rows, b_cols);
     bool a_copy = c.a_repack, b_copy = c.b_repack;
@@ -1093,8 +1093,11 @@ bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* w
     if (!a_copy && !b_copy) return true;
     const uint64_t a_bytes = a_copy ? (a_rows * a_pitch * es + 255) / 256 * 256 : 0, b_bytes = b_copy ? b_rows * b_pitch * es : 0;
     if (a_bytes / 16 + b_bytes / 16 > 0x7FFFFFFFull) return !needed;  // the copy counts vectors in 32 bits
-    if (!ws.take(a_bytes + b_bytes)) return !needed;
-    char *const a_dst = static_cast<char*>(ws.ptr), *const b_dst = a_dst + a_bytes;
+    if (!place || a_bytes + b_bytes > room) {
+        if (!ws.take(a_bytes + b_bytes)) return !needed;
+        place = static_cast<char*>(ws.ptr);
+    }
+    char *const a_dst = place, *const b_dst = a_dst + a_bytes;
     auto launch = [&](auto w) {
         typedef decltype(w) W;
         const auto copy = [&](bool yes, const char* in, char* out, uint64_t rows, uint64_t cols, uint64_t pitch) {

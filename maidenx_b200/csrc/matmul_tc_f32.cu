@@ -794,8 +794,10 @@ int resident_clusters(const void* kernel, int threads, size_t shared, int n) {
 static bool repack_and_launch(TcProduct& c, void* out, const char* where) {
     StreamWorkspace pairs, ws;
     const Choice choice = choose(c);
-    tc_launch_f32_pairs(c, choice.us, out, c.gate, pairs, where);
-    return repack_operands(4, c, ws, where) && launch(c, choice, out, where);
+    PairsRun run;
+    tc_launch_f32_pairs(c, choice.us, out, run, pairs, where);
+    c.gate = run.gate;
+    return repack_operands(4, c, ws, where, run.place, run.room) && launch(c, choice, out, where);
 }
 
 bool tc_launch_f32(const TcProduct& c, void* out, const char* where) {

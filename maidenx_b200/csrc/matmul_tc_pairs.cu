@@ -445,7 +445,9 @@ std::atomic<int> g_pairs{1};  // 0: never, 2: wherever possible, 3: the same wit
 thread_local int t_last_pairs = 0;
 std::atomic<unsigned long long> g_next_tag{1};
 
-constexpr uint64_t kPairsMost = 512ull << 20;  // bytes of pairs: what the workspace pool keeps between calls
+// Bytes of a call's workspace: what the pool keeps between calls.  Beyond it each call maps memory anew, which took longer than pairs gain: [13712 x 4025] by 59
+// columns and its gradients 772 us in tf32, 1180 while the copies behind the gate had memory of their own, 716 in the pairs'.
+constexpr uint64_t kPairsMost = 512ull << 20;
 
 // From which time in the tf32 kernel on pairs are considered, and by a seventh they have to be faster there, what the estimates are off by.  The two to four launches more, their tensor maps and
 // the workspace are 5 us of the calling thread (3.4 to 9.6 us a call, 8.7 to 14.4 as pairs): below this line a pass that is issued from the host waits for them.
@@ -492,21 +494,21 @@ Plan make_plan(const TcProduct& c) {
 
 }  // namespace
 
-// false: nothing was launched and the caller goes on as without this; true: the product has been launched, and `gate` says what the caller's own kernel
+// false: nothing was launched and the caller goes on as without this; true: the product has been launched, and `run.gate` says what the caller's own kernel
 // has to find in order to run behind it.
-bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* D, Gate& gate, StreamWorkspace& ws, const char* where) {
+bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* D, PairsRun& run, StreamWorkspace& ws, const char* where) {
     t_last_pairs = 0;
     const int mode = g_pairs.load(std::memory_order_relaxed);
     if (!mode) return false;
     if (c.batch > 0x3FFF || c.m > 0x3FFFFFFF || c.n > 0x3FFFFFFF || c.k > 0x3FFFFFFF) return false;
     const Plan q = make_plan(c);
-    if (q.a_bytes + q.b_bytes > kPairsMost || (mode == 1 && (tf32_us < kPairsLeastUs || 1.15 * q.cost > tf32_us))) return false;
+    if (q.a_bytes + q.b_bytes >= kPairsMost || (mode == 1 && (tf32_us < kPairsLeastUs || 1.15 * q.cost > tf32_us))) return false;
     if (q.a_zs * ((q.a_rows + 127) / 128) * ((q.a_cols + 127) / 128) + q.b_zs * ((q.b_rows + 127) / 128) * ((q.b_cols + 127) / 128) > 0x7FFFFFFFull) return false;
     if (!opt_in_shared_memory()) return false;
     auto line = [](uint64_t bytes) { return (bytes + 255) / 256 * 256; };
     const uint64_t n_pitch = (c.n + 3) / 4 * 4, partial_bytes = q.slices > 1 ? (uint64_t)q.slices * c.m * n_pitch * 4 : 0;
     const uint64_t a_at = 256, b_at = a_at + line(q.a_bytes), sa_at = b_at + line(q.b_bytes), sb_at = sa_at + line(q.a_scales * 4), part_at = sb_at + line(q.b_scales * 4);
-    if (!ws.take(part_at + partial_bytes)) return false;
+    if (part_at + partial_bytes > kPairsMost || !ws.take(part_at + partial_bytes)) return false;
     char* base = static_cast<char*>(ws.ptr);
     // a tag is never given twice, and what the workspace held before does not look like one
     Gate mine;
@@ -557,7 +559,9 @@ bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* D, Gate& gate
     p.out = static_cast<float*>(D);
     p.unfit = mine.word, p.tag = mine.tag;
     t_last_pairs = q.slices;
-    gate = mine;  // only here: a caller whose product was not launched goes on without a gate, for nothing would open it
+    run.gate = mine;  // only here: a caller whose product was not launched goes on without a gate, for nothing would open it
+    run.place = base + a_at;
+    run.room = sa_at - a_at;
     launch_kernel(split_pairs_kernel, oa.blocks + ob.blocks, SPLIT_THREADS, 0, ctx().stream, oa, ob, reinterpret_cast<unsigned long long*>(base), mine.tag);
     launch_kernel(tc_gemm_pairs_kernel, std::min(q.grid, p.num_tiles), THREADS, SMEM_BYTES, ctx().stream, ma, mb, md, p, err, tag);
     check_launch(where);

@@ -269,8 +269,8 @@ struct TcProduct;
 namespace tc {
 constexpr uint64_t kCopyFree = 8ull << 20;  // bytes of a copy that need no justification
 uint64_t copy_pitch(size_t elem_size, uint64_t rows, uint64_t cols);
-// Copies the operands a product marks for it into `ws` and points the product at the copies.  false: no workspace to be had
-// (nothing launched); the caller falls back to the CUDA-core kernel.
-bool repack_operands(size_t elem_size, TcProduct& c, StreamWorkspace& ws, const char* where);
+// Copies the operands a product marks for it into `place`, where `room` bytes are enough, or into `ws` and points the product at the copies.  false: no
+// workspace to be had (nothing launched); the caller falls back to the CUDA-core kernel.
+bool repack_operands(size_t elem_size, TcProduct& c, StreamWorkspace& ws, const char* where, char* place = nullptr, uint64_t room = 0);
 }  // namespace tc
 }  // namespace mx

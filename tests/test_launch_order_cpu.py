@@ -78,11 +78,11 @@ def gate_without_launch(source):
     s = _without_comments(source)
     head = re.search(r"bool tc_launch_f32_pairs\([^)]*\)\s*\{", s)
     body = s[head.end():_closing(s, head.end() - 1, "{}")]
-    at = [m.start() for m in re.finditer(r"\bgate(\.\w+)?\s*=[^=]", body)]
+    at = [m.start() for m in re.finditer(r"\brun\.gate(\.\w+)?\s*=[^=]", body)]
     return [] if at and "return false" not in body[at[0]:] and body.index("split_pairs_kernel") > at[0] else ["the caller's gate is set before the last way out without a launch"]
 
 
 def test_a_product_in_pairs_that_is_not_launched_leaves_no_gate():
     s = _sources()["matmul_tc_pairs.cu"]
     assert not gate_without_launch(s)
-    assert gate_without_launch(s.replace("Gate mine;", "Gate mine; gate = mine;"))
+    assert gate_without_launch(s.replace("Gate mine;", "Gate mine; run.gate = mine;"))

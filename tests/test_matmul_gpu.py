@@ -960,3 +960,23 @@ def test_short_f32_products_run_without_the_launches_of_pairs(cuda, batch, fan_i
 
     assert not ran_as_pairs(batch, fan_out, fan_in, "kk") and not ran_as_pairs(batch, fan_in, fan_out, "km") and not ran_as_pairs(fan_out, fan_in, batch, "mm")
     assert ran_as_pairs(2048, 2048, 1024, "kk") and ran_as_pairs(2100, 1500, 1001, "km")
+
+
+def test_a_large_product_in_pairs_stays_within_the_pool(cuda):
+    """Ragged operands of 392 MB: the pairs and the copies of the kernel behind them share their memory, so that the next call finds all of it in the pool and maps none."""
+    import torch
+
+    from maidenx_b200 import _lib, device
+    lib, (m, n, k) = _lib.load(), (6065, 12, 16147)
+    a, b, out = torch.ones(m, k, device="cuda"), torch.ones(n, k, device="cuda"), torch.empty(m, n, device="cuda")
+    lib.mx_debug_set_gemm_f32_pairs(2)
+    try:
+        for _ in range(3):
+            torch.cuda.synchronize()
+            before = torch.cuda.mem_get_info()[0]
+            device.dispatch("matmul", "f32", H.matmul_metadata([m, n], [m, k], [k, n], [k, 1], [1, k], 0, 0), m * n, "META", a.data_ptr(), b.data_ptr(), out.data_ptr())
+            mapped = before - torch.cuda.mem_get_info()[0]
+        assert lib.mx_debug_gemm_f32_last_pairs() > 0 and mapped < 64 << 20
+        assert bool((out == k).all())
+    finally:
+        lib.mx_debug_set_gemm_f32_pairs(1)
