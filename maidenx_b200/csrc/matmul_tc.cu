@@ -937,8 +937,10 @@ int splitk_short(uint64_t tiles, uint64_t num_kb, int sms, double kb_cost, doubl
 // `vec` elements per step: 4 when the output's rows are whole vectors (then rows and padded rows coincide), else 1.
 template <class T, int VEC>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* partial, int slices, size_t rows, uint32_t cols, uint32_t pitch, FastDiv div,
-                                                            T* out) {
+                                                            T* out, Gate gate, int shut_slices) {
     after_previous_kernel();
+    if (gate.shut()) slices = shut_slices;
+    if (!slices) return;
     const size_t nvec = rows * cols / VEC, stride = (size_t)gridDim.x * 256, slice = rows * pitch;
     for (size_t v = (size_t)blockIdx.x * 256 + threadIdx.x; v < nvec; v += stride) {
         size_t src = VEC * v;
@@ -964,21 +966,22 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* partial
 }
 
 template <class T>
-static void splitk_reduce_t(const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out) {
+static void splitk_reduce_t(const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out, const Gate& gate, int shut_slices) {
     const bool vec = cols == pitch && reinterpret_cast<uintptr_t>(out) % (4 * sizeof(T)) == 0;
     size_t blocks = (rows * cols / (vec ? 4 : 1) + 255) / 256;
     const size_t cap = (size_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     const FastDiv div((uint32_t)cols);
-    if (vec) launch_kernel(splitk_reduce_kernel<T, 4>, (unsigned)blocks, 256, 0, ctx().stream, partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out));
-    else launch_kernel(splitk_reduce_kernel<T, 1>, (unsigned)blocks, 256, 0, ctx().stream, partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out));
+    if (vec) launch_kernel(splitk_reduce_kernel<T, 4>, (unsigned)blocks, 256, 0, ctx().stream, partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out), gate, shut_slices);
+    else launch_kernel(splitk_reduce_kernel<T, 1>, (unsigned)blocks, 256, 0, ctx().stream, partial, slices, rows, (uint32_t)cols, (uint32_t)pitch, div, static_cast<T*>(out), gate, shut_slices);
 }
 
-void splitk_reduce(int dtype, const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out, const char* where) {
-    if (dtype == 0) splitk_reduce_t<bf16>(partial, slices, rows, cols, pitch, out);
-    else if (dtype == 1) splitk_reduce_t<f16>(partial, slices, rows, cols, pitch, out);
-    else splitk_reduce_t<float>(partial, slices, rows, cols, pitch, out);
+void splitk_reduce(int dtype, const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out, const char* where, const Gate* behind, int shut_slices) {
+    const Gate gate = behind ? *behind : Gate();
+    if (dtype == 0) splitk_reduce_t<bf16>(partial, slices, rows, cols, pitch, out, gate, shut_slices);
+    else if (dtype == 1) splitk_reduce_t<f16>(partial, slices, rows, cols, pitch, out, gate, shut_slices);
+    else splitk_reduce_t<float>(partial, slices, rows, cols, pitch, out, gate, shut_slices);
     check_launch(where);
 }
 

@@ -58,13 +58,16 @@ bool tc_conv_grad_input(bool is_bf16, uint64_t batch, uint64_t c, uint64_t h, ui
                         const void* g, const void* wt, void* grad_x, const char* where);
 bool tc_launch_f32(const TcProduct& c, void* out, const char* where);
 // The product in pairs of f16 (matmul_tc_pairs.cu), if that is estimated to take less than `tf32_us`.  true: launched, and whoever called runs the product behind
-// a gate, which is open when an operand was not fit for pairs and lies in `ws`; false: nothing launched.
+// a gate, which is open when an operand was not fit for pairs and lies in `ws`, and behind that the sum of the slices, of whichever product ran; false: nothing launched.
 struct PairsRun {
     Gate gate;
-    char* place = nullptr;  // the pairs' own memory, for what runs behind the open gate: nothing reads them there
+    int slices = 1;            // of the product in pairs: its partial results, [slices][m][n rounded up to 4], are still to be added
+    float* partial = nullptr;  // where they are, and where the product behind the gate has its own
+    char* place = nullptr;     // the pairs' own memory, for what else runs behind the open gate: nothing reads them there
     uint64_t room = 0;
 };
-bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* out, PairsRun& run, StreamWorkspace& ws, const char* where);
+// partial_bytes: what the product behind the gate takes for partial results.
+bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, uint64_t partial_bytes, void* out, PairsRun& run, StreamWorkspace& ws, const char* where);
 bool tc_gemm_f32(const MmDesc& d, int which, size_t num_els, size_t nea, size_t neb, const void* x, const void* y, void* out, const char* where);
 
 template <class T>

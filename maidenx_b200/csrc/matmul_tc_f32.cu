@@ -637,6 +637,7 @@ struct Choice {
     int slices, cluster;
     int bn_cut, bn_whole;  // columns of a tile where the product is cut along K, where it is not
     double us;             // what it is estimated to take
+    uint64_t partial_bytes(uint64_t m, uint64_t n) const { return slices > 1 && !cluster ? (uint64_t)slices * m * ((n + 3) / 4 * 4) * sizeof(float) : 0; }
 };
 Choice choose(const TcProduct& c) {
     Choice f;
@@ -674,7 +675,9 @@ Choice choose(const TcProduct& c) {
 }
 
 // D[M,N] = sum_k Aop[m,k] * Bop[n,k]; K-major operand = row-major [MN, K], MN-major = row-major [K, MN].
-bool launch(const TcProduct& c, const Choice& f, void* D, const char* where) {
+// Behind a gate (c.gate, `run`) in the same form as alone, slices included: without them 512 x 512 x 8192 took 219 us as pairs with an operand that is not fit, 16 tiles on 16 SMs, 51 so (tf32 alone 38).  The sum of the slices is one launch for this
+// product and for the one in pairs, whichever ran.
+bool launch(const TcProduct& c, const Choice& f, const PairsRun& run, void* D, const char* where) {
     const bool a_mn = c.a_mn, b_mn = c.b_mn;
     const uint64_t M = c.m, N = c.n, K = c.k;
     uint64_t batch = c.batch;
@@ -698,10 +701,13 @@ bool launch(const TcProduct& c, const Choice& f, void* D, const char* where) {
     p.gate = c.gate;
     p.cluster = f.cluster;
     int slices = f.slices;
-    if (c.gate.word && !p.cluster) slices = 1;  // behind a gate in one launch
-    StreamWorkspace partial;
+    StreamWorkspace workspace;
+    float* partial = run.partial;
     const uint64_t n_pitch = (N + 3) / 4 * 4;
-    if (slices > 1 && !p.cluster && !partial.take((size_t)slices * M * n_pitch * sizeof(float), true)) slices = 1;
+    if (slices > 1 && !p.cluster && !partial) {
+        if (workspace.take(f.partial_bytes(M, N), true)) partial = static_cast<float*>(workspace.ptr);
+        else slices = 1;
+    }
     if (slices > 1) {
         p.split_kb = (p.num_kb + slices - 1) / slices;
         p.num_kb = p.split_kb;
@@ -724,7 +730,7 @@ bool launch(const TcProduct& c, const Choice& f, void* D, const char* where) {
     p.d_plain = slices > 1 ? 0 : c.d_plain;
     p.vec_out = N % 4 == 0 && (uintptr_t)D % 16 == 0 ? 1 : 0;
     if (p.d_plain || p.cluster) md = ma;  // not used
-    else if (slices > 1 ? !make_map(&md, partial.ptr, M, N, batch, M * n_pitch, 32, false, n_pitch) : !make_map(&md, D, M, N, batch, M * N, 32)) return false;
+    else if (slices > 1 ? !make_map(&md, partial, M, N, batch, M * n_pitch, 32, false, n_pitch) : !make_map(&md, D, M, N, batch, M * N, 32)) return false;
     p.num_tiles = (int)batch * p.tiles_per_batch;
     p.a_batched = (c.batch > 1 && a_bs != 0) ? 1 : 0;
     p.b_batched = (c.batch > 1 && b_bs != 0) ? 1 : 0;
@@ -741,7 +747,7 @@ bool launch(const TcProduct& c, const Choice& f, void* D, const char* where) {
     p.b_ks = b_mn ? b_ld : 1;
     p.K = (int)K;
     p.zs = (int)c.batch;
-    p.out = static_cast<float*>(slices > 1 && !p.cluster ? partial.ptr : D);
+    p.out = slices > 1 && !p.cluster ? partial : static_cast<float*>(D);
     p.out_ld = (int64_t)(slices > 1 && !p.cluster ? n_pitch : N);
     if (grid > p.num_tiles) grid = p.num_tiles;
     const int form = p.cluster ? CLUSTERED : p.chunk_kb == CHUNK_FAST && slices == 1 && p.num_kb >= kWideLeast && g_wide.load(std::memory_order_relaxed) ? WIDE : PLAIN;
@@ -755,7 +761,8 @@ bool launch(const TcProduct& c, const Choice& f, void* D, const char* where) {
                                        : (fixed ? tc_gemm_f32_kernel<BN> : tc_gemm_f32_kernel<0>);
     launch_clusters(kernel, p.cluster ? p.num_tiles : grid, THREADS, SMEM_BYTES, p.cluster, ma, mb, md, p, err, tag);
     check_launch(where);
-    if (slices > 1 && !p.cluster) splitk_reduce(2, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
+    const int to_add = slices > 1 && !p.cluster ? slices : 0, in_pairs = run.slices > 1 ? run.slices : 0;
+    if (to_add || in_pairs) splitk_reduce(2, partial, to_add, M, N, n_pitch, D, where, &c.gate, in_pairs);
     return true;
 }
 
@@ -795,9 +802,9 @@ static bool repack_and_launch(TcProduct& c, void* out, const char* where) {
     StreamWorkspace pairs, ws;
     const Choice choice = choose(c);
     PairsRun run;
-    tc_launch_f32_pairs(c, choice.us, out, run, pairs, where);
+    tc_launch_f32_pairs(c, choice.us, choice.partial_bytes(c.m, c.n), out, run, pairs, where);
     c.gate = run.gate;
-    return repack_operands(4, c, ws, where, run.place, run.room) && launch(c, choice, out, where);
+    return repack_operands(4, c, ws, where, run.place, run.room) && launch(c, choice, run, out, where);
 }
 
 bool tc_launch_f32(const TcProduct& c, void* out, const char* where) {

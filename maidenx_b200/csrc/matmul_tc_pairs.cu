@@ -496,7 +496,7 @@ Plan make_plan(const TcProduct& c) {
 
 // false: nothing was launched and the caller goes on as without this; true: the product has been launched, and `run.gate` says what the caller's own kernel
 // has to find in order to run behind it.
-bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* D, PairsRun& run, StreamWorkspace& ws, const char* where) {
+bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, uint64_t partial_bytes, void* D, PairsRun& run, StreamWorkspace& ws, const char* where) {
     t_last_pairs = 0;
     const int mode = g_pairs.load(std::memory_order_relaxed);
     if (!mode) return false;
@@ -506,9 +506,9 @@ bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* D, PairsRun& 
     if (q.a_zs * ((q.a_rows + 127) / 128) * ((q.a_cols + 127) / 128) + q.b_zs * ((q.b_rows + 127) / 128) * ((q.b_cols + 127) / 128) > 0x7FFFFFFFull) return false;
     if (!opt_in_shared_memory()) return false;
     auto line = [](uint64_t bytes) { return (bytes + 255) / 256 * 256; };
-    const uint64_t n_pitch = (c.n + 3) / 4 * 4, partial_bytes = q.slices > 1 ? (uint64_t)q.slices * c.m * n_pitch * 4 : 0;
+    const uint64_t n_pitch = (c.n + 3) / 4 * 4, partials = std::max(partial_bytes, q.slices > 1 ? (uint64_t)q.slices * c.m * n_pitch * 4 : 0);
     const uint64_t a_at = 256, b_at = a_at + line(q.a_bytes), sa_at = b_at + line(q.b_bytes), sb_at = sa_at + line(q.a_scales * 4), part_at = sb_at + line(q.b_scales * 4);
-    if (part_at + partial_bytes > kPairsMost || !ws.take(part_at + partial_bytes)) return false;
+    if (part_at + partials > kPairsMost || !ws.take(part_at + partials)) return false;
     char* base = static_cast<char*>(ws.ptr);
     // a tag is never given twice, and what the workspace held before does not look like one
     Gate mine;
@@ -560,12 +560,13 @@ bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, void* D, PairsRun& 
     p.unfit = mine.word, p.tag = mine.tag;
     t_last_pairs = q.slices;
     run.gate = mine;  // only here: a caller whose product was not launched goes on without a gate, for nothing would open it
+    run.slices = q.slices;
+    run.partial = reinterpret_cast<float*>(base + part_at);
     run.place = base + a_at;
     run.room = sa_at - a_at;
     launch_kernel(split_pairs_kernel, oa.blocks + ob.blocks, SPLIT_THREADS, 0, ctx().stream, oa, ob, reinterpret_cast<unsigned long long*>(base), mine.tag);
     launch_kernel(tc_gemm_pairs_kernel, std::min(q.grid, p.num_tiles), THREADS, SMEM_BYTES, ctx().stream, ma, mb, md, p, err, tag);
     check_launch(where);
-    if (q.slices > 1) splitk_reduce(2, reinterpret_cast<const float*>(base + part_at), q.slices, c.m, c.n, n_pitch, D, where);
     return true;
 }
 

@@ -7,6 +7,7 @@
 #include "common.cuh"
 
 namespace mx {
+struct Gate;
 namespace tc {
 
 constexpr long long TC_WAIT_BUDGET_CYCLES = 4000000000ll;  // about two seconds
@@ -255,7 +256,8 @@ int splitk_slices(uint64_t tiles, uint64_t K, int block_k, int sms);
 // (k-blocks * kb_cost) comes out below `below`, the cost of the unsplit product less that of the second launch.
 int splitk_short(uint64_t tiles, uint64_t num_kb, int sms, double kb_cost, double below);
 // out[r * cols + c] = round(sum_s partial[(s * rows + r) * pitch + c]); dtype: 0 bf16, 1 f16, 2 f32.  pitch: cols rounded up to 4.
-void splitk_reduce(int dtype, const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out, const char* where);
+// `behind`: slices where that gate is open, `shut_slices` where it is shut; no slices: nothing is written.
+void splitk_reduce(int dtype, const float* partial, int slices, uint64_t rows, uint64_t cols, uint64_t pitch, void* out, const char* where, const Gate* behind = nullptr, int shut_slices = 0);
 
 // The error word of the calling thread's current device (allocated on first use) and the tag of the launch about
 // to be made.  Returns nullptr when there is no usable device.

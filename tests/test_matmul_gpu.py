@@ -980,3 +980,24 @@ def test_a_large_product_in_pairs_stays_within_the_pool(cuda):
         assert bool((out == k).all())
     finally:
         lib.mx_debug_set_gemm_f32_pairs(1)
+
+
+# products that are cut along K as pairs and by the tf32 kernel, by the latter alone, into a cluster; ragged
+@pytest.mark.parametrize("case,slices", [((1, 512, 512, 8192, "kk", "", 0), "both"), ((1, 300, 261, 9001, "km", "", 1), "both"), ((1, 400, 400, 256, "kk", "", 0), "tf32"),
+                                         ((1, 300, 784, 8192, "kk", "", 0), "cluster")], ids=str)
+def test_the_kernel_behind_the_gate_is_cut_along_k(cuda, case, slices):
+    """A product that is not fit for pairs runs in the form, and to the bits, that it has without them; the same product with fit operands is the pairs' own sum."""
+    import ctypes
+
+    from maidenx_b200 import _lib
+    lib, form = _lib.load(), (ctypes.c_int * 4)()
+    a, b, x, y = _pairs_operands(case, np.random.default_rng(3), "normal")
+    got, pairs = _pairs_product(cuda, lib, case, a, b, 2)
+    lib.mx_debug_gemm_f32_last_form(form)
+    assert (pairs > 1) == (slices in ("both", "cluster")) and form[0] > 1 and (form[1] > 0) == (slices == "cluster")
+    ref = x.astype(np.float64) @ y.astype(np.float64)
+    assert np.linalg.norm(got - ref) < 6e-7 * np.linalg.norm(ref)
+    a[case[6] + 5] = np.float32(1e-13)  # below 2^-40 of its neighbours
+    got, pairs = _pairs_product(cuda, lib, case, a, b, 2)
+    want, _ = _pairs_product(cuda, lib, case, a, b, 0)
+    assert pairs > 0 and np.array_equal(got, want)
