@@ -138,6 +138,8 @@ struct StreamWorkspace {
     StreamWorkspace& operator=(const StreamWorkspace&) = delete;
     ~StreamWorkspace();
 };
+// For a call that has taken another route than it will take under capture: the thread's scratch block as large as that one borrows.
+void reserve_for_capture(size_t bytes);
 
 // Launches `kernel` so that it is scheduled as soon as the blocks of the kernel before it in the stream have ended, without the launch's own latency
 // between the two (programmatic dependent launch): 2 us less for each of a chain of kernels on small tensors (1e6 floats 5.1 us a launch, now 3.1), up to a

@@ -316,6 +316,16 @@ bool StreamWorkspace::take(size_t bytes, bool under_capture) {
     }
     return true;
 }
+void reserve_for_capture(size_t bytes) {
+    int dev = 0;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (!bytes || bytes > kUnderCaptureMost || cudaStreamIsCapturing(ctx().stream, &capturing) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return;
+    }
+    cudaError_t e = cudaSuccess;
+    if (capturing == cudaStreamCaptureStatusNone && !scratch_block(dev, bytes, &e)) cudaGetLastError();
+}
 StreamWorkspace::~StreamWorkspace() {
     if (ptr && !borrowed && cudaFreeAsync(ptr, stream) != cudaSuccess) cudaGetLastError();
 }

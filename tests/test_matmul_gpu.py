@@ -1001,3 +1001,50 @@ def test_the_kernel_behind_the_gate_is_cut_along_k(cuda, case, slices):
     got, pairs = _pairs_product(cuda, lib, case, a, b, 2)
     want, _ = _pairs_product(cuda, lib, case, a, b, 0)
     assert pairs > 0 and np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("case", [(512, 512, 8192), (768, 768, 16384), (512, 1024, 4096)], ids=str)
+def test_products_in_pairs_are_cut_along_k_under_capture(cuda, case):
+    """There is no workspace for pairs in a graph: a product that runs as pairs in a direct call runs there in the tf32 kernel, cut along K and with the bits of a direct call of that kernel,
+    although the thread has made no other call that left it a scratch block."""
+    import ctypes
+    import threading
+
+    import torch
+
+    from maidenx_b200 import _lib
+    lib, (m, n, k) = _lib.load(), case
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a, b = torch.randn(m, k, device="cuda", generator=g), torch.randn(n, k, device="cuda", generator=g)
+    meta = np.asarray(H.matmul_metadata([m, n], [m, k], [k, n], [k, 1], [1, k], 0, 0), dtype=np.uint64)
+    direct, replayed, tf32 = (torch.zeros(m, n, device="cuda") for _ in range(3))
+    call = lambda out: _lib.op("matmul", "f32")(ctypes.c_size_t(m * n), meta.ctypes.data, a.data_ptr(), b.data_ptr(), out.data_ptr())  # noqa: E731
+    seen = {}
+
+    def new_thread():
+        form, s = (ctypes.c_int * 4)(), torch.cuda.Stream()
+        lib.mx_set_stream(s.cuda_stream)
+        graph = torch.cuda.CUDAGraph()
+        call(direct)
+        s.synchronize()
+        seen["pairs"] = lib.mx_debug_gemm_f32_last_pairs()
+        with torch.cuda.graph(graph, stream=s):
+            call(replayed)
+        lib.mx_debug_gemm_f32_last_form(form)
+        seen["slices"] = form[0]
+        graph.replay()
+        torch.cuda.synchronize()
+        lib.mx_debug_set_gemm_f32_pairs(0)
+        call(tf32)
+        s.synchronize()
+        lib.mx_set_stream(None)
+
+    lib.mx_debug_set_gemm_f32_pairs(2)
+    try:
+        t = threading.Thread(target=new_thread)
+        t.start()
+        t.join()
+    finally:
+        lib.mx_debug_set_gemm_f32_pairs(1)
+    assert seen["pairs"] > 0 and seen["slices"] > 1 and torch.equal(replayed, tf32)
+    assert float((direct - replayed).norm() / replayed.norm()) < 1e-6
