@@ -120,6 +120,8 @@ struct TcParams {
     // CONV: the product's B is read out of images, K runs over a kernel's taps and, for each, over the channels of B's images in k-blocks (conv_cb of them); a column tile
     // is conv_rows whole rows of an output image of width conv_w, whose source pixels for tap (i, j) begin at row + conv_y - i, column conv_x - j.
     int conv_cb, conv_kw, conv_rows, conv_w, conv_x, conv_y;
+    int conv_kh, conv_co, conv_oh, conv_ow;  // and both operands as plain memory, for conv_redo
+    const void *conv_g, *conv_wt;
     int poll_ns;  // between the epilogue's looks at a tile's accumulator: 3 to 4 % of the time a tile's reduction takes (training step of 512 x 1024 x 1024 49.5 us at 400, 48.8 so)
 };
 
@@ -243,6 +245,48 @@ __device__ __forceinline__ void store_rows(uint16_t* tile, size_t ld, int r0, in
 
 // What the epilogue does is compiled in: each form keeps its registers and its code to itself, and the plain product's loop is
 // not laid out around the others.
+// CONV: a pixel outside grad_out arrives as zeros, and zero times a weight that is infinite or NaN is a NaN that the sum over the pixels inside does not have.  The epilogue looks for totals that
+// are not finite, and a CTA that saw one goes through its tiles here: a NaN whose taps do not all lie inside is summed anew over those that do, up to the first NaN among them.
+// A warp takes a row, eight pixels a lane in flight; bound by the sums' serial chains.  Finite totals cost nothing that shows (64 x 256 x 56 x 56 -> 256, 3 x 3, input gradient 205 us with the look
+// and without), one infinite weight 1075, a gradient of NaNs 468.
+struct ConvRedo {
+    const void *g, *wt;
+    void* out;  // of the tile's batch
+    int rows, pixels, c0, pix0, n, w, x, y, kh, kw, co, oh, ow;
+};
+template <class T>
+__device__ __noinline__ void conv_redo(const ConvRedo q) {
+    const T *const g = static_cast<const T*>(q.g), *const wt = static_cast<const T*>(q.wt);
+    const int lane = threadIdx.x & 31;
+    auto tap_row = [&](int s) { return (q.pix0 + lane + 32 * s) / q.w + q.y; };  // tap (i, j) of the lane's s-th pixel reads (tap_row - i, tap_col - j)
+    auto tap_col = [&](int s) { return (q.pix0 + lane + 32 * s) % q.w + q.x; };
+    uint32_t edge = 0;  // the pixels that not all taps of lie inside; a tile has 256 at most
+    for (int s = 0; s < 8; s++)
+        if (lane + 32 * s < q.pixels && (tap_row(s) >= q.oh || tap_col(s) >= q.ow || tap_row(s) < q.kh - 1 || tap_col(s) < q.kw - 1)) edge |= 1u << s;
+    for (int r = threadIdx.x >> 5; r < q.rows; r += blockDim.x >> 5) {
+        const int c = q.c0 + r;
+        T* const row = static_cast<T*>(q.out) + (size_t)c * q.n + q.pix0 + lane;
+        uint32_t wrong = 0;
+#pragma unroll
+        for (int s = 0; s < 8; s++)
+            if (edge >> s & 1 && isnan(to_f32(row[32 * s]))) wrong |= 1u << s;
+        for (; wrong; wrong &= wrong - 1) {
+            const int s = __ffs(wrong) - 1, y = tap_row(s), x = tap_col(s);
+            float sum = 0.0f;
+            for (int i = max(0, y - q.oh + 1); i < q.kh && i <= y && !isnan(sum); i++)
+                for (int j = max(0, x - q.ow + 1); j < q.kw && j <= x && !isnan(sum); j++) {
+                    const T *const a = wt + ((size_t)c * q.kh * q.kw + i * q.kw + j) * q.co, *const b = g + ((size_t)(y - i) * q.ow + (x - j)) * q.co;
+                    for (int o = 0; o < q.co && !isnan(sum); o += 8) {  // co is a multiple of 8 and both start on 16-byte boundaries
+                        const Vec<T, 8> va = *reinterpret_cast<const Vec<T, 8>*>(a + o), vb = *reinterpret_cast<const Vec<T, 8>*>(b + o);
+#pragma unroll
+                        for (int k = 0; k < 8; k++) sum = fmaf(to_f32(va.v[k]), to_f32(vb.v[k]), sum);
+                    }
+                }
+            row[32 * s] = from_f32<T>(sum);
+        }
+    }
+}
+
 enum TcMode {
     TC_STORE = 0,  // tensor stores of the rounded product or of f32 split-K partials
     TC_BIAS,       // fuse 1..3, tensor stores
@@ -280,10 +324,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * MAX_STAGES + 2 + a); };
     volatile uint32_t* tmem_base_slot = reinterpret_cast<volatile uint32_t*>(smem + SmemLayout::bars + 8 * (2 * MAX_STAGES + 4));
 
+    int* const not_finite = reinterpret_cast<int*>(smem + SmemLayout::bars + 8 * (2 * MAX_STAGES + 5));  // CONV: a total of this CTA is not
     const int warp = warp_number(), lane = threadIdx.x & 31;
     const int bn = BN_T ? BN_T : p.bn, stages = BN_T ? STAGES : p.stages, stage_bytes = BN_T ? A_STAGE_BYTES + BN_T * BK * 2 : p.stage_bytes;
 
     if (threadIdx.x == 0) {
+        if (CONV) *not_finite = 0;
         for (int s = 0; s < MAX_STAGES; s++) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
@@ -533,6 +579,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     } else {
                         pack(e, q);
                     }
+                    if constexpr (CONV) {  // columns behind the tile's pixels hold what the ring and the accumulator held before
+                        const int mine = p.conv_rows * p.conv_w - c * EPI_CHUNK_COLS - half * CW;
+                        F32x2 zero[4] = {twice(0.0f), twice(0.0f), twice(0.0f), twice(0.0f)};  // NaN from the first total on that is not finite
+                        if (mine >= CW) {
+#pragma unroll
+                            for (int j = 0; j < CW; j += 2) zero[j / 2 % 4] = fma2(pair_of(make_float2(e[j], e[j + 1])), twice(0.0f), zero[j / 2 % 4]);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < CW; j += 2) zero[j / 2 % 4] = fma2(pair_of(make_float2(j < mine ? e[j] : 0.0f, j + 1 < mine ? e[j + 1] : 0.0f)), twice(0.0f), zero[j / 2 % 4]);
+                        }
+                        const float2 z = halves(zero[0] + zero[1] + (zero[2] + zero[3]));
+                        if (z.x + z.y != 0.0f) *not_finite = 1;
+                    }
                     flush(&map_d, col, q);
                 }
             };
@@ -620,6 +679,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+    if constexpr (CONV) {
+        if (!*not_finite) return;
+        int tm, tn, tb;
+        for (int it = 0; next_tile<PANELS>(it, p, tm, tn, tb); it++) {
+            const int width = p.conv_rows * p.conv_w;
+            const uint16_t* g = static_cast<const uint16_t*>(p.conv_g) + (size_t)tb * p.conv_oh * p.conv_ow * p.conv_co;
+            const ConvRedo q = {g, p.conv_wt, static_cast<uint16_t*>(p.d) + (size_t)tb * p.M * p.N, min(BM, p.M - tm * BM), min(width, p.N - tn * width), tm * BM, tn * width, p.N, p.conv_w, p.conv_x, p.conv_y,
+                                p.conv_kh, p.conv_kw, p.conv_co, p.conv_oh, p.conv_ow};
+            if (p.is_bf16) conv_redo<bf16>(q);
+            else conv_redo<f16>(q);
+        }
     }
 }
 
@@ -1439,6 +1510,12 @@ bool tc_conv_grad_input(bool is_bf16, uint64_t batch, uint64_t c, uint64_t h, ui
     p.conv_cb = (int)((co + BK - 1) / BK);
     p.conv_x = (int)pw;
     p.conv_y = (int)ph;
+    p.conv_kh = (int)kh;
+    p.conv_co = (int)co;
+    p.conv_oh = (int)oh;
+    p.conv_ow = (int)ow;
+    p.conv_g = g;
+    p.conv_wt = wt;
     p.M = (int)c;
     p.N = (int)(h * w);
     p.num_kb = (int)(kh * kw) * p.conv_cb;

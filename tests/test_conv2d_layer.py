@@ -213,3 +213,45 @@ def test_input_gradient_without_columns(cuda, dt, shape):
     step = 2.0 ** -9 if dt is D.BF16 else 2.0 ** -12
     terms = shape[4] * shape[5] * shape[6]
     assert np.all(np.abs(D.decode(got[2]["grad_x"], dt) - want) <= 1.001 * step * 2 * np.abs(want) + 2.0 ** -20 * _scales(shape)["grad_x"] * np.sqrt(terms) + 1e-7)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("what", ["weight_inf", "weight_nan", "many", "gradient", "channel"])
+@pytest.mark.parametrize("shape", [(2, 130, 9, 31, 64, 3, 3, 1, 1, 1, 1), (1, 64, 33, 56, 64, 7, 7, 1, 1, 3, 3), (2, 72, 12, 20, 64, 4, 2, 1, 1, 3, 0), (40, 128, 7, 7, 72, 3, 3, 1, 1, 1, 1)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_input_gradient_without_columns_keeps_what_is_not_finite(cuda, dt, shape, what):
+    """A pixel outside the gradient takes no part in a sum, whatever its weight: infinities and NaNs are where the definition and the columns' form have them, and all else is as without them."""
+    from maidenx_b200 import _lib
+    lib = _lib.load()
+    x, w, b, g = _data(17, dt, shape)
+    B, C, Hh, W, Co, kh, kw = shape[:7]
+    wf, gf = D.decode(w, dt).astype(np.float64).reshape(Co, C, kh, kw), D.decode(g, dt).astype(np.float64).reshape(B, Co, -1)
+    gf[gf == 0.0] = 0.5  # an infinity times one of these would be NaN in either form
+    if what == "weight_inf":
+        wf[Co - 1, 3, 0, 0], wf[0, C - 1, kh - 1, kw - 1] = np.inf, -np.inf
+    elif what == "weight_nan":
+        wf[5, 0, kh - 1, 0], wf[Co // 2, C // 2, 0, kw - 1] = np.nan, np.nan
+    elif what == "many":
+        wf[:, 1], wf[:, 2, 0], wf[3, :, kh // 2, 0] = np.inf, np.nan, -np.inf
+    elif what == "gradient":
+        gf[0, 1, 0], gf[B - 1, Co - 1, -1], gf[B // 2, 2, 5] = np.inf, np.nan, -np.inf
+    else:
+        wf[:, 7 % C], gf[0, 3, :4] = np.inf, np.nan
+    w, g = D.encode(wf.ravel(), dt), D.encode(gf.ravel(), dt)
+    got = {}
+    for mode in (0, 2):
+        lib.mx_debug_set_conv_implicit(mode)
+        try:
+            got[mode] = D.decode(CC.run_layer(dt, 1, shape, x, w, b, g)["grad_x"], dt)
+        finally:
+            lib.mx_debug_set_conv_implicit(1)
+    with np.errstate(all="ignore"):
+        want = CC.direct_conv_f64(shape, D.decode(x, dt), D.decode(w, dt), D.decode(b, dt), D.decode(g, dt))["grad_x"].reshape(-1)
+    for other in (got[0], want):
+        assert np.array_equal(np.isnan(got[2]), np.isnan(other)) and np.array_equal(np.isposinf(got[2]), np.isposinf(other)) and np.array_equal(np.isneginf(got[2]), np.isneginf(other))
+    fine = np.isfinite(want)
+    assert not fine.all() and fine.any()
+    step = 2.0 ** -9 if dt is D.BF16 else 2.0 ** -12
+    terms = Co * kh * kw
+    assert np.all(np.abs(got[2] - want)[fine] <= 1.001 * step * 2 * np.abs(want)[fine] + 2.0 ** -20 * _scales(shape)["grad_x"] * np.sqrt(terms) + 1e-7)
