@@ -331,7 +331,8 @@ void mx_linear_bias_gelu_f16(size_t rows, size_t in_features, size_t out_feature
  * gradient).  mode 0 issues exactly the calls the reference's layer issues (column buffer declared [B*oh*ow, K],
  * stride/padding slot order, col2im with num_els = B*C*H*W); mode 1 uses the same ops consistently (batched
  * product with the weight shared by every batch) and is a true convolution; there a 16-bit type's input gradient
- * with strides of 1 may be one product without columns, rounded once.  x [B, C, H, W], weight
+ * with strides of 1 may be one product without columns, rounded once, and the first two sums of its bias gradient
+ * one pass, each with its own rounding.  x [B, C, H, W], weight
  * [Cout, C, kh, kw], bias [Cout] or NULL, out / grad_out [B, Cout, oh, ow], all dense; `cols` has
  * mx_conv2d_cols_elems elements and carries im2col's result from forward to backward; `workspace` has
  * mx_conv2d_workspace_elems(conv, mode, backward) elements.  Any of grad_x / grad_weight / grad_bias may be NULL.

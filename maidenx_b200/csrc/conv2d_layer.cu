@@ -3,7 +3,7 @@
 // im2col -> matmul -> (views) -> bias add, and in backward matmul -> col2im for the input gradient, matmul for
 // the weight gradient and three sums for the bias gradient.  Every step is a call of a cuda_<op>_<dtype> symbol of
 // this library with the metadata the reference's tensor layer would build, but for 16-bit types' input gradient (one product without columns, where that is faster) and
-// the first two of their bias sums (one pass with the roundings of both).
+// the first two of their bias sums (one pass with the roundings of both), both in mode 1 alone.
 //
 // Two compositions are offered (argument `mode`):
 //
@@ -153,12 +153,12 @@ void plane_sums(const Geometry& g, const void* grad_out, void* out) {
     check_launch("mx_conv2d_backward");
 }
 
-// grad_bias = grad_out.sum(3).sum(2).sum(0) (conv.rs:283-288); tmp holds B*Co*oh + B*Co elements
-void bias_gradient(const Ops& ops, const Geometry& g, size_t es, const void* grad_out, char* tmp, void* grad_bias) {
+// grad_bias = grad_out.sum(3).sum(2).sum(0) (conv.rs:283-288); tmp holds B*Co*oh + B*Co elements.  The first two as one pass in mode 1 alone: mode 0 is the reference's calls.
+void bias_gradient(const Ops& ops, const Geometry& g, size_t es, int mode, const void* grad_out, char* tmp, void* grad_bias) {
     const size_t d4[4] = {g.B, g.Co, g.oh, g.ow}, d3[3] = {g.B, g.Co, g.oh}, d2[2] = {g.B, g.Co};
     char* t1 = tmp;
     char* t2 = tmp + round16(g.B * g.Co * g.oh) * es;
-    if (ops.half_kind && g.B * g.Co <= 0x7FFFFFFFull && g.oh <= 0x7FFFFFFFull && g.ow <= 0x7FFFFFFFull) {
+    if (mode == 1 && ops.half_kind && g.B * g.Co <= 0x7FFFFFFFull && g.oh <= 0x7FFFFFFFull && g.ow <= 0x7FFFFFFFull) {
         if (ops.half_kind == 1) plane_sums<bf16>(g, grad_out, t2);
         else plane_sums<f16>(g, grad_out, t2);
     } else {
@@ -282,7 +282,7 @@ void backward(const Ops& ops, size_t es, const MxConv2d* c, int mode, const void
             const size_t mm[15] = {2, 2, 2, g.K, g.Co, g.K, M, M, g.Co, 1, g.K, g.Co, 1, 0, 0};
             ops.matmul(g.K * g.Co, mm, cols, grad_flat, grad_w);
         }
-        if (grad_bias) bias_gradient(ops, g, es, grad_out, sums, grad_bias);
+        if (grad_bias) bias_gradient(ops, g, es, mode, grad_out, sums, grad_bias);
         return;
     }
     char* grad_cols = ws;
@@ -311,7 +311,7 @@ void backward(const Ops& ops, size_t es, const MxConv2d* c, int mode, const void
         const size_t fm[10] = {g.B, g.Co, g.P, g.Co * g.P, g.P, 1, 1, g.Co, 1, 0};
         ops.sum_to_shape(g.B * g.Co * g.P, 3, fm, grad_out, grad_bias);
     } else if (grad_bias) {
-        bias_gradient(ops, g, es, grad_out, sums, grad_bias);
+        bias_gradient(ops, g, es, mode, grad_out, sums, grad_bias);
     }
 }
 

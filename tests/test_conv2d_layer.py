@@ -254,4 +254,19 @@ def test_input_gradient_without_columns_keeps_what_is_not_finite(cuda, dt, shape
     assert not fine.all() and fine.any()
     step = 2.0 ** -9 if dt is D.BF16 else 2.0 ** -12
     terms = Co * kh * kw
-    assert np.all(np.abs(got[2] - want)[fine] <= 1.001 * step * 2 * np.abs(want)[fine] + 2.0 ** -20 * _scales(shape)["grad_x"] * np.sqrt(terms) + 1e-7)
+    assert np.all(np.abs(got[2][fine] - want[fine]) <= 1.001 * step * 2 * np.abs(want)[fine] + 2.0 ** -20 * _scales(shape)["grad_x"] * np.sqrt(terms) + 1e-7)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
+def test_literal_call_sequence_is_these_calls(cuda, dt):
+    """Mode 0 gives what the reference's calls give one after the other, bit for bit: here a sum in another order would not (each row holds a large number and its negative)."""
+    shape = (4, 3, 100, 223, 16, 3, 3, 1, 1, 1, 1)
+    x, w, b, _ = _data(18, dt, shape)
+    rng = np.random.default_rng(18)
+    g = rng.standard_normal((4 * 16 * 100, 223)) * 1e-3
+    at = np.argsort(rng.random(g.shape), axis=1)[:, :2]
+    np.put_along_axis(g, at, np.array([30000.0, -30000.0]), axis=1)
+    g = D.encode(g.ravel(), dt)
+    got, want = CC.run_layer(dt, 0, shape, x, w, b, g), CC.compose(cuda, dt, 0, shape, x, w, b, g)
+    assert np.array_equal(got["grad_bias"], want["grad_bias"])
