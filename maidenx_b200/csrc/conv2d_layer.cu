@@ -103,7 +103,7 @@ void sum_dim(const Ops& ops, const size_t* dims, size_t nd, size_t dim, const vo
 }
 
 // The first two of the bias gradient's sums, over rows and over their sums, each rounded: out[plane] = round(sum_h round(sum_w in[plane][h][w])).  A warp has a plane, G lanes a row of `nv`
-// vectors, four rows in flight.  Bound by HBM: one read of grad_out, where the sums as two launches took more than that ([64, 256, 56, 56] bf16 33 us, 26 so; rows of 14 [32, 256, 14, 14] 25 us, 4).
+// vectors, four rows in flight.  Bound by the trips of a warp through its plane, one after the other, and by HBM where planes fill the SMs: see plane_sums for where it is taken.
 constexpr int kPlaneThreads = 256;
 template <class T, int VEC, int G>
 __global__ void __launch_bounds__(kPlaneThreads) plane_sums_kernel(const T* in, T* out, size_t planes, uint32_t h, uint32_t w) {
@@ -142,15 +142,26 @@ __global__ void __launch_bounds__(kPlaneThreads) plane_sums_kernel(const T* in, 
     for (int o = 16; o >= G; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
     if (lane == 0) out[plane] = from_f32<T>(sum);
 }
+// false: the two sums as they are.  One warp a plane pays for small maps, where it saves a launch, until their planes fill the SMs (two sums / a warp each, us, bf16: 512 x 7 x 7 4.4 / 3.7, 840 x 27 x 24
+// 5.5 / 4.8, 4576 x 14 x 14 5.4 / 5.1, 8475 x 10 x 10 5.8 / 6.8, 28556 x 6 x 5 6.1 / 9.2), and for many planes of a middle size whose rows the first sum does not
+// read in whole lines: of vectors (16384 x 56 x 56 30.9 / 25.1, 12068 x 81 x 80 56.1 / 42.5; 1150 x 56 x 56 6.1 / 6.1, 2345 x 104 x 224 21.2 / 29.8, 15498 x 64 x 64 24.6 / 26.2) or by elements that fill
+// most of a warp's two rounds (16384 x 55 x 55 92 / 53, 2184 x 41 x 41 11.2 / 9.6; 16384 x 28 x 28 15.3 / 22.2, 4096 x 109 x 109 29.9 / 54.4).  A few large planes would wait for one
+// warp each: 16 x 112 x 112 4.8 / 11.3, 16 x 109 x 109 4.8 / 26.3, 16 x 512 x 512 5.8 / 114.
 template <class T>
-void plane_sums(const Geometry& g, const void* grad_out, void* out) {
+bool plane_sums(const Geometry& g, const void* grad_out, void* out) {
     const bool vec = g.ow % 8 == 0 && (uintptr_t)grad_out % 16 == 0;
     const size_t planes = g.B * g.Co, nv = vec ? g.ow / 8 : g.ow;
-    const auto kernel = vec ? (nv <= 4 ? plane_sums_kernel<T, 8, 4> : nv <= 8 ? plane_sums_kernel<T, 8, 8> : nv <= 16 ? plane_sums_kernel<T, 8, 16> : plane_sums_kernel<T, 8, 32>)
-                            : (nv <= 8 ? plane_sums_kernel<T, 1, 8> : nv <= 16 ? plane_sums_kernel<T, 1, 16> : plane_sums_kernel<T, 1, 32>);
+    if (planes > 0x7FFFFFFFull || g.oh > 0x7FFFFFFFull || g.ow > 0x7FFFFFFFull) return false;
+    const size_t lanes = vec && nv <= 4 ? 4 : nv <= 8 ? 8 : nv <= 16 ? 16 : 32, trips = (g.oh + 128 / lanes - 1) / (128 / lanes) * ((nv + lanes - 1) / lanes);
+    const bool small = trips <= 2 && planes <= 4096;
+    const bool many = planes >= 2048 && (vec ? trips >= 3 && trips <= 14 && g.ow >= 40 && g.ow % 64 != 0 : trips <= 32 && g.ow >= 40 && g.ow < 64);
+    if (!small && !many) return false;
+    const auto kernel = vec ? (lanes == 4 ? plane_sums_kernel<T, 8, 4> : lanes == 8 ? plane_sums_kernel<T, 8, 8> : lanes == 16 ? plane_sums_kernel<T, 8, 16> : plane_sums_kernel<T, 8, 32>)
+                            : (lanes == 8 ? plane_sums_kernel<T, 1, 8> : lanes == 16 ? plane_sums_kernel<T, 1, 16> : plane_sums_kernel<T, 1, 32>);
     launch_kernel(kernel, (unsigned)((planes + kPlaneThreads / 32 - 1) / (kPlaneThreads / 32)), kPlaneThreads, 0, ctx().stream, static_cast<const T*>(grad_out), static_cast<T*>(out), planes,
                   (uint32_t)g.oh, (uint32_t)g.ow);
     check_launch("mx_conv2d_backward");
+    return true;
 }
 
 // grad_bias = grad_out.sum(3).sum(2).sum(0) (conv.rs:283-288); tmp holds B*Co*oh + B*Co elements.  The first two as one pass in mode 1 alone: mode 0 is the reference's calls.
@@ -158,10 +169,8 @@ void bias_gradient(const Ops& ops, const Geometry& g, size_t es, int mode, const
     const size_t d4[4] = {g.B, g.Co, g.oh, g.ow}, d3[3] = {g.B, g.Co, g.oh}, d2[2] = {g.B, g.Co};
     char* t1 = tmp;
     char* t2 = tmp + round16(g.B * g.Co * g.oh) * es;
-    if (mode == 1 && ops.half_kind && g.B * g.Co <= 0x7FFFFFFFull && g.oh <= 0x7FFFFFFFull && g.ow <= 0x7FFFFFFFull) {
-        if (ops.half_kind == 1) plane_sums<bf16>(g, grad_out, t2);
-        else plane_sums<f16>(g, grad_out, t2);
-    } else {
+    const bool fused = mode == 1 && (ops.half_kind == 1 ? plane_sums<bf16>(g, grad_out, t2) : ops.half_kind == 2 && plane_sums<f16>(g, grad_out, t2));
+    if (!fused) {
         sum_dim(ops, d4, 4, 3, grad_out, t1);
         sum_dim(ops, d3, 3, 2, t1, t2);
     }

@@ -270,3 +270,29 @@ def test_literal_call_sequence_is_these_calls(cuda, dt):
     g = D.encode(g.ravel(), dt)
     got, want = CC.run_layer(dt, 0, shape, x, w, b, g), CC.compose(cuda, dt, 0, shape, x, w, b, g)
     assert np.array_equal(got["grad_bias"], want["grad_bias"])
+
+
+# batch, channels, height, width: lanes a row by vectors (4, 8, 16, 32) and by elements (8, 16, 32), one and two trips, many planes of middle sizes - and, from "sums" on, maps whose two sums stay as they are
+BIAS_SUMS = [(1, 16, 13, 8), (3, 40, 33, 32), (2, 8, 31, 56), (1, 9, 15, 104), (1, 5, 7, 136), (2, 3, 4, 480), (7, 40, 16, 7), (5, 64, 14, 14), (1, 33, 4, 63), (32, 64, 20, 48), (64, 32, 33, 41),
+             "sums", (1, 16, 112, 112), (1, 16, 55, 55), (1, 64, 56, 56), (2, 3, 300, 200), (70, 60, 7, 7), (64, 32, 28, 28)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", [D.BF16, D.F16], ids=lambda d: d.name)
+@pytest.mark.parametrize("case", [c for c in BIAS_SUMS if c != "sums"], ids=str)
+def test_bias_gradient_s_sums(cuda, dt, case):
+    """Whole numbers, whose sums are exact in f32: the bits of the sums one after the other, whichever way they are taken.  Where a warp a plane does not pay they are those calls, and then also
+    have their bits for rows that a sum in another order would change."""
+    B, Co, h, w = case
+    shape = (B, 1, h, w, Co, 1, 1, 1, 1, 0, 0)
+    rng = np.random.default_rng(19)
+    data = [rng.integers(-8, 9, (B * Co * h, w)).astype(np.float64)]
+    if BIAS_SUMS.index(case) > BIAS_SUMS.index("sums"):
+        g = rng.standard_normal(data[0].shape) * 1e-3
+        np.put_along_axis(g, np.argsort(rng.random(g.shape), axis=1)[:, :2], np.array([30000.0, -30000.0]), axis=1)
+        data.append(g)
+    x, wt = D.encode(rng.standard_normal(B * h * w), dt), D.encode(rng.standard_normal(Co), dt)
+    for g in data:
+        g = D.encode(g.ravel(), dt)
+        got, want = CC.run_layer(dt, 1, shape, x, wt, None, g), CC.compose(cuda, dt, 1, shape, x, wt, None, g)
+        assert np.array_equal(got["grad_bias"], want["grad_bias"])
