@@ -40,7 +40,7 @@ int mx_debug_gemm_max_resident_pairs(void);
  * possible. */
 void mx_debug_set_conv_implicit(int mode);
 /* f32 products as pairs of f16 values: 1 = by the rule on their cost (default), 0 = never, 2 = wherever possible, 3 = the same, emptying the accumulator after
- * every k-block of 64.  The query: the calling thread's last f32 product ran as pairs in this many slices (0: not as pairs). */
+ * every 32 values of K.  The query: the calling thread's last f32 product ran as pairs in this many slices (0: not as pairs). */
 void mx_debug_set_gemm_f32_pairs(int mode);
 int mx_debug_gemm_f32_last_pairs(void);
 /* 16-bit operands whose rows are 16-byte multiples but no whole 128-byte lines are copied in lines where that pays: 1 = by the rule (default), 0 = never, 2 =

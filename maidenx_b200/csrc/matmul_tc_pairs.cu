@@ -441,7 +441,7 @@ bool opt_in_shared_memory() {
     return true;
 }
 
-std::atomic<int> g_pairs{1};  // 0: never, 2: wherever possible, 3: the same with the accumulator emptied after every k-block (tests, A/B timing)
+std::atomic<int> g_pairs{1};  // 0: never, 2: wherever possible, 3: the same with the accumulator emptied after every 32 values of K (tests, A/B timing)
 thread_local int t_last_pairs = 0;
 std::atomic<unsigned long long> g_next_tag{1};
 
@@ -572,7 +572,7 @@ bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, uint64_t partial_by
 
 }  // namespace mx
 
-// 1 (default): f32 products as pairs of f16 by the rule on their cost; 0: never; 2: wherever possible; 3: the same, emptying the accumulator after every k-block
+// 1 (default): f32 products as pairs of f16 by the rule on their cost; 0: never; 2: wherever possible; 3: the same, emptying the accumulator after every 32 values of K
 extern "C" void mx_debug_set_gemm_f32_pairs(int mode) { mx::g_pairs.store(mode, std::memory_order_relaxed); }
 // of the calling thread's last f32 product: 0 not as pairs, else its slices
 extern "C" int mx_debug_gemm_f32_last_pairs(void) { return mx::t_last_pairs; }
