@@ -44,8 +44,9 @@ void mx_debug_set_conv_implicit(int mode);
 void mx_debug_set_gemm_f32_pairs(int mode);
 int mx_debug_gemm_f32_last_pairs(void);
 /* 16-bit operands whose rows are 16-byte multiples but no whole 128-byte lines are copied in lines where that pays: 1 = by the rule (default), 0 = never, 2 =
- * always. */
+ * always.  The query: the operands that the calling thread's last product on the tensor cores copied first, for this or because it had to (1 A, 2 B). */
 void mx_debug_set_gemm_realign(int mode);
+int mx_debug_gemm_last_copies(void);
 /* Short reductions (K <= 256, one batch, many row tiles) keep the B panel of a column tile in shared memory and stream
  * only A.  set: 1 = on (default), 0 = always the general schedule.  The query returns the CTAs per column tile a launch
  * with these tile counts takes (0 = general schedule). */

@@ -85,6 +85,7 @@ RUNTIME_SIGNATURES = {
     "mx_debug_gemm_f32_last_pairs": ([], ctypes.c_int),
     "mx_debug_set_conv_implicit": ([ctypes.c_int], None),
     "mx_debug_set_gemm_realign": ([ctypes.c_int], None),
+    "mx_debug_gemm_last_copies": ([], ctypes.c_int),
     "mx_debug_set_gemm_f32_cluster": ([ctypes.c_int], None),
     "mx_debug_set_gemm_f32_wide": ([ctypes.c_int], None),
     "mx_debug_gemm_f32_last_form": ([ctypes.POINTER(ctypes.c_int)], None),

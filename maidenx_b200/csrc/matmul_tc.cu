@@ -1127,17 +1127,19 @@ uint64_t copy_pitch(size_t es, uint64_t rows, uint64_t cols) {
 }
 
 // A 16-bit operand whose rows lie 16-byte multiples apart, but no whole 128-byte lines: each row of a tensor copy's box reads parts of two lines.  What that costs a
-// product is counted in us a KB of the box and k-block (bf16 4096 x 1536 x 1024 15.0 us; x 1000, 16 bytes off, 24.4, x 1008 18.3, x 992 16.6), on as many
-// k-blocks as a CTA has (of long reductions cut into slices at least a quarter); a copy in lines costs its bytes, read and written, at 5 TB/s, and 1.5 us where
+// product is counted in us a KB of the box's rows inside the matrix and k-block (bf16 4096 x 1536 x 1024 15.0 us; x 1000, 16 bytes off, 24.4, x 1008 18.3, x 992 16.6), on as many
+// k-blocks as an SM has of the whole product: with few tiles its slices of K run side by side; a copy in lines costs its bytes, read and written, at 5 TB/s, and 2 us where
 // no other operand has to be copied.  In place / by the rule, us: 4104^3 209 / 137, 4112^3 135 / 127, 4128^3 both 126, 4096 x 1536 x 1000 24.6 / 19.9, 16384 x 4088 x
-// 520 97 / 79, 8192 x 1000 x 1000 25.0 / 20.4, and both alike 1024 x 1024 x 1000 8.2, 16384 x 200 x 200 10.2.  The products' sums are the same either way.
+// 520 97 / 79, 8192 x 1000 x 1000 25.0 / 20.4, and both alike 1024 x 1024 x 1000 8.2, 16384 x 200 x 200 10.2.  Left in place, copied: 336 x 8 x 11560 10.0, 13.1; 224 x 32 x 10248 12.3,
+// 15.6; 5440 x 6800 x 168 20.2, 22.6 (reductions of fewer than five k-blocks are bound by their output).  The products' sums are the same either way.
 std::atomic<int> g_realign{1};  // 0: never, 2: always (tests, A/B timing)
+thread_local int t_last_copies = 0;  // operands that the thread's last product copied: 1 A, 2 B (tests)
 constexpr uint64_t kRealignMost = 256ull << 20;  // what the workspace pool keeps between calls, halved: beyond it a call would map memory anew
-static double misaligned_us(const TcProduct& c, uint64_t pitch, int box_kb) {
-    const uint64_t off = pitch * 2 % 128;
-    const double us_kb = off == 0 ? 0.0 : off % 32 ? 0.006 : off % 64 ? 0.0025 : 0.00125;
+static double misaligned_us(const TcProduct& c, uint64_t pitch, double box_kb) {
+    const uint64_t off = pitch * 2 % 128, num_kb = (c.k + 63) / 64;
+    const double us_kb = off == 0 || num_kb < 5 ? 0.0 : off % 32 ? 0.006 : off % 64 ? 0.0025 : 0.00125;
     const double tiles = (double)c.batch * (double)((c.m + 127) / 128) * (double)((c.n + 255) / 256);
-    return us_kb * box_kb * (double)((c.k + 63) / 64) * std::max(0.25, tiles / sm_count());
+    return us_kb * box_kb * (double)num_kb * tiles / sm_count();
 }
 static double copy_us(uint64_t rows, uint64_t cols) { return (double)rows * (double)cols * 4.0 / 5.0e6; }
 
@@ -1158,12 +1160,13 @@ bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* w
         const bool a_dense = !c.a_bs || c.a_bs == (int64_t)(c.m * c.k), b_dense = !c.b_bs || c.b_bs == (int64_t)(c.k * c.n);
         const auto fits = [&](uint64_t rows, uint64_t pitch) { return rows * pitch * es <= kRealignMost / 2; };
         const bool a_may = !a_copy && a_dense && a_pitch != a_cols && fits(a_rows, a_pitch), b_may = !b_copy && b_dense && b_pitch != b_cols && fits(b_rows, b_pitch);
-        const double a_gain = a_may ? std::max(0.0, misaligned_us(c, a_cols, 16) - copy_us(a_rows, a_cols)) : 0.0;
-        const double b_gain = b_may ? std::max(0.0, misaligned_us(c, b_cols, 32) - copy_us(b_rows, b_cols)) : 0.0;
-        const bool pays = mode == 2 || a_gain + b_gain > (needed ? 0.0 : 1.5);
+        const double a_gain = a_may ? std::max(0.0, misaligned_us(c, a_cols, std::min<double>(16, c.m / 8.0)) - copy_us(a_rows, a_cols)) : 0.0;
+        const double b_gain = b_may ? std::max(0.0, misaligned_us(c, b_cols, std::min<double>(32, c.n / 8.0)) - copy_us(b_rows, b_cols)) : 0.0;
+        const bool pays = mode == 2 || a_gain + b_gain > (needed ? 0.0 : 2.0);
         a_copy = a_copy || (pays && a_may && (mode == 2 || a_gain > 0.0));
         b_copy = b_copy || (pays && b_may && (mode == 2 || b_gain > 0.0));
     }
+    t_last_copies = 0;
     if (!a_copy && !b_copy) return true;
     const uint64_t a_bytes = a_copy ? (a_rows * a_pitch * es + 255) / 256 * 256 : 0, b_bytes = b_copy ? b_rows * b_pitch * es : 0;
     if (a_bytes / 16 + b_bytes / 16 > 0x7FFFFFFFull) return !needed;  // the copy counts vectors in 32 bits
@@ -1182,6 +1185,7 @@ bool repack_operands(size_t es, TcProduct& c, StreamWorkspace& ws, const char* w
     };
     if (es == 2) launch(uint16_t());
     else launch(uint32_t());
+    t_last_copies = (a_copy ? 1 : 0) + (b_copy ? 2 : 0);
     if (a_copy) {
         c.A = a_dst;
         c.a_pitch = a_pitch;
@@ -1605,6 +1609,7 @@ extern "C" int mx_debug_gemm_max_resident_pairs(void) { return mx::tc2::max_resi
 extern "C" void mx_debug_set_gemm_group_m(int rows) { mx::g_group_m.store(rows > 0 ? rows : 16, std::memory_order_relaxed); }
 // 1 (default): products with a reduction of at most 256 run with the B panel resident in shared memory; 0: general schedule
 extern "C" void mx_debug_set_gemm_keep_b(int on) { mx::g_keep_b.store(on ? 1 : 0, std::memory_order_relaxed); }
+extern "C" int mx_debug_gemm_last_copies(void) { return mx::tc::t_last_copies; }
 extern "C" void mx_debug_set_gemm_realign(int mode) { mx::tc::g_realign.store(mode, std::memory_order_relaxed); }
 extern "C" int mx_debug_gemm_keep_b_ctas(int tiles_m, int tiles_n, int num_kb, int batch, int ctas) { return mx::keep_b_ctas(tiles_m, tiles_n, num_kb, batch, ctas); }
 extern "C" int mx_debug_gemm_last_schedule(void) { return mx::t_last_schedule; }

@@ -1046,3 +1046,15 @@ def test_products_in_pairs_are_cut_along_k_under_capture(cuda, case):
         lib.mx_debug_set_gemm_f32_pairs(1)
     assert seen["pairs"] > 0 and seen["slices"] > 1 and torch.equal(replayed, tf32)
     assert float((direct - replayed).norm() / replayed.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("m,n,k,copies", [(336, 8, 11560, 0), (224, 32, 10248, 0), (24, 24, 10592, 0), (200, 8, 6896, 0), (544, 680, 168, 0), (2504, 2480, 3688, 3)], ids=str)
+def test_which_operands_off_whole_lines_are_copied(cuda, m, n, k, copies):
+    """Few tiles, whose slices of K run side by side, and short reductions are read in place; many tiles of a long reduction are worth the copies."""
+    from maidenx_b200 import _lib
+    rng = np.random.default_rng(0)
+    a, b = (D.encode(rng.standard_normal(s), D.BF16) for s in (m * k, n * k))
+    got = H.run_matmul(cuda, D.BF16, H.matmul_metadata([m, n], [m, k], [k, n], [k, 1], [1, k], 0, 0), m * n, a, b)
+    assert _lib.load().mx_debug_gemm_last_copies() == copies
+    ref = D.decode(a, D.BF16).reshape(m, k).astype(np.float64) @ D.decode(b, D.BF16).reshape(n, k).T.astype(np.float64)
+    assert np.all(np.abs(D.decode(got, D.BF16).reshape(m, n) - ref) <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -22 * k)
