@@ -22,6 +22,7 @@
 //
 // The caller owns every buffer, as everywhere in this ABI: `cols` (B*P*K elements) is written by forward and read
 // by backward; `workspace` holds the intermediates (sizes from mx_conv2d_workspace_elems).
+#include <algorithm>
 #include <atomic>
 
 #include "abi_common.cuh"
@@ -237,6 +238,27 @@ void forward(const Ops& ops, size_t es, const MxConv2d* c, int mode, const void*
 
 std::atomic<int> g_implicit{1};  // 0: never, 2: wherever possible (tests, A/B timing)
 
+// Whether the input gradient in one product is faster than by columns: half a tile's rows and a third of the SMs at least, and then by what the product takes (`per`: k-blocks of a 256-wide tile, one
+// after the other on an SM, parts of tiles and of waves included) for each million elements of columns that are not written, multiplied and added up.  What columns cost goes by the planes of
+// grad_out: whole 128-byte lines the first product and col2im read at their best, vectors off the lines less so, ragged planes several times that.  A kernel of 5 x 5 or 7 x 7 has the
+// most columns for each input element; 1 x 1 is one product either way, without columns only where its planes lie off the lines.  The lines stand where 700 random layers have them, of which
+// 33 are slower than by columns with this rule (a quarter of half a tile's rows and a third of the SMs alone).  Columns / in one product, us: 3 x 3 64 x 256 x 56 x 56 -> 256 365 / 205, 24 x 352 x 56 x 56 -> 32
+// 639 / 54, 36 x 224 x 14 x 14 -> 112 36 / 21; left: 11 x 88 x 56 x 56 -> 8 25 / 33, 50 x 112 x 28 x 28 -> 488 95 / 123, 3 x 223 x 56 x 56 -> 328 29 / 43; 7 x 7 34 x 208 x 14 x 14 -> 408 116 / 140; 1 x 1 23 x 427
+// x 48 x 48 -> 8 31 / 49, but 48 x 344 x 14 x 14 -> 48 28 / 15.
+bool implicit_pays(const Geometry& g) {
+    const size_t most = 256 / g.W < g.H ? 256 / g.W : g.H, blocks = (g.H + most - 1) / most, rows = (g.H + blocks - 1) / blocks, bn = (rows * g.W + 15) / 16 * 16, sms = (size_t)sm_count();
+    const size_t tiles = g.B * ((g.C + 127) / 128) * blocks, taps = g.kh * g.kw, num_kb = taps * ((g.Co + 63) / 64);
+    if (g.C < 64 || tiles * 3 < sms) return false;
+    const double serial = (double)((tiles + sms - 1) / sms * num_kb) * std::max((128 + bn) / 512.0, 0.4), columns = (double)g.B * g.K * g.P * 1e-6, per = serial / columns;
+    const double useful = (double)g.B * g.C * g.H * g.W * taps * g.Co / (128.0 * 256 * 64) / ((double)sms * serial);  // of the multiplications
+    const bool lines = g.P % 64 == 0, ragged = g.P % 8 != 0;
+    if (taps == 1) return !lines && (columns > 0.96 || tiles <= sms);
+    if (taps >= 20) return ragged ? per <= 6.0 || g.P < 64 : per <= (taps >= 40 ? 3.9 : 2.7);
+    if (ragged) return per <= 2.7 || g.Co <= 280;
+    if (lines) return columns > 31 ? per <= 1.0 : columns > 21 && per <= 0.6 && useful > 1.0 / 12;
+    return per <= 1.15 || per <= (columns > 60 ? 2.2 : columns > 30 ? 1.76 : 0.0) || (per <= 4.0 && useful > 0.6);
+}
+
 // 16-bit types, strides of 1: the input gradient without its columns, from grad_out with the channels last and the transposed weights, both in the place of the columns.
 bool implicit_grad_x(const Ops& ops, const Geometry& g, const void* grad_out, const void* w, char* place, void* grad_x) {
     const int mode = g_implicit.load(std::memory_order_relaxed);
@@ -244,10 +266,7 @@ bool implicit_grad_x(const Ops& ops, const Geometry& g, const void* grad_out, co
     const size_t g_elems = (g.B * g.P * g.Co + 63) / 64 * 64;
     char* base = reinterpret_cast<char*>(((uintptr_t)place + 127) & ~(uintptr_t)127);
     if (g_elems + g.K * g.Co + 64 > g.B * g.K * g.P) return false;
-    // Half a tile's rows and a third of the SMs: columns / in one product, the whole backward pass and forward of a bf16 layer 3 x 3, us: 64 x 256 x 56 x 56 -> 256 1024 / 854, 64 x 64 x 7 x 7 -> 64 (64
-    // tiles) 45.2 / 41.5, 16 x 128 x 20 x 20 -> 96 (32) 43.4 / 44.5, 2 x 256 x 14 x 14 -> 256 (4) 48.8 / 58.6, 64 x 16 x 28 x 28 -> 32 58.8 / 65.7; 1 x 1: 64 x 256 x 14 x 14 -> 64 57.8 / 46.0.
-    const size_t rows = 256 / g.W < g.H ? 256 / g.W : g.H, tiles = g.B * ((g.C + 127) / 128) * ((g.H + rows - 1) / rows);
-    if (mode == 1 && (g.C < 64 || tiles * 3 < (size_t)sm_count())) return false;
+    if (mode == 1 && !implicit_pays(g)) return false;
     char *last = base, *wt = base + g_elems * 2;
     const size_t gm[7] = {g.B, g.P, g.Co, g.Co * g.P, 1, g.P, 0};
     ops.contiguous(g.B * g.P * g.Co, 3, gm, grad_out, last);

@@ -296,3 +296,28 @@ def test_bias_gradient_s_sums(cuda, dt, case):
         g = D.encode(g.ravel(), dt)
         got, want = CC.run_layer(dt, 1, shape, x, wt, None, g), CC.compose(cuda, dt, 1, shape, x, wt, None, g)
         assert np.array_equal(got["grad_bias"], want["grad_bias"])
+
+
+# a few output channels on planes of whole lines, a ragged plane with many, more rows of weights than columns pay for - and maps, ragged or large, whose columns cost more
+ROUTES = [((11, 88, 56, 56, 8, 3, 3, 1, 1, 1, 1), "columns"), ((14, 152, 28, 28, 408, 3, 3, 1, 1, 0, 0), "columns"), ((13, 80, 28, 28, 288, 3, 3, 1, 1, 1, 1), "columns"),
+          ((36, 224, 14, 14, 112, 3, 3, 1, 1, 1, 1), "one product"), ((8, 192, 56, 56, 64, 3, 3, 1, 1, 1, 1), "one product"), ((42, 153, 14, 14, 16, 7, 7, 1, 1, 0, 0), "one product")]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,way", ROUTES, ids=str)
+def test_which_input_gradients_go_without_columns(cuda, shape, way):
+    """The rule on sizes takes the way that was measured to be the faster one: the bits of the switch for that way, which differ where sums are rounded once and not once a tap."""
+    from maidenx_b200 import _lib
+    lib, dt = _lib.load(), D.BF16
+    rng = np.random.default_rng(20)
+    oh, ow, P, K = CC.geometry(*shape)
+    B, C, Hh, W, Co = shape[:5]
+    x, w, g = (D.encode(rng.standard_normal(n).astype(np.float32), dt) for n in (B * C * Hh * W, Co * K, B * Co * P))
+    got = {}
+    for mode in (0, 1, 2):
+        lib.mx_debug_set_conv_implicit(mode)
+        try:
+            got[mode] = CC.run_layer(dt, 1, shape, x, w, None, g)["grad_x"]
+        finally:
+            lib.mx_debug_set_conv_implicit(1)
+    assert not np.array_equal(got[0], got[2]) and np.array_equal(got[1], got[0 if way == "columns" else 2])
