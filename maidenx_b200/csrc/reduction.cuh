@@ -430,10 +430,11 @@ __device__ __noinline__ void fold_columns(const typename RedTraits<T, KIND>::Acc
 // aligned base.
 // Vectors of 16-bit floats are held to four blocks an SM (see fold_published), maxima of eight-byte integers to five (they took 54 registers instead of 44 since
 // the wait at the top, four blocks: [48950, 873] u64 66 us before, 74, 54 so).  0: the compiler's own choice for all others; 1 would let it take every register (bf16 [130, 300000] 9.0 us, 9.8; minima of f32 [811, 2, 13536] 403, 888).
-template <class T, int KIND>
-constexpr int kColBlocks = is_half_v<T> ? 4 : KIND >= RED_MAX && std::is_integral<T>::value && sizeof(T) == 8 ? 5 : 0;
+// The means of f64 with their fold together would take 58 registers and four blocks, 48 without it ([6856, 1784] 11.9 us, 15.9 so).
+template <class T, int KIND, bool TOGETHER = false>
+constexpr int kColBlocks = is_half_v<T> ? 4 : (KIND >= RED_MAX && std::is_integral<T>::value && sizeof(T) == 8) || (TOGETHER && KIND == RED_MEAN && sizeof(T) == 8) ? 5 : 0;
 template <class T, int KIND, int VEC, bool TOGETHER = false>
-__global__ void __launch_bounds__(kColLanes* kColRows, VEC > 1 ? kColBlocks<T, KIND> : 0) reduce_cols_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial, u64 O,
+__global__ void __launch_bounds__(kColLanes* kColRows, VEC > 1 ? kColBlocks<T, KIND, TOGETHER> : 0) reduce_cols_kernel(const T* in, T* out, typename RedTraits<T, KIND>::Acc* partial, u64 O,
                                                                          u64 R, u64 I, u64 seg, u32 splits, u64 factor, u32* counters) {
     after_previous_kernel();
     typedef RedTraits<T, KIND> TR;
@@ -515,7 +516,9 @@ __global__ void __launch_bounds__(kColLanes* kColRows, VEC > 1 ? kColBlocks<T, K
 template <class T, int KIND, int VEC>
 auto reduce_cols_choice(bool vec, u64 splits) {
     constexpr int TV = VEC < kColRows ? VEC : 1;  // a wider vector's columns have a thread each
-    if (vec) return TV == VEC && splits >= 2 * kColFoldTogether ? reduce_cols_kernel<T, KIND, TV, true> : reduce_cols_kernel<T, KIND, VEC>;
+    // what the means of f64 spill for it counts while a thread adds few parts ([11394, 1174], 31 parts, 17.8 us, 19.5 together; 2 x [45888, 146] 26.6, 23.6)
+    constexpr u64 FROM = kColFoldTogether * (KIND == RED_MEAN && sizeof(T) == 8 ? 5 : 2);
+    if (vec) return TV == VEC && splits >= FROM ? reduce_cols_kernel<T, KIND, TV, true> : reduce_cols_kernel<T, KIND, VEC>;
     return splits >= kColFoldTogether ? reduce_cols_kernel<T, KIND, 1, true> : reduce_cols_kernel<T, KIND, 1>;
 }
 
