@@ -99,6 +99,9 @@ MANY_PLANES = [
     ("large-planes-few-outputs", 2, 3, 150, 150, 15, 15, 0, 0, 15, 15),
     ("large-planes", 1, 3, 160, 160, 3, 3, 1, 1, 2, 2),
     ("even-kernel", 3, 257, 6, 10, 2, 4, 1, 0, 1, 3),
+    ("one-output-row", 9, 120, 7, 31, 7, 7, 0, 0, 1, 1),   # square kernels by ranges: most of a pixel's terms lie outside
+    ("a-quarter-of-the-terms", 9, 120, 12, 12, 7, 7, 0, 0, 1, 1),
+    ("half-of-the-terms", 9, 120, 14, 14, 5, 5, 0, 0, 1, 1),
     ("plane-beyond-shared-memory", 1, 2, 170, 331, 3, 3, 1, 1, 2, 2),
 ]
 
