@@ -1013,7 +1013,7 @@ __global__ void __launch_bounds__(kEwThreads) ew_chan_kernel(F f, const T* a, co
 // SHIFTED, for rows of kEwRepeatLong and more: the repeated row's vectors from the two aligned words they lie in instead of by elements, which meet in L1's banks ([4099, 1543] bf16 6.1 us,
 // 4.9 so, [2277, 5799] 10.5, 7.8; f32 [8191, 1023] 9.7, 8.9).  In shorter rows the vectors that wrap, which go by elements, are in too many warps ([30000, 197] bf16 5.2,
 // 6.1), below two vectors a thread the way to the words is longer than what they save ([3, 100001] bf16 1.7, 2.0), and quotients and saturating sums of 16 bits have
-// no registers for it ([5789, 3853] f32 28.1, 31.6; [12489, 523] i16 7.5, 8.4).
+// no registers for it ([5789, 3853] f32 28.1, 31.6; [12489, 523] i16 7.5, 8.4), nor comparisons, whose vectors are longer ([11611, 4195] f32 >= 37.5, 43.6; [16463, 637] f16 8.8, 9.5).
 constexpr uint32_t kEwRepeatLong = 512;
 template <class F>
 struct EwShiftsRepeated : std::true_type {};
@@ -1224,7 +1224,7 @@ void ew_launch(const EwPlan& pl, const F& f, const T* a, const T* b, O* out, con
                         break;
                     }
                     if (ew_fill_repeat_params(D, VEC, Q)) {
-                        constexpr bool kShifts = EwShiftsRepeated<F>::value && (is_half_v<T> || std::is_same<T, f32>::value);
+                        constexpr bool kShifts = EwShiftsRepeated<F>::value && std::is_same<T, O>::value && (is_half_v<T> || std::is_same<T, f32>::value);
                         if (kShifts && Q.q >= kEwRepeatLong && Q.units > 1) launch_kernel(ew_repeat_kernel<F, T, O, VEC, kShifts>, blocks, kEwThreads, 0, s, f, a, b, out, Q);
                         else launch_kernel(ew_repeat_kernel<F, T, O, VEC>, blocks, kEwThreads, 0, s, f, a, b, out, Q);
                         break;
