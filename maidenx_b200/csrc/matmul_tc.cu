@@ -1134,7 +1134,7 @@ uint64_t copy_pitch(size_t es, uint64_t rows, uint64_t cols) {
 // 15.6; 5440 x 6800 x 168 20.2, 22.6 (reductions of fewer than five k-blocks are bound by their output).  The products' sums are the same either way.
 std::atomic<int> g_realign{1};  // 0: never, 2: always (tests, A/B timing)
 thread_local int t_last_copies = 0;  // operands that the thread's last product copied: 1 A, 2 B (tests)
-constexpr uint64_t kRealignMost = 256ull << 20;  // what the workspace pool keeps between calls, halved: beyond it a call would map memory anew
+constexpr uint64_t kRealignMost = 256ull << 20;  // half of what the workspace pools keep between calls: beyond it a call would map memory anew
 static double misaligned_us(const TcProduct& c, uint64_t pitch, double box_kb) {
     const uint64_t off = pitch * 2 % 128, num_kb = (c.k + 63) / 64;
     const double us_kb = off == 0 || num_kb < 5 ? 0.0 : off % 32 ? 0.006 : off % 64 ? 0.0025 : 0.00125;

@@ -445,7 +445,7 @@ std::atomic<int> g_pairs{1};  // 0: never, 2: wherever possible, 3: the same wit
 thread_local int t_last_pairs = 0;
 std::atomic<unsigned long long> g_next_tag{1};
 
-// Bytes of a call's workspace: what the pool keeps between calls.  Beyond it each call maps memory anew, which took longer than pairs gain: [13712 x 4025] by 59
+// Bytes of a call's workspace: what the pools keep of it between calls.  Beyond it each call maps memory anew, which took longer than pairs gain: [13712 x 4025] by 59
 // columns and its gradients 772 us in tf32, 1180 while the copies behind the gate had memory of their own, 716 in the pairs'.
 constexpr uint64_t kPairsMost = 512ull << 20;
 

@@ -1058,3 +1058,24 @@ def test_which_operands_off_whole_lines_are_copied(cuda, m, n, k, copies):
     assert _lib.load().mx_debug_gemm_last_copies() == copies
     ref = D.decode(a, D.BF16).reshape(m, k).astype(np.float64) @ D.decode(b, D.BF16).reshape(n, k).T.astype(np.float64)
     assert np.all(np.abs(D.decode(got, D.BF16).reshape(m, n) - ref) <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -22 * k)
+
+
+def test_large_workspaces_of_two_sizes_find_each_other_s_block(cuda):
+    """Products whose workspaces are 392 and 401 MB, in turn behind a synchronisation: the larger one's block serves both, and no call maps memory."""
+    import torch
+
+    from maidenx_b200 import _lib, device
+    lib, n, k = _lib.load(), 12, 16147
+    a, b, out = torch.ones(6200, k, device="cuda"), torch.ones(n, k, device="cuda"), torch.empty(6200, n, device="cuda")
+    lib.mx_debug_set_gemm_f32_pairs(2)
+    try:
+        for _ in range(3):
+            torch.cuda.synchronize()
+            before = torch.cuda.mem_get_info()[0]
+            for m in (6065, 6200):
+                device.dispatch("matmul", "f32", H.matmul_metadata([m, n], [m, k], [k, n], [k, 1], [1, k], 0, 0), m * n, "META", a.data_ptr(), b.data_ptr(), out.data_ptr())
+                assert lib.mx_debug_gemm_f32_last_pairs() > 0
+            mapped = before - torch.cuda.mem_get_info()[0]
+        assert mapped < 64 << 20 and bool((out == k).all())
+    finally:
+        lib.mx_debug_set_gemm_f32_pairs(1)
