@@ -449,11 +449,11 @@ std::atomic<unsigned long long> g_next_tag{1};
 // columns and its gradients 772 us in tf32, 1180 while the copies behind the gate had memory of their own, 716 in the pairs'.
 constexpr uint64_t kPairsMost = 512ull << 20;
 
-// From which time in the tf32 kernel on pairs are considered, and by a seventh they have to be faster there, what the estimates are off by.  The two to four launches more, their tensor maps and
+// From which time in the tf32 kernel on pairs are considered, and by an eighth they have to be faster there, what the estimates are off by.  The two to four launches more, their tensor maps and
 // the workspace are 5 us of the calling thread (3.4 to 9.6 us a call, 8.7 to 14.4 as pairs): below this line a pass that is issued from the host waits for them.
 // Linear layers op by op, forward and gradients, tf32 / pairs, us: 550 x 192 -> 630 41.9 / 52.2, 596 x 53 -> 3816 62.4 / 75.2, 880 x 43 -> 792 39.2 / 46.9; 162 x (635 x 16 x 88) and its
 // gradients 92.7 / 120.
-constexpr double kPairsLeastUs = 28.0;
+constexpr double kPairsLeastUs = 24.0;
 
 struct Plan {
     uint64_t a_rows, a_cols, b_rows, b_cols, a_zs, b_zs, a_pitch, b_pitch, a_bytes, b_bytes, a_scales, b_scales;
@@ -502,7 +502,7 @@ bool tc_launch_f32_pairs(const TcProduct& c, double tf32_us, uint64_t partial_by
     if (!mode) return false;
     if (c.batch > 0x3FFF || c.m > 0x3FFFFFFF || c.n > 0x3FFFFFFF || c.k > 0x3FFFFFFF) return false;
     const Plan q = make_plan(c);
-    if (q.a_bytes + q.b_bytes >= kPairsMost || (mode == 1 && (tf32_us < kPairsLeastUs || 1.15 * q.cost > tf32_us))) return false;
+    if (q.a_bytes + q.b_bytes >= kPairsMost || (mode == 1 && (tf32_us < kPairsLeastUs || 1.12 * q.cost > tf32_us))) return false;
     if (q.a_zs * ((q.a_rows + 127) / 128) * ((q.a_cols + 127) / 128) + q.b_zs * ((q.b_rows + 127) / 128) * ((q.b_cols + 127) / 128) > 0x7FFFFFFFull) return false;
     if (!opt_in_shared_memory()) return false;
     auto line = [](uint64_t bytes) { return (bytes + 255) / 256 * 256; };
