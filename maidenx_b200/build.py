@@ -23,7 +23,8 @@ CSRC = PKG_DIR / "csrc"
 INCLUDE = PKG_DIR.parent / "include"
 BUILD = CSRC / "build"
 LIB_PATH = PKG_DIR / "libmaidenx_cuda.so"
-DISPATCH_PATH = PKG_DIR / "_dispatch.so"  # extension module: device.dispatch as one native call
+# extension module: device.dispatch as one native call, for the interpreter that builds it
+DISPATCH_PATH = PKG_DIR / f"_dispatch{sysconfig.get_config_var('EXT_SUFFIX')}"
 
 # suffix -> class id (see abi_common.cuh)
 DTYPES = {
@@ -136,6 +137,7 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False, p
 
 def build_dispatch(force: bool = False) -> Path:
     src = CSRC / "pydispatch.cpp"
+    (PKG_DIR / "_dispatch.so").unlink(missing_ok=True)  # without the interpreter's tag, which any would load
     if force or not DISPATCH_PATH.exists() or DISPATCH_PATH.stat().st_mtime < max(src.stat().st_mtime, Path(__file__).stat().st_mtime):
         cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(DISPATCH_PATH)]
         r = subprocess.run(cmd, capture_output=True, text=True)

@@ -1078,6 +1078,7 @@ bool softmax_rows_any_launch(const T* in, T* out, u64 rows, u32 n, cudaStream_t 
     const u32 words = n / 2 + 1;  // at most
     // Pairs: rows of few words always or from one an SM on, longer ones where their fewer warps still fill the SMs (us, elements / pairs: 300 rows of 127 bf16 1.65 / 2.02, 5000 2.16 / 2.25, 37824 6.55 / 5.68; 5000 of 197 2.60 /
     // 3.07, 37824 8.98 / 7.95; 5000 of 333 3.65 / 3.22), and those of 512 and more, which keep a warp to a row.
+    // What a row has less than its bracket's last word is work for nothing: brackets at octaves to 64 words, at its thirds to 128 (80, 104), at its half to 256.
     if constexpr (is_half_v<T> && G == 32) if (words <= 16 || words > 256 || rows >= (words <= 32 ? 1 : words <= 128 ? 128 : 24) * (u64)sm_count()) {
         auto pairs = [&](auto kernel, int g) {
             launch_kernel(kernel, (unsigned)((rows + kExThreads / g - 1) / (kExThreads / g)), kExThreads, 0, s, in, out, rows, n);

@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kFusedThreads, is_half_v<T> || SUM ? 5 : 6) ge
         for (int i = 0; i < UN; i++)
             if (v0 + i * stride < nvec) {
                 Vec<T, VEC> o;
-if constexpr (is_half_v<T>) {
+                if constexpr (is_half_v<T>) {
 #pragma unroll
                     for (int j = 0; j < VEC / 2; j++) {
                         const float2 r = halves(pair_of(unpack2<T>(words(g[i])[j])) * gelu_grad_pair(unpack2<T>(words(x[i])[j])));

@@ -304,14 +304,14 @@ enum TcMode {
 // with one), and so do tiles with a bias or an activation: their arithmetic is what a wave of few narrow tiles ends with (training step of two layers 1024 x 2048 x 2048 96.2 us, 94.5 so;
 // 256 x 256 x 256 34.9, 33.9) and what full-width tiles of a short reduction wait for (8192 x 4096 x 512 with GELU 58.3 us, 46.9 so; 4096 x 4096 x 1024 39.5, 35.2); products that only leave
 // through the copy engine gain nothing from a second one (16384 x 4096 x 256: 55 us, 50 with one; 128 x (384 x 384 x 64) and its gradients 31.1, 29.8).
-constexpr int epi_warps(int mode, int bn_t, bool drain) { return mode == TC_PLAIN || (mode == TC_BIAS && !drain) ? 2 : 1; }
+constexpr int epi_warps(int mode, bool drain) { return mode == TC_PLAIN || (mode == TC_BIAS && !drain) ? 2 : 1; }
 constexpr int tc_threads(int w) { return 32 * (2 + 4 * w); }
 // CONV (TC_PLAIN): TcParams::conv_*; an instantiation of its own for the producer's sake too.
 template <int MODE, int BN_T, bool DRAIN = false, bool PANELS = false, bool CONV = false>
-__global__ void __launch_bounds__(tc_threads(epi_warps(MODE, BN_T, DRAIN)), 1)
+__global__ void __launch_bounds__(tc_threads(epi_warps(MODE, DRAIN)), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                const __grid_constant__ CUtensorMap map_d2, TcParams p, int* err, int tag) {
-    constexpr int W = epi_warps(MODE, BN_T, DRAIN), CW = EPI_CHUNK_COLS / W;  // columns of a chunk that a warp has
+    constexpr int W = epi_warps(MODE, DRAIN), CW = EPI_CHUNK_COLS / W;  // columns of a chunk that a warp has
     extern __shared__ unsigned char tc_smem_raw[];
     // 128-byte swizzled TMA tiles and UMMA descriptors want 1024-byte aligned bases
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -915,7 +915,7 @@ bool launch_gemm(bool is_bf16, const TcProduct& c, void* D, const char* where, i
                         : drain ? (p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0, true> : (fuse ? tc_gemm_kernel<TC_BIAS, 0, true> : tc_gemm_kernel<TC_STORE, 0, true>))
                         : p.d_plain ? tc_gemm_kernel<TC_PLAIN, 0>
                                   : (fuse ? (full ? tc_gemm_kernel<TC_BIAS, BN> : tc_gemm_kernel<TC_BIAS, 0>) : (full ? tc_gemm_kernel<TC_STORE, BN> : tc_gemm_kernel<TC_STORE, 0>));
-    const int warps = epi_warps(p.d_plain ? TC_PLAIN : fuse ? TC_BIAS : TC_STORE, panels || full ? BN : 0, drain);
+    const int warps = epi_warps(p.d_plain ? TC_PLAIN : fuse ? TC_BIAS : TC_STORE, drain);
     launch_kernel(kernel, grid, tc_threads(warps), TC_SMEM_BYTES, ctx().stream, ma, mb, md, md2, p, err, tag);
     check_launch(where);
     if (slices > 1) splitk_reduce(is_bf16 ? 0 : 1, static_cast<const float*>(partial.ptr), slices, M, N, n_pitch, D, where);
@@ -1556,7 +1556,7 @@ bool tc_conv_grad_input(bool is_bf16, uint64_t batch, uint64_t c, uint64_t h, ui
     int grid = sm_count();
     if (ctx().gemm_sm_limit > 0 && ctx().gemm_sm_limit < grid) grid = ctx().gemm_sm_limit;
     if (grid > p.num_tiles) grid = p.num_tiles;
-    launch_kernel(tc_gemm_kernel<TC_PLAIN, 0, false, false, true>, grid, tc_threads(epi_warps(TC_PLAIN, 0, false)), TC_SMEM_BYTES, ctx().stream, ma, mb, ma, ma, p, err, tag);
+    launch_kernel(tc_gemm_kernel<TC_PLAIN, 0, false, false, true>, grid, tc_threads(epi_warps(TC_PLAIN, false)), TC_SMEM_BYTES, ctx().stream, ma, mb, ma, ma, p, err, tag);
     check_launch(where);
     return true;
 }
