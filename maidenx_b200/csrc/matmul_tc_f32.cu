@@ -664,13 +664,13 @@ Choice choose(const TcProduct& c) {
                                        [](int n) { return resident_clusters(reinterpret_cast<const void*>(tc_gemm_f32_kernel<0, CLUSTERED>), THREADS, SMEM_BYTES, n); });
         if (f.cluster) f.slices = f.cluster;
     }
-    // us of a k-block of 128 columns, of a tile's end, of the launch and of what else is launched, fitted to 1400 products of 1.6e7 to 3e11 multiply-adds (four of five within 11 %)
+    // us of a k-block of 64 or 128 columns, of a tile's end, of the launch and of what else is launched, fitted to 1400 products of 1.6e7 to 3e11 multiply-adds (four of five within 11 %)
     const int bn = f.slices > 1 ? f.bn_cut : f.bn_whole, per = (num_kb + f.slices - 1) / f.slices;
     const double waves = (double)((batch * tiles_m * ((c.n + bn - 1) / bn) * f.slices + f.grid - 1) / f.grid), columns = bn / 128.0;
     const bool wide = !c.ragged && f.slices == 1 && num_kb >= kWideLeast;
     const double copies = (c.a_repack ? (double)(c.a_bs ? c.batch : 1) * c.m * c.k : 0.0) + (c.b_repack ? (double)(c.b_bs ? c.batch : 1) * c.n * c.k : 0.0);
-    f.us = waves * ((c.ragged ? 1.09 : 0.87) * per * (128 + bn) / 256.0 + (c.d_plain && f.slices == 1 ? 4.5 : wide ? 0.25 : 0.73) * columns) + 5.0 + (f.cluster ? 3.4 : f.slices > 1 ? 2.5 : 0.0) +
-           (copies > 0 ? 1.6 + copies * 8 / 8.6e6 : 0.0);
+    const double kb_us = bn == 64 ? (c.ragged ? 0.79 : 0.76) : c.ragged ? 1.06 : 0.86, end_us = c.d_plain && f.slices == 1 ? 5.9 : wide ? 0.6 : 0.8;
+    f.us = waves * (kb_us * per + end_us * columns) + 4.7 + (f.cluster ? 3.3 : f.slices > 1 ? 2.8 : 0.0) + (copies > 0 ? 1.4 + copies * 8 / 8.1e6 : 0.0);
     return f;
 }
 

@@ -19,7 +19,7 @@
 // tf32 kernel / pairs, all launches, us: 4096^3 745 to 850 / 380, 2048 x 2048 x 1024 62 / 34, 4100 x 1544 x 1000 85 / 48, ragged 4099 x 1543 x 1000 124 / 62, 32 x (1152 x
 // 196 x 256) with one A 34.6 / 23.8, [256 x 1152] by 32 x [1152 x 196] 36.0 / 30.6; small products and short reductions stay there (512 x 1024 x 1024 17.5 / 22.5, 128 x (384 x
 // 384 x 64) 25.5 / 35). Error against 64 bits (2-norm): K = 1024 normal 4.2e-7 / 2.1e-7, positive 6.6e-7 / 4.6e-7; ragged forms, whose accumulator is emptied every 32
-// values of K, 2.4e-7 / 1.5e-7, positive 1.85e-7 / 1.1e-7.  What bounds the loop: tensor pipe 59 % busy, its stages of 64 KB wait for L2.
+// values of K, 2.4e-7 / 1.5e-7, positive 1.85e-7 / 1.1e-7.  What bounds the loop: tensor pipe 61 % busy (4096 x 4096 x 2048), its stages of 64 KB wait for L2.
 #include <cuda.h>
 
 #include <algorithm>
@@ -358,7 +358,7 @@ struct SplitOperand {
 constexpr int SPLIT_THREADS = 512, SPLIT_ROWS = BLOCK / (SPLIT_THREADS / 32);
 
 // One block of 128 x 128 elements: read once into registers, its largest and its smallest nonzero magnitude found, written as pairs.  Bound by HBM or L2:
-// four bytes read and four written an element ([256 x 1152] and 32 x [1152 x 196] 7.5 us).
+// four bytes read and four written an element ([256 x 1152] and 32 x [1152 x 196] 12.9 us behind the im2col that writes the latter).
 __global__ void __launch_bounds__(SPLIT_THREADS) split_pairs_kernel(SplitOperand a, SplitOperand b, unsigned long long* unfit, unsigned long long tag) {
     __shared__ uint32_t part[2][SPLIT_THREADS / 32];
     after_previous_kernel();
@@ -453,7 +453,7 @@ constexpr uint64_t kPairsMost = 512ull << 20;
 // the workspace are 5 us of the calling thread (3.4 to 9.6 us a call, 8.7 to 14.4 as pairs): below this line a pass that is issued from the host waits for them.
 // Linear layers op by op, forward and gradients, tf32 / pairs, us: 550 x 192 -> 630 41.9 / 52.2, 596 x 53 -> 3816 62.4 / 75.2, 880 x 43 -> 792 39.2 / 46.9; 162 x (635 x 16 x 88) and its
 // gradients 92.7 / 120.
-constexpr double kPairsLeastUs = 24.0;
+constexpr double kPairsLeastUs = 22.0;
 
 struct Plan {
     uint64_t a_rows, a_cols, b_rows, b_cols, a_zs, b_zs, a_pitch, b_pitch, a_bytes, b_bytes, a_scales, b_scales;
