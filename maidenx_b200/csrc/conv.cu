@@ -497,10 +497,11 @@ void col2im_entry(size_t num_els, const size_t* meta, const T* col, T* out, cons
     const uint64_t col_plane = (uint64_t)P.KH * P.KW * P.OH * P.OW;
     const uint32_t pb = P.SH == 1 && P.SW == 1 && planes <= 0x7FFFFFFFull && col_plane && HW < 0x7FFFFFFFull ? planes_per_block(planes, col_plane * sizeof(T), 1, 48 * 1024) : 0;
     if (pb && pb * HW < 0x7FFFFFFFull && pb * HW >= kConvThreads / 2 && (HW <= kConvThreads || ((planes + pb - 1) / pb >= 512 && (sizeof(T) < 8 || P.KH * P.KW == 1)))) {
-        // terms at fixed distances where at least half of a pixel's lie inside the columns' planes; the ranges skip the others (7 x 7 without padding, by all 49 terms / by the ranges, us: [7, 281, 7, 61] f32
-        // 20.6 / 10.6, [52, 209, 48, 8] bf16 251 / 95, [9, 310, 11, 63] 80 / 48)
-        const uint32_t k = P.KH == P.KW && 2 * (uint64_t)P.OH * P.OW >= HW ? P.KH : 0;
-        const auto kernel = k == 3 ? col2im_planes_kernel<T, 3> : k == 5 ? col2im_planes_kernel<T, 5> : k == 7 ? col2im_planes_kernel<T, 7> : col2im_planes_kernel<T, 0>;
+        // Terms at fixed distances (by the ranges / so, us): 3 x 3, [300, 100, 14, 14] f32 94 / 42, and 5 x 5 in rows of an even length, [300, 100, 14, 14] bf16 181 / 144; odd ones, [300, 100, 13, 13] bf16
+        // 190 / 220, and the 49 terms of 7 x 7, [300, 100, 7, 7] bf16 86 / 184, gain nothing from it.  And where at least half of a pixel's terms lie inside the columns' planes; the ranges skip the others (7 x 7
+        // without padding [52, 209, 48, 8] bf16 95 / 251).
+        const bool inside = P.KH == P.KW && 2 * (uint64_t)P.OH * P.OW >= HW;
+        const auto kernel = inside && P.KH == 3 ? col2im_planes_kernel<T, 3> : inside && P.KH == 5 && P.W % 2 == 0 ? col2im_planes_kernel<T, 5> : col2im_planes_kernel<T, 0>;
         launch_kernel(kernel, (unsigned)((planes + pb - 1) / pb), kConvThreads, pb * col_plane * sizeof(T), s, col, out, ConvPlanes(P, planes, pb));
         check_launch(where);
         return;
