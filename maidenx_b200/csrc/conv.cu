@@ -65,7 +65,7 @@ __device__ __forceinline__ void stage_run(T* dst, const T* src, uint32_t count) 
 // lanes meet in its banks): [32, 128, 14, 14] f32, 3 x 3: 7 us, 12 with the places found anew for every plane, 23 with one plane and one kernel offset at a time.
 // GROUPS: the block has more than one group; with a single one places kept for later cost what they take ([39, 170, 25, 25] bf16 45.7 us, 48.4).
 template <class T, int VEC, bool GROUPS>
-__global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* x, T* col, ConvPlanes P, uint32_t step) {
+__global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* x, T* col, ConvPlanes P, uint32_t group) {
     after_previous_kernel();
     extern __shared__ __align__(16) unsigned char conv_smem[];
     T* img = reinterpret_cast<T*>(conv_smem);
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kConvThreads) im2col_planes_kernel(const T* x,
         }
         return;
     }
-    const uint32_t period = step * KK * OHW, hop = step * HW;
+    const uint32_t period = group * KK * OHW, hop = group * HW;
     for (uint32_t e0 = threadIdx.x * VEC; e0 < min(total, period); e0 += kConvThreads * VEC) {
         uint32_t row, o, plane, kk, kh, kw, ho, wo;
         P.ohw_div.divmod(e0, row, o);
@@ -355,6 +355,19 @@ static uint64_t planes_most(size_t es, uint64_t step, uint64_t ohw) {
     return es == 2 || ohw < kConvThreads ? kConvSmemMost : 48 * 1024;
 }
 
+// Planes of a group of the flat im2col, whose places a thread keeps from group to group: a multiple of `step` whose vectors nearly fill the block's
+// threads, else the fewest that hold 48 vectors, twice at least in the block's `per_block` planes; else all of these, one group.  Many idle threads cost
+// less than places found anew ([30000, 7, 7] f32 3 x 3, 441 vectors: 22.1 -> 10.1 us; [30000, 14, 14] bf16 1 x 1 stride 2, 49: 5.0 -> 4.0), but a few threads
+// that write vector after vector cost more (groups of `step` planes, against one group: [30000, 5, 5] bf16 2 x 2, 8 vectors: 5.0 -> 9.2 us; [30000, 7, 7] 1 x 1
+// stride 2, 2: 3.8 -> 9.0), and full threads are best ([30000, 7, 7] bf16 5 x 5 stride 2, 50 vectors: 15.2 us in one group, 13.3 in groups of 1, 8.3 of 5).
+static uint32_t planes_per_group(uint32_t per_block, uint64_t step, uint64_t chunk, uint64_t vec) {
+    const uint64_t vecs = step * chunk / vec;  // of `step` planes
+    if (vecs == 0) return per_block;
+    uint64_t n = std::max<uint64_t>(1, kConvThreads / vecs);
+    if (8 * n * vecs < 7 * kConvThreads || 2 * n * step > per_block) n = vecs < 16 ? per_block : (48 + vecs - 1) / vecs;
+    return 2 * n * step <= per_block ? (uint32_t)(n * step) : per_block;
+}
+
 // im2col: is the flat form faster than a block per plane and a kernel offset at a time?  It is where a plane's vectors are whole on
 // their own (step 1: [16, 64, 30, 30] f32 3 x 3 15.1 -> 11.9 us, [64, 64, 29, 29] bf16 7 x 7 stride 4 113 -> 16.6).  Where `step` planes
 // have to share a block to make whole vectors, enough blocks must be left ([4, 64, 27, 27] f32, 64 blocks: 6.3 -> 10.5 us; [16, 64, 21, 21],
@@ -418,9 +431,10 @@ void im2col_entry(size_t num_els, const size_t* meta, const T* x, T* col, const 
     // four groups share their places where two blocks an SM are left ([32, 128, 14, 14] bf16, a group of two planes: 10.0 us with one group a block)
     if (pb && pb < 4 * step && 4 * step * plane_bytes <= 16 * 1024 && planes_touched >= 4 * step * 2 * (uint64_t)sm_count()) pb = (uint32_t)(4 * step);
     if (pb && pb * chunk < 0x7FFFFFFFull && planes_pay(sizeof(T), step, (planes_touched + pb - 1) / pb, ohw)) {
-        const auto kernel = pb > step ? im2col_planes_kernel<T, VEC, true> : im2col_planes_kernel<T, VEC, false>;
+        const uint32_t group = planes_per_group(pb, step, chunk, VEC);
+        const auto kernel = pb > group ? im2col_planes_kernel<T, VEC, true> : im2col_planes_kernel<T, VEC, false>;
         allow_shared_memory(kernel, pb * plane_bytes);
-        launch_kernel(kernel, (unsigned)((planes_touched + pb - 1) / pb), kConvThreads, pb * plane_bytes, s, x, col, ConvPlanes(P, planes_touched, pb), (uint32_t)step);
+        launch_kernel(kernel, (unsigned)((planes_touched + pb - 1) / pb), kConvThreads, pb * plane_bytes, s, x, col, ConvPlanes(P, planes_touched, pb), group);
     } else if (plane_bytes <= kConvSmemMost) {
         auto launch = [&](auto kernel) {
             allow_shared_memory(kernel, plane_bytes);

@@ -91,6 +91,7 @@ MANY_PLANES = [
     # name, B, C, H, W, kh, kw, ph, pw, sh, sw: enough planes for several per block, maps that are whole vectors and maps that are not
     ("14x14", 7, 131, 14, 14, 3, 3, 1, 1, 1, 1),
     ("7x7-s2", 5, 211, 7, 7, 3, 3, 1, 1, 2, 2),
+    ("7x7-s2-groups", 120, 293, 7, 7, 3, 3, 1, 1, 2, 2),  # 29 planes a block, in groups of 7 (f32) or 14 (16-bit types), the last one cut short
     ("9x11-5x5", 3, 300, 9, 11, 5, 5, 2, 2, 1, 1),
     ("1x1-odd", 4, 401, 5, 5, 1, 1, 0, 0, 1, 1),
     ("17x19", 4, 200, 17, 19, 3, 3, 1, 1, 1, 1),      # more pixels than a block has threads, blocks enough
