@@ -242,8 +242,9 @@ std::atomic<int> g_implicit{1};  // 0: never, 2: wherever possible (tests, A/B t
 // Whether the input gradient in one product is faster than by columns: half a tile's rows and a third of the SMs at least, and then by what the product takes (`per`: k-blocks of a 256-wide tile, one
 // after the other on an SM, parts of tiles and of waves included) for each million elements of columns that are not written, multiplied and added up.  What columns cost goes by the planes of
 // grad_out: whole 128-byte lines the first product and col2im read at their best, vectors off the lines less so, ragged planes several times that.  A kernel of 5 x 5 or 7 x 7 has the
-// most columns for each input element; 1 x 1 is one product either way, without columns only where its planes lie off the lines.  The lines stand where 700 random layers have them, of which
-// 33 are slower than by columns with this rule (a quarter of half a tile's rows and a third of the SMs alone).  Columns / in one product, us: 3 x 3 64 x 256 x 56 x 56 -> 256 365 / 205, 24 x 352 x 56 x 56 -> 32
+// most columns for each input element; 1 x 1 is one product either way, without columns only where its planes lie off the lines.  Pixels of grad_out (its channels last)
+// that are not whole 32-byte sectors cost the kernel half as much again and more (`whole`: 23 x 152 x 32 x 32, 5 x 5 to 208, 216, 224 channels 92, 141, 85 us, by columns 81; 1 x 184 x 112 x 112, 7 x 7
+// to 440, 448 channels 198, 103, by columns 171).  The lines stand where 2500 random layers have them.  Columns / in one product, us: 3 x 3 64 x 256 x 56 x 56 -> 256 365 / 205, 24 x 352 x 56 x 56 -> 32
 // 639 / 54, 36 x 224 x 14 x 14 -> 112 36 / 21; left: 11 x 88 x 56 x 56 -> 8 25 / 33, 50 x 112 x 28 x 28 -> 488 95 / 123, 3 x 223 x 56 x 56 -> 328 29 / 43; 7 x 7 34 x 208 x 14 x 14 -> 408 116 / 140; 1 x 1 23 x 427
 // x 48 x 48 -> 8 31 / 49, but 48 x 344 x 14 x 14 -> 48 28 / 15.
 bool implicit_pays(const Geometry& g) {
@@ -252,11 +253,17 @@ bool implicit_pays(const Geometry& g) {
     if (g.C < 64 || tiles * 3 < sms) return false;
     const double serial = (double)((tiles + sms - 1) / sms * num_kb) * std::max((128 + bn) / 512.0, 0.4), columns = (double)g.B * g.K * g.P * 1e-6, per = serial / columns;
     const double useful = (double)g.B * g.C * g.H * g.W * taps * g.Co / (128.0 * 256 * 64) / ((double)sms * serial);  // of the multiplications
-    const bool lines = g.P % 64 == 0, ragged = g.P % 8 != 0;
+    const bool lines = g.P % 64 == 0, ragged = g.P % 8 != 0, whole = g.Co % 16 == 0;
     if (taps == 1) return !lines && (columns > 0.96 || tiles <= sms);
-    if (taps >= 20) return ragged ? per <= 6.0 || g.P < 64 : per <= (taps >= 40 ? 3.9 : 2.7);
-    if (ragged) return per <= 2.7 || g.Co <= 280;
-    if (lines) return columns > 31 ? per <= 1.0 : columns > 21 && per <= 0.6 && useful > 1.0 / 12;
+    if (taps >= 20 && lines && g.P > 64 && g.H * g.W % 64 == 0) {  // col2im writes whole lines too
+        const bool seven = taps >= 40;
+        if (g.Co % 64 == 0) return seven ? per <= 3.0 : per <= 1.7 || (per <= 2.7 && useful > 0.4);
+        if (whole) return per <= (seven ? 1.8 : 1.4) || (per <= 2.2 && useful > 0.5);
+        return per <= (seven ? 1.2 : 0.8);
+    }
+    if (taps >= 20) return ragged ? per <= (whole ? 6.0 : 4.0) || g.P < 64 : per <= (taps >= 40 ? 3.9 : 2.7);
+    if (ragged) return whole ? per <= 2.7 || g.Co <= 280 : per <= 1.95 || g.Co <= 136 || (per <= 2.2 && useful > 0.6);
+    if (lines) return columns > 31 ? per <= (whole ? 1.0 : 0.79) : columns > 21 && per <= 0.6 && useful > 1.0 / 12;
     return per <= 1.15 || per <= (columns > 60 ? 2.2 : columns > 30 ? 1.76 : 0.0) || (per <= 4.0 && useful > 0.6);
 }
 

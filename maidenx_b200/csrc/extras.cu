@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(kExThreads) softmax_rows_any_kernel(const T* i
 
 // The same for 16-bit types by the aligned 4-byte words a row lies in: half the loads, stores and conversions, and no checks in the arithmetic, since what does not belong to the row counts as -inf.
 // The words at a row's ends hold one element of it, which is stored by itself.  G lanes a row (32 but for rows of few words), K words a lane.
-// Bound by instructions, a third of them per row and not per element, so that rows share a warp: [192 x 197, 197] bf16 8.0 us, 9.0 by elements, [200000, 13] 7.5, 19.8, [37824, 513] 27.6, 40.2.
+// Bound by instructions, a third of them per row and not per element, so that rows share a warp: [192 x 197, 197] bf16 8.5 us, 10.4 by elements, [200000, 13] 7.5, 19.8, [37824, 513] 27.6, 40.2.
 template <class T, int G, int K>
 __global__ void __launch_bounds__(kExThreads) softmax_rows_pairs_kernel(const T* in, T* out, u64 rows, u32 n) {
     after_previous_kernel();

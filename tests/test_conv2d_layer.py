@@ -298,8 +298,10 @@ def test_bias_gradient_s_sums(cuda, dt, case):
         assert np.array_equal(got["grad_bias"], want["grad_bias"])
 
 
+# A wide kernel on planes of whole lines, with pixels of grad_out that are not in whole 32 bytes and that are;
 # a few output channels on planes of whole lines, a ragged plane with many, more rows of weights than columns pay for - and maps, ragged or large, whose columns cost more
-ROUTES = [((11, 88, 56, 56, 8, 3, 3, 1, 1, 1, 1), "columns"), ((14, 152, 28, 28, 408, 3, 3, 1, 1, 0, 0), "columns"), ((13, 80, 28, 28, 288, 3, 3, 1, 1, 1, 1), "columns"),
+ROUTES = [((4, 80, 64, 64, 248, 5, 5, 1, 1, 2, 2), "columns"), ((3, 184, 56, 56, 160, 5, 5, 1, 1, 2, 2), "one product"),
+          ((11, 88, 56, 56, 8, 3, 3, 1, 1, 1, 1), "columns"), ((14, 152, 28, 28, 408, 3, 3, 1, 1, 0, 0), "columns"), ((13, 80, 28, 28, 288, 3, 3, 1, 1, 1, 1), "columns"),
           ((36, 224, 14, 14, 112, 3, 3, 1, 1, 1, 1), "one product"), ((8, 192, 56, 56, 64, 3, 3, 1, 1, 1, 1), "one product"), ((42, 153, 14, 14, 16, 7, 7, 1, 1, 0, 0), "one product")]
 
 
