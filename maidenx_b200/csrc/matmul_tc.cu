@@ -120,10 +120,15 @@ struct TcParams {
     // CONV: the product's B is read out of images, K runs over a kernel's taps and, for each, over the channels of B's images in k-blocks (conv_cb of them); a column tile
     // is conv_rows whole rows of an output image of width conv_w, whose source pixels for tap (i, j) begin at row + conv_y - i, column conv_x - j.
     int conv_cb, conv_kw, conv_rows, conv_w, conv_x, conv_y;
-    int conv_kh, conv_co, conv_oh, conv_ow;  // and both operands as plain memory, for conv_redo
-    const void *conv_g, *conv_wt;
     int poll_ns;  // between the epilogue's looks at a tile's accumulator: 3 to 4 % of the time a tile's reduction takes (training step of 512 x 1024 x 1024 49.5 us at 400, 48.8 so)
 };
+// CONV: and both operands as plain memory, for conv_redo.  Not among the parameters of the other kernels: a launch that the host does not run ahead of takes 2.02 us where its parameters, rounded up to
+// 16 bytes, end 32 behind a multiple of 64, and 2.40 where they end elsewhere (4 maps, these and two words: 668 bytes; with this 700, and three products of 23 x 45 x 496 x 123 19.0 us for 17.8).
+struct TcConvParams : TcParams {
+    int conv_kh, conv_co, conv_oh, conv_ow;
+    const void *conv_g, *conv_wt;
+};
+static_assert((4 * sizeof(CUtensorMap) + sizeof(TcParams) + sizeof(int*) + sizeof(int) + 15) / 16 * 16 % 64 == 32, "parameters of tc_gemm_kernel");
 
 __device__ __forceinline__ void tile_coords(int tile, const TcParams& p, int& tm, int& tn, int& tb) {
     tb = tile / p.tiles_per_batch;
@@ -306,11 +311,11 @@ enum TcMode {
 // through the copy engine gain nothing from a second one (16384 x 4096 x 256: 55 us, 50 with one; 128 x (384 x 384 x 64) and its gradients 31.1, 29.8).
 constexpr int epi_warps(int mode, bool drain) { return mode == TC_PLAIN || (mode == TC_BIAS && !drain) ? 2 : 1; }
 constexpr int tc_threads(int w) { return 32 * (2 + 4 * w); }
-// CONV (TC_PLAIN): TcParams::conv_*; an instantiation of its own for the producer's sake too.
+// CONV (TC_PLAIN): TcConvParams; an instantiation of its own for the producer's sake too.
 template <int MODE, int BN_T, bool DRAIN = false, bool PANELS = false, bool CONV = false>
 __global__ void __launch_bounds__(tc_threads(epi_warps(MODE, DRAIN)), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
-               const __grid_constant__ CUtensorMap map_d2, TcParams p, int* err, int tag) {
+               const __grid_constant__ CUtensorMap map_d2, std::conditional_t<CONV, TcConvParams, TcParams> p, int* err, int tag) {
     constexpr int W = epi_warps(MODE, DRAIN), CW = EPI_CHUNK_COLS / W;  // columns of a chunk that a warp has
     extern __shared__ unsigned char tc_smem_raw[];
     // 128-byte swizzled TMA tiles and UMMA descriptors want 1024-byte aligned bases
@@ -710,12 +715,15 @@ bool opt_in_shared_memory() {
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
         for (auto kernel : {tc_gemm_kernel<TC_STORE, BN>, tc_gemm_kernel<TC_BIAS, BN>, tc_gemm_kernel<TC_STORE, 0>, tc_gemm_kernel<TC_BIAS, 0>, tc_gemm_kernel<TC_PLAIN, 0>, tc_gemm_kernel<TC_STORE, BN, false, true>, tc_gemm_kernel<TC_BIAS, BN, false, true>,
-                            tc_gemm_kernel<TC_STORE, 0, true>, tc_gemm_kernel<TC_BIAS, 0, true>, tc_gemm_kernel<TC_PLAIN, 0, true>,
-                            tc_gemm_kernel<TC_PLAIN, 0, false, false, true>})
+                            tc_gemm_kernel<TC_STORE, 0, true>, tc_gemm_kernel<TC_BIAS, 0, true>, tc_gemm_kernel<TC_PLAIN, 0, true>})
             if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess) {
                 cudaGetLastError();
                 return false;
             }
+        if (cudaFuncSetAttribute(tc_gemm_kernel<TC_PLAIN, 0, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
         done[dev] = true;
     }
     return true;
@@ -1506,7 +1514,7 @@ bool conv_grad_input_fits(uint64_t batch, uint64_t c, uint64_t h, uint64_t w, ui
 bool tc_conv_grad_input(bool is_bf16, uint64_t batch, uint64_t c, uint64_t h, uint64_t w, uint64_t co, uint64_t kh, uint64_t kw, uint64_t ph, uint64_t pw, uint64_t oh, uint64_t ow,
                         const void* g, const void* wt, void* grad_x, const char* where) {
     if (!conv_grad_input_fits(batch, c, h, w, co, kh, kw, ph, pw) || ((uintptr_t)g | (uintptr_t)wt) % 16 != 0 || (uintptr_t)grad_x % 2 != 0 || !opt_in_shared_memory()) return false;
-    TcParams p = {};
+    TcConvParams p = {};
     const uint64_t blocks = (h + 256 / w - 1) / (256 / w);
     p.conv_rows = (int)((h + blocks - 1) / blocks);
     p.conv_w = (int)w;
