@@ -144,8 +144,9 @@ __global__ void __launch_bounds__(kPlaneThreads) plane_sums_kernel(const T* in, 
     if (lane == 0) out[plane] = from_f32<T>(sum);
 }
 // false: the two sums as they are.  One warp a plane pays for small maps, where it saves a launch, until their planes fill the SMs (two sums / a warp each, us, bf16: 512 x 7 x 7 4.4 / 3.7, 840 x 27 x 24
-// 5.5 / 4.8, 5720 x 32 x 32 6.5 / 5.5, 4576 x 14 x 14 5.4 / 5.1, 8475 x 10 x 10 5.8 / 6.8, 28556 x 6 x 5 6.1 / 9.2), and for many planes of a middle size whose rows the first sum does not
-// read in whole lines: of vectors (16384 x 56 x 56 31.1 / 25.1, 8192 x 80 x 80 40.8 / 30.9; f16, whose rows the first sum reads faster, 21.4 / 24.5 and 26.8 / 29.8, but 4096 x 48 x 48 8.1 / 7.4; 1150 x 56 x 56 6.1 / 6.1, 2345 x 104 x 224 21.2 / 29.8, 15498 x 64 x 64 24.6 / 26.2) or by elements in a
+// 5.5 / 4.8, 5720 x 32 x 32 6.5 / 5.5, 4576 x 14 x 14 5.4 / 5.1, 8475 x 10 x 10 5.8 / 6.8, 28556 x 6 x 5 6.1 / 9.2), and for many planes whose rows the first sum reads slower:
+// bf16 vectors (16384 x 56 x 56 31.1 / 25.1, 8192 x 80 x 80 40.8 / 30.9, 9456 x 64 x 64 16.6 / 13.1, 9456 x 128 x 128 68.9 / 50.5; 2048 x 160 x 160 38.6 / 41.9, 3200 of them 58.7 / 48.0; f16,
+// which it reads faster, 16384 x 56 x 56 21.4 / 24.5, 13024 x 112 x 112 51.6 / 57.9, but 4096 x 48 x 48 8.1 / 7.4; 1150 x 56 x 56 6.1 / 6.1) or elements in a
 // warp's two rounds (16384 x 55 x 55 92 / 53, 2048 x 33 x 33 9.9 / 8.4; 16384 x 28 x 28 15.3 / 22.2, 4096 x 109 x 109 29.9 / 54.4).  A few large planes would wait for one
 // warp each: 16 x 112 x 112 4.8 / 11.3, 16 x 109 x 109 4.8 / 26.3, 16 x 512 x 512 5.8 / 114.
 template <class T>
@@ -155,7 +156,7 @@ bool plane_sums(const Geometry& g, const void* grad_out, void* out) {
     if (planes > 0x7FFFFFFFull || g.oh > 0x7FFFFFFFull || g.ow > 0x7FFFFFFFull) return false;
     const size_t lanes = vec && nv <= 4 ? 4 : nv <= 8 ? 8 : nv <= 16 ? 16 : 32, trips = (g.oh + 128 / lanes - 1) / (128 / lanes) * ((nv + lanes - 1) / lanes);
     const bool small = trips <= 2 && planes <= (trips > 1 ? 4608 : 8192);
-    const bool of_vectors = trips >= 3 && g.ow >= 40 && g.ow % 64 != 0 && (std::is_same<T, bf16>::value ? trips <= 14 : trips <= 4 && planes <= 8192);
+    const bool of_vectors = std::is_same<T, bf16>::value ? g.ow >= 40 && g.ow <= 256 && (trips <= 14 || planes >= 3072) : trips >= 3 && trips <= 4 && g.ow >= 40 && g.ow % 64 != 0 && planes <= 8192;
     const bool many = planes >= 2048 && (vec ? of_vectors : trips <= 32 && g.ow > 32 && g.ow < 64);
     if (!small && !many) return false;
     const auto kernel = vec ? (lanes == 4 ? plane_sums_kernel<T, 8, 4> : lanes == 8 ? plane_sums_kernel<T, 8, 8> : lanes == 16 ? plane_sums_kernel<T, 8, 16> : plane_sums_kernel<T, 8, 32>)
