@@ -1060,6 +1060,23 @@ def test_which_operands_off_whole_lines_are_copied(cuda, m, n, k, copies):
     assert np.all(np.abs(D.decode(got, D.BF16).reshape(m, n) - ref) <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -22 * k)
 
 
+@pytest.mark.parametrize("m,n,k,copies", [(8, 3136, 400, 1), (40, 3136, 400, 0), (3136, 40, 320, 2)], ids=str)
+def test_which_operands_of_short_mn_major_rows_are_copied(cuda, m, n, k, copies):
+    """Rows of K of few elements, read by many tiles of a batch that shares them: what was measured to be the faster way."""
+    from maidenx_b200 import _lib
+    rng, batch = np.random.default_rng(1), 32
+    a_b, b_b = (0, k * n) if m < n else (m * k, 0)
+    a, b = (D.encode(rng.standard_normal(s), D.BF16) for s in ((batch if a_b else 1) * m * k, (batch if b_b else 1) * n * k))
+    a_st = [1, m] if m < n else [k, 1]
+    meta = H.matmul_metadata([batch, m, n], [batch, m, k], [batch, k, n], [a_b, *a_st], [b_b, n, 1], 0, 0)
+    got = H.run_matmul(cuda, D.BF16, meta, batch * m * n, a, b)
+    assert _lib.load().mx_debug_gemm_last_copies() == copies
+    x = np.broadcast_to(D.decode(a, D.BF16).reshape((-1, k, m) if m < n else (-1, m, k)), (batch, k, m) if m < n else (batch, m, k)).astype(np.float32)
+    y = np.broadcast_to(D.decode(b, D.BF16).reshape(-1, k, n), (batch, k, n)).astype(np.float32)
+    ref = ((x.transpose(0, 2, 1) if m < n else x) @ y).astype(np.float64)
+    assert np.all(np.abs(D.decode(got, D.BF16).reshape(batch, m, n) - ref) <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -18 * k)
+
+
 def test_large_workspaces_of_two_sizes_find_each_other_s_block(cuda):
     """Products whose workspaces are 392 and 401 MB, in turn behind a synchronisation: the larger one's block serves both, and no call maps memory."""
     import torch
